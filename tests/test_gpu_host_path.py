@@ -1,0 +1,129 @@
+"""The native host path of eager calls against the general path (torch custom ops / checked ctypes calls): same results,
+and what it does not handle is declined and behaves as before."""
+import math
+
+import pytest
+import torch
+
+from turboquant.core import PolarQuantConfig, make_codebook, make_wht_matrix, polarquant_compress
+from turboquant.kernels import _native
+from turboquant.kernels.packed_attention import packed_attention
+from turboquant.kernels.packed_compress import compress_k, compress_k_permuted, compress_v
+from turboquant.kernels.paged import CacheFormat, Codebooks, allocate_cache, compress_and_scatter, paged_decode_attention
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+class _Declines:
+    """Stands in for the native module: every call takes the general path."""
+
+    def __getattr__(self, name):
+        return lambda *a: None
+
+
+@pytest.fixture
+def general(monkeypatch):
+    def call(f, *a, **k):
+        with monkeypatch.context() as m:
+            m.setattr(_native, "_host", _Declines())
+            return f(*a, **k)
+    return call
+
+
+def _filled(fmt, lens, hkv, bs, dtype, seed=0):
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    nb = [-(-n // bs) for n in lens]
+    tables = torch.zeros(len(lens), max(nb), dtype=torch.int32, device=DEV)
+    perm = torch.randperm(sum(nb), generator=g, device=DEV).int()
+    slots, o = [], 0
+    for i, n in enumerate(lens):
+        tables[i, :nb[i]] = perm[o:o + nb[i]]
+        pos = torch.arange(n, device=DEV)
+        slots.append(tables[i, pos // bs].long() * bs + pos % bs)
+        o += nb[i]
+    K = torch.randn(sum(lens), hkv, 128, generator=g, device=DEV, dtype=dtype)
+    V = torch.randn(sum(lens), hkv, 128, generator=g, device=DEV, dtype=dtype)
+    return allocate_cache(sum(nb), bs, hkv, fmt, DEV), tables, torch.tensor(lens, dtype=torch.int32, device=DEV), K, V, torch.cat(slots)
+
+
+@pytest.mark.parametrize("fmt,dtype,bs", [(CacheFormat(2, 2, True), torch.float16, 16), (CacheFormat(3, 3, True), torch.bfloat16, 32),
+                                          (CacheFormat(4, 3, False), torch.float16, 16)])
+def test_paged_calls_match_the_general_path(general, fmt, dtype, bs):
+    cache, tables, lens, K, V, slots = _filled(fmt, [1, 17, 900, 33], 2, bs, dtype)
+    books = Codebooks(fmt, DEV)
+    other = cache.clone()
+    version = cache._version
+    compress_and_scatter(K, V, cache, slots, books, bs)
+    assert cache._version > version
+    general(compress_and_scatter, K, V, other, slots, books, bs)
+    assert torch.equal(cache, other)
+    qkv = torch.randn(4, 8 * 128 + 64, device=DEV, dtype=dtype)
+    q = qkv[:, :8 * 128].view(4, 8, 128)                         # rows of a wider projection: not contiguous
+    for kw in (dict(), dict(rotate_q=True, derotate_out=True, max_seq_len=900), dict(sparse_thresh=1e-6, chunk_pages=16),
+               dict(q_proj=q.contiguous().flip(0), rotate_q=True)):
+        a = paged_decode_attention(q, cache, tables, lens, books, bs, **kw)
+        b = general(paged_decode_attention, q, cache, tables, lens, books, bs, **kw)
+        assert a.dtype == dtype and torch.equal(a, b), kw
+    out = torch.empty(4, 8, 128, dtype=dtype, device=DEV)
+    stats = torch.zeros(2, dtype=torch.int32, device=DEV)
+    res = paged_decode_attention(q, cache, tables, lens, books, bs, sparse_thresh=1e-6, out=out, skip_stats=stats)
+    assert res is out and torch.equal(out, paged_decode_attention(q, cache, tables, lens, books, bs, sparse_thresh=1e-6))
+    assert stats[0].item() == 2 * (1 + 2 + 57 + 3)                # pages of both KV heads
+    assert torch.equal(paged_decode_attention(q, cache, tables.long(), lens.long(), books, bs),
+                       paged_decode_attention(q, cache, tables, lens, books, bs))       # converted on the general path
+    assert _native.read_status(DEV) == 0
+
+
+@pytest.mark.parametrize("bits", [2, 3, 4])
+@pytest.mark.parametrize("n", [1, 130])
+def test_contiguous_calls_match_the_general_path(general, bits, n):
+    c, b = make_codebook(128, bits, device=DEV)
+    h = make_wht_matrix(128, device=DEV)
+    g = torch.Generator(device=DEV).manual_seed(n)
+    X = torch.randn(2 * n, 128, generator=g, device=DEV)
+    for x in (X, X.half(), X.half()[::2], X.double()):
+        for f, a in ((compress_k, (h, None, c, b)), (compress_k_permuted, (None, None, c, b)), (compress_v, (h, c, b))):
+            got, want = f(x, *a), general(f, x, *a)
+            assert all(torch.equal(p, q) and p.dtype == q.dtype for p, q in zip(got, want))
+    for qjl in (True, False):
+        got = polarquant_compress(X.view(n, 2, 128), c, b, PolarQuantConfig(bits=bits, use_qjl=qjl), h)
+        want = general(polarquant_compress, X.view(n, 2, 128), c, b, PolarQuantConfig(bits=bits, use_qjl=qjl), h)
+        assert got.keys() == want.keys() and all(torch.equal(got[k], want[k]) for k in want)
+    k, v = compress_k_permuted(X, h, None, c, b), compress_v(X, h, c, b)
+    packed = [t.view(2, n, *t.shape[1:]) for t in (*k, *v)]
+    q = torch.randn(2, 128, generator=g, device=DEV).half()
+    for splits in (None, 3):
+        assert torch.equal(packed_attention(q, q, *packed, c, 0.01, num_splits=splits),
+                           general(packed_attention, q, q, *packed, c, 0.01, num_splits=splits))
+    assert torch.equal(_native.wht_rows(X, 0.5), general(_native.wht_rows, X, 0.5))
+
+
+def test_declined_inputs_behave_as_before():
+    fmt = CacheFormat.named("turbo3")
+    cache, tables, lens, K, V, slots = _filled(fmt, [40], 2, 16, torch.float16)
+    books = Codebooks(fmt, DEV)
+    with pytest.raises(RuntimeError, match="no CPU path"):
+        compress_and_scatter(K.cpu(), V, cache, slots, books, 16)
+    with pytest.raises(ValueError, match="share a dtype"):
+        compress_and_scatter(K, V.float(), cache, slots, books, 16)
+    with pytest.raises(ValueError, match="cache shape"):
+        compress_and_scatter(K, V, cache, slots, books, 32)
+    compress_and_scatter(K, V, cache, slots, books, 16)
+    q = torch.randn(1, 8, 128, device=DEV, dtype=torch.float16)
+    want = paged_decode_attention(q, cache, tables, lens, books, 16)
+    with pytest.raises(ValueError, match="fp16 or bf16"):
+        paged_decode_attention(q.float(), cache, tables, lens, books, 16)
+    with pytest.raises(ValueError, match="multiple of kv heads"):
+        paged_decode_attention(q[:, :7], cache, tables, lens, books, 16)
+    with torch._subclasses.FakeTensorMode(allow_non_fake_inputs=True) as mode:
+        fake = mode.from_tensor(q)
+        assert type(paged_decode_attention(fake, cache, tables, lens, books, 16)).__name__ == "FakeTensor"
+    traced = q.clone().requires_grad_(True)                      # autograd sees the operator
+    assert torch.equal(paged_decode_attention(traced, cache, tables, lens, books, 16), want)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):                                # launches follow the current stream
+        again = paged_decode_attention(q, cache, tables, lens, books, 16, chunk_pages=1, sm_scale=1 / math.sqrt(128))
+    side.synchronize()
+    assert (again.float() - want.float()).abs().max() <= 2e-3

@@ -1,8 +1,12 @@
-"""ctypes binding of libtq_b200.so and its registration as torch custom ops.
+"""Bindings of libtq_b200.so: the native host path of eager calls, ctypes, and torch custom ops.
 
 The library is the only implementation: if it cannot be loaded, every entry
 point raises.  Set TQ_B200_SO to load it from a non-default path (the role
 TQ_FP4_PA_SO plays in the reference, turboquant/integration/tq_fp4_backend.py:59-76).
+
+Eager calls go through `_tq_host.so` (csrc/tq_host.cpp), which checks the arguments, allocates the outputs and
+launches in one native call.  It declines (returns None) whatever it does not handle: tracing, tensor subclasses,
+dispatch modes, autograd, inputs that need a conversion, invalid arguments.  Those take the general path below.
 
 Ops registered (namespace `tq_b200`):
   compress_paged(key, value, cache, slot_mapping, kc, kb, vc, vb, block_size, k_bits, v_bits, use_qjl, prerotated)
@@ -13,6 +17,7 @@ Ops registered (namespace `tq_b200`):
 from __future__ import annotations
 
 import ctypes
+import importlib.util
 import os
 from typing import Optional
 
@@ -29,6 +34,7 @@ IO_DEROTATE_OUT = 0x200    # write the decode output in original space
 IO_TCGEN05 = 0x400         # tensor-memory variant of the decode kernel (2- / 3-bit codebooks, no Sparse-V)
 
 _lib: Optional[ctypes.CDLL] = None
+_host = None
 
 
 def library_path() -> str:
@@ -73,8 +79,28 @@ def lib() -> ctypes.CDLL:
                  "tq_decode_paged_static", "tq_wht_rows", "tq_compress_k", "tq_compress_v", "tq_polarquant_compress",
                  "tq_packed_attention_auto_splits", "tq_packed_attention"):
         getattr(L, name).restype = i32
+    _load_host(path)
     _lib = L
     return L
+
+
+def _load_host(library: str) -> None:
+    global _host
+    path = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "lib", "_tq_host.so")
+    if not os.path.exists(path):
+        raise RuntimeError(f"_tq_host.so not found at {path}: build it with `python turboquant-amd_b200/build.py`")
+    spec = importlib.util.spec_from_file_location("_tq_host", path)
+    module = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(module)
+    module.bind(library)
+    _host = module
+
+
+def host():
+    """The native host module (csrc/tq_host.cpp)."""
+    if _host is None:
+        lib()
+    return _host
 
 
 def _check(rc: int, what: str) -> None:
@@ -130,6 +156,8 @@ def status_word(device: torch.device) -> torch.Tensor:
         device = torch.device("cuda", torch.cuda.current_device())
     if device not in _status:
         _status[device] = torch.zeros(1, dtype=torch.int32, device=device)
+        if device.type == "cuda":
+            host().set_status(device.index, _status[device])   # from now on the native path knows it
     return _status[device]
 
 
@@ -263,6 +291,10 @@ def _decode_paged_impl(out, q_rot, q_proj, cache, block_tables, seq_lens, kc, vc
 
 def wht_rows(x: torch.Tensor, scale: float = 1.0, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """x [..., 128] -> scale * (x @ H) with the fast transform; same dtype."""
+    if out is None and not torch.compiler.is_compiling():
+        res = host().wht_rows(x, scale)
+        if res is not None:
+            return res
     dev = _require_cuda(x)
     if x.shape[-1] != 128 or x.dtype not in _DTYPES:
         raise ValueError("x must be [..., 128] in fp16, bf16 or fp32")
@@ -276,6 +308,9 @@ def wht_rows(x: torch.Tensor, scale: float = 1.0, out: Optional[torch.Tensor] = 
 
 
 def polarquant(x: torch.Tensor, centroids, boundaries, bits: int, use_qjl: bool, rotate: bool) -> dict:
+    res = None if torch.compiler.is_compiling() else host().polarquant(x, centroids, boundaries, bits, use_qjl, rotate)
+    if res is not None:
+        return dict(zip(("indices", "norms", "k_mse_rot", "signs", "rot_residual_norm"), res))
     dev = _require_cuda(x)
     if x.shape[-1] != 128:
         raise ValueError("only head_dim 128 is supported")

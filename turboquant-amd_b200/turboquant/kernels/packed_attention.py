@@ -39,6 +39,11 @@ def packed_attention(Q, Q_proj, k_idx_packed, k_signs_packed, k_r_norm, k_norm,
                      num_splits=None, block_sk=None, num_warps=None, num_stages=None):
     """Q, Q_proj fp16 [BH, 128]; packed K/V as produced by compress_k_permuted / compress_v,
     reshaped to [BH, Sk, ...]; centroids fp32 [4 | 8 | 16]; returns fp16 [BH, 128]."""
+    if not torch.compiler.is_compiling():
+        res = _native.host().packed_attention(Q, Q_proj, k_idx_packed, k_signs_packed, k_r_norm, k_norm, v_idx_packed, v_norm,
+                                              centroids, corr_scale, num_splits or 0)
+        if res is not None:
+            return res
     dev = _native._require_cuda(Q, Q_proj, k_idx_packed, k_signs_packed, k_r_norm, k_norm, v_idx_packed, v_norm)
     BH, D = Q.shape
     if D != 128:

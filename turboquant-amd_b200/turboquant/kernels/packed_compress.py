@@ -159,10 +159,15 @@ def _compress_k_general(K, PiT, PiST, centroids, boundaries, permute: bool):
 
 
 def _compress_k(K, PiT, PiST, centroids, boundaries, permute: bool):
+    fused = _fused_ok(PiT, PiST)
+    if fused and not torch.compiler.is_compiling():
+        res = _native.host().compress_k(K, centroids, boundaries, PiT is not None, permute)
+        if res is not None:
+            return res
     dev = _native._require_cuda(K)
     if K.dim() != 2 or K.shape[1] != 128:
         raise ValueError("K must be [N, 128]")
-    if not _fused_ok(PiT, PiST):
+    if not fused:
         return _compress_k_general(K, PiT, PiST, centroids, boundaries, permute)
     rotate = _check_rotation(PiT, PiST)
     bits = _bits_of(centroids)
@@ -196,10 +201,15 @@ def compress_k_permuted(K, PiT, PiST, centroids, boundaries):
 
 def compress_v(V, PiT, centroids, boundaries):
     """-> (v_idx uint8 [N, 16*bits], v_norm fp16 [N])."""
+    fused = PiT is None or _is_wht(PiT)
+    if fused and not torch.compiler.is_compiling():
+        res = _native.host().compress_v(V, centroids, boundaries, PiT is not None)
+        if res is not None:
+            return res
     dev = _native._require_cuda(V)
     if V.dim() != 2 or V.shape[1] != 128:
         raise ValueError("V must be [N, 128]")
-    if PiT is not None and not _is_wht(PiT):      # an orthogonal matrix other than the WHT: rotate by a matrix product
+    if not fused:      # an orthogonal matrix other than the WHT: rotate by a matrix product
         return compress_v(_rotate_general(V, PiT).contiguous(), None, centroids, boundaries)
     rotate = _check_rotation(PiT, None)
     bits = _bits_of(centroids)

@@ -82,11 +82,14 @@ def compress_and_scatter(key: torch.Tensor, value: torch.Tensor, cache: torch.Te
     slots are clamped to 0 like the reference's scatter does.
     """
     fmt = books.fmt
+    if not torch.compiler.is_compiling() and _native.host().compress_paged(
+            key, value, cache, slot_mapping, books.kc, books.kb, books.vb, block_size, fmt.k_bits, fmt.v_bits, fmt.use_qjl,
+            (1 if prerotated else 0) | (_native.COMPRESS_TCGEN05 if tcgen05 else 0)):
+        return
     if slot_mapping.dtype != torch.int64:
         slot_mapping = slot_mapping.to(torch.int64)
     if tcgen05:
         # opt-in variant: rotation of fp16 / bf16 rows as a tcgen05 product (large launches only; otherwise ignored)
-        from turboquant.kernels import _native
         _native._compress_paged_impl(key, value, cache, slot_mapping.contiguous(), books.kc, books.kb, books.vc, books.vb,
                                      block_size, fmt.k_bits, fmt.v_bits, fmt.use_qjl, prerotated, tcgen05=True)
         return
@@ -119,7 +122,6 @@ def paged_decode_attention(q: torch.Tensor, cache: torch.Tensor, block_tables: t
         sm_scale = 1.0 / math.sqrt(128)
     if corr_scale is None:
         corr_scale = math.sqrt(math.pi / 2) / 128
-    q = q.contiguous()
     # Both rotations run inside the decode kernels (query rotated while its fragments are loaded, output
     # de-rotated where it is normalised); only a separate q_proj forces the query rotation to be its own pass.
     flags = _native.IO_DEROTATE_OUT if derotate_out else 0
@@ -129,7 +131,14 @@ def paged_decode_attention(q: torch.Tensor, cache: torch.Tensor, block_tables: t
         flags |= _native.IO_ROTATE_Q
         q_in = q
     else:
-        q_in = _native.wht_rows(q) if rotate_q else q
+        q_in = _native.wht_rows(q.contiguous()) if rotate_q else q
+    if not static_scratch and not torch.compiler.is_compiling():
+        res = _native.host().decode(q_in, cache, block_tables, seq_lens, books.kc, books.vc, q_proj, out, skip_stats, sm_scale,
+                                    corr_scale, sparse_thresh, block_size, fmt.k_bits, fmt.v_bits, fmt.use_qjl, chunk_pages,
+                                    flags, max_seq_len)
+        if res is not None:
+            return res
+    q_in = q_in.contiguous()
     if block_tables.dtype != torch.int32:
         block_tables = block_tables.to(torch.int32)
     if seq_lens.dtype != torch.int32:
