@@ -112,6 +112,11 @@ int tq_decode_auto_chunk_pages(int num_seqs, int num_kv_heads, int num_q_heads, 
 int64_t tq_decode_workspace_bytes(int num_seqs, int num_q_heads, int num_kv_heads,
                                   int max_pages_per_seq, int chunk_pages);
 
+/* Bytes of workspace with which tq_decode_paged(chunk_pages = 0) runs the kernel that suits the shape best: at least
+ * tq_decode_workspace_bytes(...), with which it runs the chunked kernel; about 20 MB where the persistent kernel is the
+ * better one.  Host only. */
+int64_t tq_decode_auto_workspace_bytes(int num_seqs, int num_q_heads, int num_kv_heads, int max_pages_per_seq);
+
 /* Asymmetric packed paged decode attention with GQA and split-K, one query
  * token per sequence.  Replaces _tq_v12_sparse_v_kernel / _tq_v11_single_kernel
  * (turboquant/kernels/sparse_v.py:26-159, 164-261) and, for the score

@@ -20,6 +20,8 @@
 // turboquant/kernels/packed_attention.py:150-196,273-284, paging and GQA head
 // mapping of turboquant/kernels/sparse_v.py:39-48,70-71, skip rule of
 // sparse_v.py:108-123,149.
+#include <type_traits>
+
 #include "tq_common.cuh"
 
 namespace tq {
@@ -639,31 +641,57 @@ int launch_partial(const DecodeParams& p, dim3 grid, cudaStream_t stream) {
 }  // namespace
 }  // namespace tq
 
+#include "tq_decode_stream.cuh"
 #include "tq_decode_umma.cuh"
 
 namespace tq {
 namespace {
 
+// What a call runs: the chunked kernel on `grid`, or, with `stream` set, the persistent kernel.
+struct Plan {
+    dim3 grid;
+    const StreamParams* stream;
+    bool qjl, sparse;
+};
+
+template <int KB, int VB, bool QJL, bool SPARSE>
+int launch_planned(const DecodeParams& p, const Plan& plan, cudaStream_t stream) {
+    return plan.stream ? launch_stream<KB, VB, QJL, SPARSE>(*plan.stream, stream) : launch_partial<KB, VB, QJL, SPARSE>(p, plan.grid, stream);
+}
+
 template <int KB, int VB>
-int dispatch_flags(const DecodeParams& p, bool qjl, bool sparse, dim3 grid, cudaStream_t stream) {
+int dispatch_flags(const DecodeParams& p, const Plan& plan, cudaStream_t stream) {
     if constexpr (KB <= 3 && VB <= 3) {
         // on request (TQ_IO_TCGEN05): the tensor-memory kernel, for 2- and 3-bit codebooks without the Sparse-V skip
-        if (!sparse && p.use_tcgen05) return qjl ? launch_umma<KB, VB, true>(p, grid, stream) : launch_umma<KB, VB, false>(p, grid, stream);
+        if (!plan.sparse && p.use_tcgen05)
+            return plan.qjl ? launch_umma<KB, VB, true>(p, plan.grid, stream) : launch_umma<KB, VB, false>(p, plan.grid, stream);
     }
-    if (qjl) return sparse ? launch_partial<KB, VB, true, true>(p, grid, stream) : launch_partial<KB, VB, true, false>(p, grid, stream);
-    return sparse ? launch_partial<KB, VB, false, true>(p, grid, stream) : launch_partial<KB, VB, false, false>(p, grid, stream);
+    if (plan.qjl) return plan.sparse ? launch_planned<KB, VB, true, true>(p, plan, stream) : launch_planned<KB, VB, true, false>(p, plan, stream);
+    return plan.sparse ? launch_planned<KB, VB, false, true>(p, plan, stream) : launch_planned<KB, VB, false, false>(p, plan, stream);
 }
 
 template <int KB>
-int dispatch_v(const DecodeParams& p, int vb, bool qjl, bool sparse, dim3 grid, cudaStream_t stream) {
+int dispatch_v(const DecodeParams& p, int vb, const Plan& plan, cudaStream_t stream) {
     switch (vb) {
 #ifndef TQ_DEC_QUICK
-        case 2: return dispatch_flags<KB, 2>(p, qjl, sparse, grid, stream);
-        case 4: return dispatch_flags<KB, 4>(p, qjl, sparse, grid, stream);
+        case 2: return dispatch_flags<KB, 2>(p, plan, stream);
+        case 4: return dispatch_flags<KB, 4>(p, plan, stream);
 #endif
-        case 3: return dispatch_flags<KB, 3>(p, qjl, sparse, grid, stream);
+        case 3: return dispatch_flags<KB, 3>(p, plan, stream);
     }
     return TQ_ERR_UNSUPPORTED;
+}
+
+#ifndef TQ_STREAM_MIN
+#define TQ_STREAM_MIN 1
+#endif
+constexpr int64_t kStreamMinPages = TQ_STREAM_MIN;
+// Workspace of the persistent kernel, or 0 where the chunked kernel is the better one.
+int64_t stream_bytes(int64_t ns, int64_t hq, int64_t hkv, int64_t max_pages) {
+    const int64_t items = hkv * ((hq / hkv + 7) / 8);
+    const int64_t pages = ns * max_pages * items;
+    if (pages < kStreamMinPages || pages > INT32_MAX) return 0;
+    return 2ll * kStreamCtas * kStreamWarps * (kStreamSlotFloats + 16) * static_cast<int64_t>(sizeof(float)) + (ns + 1) * 4;
 }
 
 }  // namespace
@@ -730,6 +758,13 @@ extern "C" int64_t tq_decode_workspace_bytes(int num_seqs, int num_q_heads, int 
     return slots * (kHeadDim + 2) * static_cast<int64_t>(sizeof(float));
 }
 
+extern "C" int64_t tq_decode_auto_workspace_bytes(int num_seqs, int num_q_heads, int num_kv_heads, int max_pages_per_seq) {
+    const int64_t chunked = tq_decode_workspace_bytes(num_seqs, num_q_heads, num_kv_heads, max_pages_per_seq, 0);
+    if (chunked < 0) return chunked;
+    const int64_t stream = stream_bytes(num_seqs, num_q_heads, num_kv_heads, max_pages_per_seq);
+    return stream > chunked ? stream : chunked;
+}
+
 extern "C" int tq_decode_paged(void* out, const void* q_rot, const void* q_proj, int io_dtype, const void* cache,
                                int64_t num_blocks, int block_size, const int32_t* block_tables, int64_t bt_stride,
                                const int32_t* seq_lens, const float* k_centroids, const float* v_centroids,
@@ -751,10 +786,14 @@ extern "C" int tq_decode_paged(void* out, const void* q_rot, const void* q_proj,
     if ((reinterpret_cast<uintptr_t>(cache) | reinterpret_cast<uintptr_t>(q_rot) | reinterpret_cast<uintptr_t>(out) |
          reinterpret_cast<uintptr_t>(q_proj)) & 15)
         return TQ_ERR_ARG;
+    // The persistent kernel takes the calls that leave the split to the library and bring the workspace for it.
+    const bool tensor_memory = use_tcgen05 && k_bits <= 3 && v_bits <= 3 && !(sparse_thresh > 0.f);
+    const int64_t stream_need = chunk_pages > 0 || tensor_memory ? 0 : stream_bytes(num_seqs, num_q_heads, num_kv_heads, max_pages_per_seq);
+    const bool persistent = stream_need > 0 && workspace && workspace_bytes >= stream_need && !(reinterpret_cast<uintptr_t>(workspace) & 15);
     if (chunk_pages <= 0) chunk_pages = tq_decode_auto_chunk_pages(num_seqs, num_kv_heads, num_q_heads, max_pages_per_seq);
     const int64_t need = tq_decode_workspace_bytes(num_seqs, num_q_heads, num_kv_heads, max_pages_per_seq, chunk_pages);
     const int max_chunks = (max_pages_per_seq + chunk_pages - 1) / chunk_pages;
-    if (max_chunks > 1 && (!workspace || workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 15)))
+    if (!persistent && max_chunks > 1 && (!workspace || workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 15)))
         return TQ_ERR_WORKSPACE;
     if (num_seqs > 65535 || max_chunks > 65535) return TQ_ERR_UNSUPPORTED;
 
@@ -794,20 +833,34 @@ extern "C" int tq_decode_paged(void* out, const void* q_rot, const void* q_proj,
     p.use_tcgen05 = use_tcgen05;
     p.share_tables = (k_bits == v_bits && k_centroids == v_centroids) ? 1 : 0;
 
-    const dim3 grid(max_chunks, num_kv_heads * p.ngroups, num_seqs);
-    const bool qjl = use_qjl != 0, sparse = sparse_thresh > 0.f;
+    StreamParams sp;
+    if (persistent) {
+        sp.d = p;
+        sp.ns = num_seqs;
+        sp.HG = num_kv_heads * p.ngroups;
+        sp.n_warps = kStreamCtas * kStreamWarps;
+        sp.part_o = static_cast<float*>(workspace);
+        sp.part_ml = reinterpret_cast<float2*>(sp.part_o + 2ll * sp.n_warps * kStreamSlotFloats);
+        sp.prefix = reinterpret_cast<int32_t*>(sp.part_ml + 2ll * sp.n_warps * 8);
+    }
+    const Plan plan = {dim3(max_chunks, num_kv_heads * p.ngroups, num_seqs), persistent ? &sp : nullptr, use_qjl != 0, sparse_thresh > 0.f};
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     int rc;
     switch (k_bits) {
 #ifndef TQ_DEC_QUICK
-        case 2: rc = dispatch_v<2>(p, v_bits, qjl, sparse, grid, st); break;
-        case 4: rc = dispatch_v<4>(p, v_bits, qjl, sparse, grid, st); break;
+        case 2: rc = dispatch_v<2>(p, v_bits, plan, st); break;
+        case 4: rc = dispatch_v<4>(p, v_bits, plan, st); break;
 #endif
-        case 3: rc = dispatch_v<3>(p, v_bits, qjl, sparse, grid, st); break;
+        case 3: rc = dispatch_v<3>(p, v_bits, plan, st); break;
         default: return TQ_ERR_UNSUPPORTED;
     }
     if (rc != TQ_OK) return rc;
-    if (max_chunks > 1) {
+    if (persistent) {
+        const int64_t rows = static_cast<int64_t>(num_seqs) * num_q_heads;
+        if (launch_chained(decode_stream_merge_kernel, dim3(static_cast<unsigned>((rows + kMergeWarps - 1) / kMergeWarps)), dim3(kMergeWarps * 32),
+                           0, st, sp) != cudaSuccess)
+            return TQ_ERR_LAUNCH;
+    } else if (max_chunks > 1) {
         if (launch_chained(decode_merge_kernel, dim3(num_q_heads, num_seqs), dim3(kHeadDim), 0, st, p) != cudaSuccess)
             return TQ_ERR_LAUNCH;
     }

@@ -1,0 +1,626 @@
+// Decode attention for launches that fill the GPU: one persistent CTA of 16 warps per SM, every warp streams its own
+// contiguous share of all pages.
+//
+// All (sequence, KV head, query group) items of the batch are laid end to end, page after page; warp w of W takes pages
+// [w U / W, (w + 1) U / W).  The warps never wait for one another: a warp keeps its running maximum, denominators and
+// accumulators while it stays inside an item, writes the output itself when it saw the whole item, and otherwise leaves
+// one of at most two partial results (the item it started in the middle of, the item it could not finish) for
+// decode_stream_merge_kernel.  Against the chunked kernel (4-warp CTAs, one chunk of one item each) this takes away the
+// last wave that is three quarters full, the table fill, pipeline start and block-wide merge per chunk, and the empty
+// CTAs of a ragged batch.
+namespace tq {
+namespace {
+
+constexpr int kStreamWarps = 16;
+constexpr int kStreamThreads = kStreamWarps * 32;
+constexpr int kStreamStages = 4;
+constexpr int kStreamTable = 65536;          // 256 entries of 256 bytes: 128 bytes for K, 128 bytes for V
+constexpr int kStreamCtas = 148;             // one per SM
+constexpr int kStreamSmem = 230144;          // dynamic part of the 227 KB an SM gives one CTA
+constexpr int kStreamSlotFloats = 8 * kHeadDim;
+
+struct StreamParams {
+    DecodeParams d;
+    int ns, HG;          // sequences; items per sequence (KV heads x query groups)
+    int n_warps;
+    float* part_o;       // [2 n_warps][8][128]: slot 2 w + 1 starts at its item's first page, slot 2 w does not
+    float2* part_ml;     // [2 n_warps][8] (maximum, denominator)
+    int32_t* prefix;     // [ns + 1] pages of all sequences before s
+};
+
+// Warps that share `total` pages: all of them, but none with fewer than kStreamMinShare pages.
+#ifndef TQ_MIN_SHARE
+#define TQ_MIN_SHARE 4
+#endif
+constexpr int kStreamMinShare = TQ_MIN_SHARE;
+__device__ __forceinline__ int active_warps(const StreamParams& sp, int64_t total) {
+    const int64_t most = (total + kStreamMinShare - 1) / kStreamMinShare;
+    return most < sp.n_warps ? static_cast<int>(most) : sp.n_warps;
+}
+
+__device__ __forceinline__ int pages_of(const DecodeParams& p, int len) {
+    return len <= 0 ? 0 : min((len + kPageTokens - 1) / kPageTokens, p.max_pages);
+}
+
+// Byte k of w as the second byte of a table address: entry stride 256, so the address is one byte permute.
+template <int K>
+__device__ __forceinline__ uint32_t table_pair(uint32_t w, uint32_t base) {
+    uint32_t v;
+    asm("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(prmt(w, base, 0x7604u | (K << 4))));
+    return v;
+}
+template <int K>
+__device__ __forceinline__ uint2 table_quad(uint32_t w, uint32_t base) {
+    uint2 v;
+    asm("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(prmt(w, base, 0x7604u | (K << 4))));
+    return v;
+}
+
+__device__ __forceinline__ uint32_t bit_select(uint32_t a, uint32_t b, uint32_t mask) { return (a & ~mask) | (b & mask); }
+
+// Words whose bytes address the table.  The table does not look at the spare top bit of a 3-bit nibble.
+template <int BITS>
+__device__ __forceinline__ void table_words(const uint32_t* w, uint32_t (&mw)[4]) {
+    if constexpr (BITS == 4) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) mw[j] = w[j];
+    } else {
+        mw[0] = w[0];
+        mw[1] = w[1];
+        mw[2] = w[2];
+        mw[3] = bit_select(bit_select(w[0] >> 3, w[1] >> 2, 0x22222222u), w[2] >> 1, 0x44444444u);
+    }
+}
+
+template <int BITS>
+__device__ __forceinline__ void fill_stream_table(uint32_t smem_addr, const float* __restrict__ c, int warp, int lane) {
+    const float cv = __half2float(__float2half_rn(__ldg(c + (lane & ((1 << BITS) - 1)))));
+    for (int b = warp; b < 256; b += kStreamWarps) {
+        int i0, i1;
+        if constexpr (BITS == 2) {
+            i0 = (lane & 1) ? (b >> 2) & 3 : b & 3;
+            i1 = (lane & 1) ? (b >> 6) & 3 : (b >> 4) & 3;
+        } else {
+            i0 = b & ((1 << BITS) - 1);
+            i1 = (b >> 4) & ((1 << BITS) - 1);
+        }
+        const uint32_t v = pack_half2(__shfl_sync(0xffffffffu, cv, i0), __shfl_sync(0xffffffffu, cv, i1));
+        asm volatile("st.shared.u32 [%0], %1;" ::"r"(smem_addr + b * 256 + lane * 4), "r"(v) : "memory");
+    }
+}
+
+__device__ __forceinline__ bool wait_bounded(uint32_t bar, uint32_t parity) {
+    for (int i = 0; i < (1 << 22); ++i) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(bar), "r"(parity)
+            : "memory");
+        if (ok) return true;
+    }
+    return false;
+}
+
+__device__ __forceinline__ void copy_in(uint32_t dst, const uint8_t* src, uint32_t bytes, uint32_t bar) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src),
+                 "r"(bytes), "r"(bar)
+                 : "memory");
+}
+
+// 32 values (the lane's quarter of a row of 128) to fp16 / bf16.
+__device__ __forceinline__ void store_row32(void* out, int64_t off, int io_dtype, const float (&x)[32]) {
+    uint4* dst = reinterpret_cast<uint4*>(static_cast<uint16_t*>(out) + off);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        uint32_t w[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float a = x[8 * i + 2 * j], b = x[8 * i + 2 * j + 1];
+            if (io_dtype == TQ_DTYPE_F16) {
+                w[j] = pack_half2(a, b);
+            } else {
+                const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+                w[j] = *reinterpret_cast<const uint32_t*>(&h);
+            }
+        }
+        dst[i] = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+}
+
+template <int KB, int VB, bool QJL, bool SPARSE>
+__global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const StreamParams sp) {
+    constexpr int NWK = KB + (QJL ? 1 : 0);
+    constexpr int RK = 16 * NWK;
+    constexpr int KN_OFF = 16 * RK;
+    constexpr int KRN_OFF = KN_OFF + 32;
+    constexpr int KPART = KN_OFF + 32 + (QJL ? 32 : 0);
+    constexpr int VN_OFF = KPART + 256 * VB;
+    constexpr int PAGE = KPART + 256 * VB + 32;
+    constexpr int NSTAGE = kStreamStages;
+    constexpr int RING = NSTAGE * PAGE;
+    constexpr int kBars = kStreamWarps * 2 * NSTAGE * 8;
+    // Wherever the dynamic part starts in the first 4 KB, the rings fit around the table.
+    static_assert((kStreamTable - 4096 - kBars) / RING + (kStreamSmem + 1024 - 2 * kStreamTable) / RING >= kStreamWarps, "rings do not fit");
+    const DecodeParams& p = sp.d;
+
+    extern __shared__ __align__(128) uint8_t smem[];
+    __shared__ int sm_scan[kStreamThreads + 1];
+    __shared__ int sm_wsum[kStreamWarps];
+
+    pdl_release_and_wait();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int gid = lane >> 2, tig = lane & 3;
+
+    // ---- shared memory: the table on a 64 KB boundary (its addresses are built by a byte permute), barriers and the
+    // rings of as many warps as fit below it, the other rings above it
+    const uint32_t base = smem_u32(smem);
+    const uint32_t tab = (base + kStreamTable - 1) & ~static_cast<uint32_t>(kStreamTable - 1);
+    const uint32_t room = tab - base;
+    const bool bars_low = room >= kBars;
+    const uint32_t bars = bars_low ? base : tab + kStreamTable;
+    const int n_low = bars_low ? static_cast<int>((room - kBars) / RING) : static_cast<int>(room / RING);
+    const uint32_t ring = warp < n_low ? base + (bars_low ? kBars : 0) + warp * RING
+                                       : tab + kStreamTable + (bars_low ? 0 : kBars) + (warp - n_low) * RING;
+    const uint32_t bar = bars + warp * 2 * NSTAGE * 8;     // [0 .. NSTAGE) page (or K part), [NSTAGE ..) late V part
+
+    if (lane < 2 * NSTAGE) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar + lane * 8) : "memory");
+    fence_barrier_init();
+
+    // ---- pages before each thread's run of sequences (every CTA does the same scan over all lengths)
+    const int per = (sp.ns + kStreamThreads - 1) / kStreamThreads;
+    int own = 0;
+    for (int s = threadIdx.x * per; s < min(sp.ns, (static_cast<int>(threadIdx.x) + 1) * per); ++s) own += pages_of(p, p.seq_lens[s]);
+    int incl = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+    }
+    if (lane == 31) sm_wsum[warp] = incl;
+    fill_stream_table<KB>(tab, p.kc, warp, lane);
+    fill_stream_table<VB>(tab + 128, p.vc, warp, lane);
+    __syncthreads();
+    int before = incl - own;
+    for (int w = 0; w < warp; ++w) before += sm_wsum[w];
+    sm_scan[threadIdx.x] = before;
+    if (threadIdx.x == kStreamThreads - 1) sm_scan[kStreamThreads] = before + own;
+    if (blockIdx.x == 0) {   // for the merge kernel; flags and zero outputs are written once, too
+        int acc = before;
+        for (int s = threadIdx.x * per; s < min(sp.ns, (static_cast<int>(threadIdx.x) + 1) * per); ++s) {
+            const int len = p.seq_lens[s];
+            sp.prefix[s] = acc;
+            acc += pages_of(p, len);
+            if (len > p.max_pages * kPageTokens && p.status) atomicOr(p.status, TQ_STATUS_BAD_BLOCK);
+            if (len <= 0) {
+                uint4* o = reinterpret_cast<uint4*>(static_cast<uint16_t*>(p.out) + static_cast<int64_t>(s) * p.Hq * kHeadDim);
+                for (int i = 0; i < p.Hq * kHeadDim / 8; ++i) o[i] = make_uint4(0, 0, 0, 0);
+            }
+        }
+        if (threadIdx.x == kStreamThreads - 1) sp.prefix[sp.ns] = acc;
+    }
+    __syncthreads();
+
+    const int64_t total = static_cast<int64_t>(sm_scan[kStreamThreads]) * sp.HG;
+    const int gw = warp * gridDim.x + blockIdx.x;       // neighbouring shares on different SMs: few shares use all SMs
+    const int W = active_warps(sp, total);
+    if (gw >= W) return;
+    const int64_t first = total * gw / W;
+    const int n = static_cast<int>(total * (gw + 1) / W - first);   // this warp's pages, at least one
+
+    // ---- the item and page this warp starts in
+    int seq, hg, page, np, len;
+    {
+        int lo = 0, hi = kStreamThreads;
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if (static_cast<int64_t>(sm_scan[mid]) * sp.HG <= first) lo = mid; else hi = mid;
+        }
+        seq = lo * per;
+        int64_t at = static_cast<int64_t>(sm_scan[lo]) * sp.HG;
+        for (;; ++seq) {
+            len = __ldg(p.seq_lens + seq);
+            np = pages_of(p, len);
+            if (first < at + static_cast<int64_t>(np) * sp.HG) break;
+            at += static_cast<int64_t>(np) * sp.HG;
+        }
+        const int r = static_cast<int>(first - at);
+        hg = r / np;
+        page = r - hg * np;
+    }
+    auto kv_head = [&](int h) { return p.ngroups == 1 ? h : h / p.ngroups; };
+
+    // ---- copies in: lane l holds the source address of page 32 k + l of the warp's share, one window of 32 ahead
+    bool bad_block = false;
+    auto locate = [&](int s, int h, int pg) -> const uint8_t* {
+        int32_t blk = __ldg(p.block_tables + static_cast<int64_t>(s) * p.bt_stride + (pg >> p.sub_shift));
+        if (blk < 0 || blk >= p.num_blocks) {
+            bad_block = true;
+            blk = 0;
+        }
+        return p.cache + blk * p.block_stride + ((kv_head(h) << p.sub_shift) + (pg & ((1 << p.sub_shift) - 1))) * PAGE;
+    };
+    int wseq = seq, whg = hg, wpage = page, wnp = np, wbase = 0;     // where window `wbase / 32` starts
+    auto next_window = [&]() -> const uint8_t* {
+        const uint8_t* src = p.cache;
+        int s = wseq, h = whg, pg = wpage + lane, m = wnp;
+        if (wbase + lane < n) {
+            while (pg >= m) {
+                pg -= m;
+                if (++h == sp.HG) {
+                    h = 0;
+                    do m = pages_of(p, __ldg(p.seq_lens + ++s)); while (m == 0);
+                }
+            }
+            src = locate(s, h, pg);
+        }
+        wseq = __shfl_sync(0xffffffffu, s, 31);
+        whg = __shfl_sync(0xffffffffu, h, 31);
+        wpage = __shfl_sync(0xffffffffu, pg, 31) + 1;
+        wnp = __shfl_sync(0xffffffffu, m, 31);
+        wbase += 32;
+        return src;
+    };
+    const uint8_t* src = next_window();
+    const uint8_t* src_next = src;
+    const int first_lot = min(n, NSTAGE);
+    if (lane < first_lot) copy_in(ring + lane * PAGE, src, PAGE, bar + lane * 8);
+    if (n > 32) src_next = next_window();
+
+    const uint32_t klut = tab + (KB == 2 ? 8 * (lane & 15) : 4 * lane);
+    const uint32_t vlut = tab + 128 + (VB == 2 ? 8 * (lane & 15) : 4 * lane);
+    const uint32_t ring_k = ring + lane * (NWK * 4);
+    const uint32_t ring_n = ring + gid * 4;
+    const uint32_t ring_v = ring + (tig * 8 + gid) * 4;
+
+    bool timed_out = false;
+    uint32_t stage = 0, parity = 0;           // ring stage of the current page and the phase of its barrier
+    uint32_t v_parity = 0;                    // Sparse-V: bit s = phase of the late-V barrier of stage s
+    uint32_t v_with_k = (1u << NSTAGE) - 1u;  // Sparse-V: bit s = the page in stage s brought its V part along
+    uint32_t v_skipped = 0;
+    int idx = 0;                              // pages of the share that are done
+
+    while (idx < n && !timed_out) {
+        const int seg = min(np - page, n - idx);           // pages of this item in the share
+        const int kvh = kv_head(hg), qg = hg - kvh * p.ngroups;
+        const int head0 = kvh * p.G + qg * 8, nq = min(8, p.G - qg * 8);
+        const int64_t row = (static_cast<int64_t>(seq) * p.Hq + head0 + gid) * kHeadDim;
+
+        uint32_t qf[16], qpf[QJL ? 16 : 1];
+        float sq_init0 = 0.f, sq_init1 = 0.f;   // minus the query sums of the one-sided sign forms
+        {
+            float xq[32];
+            load_q32(p.q, row, tig, p.io_dtype, gid < nq, xq);
+            if (p.rotate_q) rotate_q32(xq, lane, p.io_dtype);
+            q_frag_from(xq, qf);
+            if constexpr (QJL) {
+                if (p.qp) load_q32(p.qp, row, tig, p.io_dtype, gid < nq, xq);
+                float corr;
+                qp_frag_signed_from(xq, qpf, corr);
+                corr += __shfl_xor_sync(0xffffffffu, corr, 1);
+                corr += __shfl_xor_sync(0xffffffffu, corr, 2);
+                sq_init0 = -__shfl_sync(0xffffffffu, corr, 8 * tig);
+                sq_init1 = -__shfl_sync(0xffffffffu, corr, 8 * tig + 4);
+            }
+        }
+        float m0 = -INFINITY, m1 = -INFINITY;   // softmax reference of queries 2 tig, 2 tig + 1 (log2 domain)
+        float l0 = 0.f, l1 = 0.f;
+        float oacc[8][4];
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int r = 0; r < 4; ++r) oacc[i][r] = 0.f;
+
+        auto one_page = [&](auto have_v, int j) {
+            constexpr bool HAVE_V = decltype(have_v)::value;
+            const uint32_t so = stage * PAGE;
+            if (!wait_bounded(bar + stage * 8, parity)) {
+                timed_out = true;
+                return;
+            }
+            // ---- scores of 16 tokens x 8 queries
+            uint32_t wa[NWK], wb[NWK];
+            lds_words<NWK, 0>(ring_k + so, wa);
+            lds_words<NWK, 32 * NWK * 4>(ring_k + so, wb);
+            float sm[4] = {0.f, 0.f, 0.f, 0.f};
+            float sq[4] = {sq_init0, sq_init1, sq_init0, sq_init1}, sq2[4] = {0.f, 0.f, 0.f, 0.f};
+            if constexpr (KB == 2) {
+#pragma unroll
+                for (int jw = 0; jw < 2; ++jw) {
+                    const uint2 a0 = table_quad<0>(wa[jw], klut), a1 = table_quad<1>(wa[jw], klut);
+                    const uint2 b0 = table_quad<0>(wb[jw], klut), b1 = table_quad<1>(wb[jw], klut);
+                    mma_f16_16816(sm, a0.x, b0.x, a1.x, b1.x, qf[8 * jw], qf[8 * jw + 1]);
+                    mma_f16_16816(sm, a0.y, b0.y, a1.y, b1.y, qf[8 * jw + 4], qf[8 * jw + 5]);
+                    const uint2 c0 = table_quad<2>(wa[jw], klut), c1 = table_quad<3>(wa[jw], klut);
+                    const uint2 d0 = table_quad<2>(wb[jw], klut), d1 = table_quad<3>(wb[jw], klut);
+                    mma_f16_16816(sm, c0.x, d0.x, c1.x, d1.x, qf[8 * jw + 2], qf[8 * jw + 3]);
+                    mma_f16_16816(sm, c0.y, d0.y, c1.y, d1.y, qf[8 * jw + 6], qf[8 * jw + 7]);
+                }
+            } else {
+                uint32_t mwa[4], mwb[4];
+                table_words<KB>(wa, mwa);
+                table_words<KB>(wb, mwb);
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    const uint32_t a0 = table_pair<0>(mwa[c], klut), a1 = table_pair<1>(mwa[c], klut);
+                    const uint32_t b0 = table_pair<0>(mwb[c], klut), b1 = table_pair<1>(mwb[c], klut);
+                    mma_f16_16816(sm, a0, b0, a1, b1, qf[4 * c], qf[4 * c + 1]);
+                    const uint32_t a2 = table_pair<2>(mwa[c], klut), a3 = table_pair<3>(mwa[c], klut);
+                    const uint32_t b2 = table_pair<2>(mwb[c], klut), b3 = table_pair<3>(mwb[c], klut);
+                    mma_f16_16816(sm, a2, b2, a3, b3, qf[4 * c + 2], qf[4 * c + 3]);
+                }
+            }
+            if constexpr (QJL) {
+#pragma unroll
+                for (int ki = 0; ki < 4; ++ki) {
+                    const uint32_t xa = wa[KB] << (4 * ki), xb = wb[KB] << (4 * ki);
+                    mma_f16_16816(sq, (xa & 0x80008000u) | 0x3C003C00u, (xb & 0x80008000u) | 0x3C003C00u,
+                                  xa & 0x40004000u, xb & 0x40004000u, qpf[4 * ki], qpf[4 * ki + 1]);
+                    mma_f16_16816(sq2, xa & 0x20002000u, xb & 0x20002000u, xa & 0x10001000u, xb & 0x10001000u,
+                                  qpf[4 * ki + 2], qpf[4 * ki + 3]);
+                }
+            }
+            float2 kn = unpack_half2(lds_u32<KN_OFF>(ring_n + so));
+            kn.x *= p.qscale;
+            kn.y *= p.qscale;
+            float s0 = sm[0] * kn.x, s1 = sm[1] * kn.x, s2 = sm[2] * kn.y, s3 = sm[3] * kn.y;
+            if constexpr (QJL) {
+                float2 krn = unpack_half2(lds_u32<KRN_OFF>(ring_n + so));
+                krn.x *= p.qpscale;
+                krn.y *= p.qpscale;
+                s0 = fmaf(sq[0] + sq2[0], krn.x, s0);
+                s1 = fmaf(sq[1] + sq2[1], krn.x, s1);
+                s2 = fmaf(sq[2] + sq2[2], krn.y, s2);
+                s3 = fmaf(sq[3] + sq2[3], krn.y, s3);
+            }
+            const int valid_tokens = len - (page + j) * kPageTokens;
+            if (valid_tokens < kPageTokens) {   // only the last page of a sequence is partly filled
+                if (gid >= valid_tokens) { s0 = -INFINITY; s1 = -INFINITY; }
+                if (gid + 8 >= valid_tokens) { s2 = -INFINITY; s3 = -INFINITY; }
+            }
+            // ---- online softmax.  The reference m is raised only when a score exceeds it, and then to one above the
+            // largest score, so weights stay <= 1 and most pages need no shuffle and no rescaling.
+            const bool over = fmaxf(s0, s2) > m0 || fmaxf(s1, s3) > m1;
+            if (__any_sync(0xffffffffu, over)) {
+                float mx0 = fmaxf(s0, s2), mx1 = fmaxf(s1, s3);
+#pragma unroll
+                for (int o = 4; o < 32; o <<= 1) {
+                    mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, o));
+                    mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, o));
+                }
+                const float mn0 = mx0 > m0 ? mx0 + 1.f : m0, mn1 = mx1 > m1 ? mx1 + 1.f : m1;
+                const float al0 = ex2(m0 - mn0), al1 = ex2(m1 - mn1);
+                l0 *= al0;
+                l1 *= al1;
+                // accumulator rows belong to query gid: its factor comes from the lane that scored it
+                const float t0 = __shfl_sync(0xffffffffu, al0, gid >> 1);
+                const float t1 = __shfl_sync(0xffffffffu, al1, gid >> 1);
+                const float ag = (gid & 1) ? t1 : t0;
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) oacc[i][r] *= ag;
+                m0 = mn0;
+                m1 = mn1;
+            }
+            const float p0v = ex2(s0 - m0), p1v = ex2(s1 - m1), p2v = ex2(s2 - m0), p3v = ex2(s3 - m1);
+            l0 += p0v + p2v;
+            l1 += p1v + p3v;
+
+            // ---- Sparse-V: the V part is not needed when no weight of the group exceeds the threshold.  The reference is
+            // at most one above the running maximum.
+            bool do_v = true;
+            if constexpr (SPARSE) {
+                const float e = fmaxf(fmaxf(s0 - m0, s1 - m1), fmaxf(s2 - m0, s3 - m1));
+                do_v = __any_sync(0xffffffffu, e > p.log2_thresh - 1.f);
+            }
+            bool have = true;
+            if constexpr (SPARSE && !HAVE_V) {
+                if (do_v) {   // first needed page after a run of skipped ones: fetch its V part now
+                    const uint32_t vbar = bar + (NSTAGE + stage) * 8;
+                    if (lane == 0) copy_in(ring + so + KPART, locate(seq, hg, page + j) + KPART, PAGE - KPART, vbar);
+                    if (!wait_bounded(vbar, (v_parity >> stage) & 1u)) timed_out = true;
+                    v_parity ^= 1u << stage;
+                } else {
+                    ++v_skipped;
+                    have = false;
+                }
+            }
+            if (have) {
+                float2 vn = unpack_half2(lds_u32<VN_OFF>(ring_n + so));
+                if (valid_tokens < kPageTokens) {
+                    if (gid >= valid_tokens) vn.x = 0.f;
+                    if (gid + 8 >= valid_tokens) vn.y = 0.f;
+                }
+                const uint32_t t[2] = {movmatrix_trans(pack_half2(p0v * vn.x, p1v * vn.x)), movmatrix_trans(pack_half2(p2v * vn.y, p3v * vn.y))};
+#pragma unroll
+                for (int o = 0; o < 2; ++o) {
+                    const uint32_t vo = ring_v + so + o * 128;
+                    const uint32_t pa0 = t[o] & 0xffffu, pa1 = t[o] << 16, pa2 = t[o] >> 16, pa3 = t[o] & 0xffff0000u;
+                    uint32_t pw[VB];
+                    pw[0] = lds_u32<KPART>(vo);
+                    pw[1] = lds_u32<KPART + 256>(vo);
+                    if constexpr (VB > 2) pw[2] = lds_u32<KPART + 512>(vo);
+                    if constexpr (VB > 3) pw[3] = lds_u32<KPART + 768>(vo);
+                    if constexpr (VB == 2) {
+#pragma unroll
+                        for (int jw = 0; jw < 2; ++jw) {
+                            const uint2 a0 = table_quad<0>(pw[jw], vlut), b0 = table_quad<2>(pw[jw], vlut);
+                            mma_f16_16816(oacc[4 * jw], pa0, pa1, pa2, pa3, a0.x, b0.x);
+                            mma_f16_16816(oacc[4 * jw + 2], pa0, pa1, pa2, pa3, a0.y, b0.y);
+                            const uint2 a1 = table_quad<1>(pw[jw], vlut), b1 = table_quad<3>(pw[jw], vlut);
+                            mma_f16_16816(oacc[4 * jw + 1], pa0, pa1, pa2, pa3, a1.x, b1.x);
+                            mma_f16_16816(oacc[4 * jw + 3], pa0, pa1, pa2, pa3, a1.y, b1.y);
+                        }
+                    } else {
+                        uint32_t mv[4];
+                        table_words<VB>(pw, mv);   // bytes 0, 1: token a (dims 4u .. 4u + 3), bytes 2, 3: token b
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            const uint32_t a0 = table_pair<0>(mv[u], vlut), b0 = table_pair<2>(mv[u], vlut);
+                            mma_f16_16816(oacc[2 * u], pa0, pa1, pa2, pa3, a0, b0);
+                            const uint32_t a1 = table_pair<1>(mv[u], vlut), b1 = table_pair<3>(mv[u], vlut);
+                            mma_f16_16816(oacc[2 * u + 1], pa0, pa1, pa2, pa3, a1, b1);
+                        }
+                    }
+                }
+            }
+            // ---- refill this stage
+            __syncwarp();
+            const int i = idx + j + NSTAGE;
+            if (i < n) {
+                if ((i & 31) == 0) {
+                    src = src_next;
+                    if (i + 32 < n) src_next = next_window();
+                }
+                const bool whole = !SPARSE || do_v;
+                if (lane == (i & 31)) copy_in(ring + so, src, whole ? PAGE : KPART, bar + stage * 8);
+                if constexpr (SPARSE) v_with_k = whole ? (v_with_k | (1u << stage)) : (v_with_k & ~(1u << stage));
+            }
+            if (++stage == NSTAGE) {
+                stage = 0;
+                parity ^= 1u;
+            }
+        };
+        for (int j = 0; j < seg && !timed_out; ++j) {
+            if constexpr (SPARSE) {
+                if ((v_with_k >> stage) & 1u) one_page(std::true_type{}, j);
+                else one_page(std::false_type{}, j);
+            } else {
+                one_page(std::true_type{}, j);
+            }
+        }
+        if (timed_out) {   // let copies that are under way land before the CTA may end
+            for (int s = 0; s < NSTAGE; ++s) (void)wait_bounded(bar + s * 8, s < static_cast<int>(stage) ? parity ^ 1u : parity);
+            break;
+        }
+
+        // ---- the item's result, or this warp's part of it
+#pragma unroll
+        for (int o = 4; o < 32; o <<= 1) {
+            l0 += __shfl_xor_sync(0xffffffffu, l0, o);
+            l1 += __shfl_xor_sync(0xffffffffu, l1, o);
+        }
+        const float la = __shfl_sync(0xffffffffu, l0, gid >> 1), lb = __shfl_sync(0xffffffffu, l1, gid >> 1);
+        const float ma = __shfl_sync(0xffffffffu, m0, gid >> 1), mb = __shfl_sync(0xffffffffu, m1, gid >> 1);
+        const float lq = (gid & 1) ? lb : la, mq = (gid & 1) ? mb : ma;   // of query gid
+        float x[32];                                                      // dims 32 tig .. 32 tig + 31 of query gid
+#pragma unroll
+        for (int nt = 0; nt < 8; ++nt)
+#pragma unroll
+            for (int r = 0; r < 4; ++r) x[16 * (r & 1) + 2 * nt + (r >> 1)] = oacc[nt][r];
+        if (page == 0 && seg == np) {
+            const float inv = 1.f / lq;
+#pragma unroll
+            for (int i = 0; i < 32; ++i) x[i] *= inv;
+            if (p.derotate_out) {
+                fwht128(x, lane);
+#pragma unroll
+                for (int i = 0; i < 32; ++i) x[i] *= kWhtScale;
+            }
+            if (gid < nq) store_row32(p.out, row + 32 * tig, p.io_dtype, x);
+        } else {
+            const int slot = 2 * gw + (page == 0 ? 1 : 0);
+            float4* dst = reinterpret_cast<float4*>(sp.part_o + static_cast<int64_t>(slot) * kStreamSlotFloats + gid * kHeadDim + 32 * tig);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) dst[i] = make_float4(x[4 * i], x[4 * i + 1], x[4 * i + 2], x[4 * i + 3]);
+            if (tig == 0) sp.part_ml[slot * 8 + gid] = make_float2(mq, lq);
+        }
+        idx += seg;
+        page = 0;
+        if (idx < n && ++hg == sp.HG) {
+            hg = 0;
+            do {
+                len = __ldg(p.seq_lens + ++seq);
+                np = pages_of(p, len);
+            } while (np == 0);
+        }
+    }
+    if (p.status) {
+        int bits = 0;
+        if (__any_sync(0xffffffffu, bad_block)) bits |= TQ_STATUS_BAD_BLOCK;
+        if (__any_sync(0xffffffffu, timed_out)) bits |= TQ_STATUS_TIMEOUT;
+        if (bits && lane == 0) atomicOr(p.status, bits);
+    }
+    if constexpr (SPARSE) {
+        if (p.skip_stats && lane == 0) {
+            atomicAdd(p.skip_stats, static_cast<uint32_t>(idx));
+            atomicAdd(p.skip_stats + 1, v_skipped);
+        }
+    }
+}
+
+template <int KB, int VB, bool QJL, bool SPARSE>
+int launch_stream(const StreamParams& sp, cudaStream_t stream) {
+    auto kern = decode_stream_kernel<KB, VB, QJL, SPARSE>;
+    static bool configured[64] = {};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return TQ_ERR_LAUNCH;
+    if (!configured[dev]) {
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kStreamSmem) != cudaSuccess) return TQ_ERR_LAUNCH;
+        configured[dev] = true;
+    }
+    return launch_chained(kern, dim3(sp.n_warps / kStreamWarps), dim3(kStreamThreads), kStreamSmem, stream, sp) == cudaSuccess ? TQ_OK : TQ_ERR_LAUNCH;
+}
+
+// One warp per query head: combines the parts of an item that more than one warp worked on.
+constexpr int kMergeWarps = 4;
+__global__ void __launch_bounds__(kMergeWarps * 32) decode_stream_merge_kernel(const StreamParams sp) {
+    pdl_release_and_wait();
+    const DecodeParams& p = sp.d;
+    const int64_t id = static_cast<int64_t>(blockIdx.x) * kMergeWarps + (threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31;
+    if (id >= static_cast<int64_t>(sp.ns) * p.Hq) return;
+    const int seq = static_cast<int>(id / p.Hq), head = static_cast<int>(id - static_cast<int64_t>(seq) * p.Hq);
+    const int kvh = head / p.G, gi = head - kvh * p.G, g = gi & 7;
+    const int s0 = sp.prefix[seq], np = sp.prefix[seq + 1] - s0;
+    if (np == 0) return;   // zeros, already written
+    const int64_t total = static_cast<int64_t>(sp.prefix[sp.ns]) * sp.HG;
+    const int64_t a = static_cast<int64_t>(s0) * sp.HG + static_cast<int64_t>(kvh * p.ngroups + (gi >> 3)) * np;
+    // the warp whose share holds page u is the largest w with floor(w * total / W) <= u
+    const int W = active_warps(sp, total);
+    const int w0 = static_cast<int>(((a + 1) * W - 1) / total), w1 = static_cast<int>(((a + np) * W - 1) / total);
+    if (w0 == w1) return;  // written by that warp
+    float M = -INFINITY;
+    for (int w = w0; w <= w1; ++w) M = fmaxf(M, sp.part_ml[(2 * w + (w == w0)) * 8 + g].x);
+    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+    float l = 0.f;
+    for (int w = w0; w <= w1; ++w) {
+        const int slot = 2 * w + (w == w0);
+        const float2 ml = sp.part_ml[slot * 8 + g];
+        const float sc = ex2(ml.x - M);
+        const float4 v = *reinterpret_cast<const float4*>(sp.part_o + static_cast<int64_t>(slot) * kStreamSlotFloats + g * kHeadDim + 4 * lane);
+        o.x = fmaf(sc, v.x, o.x);
+        o.y = fmaf(sc, v.y, o.y);
+        o.z = fmaf(sc, v.z, o.z);
+        o.w = fmaf(sc, v.w, o.w);
+        l = fmaf(sc, ml.y, l);
+    }
+    float x[4] = {o.x / l, o.y / l, o.z / l, o.w / l};
+    if (p.derotate_out) {   // dims 4 lane .. 4 lane + 3: two stages in the lane, five across lanes
+        const float b0 = x[0] + x[1], b1 = x[0] - x[1], b2 = x[2] + x[3], b3 = x[2] - x[3];
+        x[0] = b0 + b2; x[1] = b1 + b3; x[2] = b0 - b2; x[3] = b1 - b3;
+#pragma unroll
+        for (int m = 1; m < 32; m <<= 1) {
+            const float sgn = (lane & m) ? -1.f : 1.f;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) x[i] = fmaf(sgn, x[i], __shfl_xor_sync(0xffffffffu, x[i], m));
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) x[i] *= kWhtScale;
+    }
+    uint2 w;
+    if (p.io_dtype == TQ_DTYPE_F16) {
+        w = make_uint2(pack_half2(x[0], x[1]), pack_half2(x[2], x[3]));
+    } else {
+        const __nv_bfloat162 lo = __floats2bfloat162_rn(x[0], x[1]), hi = __floats2bfloat162_rn(x[2], x[3]);
+        w = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+    }
+    *reinterpret_cast<uint2*>(static_cast<uint16_t*>(p.out) + id * kHeadDim + 4 * lane) = w;
+}
+
+}  // namespace
+}  // namespace tq

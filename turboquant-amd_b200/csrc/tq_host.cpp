@@ -29,8 +29,8 @@ namespace {
 struct Library {
     decltype(&tq_page_bytes) page_bytes;
     decltype(&tq_compress_paged) compress_paged;
-    decltype(&tq_decode_auto_chunk_pages) auto_chunk_pages;
     decltype(&tq_decode_workspace_bytes) decode_workspace_bytes;
+    decltype(&tq_decode_auto_workspace_bytes) decode_auto_workspace_bytes;
     decltype(&tq_decode_paged) decode_paged;
     decltype(&tq_wht_rows) wht_rows;
     decltype(&tq_compress_k) compress_k;
@@ -145,7 +145,7 @@ PyObject* decode(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
         return declined();
     const at::Tensor &cache = *t[1], &tables = *t[2], &lens = *t[3], &kc = *t[4], &vc = *t[5];
     const long long block_size = v[0], kb = v[1], vb = v[2], qjl = v[3] != 0, flags = v[5], max_len = v[6];
-    long long chunk = v[4];
+    const long long chunk = std::max(v[4], 0ll);
     const int dev = cache.get_device();
     if (dev >= kMaxDevices || !g_status[dev]) return declined();
     if (t[0]->dim() != 3 || t[0]->size(2) != 128 || t[0]->size(0) == 0) return declined();
@@ -192,16 +192,12 @@ PyObject* decode(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
         out = empty(q.sizes(), q.scalar_type(), device);
         out_ptr = out.data_ptr();
     }
-    if (chunk <= 0) chunk = L.auto_chunk_pages(int(ns), int(hkv), int(hq), int(pages));
     // Split-K partials: a block of the caching allocator, held for this call only.  Its reuse is ordered by the
     // stream, so calls on other streams and threads never share it.
-    at::DataPtr workspace;
-    int64_t bytes = 0;
-    if (pages > chunk) {
-        bytes = L.decode_workspace_bytes(int(ns), int(hq), int(hkv), int(pages), int(chunk));
-        if (bytes < 0) return failed("tq_decode_paged", int(bytes));
-        workspace = c10::cuda::CUDACachingAllocator::get()->allocate(bytes);
-    }
+    const int64_t bytes = chunk > 0 ? L.decode_workspace_bytes(int(ns), int(hq), int(hkv), int(pages), int(chunk))
+                                    : L.decode_auto_workspace_bytes(int(ns), int(hq), int(hkv), int(pages));
+    if (bytes < 0) return failed("tq_decode_paged", int(bytes));
+    at::DataPtr workspace = c10::cuda::CUDACachingAllocator::get()->allocate(bytes);
     const tq_stream_t stream = stream_of(device);
     const int rc = launch([&] {
         return L.decode_paged(out_ptr, q.data_ptr(), proj, dtype | int(flags), cache.data_ptr(), cache.size(0), int(block_size),
@@ -426,8 +422,8 @@ PyObject* bind(PyObject*, PyObject* args) {
     };
     take(L.page_bytes, "tq_page_bytes");
     take(L.compress_paged, "tq_compress_paged");
-    take(L.auto_chunk_pages, "tq_decode_auto_chunk_pages");
     take(L.decode_workspace_bytes, "tq_decode_workspace_bytes");
+    take(L.decode_auto_workspace_bytes, "tq_decode_auto_workspace_bytes");
     take(L.decode_paged, "tq_decode_paged");
     take(L.wht_rows, "tq_wht_rows");
     take(L.compress_k, "tq_compress_k");

@@ -63,6 +63,8 @@ def lib() -> ctypes.CDLL:
     L.tq_decode_auto_chunk_pages.argtypes = [i32, i32, i32, i32]
     L.tq_decode_workspace_bytes.argtypes = [i32, i32, i32, i32, i32]
     L.tq_decode_workspace_bytes.restype = i64
+    L.tq_decode_auto_workspace_bytes.argtypes = [i32, i32, i32, i32]
+    L.tq_decode_auto_workspace_bytes.restype = i64
     L.tq_decode_paged.argtypes = [vp, vp, vp, i32, vp, i64, i32, vp, i64, vp, vp, vp, f32, f32, f32, vp, i64,
                                   vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, vp]
     L.tq_decode_paged_static.argtypes = [vp, vp, vp, i32, vp, i64, i32, vp, i64, vp, vp, vp, f32, f32, f32,
@@ -272,8 +274,7 @@ def _decode_paged_impl(out, q_rot, q_proj, cache, block_tables, seq_lens, kc, vc
     if max_seq_len > 0:
         max_pages = max(1, min(max_pages, (int(max_seq_len) + 15) // 16))
     L = lib()
-    if chunk_pages <= 0:
-        chunk_pages = L.tq_decode_auto_chunk_pages(ns, Hkv, Hq, max_pages)
+    chunk_pages = max(int(chunk_pages), 0)          # 0: the library picks the kernel and the split
     common_tail = (_ptr(status_word(dev)), _ptr(skip_stats), ns, Hq, Hkv, max_pages, k_bits, v_bits, int(use_qjl),
                    chunk_pages, _stream(dev))
     head = (_ptr(out), _ptr(q_rot), _ptr(q_proj), _DTYPES[q_rot.dtype] | int(io_flags), _ptr(cache), nb, block_size,
@@ -283,7 +284,8 @@ def _decode_paged_impl(out, q_rot, q_proj, cache, block_tables, seq_lens, kc, vc
         if static_scratch:
             rc = L.tq_decode_paged_static(*head, *common_tail)
         else:
-            need = L.tq_decode_workspace_bytes(ns, Hq, Hkv, max_pages, chunk_pages)
+            need = (L.tq_decode_workspace_bytes(ns, Hq, Hkv, max_pages, chunk_pages) if chunk_pages
+                    else L.tq_decode_auto_workspace_bytes(ns, Hq, Hkv, max_pages))
             ws = workspace(dev, need)
             rc = L.tq_decode_paged(*head, _ptr(ws), ws.numel(), *common_tail)
     _check(rc, "tq_decode_paged_static" if static_scratch else "tq_decode_paged")
