@@ -72,6 +72,12 @@ __device__ __forceinline__ void table_words(const uint32_t* w, uint32_t (&mw)[4]
     }
 }
 
+// A V word holds the nibbles e = 0 .. 3 of token a in its low and of token b in its high half.  Bytes 2 and 3 become
+// (b_0, a_0), (b_2, a_2) or (a_1, b_1), (a_3, b_3), low nibble first: a table entry is then one dim of two tokens, which
+// is what the tensor core wants of V^T as its A operand (dims on M, tokens on K), with all 16 rows in use.
+__device__ __forceinline__ uint32_t even_pairs(uint32_t w) { return bit_select(w << 20, w, 0x0f0f0000u); }
+__device__ __forceinline__ uint32_t odd_pairs(uint32_t w) { return bit_select(w << 12, w, 0xf0f00000u); }
+
 template <int BITS>
 __device__ __forceinline__ void fill_stream_table(uint32_t smem_addr, const float* __restrict__ c, int warp, int lane) {
     const float cv = __half2float(__float2half_rn(__ldg(c + (lane & ((1 << BITS) - 1)))));
@@ -111,11 +117,11 @@ __device__ __forceinline__ void copy_in(uint32_t dst, const uint8_t* src, uint32
                  : "memory");
 }
 
-// 32 values (the lane's quarter of a row of 128) to fp16 / bf16.
-__device__ __forceinline__ void store_row32(void* out, int64_t off, int io_dtype, const float (&x)[32]) {
+// 16 consecutive values of a row to fp16 / bf16.
+__device__ __forceinline__ void store_row16(void* out, int64_t off, int io_dtype, const float (&x)[16]) {
     uint4* dst = reinterpret_cast<uint4*>(static_cast<uint16_t*>(out) + off);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < 2; ++i) {
         uint32_t w[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -129,6 +135,29 @@ __device__ __forceinline__ void store_row32(void* out, int64_t off, int io_dtype
         }
         dst[i] = make_uint4(w[0], w[1], w[2], w[3]);
     }
+}
+
+// x H for a row of which this lane holds dims 16 gid .. 16 gid + 15 (gid = lane >> 2): four stages in the lane, three across.
+__device__ __forceinline__ void wht_16x8(float (&x)[16], int lane) {
+#pragma unroll
+    for (int h = 1; h < 16; h <<= 1) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            if (!(i & h)) {
+                const float a = x[i], b = x[i + h];
+                x[i] = a + b;
+                x[i + h] = a - b;
+            }
+        }
+    }
+#pragma unroll
+    for (int m = 4; m < 32; m <<= 1) {
+        const float sgn = (lane & m) ? -1.f : 1.f;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) x[i] = fmaf(sgn, x[i], __shfl_xor_sync(0xffffffffu, x[i], m));
+    }
+#pragma unroll
+    for (int i = 0; i < 16; ++i) x[i] *= kWhtScale;
 }
 
 template <int KB, int VB, bool QJL, bool SPARSE>
@@ -205,8 +234,10 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
     __syncthreads();
 
     const int64_t total = static_cast<int64_t>(sm_scan[kStreamThreads]) * sp.HG;
-    const int gw = warp * gridDim.x + blockIdx.x;       // neighbouring shares on different SMs: few shares use all SMs
     const int W = active_warps(sp, total);
+    // With work for every warp, the 16 shares of a CTA are neighbours (same query rows and table lines; measured 3 %
+    // faster than neighbours on different SMs); fewer shares are dealt out over the SMs.
+    const int gw = W == sp.n_warps ? blockIdx.x * kStreamWarps + warp : warp * static_cast<int>(gridDim.x) + static_cast<int>(blockIdx.x);
     if (gw >= W) return;
     const int64_t first = total * gw / W;
     const int n = static_cast<int>(total * (gw + 1) / W - first);   // this warp's pages, at least one
@@ -395,14 +426,13 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
                 const float al0 = ex2(m0 - mn0), al1 = ex2(m1 - mn1);
                 l0 *= al0;
                 l1 *= al1;
-                // accumulator rows belong to query gid: its factor comes from the lane that scored it
-                const float t0 = __shfl_sync(0xffffffffu, al0, gid >> 1);
-                const float t1 = __shfl_sync(0xffffffffu, al1, gid >> 1);
-                const float ag = (gid & 1) ? t1 : t0;
 #pragma unroll
-                for (int i = 0; i < 8; ++i)
-#pragma unroll
-                    for (int r = 0; r < 4; ++r) oacc[i][r] *= ag;
+                for (int i = 0; i < 8; ++i) {
+                    oacc[i][0] *= al0;
+                    oacc[i][1] *= al1;
+                    oacc[i][2] *= al0;
+                    oacc[i][3] *= al1;
+                }
                 m0 = mn0;
                 m1 = mn1;
             }
@@ -435,35 +465,55 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
                     if (gid >= valid_tokens) vn.x = 0.f;
                     if (gid + 8 >= valid_tokens) vn.y = 0.f;
                 }
-                const uint32_t t[2] = {movmatrix_trans(pack_half2(p0v * vn.x, p1v * vn.x)), movmatrix_trans(pack_half2(p2v * vn.y, p3v * vn.y))};
+                // B operand: weights of query gid, tokens 2 tig, 2 tig + 1 (then + 8); `back` has the two swapped
+                const uint32_t t0 = movmatrix_trans(pack_half2(p0v * vn.x, p1v * vn.x)), t1 = movmatrix_trans(pack_half2(p2v * vn.y, p3v * vn.y));
+                const uint32_t back0 = prmt(t0, 0u, 0x1032u), back1 = prmt(t1, 0u, 0x1032u);
+                uint32_t va[VB], vb[VB];   // token pairs tig and tig + 4, dim group gid
+                va[0] = lds_u32<KPART>(ring_v + so);
+                vb[0] = lds_u32<KPART + 128>(ring_v + so);
+                va[1] = lds_u32<KPART + 256>(ring_v + so);
+                vb[1] = lds_u32<KPART + 384>(ring_v + so);
+                if constexpr (VB > 2) {
+                    va[2] = lds_u32<KPART + 512>(ring_v + so);
+                    vb[2] = lds_u32<KPART + 640>(ring_v + so);
+                }
+                if constexpr (VB > 3) {
+                    va[3] = lds_u32<KPART + 768>(ring_v + so);
+                    vb[3] = lds_u32<KPART + 896>(ring_v + so);
+                }
+                if constexpr (VB == 2) {
 #pragma unroll
-                for (int o = 0; o < 2; ++o) {
-                    const uint32_t vo = ring_v + so + o * 128;
-                    const uint32_t pa0 = t[o] & 0xffffu, pa1 = t[o] << 16, pa2 = t[o] >> 16, pa3 = t[o] & 0xffff0000u;
-                    uint32_t pw[VB];
-                    pw[0] = lds_u32<KPART>(vo);
-                    pw[1] = lds_u32<KPART + 256>(vo);
-                    if constexpr (VB > 2) pw[2] = lds_u32<KPART + 512>(vo);
-                    if constexpr (VB > 3) pw[3] = lds_u32<KPART + 768>(vo);
-                    if constexpr (VB == 2) {
-#pragma unroll
-                        for (int jw = 0; jw < 2; ++jw) {
-                            const uint2 a0 = table_quad<0>(pw[jw], vlut), b0 = table_quad<2>(pw[jw], vlut);
-                            mma_f16_16816(oacc[4 * jw], pa0, pa1, pa2, pa3, a0.x, b0.x);
-                            mma_f16_16816(oacc[4 * jw + 2], pa0, pa1, pa2, pa3, a0.y, b0.y);
-                            const uint2 a1 = table_quad<1>(pw[jw], vlut), b1 = table_quad<3>(pw[jw], vlut);
-                            mma_f16_16816(oacc[4 * jw + 1], pa0, pa1, pa2, pa3, a1.x, b1.x);
-                            mma_f16_16816(oacc[4 * jw + 3], pa0, pa1, pa2, pa3, a1.y, b1.y);
+                    for (int j = 0; j < 2; ++j) {
+                        {
+                            const uint32_t ya = even_pairs(va[j]), yb = even_pairs(vb[j]);
+                            const uint2 a0 = table_quad<2>(ya, vlut), a1 = table_quad<3>(ya, vlut);
+                            const uint2 a2 = table_quad<2>(yb, vlut), a3 = table_quad<3>(yb, vlut);
+                            mma_f16_16816(oacc[4 * j], a0.x, a1.x, a2.x, a3.x, back0, back1);
+                            mma_f16_16816(oacc[4 * j + 2], a0.y, a1.y, a2.y, a3.y, back0, back1);
                         }
-                    } else {
-                        uint32_t mv[4];
-                        table_words<VB>(pw, mv);   // bytes 0, 1: token a (dims 4u .. 4u + 3), bytes 2, 3: token b
+                        {
+                            const uint32_t ya = odd_pairs(va[j]), yb = odd_pairs(vb[j]);
+                            const uint2 a0 = table_quad<2>(ya, vlut), a1 = table_quad<3>(ya, vlut);
+                            const uint2 a2 = table_quad<2>(yb, vlut), a3 = table_quad<3>(yb, vlut);
+                            mma_f16_16816(oacc[4 * j + 1], a0.x, a1.x, a2.x, a3.x, t0, t1);
+                            mma_f16_16816(oacc[4 * j + 3], a0.y, a1.y, a2.y, a3.y, t0, t1);
+                        }
+                    }
+                } else {
+                    uint32_t ma[4], mb[4];
+                    table_words<VB>(va, ma);
+                    table_words<VB>(vb, mb);
 #pragma unroll
-                        for (int u = 0; u < 4; ++u) {
-                            const uint32_t a0 = table_pair<0>(mv[u], vlut), b0 = table_pair<2>(mv[u], vlut);
-                            mma_f16_16816(oacc[2 * u], pa0, pa1, pa2, pa3, a0, b0);
-                            const uint32_t a1 = table_pair<1>(mv[u], vlut), b1 = table_pair<3>(mv[u], vlut);
-                            mma_f16_16816(oacc[2 * u + 1], pa0, pa1, pa2, pa3, a1, b1);
+                    for (int u = 0; u < 4; ++u) {
+                        {
+                            const uint32_t ya = even_pairs(ma[u]), yb = even_pairs(mb[u]);
+                            mma_f16_16816(oacc[2 * u], table_pair<2>(ya, vlut), table_pair<3>(ya, vlut), table_pair<2>(yb, vlut),
+                                          table_pair<3>(yb, vlut), back0, back1);
+                        }
+                        {
+                            const uint32_t ya = odd_pairs(ma[u]), yb = odd_pairs(mb[u]);
+                            mma_f16_16816(oacc[2 * u + 1], table_pair<2>(ya, vlut), table_pair<3>(ya, vlut), table_pair<2>(yb, vlut),
+                                          table_pair<3>(yb, vlut), t0, t1);
                         }
                     }
                 }
@@ -504,30 +554,29 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
             l0 += __shfl_xor_sync(0xffffffffu, l0, o);
             l1 += __shfl_xor_sync(0xffffffffu, l1, o);
         }
-        const float la = __shfl_sync(0xffffffffu, l0, gid >> 1), lb = __shfl_sync(0xffffffffu, l1, gid >> 1);
-        const float ma = __shfl_sync(0xffffffffu, m0, gid >> 1), mb = __shfl_sync(0xffffffffu, m1, gid >> 1);
-        const float lq = (gid & 1) ? lb : la, mq = (gid & 1) ? mb : ma;   // of query gid
-        float x[32];                                                      // dims 32 tig .. 32 tig + 31 of query gid
+        // accumulator 2 u + s, register r: dim 16 gid + 4 u + s + 2 (r >> 1) of query 2 tig + (r & 1)
 #pragma unroll
-        for (int nt = 0; nt < 8; ++nt)
+        for (int k = 0; k < 2; ++k) {
+            const int g = 2 * tig + k;
+            const float l = k ? l1 : l0;
+            float x[16];
 #pragma unroll
-            for (int r = 0; r < 4; ++r) x[16 * (r & 1) + 2 * nt + (r >> 1)] = oacc[nt][r];
-        if (page == 0 && seg == np) {
-            const float inv = 1.f / lq;
+            for (int u = 0; u < 4; ++u)
 #pragma unroll
-            for (int i = 0; i < 32; ++i) x[i] *= inv;
-            if (p.derotate_out) {
-                fwht128(x, lane);
+                for (int e = 0; e < 4; ++e) x[4 * u + e] = oacc[2 * u + (e & 1)][(e & 2) + k];
+            if (page == 0 && seg == np) {
+                const float inv = 1.f / l;
 #pragma unroll
-                for (int i = 0; i < 32; ++i) x[i] *= kWhtScale;
+                for (int i = 0; i < 16; ++i) x[i] *= inv;
+                if (p.derotate_out) wht_16x8(x, lane);
+                if (g < nq) store_row16(p.out, (static_cast<int64_t>(seq) * p.Hq + head0 + g) * kHeadDim + 16 * gid, p.io_dtype, x);
+            } else {
+                const int slot = 2 * gw + (page == 0 ? 1 : 0);
+                float4* dst = reinterpret_cast<float4*>(sp.part_o + static_cast<int64_t>(slot) * kStreamSlotFloats + g * kHeadDim + 16 * gid);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) dst[i] = make_float4(x[4 * i], x[4 * i + 1], x[4 * i + 2], x[4 * i + 3]);
+                if (gid == 0) sp.part_ml[slot * 8 + g] = make_float2(k ? m1 : m0, l);
             }
-            if (gid < nq) store_row32(p.out, row + 32 * tig, p.io_dtype, x);
-        } else {
-            const int slot = 2 * gw + (page == 0 ? 1 : 0);
-            float4* dst = reinterpret_cast<float4*>(sp.part_o + static_cast<int64_t>(slot) * kStreamSlotFloats + gid * kHeadDim + 32 * tig);
-#pragma unroll
-            for (int i = 0; i < 8; ++i) dst[i] = make_float4(x[4 * i], x[4 * i + 1], x[4 * i + 2], x[4 * i + 3]);
-            if (tig == 0) sp.part_ml[slot * 8 + gid] = make_float2(mq, lq);
         }
         idx += seg;
         page = 0;
