@@ -838,6 +838,8 @@ extern "C" int tq_decode_paged(void* out, const void* q_rot, const void* q_proj,
         sp.d = p;
         sp.ns = num_seqs;
         sp.HG = num_kv_heads * p.ngroups;
+        sp.two12 = 1u << 12;
+        sp.two20 = 1u << 20;
         sp.n_warps = kStreamCtas * kStreamWarps;
         sp.part_o = static_cast<float*>(workspace);
         sp.part_ml = reinterpret_cast<float2*>(sp.part_o + 2ll * sp.n_warps * kStreamSlotFloats);

@@ -26,6 +26,7 @@ struct StreamParams {
     float* part_o;       // [2 n_warps][8][128]: slot 2 w + 1 starts at its item's first page, slot 2 w does not
     float2* part_ml;     // [2 n_warps][8] (maximum, denominator)
     int32_t* prefix;     // [ns + 1] pages of all sequences before s
+    uint32_t two12, two20;
 };
 
 // Warps that share `total` pages: all of them, but none with fewer than kStreamMinShare pages.
@@ -56,7 +57,23 @@ __device__ __forceinline__ uint2 table_quad(uint32_t w, uint32_t base) {
     return v;
 }
 
-__device__ __forceinline__ uint32_t bit_select(uint32_t a, uint32_t b, uint32_t mask) { return (a & ~mask) | (b & mask); }
+// mask ? b : a, bit by bit; and a and-or.  As PTX, so that the shift that makes an operand is not moved behind a mask of
+// its own (the compiler then spends two logic instructions on each of these).
+__device__ __forceinline__ uint32_t bit_select(uint32_t a, uint32_t b, uint32_t mask) {
+    uint32_t r;
+    asm("lop3.b32 %0, %1, %2, %3, 0xd8;" : "=r"(r) : "r"(a), "r"(b), "r"(mask));
+    return r;
+}
+__device__ __forceinline__ uint32_t and_or(uint32_t a, uint32_t mask, uint32_t bits) {
+    uint32_t r;
+    asm("lop3.b32 %0, %1, %2, %3, 0xea;" : "=r"(r) : "r"(a), "r"(mask), "r"(bits));
+    return r;
+}
+__device__ __forceinline__ uint32_t and_bits(uint32_t a, uint32_t mask) {
+    uint32_t r;
+    asm("and.b32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(mask));
+    return r;
+}
 
 // Words whose bytes address the table.  The table does not look at the spare top bit of a 3-bit nibble.
 template <int BITS>
@@ -75,8 +92,9 @@ __device__ __forceinline__ void table_words(const uint32_t* w, uint32_t (&mw)[4]
 // A V word holds the nibbles e = 0 .. 3 of token a in its low and of token b in its high half.  Bytes 2 and 3 become
 // (b_0, a_0), (b_2, a_2) or (a_1, b_1), (a_3, b_3), low nibble first: a table entry is then one dim of two tokens, which
 // is what the tensor core wants of V^T as its A operand (dims on M, tokens on K), with all 16 rows in use.
-__device__ __forceinline__ uint32_t even_pairs(uint32_t w) { return bit_select(w << 20, w, 0x0f0f0000u); }
-__device__ __forceinline__ uint32_t odd_pairs(uint32_t w) { return bit_select(w << 12, w, 0xf0f00000u); }
+// The shifts are multiplications by kernel parameters: they run on the multiply-add pipe, the logic pipe is the busy one.
+__device__ __forceinline__ uint32_t even_pairs(uint32_t w, uint32_t two20) { return bit_select(w * two20, w, 0x0f0f0000u); }
+__device__ __forceinline__ uint32_t odd_pairs(uint32_t w, uint32_t two12) { return bit_select(w * two12, w, 0xf0f00000u); }
 
 template <int BITS>
 __device__ __forceinline__ void fill_stream_table(uint32_t smem_addr, const float* __restrict__ c, int warp, int lane) {
@@ -160,7 +178,24 @@ __device__ __forceinline__ void wht_16x8(float (&x)[16], int lane) {
     for (int i = 0; i < 16; ++i) x[i] *= kWhtScale;
 }
 
-template <int KB, int VB, bool QJL, bool SPARSE>
+// Sign table: entry b holds the eight values +-1 of byte b as four half2, in the order of eight consecutive dims, 8 copies.
+__device__ __forceinline__ void fill_sign_table(uint32_t smem_addr, int warp, int lane) {
+    for (int b = warp; b < 256; b += kStreamWarps) {
+        const int pair = b >> (2 * (lane & 3));
+        const uint32_t v = 0xBC00BC00u ^ ((pair & 1) ? 0x8000u : 0u) ^ ((pair & 2) ? 0x80000000u : 0u);
+        asm volatile("st.shared.u32 [%0], %1;" ::"r"(smem_addr + b * 256 + lane * 4), "r"(v) : "memory");
+    }
+}
+template <int K>
+__device__ __forceinline__ uint4 table_signs(uint32_t w, uint32_t base) {
+    uint4 v;
+    asm("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(prmt(w, base, 0x7604u | (K << 4))));
+    return v;
+}
+
+// SIGN_TABLE: K and V share a codebook and S = I, so the V half of the table has room for the signs, and the query
+// operands of the index term serve the sign term as well.
+template <int KB, int VB, bool QJL, bool SPARSE, bool SIGN_TABLE>
 __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const StreamParams sp) {
     constexpr int NWK = KB + (QJL ? 1 : 0);
     constexpr int RK = 16 * NWK;
@@ -211,7 +246,8 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
     }
     if (lane == 31) sm_wsum[warp] = incl;
     fill_stream_table<KB>(tab, p.kc, warp, lane);
-    fill_stream_table<VB>(tab + 128, p.vc, warp, lane);
+    if constexpr (SIGN_TABLE) fill_sign_table(tab + 128, warp, lane);
+    else fill_stream_table<VB>(tab + 128, p.vc, warp, lane);
     __syncthreads();
     int before = incl - own;
     for (int w = 0; w < warp; ++w) before += sm_wsum[w];
@@ -302,11 +338,13 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
     if (n > 32) src_next = next_window();
 
     const uint32_t klut = tab + (KB == 2 ? 8 * (lane & 15) : 4 * lane);
-    const uint32_t vlut = tab + 128 + (VB == 2 ? 8 * (lane & 15) : 4 * lane);
+    const uint32_t vlut = tab + (SIGN_TABLE ? 0 : 128) + (VB == 2 ? 8 * (lane & 15) : 4 * lane);
+    const uint32_t slut = tab + 128 + 16 * (lane & 7);
     const uint32_t ring_k = ring + lane * (NWK * 4);
     const uint32_t ring_n = ring + gid * 4;
     const uint32_t ring_v = ring + (tig * 8 + gid) * 4;
 
+    const float qpscale = SIGN_TABLE ? p.qpscale * (1.f / 16.f) : p.qpscale;   // the one-sided forms carry 1/16 in the query
     bool timed_out = false;
     uint32_t stage = 0, parity = 0;           // ring stage of the current page and the phase of its barrier
     uint32_t v_parity = 0;                    // Sparse-V: bit s = phase of the late-V barrier of stage s
@@ -320,14 +358,14 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
         const int head0 = kvh * p.G + qg * 8, nq = min(8, p.G - qg * 8);
         const int64_t row = (static_cast<int64_t>(seq) * p.Hq + head0 + gid) * kHeadDim;
 
-        uint32_t qf[16], qpf[QJL ? 16 : 1];
+        uint32_t qf[16], qpf[QJL && !SIGN_TABLE ? 16 : 1];
         float sq_init0 = 0.f, sq_init1 = 0.f;   // minus the query sums of the one-sided sign forms
         {
             float xq[32];
             load_q32(p.q, row, tig, p.io_dtype, gid < nq, xq);
             if (p.rotate_q) rotate_q32(xq, lane, p.io_dtype);
             q_frag_from(xq, qf);
-            if constexpr (QJL) {
+            if constexpr (QJL && !SIGN_TABLE) {
                 if (p.qp) load_q32(p.qp, row, tig, p.io_dtype, gid < nq, xq);
                 float corr;
                 qp_frag_signed_from(xq, qpf, corr);
@@ -345,8 +383,8 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
 #pragma unroll
             for (int r = 0; r < 4; ++r) oacc[i][r] = 0.f;
 
-        auto one_page = [&](auto have_v, int j) {
-            constexpr bool HAVE_V = decltype(have_v)::value;
+        auto one_page = [&](auto have_v, auto at_end, int j) {
+            constexpr bool HAVE_V = decltype(have_v)::value, AT_END = decltype(at_end)::value;
             const uint32_t so = stage * PAGE;
             if (!wait_bounded(bar + stage * 8, parity)) {
                 timed_out = true;
@@ -357,58 +395,72 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
             lds_words<NWK, 0>(ring_k + so, wa);
             lds_words<NWK, 32 * NWK * 4>(ring_k + so, wb);
             float sm[4] = {0.f, 0.f, 0.f, 0.f};
+            float smb[4] = {0.f, 0.f, 0.f, 0.f};   // two chains of products for each of the two terms
             float sq[4] = {sq_init0, sq_init1, sq_init0, sq_init1}, sq2[4] = {0.f, 0.f, 0.f, 0.f};
-            if constexpr (KB == 2) {
-#pragma unroll
-                for (int jw = 0; jw < 2; ++jw) {
-                    const uint2 a0 = table_quad<0>(wa[jw], klut), a1 = table_quad<1>(wa[jw], klut);
-                    const uint2 b0 = table_quad<0>(wb[jw], klut), b1 = table_quad<1>(wb[jw], klut);
-                    mma_f16_16816(sm, a0.x, b0.x, a1.x, b1.x, qf[8 * jw], qf[8 * jw + 1]);
-                    mma_f16_16816(sm, a0.y, b0.y, a1.y, b1.y, qf[8 * jw + 4], qf[8 * jw + 5]);
-                    const uint2 c0 = table_quad<2>(wa[jw], klut), c1 = table_quad<3>(wa[jw], klut);
-                    const uint2 d0 = table_quad<2>(wb[jw], klut), d1 = table_quad<3>(wb[jw], klut);
-                    mma_f16_16816(sm, c0.x, d0.x, c1.x, d1.x, qf[8 * jw + 2], qf[8 * jw + 3]);
-                    mma_f16_16816(sm, c0.y, d0.y, c1.y, d1.y, qf[8 * jw + 6], qf[8 * jw + 7]);
+            auto sign_term = [&](auto quarter) {   // eight dims of two tokens, two products
+                constexpr int B = decltype(quarter)::value;
+                if constexpr (QJL && SIGN_TABLE) {
+                    const uint4 ga = table_signs<B>(wa[KB], slut), gb = table_signs<B>(wb[KB], slut);
+                    mma_f16_16816(sq, ga.x, gb.x, ga.y, gb.y, qf[4 * B], qf[4 * B + 1]);
+                    mma_f16_16816(sq2, ga.z, gb.z, ga.w, gb.w, qf[4 * B + 2], qf[4 * B + 3]);
+                } else if constexpr (QJL) {
+                    const uint32_t xa = wa[KB] << (4 * B), xb = wb[KB] << (4 * B);
+                    mma_f16_16816(sq, and_or(xa, 0x80008000u, 0x3C003C00u), and_or(xb, 0x80008000u, 0x3C003C00u),
+                                  and_bits(xa, 0x40004000u), and_bits(xb, 0x40004000u), qpf[4 * B], qpf[4 * B + 1]);
+                    mma_f16_16816(sq2, and_bits(xa, 0x20002000u), and_bits(xb, 0x20002000u), and_bits(xa, 0x10001000u),
+                                  and_bits(xb, 0x10001000u), qpf[4 * B + 2], qpf[4 * B + 3]);
                 }
+            };
+            if constexpr (KB == 2) {
+                auto quads = [&](auto word) {
+                    constexpr int J = decltype(word)::value;
+                    const uint2 a0 = table_quad<0>(wa[J], klut), a1 = table_quad<1>(wa[J], klut);
+                    const uint2 b0 = table_quad<0>(wb[J], klut), b1 = table_quad<1>(wb[J], klut);
+                    mma_f16_16816(sm, a0.x, b0.x, a1.x, b1.x, qf[8 * J], qf[8 * J + 1]);
+                    mma_f16_16816(smb, a0.y, b0.y, a1.y, b1.y, qf[8 * J + 4], qf[8 * J + 5]);
+                    sign_term(std::integral_constant<int, 2 * J>{});
+                    const uint2 c0 = table_quad<2>(wa[J], klut), c1 = table_quad<3>(wa[J], klut);
+                    const uint2 d0 = table_quad<2>(wb[J], klut), d1 = table_quad<3>(wb[J], klut);
+                    mma_f16_16816(sm, c0.x, d0.x, c1.x, d1.x, qf[8 * J + 2], qf[8 * J + 3]);
+                    mma_f16_16816(smb, c0.y, d0.y, c1.y, d1.y, qf[8 * J + 6], qf[8 * J + 7]);
+                    sign_term(std::integral_constant<int, 2 * J + 1>{});
+                };
+                quads(std::integral_constant<int, 0>{});
+                quads(std::integral_constant<int, 1>{});
             } else {
                 uint32_t mwa[4], mwb[4];
                 table_words<KB>(wa, mwa);
                 table_words<KB>(wb, mwb);
-#pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    const uint32_t a0 = table_pair<0>(mwa[c], klut), a1 = table_pair<1>(mwa[c], klut);
-                    const uint32_t b0 = table_pair<0>(mwb[c], klut), b1 = table_pair<1>(mwb[c], klut);
-                    mma_f16_16816(sm, a0, b0, a1, b1, qf[4 * c], qf[4 * c + 1]);
-                    const uint32_t a2 = table_pair<2>(mwa[c], klut), a3 = table_pair<3>(mwa[c], klut);
-                    const uint32_t b2 = table_pair<2>(mwb[c], klut), b3 = table_pair<3>(mwb[c], klut);
-                    mma_f16_16816(sm, a2, b2, a3, b3, qf[4 * c + 2], qf[4 * c + 3]);
-                }
-            }
-            if constexpr (QJL) {
-#pragma unroll
-                for (int ki = 0; ki < 4; ++ki) {
-                    const uint32_t xa = wa[KB] << (4 * ki), xb = wb[KB] << (4 * ki);
-                    mma_f16_16816(sq, (xa & 0x80008000u) | 0x3C003C00u, (xb & 0x80008000u) | 0x3C003C00u,
-                                  xa & 0x40004000u, xb & 0x40004000u, qpf[4 * ki], qpf[4 * ki + 1]);
-                    mma_f16_16816(sq2, xa & 0x20002000u, xb & 0x20002000u, xa & 0x10001000u, xb & 0x10001000u,
-                                  qpf[4 * ki + 2], qpf[4 * ki + 3]);
-                }
+                auto eight_dims = [&](auto word) {
+                    constexpr int C = decltype(word)::value;
+                    const uint32_t a0 = table_pair<0>(mwa[C], klut), a1 = table_pair<1>(mwa[C], klut);
+                    const uint32_t b0 = table_pair<0>(mwb[C], klut), b1 = table_pair<1>(mwb[C], klut);
+                    mma_f16_16816(sm, a0, b0, a1, b1, qf[4 * C], qf[4 * C + 1]);
+                    const uint32_t a2 = table_pair<2>(mwa[C], klut), a3 = table_pair<3>(mwa[C], klut);
+                    const uint32_t b2 = table_pair<2>(mwb[C], klut), b3 = table_pair<3>(mwb[C], klut);
+                    mma_f16_16816(smb, a2, b2, a3, b3, qf[4 * C + 2], qf[4 * C + 3]);
+                    sign_term(word);
+                };
+                eight_dims(std::integral_constant<int, 0>{});
+                eight_dims(std::integral_constant<int, 1>{});
+                eight_dims(std::integral_constant<int, 2>{});
+                eight_dims(std::integral_constant<int, 3>{});
             }
             float2 kn = unpack_half2(lds_u32<KN_OFF>(ring_n + so));
             kn.x *= p.qscale;
             kn.y *= p.qscale;
-            float s0 = sm[0] * kn.x, s1 = sm[1] * kn.x, s2 = sm[2] * kn.y, s3 = sm[3] * kn.y;
+            float s0 = (sm[0] + smb[0]) * kn.x, s1 = (sm[1] + smb[1]) * kn.x, s2 = (sm[2] + smb[2]) * kn.y, s3 = (sm[3] + smb[3]) * kn.y;
             if constexpr (QJL) {
                 float2 krn = unpack_half2(lds_u32<KRN_OFF>(ring_n + so));
-                krn.x *= p.qpscale;
-                krn.y *= p.qpscale;
+                krn.x *= qpscale;
+                krn.y *= qpscale;
                 s0 = fmaf(sq[0] + sq2[0], krn.x, s0);
                 s1 = fmaf(sq[1] + sq2[1], krn.x, s1);
                 s2 = fmaf(sq[2] + sq2[2], krn.y, s2);
                 s3 = fmaf(sq[3] + sq2[3], krn.y, s3);
             }
-            const int valid_tokens = len - (page + j) * kPageTokens;
-            if (valid_tokens < kPageTokens) {   // only the last page of a sequence is partly filled
+            const int valid_tokens = AT_END ? len - (page + j) * kPageTokens : kPageTokens;
+            if (AT_END && valid_tokens < kPageTokens) {   // only the last page of a sequence is partly filled
                 if (gid >= valid_tokens) { s0 = -INFINITY; s1 = -INFINITY; }
                 if (gid + 8 >= valid_tokens) { s2 = -INFINITY; s3 = -INFINITY; }
             }
@@ -461,7 +513,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
             }
             if (have) {
                 float2 vn = unpack_half2(lds_u32<VN_OFF>(ring_n + so));
-                if (valid_tokens < kPageTokens) {
+                if (AT_END && valid_tokens < kPageTokens) {
                     if (gid >= valid_tokens) vn.x = 0.f;
                     if (gid + 8 >= valid_tokens) vn.y = 0.f;
                 }
@@ -485,14 +537,14 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
 #pragma unroll
                     for (int j = 0; j < 2; ++j) {
                         {
-                            const uint32_t ya = even_pairs(va[j]), yb = even_pairs(vb[j]);
+                            const uint32_t ya = even_pairs(va[j], sp.two20), yb = even_pairs(vb[j], sp.two20);
                             const uint2 a0 = table_quad<2>(ya, vlut), a1 = table_quad<3>(ya, vlut);
                             const uint2 a2 = table_quad<2>(yb, vlut), a3 = table_quad<3>(yb, vlut);
                             mma_f16_16816(oacc[4 * j], a0.x, a1.x, a2.x, a3.x, back0, back1);
                             mma_f16_16816(oacc[4 * j + 2], a0.y, a1.y, a2.y, a3.y, back0, back1);
                         }
                         {
-                            const uint32_t ya = odd_pairs(va[j]), yb = odd_pairs(vb[j]);
+                            const uint32_t ya = odd_pairs(va[j], sp.two12), yb = odd_pairs(vb[j], sp.two12);
                             const uint2 a0 = table_quad<2>(ya, vlut), a1 = table_quad<3>(ya, vlut);
                             const uint2 a2 = table_quad<2>(yb, vlut), a3 = table_quad<3>(yb, vlut);
                             mma_f16_16816(oacc[4 * j + 1], a0.x, a1.x, a2.x, a3.x, t0, t1);
@@ -506,12 +558,12 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
 #pragma unroll
                     for (int u = 0; u < 4; ++u) {
                         {
-                            const uint32_t ya = even_pairs(ma[u]), yb = even_pairs(mb[u]);
+                            const uint32_t ya = even_pairs(ma[u], sp.two20), yb = even_pairs(mb[u], sp.two20);
                             mma_f16_16816(oacc[2 * u], table_pair<2>(ya, vlut), table_pair<3>(ya, vlut), table_pair<2>(yb, vlut),
                                           table_pair<3>(yb, vlut), back0, back1);
                         }
                         {
-                            const uint32_t ya = odd_pairs(ma[u]), yb = odd_pairs(mb[u]);
+                            const uint32_t ya = odd_pairs(ma[u], sp.two12), yb = odd_pairs(mb[u], sp.two12);
                             mma_f16_16816(oacc[2 * u + 1], table_pair<2>(ya, vlut), table_pair<3>(ya, vlut), table_pair<2>(yb, vlut),
                                           table_pair<3>(yb, vlut), t0, t1);
                         }
@@ -535,14 +587,16 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
                 parity ^= 1u;
             }
         };
-        for (int j = 0; j < seg && !timed_out; ++j) {
+        auto next_page = [&](auto at_end, int j) {
             if constexpr (SPARSE) {
-                if ((v_with_k >> stage) & 1u) one_page(std::true_type{}, j);
-                else one_page(std::false_type{}, j);
+                if ((v_with_k >> stage) & 1u) one_page(std::true_type{}, at_end, j);
+                else one_page(std::false_type{}, at_end, j);
             } else {
-                one_page(std::true_type{}, j);
+                one_page(std::true_type{}, at_end, j);
             }
-        }
+        };
+        for (int j = 0; j < seg - 1 && !timed_out; ++j) next_page(std::false_type{}, j);
+        if (!timed_out) next_page(std::true_type{}, seg - 1);
         if (timed_out) {   // let copies that are under way land before the CTA may end
             for (int s = 0; s < NSTAGE; ++s) (void)wait_bounded(bar + s * 8, s < static_cast<int>(stage) ? parity ^ 1u : parity);
             break;
@@ -602,9 +656,9 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
     }
 }
 
-template <int KB, int VB, bool QJL, bool SPARSE>
-int launch_stream(const StreamParams& sp, cudaStream_t stream) {
-    auto kern = decode_stream_kernel<KB, VB, QJL, SPARSE>;
+template <int KB, int VB, bool QJL, bool SPARSE, bool SIGN_TABLE>
+int launch_stream_as(const StreamParams& sp, cudaStream_t stream) {
+    auto kern = decode_stream_kernel<KB, VB, QJL, SPARSE, SIGN_TABLE>;
     static bool configured[64] = {};
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return TQ_ERR_LAUNCH;
@@ -613,6 +667,14 @@ int launch_stream(const StreamParams& sp, cudaStream_t stream) {
         configured[dev] = true;
     }
     return launch_chained(kern, dim3(sp.n_warps / kStreamWarps), dim3(kStreamThreads), kStreamSmem, stream, sp) == cudaSuccess ? TQ_OK : TQ_ERR_LAUNCH;
+}
+
+template <int KB, int VB, bool QJL, bool SPARSE>
+int launch_stream(const StreamParams& sp, cudaStream_t stream) {
+    if constexpr (QJL && KB == VB) {
+        if (sp.d.share_tables && !sp.d.qp) return launch_stream_as<KB, VB, QJL, SPARSE, true>(sp, stream);
+    }
+    return launch_stream_as<KB, VB, QJL, SPARSE, false>(sp, stream);
 }
 
 // One warp per query head: combines the parts of an item that more than one warp worked on.
