@@ -49,11 +49,19 @@ constexpr int kBarBytes = kWarps * 2 * kStages * 8;  // mbarriers at the start o
 // stream-serialization attribute, so a kernel's CTAs are scheduled while the previous kernel drains.  Each kernel
 // lets its successor go at once and waits for its predecessor's results before it reads or writes anything; both
 // instructions do nothing in a kernel that was launched without the attribute.
-__device__ __forceinline__ void pdl_release_and_wait() {
+__device__ __forceinline__ void pdl_release() {
 #if TQ_DEC_PDL
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+#endif
+}
+__device__ __forceinline__ void pdl_wait() {
+#if TQ_DEC_PDL
     asm volatile("griddepcontrol.wait;" ::: "memory");
 #endif
+}
+__device__ __forceinline__ void pdl_release_and_wait() {
+    pdl_release();
+    pdl_wait();
 }
 
 template <typename Kernel, typename... Args>
@@ -682,16 +690,22 @@ int dispatch_v(const DecodeParams& p, int vb, const Plan& plan, cudaStream_t str
     return TQ_ERR_UNSUPPORTED;
 }
 
-#ifndef TQ_STREAM_MIN
-#define TQ_STREAM_MIN 1
-#endif
-constexpr int64_t kStreamMinPages = TQ_STREAM_MIN;
-// Workspace of the persistent kernel, or 0 where the chunked kernel is the better one.
-int64_t stream_bytes(int64_t ns, int64_t hq, int64_t hkv, int64_t max_pages) {
-    const int64_t items = hkv * ((hq / hkv + 7) / 8);
-    const int64_t pages = ns * max_pages * items;
+// Which kernel is the better one, by the pages that the batch can have at most.  The persistent kernel pays about 13 us
+// however few pages there are (all its tables, one more level of merging), the chunked one 8 to 11, but it takes
+// 0.43 (4-bit) to 0.6 us (with sign term) per 1000 pages where the chunked one takes 0.68 to 0.78.  Measured us, chunked /
+// persistent, 8 KV heads: turbo4 2 x 8192 tokens (8192 pages) 26.2 / 19.4, 4 x 2048 (4096 pages) 14.6 / 16.6; turbo3
+// 2 x 8192 22.2 / 20.7, 16 x 2048 (16384 pages) 27.1 / 26.9, 32 x 1024 26.9 / 27.4, 64 x 1024 39.4 / 39.6.
+constexpr int64_t kStreamMinPages = 8192;
+constexpr int64_t kStreamSlots = static_cast<int64_t>(kStreamCtas) * (kStreamWarps + 2);   // partials of warps and of CTAs
+int64_t pages_at_most(int64_t ns, int64_t hq, int64_t hkv, int64_t max_pages) { return ns * max_pages * hkv * ((hq / hkv + 7) / 8); }
+bool stream_is_better(int64_t pages, int max_pages, bool qjl) {
+    if (pages < kStreamMinPages || pages > INT32_MAX) return false;
+    return !qjl || max_pages >= 512 || pages >= 49152 || (pages >= 16384 && max_pages >= 128);
+}
+// Workspace of the persistent kernel, or 0 where no format would take it.
+int64_t stream_bytes(int64_t pages) {
     if (pages < kStreamMinPages || pages > INT32_MAX) return 0;
-    return 2ll * kStreamCtas * kStreamWarps * (kStreamSlotFloats + 16) * static_cast<int64_t>(sizeof(float)) + (ns + 1) * 4;
+    return kStreamSlots * (kStreamSlotFloats + 16) * static_cast<int64_t>(sizeof(float)) + kStreamCtas * static_cast<int64_t>(sizeof(int4));
 }
 
 }  // namespace
@@ -761,7 +775,7 @@ extern "C" int64_t tq_decode_workspace_bytes(int num_seqs, int num_q_heads, int 
 extern "C" int64_t tq_decode_auto_workspace_bytes(int num_seqs, int num_q_heads, int num_kv_heads, int max_pages_per_seq) {
     const int64_t chunked = tq_decode_workspace_bytes(num_seqs, num_q_heads, num_kv_heads, max_pages_per_seq, 0);
     if (chunked < 0) return chunked;
-    const int64_t stream = stream_bytes(num_seqs, num_q_heads, num_kv_heads, max_pages_per_seq);
+    const int64_t stream = stream_bytes(pages_at_most(num_seqs, num_q_heads, num_kv_heads, max_pages_per_seq));
     return stream > chunked ? stream : chunked;
 }
 
@@ -788,7 +802,8 @@ extern "C" int tq_decode_paged(void* out, const void* q_rot, const void* q_proj,
         return TQ_ERR_ARG;
     // The persistent kernel takes the calls that leave the split to the library and bring the workspace for it.
     const bool tensor_memory = use_tcgen05 && k_bits <= 3 && v_bits <= 3 && !(sparse_thresh > 0.f);
-    const int64_t stream_need = chunk_pages > 0 || tensor_memory ? 0 : stream_bytes(num_seqs, num_q_heads, num_kv_heads, max_pages_per_seq);
+    const int64_t pages = pages_at_most(num_seqs, num_q_heads, num_kv_heads, max_pages_per_seq);
+    const int64_t stream_need = chunk_pages <= 0 && !tensor_memory && stream_is_better(pages, max_pages_per_seq, use_qjl != 0) ? stream_bytes(pages) : 0;
     const bool persistent = stream_need > 0 && workspace && workspace_bytes >= stream_need && !(reinterpret_cast<uintptr_t>(workspace) & 15);
     if (chunk_pages <= 0) chunk_pages = tq_decode_auto_chunk_pages(num_seqs, num_kv_heads, num_q_heads, max_pages_per_seq);
     const int64_t need = tq_decode_workspace_bytes(num_seqs, num_q_heads, num_kv_heads, max_pages_per_seq, chunk_pages);
@@ -838,12 +853,13 @@ extern "C" int tq_decode_paged(void* out, const void* q_rot, const void* q_proj,
         sp.d = p;
         sp.ns = num_seqs;
         sp.HG = num_kv_heads * p.ngroups;
+        sp.weight_thresh = sparse_thresh > 0.f ? 0.5f * sparse_thresh : 0.f;
         sp.two12 = 1u << 12;
         sp.two20 = 1u << 20;
         sp.n_warps = kStreamCtas * kStreamWarps;
         sp.part_o = static_cast<float*>(workspace);
-        sp.part_ml = reinterpret_cast<float2*>(sp.part_o + 2ll * sp.n_warps * kStreamSlotFloats);
-        sp.prefix = reinterpret_cast<int32_t*>(sp.part_ml + 2ll * sp.n_warps * 8);
+        sp.part_ml = reinterpret_cast<float2*>(sp.part_o + kStreamSlots * kStreamSlotFloats);
+        sp.split = reinterpret_cast<int4*>(sp.part_ml + kStreamSlots * 8);
     }
     const Plan plan = {dim3(max_chunks, num_kv_heads * p.ngroups, num_seqs), persistent ? &sp : nullptr, use_qjl != 0, sparse_thresh > 0.f};
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
@@ -858,9 +874,7 @@ extern "C" int tq_decode_paged(void* out, const void* q_rot, const void* q_proj,
     }
     if (rc != TQ_OK) return rc;
     if (persistent) {
-        const int64_t rows = static_cast<int64_t>(num_seqs) * num_q_heads;
-        if (launch_chained(decode_stream_merge_kernel, dim3(static_cast<unsigned>((rows + kMergeWarps - 1) / kMergeWarps)), dim3(kMergeWarps * 32),
-                           0, st, sp) != cudaSuccess)
+        if (launch_chained(decode_stream_merge_kernel, dim3(kStreamCtas), dim3(256), 0, st, sp) != cudaSuccess)
             return TQ_ERR_LAUNCH;
     } else if (max_chunks > 1) {
         if (launch_chained(decode_merge_kernel, dim3(num_q_heads, num_seqs), dim3(kHeadDim), 0, st, p) != cudaSuccess)

@@ -2,12 +2,12 @@
 // contiguous share of all pages.
 //
 // All (sequence, KV head, query group) items of the batch are laid end to end, page after page; warp w of W takes pages
-// [w U / W, (w + 1) U / W).  The warps never wait for one another: a warp keeps its running maximum, denominators and
-// accumulators while it stays inside an item, writes the output itself when it saw the whole item, and otherwise leaves
-// one of at most two partial results (the item it started in the middle of, the item it could not finish) for
-// decode_stream_merge_kernel.  Against the chunked kernel (4-warp CTAs, one chunk of one item each) this takes away the
-// last wave that is three quarters full, the table fill, pipeline start and block-wide merge per chunk, and the empty
-// CTAs of a ragged batch.
+// [w U / W, (w + 1) U / W).  The warps never wait for one another while they stream: a warp keeps its running maximum,
+// denominators and accumulators while it stays inside an item and writes the output itself when it saw the whole item.
+// Otherwise it leaves a partial result; the CTA combines the partials of its 16 (neighbouring) warps and leaves at most
+// two of its own, the item it started in the middle of and the item it could not finish, for decode_stream_merge_kernel.
+// Against the chunked kernel (4-warp CTAs, one chunk of one item each) this takes away the last wave that is three
+// quarters full, the table fill, pipeline start and merge per chunk, and the empty CTAs of a ragged batch.
 namespace tq {
 namespace {
 
@@ -16,28 +16,19 @@ constexpr int kStreamThreads = kStreamWarps * 32;
 constexpr int kStreamStages = 4;
 constexpr int kStreamTable = 65536;          // 256 entries of 256 bytes: 128 bytes for K, 128 bytes for V
 constexpr int kStreamCtas = 148;             // one per SM
-constexpr int kStreamSmem = 230144;          // dynamic part of the 227 KB an SM gives one CTA
+constexpr int kStreamSmem = 229376;          // dynamic part of the 227 KB an SM gives one CTA
 constexpr int kStreamSlotFloats = 8 * kHeadDim;
 
 struct StreamParams {
     DecodeParams d;
     int ns, HG;          // sequences; items per sequence (KV heads x query groups)
     int n_warps;
-    float* part_o;       // [2 n_warps][8][128]: slot 2 w + 1 starts at its item's first page, slot 2 w does not
-    float2* part_ml;     // [2 n_warps][8] (maximum, denominator)
-    int32_t* prefix;     // [ns + 1] pages of all sequences before s
+    float* part_o;       // [n_warps + 2 n_ctas][8][128]: one slot per warp, then two per CTA (1: starts at its item's first page)
+    float2* part_ml;     // [n_warps + 2 n_ctas][8] (maximum, denominator)
+    int4* split;         // [n_ctas] item that starts in the CTA and ends in a later one: (sequence, item of it, last CTA or -1)
     uint32_t two12, two20;
+    float weight_thresh; // Sparse-V: weights are relative to a reference at most one (log2) above the running maximum
 };
-
-// Warps that share `total` pages: all of them, but none with fewer than kStreamMinShare pages.
-#ifndef TQ_MIN_SHARE
-#define TQ_MIN_SHARE 4
-#endif
-constexpr int kStreamMinShare = TQ_MIN_SHARE;
-__device__ __forceinline__ int active_warps(const StreamParams& sp, int64_t total) {
-    const int64_t most = (total + kStreamMinShare - 1) / kStreamMinShare;
-    return most < sp.n_warps ? static_cast<int>(most) : sp.n_warps;
-}
 
 __device__ __forceinline__ int pages_of(const DecodeParams& p, int len) {
     return len <= 0 ? 0 : min((len + kPageTokens - 1) / kPageTokens, p.max_pages);
@@ -193,6 +184,36 @@ __device__ __forceinline__ uint4 table_signs(uint32_t w, uint32_t base) {
     return v;
 }
 
+// Output row g of an item from its weighted sum (lane: dims 4 lane .. 4 lane + 3) and denominator.
+__device__ __forceinline__ void finish_row(const DecodeParams& p, int seq, int hg, int g, int lane, float (&x)[4], float l) {
+    const int kvh = p.ngroups == 1 ? hg : hg / p.ngroups, qg = hg - kvh * p.ngroups;
+    if (g >= p.G - qg * 8) return;
+    const float inv = 1.f / l;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) x[i] *= inv;
+    if (p.derotate_out) {   // two stages in the lane, five across lanes
+        const float b0 = x[0] + x[1], b1 = x[0] - x[1], b2 = x[2] + x[3], b3 = x[2] - x[3];
+        x[0] = b0 + b2; x[1] = b1 + b3; x[2] = b0 - b2; x[3] = b1 - b3;
+#pragma unroll
+        for (int m = 1; m < 32; m <<= 1) {
+            const float sgn = (lane & m) ? -1.f : 1.f;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) x[i] = fmaf(sgn, x[i], __shfl_xor_sync(0xffffffffu, x[i], m));
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) x[i] *= kWhtScale;
+    }
+    uint2 w;
+    if (p.io_dtype == TQ_DTYPE_F16) {
+        w = make_uint2(pack_half2(x[0], x[1]), pack_half2(x[2], x[3]));
+    } else {
+        const __nv_bfloat162 lo = __floats2bfloat162_rn(x[0], x[1]), hi = __floats2bfloat162_rn(x[2], x[3]);
+        w = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+    }
+    const int64_t row = static_cast<int64_t>(seq) * p.Hq + kvh * p.G + qg * 8 + g;
+    *reinterpret_cast<uint2*>(static_cast<uint16_t*>(p.out) + row * kHeadDim + 4 * lane) = w;
+}
+
 // SIGN_TABLE: K and V share a codebook and S = I, so the V half of the table has room for the signs, and the query
 // operands of the index term serve the sign term as well.
 template <int KB, int VB, bool QJL, bool SPARSE, bool SIGN_TABLE>
@@ -214,8 +235,8 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ int sm_scan[kStreamThreads + 1];
     __shared__ int sm_wsum[kStreamWarps];
+    __shared__ int4 sm_part[2 * kStreamWarps];   // partials: (item or -1, sequence, pages of the item after this share, flags)
 
-    pdl_release_and_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int gid = lane >> 2, tig = lane & 3;
 
@@ -231,8 +252,15 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
                                        : tab + kStreamTable + (bars_low ? 0 : kBars) + (warp - n_low) * RING;
     const uint32_t bar = bars + warp * 2 * NSTAGE * 8;     // [0 .. NSTAGE) page (or K part), [NSTAGE ..) late V part
 
+    // Only the codebooks, which no kernel of this library writes, are read before the previous kernel is known to be done.
+    pdl_release();
+    fill_stream_table<KB>(tab, p.kc, warp, lane);
+    if constexpr (SIGN_TABLE) fill_sign_table(tab + 128, warp, lane);
+    else fill_stream_table<VB>(tab + 128, p.vc, warp, lane);
+    if (lane < 2) sm_part[2 * warp + lane] = make_int4(-1, 0, 0, 0);
     if (lane < 2 * NSTAGE) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar + lane * 8) : "memory");
     fence_barrier_init();
+    pdl_wait();
 
     // ---- pages before each thread's run of sequences (every CTA does the same scan over all lengths)
     const int per = (sp.ns + kStreamThreads - 1) / kStreamThreads;
@@ -245,42 +273,32 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
         if (lane >= o) incl += v;
     }
     if (lane == 31) sm_wsum[warp] = incl;
-    fill_stream_table<KB>(tab, p.kc, warp, lane);
-    if constexpr (SIGN_TABLE) fill_sign_table(tab + 128, warp, lane);
-    else fill_stream_table<VB>(tab + 128, p.vc, warp, lane);
     __syncthreads();
     int before = incl - own;
     for (int w = 0; w < warp; ++w) before += sm_wsum[w];
     sm_scan[threadIdx.x] = before;
     if (threadIdx.x == kStreamThreads - 1) sm_scan[kStreamThreads] = before + own;
-    if (blockIdx.x == 0) {   // for the merge kernel; flags and zero outputs are written once, too
-        int acc = before;
+    if (blockIdx.x == 0) {   // flags and zero outputs are written once
         for (int s = threadIdx.x * per; s < min(sp.ns, (static_cast<int>(threadIdx.x) + 1) * per); ++s) {
             const int len = p.seq_lens[s];
-            sp.prefix[s] = acc;
-            acc += pages_of(p, len);
             if (len > p.max_pages * kPageTokens && p.status) atomicOr(p.status, TQ_STATUS_BAD_BLOCK);
             if (len <= 0) {
                 uint4* o = reinterpret_cast<uint4*>(static_cast<uint16_t*>(p.out) + static_cast<int64_t>(s) * p.Hq * kHeadDim);
                 for (int i = 0; i < p.Hq * kHeadDim / 8; ++i) o[i] = make_uint4(0, 0, 0, 0);
             }
         }
-        if (threadIdx.x == kStreamThreads - 1) sp.prefix[sp.ns] = acc;
     }
     __syncthreads();
 
     const int64_t total = static_cast<int64_t>(sm_scan[kStreamThreads]) * sp.HG;
-    const int W = active_warps(sp, total);
-    // With work for every warp, the 16 shares of a CTA are neighbours (same query rows and table lines; measured 3 %
-    // faster than neighbours on different SMs); fewer shares are dealt out over the SMs.
-    const int gw = W == sp.n_warps ? blockIdx.x * kStreamWarps + warp : warp * static_cast<int>(gridDim.x) + static_cast<int>(blockIdx.x);
-    if (gw >= W) return;
+    const int W = sp.n_warps;
+    const int gw = blockIdx.x * kStreamWarps + warp;
     const int64_t first = total * gw / W;
-    const int n = static_cast<int>(total * (gw + 1) / W - first);   // this warp's pages, at least one
+    const int n = static_cast<int>(total * (gw + 1) / W - first);   // this warp's pages
 
     // ---- the item and page this warp starts in
-    int seq, hg, page, np, len;
-    {
+    int seq = 0, hg = 0, page = 0, np = 0, len = 0;
+    if (n > 0) {
         int lo = 0, hi = kStreamThreads;
         while (hi - lo > 1) {
             const int mid = (lo + hi) >> 1;
@@ -348,7 +366,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
     bool timed_out = false;
     uint32_t stage = 0, parity = 0;           // ring stage of the current page and the phase of its barrier
     uint32_t v_parity = 0;                    // Sparse-V: bit s = phase of the late-V barrier of stage s
-    uint32_t v_with_k = (1u << NSTAGE) - 1u;  // Sparse-V: bit s = the page in stage s brought its V part along
+    uint32_t k_only = 0;                      // Sparse-V: bit s = the page in stage s came without its V part
     uint32_t v_skipped = 0;
     int idx = 0;                              // pages of the share that are done
 
@@ -383,8 +401,8 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
 #pragma unroll
             for (int r = 0; r < 4; ++r) oacc[i][r] = 0.f;
 
-        auto one_page = [&](auto have_v, auto at_end, int j) {
-            constexpr bool HAVE_V = decltype(have_v)::value, AT_END = decltype(at_end)::value;
+        auto one_page = [&](auto have_v, int j) {
+            constexpr bool HAVE_V = decltype(have_v)::value;
             const uint32_t so = stage * PAGE;
             if (!wait_bounded(bar + stage * 8, parity)) {
                 timed_out = true;
@@ -395,7 +413,6 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
             lds_words<NWK, 0>(ring_k + so, wa);
             lds_words<NWK, 32 * NWK * 4>(ring_k + so, wb);
             float sm[4] = {0.f, 0.f, 0.f, 0.f};
-            float smb[4] = {0.f, 0.f, 0.f, 0.f};   // two chains of products for each of the two terms
             float sq[4] = {sq_init0, sq_init1, sq_init0, sq_init1}, sq2[4] = {0.f, 0.f, 0.f, 0.f};
             auto sign_term = [&](auto quarter) {   // eight dims of two tokens, two products
                 constexpr int B = decltype(quarter)::value;
@@ -417,12 +434,12 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
                     const uint2 a0 = table_quad<0>(wa[J], klut), a1 = table_quad<1>(wa[J], klut);
                     const uint2 b0 = table_quad<0>(wb[J], klut), b1 = table_quad<1>(wb[J], klut);
                     mma_f16_16816(sm, a0.x, b0.x, a1.x, b1.x, qf[8 * J], qf[8 * J + 1]);
-                    mma_f16_16816(smb, a0.y, b0.y, a1.y, b1.y, qf[8 * J + 4], qf[8 * J + 5]);
+                    mma_f16_16816(sm, a0.y, b0.y, a1.y, b1.y, qf[8 * J + 4], qf[8 * J + 5]);
                     sign_term(std::integral_constant<int, 2 * J>{});
                     const uint2 c0 = table_quad<2>(wa[J], klut), c1 = table_quad<3>(wa[J], klut);
                     const uint2 d0 = table_quad<2>(wb[J], klut), d1 = table_quad<3>(wb[J], klut);
                     mma_f16_16816(sm, c0.x, d0.x, c1.x, d1.x, qf[8 * J + 2], qf[8 * J + 3]);
-                    mma_f16_16816(smb, c0.y, d0.y, c1.y, d1.y, qf[8 * J + 6], qf[8 * J + 7]);
+                    mma_f16_16816(sm, c0.y, d0.y, c1.y, d1.y, qf[8 * J + 6], qf[8 * J + 7]);
                     sign_term(std::integral_constant<int, 2 * J + 1>{});
                 };
                 quads(std::integral_constant<int, 0>{});
@@ -438,7 +455,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
                     mma_f16_16816(sm, a0, b0, a1, b1, qf[4 * C], qf[4 * C + 1]);
                     const uint32_t a2 = table_pair<2>(mwa[C], klut), a3 = table_pair<3>(mwa[C], klut);
                     const uint32_t b2 = table_pair<2>(mwb[C], klut), b3 = table_pair<3>(mwb[C], klut);
-                    mma_f16_16816(smb, a2, b2, a3, b3, qf[4 * C + 2], qf[4 * C + 3]);
+                    mma_f16_16816(sm, a2, b2, a3, b3, qf[4 * C + 2], qf[4 * C + 3]);
                     sign_term(word);
                 };
                 eight_dims(std::integral_constant<int, 0>{});
@@ -449,7 +466,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
             float2 kn = unpack_half2(lds_u32<KN_OFF>(ring_n + so));
             kn.x *= p.qscale;
             kn.y *= p.qscale;
-            float s0 = (sm[0] + smb[0]) * kn.x, s1 = (sm[1] + smb[1]) * kn.x, s2 = (sm[2] + smb[2]) * kn.y, s3 = (sm[3] + smb[3]) * kn.y;
+            float s0 = sm[0] * kn.x, s1 = sm[1] * kn.x, s2 = sm[2] * kn.y, s3 = sm[3] * kn.y;
             if constexpr (QJL) {
                 float2 krn = unpack_half2(lds_u32<KRN_OFF>(ring_n + so));
                 krn.x *= qpscale;
@@ -459,8 +476,8 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
                 s2 = fmaf(sq[2] + sq2[2], krn.y, s2);
                 s3 = fmaf(sq[3] + sq2[3], krn.y, s3);
             }
-            const int valid_tokens = AT_END ? len - (page + j) * kPageTokens : kPageTokens;
-            if (AT_END && valid_tokens < kPageTokens) {   // only the last page of a sequence is partly filled
+            const int valid_tokens = len - (page + j) * kPageTokens;
+            if (valid_tokens < kPageTokens) {   // only the last page of a sequence is partly filled
                 if (gid >= valid_tokens) { s0 = -INFINITY; s1 = -INFINITY; }
                 if (gid + 8 >= valid_tokens) { s2 = -INFINITY; s3 = -INFINITY; }
             }
@@ -495,10 +512,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
             // ---- Sparse-V: the V part is not needed when no weight of the group exceeds the threshold.  The reference is
             // at most one above the running maximum.
             bool do_v = true;
-            if constexpr (SPARSE) {
-                const float e = fmaxf(fmaxf(s0 - m0, s1 - m1), fmaxf(s2 - m0, s3 - m1));
-                do_v = __any_sync(0xffffffffu, e > p.log2_thresh - 1.f);
-            }
+            if constexpr (SPARSE) do_v = __any_sync(0xffffffffu, fmaxf(fmaxf(p0v, p1v), fmaxf(p2v, p3v)) > sp.weight_thresh);
             bool have = true;
             if constexpr (SPARSE && !HAVE_V) {
                 if (do_v) {   // first needed page after a run of skipped ones: fetch its V part now
@@ -513,7 +527,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
             }
             if (have) {
                 float2 vn = unpack_half2(lds_u32<VN_OFF>(ring_n + so));
-                if (AT_END && valid_tokens < kPageTokens) {
+                if (valid_tokens < kPageTokens) {
                     if (gid >= valid_tokens) vn.x = 0.f;
                     if (gid + 8 >= valid_tokens) vn.y = 0.f;
                 }
@@ -580,23 +594,24 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
                 }
                 const bool whole = !SPARSE || do_v;
                 if (lane == (i & 31)) copy_in(ring + so, src, whole ? PAGE : KPART, bar + stage * 8);
-                if constexpr (SPARSE) v_with_k = whole ? (v_with_k | (1u << stage)) : (v_with_k & ~(1u << stage));
+                if constexpr (SPARSE) {
+                    if (whole != HAVE_V) k_only ^= 1u << stage;
+                }
             }
             if (++stage == NSTAGE) {
                 stage = 0;
                 parity ^= 1u;
             }
         };
-        auto next_page = [&](auto at_end, int j) {
+        auto next_page = [&](int j) {
             if constexpr (SPARSE) {
-                if ((v_with_k >> stage) & 1u) one_page(std::true_type{}, at_end, j);
-                else one_page(std::false_type{}, at_end, j);
+                if (k_only == 0 || !((k_only >> stage) & 1u)) one_page(std::true_type{}, j);
+                else one_page(std::false_type{}, j);
             } else {
-                one_page(std::true_type{}, at_end, j);
+                one_page(std::true_type{}, j);
             }
         };
-        for (int j = 0; j < seg - 1 && !timed_out; ++j) next_page(std::false_type{}, j);
-        if (!timed_out) next_page(std::true_type{}, seg - 1);
+        for (int j = 0; j < seg && !timed_out; ++j) next_page(j);
         if (timed_out) {   // let copies that are under way land before the CTA may end
             for (int s = 0; s < NSTAGE; ++s) (void)wait_bounded(bar + s * 8, s < static_cast<int>(stage) ? parity ^ 1u : parity);
             break;
@@ -609,6 +624,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
             l1 += __shfl_xor_sync(0xffffffffu, l1, o);
         }
         // accumulator 2 u + s, register r: dim 16 gid + 4 u + s + 2 (r >> 1) of query 2 tig + (r & 1)
+        const bool whole_item = page == 0 && seg == np, at_end = idx + seg == n;
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
             const int g = 2 * tig + k;
@@ -618,20 +634,28 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
             for (int u = 0; u < 4; ++u)
 #pragma unroll
                 for (int e = 0; e < 4; ++e) x[4 * u + e] = oacc[2 * u + (e & 1)][(e & 2) + k];
-            if (page == 0 && seg == np) {
+            if (whole_item) {
                 const float inv = 1.f / l;
 #pragma unroll
                 for (int i = 0; i < 16; ++i) x[i] *= inv;
                 if (p.derotate_out) wht_16x8(x, lane);
                 if (g < nq) store_row16(p.out, (static_cast<int64_t>(seq) * p.Hq + head0 + g) * kHeadDim + 16 * gid, p.io_dtype, x);
+            } else if (at_end) {   // the ring has served its purpose
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(ring + (g * kHeadDim + 16 * gid + 4 * i) * 4), "f"(x[4 * i]),
+                                 "f"(x[4 * i + 1]), "f"(x[4 * i + 2]), "f"(x[4 * i + 3])
+                                 : "memory");
+                if (gid == 0) asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(ring + (kStreamSlotFloats + 2 * g) * 4), "f"(k ? m1 : m0), "f"(l) : "memory");
             } else {
-                const int slot = 2 * gw + (page == 0 ? 1 : 0);
-                float4* dst = reinterpret_cast<float4*>(sp.part_o + static_cast<int64_t>(slot) * kStreamSlotFloats + g * kHeadDim + 16 * gid);
+                float4* dst = reinterpret_cast<float4*>(sp.part_o + static_cast<int64_t>(gw) * kStreamSlotFloats + g * kHeadDim + 16 * gid);
 #pragma unroll
                 for (int i = 0; i < 4; ++i) dst[i] = make_float4(x[4 * i], x[4 * i + 1], x[4 * i + 2], x[4 * i + 3]);
-                if (gid == 0) sp.part_ml[slot * 8 + g] = make_float2(k ? m1 : m0, l);
+                if (gid == 0) sp.part_ml[gw * 8 + g] = make_float2(k ? m1 : m0, l);
             }
         }
+        if (!whole_item && lane == 0)
+            sm_part[2 * warp + (at_end ? 1 : 0)] = make_int4(hg, seq, np - page - seg, page == 0 ? 1 : 0);
         idx += seg;
         page = 0;
         if (idx < n && ++hg == sp.HG) {
@@ -654,6 +678,71 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
             atomicAdd(p.skip_stats + 1, v_skipped);
         }
     }
+    // ---- combine the partials of the CTA's warps: entry 2 w (item that ended inside warp w's share) and 2 w + 1 (the one
+    // its share ended in), in page order.  Warp (c, q) takes query row q of every other run of entries of one item.
+    __syncthreads();
+    const int4 part = sm_part[lane];
+    const uint32_t live = __ballot_sync(0xffffffffu, part.x >= 0);
+    const int prev = 31 - __clz(live & ((1u << lane) - 1u));   // the live entry before this one, or -1
+    const int4 before_me = make_int4(__shfl_sync(0xffffffffu, part.x, max(prev, 0)), __shfl_sync(0xffffffffu, part.y, max(prev, 0)), 0, 0);
+    uint32_t heads = __ballot_sync(0xffffffffu, part.x >= 0 && (prev < 0 || before_me.x != part.x || before_me.y != part.y));
+    bool split = false;
+    int run = 0;
+    for (; heads; ++run) {
+        const int head = __ffs(heads) - 1;
+        heads &= heads - 1;
+        const uint32_t mine = live & ~((1u << head) - 1u) & (heads ? (1u << (__ffs(heads) - 1)) - 1u : 0xffffffffu);
+        const int last = 31 - __clz(mine);
+        const int rhg = __shfl_sync(0xffffffffu, part.x, head), rseq = __shfl_sync(0xffffffffu, part.y, head);
+        const bool starts = __shfl_sync(0xffffffffu, part.w, head) != 0;
+        const int after = __shfl_sync(0xffffffffu, part.z, last);
+        if (starts && after > 0 && threadIdx.x == 0) {
+            split = true;
+            const int64_t end = total * (static_cast<int64_t>(blockIdx.x + 1) * kStreamWarps) / W + after;   // pages before the item's end
+            // the warp whose share holds page u is the largest w with floor(w * total / W) <= u
+            sp.split[blockIdx.x] = make_int4(rseq, rhg, static_cast<int>((end * W - 1) / total) / kStreamWarps, 0);
+        }
+        if ((run & 1) != (warp >> 3)) continue;
+        const int g = warp & 7;
+        auto ring_of = [&](int w) {
+            return w < n_low ? base + (bars_low ? kBars : 0) + w * RING : tab + kStreamTable + (bars_low ? 0 : kBars) + (w - n_low) * RING;
+        };
+        // lane e holds (maximum, denominator) of entry e
+        float2 ml = make_float2(-INFINITY, 0.f);
+        if ((mine >> lane) & 1u) {
+            if (lane & 1) asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(ml.x), "=f"(ml.y) : "r"(ring_of(lane >> 1) + (kStreamSlotFloats + 2 * g) * 4));
+            else ml = __ldcg(sp.part_ml + (blockIdx.x * kStreamWarps + (lane >> 1)) * 8 + g);
+        }
+        float M = ml.x;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
+        const float scale = ex2(ml.x - M);
+        float l = scale * ml.y;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+        float x[4] = {0.f, 0.f, 0.f, 0.f};
+        for (uint32_t rest = mine; rest; rest &= rest - 1) {
+            const int e = __ffs(rest) - 1;
+            float4 v;
+            if (e & 1)
+                asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(ring_of(e >> 1) + (g * kHeadDim + 4 * lane) * 4));
+            else
+                v = __ldcg(reinterpret_cast<const float4*>(sp.part_o + static_cast<int64_t>(blockIdx.x * kStreamWarps + (e >> 1)) * kStreamSlotFloats + g * kHeadDim + 4 * lane));
+            const float sc = __shfl_sync(0xffffffffu, scale, e);
+            x[0] = fmaf(sc, v.x, x[0]);
+            x[1] = fmaf(sc, v.y, x[1]);
+            x[2] = fmaf(sc, v.z, x[2]);
+            x[3] = fmaf(sc, v.w, x[3]);
+        }
+        if (starts && after == 0) {
+            finish_row(p, rseq, rhg, g, lane, x, l);
+        } else {
+            const int slot = sp.n_warps + 2 * blockIdx.x + (starts ? 1 : 0);
+            *reinterpret_cast<float4*>(sp.part_o + static_cast<int64_t>(slot) * kStreamSlotFloats + g * kHeadDim + 4 * lane) = make_float4(x[0], x[1], x[2], x[3]);
+            if (lane == 0) sp.part_ml[slot * 8 + g] = make_float2(M, l);
+        }
+    }
+    if (threadIdx.x == 0 && !split) sp.split[blockIdx.x].z = -1;
 }
 
 template <int KB, int VB, bool QJL, bool SPARSE, bool SIGN_TABLE>
@@ -677,60 +766,40 @@ int launch_stream(const StreamParams& sp, cudaStream_t stream) {
     return launch_stream_as<KB, VB, QJL, SPARSE, false>(sp, stream);
 }
 
-// One warp per query head: combines the parts of an item that more than one warp worked on.
-constexpr int kMergeWarps = 4;
-__global__ void __launch_bounds__(kMergeWarps * 32) decode_stream_merge_kernel(const StreamParams sp) {
-    pdl_release_and_wait();
-    const DecodeParams& p = sp.d;
-    const int64_t id = static_cast<int64_t>(blockIdx.x) * kMergeWarps + (threadIdx.x >> 5);
-    const int lane = threadIdx.x & 31;
-    if (id >= static_cast<int64_t>(sp.ns) * p.Hq) return;
-    const int seq = static_cast<int>(id / p.Hq), head = static_cast<int>(id - static_cast<int64_t>(seq) * p.Hq);
-    const int kvh = head / p.G, gi = head - kvh * p.G, g = gi & 7;
-    const int s0 = sp.prefix[seq], np = sp.prefix[seq + 1] - s0;
-    if (np == 0) return;   // zeros, already written
-    const int64_t total = static_cast<int64_t>(sp.prefix[sp.ns]) * sp.HG;
-    const int64_t a = static_cast<int64_t>(s0) * sp.HG + static_cast<int64_t>(kvh * p.ngroups + (gi >> 3)) * np;
-    // the warp whose share holds page u is the largest w with floor(w * total / W) <= u
-    const int W = active_warps(sp, total);
-    const int w0 = static_cast<int>(((a + 1) * W - 1) / total), w1 = static_cast<int>(((a + np) * W - 1) / total);
-    if (w0 == w1) return;  // written by that warp
+// One block per CTA of the stream kernel: combines the parts of the item that starts there and ends in a later CTA, one
+// warp per query row.
+__global__ void __launch_bounds__(256) decode_stream_merge_kernel(const StreamParams sp) {
+    pdl_release();
+    pdl_wait();
+    const int cta = blockIdx.x, g = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int4 item = sp.split[cta];
+    if (item.z < 0) return;
+    const int parts = item.z - cta + 1;   // slot 1 of this CTA, slot 0 of the others
+    auto slot_of = [&](int i) { return sp.n_warps + 2 * (cta + i) + (i == 0 ? 1 : 0); };
     float M = -INFINITY;
-    for (int w = w0; w <= w1; ++w) M = fmaxf(M, sp.part_ml[(2 * w + (w == w0)) * 8 + g].x);
-    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int i = lane; i < parts; i += 32) M = fmaxf(M, sp.part_ml[slot_of(i) * 8 + g].x);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
+    float x[4] = {0.f, 0.f, 0.f, 0.f};
     float l = 0.f;
-    for (int w = w0; w <= w1; ++w) {
-        const int slot = 2 * w + (w == w0);
-        const float2 ml = sp.part_ml[slot * 8 + g];
-        const float sc = ex2(ml.x - M);
-        const float4 v = *reinterpret_cast<const float4*>(sp.part_o + static_cast<int64_t>(slot) * kStreamSlotFloats + g * kHeadDim + 4 * lane);
-        o.x = fmaf(sc, v.x, o.x);
-        o.y = fmaf(sc, v.y, o.y);
-        o.z = fmaf(sc, v.z, o.z);
-        o.w = fmaf(sc, v.w, o.w);
-        l = fmaf(sc, ml.y, l);
-    }
-    float x[4] = {o.x / l, o.y / l, o.z / l, o.w / l};
-    if (p.derotate_out) {   // dims 4 lane .. 4 lane + 3: two stages in the lane, five across lanes
-        const float b0 = x[0] + x[1], b1 = x[0] - x[1], b2 = x[2] + x[3], b3 = x[2] - x[3];
-        x[0] = b0 + b2; x[1] = b1 + b3; x[2] = b0 - b2; x[3] = b1 - b3;
-#pragma unroll
-        for (int m = 1; m < 32; m <<= 1) {
-            const float sgn = (lane & m) ? -1.f : 1.f;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) x[i] = fmaf(sgn, x[i], __shfl_xor_sync(0xffffffffu, x[i], m));
+    for (int i0 = 0; i0 < parts; i0 += 32) {
+        float2 ml = make_float2(-INFINITY, 0.f);
+        if (i0 + lane < parts) ml = sp.part_ml[slot_of(i0 + lane) * 8 + g];
+        const float scale = ex2(ml.x - M);
+        l = fmaf(scale, ml.y, l);
+#pragma unroll 4
+        for (int i = 0; i < min(32, parts - i0); ++i) {
+            const float4 v = *reinterpret_cast<const float4*>(sp.part_o + static_cast<int64_t>(slot_of(i0 + i)) * kStreamSlotFloats + g * kHeadDim + 4 * lane);
+            const float sc = __shfl_sync(0xffffffffu, scale, i);
+            x[0] = fmaf(sc, v.x, x[0]);
+            x[1] = fmaf(sc, v.y, x[1]);
+            x[2] = fmaf(sc, v.z, x[2]);
+            x[3] = fmaf(sc, v.w, x[3]);
         }
+    }
 #pragma unroll
-        for (int i = 0; i < 4; ++i) x[i] *= kWhtScale;
-    }
-    uint2 w;
-    if (p.io_dtype == TQ_DTYPE_F16) {
-        w = make_uint2(pack_half2(x[0], x[1]), pack_half2(x[2], x[3]));
-    } else {
-        const __nv_bfloat162 lo = __floats2bfloat162_rn(x[0], x[1]), hi = __floats2bfloat162_rn(x[2], x[3]);
-        w = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
-    }
-    *reinterpret_cast<uint2*>(static_cast<uint16_t*>(p.out) + id * kHeadDim + 4 * lane) = w;
+    for (int o = 1; o < 32; o <<= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+    finish_row(sp.d, item.x, item.y, g, lane, x, l);
 }
 
 }  // namespace
