@@ -343,7 +343,7 @@ namespace tq {
 namespace {
 
 // ---- contiguous outputs ---------------------------------------------------------------------------
-enum class OutMode { kPackedK, kPackedV, kUnpacked };
+enum class OutMode { kPackedK, kPackedV };
 
 struct ContigParams {
     const void* x;
@@ -424,42 +424,10 @@ __device__ __forceinline__ void compress_contig_rows(const ContigParams& p, int6
 #pragma unroll
         for (int i = 0; i < 32; ++i) x[i] = 0.f;
     }
-    if constexpr (MODE == OutMode::kUnpacked) {
-        const bool with_signs = p.signs != nullptr;   // uniform over the grid
-        if (with_signs) quantize_quarter<BITS, true>(x, p.rotate != 0, lane, bd, csm, q);
-        else quantize_quarter<BITS, false>(x, p.rotate != 0, lane, bd, csm, q);
-        if (!live) return;
-        const int64_t o = row * kHeadDim + 32 * quarter;
-#pragma unroll
-        for (int i = 0; i < 32; i += 2) {
-            longlong2 v;
-            v.x = q.idx[i];
-            v.y = q.idx[i + 1];
-            *reinterpret_cast<longlong2*>(p.indices + o + i) = v;
-        }
-#pragma unroll
-        for (int i = 0; i < 32; i += 4)
-            *reinterpret_cast<float4*>(p.mse + o + i) = make_float4(csm[q.idx[i]] * q.norm, csm[q.idx[i + 1]] * q.norm,
-                                                                   csm[q.idx[i + 2]] * q.norm, csm[q.idx[i + 3]] * q.norm);
-        if (with_signs) {
-#pragma unroll
-            for (int i = 0; i < 32; i += 4) {
-                float s[4];
-#pragma unroll
-                for (int e = 0; e < 4; ++e) s[e] = ((q.signs >> (i + e)) & 1u) ? 1.f : -1.f;
-                *reinterpret_cast<float4*>(p.signs + o + i) = make_float4(s[0], s[1], s[2], s[3]);
-            }
-        }
-        if (quarter == 0) {
-            p.norms[row] = q.norm;
-            if (p.rnorm) p.rnorm[row] = q.rnorm;
-        }
-    } else {
-        quantize_quarter<BITS, QJL>(x, p.rotate != 0, lane, bd, csm, q);
-        if (!live) return;
-        store_idx_contig<BITS>(p.idx_out + row * (16 * BITS), quarter, q.idx);
-        store_contig_tail<QJL>(p, row, quarter, q.signs, q.norm, q.rnorm);
-    }
+    quantize_quarter<BITS, QJL>(x, p.rotate != 0, lane, bd, csm, q);
+    if (!live) return;
+    store_idx_contig<BITS>(p.idx_out + row * (16 * BITS), quarter, q.idx);
+    store_contig_tail<QJL>(p, row, quarter, q.signs, q.norm, q.rnorm);
 }
 
 template <int BITS, OutMode MODE>
@@ -470,6 +438,165 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) compress_contig_kernel(cons
     const int lane = threadIdx.x & 31;
     compress_contig_rows<BITS, MODE>(
         p, (static_cast<int64_t>(blockIdx.x) * kWarpsPerCta + (threadIdx.x >> 5)) * kItemsPerWarp + (lane >> 2), lane, csm);
+}
+
+// ---- unpacked outputs (polarquant_compress) -------------------------------------------------------------------
+// Four fifths of the traffic are stores (int64 indices, fp32 reconstruction and signs), so what counts is that every store
+// fills whole 32-byte sectors.  Four lanes share a row as elsewhere, but lane j holds dims 32 i + 8 j .. + 7 for i = 0 .. 3:
+// the four lanes write 128 contiguous bytes of fp32 per chunk, each lane one 32-byte access (two accesses of 16 bytes when
+// a pointer is not that aligned).  With 32 consecutive dims per lane every 16-byte store met half a sector of its own:
+// 65537 fp32 rows with signs took 73 us.
+template <bool WIDE>
+__device__ __forceinline__ void store8(void* dst, const uint32_t (&w)[8]) {
+    if constexpr (WIDE) {
+        asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]),
+                     "r"(w[5]), "r"(w[6]), "r"(w[7])
+                     : "memory");
+    } else {
+        reinterpret_cast<uint4*>(dst)[0] = make_uint4(w[0], w[1], w[2], w[3]);
+        reinterpret_cast<uint4*>(dst)[1] = make_uint4(w[4], w[5], w[6], w[7]);
+    }
+}
+
+template <bool WIDE>
+__device__ __forceinline__ void load8(const void* base, int64_t elem_off, int dtype, float* x) {
+    if (dtype == TQ_DTYPE_F32) {
+        const float* src = static_cast<const float*>(base) + elem_off;
+        if constexpr (WIDE) {
+            asm volatile("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                         : "=f"(x[0]), "=f"(x[1]), "=f"(x[2]), "=f"(x[3]), "=f"(x[4]), "=f"(x[5]), "=f"(x[6]), "=f"(x[7])
+                         : "l"(src));
+        } else {
+            const float4 a = __ldg(reinterpret_cast<const float4*>(src)), b = __ldg(reinterpret_cast<const float4*>(src) + 1);
+            x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w;
+            x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
+        }
+    } else {
+        const uint4 v = __ldg(reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(base) + elem_off));
+        const uint32_t r[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (dtype == TQ_DTYPE_F16) {
+                const float2 t = unpack_half2(r[k]);
+                x[2 * k] = t.x;
+                x[2 * k + 1] = t.y;
+            } else {
+                x[2 * k] = __uint_as_float(r[k] << 16);
+                x[2 * k + 1] = __uint_as_float(r[k] & 0xffff0000u);
+            }
+        }
+    }
+}
+
+// x[8 i + e] is dim 32 i + 8 j + e.  The stages run from dim bit 0 to dim bit 6, as in fwht128: same sums, same rounding.
+__device__ __forceinline__ void fwht128_chunks(float (&x)[32], int lane) {
+    auto in_lane = [&](int h) {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+            if (!(i & h)) {
+                const float a = x[i], b = x[i + h];
+                x[i] = a + b;
+                x[i + h] = a - b;
+            }
+        }
+    };
+    in_lane(1);
+    in_lane(2);
+    in_lane(4);
+#pragma unroll
+    for (int m = 1; m < 4; m <<= 1) {
+        const float sgn = (lane & m) ? -1.f : 1.f;
+#pragma unroll
+        for (int i = 0; i < 32; ++i) x[i] = fmaf(sgn, x[i], __shfl_xor_sync(0xffffffffu, x[i], m));
+    }
+    in_lane(8);
+    in_lane(16);
+}
+
+template <int BITS, bool SIGNS, bool WIDE>
+__global__ void __launch_bounds__(kWarpsPerCta * 32) compress_unpacked_kernel(const ContigParams p) {
+    __shared__ float csm[1 << BITS];
+    if (threadIdx.x < (1 << BITS)) csm[threadIdx.x] = p.c[threadIdx.x];
+    __syncthreads();
+    const int lane = threadIdx.x & 31, j = lane & 3;
+    const int64_t row = (static_cast<int64_t>(blockIdx.x) * kWarpsPerCta + (threadIdx.x >> 5)) * kItemsPerWarp + (lane >> 2);
+    const bool live = row < p.n;   // lanes of rows past the end take part in the shuffles, on zeros
+    const int64_t at = row * kHeadDim + 8 * j;
+    Boundaries<BITS> bd;
+    bd.load(p.b);
+    float x[32];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        if (live) load8<WIDE>(p.x, at + 32 * i, p.in_dtype, x + 8 * i);
+        else {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) x[8 * i + e] = 0.f;
+        }
+    }
+    if (p.rotate) {
+        fwht128_chunks(x, lane);
+#pragma unroll
+        for (int i = 0; i < 32; ++i) x[i] *= kWhtScale;
+    }
+    float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
+#pragma unroll
+    for (int i = 0; i < 32; i += 4) {
+        s0 = fmaf(x[i], x[i], s0);
+        s1 = fmaf(x[i + 1], x[i + 1], s1);
+        s2 = fmaf(x[i + 2], x[i + 2], s2);
+        s3 = fmaf(x[i + 3], x[i + 3], s3);
+    }
+    const float n = sqrtf(group_sum((s0 + s1) + (s2 + s3)));
+    const float den = n + 1e-8f;
+    const float inv = __frcp_rn(den);
+    float r0 = 0.f, r1 = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        uint32_t idx[8], mse[8], sign[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            const float v = x[8 * i + e];
+            const float q0 = v * inv;
+            const float u = fmaf(fmaf(-q0, den, v), inv, q0);   // = v / den, correctly rounded
+            idx[e] = static_cast<uint32_t>(bd.bucket(u));
+            const float c = csm[idx[e]];
+            mse[e] = __float_as_uint(c * n);
+            if constexpr (SIGNS) {
+                const float r = (u - c) * n;
+                if (e & 1) r1 = fmaf(r, r, r1);
+                else r0 = fmaf(r, r, r0);
+                sign[e] = r >= 0.f ? 0x3f800000u : 0xbf800000u;   // -0.0 and +0.0 both count as +
+            }
+        }
+        if (live) {
+            const int64_t o = at + 32 * i;
+            const uint32_t lo[8] = {idx[0], 0u, idx[1], 0u, idx[2], 0u, idx[3], 0u}, hi[8] = {idx[4], 0u, idx[5], 0u, idx[6], 0u, idx[7], 0u};
+            store8<WIDE>(p.indices + o, lo);
+            store8<WIDE>(p.indices + o + 4, hi);
+            store8<WIDE>(p.mse + o, mse);
+            if constexpr (SIGNS) store8<WIDE>(p.signs + o, sign);
+        }
+    }
+    const float rn = SIGNS ? sqrtf(group_sum(r0 + r1)) : 0.f;
+    if (live && j == 0) {
+        p.norms[row] = n;
+        if (p.rnorm) p.rnorm[row] = rn;
+    }
+}
+
+template <int BITS>
+void launch_unpacked(const ContigParams& p, cudaStream_t st) {
+    const unsigned grid = static_cast<unsigned>((p.n + kItemsPerCta - 1) / kItemsPerCta);
+    const uintptr_t all = reinterpret_cast<uintptr_t>(p.x) | reinterpret_cast<uintptr_t>(p.indices) | reinterpret_cast<uintptr_t>(p.mse) |
+                          reinterpret_cast<uintptr_t>(p.signs);
+    const bool wide = (all & 31) == 0;
+    if (p.signs) {
+        if (wide) compress_unpacked_kernel<BITS, true, true><<<grid, kWarpsPerCta * 32, 0, st>>>(p);
+        else compress_unpacked_kernel<BITS, true, false><<<grid, kWarpsPerCta * 32, 0, st>>>(p);
+    } else {
+        if (wide) compress_unpacked_kernel<BITS, false, true><<<grid, kWarpsPerCta * 32, 0, st>>>(p);
+        else compress_unpacked_kernel<BITS, false, false><<<grid, kWarpsPerCta * 32, 0, st>>>(p);
+    }
 }
 
 // ---- packed contiguous outputs on the table-driven quantizer ------------------------------------------------------
@@ -582,18 +709,16 @@ int launch_paged_v(const PagedParams& p, int vb, bool qjl, cudaStream_t st) {
 
 template <OutMode MODE>
 int launch_contig(const ContigParams& p, int bits, cudaStream_t st) {
-    if constexpr (MODE != OutMode::kUnpacked) {
-        // large packed launches: the persistent table-driven kernel.  Measured on fp16 rows with the rotation: 16384
-        // rows 5.9 us (binary-search kernel) against 6.8 us, 32768 rows about 11 us either way, 65536 rows 22 against
-        // 15 us: below about two groups of 128 rows per SM the persistent kernel mostly builds its table.
-        if (p.n > 2 * kSmallLaunchItems) {
-            constexpr bool QJL = MODE == OutMode::kPackedK;
-            switch (bits) {
-                case 2: return launch_contig_fast<2, QJL>(p, st);
-                case 3: return launch_contig_fast<3, QJL>(p, st);
-                case 4: return launch_contig_fast<4, QJL>(p, st);
-                default: return TQ_ERR_UNSUPPORTED;
-            }
+    // large packed launches: the persistent table-driven kernel.  Measured on fp16 rows with the rotation: 16384
+    // rows 5.9 us (binary-search kernel) against 6.8 us, 32768 rows about 11 us either way, 65536 rows 22 against
+    // 15 us: below about two groups of 128 rows per SM the persistent kernel mostly builds its table.
+    if (p.n > 2 * kSmallLaunchItems) {
+        constexpr bool QJL = MODE == OutMode::kPackedK;
+        switch (bits) {
+            case 2: return launch_contig_fast<2, QJL>(p, st);
+            case 3: return launch_contig_fast<3, QJL>(p, st);
+            case 4: return launch_contig_fast<4, QJL>(p, st);
+            default: return TQ_ERR_UNSUPPORTED;
         }
     }
     const unsigned grid = static_cast<unsigned>((p.n + kItemsPerCta - 1) / kItemsPerCta);
@@ -709,5 +834,11 @@ extern "C" int tq_polarquant_compress(const void* x, int in_dtype, int64_t n, co
     p.x = x; p.c = centroids; p.b = boundaries; p.indices = indices; p.norms = norms; p.mse = k_mse_rot;
     p.signs = use_qjl ? signs : nullptr; p.rnorm = use_qjl ? rnorm : nullptr;
     p.n = n; p.in_dtype = in_dtype; p.rotate = prerotated ? 0 : 1;
-    return launch_contig<OutMode::kUnpacked>(p, bits, reinterpret_cast<cudaStream_t>(stream));
+    switch (bits) {
+        case 2: launch_unpacked<2>(p, reinterpret_cast<cudaStream_t>(stream)); break;
+        case 3: launch_unpacked<3>(p, reinterpret_cast<cudaStream_t>(stream)); break;
+        case 4: launch_unpacked<4>(p, reinterpret_cast<cudaStream_t>(stream)); break;
+        default: return TQ_ERR_UNSUPPORTED;
+    }
+    return cudaGetLastError() == cudaSuccess ? TQ_OK : TQ_ERR_LAUNCH;
 }

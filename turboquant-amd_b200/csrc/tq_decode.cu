@@ -698,8 +698,8 @@ int dispatch_v(const DecodeParams& p, int vb, const Plan& plan, cudaStream_t str
 constexpr int64_t kStreamMinPages = 8192;
 constexpr int64_t kStreamSlots = static_cast<int64_t>(kStreamCtas) * (kStreamWarps + 2);   // partials of warps and of CTAs
 int64_t pages_at_most(int64_t ns, int64_t hq, int64_t hkv, int64_t max_pages) { return ns * max_pages * hkv * ((hq / hkv + 7) / 8); }
-bool stream_is_better(int64_t pages, int max_pages, bool qjl) {
-    if (pages < kStreamMinPages || pages > INT32_MAX) return false;
+bool stream_is_better(int64_t pages, int64_t cache_pages, int max_pages, bool qjl) {
+    if (pages < kStreamMinPages || pages > INT32_MAX || cache_pages > UINT32_MAX) return false;
     return !qjl || max_pages >= 512 || pages >= 49152 || (pages >= 16384 && max_pages >= 128);
 }
 // Workspace of the persistent kernel, or 0 where no format would take it.
@@ -803,7 +803,7 @@ extern "C" int tq_decode_paged(void* out, const void* q_rot, const void* q_proj,
     // The persistent kernel takes the calls that leave the split to the library and bring the workspace for it.
     const bool tensor_memory = use_tcgen05 && k_bits <= 3 && v_bits <= 3 && !(sparse_thresh > 0.f);
     const int64_t pages = pages_at_most(num_seqs, num_q_heads, num_kv_heads, max_pages_per_seq);
-    const int64_t stream_need = chunk_pages <= 0 && !tensor_memory && stream_is_better(pages, max_pages_per_seq, use_qjl != 0) ? stream_bytes(pages) : 0;
+    const int64_t stream_need = chunk_pages <= 0 && !tensor_memory && stream_is_better(pages, num_blocks * num_kv_heads * (block_size / kPageTokens), max_pages_per_seq, use_qjl != 0) ? stream_bytes(pages) : 0;
     const bool persistent = stream_need > 0 && workspace && workspace_bytes >= stream_need && !(reinterpret_cast<uintptr_t>(workspace) & 15);
     if (chunk_pages <= 0) chunk_pages = tq_decode_auto_chunk_pages(num_seqs, num_kv_heads, num_q_heads, max_pages_per_seq);
     const int64_t need = tq_decode_workspace_bytes(num_seqs, num_q_heads, num_kv_heads, max_pages_per_seq, chunk_pages);

@@ -318,19 +318,20 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
     }
     auto kv_head = [&](int h) { return p.ngroups == 1 ? h : h / p.ngroups; };
 
-    // ---- copies in: lane l holds the source address of page 32 k + l of the warp's share, one window of 32 ahead
+    // ---- copies in: lane l holds the place in the cache (in pages) of page 32 k + l of the warp's share, one window of 32 ahead
     bool bad_block = false;
-    auto locate = [&](int s, int h, int pg) -> const uint8_t* {
+    auto locate = [&](int s, int h, int pg) -> uint32_t {
         int32_t blk = __ldg(p.block_tables + static_cast<int64_t>(s) * p.bt_stride + (pg >> p.sub_shift));
         if (blk < 0 || blk >= p.num_blocks) {
             bad_block = true;
             blk = 0;
         }
-        return p.cache + blk * p.block_stride + ((kv_head(h) << p.sub_shift) + (pg & ((1 << p.sub_shift) - 1))) * PAGE;
+        return (static_cast<uint32_t>(blk * p.Hkv + kv_head(h)) << p.sub_shift) + (pg & ((1 << p.sub_shift) - 1));
     };
+    auto page_at = [&](uint32_t at) { return p.cache + static_cast<uint64_t>(at) * PAGE; };
     int wseq = seq, whg = hg, wpage = page, wnp = np, wbase = 0;     // where window `wbase / 32` starts
-    auto next_window = [&]() -> const uint8_t* {
-        const uint8_t* src = p.cache;
+    auto next_window = [&]() -> uint32_t {
+        uint32_t src = 0;
         int s = wseq, h = whg, pg = wpage + lane, m = wnp;
         if (wbase + lane < n) {
             while (pg >= m) {
@@ -349,10 +350,10 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
         wbase += 32;
         return src;
     };
-    const uint8_t* src = next_window();
-    const uint8_t* src_next = src;
+    uint32_t src = next_window();
+    uint32_t src_next = src;
     const int first_lot = min(n, NSTAGE);
-    if (lane < first_lot) copy_in(ring + lane * PAGE, src, PAGE, bar + lane * 8);
+    if (lane < first_lot) copy_in(ring + lane * PAGE, page_at(src), PAGE, bar + lane * 8);
     if (n > 32) src_next = next_window();
 
     const uint32_t klut = tab + (KB == 2 ? 8 * (lane & 15) : 4 * lane);
@@ -517,7 +518,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
             if constexpr (SPARSE && !HAVE_V) {
                 if (do_v) {   // first needed page after a run of skipped ones: fetch its V part now
                     const uint32_t vbar = bar + (NSTAGE + stage) * 8;
-                    if (lane == 0) copy_in(ring + so + KPART, locate(seq, hg, page + j) + KPART, PAGE - KPART, vbar);
+                    if (lane == 0) copy_in(ring + so + KPART, page_at(locate(seq, hg, page + j)) + KPART, PAGE - KPART, vbar);
                     if (!wait_bounded(vbar, (v_parity >> stage) & 1u)) timed_out = true;
                     v_parity ^= 1u << stage;
                 } else {
@@ -593,7 +594,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
                     if (i + 32 < n) src_next = next_window();
                 }
                 const bool whole = !SPARSE || do_v;
-                if (lane == (i & 31)) copy_in(ring + so, src, whole ? PAGE : KPART, bar + stage * 8);
+                if (lane == (i & 31)) copy_in(ring + so, page_at(src), whole ? PAGE : KPART, bar + stage * 8);
                 if constexpr (SPARSE) {
                     if (whole != HAVE_V) k_only ^= 1u << stage;
                 }
@@ -681,6 +682,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
     // ---- combine the partials of the CTA's warps: entry 2 w (item that ended inside warp w's share) and 2 w + 1 (the one
     // its share ended in), in page order.  Warp (c, q) takes query row q of every other run of entries of one item.
     __syncthreads();
+    const int64_t all = static_cast<int64_t>(*static_cast<volatile int*>(sm_scan + kStreamThreads)) * sp.HG;   // `total`, not kept over the loop
     const int4 part = sm_part[lane];
     const uint32_t live = __ballot_sync(0xffffffffu, part.x >= 0);
     const int prev = 31 - __clz(live & ((1u << lane) - 1u));   // the live entry before this one, or -1
@@ -698,9 +700,9 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
         const int after = __shfl_sync(0xffffffffu, part.z, last);
         if (starts && after > 0 && threadIdx.x == 0) {
             split = true;
-            const int64_t end = total * (static_cast<int64_t>(blockIdx.x + 1) * kStreamWarps) / W + after;   // pages before the item's end
+            const int64_t end = all * (static_cast<int64_t>(blockIdx.x + 1) * kStreamWarps) / W + after;   // pages before the item's end
             // the warp whose share holds page u is the largest w with floor(w * total / W) <= u
-            sp.split[blockIdx.x] = make_int4(rseq, rhg, static_cast<int>((end * W - 1) / total) / kStreamWarps, 0);
+            sp.split[blockIdx.x] = make_int4(rseq, rhg, static_cast<int>((end * W - 1) / all) / kStreamWarps, 0);
         }
         if ((run & 1) != (warp >> 3)) continue;
         const int g = warp & 7;
