@@ -243,3 +243,40 @@ def test_fast_kernel_residual_underflow_is_the_only_sign_deviation():
     tiny_rows = tiny[:, None].expand(T_BIG, HKV).reshape(-1).numpy()
     assert (ok["norms"][tiny_rows] == 0).all() and not differs[~tiny_rows].any()
     assert differs[tiny_rows].any()                               # the deviation is real: -0.0 read as negative
+
+
+@pytest.mark.parametrize("kb,vb,qjl", [(2, 2, True), (3, 3, True), (4, 4, False), (4, 2, False), (2, 3, True)])
+@pytest.mark.parametrize("T,hkv", [(1, 1), (2, 3), (7, 8), (16, 8), (149, 8), (2400, 8), (301, 5)])
+def test_units_of_all_sizes_and_slot_orders(kb, vb, qjl, T, hkv):
+    """Launches from one item to several rounds of warps, odd token counts, and slots that are contiguous (two tokens share a
+    32-bit V word and are written together), odd-aligned, or scattered: the same record for the same row, whatever the order."""
+    dev = "cuda:0"
+    fmt = CacheFormat(kb, vb, qjl)
+    books = Codebooks(fmt, dev)
+    g = torch.Generator(device=dev).manual_seed(T + hkv)
+    K = torch.randn(T, hkv, 128, generator=g, device=dev).half()
+    V = torch.randn(T, hkv, 128, generator=g, device=dev).half()
+    nb = T // 16 + 3
+    orders = {"contiguous": torch.arange(T, device=dev), "odd": torch.arange(T, device=dev) + 1,
+              "scattered": torch.randperm(T, generator=g, device=dev)}
+    seen = {}
+    for name, slots in orders.items():
+        cache = allocate_cache(nb, 16, hkv, fmt, dev)
+        compress_and_scatter(K, V, cache, slots.to(torch.int64), books, 16)
+        f = paged_layout.unpack_cache(cache.cpu(), 16, kb, vb, qjl)
+        s = slots.cpu()
+        seen[name] = {k: v[s // 16, s % 16] for k, v in f.items()}
+        untouched = torch.ones(nb * 16, dtype=torch.bool)
+        untouched[s] = False
+        assert (f["k_norm"].reshape(-1, hkv)[untouched] == 0).all() and (f["v_idx"].reshape(nb * 16, -1)[untouched] == 0).all()
+    for name in ("odd", "scattered"):
+        for k, v in seen["contiguous"].items():
+            assert torch.equal(seen[name][k], v), (name, k)
+    ok = O.polarquant_compress(K.float().cpu().numpy().reshape(-1, 128), books.kc.cpu().numpy(), books.kb.cpu().numpy(), kb, qjl,
+                               O.make_wht_matrix(128))
+    ov = O.polarquant_compress(V.float().cpu().numpy().reshape(-1, 128), books.vc.cpu().numpy(), books.vb.cpu().numpy(), vb, False,
+                               O.make_wht_matrix(128))
+    # the rotation's own rounding: at most 1e-4 of the coordinates, and one coordinate where that is less than one
+    for got, want in ((seen["odd"]["k_idx"], ok["indices"]), (seen["odd"]["v_idx"], ov["indices"])):
+        wrong = (got.numpy().reshape(-1, 128) != want).sum()
+        assert wrong <= max(1, 1e-4 * want.size)

@@ -233,6 +233,7 @@ struct PagedParams {
     int64_t ks_t, ks_h, vs_t, vs_h;
     int64_t num_slots;
     int64_t n_items;   // n_tokens * n_kv_heads
+    int64_t n_tokens;
     int Hkv, block_size, in_dtype, rotate;
     int use_tcgen05;       // TQ_COMPRESS_TCGEN05 was given
 };
@@ -384,28 +385,37 @@ __device__ __forceinline__ void store_idx_contig(uint8_t* row, int quarter, cons
     }
 }
 
-// Sign bits and norms of one packed row (this lane's quarter).  signs: bit l = 1 when the residual of local dim l is >= 0.
+// Sign bits and norms of one packed row (this lane's quarter); lanes of rows past the end take part in the shuffles.  signs: bit l = 1 when the residual of local dim l is >= 0.
 template <bool QJL>
 __device__ __forceinline__ void store_contig_tail(const ContigParams& p, int64_t row, int quarter, uint32_t signs, float norm,
-                                                  float rnorm) {
+                                                  float rnorm, bool live) {
     if constexpr (QJL) {
         uint8_t* srow = p.sign_out + row * 16;
         if (p.permute) {
-            // stride-4 order: output bit 32 c + i <- dim c + 4 i.  This lane's dim 32 q + l has
-            // c = l & 3 and i = 8 q + (l >> 2): it fills byte q of each of the four 32-bit words.
+            // stride-4 order: output bit 32 c + i <- dim c + 4 i.  This lane's dim 32 q + l has c = l & 3 and
+            // i = 8 q + (l >> 2): it fills byte q of each of the four 32-bit words.  Two unshuffles (even bits down, odd bits
+            // up) turn bit l into bit 8 (l & 3) + (l >> 2), then the four lanes of the row transpose their bytes, so that
+            // lane c holds word c.
+            uint32_t v = signs;
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                uint32_t v = 0;
-#pragma unroll
-                for (int k = 0; k < 8; ++k) v |= ((signs >> (4 * k + c)) & 1u) << k;
-                srow[4 * c + quarter] = static_cast<uint8_t>(v);
+            for (int i = 0; i < 2; ++i) {
+                uint32_t x;
+                x = (v ^ (v >> 1)) & 0x22222222u; v ^= x ^ (x << 1);
+                x = (v ^ (v >> 2)) & 0x0c0c0c0cu; v ^= x ^ (x << 2);
+                x = (v ^ (v >> 4)) & 0x00f000f0u; v ^= x ^ (x << 4);
+                x = (v ^ (v >> 8)) & 0x0000ff00u; v ^= x ^ (x << 8);
             }
+            const uint32_t o = __shfl_xor_sync(0xffffffffu, v, 2);
+            v = (quarter & 2) ? prmt(o, v, 0x7632u) : prmt(v, o, 0x5410u);
+            const uint32_t n = __shfl_xor_sync(0xffffffffu, v, 1);
+            v = (quarter & 1) ? prmt(n, v, 0x7351u) : prmt(v, n, 0x6240u);
+            if (live) reinterpret_cast<uint32_t*>(srow)[quarter] = v;
         } else {
-            reinterpret_cast<uint32_t*>(srow)[quarter] = signs;   // byte j bit b <- dim 8 j + b
+            if (live) reinterpret_cast<uint32_t*>(srow)[quarter] = signs;   // byte j bit b <- dim 8 j + b
         }
-        if (quarter == 0) p.rnorm_h[row] = __float2half_rn(rnorm);
+        if (live && quarter == 0) p.rnorm_h[row] = __float2half_rn(rnorm);
     }
-    if (quarter == 0) p.norm_h[row] = __float2half_rn(norm);
+    if (live && quarter == 0) p.norm_h[row] = __float2half_rn(norm);
 }
 
 // One group of 8 rows per warp on the generic quantizer (binary-search bucketize over arbitrary sorted boundaries).
@@ -425,9 +435,8 @@ __device__ __forceinline__ void compress_contig_rows(const ContigParams& p, int6
         for (int i = 0; i < 32; ++i) x[i] = 0.f;
     }
     quantize_quarter<BITS, QJL>(x, p.rotate != 0, lane, bd, csm, q);
-    if (!live) return;
-    store_idx_contig<BITS>(p.idx_out + row * (16 * BITS), quarter, q.idx);
-    store_contig_tail<QJL>(p, row, quarter, q.signs, q.norm, q.rnorm);
+    if (live) store_idx_contig<BITS>(p.idx_out + row * (16 * BITS), quarter, q.idx);
+    store_contig_tail<QJL>(p, row, quarter, q.signs, q.norm, q.rnorm, live);
 }
 
 template <int BITS, OutMode MODE>
@@ -605,82 +614,88 @@ void launch_unpacked(const ContigParams& p, cudaStream_t st) {
 // warp, two groups ahead, and rotated on the tensor cores; fp32 and already rotated rows take plain loads.
 template <int BITS, bool QJL>
 __device__ __forceinline__ void store_contig_fast(const ContigParams& p, int64_t row, int quarter, const Packed& q) {
+    const bool live = row < p.n;
     uint32_t* dst = reinterpret_cast<uint32_t*>(p.idx_out + row * (16 * BITS) + quarter * (4 * BITS));
-    if constexpr (BITS == 4) *reinterpret_cast<uint4*>(dst) = make_uint4(q.word[0], q.word[1], q.word[2], q.word[3]);
-    else if constexpr (BITS == 2) *reinterpret_cast<uint2*>(dst) = make_uint2(q.word[0], q.word[1]);
-    else {
+    if (live) {
+        if constexpr (BITS == 4) *reinterpret_cast<uint4*>(dst) = make_uint4(q.word[0], q.word[1], q.word[2], q.word[3]);
+        else if constexpr (BITS == 2) *reinterpret_cast<uint2*>(dst) = make_uint2(q.word[0], q.word[1]);
+        else {
 #pragma unroll
-        for (int j = 0; j < BITS; ++j) dst[j] = q.word[j];
+            for (int j = 0; j < BITS; ++j) dst[j] = q.word[j];
+        }
     }
-    store_contig_tail<QJL>(p, row, quarter, q.signs, q.norm, q.rnorm);
+    store_contig_tail<QJL>(p, row, quarter, q.signs, q.norm, q.rnorm, live);
 }
 
 template <int BITS, bool QJL>
-__global__ void __launch_bounds__(kFastWarps * 32, 1) compress_contig_fast_kernel(const ContigParams p, int64_t n_groups) {
+__global__ void __launch_bounds__(kFastWarps * 32, 1) compress_contig_fast_kernel(const ContigParams p, int64_t n_units) {
     extern __shared__ __align__(128) unsigned char tables[];
     __shared__ float csm[1 << BITS];
     __shared__ int bad;
+    const int lane = threadIdx.x & 31, quarter = lane & 3, warp = threadIdx.x >> 5;
+    const bool mma = p.rotate && p.in_dtype != TQ_DTYPE_F32;
+    const uint32_t buf = ((smem_u32(tables) + kTableBytes + 255) & ~255u) + warp * kStagePerWarp;   // two buffers of 8 rows
+    const uint32_t dst = stage_at(buf, lane), src = staged_at(buf, lane);
+    // units of 8 rows; as in the paged kernel the last round is spread over all SMs, and the first copies go out first
+    int64_t unit = static_cast<int64_t>(warp) * gridDim.x + blockIdx.x;
+    const int64_t step = static_cast<int64_t>(gridDim.x) * kFastWarps;
+    auto row_of = [&](int64_t u) { return u * kItemsPerWarp + (lane >> 2); };
+    if (mma) {
+        stage_row(dst, p.x, row_of(unit) * kHeadDim + 8 * quarter, row_of(unit) < p.n);
+        stage_row(dst + kRowBuffer, p.x, row_of(unit + step) * kHeadDim + 8 * quarter, row_of(unit + step) < p.n);
+    }
     if (threadIdx.x == 0) bad = 0;
     if (threadIdx.x < (1 << BITS)) csm[threadIdx.x] = p.c ? p.c[threadIdx.x] : 0.f;
     __syncthreads();
-    build_table<BITS, QJL>(tables, p.b, p.c, &bad);
+    if (!mma) build_table<BITS, QJL>(tables, p.b, p.c, &bad);
+    else if constexpr (BITS > 2) build_table<BITS, QJL, true>(tables, p.b, p.c, &bad);
     __syncthreads();
-    const int lane = threadIdx.x & 31, quarter = lane & 3, warp = threadIdx.x >> 5;
-    const int64_t row0 = warp * kItemsPerWarp + (lane >> 2);   // + group * 128
     if (bad != 0) {   // two boundaries inside one cell: the generic quantizer
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
         const ContigParams pc = p;
-        for (int64_t grp = blockIdx.x; grp < n_groups; grp += gridDim.x)
-            compress_contig_rows<BITS, QJL ? OutMode::kPackedK : OutMode::kPackedV>(pc, grp * kFastItemsPerCta + row0, lane, csm);
+        for (; unit < n_units; unit += step)
+            compress_contig_rows<BITS, QJL ? OutMode::kPackedK : OutMode::kPackedV>(pc, row_of(unit), lane, csm);
         return;
     }
     constexpr uint32_t kBias = kMagicBits * static_cast<uint32_t>(kCellStride);   // modulo 2^32
     const uint32_t tab = smem_u32(tables) + (QJL ? (lane & 7) * 16 : (lane & 15) * 8) - kBias;
     Packed q;
-    if (p.rotate && p.in_dtype != TQ_DTYPE_F32) {
+    if (mma) {
         const bool bf16 = p.in_dtype == TQ_DTYPE_BF16;
-        uint4* buf = reinterpret_cast<uint4*>(tables + kTableBytes + warp * kStagePerWarp);   // two buffers of 128 uint4
         const WhtFragments hf = make_wht_fragments(lane, bf16);
-        int64_t grp = blockIdx.x;
-        const int64_t step = gridDim.x;
-        {
-            const int64_t r0 = grp * kFastItemsPerCta + row0, r1 = (grp + step) * kFastItemsPerCta + row0;
-            stage_row(buf, lane, p.x, r0 * kHeadDim + 32 * quarter, r0 < p.n);
-            stage_row(buf + 128, lane, p.x, r1 * kHeadDim + 32 * quarter, grp + step < n_groups && r1 < p.n);
-        }
-        int cur = 0;
-        for (; grp < n_groups; grp += step, cur ^= 1) {
-            const int64_t row = grp * kFastItemsPerCta + row0;
-            const int64_t nxt = (grp + 2 * step) * kFastItemsPerCta + row0;
-            const bool nxt_live = grp + 2 * step < n_groups && nxt < p.n;
-            uint4* b = buf + 128 * cur;
+        Codebook2<BITS> cb;
+        if constexpr (BITS == 2) cb.load(p.b, QJL ? p.c : nullptr);
+        uint32_t cur = 0;   // offset of the buffer whose turn it is
+        for (; unit < n_units; unit += step, cur ^= kRowBuffer) {
+            const int64_t row = row_of(unit), nxt = row_of(unit + 2 * step);
             wait_staged();
-            compress_row_mma<BITS, QJL, false, true>(smem_u32(b + lane), row < p.n, lane, bf16, hf, tab, q, [&] {
-                stage_row(b, lane, p.x, nxt * kHeadDim + 32 * quarter, nxt_live);
+            compress_row_mma<BITS, QJL, false, true>(src + cur, row < p.n, lane, bf16, hf, tab, cb, q, [&] {
+                stage_row(dst + cur, p.x, nxt * kHeadDim + 8 * quarter, nxt < p.n);
             });
-            if (row < p.n) store_contig_fast<BITS, QJL>(p, row, quarter, q);
+            store_contig_fast<BITS, QJL>(p, row, quarter, q);
         }
         asm volatile("cp.async.wait_group 0;" ::: "memory");
     } else {
         const bool rotate = p.rotate != 0;
         const float scale = rotate ? kWhtScale : 1.f, inv_scale = rotate ? 11.313708498984761f : 1.f;
-        for (int64_t grp = blockIdx.x; grp < n_groups; grp += gridDim.x) {
-            const int64_t row = grp * kFastItemsPerCta + row0;
+        for (; unit < n_units; unit += step) {
+            const int64_t row = row_of(unit);
             f2 y[16];
             fetch_plain(p.x, row * kHeadDim + 32 * quarter, row < p.n, p.in_dtype, rotate, lane, y);
             quantize_fast<BITS, QJL, false, true>(y, scale, inv_scale, tab, q);
-            if (row < p.n) store_contig_fast<BITS, QJL>(p, row, quarter, q);
+            store_contig_fast<BITS, QJL>(p, row, quarter, q);
         }
     }
 }
 
 template <int BITS, bool QJL>
 int launch_contig_fast(const ContigParams& p, cudaStream_t st) {
-    const int64_t n_groups = (p.n + kFastItemsPerCta - 1) / kFastItemsPerCta;
+    const int64_t n_units = (p.n + kItemsPerWarp - 1) / kItemsPerWarp;
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return TQ_ERR_LAUNCH;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return TQ_ERR_LAUNCH;
-    const unsigned grid = static_cast<unsigned>(n_groups < sms ? n_groups : sms);
-    constexpr int kSmem = kTableBytes + kFastWarps * kStagePerWarp;
+    const unsigned grid = static_cast<unsigned>(n_units < sms ? n_units : sms);
+    constexpr int kSmem = kTableBytes + kFastWarps * kStagePerWarp + 256;
     static bool configured[64] = {false};
     if (dev < 0 || dev >= 64 || !configured[dev]) {
         if (cudaFuncSetAttribute(compress_contig_fast_kernel<BITS, QJL>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) !=
@@ -688,7 +703,7 @@ int launch_contig_fast(const ContigParams& p, cudaStream_t st) {
             return TQ_ERR_LAUNCH;
         if (dev >= 0 && dev < 64) configured[dev] = true;
     }
-    compress_contig_fast_kernel<BITS, QJL><<<grid, kFastWarps * 32, kSmem, st>>>(p, n_groups);
+    compress_contig_fast_kernel<BITS, QJL><<<grid, kFastWarps * 32, kSmem, st>>>(p, n_units);
     return cudaGetLastError() == cudaSuccess ? TQ_OK : TQ_ERR_LAUNCH;
 }
 
@@ -709,9 +724,9 @@ int launch_paged_v(const PagedParams& p, int vb, bool qjl, cudaStream_t st) {
 
 template <OutMode MODE>
 int launch_contig(const ContigParams& p, int bits, cudaStream_t st) {
-    // large packed launches: the persistent table-driven kernel.  Measured on fp16 rows with the rotation: 16384
-    // rows 5.9 us (binary-search kernel) against 6.8 us, 32768 rows about 11 us either way, 65536 rows 22 against
-    // 15 us: below about two groups of 128 rows per SM the persistent kernel mostly builds its table.
+    // Large launches: the persistent table-driven kernel.  fp16 rows with the rotation, us, binary-search kernel / persistent:
+    // K 16384 rows 5.8 / 5.6, 32768 8.5 / 8.0, 65536 15.4 / 12.0; V 4.9 / 4.3, 7.0 / 5.8, 12.0 / 8.4.  The line stays above
+    // the crossing: the two rotations round differently.
     if (p.n > 2 * kSmallLaunchItems) {
         constexpr bool QJL = MODE == OutMode::kPackedK;
         switch (bits) {
@@ -781,6 +796,7 @@ extern "C" int tq_compress_paged(const void* key, const void* value, int in_dtyp
     p.vs_h = v_stride_head;
     p.num_slots = num_blocks * block_size;
     p.n_items = static_cast<int64_t>(n_tokens) * n_kv_heads;
+    p.n_tokens = n_tokens;
     p.Hkv = n_kv_heads;
     p.block_size = block_size;
     p.in_dtype = in_dtype;

@@ -14,12 +14,16 @@
 //  * element arithmetic two at a time: sm_100 f32x2 instructions (fma / mul / add / sub on register pairs) do
 //    the butterflies, the exactly rounded quotient u = x / (n + 1e-8) and the residual energy for two adjacent
 //    dims per instruction.
-//  * bucketize: u in [-1, 1] is mapped to one of 129 cells of width 1/64; no cell holds more than one
+//  * bucketize, 3- and 4-bit: u in [-1, 1] is mapped to one of 129 cells of width 1/64; no cell holds more than one
 //    boundary (checked when the table is built; Lloyd-Max boundaries for 128 dims are >= 0.022 apart).  The
 //    cell's table entry gives lo = #{boundaries below the cell}, and NB = -b * 2^126 for the boundary b inside
 //    the cell (-inf when there is none), so  t = sat(u * 2^126 + NB)  is exactly [u > b]  (ties stay down,
-//    as searchsorted(right=False)), and idx = lo + t.  The entry also carries c[lo] and c[lo+1], so the
-//    centroid is c[lo] (1 - t) + c[lo+1] t: two FMAs whose result is exactly one of the two.
+//    as searchsorted(right=False)), and idx = lo + t.  The entry also carries the centroids.
+//  * bucketize, 2-bit: the three comparisons directly, t_j = sat(u * 2^126 - b_j * 2^126), idx = t_0 + t_1 + t_2: about
+//    as many instructions as the table look-up, and none of its shared-memory traffic, which at 8 wavefronts (V) and
+//    16 (K) per element and four schedulers was half of what the data path of the SM can do.
+//  * where the rotation is done here (fp16 / bf16 rows), u = y * (1 / (n + 1e-8)) is a plain product, the centroid one FMA
+//    (c[lo] + t (c[lo+1] - c[lo])), and ||residual|| = n ||u - c|| is scaled once per vector.
 //  * packing: the four indices of a chunk of adjacent dims are combined by three FMAs into one float (one index
 //    per nibble, exact below 2^24) and converted once; residual signs are shifted in with funnel shifts.
 //  * rows are staged through shared memory with cp.async one group of items ahead of their use.
@@ -95,14 +99,16 @@ constexpr int kCellStride = 128;
 constexpr int kTableBytes = kCells * kCellStride;
 
 // Scans sorted boundaries for one cell.  Returns how many boundaries fall inside the cell.
-__device__ __forceinline__ int scan_cell(int cell, const float* __restrict__ b, int nb, int& lo, float& nbv) {
+template <int NB>
+__device__ __forceinline__ int scan_cell(int cell, const float* __restrict__ b, int& lo, float& nbv) {
     const float center = static_cast<float>(cell - kCellScale) * (1.f / kCellScale);
     const float half = 0.5f / kCellScale + 1.f / 1048576.f;   // rounding of the cell index is absorbed by the margin
     const float lo_e = center - half, hi_e = center + half;
     int inside = 0;
     float bin = 0.f;
     lo = 0;
-    for (int j = 0; j < nb; ++j) {
+#pragma unroll
+    for (int j = 0; j < NB; ++j) {
         const float bj = __ldg(b + j);
         lo += bj < lo_e ? 1 : 0;
         if (bj >= lo_e && bj <= hi_e) {
@@ -114,24 +120,35 @@ __device__ __forceinline__ int scan_cell(int cell, const float* __restrict__ b, 
     return inside;
 }
 
-template <int BITS, bool WIDE>
+// d with -c_lo + d == -c_hi in fp32: the rounded difference, or one of its neighbours.
+__device__ __forceinline__ float centroid_step(float c_lo, float c_hi) {
+    float d = c_lo - c_hi;
+    const float off = (d - c_lo) + c_hi;
+    if (off > 0.f) d = nextafterf(d, -INFINITY);
+    if (off < 0.f) d = nextafterf(d, INFINITY);
+    return d;
+}
+
+// Wide entries hold (NB, lo, c[lo], c[lo+1]), or, STEP, (NB, lo, -c[lo], c[lo] - c[lo+1]).  Four lanes write the 128 bytes
+// of a cell.
+template <int BITS, bool WIDE, bool STEP = false>
 __device__ void build_table(unsigned char* tab, const float* __restrict__ b, const float* __restrict__ c, int* bad) {
-    for (int cell = threadIdx.x; cell < kCells; cell += blockDim.x) {
+    const int lane = threadIdx.x & 31;
+    for (int cell = (threadIdx.x >> 5) * 8 + (lane >> 2); cell < kCells; cell += static_cast<int>(blockDim.x) / 4) {
         int lo;
         float nbv;
-        const int inside = scan_cell(cell, b, (1 << BITS) - 1, lo, nbv);
+        const int inside = scan_cell<(1 << BITS) - 1>(cell, b, lo, nbv);
         if (inside > 1) atomicOr(bad, 1);
+        float4* dst = reinterpret_cast<float4*>(tab + cell * kCellStride) + 2 * (lane & 3);
+        float4 e = make_float4(nbv, static_cast<float>(lo), nbv, static_cast<float>(lo));
         if constexpr (WIDE) {
             const float c_lo = __ldg(c + lo);
             const float c_hi = lo + 1 < (1 << BITS) ? __ldg(c + lo + 1) : c_lo;
-            const float4 e = make_float4(nbv, static_cast<float>(lo), c_lo, c_hi);
-#pragma unroll
-            for (int r = 0; r < 8; ++r) reinterpret_cast<float4*>(tab + cell * kCellStride)[r] = e;
-        } else {
-            const float2 e = make_float2(nbv, static_cast<float>(lo));
-#pragma unroll
-            for (int r = 0; r < 16; ++r) reinterpret_cast<float2*>(tab + cell * kCellStride)[r] = e;
+            e.z = STEP ? -c_lo : c_lo;
+            e.w = STEP ? centroid_step(c_lo, c_hi) : c_hi;
         }
+        dst[0] = e;
+        dst[1] = e;
     }
 }
 
@@ -225,6 +242,74 @@ __device__ __forceinline__ void quant_pair(f2 y, const VecConsts& vc, f2& rr, ui
         const float2 ea = lds64(addr_a), eb = lds64(addr_b);     // NB, lo
         kfa = ea.y + fma_sat(ua, kBig, ea.x);
         kfb = eb.y + fma_sat(ub, kBig, eb.x);
+    }
+}
+
+// The same for rows rotated here: u is the plain product, residuals are not yet multiplied by the norm.
+template <int BITS>
+struct Codebook2 {};   // 3 and 4 bits: everything is in the table
+template <>
+struct Codebook2<2> {
+    float nb[3];        // -b_j * 2^126
+    float nc[4];        // -c_0 and the steps from -c_(j-1) to -c_j
+    __device__ __forceinline__ void load(const float* __restrict__ b, const float* __restrict__ c) {
+#pragma unroll
+        for (int j = 0; j < 3; ++j) nb[j] = -(__ldg(b + j) * big());
+        if (c) {
+            nc[0] = -__ldg(c);
+#pragma unroll
+            for (int j = 1; j < 4; ++j) nc[j] = centroid_step(__ldg(c + j - 1), __ldg(c + j));
+        }
+    }
+};
+
+struct RowConsts {
+    f2 inv, inv64;
+    uint32_t tab;
+};
+
+template <int BITS, bool QJL>
+__device__ __forceinline__ void quant_pair_rotated(f2 y, const RowConsts& rc, const Codebook2<BITS>& cb, f2& ee, uint32_t& sacc, float& kfa,
+                                                   float& kfb) {
+    const float kBig = big();
+    const f2 u = f2mul(y, rc.inv);
+    float ua, ub, nca = 0.f, ncb = 0.f;   // minus the centroids
+    f2unpack(u, ua, ub);
+    if constexpr (BITS == 2) {
+        const float a0 = fma_sat(ua, kBig, cb.nb[0]), a1 = fma_sat(ua, kBig, cb.nb[1]), a2 = fma_sat(ua, kBig, cb.nb[2]);
+        const float b0 = fma_sat(ub, kBig, cb.nb[0]), b1 = fma_sat(ub, kBig, cb.nb[1]), b2 = fma_sat(ub, kBig, cb.nb[2]);
+        kfa = (a0 + a1) + a2;
+        kfb = (b0 + b1) + b2;
+        if constexpr (QJL) {
+            nca = fmaf(a2, cb.nc[3], fmaf(a1, cb.nc[2], fmaf(a0, cb.nc[1], cb.nc[0])));
+            ncb = fmaf(b2, cb.nc[3], fmaf(b1, cb.nc[2], fmaf(b0, cb.nc[1], cb.nc[0])));
+        }
+    } else {
+        const f2 cellf = f2fma(y, rc.inv64, f2dup(kMagic + kCellScale));   // low mantissa bits: round(scale u) + scale
+        float cfa, cfb;
+        f2unpack(cellf, cfa, cfb);
+        const uint32_t addr_a = __float_as_uint(cfa) * static_cast<uint32_t>(kCellStride) + rc.tab;
+        const uint32_t addr_b = __float_as_uint(cfb) * static_cast<uint32_t>(kCellStride) + rc.tab;
+        if constexpr (QJL) {
+            const float4 ea = lds128(addr_a), eb = lds128(addr_b);   // NB, lo, -c[lo], c[lo] - c[lo+1]
+            const float ta = fma_sat(ua, kBig, ea.x), tb = fma_sat(ub, kBig, eb.x);
+            nca = fmaf(ta, ea.w, ea.z);
+            ncb = fmaf(tb, eb.w, eb.z);
+            kfa = ea.y + ta;
+            kfb = eb.y + tb;
+        } else {
+            const float2 ea = lds64(addr_a), eb = lds64(addr_b);     // NB, lo
+            kfa = ea.y + fma_sat(ua, kBig, ea.x);
+            kfb = eb.y + fma_sat(ub, kBig, eb.x);
+        }
+    }
+    if constexpr (QJL) {
+        const f2 e = f2add(u, f2pack(nca, ncb));
+        ee = f2fma(e, e, ee);
+        float e0, e1;
+        f2unpack(e, e0, e1);
+        sacc = __funnelshift_l(__float_as_uint(e1), sacc, 1);
+        sacc = __funnelshift_l(__float_as_uint(e0), sacc, 1);
     }
 }
 
@@ -414,14 +499,14 @@ __device__ __forceinline__ void mma_zero(bool bf16, float (&d)[4], uint32_t a0, 
     else mma_16816_zero<false>(d, a0, a1, a2, a3, b0, b1);
 }
 
-// row: shared address of this lane's first 16-byte piece of a staged row (piece j is 512 bytes further).
+// row: staged_at(...) of this lane (piece j is at row ^ 16 j).
 __device__ __forceinline__ void read_staged(uint32_t row, bool live, uint32_t (&w)[16]) {
     if (live) {
 #pragma unroll
         for (int j = 0; j < 4; ++j)
             asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
                          : "=r"(w[4 * j]), "=r"(w[4 * j + 1]), "=r"(w[4 * j + 2]), "=r"(w[4 * j + 3])
-                         : "r"(row + 512 * j));
+                         : "r"(row ^ (16 * j)));
     } else {
 #pragma unroll
         for (int i = 0; i < 16; ++i) w[i] = 0u;
@@ -432,7 +517,7 @@ __device__ __forceinline__ void read_staged(uint32_t row, bool live, uint32_t (&
 // into the same buffer there).
 template <int BITS, bool QJL, bool ISV, bool CONTIG = false, class AfterRead>
 __device__ __forceinline__ void compress_row_mma(uint32_t row, bool live, int lane, bool bf16, const WhtFragments& hf,
-                                                 uint32_t tab, Packed& out, AfterRead after_read) {
+                                                 uint32_t tab, const Codebook2<BITS>& cb, Packed& out, AfterRead after_read) {
     constexpr float kStep = CONTIG ? static_cast<float>(1 << BITS) : 16.f;   // spacing of a chunk's four indices
     uint32_t w[16];
     read_staged(row, live, w);
@@ -456,19 +541,20 @@ __device__ __forceinline__ void compress_row_mma(uint32_t row, bool live, int la
     const float n = finite ? n_out : 0.f;
     const float den = (n + 1e-8f) * 11.313708498984761f;          // the unnormalised transform is sqrt(128) larger
     const float inv = __frcp_rn(den);
-    VecConsts vc;
-    vc.inv = f2dup(inv);
-    vc.nden = f2dup(-den);
-    vc.inv64 = f2dup(inv * kCellScale);
-    vc.n = f2dup(n);
-    vc.tab = tab;
+    RowConsts rc;
+    rc.inv = f2dup(inv);
+    rc.inv64 = f2dup(inv * kCellScale);
+    rc.tab = tab;
     float cv[8];
-    f2 rr = f2dup(0.f);
+    f2 ee = f2dup(0.f);
     uint32_t sg = 0u;   // bit l = 1 when the residual of local dim l is negative
 #pragma unroll
     for (int nt = 0; nt < 2; ++nt) {
         if (nt == 1 || !live) read_staged(row, live, w);
-        if (nt == 1) after_read();
+        if (nt == 1) {
+            __syncwarp();
+            after_read();
+        }
         f2 y[8];   // pair 2 j + r = dims 8 j + 4 nt + 2 r + {0, 1}
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -493,8 +579,8 @@ __device__ __forceinline__ void compress_row_mma(uint32_t row, bool live, int la
             const int c = 2 * j + nt;   // chunk of dims 4 c .. 4 c + 3
             float k0, k1, k2, k3;
             uint32_t nib = 0u;
-            quant_pair<QJL, false>(y[2 * j + 1], vc, rr, nib, k2, k3);
-            quant_pair<QJL, false>(y[2 * j], vc, rr, nib, k0, k1);
+            quant_pair_rotated<BITS, QJL>(y[2 * j + 1], rc, cb, ee, nib, k2, k3);
+            quant_pair_rotated<BITS, QJL>(y[2 * j], rc, cb, ee, nib, k0, k1);
             cv[c] = fmaf(fmaf(fmaf(k3, kStep, k2), kStep, k1), kStep, k0);
             if constexpr (QJL) sg |= nib << (4 * c);
         }
@@ -504,8 +590,8 @@ __device__ __forceinline__ void compress_row_mma(uint32_t row, bool live, int la
     if constexpr (QJL) {
         float ra, rb;
         out.signs = ~sg;
-        f2unpack(rr, ra, rb);
-        out.rnorm = sqrtf(group_sum(ra + rb));
+        f2unpack(ee, ra, rb);
+        out.rnorm = n * sqrtf(group_sum(ra + rb));
     } else {
         out.signs = 0u;
         out.rnorm = 0.f;
@@ -514,23 +600,38 @@ __device__ __forceinline__ void compress_row_mma(uint32_t row, bool live, int la
 }
 
 // ---- input staging (fp16 / bf16 rows): global -> shared with cp.async, one group of items ahead --------------
-// Every lane copies and later reads back only its own 64 bytes of a row, as four 16-byte pieces; piece i of lane
-// l sits at uint4 index 32 i + l of the warp's buffer, so both the copies and the reads are conflict-free.
+// The four lanes of a row copy 64 contiguous bytes per instruction (whole sectors: with each lane copying its own 64 bytes,
+// 16 at a time, every sector crossed from L2 twice) and read back 64 bytes each.  16-byte chunk c of row g sits at slot
+// c ^ (c >> 2) ^ 4 (g & 1) of the row's 256 bytes, so neither the copies nor the reads of a warp collide on a bank.
 constexpr int kStagePerWarp = 2 * 4 * 32 * 16;   // K and V rows of 8 items: 4 KB
+constexpr int kRowBuffer = kStagePerWarp / 2;    // on a 256-byte boundary
 
-__device__ __forceinline__ void stage_row(uint4* buf, int lane, const void* base, int64_t elem_off, bool live) {
+// Chunk 4 i + quarter of this lane's row is copied to stage_at ^ 0x50 i, chunk 4 quarter + j is read from staged_at ^ 0x10 j.
+__device__ __forceinline__ uint32_t stage_at(uint32_t buf, int lane) {
+    const int g = lane >> 2, quarter = lane & 3;
+    return buf + g * 256 + ((g & 1) << 6) + (quarter << 4);
+}
+__device__ __forceinline__ uint32_t staged_at(uint32_t buf, int lane) {
+    const int g = lane >> 2, quarter = lane & 3;
+    return buf + g * 256 + ((quarter ^ (g & 1)) << 6) + (quarter << 4);
+}
+
+// elem_off: of the row's first element plus 8 * quarter.  The lanes of the warp have read what the buffer held before.
+__device__ __forceinline__ void stage_row(uint32_t dst, const void* base, int64_t elem_off, bool live) {
     if (live) {
         const uint16_t* src = static_cast<const uint16_t*>(base) + elem_off;
 #pragma unroll
         for (int i = 0; i < 4; ++i)
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(buf + 32 * i + lane)), "l"(src + 8 * i)
-                         : "memory");
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst ^ (0x50 * i)), "l"(src + 32 * i) : "memory");
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
 }
 
-// Waits until at most one of this thread's copy groups is still in flight.
-__device__ __forceinline__ void wait_staged() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
+// Waits until at most one of the copy groups of each lane is still in flight.
+__device__ __forceinline__ void wait_staged() {
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncwarp();
+}
 
 // Loads this lane's 32 elements of one row and returns them as fp32 pairs, rotated when asked but not yet
 // scaled by 2^-3.5.  Path for fp32 inputs and for inputs that are already rotated.
@@ -583,6 +684,22 @@ __device__ __forceinline__ void store_v_fast(uint8_t* vpart, int t, int quarter,
     if (quarter == 0) reinterpret_cast<__half*>(vpart + 256 * BITS)[norm_slot(t)] = __float2half_rn(q.norm);
 }
 
+// The V fields of two lanes that hold neighbouring tokens of one 32-bit word (lane ^ 4, same quarter): the lane of the even
+// token writes the words of dim group 2 quarter, the other one those of 2 quarter + 1, so a warp's store instruction fills
+// whole 32-byte sectors (16-bit stores of single tokens cost 10 to 17 % of the kernel).
+template <int BITS>
+__device__ __forceinline__ void store_v_pair(uint8_t* vpart, int t, int quarter, const Packed& q, bool live) {
+    const int pair = t >> 1, half = t & 1;
+    uint8_t* dst = vpart + (pair * 8 + 2 * quarter + half) * 4;
+#pragma unroll
+    for (int j = 0; j < BITS; ++j) {
+        const uint32_t keep = half ? q.field[BITS + j] : q.field[j], give = half ? q.field[j] : q.field[BITS + j];
+        const uint32_t got = __shfl_xor_sync(0xffffffffu, give, 4);
+        if (live) *reinterpret_cast<uint32_t*>(dst + j * 256) = prmt(keep, got, half ? 0x1054u : 0x5410u);
+    }
+    if (live && quarter == 0) reinterpret_cast<__half*>(vpart + 256 * BITS)[norm_slot(t)] = __float2half_rn(q.norm);
+}
+
 // fp32 inputs and inputs that are already rotated: plain loads, shuffle WHT, the same table-driven quantizer.
 // Out of line so that its registers do not weigh on the tensor-core loop.
 template <int KB, int VB, bool QJL>
@@ -603,8 +720,29 @@ __device__ __noinline__ void compress_items_plain(const void* key, const void* v
 }
 
 // ---- kernel -----------------------------------------------------------------------------------------------
-// Persistent CTAs of 16 warps, one per SM: the two tables are built once per CTA, then the CTA strides over groups of 128
-// (token, head) items, 8 per warp, first the key then the value of each item.
+// Item order of the tensor-core loop: items 2 i and 2 i + 1 are two neighbouring tokens of one head (for store_v_pair);
+// with an odd token count the last partner is not live.
+__device__ __forceinline__ int64_t paired_items(const PagedParams& p) { return (p.n_tokens + 1) / 2 * 2 * p.Hkv; }
+__device__ __forceinline__ ItemId identify_paired(const PagedParams& p, int64_t item) {
+    ItemId id;
+    const int64_t two = item >> 1;
+    if (p.n_items <= 0x3fffffff) {
+        const uint32_t tp = static_cast<uint32_t>(two) / static_cast<uint32_t>(p.Hkv);
+        id.tok = 2 * tp;
+        id.head = static_cast<int>(static_cast<uint32_t>(two) - tp * static_cast<uint32_t>(p.Hkv));
+    } else {
+        const int64_t tp = two / p.Hkv;
+        id.tok = 2 * tp;
+        id.head = static_cast<int>(two - tp * p.Hkv);
+    }
+    id.tok += item & 1;
+    id.live = id.tok < p.n_tokens;
+    return id;
+}
+
+// Persistent CTAs of 16 warps, one per SM: the tables are built once per CTA, then its warps stride over units of 8 (token,
+// head) items, first the keys then the values of a unit.  Unit u belongs to warp u / gridDim of CTA u % gridDim: the last,
+// partly filled round is spread over all SMs (3001 tokens x 8 heads: 2 rounds of 16 warps per SM on 40 SMs otherwise).
 template <int KB, int VB, bool QJL>
 __global__ void __launch_bounds__(kFastWarps * 32, TQ_CMP_MINBLOCKS) compress_paged_fast_kernel(const PagedParams p, int64_t n_groups) {
     constexpr int PAGE = page_bytes(KB, VB, QJL ? 1 : 0);
@@ -612,63 +750,84 @@ __global__ void __launch_bounds__(kFastWarps * 32, TQ_CMP_MINBLOCKS) compress_pa
     extern __shared__ __align__(128) unsigned char tables[];
     __shared__ float csm[1 << KB];
     __shared__ int bad;
-    if (threadIdx.x == 0) bad = 0;
-    if (threadIdx.x < (1 << KB)) csm[threadIdx.x] = p.kc[threadIdx.x];
-    __syncthreads();
-    build_table<KB, QJL>(tables, p.kb, p.kc, &bad);
-    build_table<VB, false>(tables + kTableBytes, p.vb, nullptr, &bad);
-    __syncthreads();
-    const bool generic = bad != 0;
     const int lane = threadIdx.x & 31, quarter = lane & 3, warp = threadIdx.x >> 5;
     constexpr uint32_t kBias = kMagicBits * static_cast<uint32_t>(kCellStride);   // modulo 2^32
     const uint32_t ktab = smem_u32(tables) + (QJL ? (lane & 7) * 16 : (lane & 15) * 8) - kBias;
     const uint32_t vtab = smem_u32(tables + kTableBytes) + (lane & 15) * 8 - kBias;
-    const bool rotate = p.rotate != 0;
-    const int64_t item0 = warp * kItemsPerWarp + (lane >> 2);   // + group * 64
-    if (generic) {
-        const PagedParams pc = p;   // the out-of-line call takes an address: keep the kernel parameters themselves in the constant bank
-        for (int64_t grp = blockIdx.x; grp < n_groups; grp += gridDim.x)
-            compress_items_generic<KB, VB, QJL>(pc, grp * kFastItemsPerCta + item0, lane, csm);
+    const bool rotate = p.rotate != 0, mma = rotate && p.in_dtype != TQ_DTYPE_F32;
+
+    // Tensor-core path.  Rows are staged through shared memory one unit ahead: the key rows of the next unit are requested
+    // as soon as this unit's have been consumed by the MMAs, the value rows likewise, so every copy has a whole unit's
+    // arithmetic to hide behind.  The first ones are under way while the tables are built.
+    const uint32_t kbuf = ((smem_u32(tables) + 2 * kTableBytes + 255) & ~255u) + warp * kStagePerWarp, vbuf = kbuf + kRowBuffer;
+    const uint32_t kdst = stage_at(kbuf, lane), vdst = stage_at(vbuf, lane);
+    const int64_t units = (paired_items(p) + kItemsPerWarp - 1) / kItemsPerWarp;
+    const int64_t step = static_cast<int64_t>(gridDim.x) * kFastWarps;
+    int64_t unit = static_cast<int64_t>(warp) * gridDim.x + blockIdx.x;
+    ItemId id = identify_paired(p, unit * kItemsPerWarp + (lane >> 2));
+    if (mma) {
+        stage_row(kdst, p.key, id.tok * p.ks_t + id.head * p.ks_h + 8 * quarter, id.live);
+        stage_row(vdst, p.value, id.tok * p.vs_t + id.head * p.vs_h + 8 * quarter, id.live);
+    }
+    if (threadIdx.x == 0) bad = 0;
+    if (threadIdx.x < (1 << KB)) csm[threadIdx.x] = p.kc[threadIdx.x];
+    __syncthreads();
+    if (mma) {   // 2-bit codebooks need no table here
+        if constexpr (KB > 2) build_table<KB, QJL, true>(tables, p.kb, p.kc, &bad);
+        if constexpr (VB > 2) build_table<VB, false, true>(tables + kTableBytes, p.vb, nullptr, &bad);
+    } else {
+        build_table<KB, QJL>(tables, p.kb, p.kc, &bad);
+        build_table<VB, false>(tables + kTableBytes, p.vb, nullptr, &bad);
+    }
+    __syncthreads();
+    if (bad != 0 || !mma) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        const bool generic = bad != 0;
+        const int64_t item0 = warp * kItemsPerWarp + (lane >> 2);   // + group * 128
+        const PagedParams pc = p;   // the out-of-line calls take an address: keep the kernel parameters themselves in the constant bank
+        for (int64_t grp = blockIdx.x; grp < n_groups; grp += gridDim.x) {
+            if (generic) compress_items_generic<KB, VB, QJL>(pc, grp * kFastItemsPerCta + item0, lane, csm);
+            else
+                compress_items_plain<KB, VB, QJL>(p.key, p.value, p.ks_t, p.ks_h, p.vs_t, p.vs_h, p.in_dtype, rotate,
+                                                  place_item<PAGE>(p, grp * kFastItemsPerCta + item0, quarter), lane, ktab, vtab);
+        }
         return;
     }
+    const bool bf16 = p.in_dtype == TQ_DTYPE_BF16;
+    const uint32_t krow = staged_at(kbuf, lane), vrow = staged_at(vbuf, lane);
+    const WhtFragments hf = make_wht_fragments(lane, bf16);
+    Codebook2<KB> kcb;
+    Codebook2<VB> vcb;
+    if constexpr (KB == 2) kcb.load(p.kb, QJL ? p.kc : nullptr);
+    if constexpr (VB == 2) vcb.load(p.vb, nullptr);
     Packed q;
-    if (rotate && p.in_dtype != TQ_DTYPE_F32) {
-        // Tensor-core rotation.  Rows are staged through shared memory one group ahead: the key rows of the next
-        // group are requested as soon as this group's have been consumed by the MMAs, the value rows likewise,
-        // so every copy has a whole group's arithmetic to hide behind.
-        const bool bf16 = p.in_dtype == TQ_DTYPE_BF16;
-        uint4* kbuf = reinterpret_cast<uint4*>(tables + 2 * kTableBytes + warp * kStagePerWarp);
-        uint4* vbuf = kbuf + 128;
-        const uint32_t krow = smem_u32(kbuf + lane), vrow = smem_u32(vbuf + lane);
-        const WhtFragments hf = make_wht_fragments(lane, bf16);
-        // Only the identity (token, head) of the next group's item is carried across the loop body; where the
-        // current item goes in the cache is looked up when its turn comes.
-        int64_t grp = blockIdx.x;
-        ItemId id = identify_item(p, grp * kFastItemsPerCta + item0);
-        stage_row(kbuf, lane, p.key, id.tok * p.ks_t + id.head * p.ks_h + 32 * quarter, id.live);
-        stage_row(vbuf, lane, p.value, id.tok * p.vs_t + id.head * p.vs_h + 32 * quarter, id.live);
-        while (grp < n_groups) {
-            const ItemPlace w = place_item<PAGE>(p, id, quarter);
-            grp += gridDim.x;
-            id.live = false;
-            if (grp < n_groups) id = identify_item(p, grp * kFastItemsPerCta + item0);
-            wait_staged();
-            compress_row_mma<KB, QJL, false>(krow, w.live, lane, bf16, hf, ktab, q, [&] {
-                stage_row(kbuf, lane, p.key, id.tok * p.ks_t + id.head * p.ks_h + 32 * quarter, id.live);
-            });
-            if (w.live) store_k_fast<KB, QJL>(w.page, w.t, quarter, q);
-            wait_staged();
-            compress_row_mma<VB, false, true>(vrow, w.live, lane, bf16, hf, vtab, q, [&] {
-                stage_row(vbuf, lane, p.value, id.tok * p.vs_t + id.head * p.vs_h + 32 * quarter, id.live);
-            });
-            if (w.live) store_v_fast<VB>(w.page + KPART, w.t, quarter, q);
+    // Only the identity (token, head) of the next unit's item is carried across the loop body; where the current item
+    // goes in the cache is looked up when its turn comes.
+    while (unit < units) {
+        const ItemPlace w = place_item<PAGE>(p, id, quarter);
+        const unsigned long long at = reinterpret_cast<unsigned long long>(w.page);
+        const unsigned long long at_other = __shfl_xor_sync(0xffffffffu, at, 4);
+        const int t_other = __shfl_xor_sync(0xffffffffu, w.t, 4);
+        // both tokens of every pair in one word of one page, or neither of them stored (no page)
+        const bool pairs = __all_sync(0xffffffffu, at_other == at && (at == 0 || t_other == (w.t ^ 1)));
+        unit += step;
+        id = identify_paired(p, unit * kItemsPerWarp + (lane >> 2));
+        wait_staged();
+        compress_row_mma<KB, QJL, false>(krow, w.live, lane, bf16, hf, ktab, kcb, q, [&] {
+            stage_row(kdst, p.key, id.tok * p.ks_t + id.head * p.ks_h + 8 * quarter, id.live);
+        });
+        if (w.live) store_k_fast<KB, QJL>(w.page, w.t, quarter, q);
+        wait_staged();
+        compress_row_mma<VB, false, true>(vrow, w.live, lane, bf16, hf, vtab, vcb, q, [&] {
+            stage_row(vdst, p.value, id.tok * p.vs_t + id.head * p.vs_h + 8 * quarter, id.live);
+        });
+        if (pairs) {
+            store_v_pair<VB>(w.page + KPART, w.t, quarter, q, w.live);
+        } else if (w.live) {
+            store_v_fast<VB>(w.page + KPART, w.t, quarter, q);
         }
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-    } else {
-        for (int64_t grp = blockIdx.x; grp < n_groups; grp += gridDim.x)
-            compress_items_plain<KB, VB, QJL>(p.key, p.value, p.ks_t, p.ks_h, p.vs_t, p.vs_h, p.in_dtype, rotate,
-                                              place_item<PAGE>(p, grp * kFastItemsPerCta + item0, quarter), lane, ktab, vtab);
     }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
 // Small launches (the new tokens of one decode step): no tables to build, one group of 32 items per CTA.
@@ -682,7 +841,10 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) compress_paged_small_kernel
     compress_items_generic<KB, VB, QJL>(p, item, lane, csm);
 }
 
-constexpr int64_t kSmallLaunchItems = 16384;   // below this the table set-up and the 512-thread CTAs of the fast kernel cost more than they save
+// Up to here launches take the generic kernel, whose rotation is the plain butterfly.  The tensor-core kernel is a little faster
+// at these sizes too (turbo3, 8 KV heads, 64 tokens 5.5 us against 6.4, 2048 tokens 8.5 against 11.3), but its rotation
+// rounds differently, and a coordinate in a million would go to the neighbouring centroid.
+constexpr int64_t kSmallLaunchItems = 16384;
 
 template <int KB, int VB, bool QJL>
 int launch_paged_tc(const PagedParams& p, cudaStream_t st);   // tq_compress_tc.cuh
@@ -697,7 +859,7 @@ int launch_paged_fast(const PagedParams& p, cudaStream_t st) {
     // on request: fp16 / bf16 rows that still need the rotation go to the tensor-memory kernel (rotation as one
     // 128 x 128 x 128 product per 128 rows, one thread per vector afterwards)
     if (p.rotate && p.in_dtype != TQ_DTYPE_F32 && p.use_tcgen05) return launch_paged_tc<KB, VB, QJL>(p, st);
-    const int64_t n_groups = (p.n_items + kFastItemsPerCta - 1) / kFastItemsPerCta;
+    const int64_t n_groups = (p.n_items + kFastItemsPerCta - 1) / kFastItemsPerCta, n_units = (p.n_items + kItemsPerWarp - 1) / kItemsPerWarp;
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return TQ_ERR_LAUNCH;
     static int sm_count[64] = {0};
@@ -707,8 +869,8 @@ int launch_paged_fast(const PagedParams& p, cudaStream_t st) {
         if (dev >= 0 && dev < 64) sm_count[dev] = sms;
     }
     const int64_t resident = static_cast<int64_t>(sms) * TQ_CMP_MINBLOCKS;
-    const unsigned grid = static_cast<unsigned>(n_groups < resident ? n_groups : resident);
-    constexpr int kSmem = 2 * kTableBytes + kFastWarps * kStagePerWarp;
+    const unsigned grid = static_cast<unsigned>(n_units < resident ? n_units : resident);
+    constexpr int kSmem = 2 * kTableBytes + kFastWarps * kStagePerWarp + 256;
     static bool configured[64] = {false};
     if (dev < 0 || dev >= 64 || !configured[dev]) {
         if (cudaFuncSetAttribute(compress_paged_fast_kernel<KB, VB, QJL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
