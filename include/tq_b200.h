@@ -214,11 +214,11 @@ int tq_polarquant_compress(const void* x, int in_dtype, int64_t n, const float* 
                            int64_t* indices, float* norms, float* k_mse_rot, float* signs, float* rnorm,
                            tq_stream_t stream);
 
-/* Bytes of workspace tq_packed_attention needs for a split count.  Host only. */
+/* Bytes of workspace tq_packed_attention needs for a split count, 0 included.  Host only. */
 int64_t tq_packed_attention_workspace_bytes(int BH, int num_splits);
 
-/* Split count tq_packed_attention picks when num_splits = 0; replaces the
- * MI355X tuning table of _get_config (packed_attention.py:236-267).  Host only. */
+/* About how many CTAs share a row when num_splits = 0; replaces the MI355X
+ * tuning table of _get_config (packed_attention.py:236-267).  Host only. */
 int tq_packed_attention_auto_splits(int BH, int Sk);
 
 /* packed_attention (turboquant/kernels/packed_attention.py:290-344):

@@ -127,3 +127,22 @@ def test_declined_inputs_behave_as_before():
         again = paged_decode_attention(q, cache, tables, lens, books, 16, chunk_pages=1, sm_scale=1 / math.sqrt(128))
     side.synchronize()
     assert (again.float() - want.float()).abs().max() <= 2e-3
+
+
+@pytest.mark.parametrize("bits", [2, 3, 4])
+@pytest.mark.parametrize("BH,Sk", [(1, 1), (3, 15), (2, 257), (5, 8192), (37, 1100), (150, 300), (301, 40), (149, 513)])
+def test_packed_attention_work_sharing(bits, BH, Sk):
+    """Rows cut by the even sharing of steps over CTAs, whole rows, several rows per CTA, tails of a step: the result of
+    explicit splits, which is held to the oracle elsewhere.  Weights, values and sums are fp32 on both sides, in another
+    order (2^-24 times the number of tokens, at worst); the output is rounded to fp16."""
+    c, b = make_codebook(128, bits, device=DEV)
+    g = torch.Generator(device=DEV).manual_seed(BH + Sk)
+    r = lambda w: torch.randint(0, 256, (BH, Sk, w), generator=g, dtype=torch.uint8, device=DEV)
+    norm = lambda lo, hi: (torch.rand(BH, Sk, generator=g, device=DEV) * (hi - lo) + lo).half()
+    q = torch.randn(BH, 128, generator=g, device=DEV).half()
+    args = (q, q, r(16 * bits), r(16), norm(0, 3), norm(8, 12), r(16 * bits), norm(8, 12), c, 0.0098)
+    got = packed_attention(*args).float()
+    for splits in (1, 3):
+        want = packed_attention(*args, num_splits=splits).float()
+        # logits reach |q| |k| ~ 11 * 12: their own rounding, 2^-24 * 132 * log2(e), moves a weight by 2^-16 of itself
+        assert ((got - want).abs() <= 2.0 ** -10 * want.abs() + (2.0 ** -15 + Sk * 2.0 ** -24) * 12 * c.abs().max()).all()

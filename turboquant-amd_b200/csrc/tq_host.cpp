@@ -37,7 +37,6 @@ struct Library {
     decltype(&tq_compress_v) compress_v;
     decltype(&tq_polarquant_compress) polarquant;
     decltype(&tq_packed_attention_workspace_bytes) attention_workspace_bytes;
-    decltype(&tq_packed_attention_auto_splits) attention_auto_splits;
     decltype(&tq_packed_attention) packed_attention;
 };
 Library L = {};
@@ -376,8 +375,7 @@ PyObject* packed_attention(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     }
     const at::Device dev = t[0]->device();
     const c10::cuda::CUDAGuard guard(dev);
-    if (splits <= 0) splits = L.attention_auto_splits(int(BH), int(Sk));
-    splits = std::max<long long>(1, std::min<long long>(splits, Sk));
+    splits = std::max<long long>(0, std::min<long long>(splits, Sk));   // 0: the library shares the work out
     const int64_t bytes = L.attention_workspace_bytes(int(BH), int(splits));
     at::DataPtr workspace = c10::cuda::CUDACachingAllocator::get()->allocate(std::max<int64_t>(bytes, 16));   // this call's only
     at::Tensor out = empty({BH, 128}, at::kHalf, dev);
@@ -430,7 +428,6 @@ PyObject* bind(PyObject*, PyObject* args) {
     take(L.compress_v, "tq_compress_v");
     take(L.polarquant, "tq_polarquant_compress");
     take(L.attention_workspace_bytes, "tq_packed_attention_workspace_bytes");
-    take(L.attention_auto_splits, "tq_packed_attention_auto_splits");
     take(L.packed_attention, "tq_packed_attention");
     if (!ok) {
         PyErr_Format(PyExc_RuntimeError, "%s lacks a tq_* entry point", path);

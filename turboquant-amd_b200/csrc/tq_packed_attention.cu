@@ -7,23 +7,22 @@
 // (turboquant/kernels/packed_compress.py:180-216) and separate fp16 norm arrays.
 // With one query per K/V stream there is no group to share tensor-core tiles, so
 // this kernel is CUDA-core code built around conflict-free shared-memory tables:
-//  * a warp takes 8 tokens per step, lane = 4 * slot + quarter: the lane reads the quarter's index words of its
-//    token (the warp's loads cover 8 whole rows) and keeps the quarter's 32 query values in registers;
-//  * pair table: (c[i0], c[i1]) as two floats for every pair of indices, one copy per lane (entry stride 256 B), so a
-//    64-bit load per two adjacent dims never collides on a bank; K scores and the V sum use f32x2 multiply-adds;
+//  * a warp takes 16 tokens per step, lane = 4 * slot + quarter: the lane reads the quarter's index words of its two
+//    tokens and keeps the quarter's 32 query values in registers;
+//  * pair table: (c[i0], c[i1]) for every pair of indices, one copy per lane, as two floats for V and as half2 for K (the
+//    operands of the score MMAs), so a load per two adjacent dims never collides on a bank;
 //  * sign table of the query: for each of a quarter's 8 sign nibbles the 16 sums of +-q' over its 4 dims, one copy
 //    per lane; the QJL term is 8 look-ups per lane instead of 32 selects;
 //  * every slot runs its own online softmax over the tokens it sees (no shuffles across tokens in the loop, the
-//    maximum is only raised when a score exceeds it by 2^8); slots, warps and splits are merged at the end.
+//    maximum is only raised when a score exceeds it by 2^8); slots, warps and CTAs are merged at the end.
 #include "tq_common.cuh"
 
 namespace tq {
 namespace {
 
-// Warps per CTA: 8 (two CTAs per SM, so that one CTA's table set-up and final merge overlap the other's token loop)
-// where two sets of tables fit in shared memory, 16 (one CTA per SM) for 4-bit indices.  Either way 16 warps per SM at
-// up to 128 registers per thread.
-template <int BITS> struct PAWarps { static constexpr int value = BITS == 4 ? 16 : 8; };
+constexpr int kPaWarps = 16;                    // one CTA per SM; up to 128 registers per thread
+constexpr int kPaThreads = kPaWarps * 32;
+constexpr int kStepTokens = kPaWarps * 16;      // tokens of one step of the CTA, 16 per warp
 constexpr int kSignTabBytes = 8 * 16 * 128;     // [nibble position][nibble value][lane]
 constexpr float kLog2e = 1.4426950408889634f;
 
@@ -37,11 +36,12 @@ struct PAParams {
     const uint8_t* v_idx;
     const __half* v_norm;
     const float* centroids;
-    float* ws_acc;   // [BH, splits, 128]
-    float* ws_lse;   // [BH, splits, 2]  (max in the log2 domain, sum)
+    float* ws_acc;   // [slots, 128]
+    float2* ws_lse;  // [slots] (max in the log2 domain, sum)
     __half* out;
     float corr_scale;
-    int Sk, num_splits;
+    int BH, Sk;
+    int num_splits;  // > 0: rows are cut into that many parts (slot row * num_splits + part); 0: the CTAs share all steps evenly
 };
 
 typedef unsigned long long pa_f2;   // two fp32 in a 64-bit register (sm_100 f32x2 arithmetic)
@@ -104,7 +104,27 @@ __device__ __forceinline__ void lds_words(uint32_t addr, uint32_t (&w)[BITS]) {
     }
 }
 
-constexpr int kPaStages = 2;   // ring of 16-token steps per warp: the one being worked on, the others in flight
+// Programmatic dependent launch of the merge kernel: its CTAs start while the partial kernel drains.  (The partial kernel is
+// launched without it: CTAs that start early are packed two to an SM next to those still running, and stay there.)
+__device__ __forceinline__ void pa_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pa_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <typename Kernel, typename... Args>
+bool pa_launch(Kernel kernel, bool chained, unsigned grid, unsigned block, size_t smem, cudaStream_t stream, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = chained ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, args...) == cudaSuccess;
+}
+
+constexpr int kPaStages = 2;   // ring of 16-token steps per warp: the one being worked on, the other in flight
 
 template <int BITS>
 struct PALayout {
@@ -115,10 +135,7 @@ struct PALayout {
     static constexpr int kSignTabOff = kPairTabBytes + kHalfTabBytes;
     static constexpr int kStageOff = kSignTabOff + kSignTabBytes;
     static constexpr int kStageBytes = 32 * kRow + 256;                 // 16 K rows, 16 V rows, 16 sign rows
-    static constexpr int kWarps = PAWarps<BITS>::value;
-    static constexpr int kThreads = kWarps * 32;
-    static constexpr int kStepTokens = kWarps * 16;                     // tokens one step of the whole CTA covers
-    static constexpr int kSmem = kStageOff + kWarps * kPaStages * kStageBytes;
+    static constexpr int kSmem = kStageOff + kPaWarps * kPaStages * kStageBytes;
 };
 
 // A warp takes 16 tokens per step.  Lane (slot, quarter) = (lane >> 2, lane & 3) owns quarter `quarter` (32 dims) of
@@ -129,38 +146,69 @@ struct PALayout {
 //  * QJL term: per quarter, 8 look-ups in the query's sign table;
 //  * V: per token 16 look-ups of (c[i0], c[i1]) as floats, f32x2 multiply-adds into the lane's 32 accumulators.
 // Every slot runs its own online softmax (no exchange between tokens inside the loop).
+//
+// Work: with num_splits = 0 the steps of all rows, laid end to end, are shared evenly by the CTAs of one wave; a CTA writes
+// the result of a row that lies inside its share, and leaves at most two partials (slot 2 c + 1: the row starts in the
+// share, 2 c: it does not).  A row costs a sign table and a merge wherever it is cut, so cutting rows into equal parts
+// until they fill whole waves cost 15 % of the largest shapes.  (Staging by bulk copies was slower than the cp.async pieces
+// below: 122 us with three copies per warp and step, 107 with three per CTA and step, against 98 on 64 x 32768, 3-bit.)
+struct Segment {   // part of a row
+    int row, tok, end;   // tokens [tok, end)
+    int slot;            // of its partial; -1: the whole row
+};
+
 template <int BITS>
-__global__ void __launch_bounds__(PAWarps<BITS>::value * 32, 16 / PAWarps<BITS>::value) packed_attn_partial(const PAParams p, int n_items) {
+__global__ void __launch_bounds__(kPaThreads, 1) packed_attn_partial(const PAParams p, int n_items) {
     using LO = PALayout<BITS>;
     constexpr int ROW = LO::kRow;
-    constexpr int kPaWarps = LO::kWarps, kThreads = LO::kThreads, kStepTokens = LO::kStepTokens;
     extern __shared__ __align__(128) unsigned char pa_smem[];
     unsigned char* pair_tab = pa_smem;
     unsigned char* half_tab = pa_smem + LO::kPairTabBytes;
     unsigned char* sign_tab = pa_smem + LO::kSignTabOff;        // [nibble position][value][lane] float
     __shared__ __align__(16) float sqp[kHeadDim];
-    __shared__ float scb[1 << BITS];
     __shared__ __align__(16) float sacc[kPaWarps][kHeadDim];
     __shared__ float sml[kPaWarps][2];
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int slot = lane >> 2, quarter = lane & 3;
-    const int per = (p.Sk + p.num_splits - 1) / p.num_splits;   // tokens per split (packed_attention.py:98-100)
-    // the pair tables depend on the codebook only: built once, the CTA then strides over (row, split) items
-    if (tid < (1 << BITS)) scb[tid] = p.centroids[tid];
-    __syncthreads();
-    for (int e = tid; e < LO::kPairs * 32; e += kThreads) {
-        const int pr = e >> 5;
-        const float c0 = scb[pr & ((1 << BITS) - 1)], c1 = scb[pr >> BITS];
-        *reinterpret_cast<float2*>(pair_tab + e * 8) = make_float2(c0, c1);
-        *reinterpret_cast<uint32_t*>(half_tab + e * 4) = pack_half2(c0, c1);
-    }
-    // ---- item state: which (row, split) the CTA works on, and the warp's asynchronous staging of it: per step a warp
+    pa_release();
+
+    // ---- the CTA's segments ----
+    const int steps = (p.Sk + kStepTokens - 1) / kStepTokens;   // per row
+    const int64_t total = static_cast<int64_t>(p.BH) * steps;
+    const int64_t u0 = total * blockIdx.x / gridDim.x, u1 = total * (blockIdx.x + 1) / gridDim.x;
+    const int per = p.num_splits > 0 ? (p.Sk + p.num_splits - 1) / p.num_splits : 0;   // tokens per split (packed_attention.py:98-100)
+    auto segment = [&](int64_t at) -> Segment {                 // the segment that starts at step `at`, or item `at`
+        Segment g;
+        if (p.num_splits > 0) {
+            g.row = static_cast<int>(at / p.num_splits);
+            const int part = static_cast<int>(at - static_cast<int64_t>(g.row) * p.num_splits);
+            g.tok = min(part * per, p.Sk);
+            g.end = min(g.tok + per, p.Sk);
+            g.slot = p.num_splits == 1 ? -1 : static_cast<int>(at);
+        } else {
+            g.row = static_cast<int>(at / steps);
+            const int k = static_cast<int>(at - static_cast<int64_t>(g.row) * steps);
+            const int64_t left = u1 - at;
+            g.tok = k * kStepTokens;
+            g.end = left < steps - k ? g.tok + static_cast<int>(left) * kStepTokens : p.Sk;
+            g.slot = k == 0 && g.end == p.Sk ? -1 : 2 * static_cast<int>(blockIdx.x) + (k == 0 ? 1 : 0);
+        }
+        return g;
+    };
+    auto after = [&](int64_t at, const Segment& g) -> int64_t { // where the next segment starts; past `stop`: there is none
+        return p.num_splits > 0 ? at + gridDim.x : at + (g.end - g.tok + kStepTokens - 1) / kStepTokens;
+    };
+    int64_t at = p.num_splits > 0 ? static_cast<int64_t>(blockIdx.x) : u0;
+    const int64_t stop = p.num_splits > 0 ? static_cast<int64_t>(n_items) : u1;
+    if (at >= stop) return;
+
+    // ---- item state: which segment the CTA works on, and the warp's asynchronous staging of it: per step a warp
     // copies its 16 K rows, 16 V rows and 16 sign rows in 16-byte pieces (every row is a multiple of 16 bytes, so any
     // token starts on a 16-byte boundary) ----
     const uint32_t stage0 = smem_u32(pa_smem + LO::kStageOff + warp * kPaStages * LO::kStageBytes);
-    int bh = 0, split = 0, t1 = 0;
-    int tok16 = 0;                                              // first token of this warp's current step
+    Segment seg;
+    int t1 = 0, tok16 = 0;                                      // end of the segment, first token of this warp's current step
     const uint8_t *kptr = nullptr, *vptr = nullptr, *sptr = nullptr;
     const uint16_t *knp = nullptr, *krnp = nullptr, *vnp = nullptr;
     int tok_issue = 0, stage_issue = 0;
@@ -200,15 +248,13 @@ __global__ void __launch_bounds__(PAWarps<BITS>::value * 32, 16 / PAWarps<BITS>:
             }
         }
     };
-    // Starts an item: its first copies and norms are requested here, i.e. (from the second item on) before the merge of
-    // the item just finished, so their latency is hidden behind it.
-    auto begin_item = [&](int item) {
-        bh = item / p.num_splits;
-        split = item - bh * p.num_splits;
-        const int t0 = min(split * per, p.Sk);
-        t1 = min(t0 + per, p.Sk);
-        const int64_t base = static_cast<int64_t>(bh) * p.Sk;
-        tok16 = t0 + warp * 16;
+    // Starts a segment: its first copies and norms are requested here, i.e. (from the second one on) before the merge of
+    // the one just finished, so their latency is hidden behind it.
+    auto begin = [&](int64_t from) {
+        seg = segment(from);
+        t1 = seg.end;
+        const int64_t base = static_cast<int64_t>(seg.row) * p.Sk;
+        tok16 = seg.tok + warp * 16;
         kptr = p.k_idx + (base + tok16) * ROW + lane * 16;
         vptr = p.v_idx + (base + tok16) * ROW + lane * 16;
         sptr = p.k_signs + (base + tok16) * 16 + lane * 16;
@@ -221,194 +267,252 @@ __global__ void __launch_bounds__(PAWarps<BITS>::value * 32, 16 / PAWarps<BITS>:
         for (int i = 0; i < kPaStages - 1; ++i) issue();
         load_norms(tok16, nrm);
     };
-    int item = blockIdx.x;
-    if (item < n_items) begin_item(item);
-  while (item < n_items) {
-    // B operands: the query's quarter `quarter` as loaded (pairs of adjacent dims), in column 0 (slot 0) only
-    uint32_t qf[16];
+    begin(at);
+
+    // the pair tables depend on the codebook only.  Every lane holds one centroid; an entry's two come by shuffle.
     {
-        const uint4* qsrc = reinterpret_cast<const uint4*>(p.Q + static_cast<int64_t>(bh) * kHeadDim + 32 * quarter);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const uint4 v = slot == 0 ? __ldg(qsrc + i) : make_uint4(0u, 0u, 0u, 0u);
-            qf[4 * i] = v.x; qf[4 * i + 1] = v.y; qf[4 * i + 2] = v.z; qf[4 * i + 3] = v.w;
+        const float cv = __ldg(p.centroids + (lane & ((1 << BITS) - 1)));
+#pragma unroll 4
+        for (int pr = warp; pr < LO::kPairs; pr += kPaWarps) {
+            const float c0 = __shfl_sync(0xffffffffu, cv, pr & ((1 << BITS) - 1)), c1 = __shfl_sync(0xffffffffu, cv, pr >> BITS);
+            *reinterpret_cast<float2*>(pair_tab + (pr * 32 + lane) * 8) = make_float2(c0, c1);
+            *reinterpret_cast<uint32_t*>(half_tab + (pr * 32 + lane) * 4) = pack_half2(c0, c1);
         }
     }
-    // ---- the query's sign table ----
-    if (tid < kHeadDim) sqp[tid] = __half2float(p.Qp[static_cast<int64_t>(bh) * kHeadDim + tid]) * p.corr_scale;
-    __syncthreads();
-    // Sign nibble g = 2 c + h of a lane's sign word (byte c = byte `quarter` of sign word c) holds, in bit kk, the
-    // sign of local dim 4 (4 h + kk) + c (stride-4 order: dim 4 i + c is bit i of word c).
-    for (int e = tid; e < 8 * 16 * 32; e += kThreads) {
-        const int ln = e & 31, v = (e >> 5) & 15, g = e >> 9, c = g >> 1, h = g & 1, q = ln & 3;
-        float acc = 0.f;
-#pragma unroll
-        for (int kk = 0; kk < 4; ++kk) {
-            const float x = sqp[32 * q + 4 * (4 * h + kk) + c];
-            acc += ((v >> kk) & 1) ? x : -x;
-        }
-        *reinterpret_cast<float*>(sign_tab + e * 4) = acc;
-    }
-    __syncthreads();
     const uint32_t lane8 = lane * 8, lane4 = lane * 4;
     // selector that gathers byte `quarter` of two sign words
     const uint32_t sel_lo = static_cast<uint32_t>(quarter) | (static_cast<uint32_t>(4 + quarter) << 4);
     const uint32_t my_words = stage0 + lane * (4 * BITS);       // this lane's K words of token A inside a stage
     const uint32_t my_signs = stage0 + 32 * ROW + slot * 16;
 
-    float m_run = -INFINITY, l_run = 0.f;     // this slot's online softmax (log2 domain)
-    pa_f2 acc[16];
-#pragma unroll
-    for (int j = 0; j < 16; ++j) acc[j] = pa_pack(0.f, 0.f);
-
-    int stage = 0;
-    for (; tok16 < t1; tok16 += kStepTokens) {
-        const bool valid_a = tok16 + slot < t1, valid_b = tok16 + slot + 8 < t1;
-        issue();
-        uint16_t nrm_n[6];
-        load_norms(tok16 + kStepTokens, nrm_n);
-        asm volatile("cp.async.wait_group %0;" ::"n"(kPaStages - 1) : "memory");
-        __syncwarp();
-        const uint32_t so = stage * LO::kStageBytes;
-        uint32_t kwa[BITS], kwb[BITS];
-        lds_words<BITS>(my_words + so, kwa);
-        lds_words<BITS>(my_words + so + 8 * ROW, kwb);
-        uint4 sga, sgb;
-        asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(sga.x), "=r"(sga.y), "=r"(sga.z), "=r"(sga.w) : "r"(my_signs + so));
-        asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(sgb.x), "=r"(sgb.y), "=r"(sgb.z), "=r"(sgb.w) : "r"(my_signs + so + 128));
-        // ---- K scores: rows = the 16 tokens, column 0 = the query ----
-        float mse[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-        for (int ks = 0; ks < 8; ++ks) {
-            const uint32_t a0 = *reinterpret_cast<const uint32_t*>(half_tab + pair_offset<BITS, 7>(kwa, 2 * ks, lane4));
-            const uint32_t a1 = *reinterpret_cast<const uint32_t*>(half_tab + pair_offset<BITS, 7>(kwb, 2 * ks, lane4));
-            const uint32_t a2 = *reinterpret_cast<const uint32_t*>(half_tab + pair_offset<BITS, 7>(kwa, 2 * ks + 1, lane4));
-            const uint32_t a3 = *reinterpret_cast<const uint32_t*>(half_tab + pair_offset<BITS, 7>(kwb, 2 * ks + 1, lane4));
-            mma_f16_16816(mse, a0, a1, a2, a3, qf[2 * ks], qf[2 * ks + 1]);
-        }
-        // ---- QJL term of this lane's quarter, both tokens ----
-        const uint32_t swa = prmt(prmt(sga.x, sga.y, sel_lo), prmt(sga.z, sga.w, sel_lo), 0x5410);
-        const uint32_t swb = prmt(prmt(sgb.x, sgb.y, sel_lo), prmt(sgb.z, sgb.w, sel_lo), 0x5410);
-        float qja = 0.f, qjb = 0.f;
-#pragma unroll
-        for (int g = 0; g < 8; ++g) {
-            const uint32_t xa = 4 * g >= 7 ? (swa >> (4 * g - 7)) : (swa << (7 - 4 * g));
-            const uint32_t xb = 4 * g >= 7 ? (swb >> (4 * g - 7)) : (swb << (7 - 4 * g));
-            qja += *reinterpret_cast<const float*>(sign_tab + g * 2048 + ((xa & (15u << 7)) | lane4));
-            qjb += *reinterpret_cast<const float*>(sign_tab + g * 2048 + ((xb & (15u << 7)) | lane4));
-        }
-        // the quarter-0 lane of a slot holds the whole MSE dot product (column 0 of rows slot and slot + 8)
-        float pa = __half2float(__ushort_as_half(nrm[1])) * qja, pb = __half2float(__ushort_as_half(nrm[4])) * qjb;
-        if (quarter == 0) {
-            pa = fmaf(__half2float(__ushort_as_half(nrm[0])), mse[0], pa);
-            pb = fmaf(__half2float(__ushort_as_half(nrm[3])), mse[2], pb);
-        }
-        pa += __shfl_xor_sync(0xffffffffu, pa, 1);
-        pb += __shfl_xor_sync(0xffffffffu, pb, 1);
-        pa += __shfl_xor_sync(0xffffffffu, pa, 2);
-        pb += __shfl_xor_sync(0xffffffffu, pb, 2);
-        const float sa = valid_a ? pa * kLog2e : -INFINITY, sb = valid_b ? pb * kLog2e : -INFINITY;
-        // ---- online softmax of this slot: the maximum is raised only when a score exceeds it by 2^8 ----
-        const float smax = fmaxf(sa, sb);
-        if (smax > m_run + 8.f) {
-            const float alpha = pa_ex2(m_run - smax);     // 0 on the first token
-            const pa_f2 al2 = pa_pack(alpha, alpha);
-            l_run *= alpha;
-#pragma unroll
-            for (int j = 0; j < 16; ++j) acc[j] = pa_mul(acc[j], al2);
-            m_run = smax;
-        }
-        const float pra = valid_a ? pa_ex2(sa - m_run) : 0.f, prb = valid_b ? pa_ex2(sb - m_run) : 0.f;
-        l_run += pra + prb;
-        // ---- V ----
+    while (at < stop) {
+        // B operands: the query's quarter `quarter` as loaded (pairs of adjacent dims), in column 0 (slot 0) only
+        uint32_t qf[16];
         {
-            uint32_t vw[BITS];
-            lds_words<BITS>(my_words + so + 16 * ROW, vw);
-            const float wv = pra * __half2float(__ushort_as_half(nrm[2]));
-            const pa_f2 wv2 = pa_pack(wv, wv);
+            const uint4* qsrc = reinterpret_cast<const uint4*>(p.Q + static_cast<int64_t>(seg.row) * kHeadDim + 32 * quarter);
 #pragma unroll
-            for (int j = 0; j < 16; ++j)
-                acc[j] = pa_fma(wv2, *reinterpret_cast<const pa_f2*>(pair_tab + pair_offset<BITS, 8>(vw, j, lane8)), acc[j]);
+            for (int i = 0; i < 4; ++i) {
+                const uint4 v = slot == 0 ? __ldg(qsrc + i) : make_uint4(0u, 0u, 0u, 0u);
+                qf[4 * i] = v.x; qf[4 * i + 1] = v.y; qf[4 * i + 2] = v.z; qf[4 * i + 3] = v.w;
+            }
         }
-        {
-            uint32_t vw[BITS];
-            lds_words<BITS>(my_words + so + 24 * ROW, vw);
-            const float wv = prb * __half2float(__ushort_as_half(nrm[5]));
-            const pa_f2 wv2 = pa_pack(wv, wv);
+        // ---- the query's sign table ----
+        if (tid < kHeadDim) sqp[tid] = __half2float(p.Qp[static_cast<int64_t>(seg.row) * kHeadDim + tid]) * p.corr_scale;
+        __syncthreads();
+        // Sign nibble g = 2 c + h of a lane's sign word (byte c = byte `quarter` of sign word c) holds, in bit kk, the
+        // sign of local dim 4 (4 h + kk) + c (stride-4 order: dim 4 i + c is bit i of word c).
+        for (int e = tid; e < 8 * 16 * 32; e += kPaThreads) {
+            const int ln = e & 31, v = (e >> 5) & 15, g = e >> 9, c = g >> 1, h = g & 1, q = ln & 3;
+            float acc = 0.f;
 #pragma unroll
-            for (int j = 0; j < 16; ++j)
-                acc[j] = pa_fma(wv2, *reinterpret_cast<const pa_f2*>(pair_tab + pair_offset<BITS, 8>(vw, j, lane8)), acc[j]);
+            for (int kk = 0; kk < 4; ++kk) {
+                const float x = sqp[32 * q + 4 * (4 * h + kk) + c];
+                acc += ((v >> kk) & 1) ? x : -x;
+            }
+            *reinterpret_cast<float*>(sign_tab + e * 4) = acc;
         }
-#pragma unroll
-        for (int i = 0; i < 6; ++i) nrm[i] = nrm_n[i];
-        stage = stage + 1 == kPaStages ? 0 : stage + 1;
-        __syncwarp();   // every lane has read this stage before the next step's copy may land in it
-    }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    const int64_t out_slot = static_cast<int64_t>(bh) * p.num_splits + split;   // of the item just finished
-    item += gridDim.x;
-    if (item < n_items) begin_item(item);
+        __syncthreads();
 
-    // ---- merge the 8 slots of the warp, then the warps ----
-    float M = m_run;
+        float m_run = -INFINITY, l_run = 0.f;     // this slot's online softmax (log2 domain)
+        pa_f2 acc[16];
 #pragma unroll
-    for (int o = 4; o < 32; o <<= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
-    const float f = (m_run == -INFINITY) ? 0.f : pa_ex2(m_run - M);
-    float L = l_run * f;
+        for (int j = 0; j < 16; ++j) acc[j] = pa_pack(0.f, 0.f);
+
+        int stage = 0;
+        for (; tok16 < t1; tok16 += kStepTokens) {
+            const bool valid_a = tok16 + slot < t1, valid_b = tok16 + slot + 8 < t1;
+            issue();
+            uint16_t nrm_n[6];
+            load_norms(tok16 + kStepTokens, nrm_n);
+            asm volatile("cp.async.wait_group %0;" ::"n"(kPaStages - 1) : "memory");
+            __syncwarp();
+            const uint32_t so = stage * LO::kStageBytes;
+            uint32_t kwa[BITS], kwb[BITS];
+            lds_words<BITS>(my_words + so, kwa);
+            lds_words<BITS>(my_words + so + 8 * ROW, kwb);
+            uint4 sga, sgb;
+            asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(sga.x), "=r"(sga.y), "=r"(sga.z), "=r"(sga.w) : "r"(my_signs + so));
+            asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(sgb.x), "=r"(sgb.y), "=r"(sgb.z), "=r"(sgb.w) : "r"(my_signs + so + 128));
+            // ---- K scores: rows = the 16 tokens, column 0 = the query ----
+            float mse[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-    for (int o = 4; o < 32; o <<= 1) L += __shfl_xor_sync(0xffffffffu, L, o);
+            for (int ks = 0; ks < 8; ++ks) {
+                const uint32_t a0 = *reinterpret_cast<const uint32_t*>(half_tab + pair_offset<BITS, 7>(kwa, 2 * ks, lane4));
+                const uint32_t a1 = *reinterpret_cast<const uint32_t*>(half_tab + pair_offset<BITS, 7>(kwb, 2 * ks, lane4));
+                const uint32_t a2 = *reinterpret_cast<const uint32_t*>(half_tab + pair_offset<BITS, 7>(kwa, 2 * ks + 1, lane4));
+                const uint32_t a3 = *reinterpret_cast<const uint32_t*>(half_tab + pair_offset<BITS, 7>(kwb, 2 * ks + 1, lane4));
+                mma_f16_16816(mse, a0, a1, a2, a3, qf[2 * ks], qf[2 * ks + 1]);
+            }
+            // ---- QJL term of this lane's quarter, both tokens ----
+            const uint32_t swa = prmt(prmt(sga.x, sga.y, sel_lo), prmt(sga.z, sga.w, sel_lo), 0x5410);
+            const uint32_t swb = prmt(prmt(sgb.x, sgb.y, sel_lo), prmt(sgb.z, sgb.w, sel_lo), 0x5410);
+            float qja = 0.f, qjb = 0.f;
 #pragma unroll
-    for (int j = 0; j < 16; ++j) {
-        float x, y;
-        pa_unpack(acc[j], x, y);
-        x *= f;
-        y *= f;
+            for (int g = 0; g < 8; ++g) {
+                const uint32_t xa = 4 * g >= 7 ? (swa >> (4 * g - 7)) : (swa << (7 - 4 * g));
+                const uint32_t xb = 4 * g >= 7 ? (swb >> (4 * g - 7)) : (swb << (7 - 4 * g));
+                qja += *reinterpret_cast<const float*>(sign_tab + g * 2048 + ((xa & (15u << 7)) | lane4));
+                qjb += *reinterpret_cast<const float*>(sign_tab + g * 2048 + ((xb & (15u << 7)) | lane4));
+            }
+            // the quarter-0 lane of a slot holds the whole MSE dot product (column 0 of rows slot and slot + 8)
+            float pa = __half2float(__ushort_as_half(nrm[1])) * qja, pb = __half2float(__ushort_as_half(nrm[4])) * qjb;
+            if (quarter == 0) {
+                pa = fmaf(__half2float(__ushort_as_half(nrm[0])), mse[0], pa);
+                pb = fmaf(__half2float(__ushort_as_half(nrm[3])), mse[2], pb);
+            }
+            pa += __shfl_xor_sync(0xffffffffu, pa, 1);
+            pb += __shfl_xor_sync(0xffffffffu, pb, 1);
+            pa += __shfl_xor_sync(0xffffffffu, pa, 2);
+            pb += __shfl_xor_sync(0xffffffffu, pb, 2);
+            const float sa = valid_a ? pa * kLog2e : -INFINITY, sb = valid_b ? pb * kLog2e : -INFINITY;
+            // ---- online softmax of this slot: the maximum is raised only when a score exceeds it by 2^8 ----
+            const float smax = fmaxf(sa, sb);
+            if (smax > m_run + 8.f) {
+                const float alpha = pa_ex2(m_run - smax);     // 0 on the first token
+                const pa_f2 al2 = pa_pack(alpha, alpha);
+                l_run *= alpha;
 #pragma unroll
-        for (int o = 4; o < 32; o <<= 1) {
-            x += __shfl_xor_sync(0xffffffffu, x, o);
-            y += __shfl_xor_sync(0xffffffffu, y, o);
+                for (int j = 0; j < 16; ++j) acc[j] = pa_mul(acc[j], al2);
+                m_run = smax;
+            }
+            const float pra = valid_a ? pa_ex2(sa - m_run) : 0.f, prb = valid_b ? pa_ex2(sb - m_run) : 0.f;
+            l_run += pra + prb;
+            // ---- V ----
+            {
+                uint32_t vw[BITS];
+                lds_words<BITS>(my_words + so + 16 * ROW, vw);
+                const float wv = pra * __half2float(__ushort_as_half(nrm[2]));
+                const pa_f2 wv2 = pa_pack(wv, wv);
+#pragma unroll
+                for (int j = 0; j < 16; ++j)
+                    acc[j] = pa_fma(wv2, *reinterpret_cast<const pa_f2*>(pair_tab + pair_offset<BITS, 8>(vw, j, lane8)), acc[j]);
+            }
+            {
+                uint32_t vw[BITS];
+                lds_words<BITS>(my_words + so + 24 * ROW, vw);
+                const float wv = prb * __half2float(__ushort_as_half(nrm[5]));
+                const pa_f2 wv2 = pa_pack(wv, wv);
+#pragma unroll
+                for (int j = 0; j < 16; ++j)
+                    acc[j] = pa_fma(wv2, *reinterpret_cast<const pa_f2*>(pair_tab + pair_offset<BITS, 8>(vw, j, lane8)), acc[j]);
+            }
+#pragma unroll
+            for (int i = 0; i < 6; ++i) nrm[i] = nrm_n[i];
+            stage = stage + 1 == kPaStages ? 0 : stage + 1;
+            __syncwarp();   // every lane has read this stage before the next step's copy may land in it
         }
-        if (slot == 0) *reinterpret_cast<float2*>(&sacc[warp][32 * quarter + 2 * j]) = make_float2(x, y);
-    }
-    if (lane == 0) {
-        sml[warp][0] = M;
-        sml[warp][1] = L;
-    }
-    __syncthreads();
-    if (tid < kHeadDim) {
-        float Mc = sml[0][0];
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        const Segment finished = seg;
+        at = after(at, seg);
+        if (at < stop) begin(at);
+
+        // ---- merge the 8 slots of the warp, then the warps ----
+        float M = m_run;
 #pragma unroll
-        for (int w = 1; w < kPaWarps; ++w) Mc = fmaxf(Mc, sml[w][0]);
-        float o = 0.f, l = 0.f;
+        for (int o = 4; o < 32; o <<= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
+        const float f = (m_run == -INFINITY) ? 0.f : pa_ex2(m_run - M);
+        float L = l_run * f;
 #pragma unroll
-        for (int w = 0; w < kPaWarps; ++w) {
-            const float fw = (sml[w][0] == -INFINITY) ? 0.f : pa_ex2(sml[w][0] - Mc);
-            o = fmaf(fw, sacc[w][tid], o);
-            l = fmaf(fw, sml[w][1], l);
+        for (int o = 4; o < 32; o <<= 1) L += __shfl_xor_sync(0xffffffffu, L, o);
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+            float x, y;
+            pa_unpack(acc[j], x, y);
+            x *= f;
+            y *= f;
+#pragma unroll
+            for (int o = 4; o < 32; o <<= 1) {
+                x += __shfl_xor_sync(0xffffffffu, x, o);
+                y += __shfl_xor_sync(0xffffffffu, y, o);
+            }
+            if (slot == 0) *reinterpret_cast<float2*>(&sacc[warp][32 * quarter + 2 * j]) = make_float2(x, y);
         }
-        p.ws_acc[out_slot * kHeadDim + tid] = o;
-        if (tid == 0) {
-            p.ws_lse[out_slot * 2] = Mc;
-            p.ws_lse[out_slot * 2 + 1] = l;
+        if (lane == 0) {
+            sml[warp][0] = M;
+            sml[warp][1] = L;
         }
+        __syncthreads();
+        if (tid < kHeadDim) {
+            float Mc = sml[0][0];
+#pragma unroll
+            for (int w = 1; w < kPaWarps; ++w) Mc = fmaxf(Mc, sml[w][0]);
+            float o = 0.f, l = 0.f;
+#pragma unroll
+            for (int w = 0; w < kPaWarps; ++w) {
+                const float fw = (sml[w][0] == -INFINITY) ? 0.f : pa_ex2(sml[w][0] - Mc);
+                o = fmaf(fw, sacc[w][tid], o);
+                l = fmaf(fw, sml[w][1], l);
+            }
+            if (finished.slot < 0) {
+                p.out[static_cast<int64_t>(finished.row) * kHeadDim + tid] = __float2half_rn(o / l);
+            } else {
+                p.ws_acc[static_cast<int64_t>(finished.slot) * kHeadDim + tid] = o;
+                if (tid == 0) p.ws_lse[finished.slot] = make_float2(Mc, l);
+            }
+        }
+        // The next segment's first __syncthreads stands between these reads and its writes of sacc and the sign table.
     }
-    __syncthreads();   // the shared partials and the sign table are free for the next item
-  }
 }
 
-__global__ void __launch_bounds__(kHeadDim) packed_attn_merge(const PAParams p) {
-    const int bh = blockIdx.x, d = threadIdx.x;
-    float M = -INFINITY;
-    for (int s = 0; s < p.num_splits; ++s) M = fmaxf(M, p.ws_lse[(static_cast<int64_t>(bh) * p.num_splits + s) * 2]);
-    float o = 0.f, l = 0.f;
-    for (int s = 0; s < p.num_splits; ++s) {
-        const int64_t slot = static_cast<int64_t>(bh) * p.num_splits + s;
-        const float m = p.ws_lse[slot * 2];
-        const float w = (m == -INFINITY) ? 0.f : pa_ex2(m - M);   // empty splits carry no weight
-        o = fmaf(w, p.ws_acc[slot * kHeadDim + d], o);
-        l = fmaf(w, p.ws_lse[slot * 2 + 1], l);
+// One block per row: four warps share the parts, a lane holds four dims.
+constexpr int kMergeWarps = 4;
+__global__ void __launch_bounds__(kMergeWarps * 32) packed_attn_merge(const PAParams p, int n_ctas) {
+    __shared__ float4 so[kMergeWarps][32];
+    __shared__ float sl[kMergeWarps];
+    pa_release();
+    pa_wait();
+    const int bh = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int64_t slot0, parts, step = 1;
+    if (p.num_splits > 0) {
+        slot0 = static_cast<int64_t>(bh) * p.num_splits;
+        parts = p.num_splits;
+    } else {
+        const int steps = (p.Sk + kStepTokens - 1) / kStepTokens;
+        const int64_t total = static_cast<int64_t>(p.BH) * steps, first = static_cast<int64_t>(bh) * steps;
+        // the CTA whose share holds step u is the largest c with floor(c total / n) <= u
+        const int64_t c0 = ((first + 1) * n_ctas - 1) / total, c1 = ((first + steps) * n_ctas - 1) / total;
+        if (c0 == c1) return;                    // written by that CTA
+        slot0 = 2 * c0;                          // slot 2 c0 + 1, then 2 c for the others
+        parts = c1 - c0 + 1;
+        step = 2;
     }
-    p.out[static_cast<int64_t>(bh) * kHeadDim + d] = __float2half_rn(o / l);
+    auto slot_of = [&](int64_t i) { return slot0 + step * i + (step == 2 && i == 0 ? 1 : 0); };
+    const float2* lse = p.ws_lse;
+    const float4* part = reinterpret_cast<const float4*>(p.ws_acc);
+    float M = -INFINITY;
+    for (int64_t i = lane; i < parts; i += 32) M = fmaxf(M, lse[slot_of(i)].x);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
+    float4 o4 = make_float4(0.f, 0.f, 0.f, 0.f);
+    float l = 0.f;
+#pragma unroll 4
+    for (int64_t i = warp; i < parts; i += kMergeWarps) {
+        const int64_t s = slot_of(i);
+        const float2 ml = lse[s];
+        const float w = (ml.x == -INFINITY) ? 0.f : pa_ex2(ml.x - M);   // empty parts carry no weight
+        const float4 v = part[s * (kHeadDim / 4) + lane];
+        o4.x = fmaf(w, v.x, o4.x);
+        o4.y = fmaf(w, v.y, o4.y);
+        o4.z = fmaf(w, v.z, o4.z);
+        o4.w = fmaf(w, v.w, o4.w);
+        l = fmaf(w, ml.y, l);
+    }
+    so[warp][lane] = o4;
+    if (lane == 0) sl[warp] = l;
+    __syncthreads();
+    if (warp == 0) {
+#pragma unroll
+        for (int w = 1; w < kMergeWarps; ++w) {
+            const float4 v = so[w][lane];
+            o4.x += v.x;
+            o4.y += v.y;
+            o4.z += v.z;
+            o4.w += v.w;
+            l += sl[w];
+        }
+        *reinterpret_cast<uint2*>(p.out + static_cast<int64_t>(bh) * kHeadDim + 4 * lane) =
+            make_uint2(pack_half2(o4.x / l, o4.y / l), pack_half2(o4.z / l, o4.w / l));
+    }
 }
 
 // ---- row-wise WHT ----------------------------------------------------------------------
@@ -446,30 +550,46 @@ __global__ void __launch_bounds__(128) wht_rows_kernel(const void* in, void* out
 
 using namespace tq;
 
-extern "C" int tq_packed_attention_auto_splits(int BH, int Sk) {
-    if (BH <= 0 || Sk <= 0) return TQ_ERR_ARG;
-    // Two 256-thread CTAs per SM (one 512-thread CTA for 4-bit indices: half as many per wave, so a grid that fills
-    // waves of 296 fills waves of 148 too).  Take the split count (at least 1024 tokens per split, at most 64 splits)
-    // whose grid fills whole waves best; a small penalty per split keeps the merge short among near-ties.
-    const double penalty = 0.002;
-    const int max_splits = Sk / 1024 < 1 ? 1 : (Sk / 1024 > 64 ? 64 : Sk / 1024);
-    int best = 1;
-    double best_score = -1.0;
-    for (int s = 1; s <= max_splits; ++s) {
-        const double waves = static_cast<double>(BH) * s / 296.0;
-        const double full = waves <= 1.0 ? 1.0 : static_cast<double>(static_cast<long long>(waves + 0.999999));
-        const double score = waves / full - penalty * s;
-        if (score > best_score) {
-            best_score = score;
-            best = s;
+constexpr int64_t kMaxCtas = 256;   // CTAs that share the steps of all rows: at most one per SM
+
+// How many CTAs share the steps of all rows.  All SMs balance best, but a share that crosses into another row pays for
+// another sign table and merge; with few steps per CTA that is dearer than idle SMs.  A step costs about 1.4 us, a row (or
+// part of one) 3 us.  Candidates: one CTA per SM; every row cut into the same number of parts; whole rows.  (64 x 1000
+// tokens: 148 CTAs 15.3 us, 128 CTAs 9; 64 x 32768: 90.8 against 95.)
+static int64_t share_out(int64_t BH, int64_t Sk, int64_t sms) {
+    const int64_t S = (Sk + kStepTokens - 1) / kStepTokens, total = BH * S;
+    auto cost = [](int64_t steps, int64_t rows) { return 1.4 * static_cast<double>(steps) + 3.0 * static_cast<double>(rows); };
+    int64_t best = total < sms ? total : sms;
+    const int64_t each = (total + best - 1) / best;
+    double least = cost(each, 1 + (each - 1 + S - 1) / S);
+    auto consider = [&](int64_t ctas, double c) {
+        if (c < least) {
+            least = c;
+            best = ctas;
         }
+    };
+    if (BH <= sms) {
+        const int64_t parts = sms / BH < S ? sms / BH : S;
+        consider(BH * parts, cost((S + parts - 1) / parts, 1));
     }
+    for (int64_t rows = (BH + sms - 1) / sms; rows <= BH && rows <= 4 * ((BH + sms - 1) / sms); ++rows)
+        if (BH % rows == 0) {
+            consider(BH / rows, cost(rows * S, rows));
+            break;
+        }
     return best;
 }
 
+extern "C" int tq_packed_attention_auto_splits(int BH, int Sk) {
+    if (BH <= 0 || Sk <= 0) return TQ_ERR_ARG;
+    const int64_t parts = share_out(BH, Sk, 148) / BH;   // CTAs per row
+    return static_cast<int>(parts < 1 ? 1 : parts);
+}
+
 extern "C" int64_t tq_packed_attention_workspace_bytes(int BH, int num_splits) {
-    if (BH <= 0 || num_splits <= 0) return TQ_ERR_ARG;
-    return static_cast<int64_t>(BH) * num_splits * (kHeadDim + 2) * static_cast<int64_t>(sizeof(float));
+    if (BH <= 0 || num_splits < 0) return TQ_ERR_ARG;
+    const int64_t slots = num_splits > 0 ? static_cast<int64_t>(BH) * num_splits : 2 * kMaxCtas;
+    return slots * (kHeadDim + 2) * static_cast<int64_t>(sizeof(float));
 }
 
 extern "C" int tq_packed_attention(const void* Q, const void* Q_proj, const uint8_t* k_idx, const uint8_t* k_signs_perm,
@@ -483,10 +603,14 @@ extern "C" int tq_packed_attention(const void* Q, const void* Q_proj, const uint
     if (bits < 2 || bits > 4) return TQ_ERR_UNSUPPORTED;
     if ((reinterpret_cast<uintptr_t>(k_idx) | reinterpret_cast<uintptr_t>(k_signs_perm) | reinterpret_cast<uintptr_t>(v_idx)) & 15)
         return TQ_ERR_ARG;
-    if (num_splits <= 0) num_splits = tq_packed_attention_auto_splits(BH, Sk);
+    if (num_splits < 0) num_splits = 0;
     if (num_splits > Sk) num_splits = Sk;
     if (num_splits > 65535) return TQ_ERR_UNSUPPORTED;
-    if (!workspace || workspace_bytes < tq_packed_attention_workspace_bytes(BH, num_splits)) return TQ_ERR_WORKSPACE;
+    if (!workspace || workspace_bytes < tq_packed_attention_workspace_bytes(BH, num_splits) ||
+        (reinterpret_cast<uintptr_t>(workspace) & 15))
+        return TQ_ERR_WORKSPACE;
+    const int64_t slots = num_splits > 0 ? static_cast<int64_t>(BH) * num_splits : 2 * kMaxCtas;
+    if (slots > 2147483647) return TQ_ERR_UNSUPPORTED;
     PAParams p;
     p.Q = static_cast<const __half*>(Q);
     p.Qp = static_cast<const __half*>(Q_proj);
@@ -498,7 +622,8 @@ extern "C" int tq_packed_attention(const void* Q, const void* Q_proj, const uint
     p.v_norm = static_cast<const __half*>(v_norm);
     p.centroids = centroids;
     p.ws_acc = static_cast<float*>(workspace);
-    p.ws_lse = p.ws_acc + static_cast<int64_t>(BH) * num_splits * kHeadDim;
+    p.ws_lse = reinterpret_cast<float2*>(p.ws_acc + slots * kHeadDim);
+    p.BH = BH;
     p.out = static_cast<__half*>(out);
     p.corr_scale = corr_scale;
     p.Sk = Sk;
@@ -517,20 +642,18 @@ extern "C" int tq_packed_attention(const void* Q, const void* Q_proj, const uint
             return TQ_ERR_LAUNCH;
         configured[dev] = true;
     }
-    // persistent CTAs: as many as are resident at once, each strides over the (row, split) items
-    const int64_t items64 = static_cast<int64_t>(BH) * num_splits;
-    if (items64 > 2147483647) return TQ_ERR_UNSUPPORTED;
-    const int n_items = static_cast<int>(items64);
-    const int resident = sm_count[dev] * (bits == 4 ? 1 : 2);
-    const unsigned grid = static_cast<unsigned>(n_items < resident ? n_items : resident);
+    const int64_t most = sm_count[dev] < kMaxCtas ? sm_count[dev] : kMaxCtas;
+    const unsigned grid = static_cast<unsigned>(num_splits > 0 ? (slots < most ? slots : most) : share_out(BH, Sk, most));
+    const int n_items = num_splits > 0 ? static_cast<int>(slots) : 0;
+    bool launched = false;
     switch (bits) {
-        case 2: packed_attn_partial<2><<<grid, PALayout<2>::kThreads, PALayout<2>::kSmem, st>>>(p, n_items); break;
-        case 3: packed_attn_partial<3><<<grid, PALayout<3>::kThreads, PALayout<3>::kSmem, st>>>(p, n_items); break;
-        case 4: packed_attn_partial<4><<<grid, PALayout<4>::kThreads, PALayout<4>::kSmem, st>>>(p, n_items); break;
+        case 2: launched = pa_launch(packed_attn_partial<2>, false, grid, kPaThreads, PALayout<2>::kSmem, st, p, n_items); break;
+        case 3: launched = pa_launch(packed_attn_partial<3>, false, grid, kPaThreads, PALayout<3>::kSmem, st, p, n_items); break;
+        case 4: launched = pa_launch(packed_attn_partial<4>, false, grid, kPaThreads, PALayout<4>::kSmem, st, p, n_items); break;
     }
-    if (cudaGetLastError() != cudaSuccess) return TQ_ERR_LAUNCH;
-    packed_attn_merge<<<BH, kHeadDim, 0, st>>>(p);
-    return cudaGetLastError() == cudaSuccess ? TQ_OK : TQ_ERR_LAUNCH;
+    if (!launched) return TQ_ERR_LAUNCH;
+    if (num_splits == 1 || (num_splits == 0 && grid == 1)) return TQ_OK;   // every row was written whole
+    return pa_launch(packed_attn_merge, true, static_cast<unsigned>(BH), kMergeWarps * 32, 0, st, p, static_cast<int>(grid)) ? TQ_OK : TQ_ERR_LAUNCH;
 }
 
 extern "C" int tq_wht_rows(const void* in, void* out, int dtype, int64_t n_rows, float scale, tq_stream_t stream) {

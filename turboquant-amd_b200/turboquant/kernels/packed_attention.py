@@ -20,10 +20,10 @@ def _get_config(BH: int, Sk: int):
 
     The reference looks these up in a table tuned on MI355X; here the split
     count comes from the library's B200 heuristic and the other three are
-    fixed properties of the CUDA kernel (128-token tiles, 4 warps, no
+    fixed properties of the CUDA kernel (steps of 256 tokens, 16 warps, no
     software pipelining stages).
     """
-    return 128, _native.lib().tq_packed_attention_auto_splits(BH, Sk), 4, 1
+    return 256, _native.lib().tq_packed_attention_auto_splits(BH, Sk), 16, 1
 
 
 def attention_unpacked_ref(Q, Q_proj, K_mse_rot, signs_float, k_r_norm, V_mse_rot, corr_scale):
@@ -63,8 +63,7 @@ def packed_attention(Q, Q_proj, k_idx_packed, k_signs_packed, k_r_norm, k_norm,
     krn, kn, vn = half(k_r_norm), half(k_norm), half(v_norm)
     cb = _native._f32(centroids, dev)
     L = _native.lib()
-    splits = int(num_splits) if num_splits else L.tq_packed_attention_auto_splits(BH, Sk)
-    splits = max(1, min(splits, Sk))
+    splits = max(0, min(int(num_splits or 0), Sk))          # 0: the library shares the work out
     need = L.tq_packed_attention_workspace_bytes(BH, splits)
     ws = _native.workspace(dev, need, tag="packed_attention")
     out = torch.empty(BH, D, dtype=torch.float16, device=dev)
