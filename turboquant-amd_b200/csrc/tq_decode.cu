@@ -280,23 +280,31 @@ __device__ __forceinline__ void lds_words(uint32_t addr, uint32_t (&w)[NW]) {
     }
 }
 
-// Output de-rotation inside a block: 128 threads hold one value each (thread = dim); returns (v H)[dim].
-// Five butterfly stages by warp shuffle, two through shared memory (buf: 128 floats).
-__device__ __forceinline__ float block_wht128(float v, float* buf, int tid) {
+// Output row of a query head from its weighted sum (lane: dims 4 lane .. 4 lane + 3) and denominator.
+__device__ __forceinline__ void write_row(const DecodeParams& p, int64_t row, int lane, float (&x)[4], float l) {
+    const float inv = 1.f / l;
 #pragma unroll
-    for (int m = 1; m < 32; m <<= 1) {
-        const float o = __shfl_xor_sync(0xffffffffu, v, m);
-        v = (tid & m) ? o - v : v + o;
-    }
+    for (int i = 0; i < 4; ++i) x[i] *= inv;
+    if (p.derotate_out) {   // two stages in the lane, five across lanes
+        const float b0 = x[0] + x[1], b1 = x[0] - x[1], b2 = x[2] + x[3], b3 = x[2] - x[3];
+        x[0] = b0 + b2; x[1] = b1 + b3; x[2] = b0 - b2; x[3] = b1 - b3;
 #pragma unroll
-    for (int m = 32; m < 128; m <<= 1) {
-        buf[tid] = v;
-        asm volatile("bar.sync 1, 128;" ::: "memory");
-        const float o = buf[tid ^ m];
-        v = (tid & m) ? o - v : v + o;
-        asm volatile("bar.sync 1, 128;" ::: "memory");
+        for (int m = 1; m < 32; m <<= 1) {
+            const float sgn = (lane & m) ? -1.f : 1.f;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) x[i] = fmaf(sgn, x[i], __shfl_xor_sync(0xffffffffu, x[i], m));
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) x[i] *= kWhtScale;
     }
-    return v * kWhtScale;
+    uint2 w;
+    if (p.io_dtype == TQ_DTYPE_F16) {
+        w = make_uint2(pack_half2(x[0], x[1]), pack_half2(x[2], x[3]));
+    } else {
+        const __nv_bfloat162 lo = __floats2bfloat162_rn(x[0], x[1]), hi = __floats2bfloat162_rn(x[2], x[3]);
+        w = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+    }
+    *reinterpret_cast<uint2*>(static_cast<uint16_t*>(p.out) + row * kHeadDim + 4 * lane) = w;
 }
 
 template <int KB, int VB, bool QJL, bool SPARSE, int NSTAGE>
@@ -317,7 +325,6 @@ __global__ void __launch_bounds__(kThreads, TQ_DEC_MINBLOCKS) decode_partial_ker
     float* sm_o = reinterpret_cast<float*>(ring);                       // reused after the page loop
     __shared__ float sm_m[kWarps][8];
     __shared__ float sm_l[kWarps][8];
-    __shared__ float sm_wht[kHeadDim];
 
     pdl_release_and_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -562,42 +569,79 @@ __global__ void __launch_bounds__(kThreads, TQ_DEC_MINBLOCKS) decode_partial_ker
             }
     }
     __syncthreads();
-    const int dim = threadIdx.x;
-    const int col = dim + (dim >> 5);
+    // a warp combines the four partials of query rows warp, warp + 4; a lane holds four dims
     const int nchunks = (npages + p.chunk_pages - 1) / p.chunk_pages;
-    for (int g = 0; g < (dim < kHeadDim ? nq : 0); ++g) {
+    for (int g = warp; g < nq; g += kWarps) {
         float M = sm_m[0][g];
 #pragma unroll
         for (int w = 1; w < kWarps; ++w) M = fmaxf(M, sm_m[w][g]);
-        float o = 0.f, l = 0.f;
+        float l = 0.f, x[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
         for (int w = 0; w < kWarps; ++w) {
             const float sc = ex2(sm_m[w][g] - M);
-            o = fmaf(sc, sm_o[(w * 8 + g) * kOPad + col], o);
+            const float* o = sm_o + (w * 8 + g) * kOPad + 4 * lane + (lane >> 3);   // dims d sit at d + d / 32
+#pragma unroll
+            for (int i = 0; i < 4; ++i) x[i] = fmaf(sc, o[i], x[i]);
             l = fmaf(sc, sm_l[w][g], l);
         }
         if (nchunks == 1) {
-            float r = o / l;
-            if (p.derotate_out) r = block_wht128(r, sm_wht, dim);
-            const int64_t off = (static_cast<int64_t>(seq) * p.Hq + head0 + g) * kHeadDim + dim;
-            if (p.io_dtype == TQ_DTYPE_F16)
-                static_cast<__half*>(p.out)[off] = __float2half_rn(r);
-            else
-                static_cast<__nv_bfloat16*>(p.out)[off] = __float2bfloat16_rn(r);
+            write_row(p, static_cast<int64_t>(seq) * p.Hq + head0 + g, lane, x, l);
         } else {
             const int64_t slot = ((static_cast<int64_t>(seq) * p.Hkv * p.ngroups + blockIdx.y) * p.max_chunks + chunk) * 8 + g;
-            p.ws_o[slot * kHeadDim + dim] = o;
-            if (dim == 0) {
-                p.ws_ml[slot * 2] = M;
-                p.ws_ml[slot * 2 + 1] = l;
-            }
+            *reinterpret_cast<float4*>(p.ws_o + slot * kHeadDim + 4 * lane) = make_float4(x[0], x[1], x[2], x[3]);
+            if (lane == 0) reinterpret_cast<float2*>(p.ws_ml)[slot] = make_float2(M, l);
         }
     }
 }
 
-__global__ void __launch_bounds__(kHeadDim) decode_merge_kernel(const DecodeParams p) {
+// Weighted combination of partial rows by one warp: part(i) is the 128 sums of part i (fp32), ml(i) its (maximum,
+// denominator).  Four parts are fetched at a time, independently of one another and of the maxima: what a merge costs is the
+// latency of its chain of loads.
+template <typename Part, typename Ml>
+__device__ __forceinline__ void merge_parts(int first, int step, int parts, int lane, Part part, Ml ml, float& M, float (&x)[4], float& l) {
+    M = -INFINITY;
+    l = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) x[i] = 0.f;
+    for (int i0 = first; i0 < parts; i0 += 4 * step) {
+        float4 v[4];
+        float2 w[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int i = i0 + k * step;
+            if (i < parts) {
+                w[k] = ml(i);
+                v[k] = *reinterpret_cast<const float4*>(part(i) + 4 * lane);
+            } else {
+                w[k] = make_float2(-INFINITY, 0.f);
+                v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+        }
+        const float m = fmaxf(fmaxf(M, fmaxf(w[0].x, w[1].x)), fmaxf(w[2].x, w[3].x));
+        const float old = ex2(M - m);
+        l *= old;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) x[i] *= old;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const float sc = ex2(w[k].x - m);
+            l = fmaf(sc, w[k].y, l);
+            x[0] = fmaf(sc, v[k].x, x[0]);
+            x[1] = fmaf(sc, v[k].y, x[1]);
+            x[2] = fmaf(sc, v[k].z, x[2]);
+            x[3] = fmaf(sc, v[k].w, x[3]);
+        }
+        M = m;
+    }
+}
+
+// One block per query head; its four warps share the chunks.
+constexpr int kChunkMergeWarps = 4;
+__global__ void __launch_bounds__(kChunkMergeWarps * 32) decode_merge_kernel(const DecodeParams p) {
+    __shared__ float4 so[kChunkMergeWarps][32];
+    __shared__ float2 sml[kChunkMergeWarps];
     pdl_release_and_wait();
-    const int head = blockIdx.x, seq = blockIdx.y, dim = threadIdx.x;
+    const int head = blockIdx.x, seq = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int L = p.seq_lens[seq];
     const int npages = min((L + kPageTokens - 1) / kPageTokens, p.max_pages);   // same cut as the partial kernel
     const int nchunks = (npages + p.chunk_pages - 1) / p.chunk_pages;
@@ -605,25 +649,29 @@ __global__ void __launch_bounds__(kHeadDim) decode_merge_kernel(const DecodePara
     const int kvh = head / p.G, gi = head % p.G;
     const int by = kvh * p.ngroups + gi / 8, g = gi % 8;
     const int64_t base = (static_cast<int64_t>(seq) * p.Hkv * p.ngroups + by) * p.max_chunks;
-    float M = -INFINITY;
-    for (int c = 0; c < nchunks; ++c) M = fmaxf(M, p.ws_ml[((base + c) * 8 + g) * 2]);
-    float o = 0.f, l = 0.f;
-    for (int c = 0; c < nchunks; ++c) {
-        const int64_t slot = (base + c) * 8 + g;
-        const float sc = ex2(p.ws_ml[slot * 2] - M);
-        o = fmaf(sc, p.ws_o[slot * kHeadDim + dim], o);
-        l = fmaf(sc, p.ws_ml[slot * 2 + 1], l);
+    float M, l, x[4];
+    merge_parts(warp, kChunkMergeWarps, nchunks, lane, [&](int c) { return p.ws_o + ((base + c) * 8 + g) * kHeadDim; },
+                [&](int c) { return reinterpret_cast<const float2*>(p.ws_ml)[(base + c) * 8 + g]; }, M, x, l);
+    so[warp][lane] = make_float4(x[0], x[1], x[2], x[3]);
+    if (lane == 0) sml[warp] = make_float2(M, l);
+    __syncthreads();
+    if (warp != 0) return;
+    float Ma = sml[0].x;
+#pragma unroll
+    for (int w = 1; w < kChunkMergeWarps; ++w) Ma = fmaxf(Ma, sml[w].x);
+    l = 0.f;
+    x[0] = x[1] = x[2] = x[3] = 0.f;
+#pragma unroll
+    for (int w = 0; w < kChunkMergeWarps; ++w) {
+        const float sc = ex2(sml[w].x - Ma);
+        const float4 v = so[w][lane];
+        l = fmaf(sc, sml[w].y, l);
+        x[0] = fmaf(sc, v.x, x[0]);
+        x[1] = fmaf(sc, v.y, x[1]);
+        x[2] = fmaf(sc, v.z, x[2]);
+        x[3] = fmaf(sc, v.w, x[3]);
     }
-    float r = o / l;
-    if (p.derotate_out) {
-        __shared__ float buf[kHeadDim];
-        r = block_wht128(r, buf, dim);
-    }
-    const int64_t off = (static_cast<int64_t>(seq) * p.Hq + head) * kHeadDim + dim;
-    if (p.io_dtype == TQ_DTYPE_F16)
-        static_cast<__half*>(p.out)[off] = __float2half_rn(r);
-    else
-        static_cast<__nv_bfloat16*>(p.out)[off] = __float2bfloat16_rn(r);
+    write_row(p, static_cast<int64_t>(seq) * p.Hq + head, lane, x, l);
 }
 
 template <int KB, int VB, bool QJL, bool SPARSE>
@@ -877,7 +925,7 @@ extern "C" int tq_decode_paged(void* out, const void* q_rot, const void* q_proj,
         if (launch_chained(decode_stream_merge_kernel, dim3(kStreamCtas), dim3(256), 0, st, sp) != cudaSuccess)
             return TQ_ERR_LAUNCH;
     } else if (max_chunks > 1) {
-        if (launch_chained(decode_merge_kernel, dim3(num_q_heads, num_seqs), dim3(kHeadDim), 0, st, p) != cudaSuccess)
+        if (launch_chained(decode_merge_kernel, dim3(num_q_heads, num_seqs), dim3(kChunkMergeWarps * 32), 0, st, p) != cudaSuccess)
             return TQ_ERR_LAUNCH;
     }
     return TQ_OK;

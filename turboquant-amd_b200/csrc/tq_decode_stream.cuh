@@ -184,34 +184,10 @@ __device__ __forceinline__ uint4 table_signs(uint32_t w, uint32_t base) {
     return v;
 }
 
-// Output row g of an item from its weighted sum (lane: dims 4 lane .. 4 lane + 3) and denominator.
+// Output row g of an item.
 __device__ __forceinline__ void finish_row(const DecodeParams& p, int seq, int hg, int g, int lane, float (&x)[4], float l) {
     const int kvh = p.ngroups == 1 ? hg : hg / p.ngroups, qg = hg - kvh * p.ngroups;
-    if (g >= p.G - qg * 8) return;
-    const float inv = 1.f / l;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) x[i] *= inv;
-    if (p.derotate_out) {   // two stages in the lane, five across lanes
-        const float b0 = x[0] + x[1], b1 = x[0] - x[1], b2 = x[2] + x[3], b3 = x[2] - x[3];
-        x[0] = b0 + b2; x[1] = b1 + b3; x[2] = b0 - b2; x[3] = b1 - b3;
-#pragma unroll
-        for (int m = 1; m < 32; m <<= 1) {
-            const float sgn = (lane & m) ? -1.f : 1.f;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) x[i] = fmaf(sgn, x[i], __shfl_xor_sync(0xffffffffu, x[i], m));
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) x[i] *= kWhtScale;
-    }
-    uint2 w;
-    if (p.io_dtype == TQ_DTYPE_F16) {
-        w = make_uint2(pack_half2(x[0], x[1]), pack_half2(x[2], x[3]));
-    } else {
-        const __nv_bfloat162 lo = __floats2bfloat162_rn(x[0], x[1]), hi = __floats2bfloat162_rn(x[2], x[3]);
-        w = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
-    }
-    const int64_t row = static_cast<int64_t>(seq) * p.Hq + kvh * p.G + qg * 8 + g;
-    *reinterpret_cast<uint2*>(static_cast<uint16_t*>(p.out) + row * kHeadDim + 4 * lane) = w;
+    if (g < p.G - qg * 8) write_row(p, static_cast<int64_t>(seq) * p.Hq + kvh * p.G + qg * 8 + g, lane, x, l);
 }
 
 // SIGN_TABLE: K and V share a codebook and S = I, so the V half of the table has room for the signs, and the query
@@ -776,31 +752,10 @@ __global__ void __launch_bounds__(256) decode_stream_merge_kernel(const StreamPa
     const int cta = blockIdx.x, g = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int4 item = sp.split[cta];
     if (item.z < 0) return;
-    const int parts = item.z - cta + 1;   // slot 1 of this CTA, slot 0 of the others
-    auto slot_of = [&](int i) { return sp.n_warps + 2 * (cta + i) + (i == 0 ? 1 : 0); };
-    float M = -INFINITY;
-    for (int i = lane; i < parts; i += 32) M = fmaxf(M, sp.part_ml[slot_of(i) * 8 + g].x);
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
-    float x[4] = {0.f, 0.f, 0.f, 0.f};
-    float l = 0.f;
-    for (int i0 = 0; i0 < parts; i0 += 32) {
-        float2 ml = make_float2(-INFINITY, 0.f);
-        if (i0 + lane < parts) ml = sp.part_ml[slot_of(i0 + lane) * 8 + g];
-        const float scale = ex2(ml.x - M);
-        l = fmaf(scale, ml.y, l);
-#pragma unroll 4
-        for (int i = 0; i < min(32, parts - i0); ++i) {
-            const float4 v = *reinterpret_cast<const float4*>(sp.part_o + static_cast<int64_t>(slot_of(i0 + i)) * kStreamSlotFloats + g * kHeadDim + 4 * lane);
-            const float sc = __shfl_sync(0xffffffffu, scale, i);
-            x[0] = fmaf(sc, v.x, x[0]);
-            x[1] = fmaf(sc, v.y, x[1]);
-            x[2] = fmaf(sc, v.z, x[2]);
-            x[3] = fmaf(sc, v.w, x[3]);
-        }
-    }
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+    auto slot_of = [&](int i) { return sp.n_warps + 2 * (cta + i) + (i == 0 ? 1 : 0); };   // slot 1 of this CTA, slot 0 of the others
+    float M, l, x[4];
+    merge_parts(0, 1, item.z - cta + 1, lane, [&](int i) { return sp.part_o + static_cast<int64_t>(slot_of(i)) * kStreamSlotFloats + g * kHeadDim; },
+                [&](int i) { return sp.part_ml[slot_of(i) * 8 + g]; }, M, x, l);
     finish_row(sp.d, item.x, item.y, g, lane, x, l);
 }
 

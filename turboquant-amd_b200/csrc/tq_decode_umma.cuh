@@ -33,6 +33,25 @@
 namespace tq {
 namespace {
 
+// Output de-rotation inside a block: 128 threads hold one value each (thread = dim); returns (v H)[dim].
+// Five butterfly stages by warp shuffle, two through shared memory (buf: 128 floats).
+__device__ __forceinline__ float block_wht128(float v, float* buf, int tid) {
+#pragma unroll
+    for (int m = 1; m < 32; m <<= 1) {
+        const float o = __shfl_xor_sync(0xffffffffu, v, m);
+        v = (tid & m) ? o - v : v + o;
+    }
+#pragma unroll
+    for (int m = 32; m < 128; m <<= 1) {
+        buf[tid] = v;
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        const float o = buf[tid ^ m];
+        v = (tid & m) ? o - v : v + o;
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+    }
+    return v * kWhtScale;
+}
+
 constexpr int kUmThreads = 320;         // warps 0-3 keys + softmax, 4-7 values + accumulate, 8 producer, 9 MMA
 constexpr int kUmTilePages = 8;
 constexpr int kUmTileTokens = kUmTilePages * kPageTokens;   // 128
