@@ -442,8 +442,10 @@ __device__ __forceinline__ void compress_contig_rows(const ContigParams& p, int6
 template <int BITS, OutMode MODE>
 __global__ void __launch_bounds__(kWarpsPerCta * 32) compress_contig_kernel(const ContigParams p) {
     __shared__ float csm[1 << BITS];
+    pdl_release();
     if (threadIdx.x < (1 << BITS)) csm[threadIdx.x] = p.c ? p.c[threadIdx.x] : 0.f;
     __syncthreads();
+    pdl_wait();
     const int lane = threadIdx.x & 31;
     compress_contig_rows<BITS, MODE>(
         p, (static_cast<int64_t>(blockIdx.x) * kWarpsPerCta + (threadIdx.x >> 5)) * kItemsPerWarp + (lane >> 2), lane, csm);
@@ -525,8 +527,10 @@ __device__ __forceinline__ void fwht128_chunks(float (&x)[32], int lane) {
 template <int BITS, bool SIGNS, bool WIDE>
 __global__ void __launch_bounds__(kWarpsPerCta * 32) compress_unpacked_kernel(const ContigParams p) {
     __shared__ float csm[1 << BITS];
+    pdl_release();
     if (threadIdx.x < (1 << BITS)) csm[threadIdx.x] = p.c[threadIdx.x];
     __syncthreads();
+    pdl_wait();
     const int lane = threadIdx.x & 31, j = lane & 3;
     const int64_t row = (static_cast<int64_t>(blockIdx.x) * kWarpsPerCta + (threadIdx.x >> 5)) * kItemsPerWarp + (lane >> 2);
     const bool live = row < p.n;   // lanes of rows past the end take part in the shuffles, on zeros
@@ -594,18 +598,17 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) compress_unpacked_kernel(co
 }
 
 template <int BITS>
-void launch_unpacked(const ContigParams& p, cudaStream_t st) {
-    const unsigned grid = static_cast<unsigned>((p.n + kItemsPerCta - 1) / kItemsPerCta);
+int launch_unpacked(const ContigParams& p, cudaStream_t st) {
+    const dim3 grid(static_cast<unsigned>((p.n + kItemsPerCta - 1) / kItemsPerCta)), block(kWarpsPerCta * 32);
     const uintptr_t all = reinterpret_cast<uintptr_t>(p.x) | reinterpret_cast<uintptr_t>(p.indices) | reinterpret_cast<uintptr_t>(p.mse) |
                           reinterpret_cast<uintptr_t>(p.signs);
     const bool wide = (all & 31) == 0;
-    if (p.signs) {
-        if (wide) compress_unpacked_kernel<BITS, true, true><<<grid, kWarpsPerCta * 32, 0, st>>>(p);
-        else compress_unpacked_kernel<BITS, true, false><<<grid, kWarpsPerCta * 32, 0, st>>>(p);
-    } else {
-        if (wide) compress_unpacked_kernel<BITS, false, true><<<grid, kWarpsPerCta * 32, 0, st>>>(p);
-        else compress_unpacked_kernel<BITS, false, false><<<grid, kWarpsPerCta * 32, 0, st>>>(p);
-    }
+    cudaError_t e;
+    if (p.signs) e = wide ? launch_chained(compress_unpacked_kernel<BITS, true, true>, grid, block, 0, st, p)
+                          : launch_chained(compress_unpacked_kernel<BITS, true, false>, grid, block, 0, st, p);
+    else e = wide ? launch_chained(compress_unpacked_kernel<BITS, false, true>, grid, block, 0, st, p)
+                  : launch_chained(compress_unpacked_kernel<BITS, false, false>, grid, block, 0, st, p);
+    return e == cudaSuccess ? TQ_OK : TQ_ERR_LAUNCH;
 }
 
 // ---- packed contiguous outputs on the table-driven quantizer ------------------------------------------------------
@@ -640,6 +643,8 @@ __global__ void __launch_bounds__(kFastWarps * 32, 1) compress_contig_fast_kerne
     int64_t unit = static_cast<int64_t>(warp) * gridDim.x + blockIdx.x;
     const int64_t step = static_cast<int64_t>(gridDim.x) * kFastWarps;
     auto row_of = [&](int64_t u) { return u * kItemsPerWarp + (lane >> 2); };
+    pdl_release();
+    pdl_wait();
     if (mma) {
         stage_row(dst, p.x, row_of(unit) * kHeadDim + 8 * quarter, row_of(unit) < p.n);
         stage_row(dst + kRowBuffer, p.x, row_of(unit + step) * kHeadDim + 8 * quarter, row_of(unit + step) < p.n);
@@ -703,8 +708,7 @@ int launch_contig_fast(const ContigParams& p, cudaStream_t st) {
             return TQ_ERR_LAUNCH;
         if (dev >= 0 && dev < 64) configured[dev] = true;
     }
-    compress_contig_fast_kernel<BITS, QJL><<<grid, kFastWarps * 32, kSmem, st>>>(p, n_units);
-    return cudaGetLastError() == cudaSuccess ? TQ_OK : TQ_ERR_LAUNCH;
+    return launch_chained(compress_contig_fast_kernel<BITS, QJL>, dim3(grid), dim3(kFastWarps * 32), kSmem, st, p, n_units) == cudaSuccess ? TQ_OK : TQ_ERR_LAUNCH;
 }
 
 template <int KB, int VB>
@@ -736,14 +740,15 @@ int launch_contig(const ContigParams& p, int bits, cudaStream_t st) {
             default: return TQ_ERR_UNSUPPORTED;
         }
     }
-    const unsigned grid = static_cast<unsigned>((p.n + kItemsPerCta - 1) / kItemsPerCta);
+    const dim3 grid(static_cast<unsigned>((p.n + kItemsPerCta - 1) / kItemsPerCta)), block(kWarpsPerCta * 32);
+    cudaError_t e;
     switch (bits) {
-        case 2: compress_contig_kernel<2, MODE><<<grid, kWarpsPerCta * 32, 0, st>>>(p); break;
-        case 3: compress_contig_kernel<3, MODE><<<grid, kWarpsPerCta * 32, 0, st>>>(p); break;
-        case 4: compress_contig_kernel<4, MODE><<<grid, kWarpsPerCta * 32, 0, st>>>(p); break;
+        case 2: e = launch_chained(compress_contig_kernel<2, MODE>, grid, block, 0, st, p); break;
+        case 3: e = launch_chained(compress_contig_kernel<3, MODE>, grid, block, 0, st, p); break;
+        case 4: e = launch_chained(compress_contig_kernel<4, MODE>, grid, block, 0, st, p); break;
         default: return TQ_ERR_UNSUPPORTED;
     }
-    return cudaGetLastError() == cudaSuccess ? TQ_OK : TQ_ERR_LAUNCH;
+    return e == cudaSuccess ? TQ_OK : TQ_ERR_LAUNCH;
 }
 
 bool dtype_ok(int d) { return d == TQ_DTYPE_F16 || d == TQ_DTYPE_BF16 || d == TQ_DTYPE_F32; }
@@ -850,11 +855,11 @@ extern "C" int tq_polarquant_compress(const void* x, int in_dtype, int64_t n, co
     p.x = x; p.c = centroids; p.b = boundaries; p.indices = indices; p.norms = norms; p.mse = k_mse_rot;
     p.signs = use_qjl ? signs : nullptr; p.rnorm = use_qjl ? rnorm : nullptr;
     p.n = n; p.in_dtype = in_dtype; p.rotate = prerotated ? 0 : 1;
+    cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     switch (bits) {
-        case 2: launch_unpacked<2>(p, reinterpret_cast<cudaStream_t>(stream)); break;
-        case 3: launch_unpacked<3>(p, reinterpret_cast<cudaStream_t>(stream)); break;
-        case 4: launch_unpacked<4>(p, reinterpret_cast<cudaStream_t>(stream)); break;
-        default: return TQ_ERR_UNSUPPORTED;
+        case 2: return launch_unpacked<2>(p, st);
+        case 3: return launch_unpacked<3>(p, st);
+        case 4: return launch_unpacked<4>(p, st);
     }
-    return cudaGetLastError() == cudaSuccess ? TQ_OK : TQ_ERR_LAUNCH;
+    return TQ_ERR_UNSUPPORTED;
 }

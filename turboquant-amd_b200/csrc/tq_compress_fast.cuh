@@ -756,6 +756,8 @@ __global__ void __launch_bounds__(kFastWarps * 32, TQ_CMP_MINBLOCKS) compress_pa
     const uint32_t vtab = smem_u32(tables + kTableBytes) + (lane & 15) * 8 - kBias;
     const bool rotate = p.rotate != 0, mma = rotate && p.in_dtype != TQ_DTYPE_F32;
 
+    pdl_release();
+    pdl_wait();
     // Tensor-core path.  Rows are staged through shared memory one unit ahead: the key rows of the next unit are requested
     // as soon as this unit's have been consumed by the MMAs, the value rows likewise, so every copy has a whole unit's
     // arithmetic to hide behind.  The first ones are under way while the tables are built.
@@ -834,8 +836,10 @@ __global__ void __launch_bounds__(kFastWarps * 32, TQ_CMP_MINBLOCKS) compress_pa
 template <int KB, int VB, bool QJL>
 __global__ void __launch_bounds__(kWarpsPerCta * 32) compress_paged_small_kernel(const PagedParams p) {
     __shared__ float csm[1 << KB];
+    pdl_release();
     if (threadIdx.x < (1 << KB)) csm[threadIdx.x] = p.kc[threadIdx.x];
     __syncthreads();
+    pdl_wait();
     const int lane = threadIdx.x & 31;
     const int64_t item = (static_cast<int64_t>(blockIdx.x) * kWarpsPerCta + (threadIdx.x >> 5)) * kItemsPerWarp + (lane >> 2);
     compress_items_generic<KB, VB, QJL>(p, item, lane, csm);
@@ -853,8 +857,7 @@ template <int KB, int VB, bool QJL>
 int launch_paged_fast(const PagedParams& p, cudaStream_t st) {
     if (p.n_items <= kSmallLaunchItems) {
         const unsigned grid = static_cast<unsigned>((p.n_items + kItemsPerCta - 1) / kItemsPerCta);
-        compress_paged_small_kernel<KB, VB, QJL><<<grid, kWarpsPerCta * 32, 0, st>>>(p);
-        return cudaGetLastError() == cudaSuccess ? TQ_OK : TQ_ERR_LAUNCH;
+        return launch_chained(compress_paged_small_kernel<KB, VB, QJL>, dim3(grid), dim3(kWarpsPerCta * 32), 0, st, p) == cudaSuccess ? TQ_OK : TQ_ERR_LAUNCH;
     }
     // on request: fp16 / bf16 rows that still need the rotation go to the tensor-memory kernel (rotation as one
     // 128 x 128 x 128 product per 128 rows, one thread per vector afterwards)
@@ -878,8 +881,7 @@ int launch_paged_fast(const PagedParams& p, cudaStream_t st) {
             return TQ_ERR_LAUNCH;
         if (dev >= 0 && dev < 64) configured[dev] = true;
     }
-    compress_paged_fast_kernel<KB, VB, QJL><<<grid, kFastWarps * 32, kSmem, st>>>(p, n_groups);
-    return cudaGetLastError() == cudaSuccess ? TQ_OK : TQ_ERR_LAUNCH;
+    return launch_chained(compress_paged_fast_kernel<KB, VB, QJL>, dim3(grid), dim3(kFastWarps * 32), kSmem, st, p, n_groups) == cudaSuccess ? TQ_OK : TQ_ERR_LAUNCH;
 }
 
 }  // namespace

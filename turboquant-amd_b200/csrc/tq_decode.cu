@@ -36,53 +36,11 @@ namespace {
 #ifndef TQ_DEC_MINBLOCKS
 #define TQ_DEC_MINBLOCKS 4
 #endif
-#ifndef TQ_DEC_PDL
-#define TQ_DEC_PDL 1
-#endif
 constexpr int kWarps = TQ_DEC_WARPS;
 constexpr int kThreads = kWarps * 32;
 constexpr int kOPad = 132;  // row stride of the merge buffer (floats)
 constexpr int kStages = TQ_DEC_STAGES;  // pages in flight per warp
 constexpr int kBarBytes = kWarps * 2 * kStages * 8;  // mbarriers at the start of dynamic shared memory
-
-// Programmatic dependent launch: the partial and merge kernels of consecutive calls are launched with the
-// stream-serialization attribute, so a kernel's CTAs are scheduled while the previous kernel drains.  Each kernel
-// lets its successor go at once and waits for its predecessor's results before it reads or writes anything; both
-// instructions do nothing in a kernel that was launched without the attribute.
-__device__ __forceinline__ void pdl_release() {
-#if TQ_DEC_PDL
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-#endif
-}
-__device__ __forceinline__ void pdl_wait() {
-#if TQ_DEC_PDL
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-#endif
-}
-__device__ __forceinline__ void pdl_release_and_wait() {
-    pdl_release();
-    pdl_wait();
-}
-
-template <typename Kernel, typename... Args>
-cudaError_t launch_chained(Kernel kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
-#if TQ_DEC_PDL
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, args...);
-#else
-    kernel<<<grid, block, smem, stream>>>(args...);
-    return cudaGetLastError();
-#endif
-}
 
 struct DecodeParams {
     void* out;
@@ -326,7 +284,8 @@ __global__ void __launch_bounds__(kThreads, TQ_DEC_MINBLOCKS) decode_partial_ker
     __shared__ float sm_m[kWarps][8];
     __shared__ float sm_l[kWarps][8];
 
-    pdl_release_and_wait();
+    pdl_release();
+    pdl_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int gid = lane >> 2, tig = lane & 3;
     const int chunk = blockIdx.x;
@@ -640,7 +599,8 @@ constexpr int kChunkMergeWarps = 4;
 __global__ void __launch_bounds__(kChunkMergeWarps * 32) decode_merge_kernel(const DecodeParams p) {
     __shared__ float4 so[kChunkMergeWarps][32];
     __shared__ float2 sml[kChunkMergeWarps];
-    pdl_release_and_wait();
+    pdl_release();
+    pdl_wait();
     const int head = blockIdx.x, seq = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int L = p.seq_lens[seq];
     const int npages = min((L + kPageTokens - 1) / kPageTokens, p.max_pages);   // same cut as the partial kernel

@@ -104,26 +104,6 @@ __device__ __forceinline__ void lds_words(uint32_t addr, uint32_t (&w)[BITS]) {
     }
 }
 
-// Programmatic dependent launch of the merge kernel: its CTAs start while the partial kernel drains.  (The partial kernel is
-// launched without it: CTAs that start early are packed two to an SM next to those still running, and stay there.)
-__device__ __forceinline__ void pa_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void pa_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
-template <typename Kernel, typename... Args>
-bool pa_launch(Kernel kernel, bool chained, unsigned grid, unsigned block, size_t smem, cudaStream_t stream, Args... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = chained ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kernel, args...) == cudaSuccess;
-}
-
 constexpr int kPaStages = 2;   // ring of 16-token steps per warp: the one being worked on, the other in flight
 
 template <int BITS>
@@ -171,7 +151,7 @@ __global__ void __launch_bounds__(kPaThreads, 1) packed_attn_partial(const PAPar
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int slot = lane >> 2, quarter = lane & 3;
-    pa_release();
+    pdl_release();
 
     // ---- the CTA's segments ----
     const int steps = (p.Sk + kStepTokens - 1) / kStepTokens;   // per row
@@ -201,7 +181,10 @@ __global__ void __launch_bounds__(kPaThreads, 1) packed_attn_partial(const PAPar
     };
     int64_t at = p.num_splits > 0 ? static_cast<int64_t>(blockIdx.x) : u0;
     const int64_t stop = p.num_splits > 0 ? static_cast<int64_t>(n_items) : u1;
-    if (at >= stop) return;
+    if (at >= stop) {
+        pdl_wait();
+        return;
+    }
 
     // ---- item state: which segment the CTA works on, and the warp's asynchronous staging of it: per step a warp
     // copies its 16 K rows, 16 V rows and 16 sign rows in 16-byte pieces (every row is a multiple of 16 bytes, so any
@@ -267,8 +250,6 @@ __global__ void __launch_bounds__(kPaThreads, 1) packed_attn_partial(const PAPar
         for (int i = 0; i < kPaStages - 1; ++i) issue();
         load_norms(tok16, nrm);
     };
-    begin(at);
-
     // the pair tables depend on the codebook only.  Every lane holds one centroid; an entry's two come by shuffle.
     {
         const float cv = __ldg(p.centroids + (lane & ((1 << BITS) - 1)));
@@ -279,6 +260,8 @@ __global__ void __launch_bounds__(kPaThreads, 1) packed_attn_partial(const PAPar
             *reinterpret_cast<uint32_t*>(half_tab + (pr * 32 + lane) * 4) = pack_half2(c0, c1);
         }
     }
+    pdl_wait();
+    begin(at);
     const uint32_t lane8 = lane * 8, lane4 = lane * 4;
     // selector that gathers byte `quarter` of two sign words
     const uint32_t sel_lo = static_cast<uint32_t>(quarter) | (static_cast<uint32_t>(4 + quarter) << 4);
@@ -459,8 +442,8 @@ constexpr int kMergeWarps = 4;
 __global__ void __launch_bounds__(kMergeWarps * 32) packed_attn_merge(const PAParams p, int n_ctas) {
     __shared__ float4 so[kMergeWarps][32];
     __shared__ float sl[kMergeWarps];
-    pa_release();
-    pa_wait();
+    pdl_release();
+    pdl_wait();
     const int bh = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int64_t slot0, parts, step = 1;
     if (p.num_splits > 0) {
@@ -517,6 +500,8 @@ __global__ void __launch_bounds__(kMergeWarps * 32) packed_attn_merge(const PAPa
 
 // ---- row-wise WHT ----------------------------------------------------------------------
 __global__ void __launch_bounds__(128) wht_rows_kernel(const void* in, void* out, int dtype, int64_t n, float scale) {
+    pdl_release();
+    pdl_wait();
     const int lane = threadIdx.x & 31;
     const int64_t row = static_cast<int64_t>(blockIdx.x) * 4 + (threadIdx.x >> 5);
     if (row >= n) return;
@@ -647,13 +632,15 @@ extern "C" int tq_packed_attention(const void* Q, const void* Q_proj, const uint
     const int n_items = num_splits > 0 ? static_cast<int>(slots) : 0;
     bool launched = false;
     switch (bits) {
-        case 2: launched = pa_launch(packed_attn_partial<2>, false, grid, kPaThreads, PALayout<2>::kSmem, st, p, n_items); break;
-        case 3: launched = pa_launch(packed_attn_partial<3>, false, grid, kPaThreads, PALayout<3>::kSmem, st, p, n_items); break;
-        case 4: launched = pa_launch(packed_attn_partial<4>, false, grid, kPaThreads, PALayout<4>::kSmem, st, p, n_items); break;
+        case 2: launched = launch_chained(packed_attn_partial<2>, dim3(grid), dim3(kPaThreads), PALayout<2>::kSmem, st, p, n_items) == cudaSuccess; break;
+        case 3: launched = launch_chained(packed_attn_partial<3>, dim3(grid), dim3(kPaThreads), PALayout<3>::kSmem, st, p, n_items) == cudaSuccess; break;
+        case 4: launched = launch_chained(packed_attn_partial<4>, dim3(grid), dim3(kPaThreads), PALayout<4>::kSmem, st, p, n_items) == cudaSuccess; break;
     }
     if (!launched) return TQ_ERR_LAUNCH;
     if (num_splits == 1 || (num_splits == 0 && grid == 1)) return TQ_OK;   // every row was written whole
-    return pa_launch(packed_attn_merge, true, static_cast<unsigned>(BH), kMergeWarps * 32, 0, st, p, static_cast<int>(grid)) ? TQ_OK : TQ_ERR_LAUNCH;
+    return launch_chained(packed_attn_merge, dim3(static_cast<unsigned>(BH)), dim3(kMergeWarps * 32), 0, st, p, static_cast<int>(grid)) == cudaSuccess
+               ? TQ_OK
+               : TQ_ERR_LAUNCH;
 }
 
 extern "C" int tq_wht_rows(const void* in, void* out, int dtype, int64_t n_rows, float scale, tq_stream_t stream) {
@@ -662,6 +649,7 @@ extern "C" int tq_wht_rows(const void* in, void* out, int dtype, int64_t n_rows,
     if (dtype != TQ_DTYPE_F16 && dtype != TQ_DTYPE_BF16 && dtype != TQ_DTYPE_F32) return TQ_ERR_UNSUPPORTED;
     if ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15) return TQ_ERR_ARG;
     const unsigned grid = static_cast<unsigned>((n_rows + 3) / 4);
-    wht_rows_kernel<<<grid, 128, 0, reinterpret_cast<cudaStream_t>(stream)>>>(in, out, dtype, n_rows, scale);
-    return cudaGetLastError() == cudaSuccess ? TQ_OK : TQ_ERR_LAUNCH;
+    return launch_chained(wht_rows_kernel, dim3(grid), dim3(128), 0, reinterpret_cast<cudaStream_t>(stream), in, out, dtype, n_rows, scale) == cudaSuccess
+               ? TQ_OK
+               : TQ_ERR_LAUNCH;
 }
