@@ -87,6 +87,14 @@ __device__ __forceinline__ void table_words(const uint32_t* w, uint32_t (&mw)[4]
 __device__ __forceinline__ uint32_t even_pairs(uint32_t w, uint32_t two20) { return bit_select(w * two20, w, 0x0f0f0000u); }
 __device__ __forceinline__ uint32_t odd_pairs(uint32_t w, uint32_t two12) { return bit_select(w * two12, w, 0xf0f00000u); }
 
+// 2-bit V words: nibble e of either half holds the indices of dims 4 u + e for u = 2 j (low two bits) and 2 j + 1.  Two swaps
+// of fields make byte s' + 2 s of it (a, b) of dim e = s and (a, b) of dim e = s + 2 of u = 2 j + s': the two half2 of an
+// entry are then neighbouring registers of one product's A operand, as with the scores.
+__device__ __forceinline__ uint32_t paired_dims(uint32_t w, uint32_t two12) {
+    w = bit_select(bit_select(w, w * two12, 0x0f0f0000u), w >> 12, 0x0000f0f0u);
+    return bit_select(bit_select(w, w << 6, 0x33003300u), w >> 6, 0x00cc00ccu);
+}
+
 template <int BITS>
 __device__ __forceinline__ void fill_stream_table(uint32_t smem_addr, const float* __restrict__ c, int warp, int lane) {
     const float cv = __half2float(__float2half_rn(__ldg(c + (lane & ((1 << BITS) - 1)))));
@@ -169,10 +177,12 @@ __device__ __forceinline__ void wht_16x8(float (&x)[16], int lane) {
     for (int i = 0; i < 16; ++i) x[i] *= kWhtScale;
 }
 
-// Sign table: entry b holds the eight values +-1 of byte b as four half2, in the order of eight consecutive dims, 8 copies.
+// Sign table, indexed by one nibble of signs (four dims) of token A and one of token B: the four half2 of +-1 that are the A
+// operand of one score product, in its register order (A dims 0 1, B dims 0 1, A dims 2 3, B dims 2 3), 8 copies.  (With the
+// eight signs of a byte of one token per entry, every second register had to be moved before the products.)
 __device__ __forceinline__ void fill_sign_table(uint32_t smem_addr, int warp, int lane) {
     for (int b = warp; b < 256; b += kStreamWarps) {
-        const int pair = b >> (2 * (lane & 3));
+        const int pair = b >> (((lane & 1) << 2) | (lane & 2));
         const uint32_t v = 0xBC00BC00u ^ ((pair & 1) ? 0x8000u : 0u) ^ ((pair & 2) ? 0x80000000u : 0u);
         asm volatile("st.shared.u32 [%0], %1;" ::"r"(smem_addr + b * 256 + lane * 4), "r"(v) : "memory");
     }
@@ -391,12 +401,17 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
             lds_words<NWK, 32 * NWK * 4>(ring_k + so, wb);
             float sm[4] = {0.f, 0.f, 0.f, 0.f};
             float sq[4] = {sq_init0, sq_init1, sq_init0, sq_init1}, sq2[4] = {0.f, 0.f, 0.f, 0.f};
+            uint32_t sgn0 = 0, sgn1 = 0;   // bytes: the nibbles 2 k (sgn0), 2 k + 1 (sgn1) of token A, then of token B
+            if constexpr (QJL && SIGN_TABLE) {
+                sgn0 = bit_select(wb[KB] << 4, wa[KB], 0x0f0f0f0fu);
+                sgn1 = bit_select(wb[KB], wa[KB] >> 4, 0x0f0f0f0fu);
+            }
             auto sign_term = [&](auto quarter) {   // eight dims of two tokens, two products
                 constexpr int B = decltype(quarter)::value;
                 if constexpr (QJL && SIGN_TABLE) {
-                    const uint4 ga = table_signs<B>(wa[KB], slut), gb = table_signs<B>(wb[KB], slut);
-                    mma_f16_16816(sq, ga.x, gb.x, ga.y, gb.y, qf[4 * B], qf[4 * B + 1]);
-                    mma_f16_16816(sq2, ga.z, gb.z, ga.w, gb.w, qf[4 * B + 2], qf[4 * B + 3]);
+                    const uint4 g0 = table_signs<B>(sgn0, slut), g1 = table_signs<B>(sgn1, slut);
+                    mma_f16_16816(sq, g0.x, g0.y, g0.z, g0.w, qf[4 * B], qf[4 * B + 1]);
+                    mma_f16_16816(sq2, g1.x, g1.y, g1.z, g1.w, qf[4 * B + 2], qf[4 * B + 3]);
                 } else if constexpr (QJL) {
                     const uint32_t xa = wa[KB] << (4 * B), xb = wb[KB] << (4 * B);
                     mma_f16_16816(sq, and_or(xa, 0x80008000u, 0x3C003C00u), and_or(xb, 0x80008000u, 0x3C003C00u),
@@ -406,17 +421,28 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
                 }
             };
             if constexpr (KB == 2) {
+                // An entry holds two half2.  Its byte is made of the pair of indices of token A and that of token B, so that
+                // the two are neighbouring registers of the A operand.
                 auto quads = [&](auto word) {
                     constexpr int J = decltype(word)::value;
-                    const uint2 a0 = table_quad<0>(wa[J], klut), a1 = table_quad<1>(wa[J], klut);
-                    const uint2 b0 = table_quad<0>(wb[J], klut), b1 = table_quad<1>(wb[J], klut);
-                    mma_f16_16816(sm, a0.x, b0.x, a1.x, b1.x, qf[8 * J], qf[8 * J + 1]);
-                    mma_f16_16816(sm, a0.y, b0.y, a1.y, b1.y, qf[8 * J + 4], qf[8 * J + 5]);
+                    const uint32_t y0 = bit_select(wb[J] << 2, wa[J], 0x33333333u), y1 = bit_select(wb[J], wa[J] >> 2, 0x33333333u);
+                    {
+                        const uint2 a = table_quad<0>(y0, klut), b = table_quad<1>(y0, klut);
+                        mma_f16_16816(sm, a.x, a.y, b.x, b.y, qf[8 * J], qf[8 * J + 1]);
+                    }
+                    {
+                        const uint2 a = table_quad<0>(y1, klut), b = table_quad<1>(y1, klut);
+                        mma_f16_16816(sm, a.x, a.y, b.x, b.y, qf[8 * J + 4], qf[8 * J + 5]);
+                    }
                     sign_term(std::integral_constant<int, 2 * J>{});
-                    const uint2 c0 = table_quad<2>(wa[J], klut), c1 = table_quad<3>(wa[J], klut);
-                    const uint2 d0 = table_quad<2>(wb[J], klut), d1 = table_quad<3>(wb[J], klut);
-                    mma_f16_16816(sm, c0.x, d0.x, c1.x, d1.x, qf[8 * J + 2], qf[8 * J + 3]);
-                    mma_f16_16816(sm, c0.y, d0.y, c1.y, d1.y, qf[8 * J + 6], qf[8 * J + 7]);
+                    {
+                        const uint2 a = table_quad<2>(y0, klut), b = table_quad<3>(y0, klut);
+                        mma_f16_16816(sm, a.x, a.y, b.x, b.y, qf[8 * J + 2], qf[8 * J + 3]);
+                    }
+                    {
+                        const uint2 a = table_quad<2>(y1, klut), b = table_quad<3>(y1, klut);
+                        mma_f16_16816(sm, a.x, a.y, b.x, b.y, qf[8 * J + 6], qf[8 * J + 7]);
+                    }
                     sign_term(std::integral_constant<int, 2 * J + 1>{});
                 };
                 quads(std::integral_constant<int, 0>{});
@@ -527,20 +553,16 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
                 if constexpr (VB == 2) {
 #pragma unroll
                     for (int j = 0; j < 2; ++j) {
-                        {
-                            const uint32_t ya = even_pairs(va[j], sp.two20), yb = even_pairs(vb[j], sp.two20);
-                            const uint2 a0 = table_quad<2>(ya, vlut), a1 = table_quad<3>(ya, vlut);
-                            const uint2 a2 = table_quad<2>(yb, vlut), a3 = table_quad<3>(yb, vlut);
-                            mma_f16_16816(oacc[4 * j], a0.x, a1.x, a2.x, a3.x, back0, back1);
-                            mma_f16_16816(oacc[4 * j + 2], a0.y, a1.y, a2.y, a3.y, back0, back1);
-                        }
-                        {
-                            const uint32_t ya = odd_pairs(va[j], sp.two12), yb = odd_pairs(vb[j], sp.two12);
-                            const uint2 a0 = table_quad<2>(ya, vlut), a1 = table_quad<3>(ya, vlut);
-                            const uint2 a2 = table_quad<2>(yb, vlut), a3 = table_quad<3>(yb, vlut);
-                            mma_f16_16816(oacc[4 * j + 1], a0.x, a1.x, a2.x, a3.x, t0, t1);
-                            mma_f16_16816(oacc[4 * j + 3], a0.y, a1.y, a2.y, a3.y, t0, t1);
-                        }
+                        const uint32_t ya = paired_dims(va[j], sp.two12), yb = paired_dims(vb[j], sp.two12);
+                        auto product = [&](auto byte, float (&acc)[4]) {
+                            constexpr int B = decltype(byte)::value;
+                            const uint2 a = table_quad<B>(ya, vlut), b = table_quad<B>(yb, vlut);
+                            mma_f16_16816(acc, a.x, a.y, b.x, b.y, t0, t1);
+                        };
+                        product(std::integral_constant<int, 0>{}, oacc[4 * j]);
+                        product(std::integral_constant<int, 1>{}, oacc[4 * j + 2]);
+                        product(std::integral_constant<int, 2>{}, oacc[4 * j + 1]);
+                        product(std::integral_constant<int, 3>{}, oacc[4 * j + 3]);
                     }
                 } else {
                     uint32_t ma[4], mb[4];
