@@ -221,6 +221,19 @@ __device__ __forceinline__ void store_v_paged(uint8_t* vpart, int t, int quarter
     if (quarter == 0) reinterpret_cast<__half*>(vpart + 256 * BITS)[norm_slot(t)] = __float2half_rn(q.norm);
 }
 
+// Division by a number that is usually a power of two: a shift then.
+struct Divisor {
+    uint32_t d;
+    int shift;   // -1: not a power of two
+    __device__ __forceinline__ uint32_t operator()(uint32_t n) const { return shift >= 0 ? n >> shift : n / d; }
+};
+Divisor divisor(int d) {
+    Divisor r = {static_cast<uint32_t>(d), -1};
+    if ((d & (d - 1)) == 0)
+        for (r.shift = 0; (1 << r.shift) < d;) ++r.shift;
+    return r;
+}
+
 struct PagedParams {
     const void* key;
     const void* value;
@@ -235,6 +248,7 @@ struct PagedParams {
     int64_t n_items;   // n_tokens * n_kv_heads
     int64_t n_tokens;
     int Hkv, block_size, in_dtype, rotate;
+    Divisor div_heads, div_block;
     int use_tcgen05;       // TQ_COMPRESS_TCGEN05 was given
 };
 
@@ -259,14 +273,9 @@ __device__ __forceinline__ ItemId identify_item(const PagedParams& p, int64_t it
     id.tok = 0; id.head = 0;
     id.live = item < p.n_items;
     if (id.live) {
-        if (p.n_items <= 0x7fffffff) {   // uniform over the grid: 32-bit division is several times cheaper
-            const uint32_t tk = static_cast<uint32_t>(item) / static_cast<uint32_t>(p.Hkv);
-            id.tok = tk;
-            id.head = static_cast<int>(static_cast<uint32_t>(item) - tk * static_cast<uint32_t>(p.Hkv));
-        } else {
-            id.tok = item / p.Hkv;
-            id.head = static_cast<int>(item - id.tok * p.Hkv);
-        }
+        const uint32_t tk = p.div_heads(static_cast<uint32_t>(item));   // launches have at most 2^30 items
+        id.tok = tk;
+        id.head = static_cast<int>(static_cast<uint32_t>(item) - tk * static_cast<uint32_t>(p.Hkv));
     }
     return id;
 }
@@ -284,7 +293,7 @@ __device__ __forceinline__ ItemPlace place_item(const PagedParams& p, const Item
             w.live = false;
         } else {
             int64_t blk;
-            if (p.num_slots <= 0x7fffffff) blk = static_cast<uint32_t>(slot) / static_cast<uint32_t>(p.block_size);
+            if (p.num_slots <= 0x7fffffff) blk = p.div_block(static_cast<uint32_t>(slot));
             else blk = slot / p.block_size;
             const int off = static_cast<int>(slot - blk * p.block_size);
             const int spb = p.block_size / kPageTokens;
@@ -440,7 +449,7 @@ __device__ __forceinline__ void compress_contig_rows(const ContigParams& p, int6
 }
 
 template <int BITS, OutMode MODE>
-__global__ void __launch_bounds__(kWarpsPerCta * 32) compress_contig_kernel(const ContigParams p) {
+__global__ void __launch_bounds__(kWarpsPerCta * 32) compress_contig_kernel(const __grid_constant__ ContigParams p) {
     __shared__ float csm[1 << BITS];
     pdl_release();
     if (threadIdx.x < (1 << BITS)) csm[threadIdx.x] = p.c ? p.c[threadIdx.x] : 0.f;
@@ -630,13 +639,13 @@ __device__ __forceinline__ void store_contig_fast(const ContigParams& p, int64_t
     store_contig_tail<QJL>(p, row, quarter, q.signs, q.norm, q.rnorm, live);
 }
 
-template <int BITS, bool QJL>
-__global__ void __launch_bounds__(kFastWarps * 32, 1) compress_contig_fast_kernel(const ContigParams p, int64_t n_units) {
+template <int BITS, bool QJL, Rows ROWS>
+__global__ void __launch_bounds__(kFastWarps * 32, 1) compress_contig_fast_kernel(const __grid_constant__ ContigParams p, int64_t n_units) {
     extern __shared__ __align__(128) unsigned char tables[];
     __shared__ float csm[1 << BITS];
     __shared__ int bad;
     const int lane = threadIdx.x & 31, quarter = lane & 3, warp = threadIdx.x >> 5;
-    const bool mma = p.rotate && p.in_dtype != TQ_DTYPE_F32;
+    constexpr bool mma = ROWS != Rows::kPlain, BF16 = ROWS == Rows::kBF16;
     const uint32_t buf = ((smem_u32(tables) + kTableBytes + 255) & ~255u) + warp * kStagePerWarp;   // two buffers of 8 rows
     const uint32_t dst = stage_at(buf, lane), src = staged_at(buf, lane);
     // units of 8 rows; as in the paged kernel the last round is spread over all SMs, and the first copies go out first
@@ -645,36 +654,34 @@ __global__ void __launch_bounds__(kFastWarps * 32, 1) compress_contig_fast_kerne
     auto row_of = [&](int64_t u) { return u * kItemsPerWarp + (lane >> 2); };
     pdl_release();
     pdl_wait();
-    if (mma) {
+    if constexpr (mma) {
         stage_row(dst, p.x, row_of(unit) * kHeadDim + 8 * quarter, row_of(unit) < p.n);
         stage_row(dst + kRowBuffer, p.x, row_of(unit + step) * kHeadDim + 8 * quarter, row_of(unit + step) < p.n);
     }
     if (threadIdx.x == 0) bad = 0;
     if (threadIdx.x < (1 << BITS)) csm[threadIdx.x] = p.c ? p.c[threadIdx.x] : 0.f;
     __syncthreads();
-    if (!mma) build_table<BITS, QJL>(tables, p.b, p.c, &bad);
+    if constexpr (!mma) build_table<BITS, QJL>(tables, p.b, p.c, &bad);
     else if constexpr (BITS > 2) build_table<BITS, QJL, true>(tables, p.b, p.c, &bad);
     __syncthreads();
     if (bad != 0) {   // two boundaries inside one cell: the generic quantizer
         asm volatile("cp.async.wait_group 0;" ::: "memory");
-        const ContigParams pc = p;
         for (; unit < n_units; unit += step)
-            compress_contig_rows<BITS, QJL ? OutMode::kPackedK : OutMode::kPackedV>(pc, row_of(unit), lane, csm);
+            compress_contig_rows<BITS, QJL ? OutMode::kPackedK : OutMode::kPackedV>(p, row_of(unit), lane, csm);
         return;
     }
     constexpr uint32_t kBias = kMagicBits * static_cast<uint32_t>(kCellStride);   // modulo 2^32
     const uint32_t tab = smem_u32(tables) + (QJL ? (lane & 7) * 16 : (lane & 15) * 8) - kBias;
     Packed q;
-    if (mma) {
-        const bool bf16 = p.in_dtype == TQ_DTYPE_BF16;
-        const WhtFragments hf = make_wht_fragments(lane, bf16);
+    if constexpr (mma) {
+        const WhtFragments hf = make_wht_fragments(lane, BF16);
         Codebook2<BITS> cb;
         if constexpr (BITS == 2) cb.load(p.b, QJL ? p.c : nullptr);
         uint32_t cur = 0;   // offset of the buffer whose turn it is
         for (; unit < n_units; unit += step, cur ^= kRowBuffer) {
             const int64_t row = row_of(unit), nxt = row_of(unit + 2 * step);
             wait_staged();
-            compress_row_mma<BITS, QJL, false, true>(src + cur, row < p.n, lane, bf16, hf, tab, cb, q, [&] {
+            compress_row_mma<BF16, BITS, QJL, false, true>(src + cur, row < p.n, lane, hf, tab, cb, q, [&] {
                 stage_row(dst + cur, p.x, nxt * kHeadDim + 8 * quarter, nxt < p.n);
             });
             store_contig_fast<BITS, QJL>(p, row, quarter, q);
@@ -701,14 +708,17 @@ int launch_contig_fast(const ContigParams& p, cudaStream_t st) {
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return TQ_ERR_LAUNCH;
     const unsigned grid = static_cast<unsigned>(n_units < sms ? n_units : sms);
     constexpr int kSmem = kTableBytes + kFastWarps * kStagePerWarp + 256;
-    static bool configured[64] = {false};
-    if (dev < 0 || dev >= 64 || !configured[dev]) {
-        if (cudaFuncSetAttribute(compress_contig_fast_kernel<BITS, QJL>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) !=
-            cudaSuccess)
-            return TQ_ERR_LAUNCH;
-        if (dev >= 0 && dev < 64) configured[dev] = true;
-    }
-    return launch_chained(compress_contig_fast_kernel<BITS, QJL>, dim3(grid), dim3(kFastWarps * 32), kSmem, st, p, n_units) == cudaSuccess ? TQ_OK : TQ_ERR_LAUNCH;
+    auto run = [&](auto kernel, bool (&configured)[64]) {
+        if (dev < 0 || dev >= 64 || !configured[dev]) {
+            if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) != cudaSuccess) return TQ_ERR_LAUNCH;
+            if (dev >= 0 && dev < 64) configured[dev] = true;
+        }
+        return launch_chained(kernel, dim3(grid), dim3(kFastWarps * 32), kSmem, st, p, n_units) == cudaSuccess ? TQ_OK : TQ_ERR_LAUNCH;
+    };
+    static bool configured[3][64] = {};
+    if (!p.rotate || p.in_dtype == TQ_DTYPE_F32) return run(compress_contig_fast_kernel<BITS, QJL, Rows::kPlain>, configured[0]);
+    if (p.in_dtype == TQ_DTYPE_F16) return run(compress_contig_fast_kernel<BITS, QJL, Rows::kF16>, configured[1]);
+    return run(compress_contig_fast_kernel<BITS, QJL, Rows::kBF16>, configured[2]);
 }
 
 template <int KB, int VB>
@@ -804,16 +814,31 @@ extern "C" int tq_compress_paged(const void* key, const void* value, int in_dtyp
     p.n_tokens = n_tokens;
     p.Hkv = n_kv_heads;
     p.block_size = block_size;
+    p.div_heads = divisor(n_kv_heads);
+    p.div_block = divisor(block_size);
     p.in_dtype = in_dtype;
     p.rotate = (prerotated & 1) ? 0 : 1;
     p.use_tcgen05 = (prerotated & TQ_COMPRESS_TCGEN05) ? 1 : 0;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    switch (k_bits) {
-        case 2: return launch_paged_v<2>(p, v_bits, use_qjl != 0, st);
-        case 3: return launch_paged_v<3>(p, v_bits, use_qjl != 0, st);
-        case 4: return launch_paged_v<4>(p, v_bits, use_qjl != 0, st);
+    // The kernels count items in 32 bits: a launch covers at most 2^30 of them (and an even number of tokens).
+    const int64_t most = n_kv_heads < (1 << 29) ? ((int64_t{1} << 30) / n_kv_heads) & ~int64_t{1} : 0;
+    if (most < 2) return TQ_ERR_UNSUPPORTED;
+    for (int64_t first = 0; first < n_tokens; first += most) {
+        PagedParams part = p;
+        part.key = static_cast<const uint8_t*>(key) + first * k_stride_token * elem_bytes(in_dtype);
+        part.value = static_cast<const uint8_t*>(value) + first * v_stride_token * elem_bytes(in_dtype);
+        part.slot_mapping = slot_mapping + first;
+        part.n_tokens = n_tokens - first < most ? n_tokens - first : most;
+        part.n_items = part.n_tokens * n_kv_heads;
+        int rc = TQ_ERR_UNSUPPORTED;
+        switch (k_bits) {
+            case 2: rc = launch_paged_v<2>(part, v_bits, use_qjl != 0, st); break;
+            case 3: rc = launch_paged_v<3>(part, v_bits, use_qjl != 0, st); break;
+            case 4: rc = launch_paged_v<4>(part, v_bits, use_qjl != 0, st); break;
+        }
+        if (rc != TQ_OK) return rc;
     }
-    return TQ_ERR_UNSUPPORTED;
+    return TQ_OK;
 }
 
 extern "C" int tq_compress_k(const void* K, int in_dtype, int64_t n, const float* centroids, const float* boundaries,

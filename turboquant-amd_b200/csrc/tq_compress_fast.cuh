@@ -457,6 +457,10 @@ struct WhtFragments {
     uint32_t b0[2], b1[2];   // B operand (16 x 8, +-1.0 in the input type) for nt = 0, 1
 };
 
+// What the rows of a launch are: already rotated or fp32 (no tensor cores), or fp16 / bf16 rows still to be rotated.  A template
+// parameter: decided at run time, both kinds of every MMA were issued, one of them predicated off.
+enum class Rows { kPlain, kF16, kBF16 };
+
 __device__ __forceinline__ WhtFragments make_wht_fragments(int lane, bool bf16) {
     const int g = lane >> 2, tig = lane & 3;
     const uint32_t one = bf16 ? 0x3F80u : 0x3C00u;
@@ -473,10 +477,10 @@ __device__ __forceinline__ WhtFragments make_wht_fragments(int lane, bool bf16) 
 }
 
 // D (+)= A B, m16n8k8, fp32 accumulate; ZERO starts from a zero accumulator.
-template <bool ZERO>
-__device__ __forceinline__ void mma_k8(bool bf16, float (&d)[4], uint32_t a0, uint32_t a1, uint32_t b0) {
+template <bool BF16, bool ZERO>
+__device__ __forceinline__ void mma_k8(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t b0) {
     const float z = 0.f;
-    if (bf16) {
+    if constexpr (BF16) {
         if constexpr (ZERO)
             asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%7,%7,%7,%7};"
                          : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3]) : "r"(a0), "r"(a1), "r"(b0), "f"(z));
@@ -491,12 +495,6 @@ __device__ __forceinline__ void mma_k8(bool bf16, float (&d)[4], uint32_t a0, ui
             asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
                          : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(b0));
     }
-}
-
-__device__ __forceinline__ void mma_zero(bool bf16, float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
-                                         uint32_t b0, uint32_t b1) {
-    if (bf16) mma_16816_zero<true>(d, a0, a1, a2, a3, b0, b1);
-    else mma_16816_zero<false>(d, a0, a1, a2, a3, b0, b1);
 }
 
 // row: staged_at(...) of this lane (piece j is at row ^ 16 j).
@@ -515,20 +513,20 @@ __device__ __forceinline__ void read_staged(uint32_t row, bool live, uint32_t (&
 
 // after_read() is called once the staged row has been read for the last time (the caller requests the next row
 // into the same buffer there).
-template <int BITS, bool QJL, bool ISV, bool CONTIG = false, class AfterRead>
-__device__ __forceinline__ void compress_row_mma(uint32_t row, bool live, int lane, bool bf16, const WhtFragments& hf,
+template <bool BF16, int BITS, bool QJL, bool ISV, bool CONTIG = false, class AfterRead>
+__device__ __forceinline__ void compress_row_mma(uint32_t row, bool live, int lane, const WhtFragments& hf,
                                                  uint32_t tab, const Codebook2<BITS>& cb, Packed& out, AfterRead after_read) {
     constexpr float kStep = CONTIG ? static_cast<float>(1 << BITS) : 16.f;   // spacing of a chunk's four indices
     uint32_t w[16];
     read_staged(row, live, w);
     // ||x||^2: even words on the diagonal of rows 0..7 of da, odd words on that of rows 8..15 of db
     float da[4], db[4];
-    mma_k8<true>(bf16, da, w[0], w[1], w[0]);
-    mma_k8<true>(bf16, db, w[0], w[1], w[1]);
+    mma_k8<BF16, true>(da, w[0], w[1], w[0]);
+    mma_k8<BF16, true>(db, w[0], w[1], w[1]);
 #pragma unroll
     for (int m = 1; m < 8; ++m) {
-        mma_k8<false>(bf16, da, w[2 * m], w[2 * m + 1], w[2 * m]);
-        mma_k8<false>(bf16, db, w[2 * m], w[2 * m + 1], w[2 * m + 1]);
+        mma_k8<BF16, false>(da, w[2 * m], w[2 * m + 1], w[2 * m]);
+        mma_k8<BF16, false>(db, w[2 * m], w[2 * m + 1], w[2 * m + 1]);
     }
     const int g = lane >> 2;
     const float diag = (g & 1) ? da[1] + db[3] : da[0] + db[2];   // column g sits in lane (g, g >> 1)
@@ -559,7 +557,7 @@ __device__ __forceinline__ void compress_row_mma(uint32_t row, bool live, int la
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             float d[4];
-            mma_zero(bf16, d, w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3], hf.b0[nt], hf.b1[nt]);
+            mma_16816_zero<BF16>(d, w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3], hf.b0[nt], hf.b1[nt]);
             y[2 * j] = f2pack(d[0], d[1]);
             y[2 * j + 1] = f2pack(d[2], d[3]);
         }
@@ -722,20 +720,12 @@ __device__ __noinline__ void compress_items_plain(const void* key, const void* v
 // ---- kernel -----------------------------------------------------------------------------------------------
 // Item order of the tensor-core loop: items 2 i and 2 i + 1 are two neighbouring tokens of one head (for store_v_pair);
 // with an odd token count the last partner is not live.
-__device__ __forceinline__ int64_t paired_items(const PagedParams& p) { return (p.n_tokens + 1) / 2 * 2 * p.Hkv; }
-__device__ __forceinline__ ItemId identify_paired(const PagedParams& p, int64_t item) {
+__device__ __forceinline__ uint32_t paired_items(const PagedParams& p) { return static_cast<uint32_t>(p.n_tokens + 1) / 2 * 2 * p.Hkv; }
+__device__ __forceinline__ ItemId identify_paired(const PagedParams& p, uint32_t item) {
     ItemId id;
-    const int64_t two = item >> 1;
-    if (p.n_items <= 0x3fffffff) {
-        const uint32_t tp = static_cast<uint32_t>(two) / static_cast<uint32_t>(p.Hkv);
-        id.tok = 2 * tp;
-        id.head = static_cast<int>(static_cast<uint32_t>(two) - tp * static_cast<uint32_t>(p.Hkv));
-    } else {
-        const int64_t tp = two / p.Hkv;
-        id.tok = 2 * tp;
-        id.head = static_cast<int>(two - tp * p.Hkv);
-    }
-    id.tok += item & 1;
+    const uint32_t two = item >> 1, tp = p.div_heads(two);
+    id.head = static_cast<int>(two - tp * p.Hkv);
+    id.tok = 2 * tp + (item & 1);
     id.live = id.tok < p.n_tokens;
     return id;
 }
@@ -743,8 +733,8 @@ __device__ __forceinline__ ItemId identify_paired(const PagedParams& p, int64_t 
 // Persistent CTAs of 16 warps, one per SM: the tables are built once per CTA, then its warps stride over units of 8 (token,
 // head) items, first the keys then the values of a unit.  Unit u belongs to warp u / gridDim of CTA u % gridDim: the last,
 // partly filled round is spread over all SMs (3001 tokens x 8 heads: 2 rounds of 16 warps per SM on 40 SMs otherwise).
-template <int KB, int VB, bool QJL>
-__global__ void __launch_bounds__(kFastWarps * 32, TQ_CMP_MINBLOCKS) compress_paged_fast_kernel(const PagedParams p, int64_t n_groups) {
+template <int KB, int VB, bool QJL, Rows ROWS>
+__global__ void __launch_bounds__(kFastWarps * 32, TQ_CMP_MINBLOCKS) compress_paged_fast_kernel(const __grid_constant__ PagedParams p, uint32_t n_groups) {
     constexpr int PAGE = page_bytes(KB, VB, QJL ? 1 : 0);
     constexpr int KPART = k_part_bytes(KB, QJL ? 1 : 0);
     extern __shared__ __align__(128) unsigned char tables[];
@@ -754,7 +744,7 @@ __global__ void __launch_bounds__(kFastWarps * 32, TQ_CMP_MINBLOCKS) compress_pa
     constexpr uint32_t kBias = kMagicBits * static_cast<uint32_t>(kCellStride);   // modulo 2^32
     const uint32_t ktab = smem_u32(tables) + (QJL ? (lane & 7) * 16 : (lane & 15) * 8) - kBias;
     const uint32_t vtab = smem_u32(tables + kTableBytes) + (lane & 15) * 8 - kBias;
-    const bool rotate = p.rotate != 0, mma = rotate && p.in_dtype != TQ_DTYPE_F32;
+    constexpr bool mma = ROWS != Rows::kPlain, BF16 = ROWS == Rows::kBF16;
 
     pdl_release();
     pdl_wait();
@@ -763,18 +753,18 @@ __global__ void __launch_bounds__(kFastWarps * 32, TQ_CMP_MINBLOCKS) compress_pa
     // arithmetic to hide behind.  The first ones are under way while the tables are built.
     const uint32_t kbuf = ((smem_u32(tables) + 2 * kTableBytes + 255) & ~255u) + warp * kStagePerWarp, vbuf = kbuf + kRowBuffer;
     const uint32_t kdst = stage_at(kbuf, lane), vdst = stage_at(vbuf, lane);
-    const int64_t units = (paired_items(p) + kItemsPerWarp - 1) / kItemsPerWarp;
-    const int64_t step = static_cast<int64_t>(gridDim.x) * kFastWarps;
-    int64_t unit = static_cast<int64_t>(warp) * gridDim.x + blockIdx.x;
+    const uint32_t units = (paired_items(p) + kItemsPerWarp - 1) / kItemsPerWarp;
+    const uint32_t step = gridDim.x * kFastWarps;
+    uint32_t unit = warp * gridDim.x + blockIdx.x;
     ItemId id = identify_paired(p, unit * kItemsPerWarp + (lane >> 2));
-    if (mma) {
+    if constexpr (mma) {
         stage_row(kdst, p.key, id.tok * p.ks_t + id.head * p.ks_h + 8 * quarter, id.live);
         stage_row(vdst, p.value, id.tok * p.vs_t + id.head * p.vs_h + 8 * quarter, id.live);
     }
     if (threadIdx.x == 0) bad = 0;
     if (threadIdx.x < (1 << KB)) csm[threadIdx.x] = p.kc[threadIdx.x];
     __syncthreads();
-    if (mma) {   // 2-bit codebooks need no table here
+    if constexpr (mma) {   // 2-bit codebooks need no table here
         if constexpr (KB > 2) build_table<KB, QJL, true>(tables, p.kb, p.kc, &bad);
         if constexpr (VB > 2) build_table<VB, false, true>(tables + kTableBytes, p.vb, nullptr, &bad);
     } else {
@@ -785,19 +775,17 @@ __global__ void __launch_bounds__(kFastWarps * 32, TQ_CMP_MINBLOCKS) compress_pa
     if (bad != 0 || !mma) {
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         const bool generic = bad != 0;
-        const int64_t item0 = warp * kItemsPerWarp + (lane >> 2);   // + group * 128
-        const PagedParams pc = p;   // the out-of-line calls take an address: keep the kernel parameters themselves in the constant bank
-        for (int64_t grp = blockIdx.x; grp < n_groups; grp += gridDim.x) {
-            if (generic) compress_items_generic<KB, VB, QJL>(pc, grp * kFastItemsPerCta + item0, lane, csm);
-            else
-                compress_items_plain<KB, VB, QJL>(p.key, p.value, p.ks_t, p.ks_h, p.vs_t, p.vs_h, p.in_dtype, rotate,
+        const uint32_t item0 = warp * kItemsPerWarp + (lane >> 2);   // + group * 128
+        for (uint32_t grp = blockIdx.x; grp < n_groups; grp += gridDim.x) {
+            if (generic) compress_items_generic<KB, VB, QJL>(p, grp * kFastItemsPerCta + item0, lane, csm);
+            else if constexpr (!mma)
+                compress_items_plain<KB, VB, QJL>(p.key, p.value, p.ks_t, p.ks_h, p.vs_t, p.vs_h, p.in_dtype, p.rotate != 0,
                                                   place_item<PAGE>(p, grp * kFastItemsPerCta + item0, quarter), lane, ktab, vtab);
         }
         return;
     }
-    const bool bf16 = p.in_dtype == TQ_DTYPE_BF16;
     const uint32_t krow = staged_at(kbuf, lane), vrow = staged_at(vbuf, lane);
-    const WhtFragments hf = make_wht_fragments(lane, bf16);
+    const WhtFragments hf = make_wht_fragments(lane, BF16);
     Codebook2<KB> kcb;
     Codebook2<VB> vcb;
     if constexpr (KB == 2) kcb.load(p.kb, QJL ? p.kc : nullptr);
@@ -815,12 +803,12 @@ __global__ void __launch_bounds__(kFastWarps * 32, TQ_CMP_MINBLOCKS) compress_pa
         unit += step;
         id = identify_paired(p, unit * kItemsPerWarp + (lane >> 2));
         wait_staged();
-        compress_row_mma<KB, QJL, false>(krow, w.live, lane, bf16, hf, ktab, kcb, q, [&] {
+        compress_row_mma<BF16, KB, QJL, false>(krow, w.live, lane, hf, ktab, kcb, q, [&] {
             stage_row(kdst, p.key, id.tok * p.ks_t + id.head * p.ks_h + 8 * quarter, id.live);
         });
         if (w.live) store_k_fast<KB, QJL>(w.page, w.t, quarter, q);
         wait_staged();
-        compress_row_mma<VB, false, true>(vrow, w.live, lane, bf16, hf, vtab, vcb, q, [&] {
+        compress_row_mma<BF16, VB, false, true>(vrow, w.live, lane, hf, vtab, vcb, q, [&] {
             stage_row(vdst, p.value, id.tok * p.vs_t + id.head * p.vs_h + 8 * quarter, id.live);
         });
         if (pairs) {
@@ -834,7 +822,7 @@ __global__ void __launch_bounds__(kFastWarps * 32, TQ_CMP_MINBLOCKS) compress_pa
 
 // Small launches (the new tokens of one decode step): no tables to build, one group of 32 items per CTA.
 template <int KB, int VB, bool QJL>
-__global__ void __launch_bounds__(kWarpsPerCta * 32) compress_paged_small_kernel(const PagedParams p) {
+__global__ void __launch_bounds__(kWarpsPerCta * 32) compress_paged_small_kernel(const __grid_constant__ PagedParams p) {
     __shared__ float csm[1 << KB];
     pdl_release();
     if (threadIdx.x < (1 << KB)) csm[threadIdx.x] = p.kc[threadIdx.x];
@@ -862,7 +850,8 @@ int launch_paged_fast(const PagedParams& p, cudaStream_t st) {
     // on request: fp16 / bf16 rows that still need the rotation go to the tensor-memory kernel (rotation as one
     // 128 x 128 x 128 product per 128 rows, one thread per vector afterwards)
     if (p.rotate && p.in_dtype != TQ_DTYPE_F32 && p.use_tcgen05) return launch_paged_tc<KB, VB, QJL>(p, st);
-    const int64_t n_groups = (p.n_items + kFastItemsPerCta - 1) / kFastItemsPerCta, n_units = (p.n_items + kItemsPerWarp - 1) / kItemsPerWarp;
+    const uint32_t n_groups = static_cast<uint32_t>((p.n_items + kFastItemsPerCta - 1) / kFastItemsPerCta);
+    const int64_t n_units = (p.n_items + kItemsPerWarp - 1) / kItemsPerWarp;
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return TQ_ERR_LAUNCH;
     static int sm_count[64] = {0};
@@ -874,14 +863,17 @@ int launch_paged_fast(const PagedParams& p, cudaStream_t st) {
     const int64_t resident = static_cast<int64_t>(sms) * TQ_CMP_MINBLOCKS;
     const unsigned grid = static_cast<unsigned>(n_units < resident ? n_units : resident);
     constexpr int kSmem = 2 * kTableBytes + kFastWarps * kStagePerWarp + 256;
-    static bool configured[64] = {false};
-    if (dev < 0 || dev >= 64 || !configured[dev]) {
-        if (cudaFuncSetAttribute(compress_paged_fast_kernel<KB, VB, QJL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 kSmem) != cudaSuccess)
-            return TQ_ERR_LAUNCH;
-        if (dev >= 0 && dev < 64) configured[dev] = true;
-    }
-    return launch_chained(compress_paged_fast_kernel<KB, VB, QJL>, dim3(grid), dim3(kFastWarps * 32), kSmem, st, p, n_groups) == cudaSuccess ? TQ_OK : TQ_ERR_LAUNCH;
+    auto run = [&](auto kernel, bool (&configured)[64]) {
+        if (dev < 0 || dev >= 64 || !configured[dev]) {
+            if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) != cudaSuccess) return TQ_ERR_LAUNCH;
+            if (dev >= 0 && dev < 64) configured[dev] = true;
+        }
+        return launch_chained(kernel, dim3(grid), dim3(kFastWarps * 32), kSmem, st, p, n_groups) == cudaSuccess ? TQ_OK : TQ_ERR_LAUNCH;
+    };
+    static bool configured[3][64] = {};
+    if (!p.rotate || p.in_dtype == TQ_DTYPE_F32) return run(compress_paged_fast_kernel<KB, VB, QJL, Rows::kPlain>, configured[0]);
+    if (p.in_dtype == TQ_DTYPE_F16) return run(compress_paged_fast_kernel<KB, VB, QJL, Rows::kF16>, configured[1]);
+    return run(compress_paged_fast_kernel<KB, VB, QJL, Rows::kBF16>, configured[2]);
 }
 
 }  // namespace

@@ -104,7 +104,7 @@ __device__ __forceinline__ void quantize_half_fast(const uint32_t (&d)[16], cons
 }
 
 template <int KB, int VB, bool QJL>
-__global__ void __launch_bounds__(kTcThreads, 1) compress_paged_tc_kernel(const PagedParams p, int64_t n_tiles) {
+__global__ void __launch_bounds__(kTcThreads, 1) compress_paged_tc_kernel(const __grid_constant__ PagedParams p, int64_t n_tiles) {
     constexpr int PAGE = page_bytes(KB, VB, QJL ? 1 : 0);
     constexpr int KPART = k_part_bytes(KB, QJL ? 1 : 0);
     extern __shared__ __align__(128) unsigned char tsm[];
@@ -316,10 +316,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) compress_paged_tc_kernel(const 
         __shared__ float csm[16];
         if (tid < (1 << KB)) csm[tid] = p.kc[tid];
         asm volatile("bar.sync 5, 512;" ::: "memory");
-        const PagedParams pc = p;
         const int64_t n_groups = (p.n_items + kTcThreads / 4 - 1) / (kTcThreads / 4);
         for (int64_t grp = blockIdx.x; grp < n_groups; grp += gridDim.x)
-            compress_items_generic<KB, VB, QJL>(pc, grp * (kTcThreads / 4) + warp * kItemsPerWarp + (lane >> 2), lane, csm);
+            compress_items_generic<KB, VB, QJL>(p, grp * (kTcThreads / 4) + warp * kItemsPerWarp + (lane >> 2), lane, csm);
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
