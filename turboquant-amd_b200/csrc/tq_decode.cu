@@ -554,7 +554,7 @@ __global__ void __launch_bounds__(kThreads, TQ_DEC_MINBLOCKS) decode_partial_ker
 }
 
 // Weighted combination of partial rows by one warp: part(i) is the 128 sums of part i (fp32), ml(i) its (maximum,
-// denominator).  Four parts are fetched at a time, independently of one another and of the maxima: what a merge costs is the
+// denominator).  Eight parts are fetched at a time, independently of one another and of the maxima: what a merge costs is the
 // latency of its chain of loads.
 template <typename Part, typename Ml>
 __device__ __forceinline__ void merge_parts(int first, int step, int parts, int lane, Part part, Ml ml, float& M, float (&x)[4], float& l) {
@@ -562,11 +562,12 @@ __device__ __forceinline__ void merge_parts(int first, int step, int parts, int 
     l = 0.f;
 #pragma unroll
     for (int i = 0; i < 4; ++i) x[i] = 0.f;
-    for (int i0 = first; i0 < parts; i0 += 4 * step) {
-        float4 v[4];
-        float2 w[4];
+    constexpr int kAtOnce = 8;
+    for (int i0 = first; i0 < parts; i0 += kAtOnce * step) {
+        float4 v[kAtOnce];
+        float2 w[kAtOnce];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
+        for (int k = 0; k < kAtOnce; ++k) {
             const int i = i0 + k * step;
             if (i < parts) {
                 w[k] = ml(i);
@@ -576,13 +577,15 @@ __device__ __forceinline__ void merge_parts(int first, int step, int parts, int 
                 v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
             }
         }
-        const float m = fmaxf(fmaxf(M, fmaxf(w[0].x, w[1].x)), fmaxf(w[2].x, w[3].x));
+        float m = M;
+#pragma unroll
+        for (int k = 0; k < kAtOnce; ++k) m = fmaxf(m, w[k].x);
         const float old = ex2(M - m);
         l *= old;
 #pragma unroll
         for (int i = 0; i < 4; ++i) x[i] *= old;
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
+        for (int k = 0; k < kAtOnce; ++k) {
             const float sc = ex2(w[k].x - m);
             l = fmaf(sc, w[k].y, l);
             x[0] = fmaf(sc, v[k].x, x[0]);
@@ -698,17 +701,18 @@ int dispatch_v(const DecodeParams& p, int vb, const Plan& plan, cudaStream_t str
     return TQ_ERR_UNSUPPORTED;
 }
 
-// Which kernel is the better one, by the pages that the batch can have at most.  The persistent kernel pays about 13 us
+// Which kernel is the better one, by the pages that the batch can have at most.  The persistent kernel pays about 12 us
 // however few pages there are (all its tables, one more level of merging), the chunked one 8 to 11, but it takes
-// 0.43 (4-bit) to 0.6 us (with sign term) per 1000 pages where the chunked one takes 0.68 to 0.78.  Measured us, chunked /
-// persistent, 8 KV heads: turbo4 2 x 8192 tokens (8192 pages) 26.2 / 19.4, 4 x 2048 (4096 pages) 14.6 / 16.6; turbo3
-// 2 x 8192 22.2 / 20.7, 16 x 2048 (16384 pages) 27.1 / 26.9, 32 x 1024 26.9 / 27.4, 64 x 1024 39.4 / 39.6.
+// 0.45 (4-bit) to 0.55 us (with sign term) per 1000 pages where the chunked one takes 0.7 to 0.8; sequences of few pages
+// cost it more, a warp then changes item every few pages.  Measured us, chunked / persistent, 8 KV heads: turbo4 2 x 4096
+// tokens (4096 pages) 12.2 / 13.9, 4 x 4096 (8192 pages) 19.2 / 16.5, 64 x 256 17.2 / 16.8; turbo3 4 x 4096 16.3 / 17.4,
+// 1 x 16384 19.1 / 18.0, 64 x 512 (16384 pages) 21.5 / 24.5, 32 x 1024 24.3 / 23.3, 256 x 256 (32768 pages) 45.2 / 40.4.
 constexpr int64_t kStreamMinPages = 8192;
 constexpr int64_t kStreamSlots = static_cast<int64_t>(kStreamCtas) * (kStreamWarps + 2);   // partials of warps and of CTAs
 int64_t pages_at_most(int64_t ns, int64_t hq, int64_t hkv, int64_t max_pages) { return ns * max_pages * hkv * ((hq / hkv + 7) / 8); }
 bool stream_is_better(int64_t pages, int64_t cache_pages, int max_pages, bool qjl) {
     if (pages < kStreamMinPages || pages > INT32_MAX || cache_pages > UINT32_MAX) return false;
-    return !qjl || max_pages >= 512 || pages >= 49152 || (pages >= 16384 && max_pages >= 128);
+    return !qjl || max_pages >= 512 || pages >= 32768 || (pages >= 16384 && max_pages >= 64);
 }
 // Workspace of the persistent kernel, or 0 where no format would take it.
 int64_t stream_bytes(int64_t pages) {
@@ -882,7 +886,7 @@ extern "C" int tq_decode_paged(void* out, const void* q_rot, const void* q_proj,
     }
     if (rc != TQ_OK) return rc;
     if (persistent) {
-        if (launch_chained(decode_stream_merge_kernel, dim3(kStreamCtas), dim3(256), 0, st, sp) != cudaSuccess)
+        if (launch_chained(decode_stream_merge_kernel, dim3(kStreamCtas), dim3(kStreamMergeWarps * 32), 0, st, sp) != cudaSuccess)
             return TQ_ERR_LAUNCH;
     } else if (max_chunks > 1) {
         if (launch_chained(decode_merge_kernel, dim3(num_q_heads, num_seqs), dim3(kChunkMergeWarps * 32), 0, st, p) != cudaSuccess)

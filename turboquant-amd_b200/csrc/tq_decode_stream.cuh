@@ -1,8 +1,8 @@
 // Decode attention for launches that fill the GPU: one persistent CTA of 16 warps per SM, every warp streams its own
 // contiguous share of all pages.
 //
-// All (sequence, KV head, query group) items of the batch are laid end to end, page after page; warp w of W takes pages
-// [w U / W, (w + 1) U / W).  The warps never wait for one another while they stream: a warp keeps its running maximum,
+// All (sequence, KV head, query group) items of the batch are laid end to end, page after page, and cut into one share per
+// warp, of equal length to within a page.  The warps never wait for one another while they stream: a warp keeps its running maximum,
 // denominators and accumulators while it stays inside an item and writes the output itself when it saw the whole item.
 // Otherwise it leaves a partial result; the CTA combines the partials of its 16 (neighbouring) warps and leaves at most
 // two of its own, the item it started in the middle of and the item it could not finish, for decode_stream_merge_kernel.
@@ -16,7 +16,7 @@ constexpr int kStreamThreads = kStreamWarps * 32;
 constexpr int kStreamStages = 4;
 constexpr int kStreamTable = 65536;          // 256 entries of 256 bytes: 128 bytes for K, 128 bytes for V
 constexpr int kStreamCtas = 148;             // one per SM
-constexpr int kStreamSmem = 229376;          // dynamic part of the 227 KB an SM gives one CTA
+constexpr int kStreamSmem = 227328;          // dynamic part of the 227 KB an SM gives one CTA
 constexpr int kStreamSlotFloats = 8 * kHeadDim;
 
 struct StreamParams {
@@ -28,6 +28,17 @@ struct StreamParams {
     int4* split;         // [n_ctas] item that starts in the CTA and ends in a later one: (sequence, item of it, last CTA or -1)
     uint32_t two12, two20;
     float weight_thresh; // Sparse-V: weights are relative to a reference at most one (log2) above the running maximum
+};
+
+// Shares of U pages for W warps: the first U % W have one page more.
+struct Shares {
+    uint32_t each, more;
+    __device__ __forceinline__ Shares(uint32_t pages, uint32_t warps) : each(pages / warps), more(pages % warps) {}
+    __device__ __forceinline__ uint32_t start(uint32_t w) const { return each * w + min(w, more); }
+    __device__ __forceinline__ uint32_t owner(uint32_t page) const {
+        const uint32_t longer = more * (each + 1);
+        return page < longer ? page / (each + 1) : more + (page - longer) / each;
+    }
 };
 
 __device__ __forceinline__ int pages_of(const DecodeParams& p, int len) {
@@ -220,6 +231,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
 
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ int sm_scan[kStreamThreads + 1];
+    __shared__ int sm_len[kStreamThreads];       // length of the first sequence of each thread's run
     __shared__ int sm_wsum[kStreamWarps];
     __shared__ int4 sm_part[2 * kStreamWarps];   // partials: (item or -1, sequence, pages of the item after this share, flags)
 
@@ -250,8 +262,13 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
 
     // ---- pages before each thread's run of sequences (every CTA does the same scan over all lengths)
     const int per = (sp.ns + kStreamThreads - 1) / kStreamThreads;
-    int own = 0;
-    for (int s = threadIdx.x * per; s < min(sp.ns, (static_cast<int>(threadIdx.x) + 1) * per); ++s) own += pages_of(p, p.seq_lens[s]);
+    int own = 0, len0 = 0;
+    for (int s = threadIdx.x * per; s < min(sp.ns, (static_cast<int>(threadIdx.x) + 1) * per); ++s) {
+        const int len = p.seq_lens[s];
+        if (s == static_cast<int>(threadIdx.x) * per) len0 = len;
+        own += pages_of(p, len);
+    }
+    sm_len[threadIdx.x] = len0;
     int incl = own;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -276,27 +293,30 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
     }
     __syncthreads();
 
-    const int64_t total = static_cast<int64_t>(sm_scan[kStreamThreads]) * sp.HG;
-    const int W = sp.n_warps;
-    const int gw = blockIdx.x * kStreamWarps + warp;
-    const int64_t first = total * gw / W;
-    const int n = static_cast<int>(total * (gw + 1) / W - first);   // this warp's pages
+    const uint32_t gw = blockIdx.x * kStreamWarps + warp;
+    uint32_t first;                                     // this warp's first page
+    int n;                                              // and how many it has
+    {
+        const Shares shares(static_cast<uint32_t>(sm_scan[kStreamThreads]) * sp.HG, sp.n_warps);   // at most 2^31 pages
+        first = shares.start(gw);
+        n = static_cast<int>(shares.start(gw + 1) - first);
+    }
 
     // ---- the item and page this warp starts in
     int seq = 0, hg = 0, page = 0, np = 0, len = 0;
     if (n > 0) {
-        int lo = 0, hi = kStreamThreads;
-        while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if (static_cast<int64_t>(sm_scan[mid]) * sp.HG <= first) lo = mid; else hi = mid;
-        }
+        // the last run that starts at or before page `first`: one probe of every 16th, one of the 16 after it
+        auto before = [&](int i) { return static_cast<uint32_t>(sm_scan[i]) * sp.HG <= first; };
+        int lo = 16 * (__popc(__ballot_sync(0xffffffffu, before(16 * lane))) - 1);
+        lo += __popc(__ballot_sync(0xffffffffu, lane < 16 && before(lo + (lane & 15)))) - 1;
         seq = lo * per;
-        int64_t at = static_cast<int64_t>(sm_scan[lo]) * sp.HG;
-        for (;; ++seq) {
-            len = __ldg(p.seq_lens + seq);
+        len = sm_len[lo];
+        uint32_t at = static_cast<uint32_t>(sm_scan[lo]) * sp.HG;
+        for (;;) {
             np = pages_of(p, len);
-            if (first < at + static_cast<int64_t>(np) * sp.HG) break;
-            at += static_cast<int64_t>(np) * sp.HG;
+            if (first < at + static_cast<uint32_t>(np) * sp.HG) break;
+            at += static_cast<uint32_t>(np) * sp.HG;
+            len = __ldg(p.seq_lens + ++seq);
         }
         const int r = static_cast<int>(first - at);
         hg = r / np;
@@ -680,7 +700,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
     // ---- combine the partials of the CTA's warps: entry 2 w (item that ended inside warp w's share) and 2 w + 1 (the one
     // its share ended in), in page order.  Warp (c, q) takes query row q of every other run of entries of one item.
     __syncthreads();
-    const int64_t all = static_cast<int64_t>(*static_cast<volatile int*>(sm_scan + kStreamThreads)) * sp.HG;   // `total`, not kept over the loop
+    const Shares shares(static_cast<uint32_t>(*static_cast<volatile int*>(sm_scan + kStreamThreads)) * sp.HG, sp.n_warps);
     const int4 part = sm_part[lane];
     const uint32_t live = __ballot_sync(0xffffffffu, part.x >= 0);
     const int prev = 31 - __clz(live & ((1u << lane) - 1u));   // the live entry before this one, or -1
@@ -698,9 +718,8 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
         const int after = __shfl_sync(0xffffffffu, part.z, last);
         if (starts && after > 0 && threadIdx.x == 0) {
             split = true;
-            const int64_t end = all * (static_cast<int64_t>(blockIdx.x + 1) * kStreamWarps) / W + after;   // pages before the item's end
-            // the warp whose share holds page u is the largest w with floor(w * total / W) <= u
-            sp.split[blockIdx.x] = make_int4(rseq, rhg, static_cast<int>((end * W - 1) / all) / kStreamWarps, 0);
+            const uint32_t end = shares.start((blockIdx.x + 1) * kStreamWarps) + after;   // pages before the item's end
+            sp.split[blockIdx.x] = make_int4(rseq, rhg, static_cast<int>(shares.owner(end - 1)) / kStreamWarps, 0);
         }
         if ((run & 1) != (warp >> 3)) continue;
         const int g = warp & 7;
@@ -721,18 +740,30 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
         float x[4] = {0.f, 0.f, 0.f, 0.f};
-        for (uint32_t rest = mine; rest; rest &= rest - 1) {
-            const int e = __ffs(rest) - 1;
-            float4 v;
-            if (e & 1)
-                asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(ring_of(e >> 1) + (g * kHeadDim + 4 * lane) * 4));
-            else
-                v = __ldcg(reinterpret_cast<const float4*>(sp.part_o + static_cast<int64_t>(blockIdx.x * kStreamWarps + (e >> 1)) * kStreamSlotFloats + g * kHeadDim + 4 * lane));
-            const float sc = __shfl_sync(0xffffffffu, scale, e);
-            x[0] = fmaf(sc, v.x, x[0]);
-            x[1] = fmaf(sc, v.y, x[1]);
-            x[2] = fmaf(sc, v.z, x[2]);
-            x[3] = fmaf(sc, v.w, x[3]);
+        for (uint32_t rest = mine; rest;) {   // two entries at a time
+            float4 v[2];
+            float sc[2];
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                const int e = rest ? __ffs(rest) - 1 : 32;
+                rest &= rest - 1;
+                sc[k] = __shfl_sync(0xffffffffu, scale, e & 31);
+                if (e == 32) {
+                    sc[k] = 0.f;
+                    v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+                } else if (e & 1) {
+                    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[k].x), "=f"(v[k].y), "=f"(v[k].z), "=f"(v[k].w) : "r"(ring_of(e >> 1) + (g * kHeadDim + 4 * lane) * 4));
+                } else {
+                    v[k] = __ldcg(reinterpret_cast<const float4*>(sp.part_o + static_cast<int64_t>(blockIdx.x * kStreamWarps + (e >> 1)) * kStreamSlotFloats + g * kHeadDim + 4 * lane));
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                x[0] = fmaf(sc[k], v[k].x, x[0]);
+                x[1] = fmaf(sc[k], v[k].y, x[1]);
+                x[2] = fmaf(sc[k], v[k].z, x[2]);
+                x[3] = fmaf(sc[k], v[k].w, x[3]);
+            }
         }
         if (starts && after == 0) {
             finish_row(p, rseq, rhg, g, lane, x, l);
@@ -766,19 +797,35 @@ int launch_stream(const StreamParams& sp, cudaStream_t stream) {
     return launch_stream_as<KB, VB, QJL, SPARSE, false>(sp, stream);
 }
 
-// One block per CTA of the stream kernel: combines the parts of the item that starts there and ends in a later CTA, one
-// warp per query row.
-__global__ void __launch_bounds__(256) decode_stream_merge_kernel(const StreamParams sp) {
+// One block per CTA of the stream kernel: combines the parts of the item that starts there and ends in a later CTA, two
+// warps per query row.
+constexpr int kStreamMergeWarps = 16;
+__global__ void __launch_bounds__(kStreamMergeWarps * 32) decode_stream_merge_kernel(const StreamParams sp) {
+    __shared__ float4 so[8][32];
+    __shared__ float2 sml[8];
     pdl_release();
     pdl_wait();
-    const int cta = blockIdx.x, g = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int cta = blockIdx.x, warp = threadIdx.x >> 5, g = warp & 7, half = warp >> 3, lane = threadIdx.x & 31;
     const int4 item = sp.split[cta];
     if (item.z < 0) return;
     auto slot_of = [&](int i) { return sp.n_warps + 2 * (cta + i) + (i == 0 ? 1 : 0); };   // slot 1 of this CTA, slot 0 of the others
     float M, l, x[4];
-    merge_parts(0, 1, item.z - cta + 1, lane, [&](int i) { return sp.part_o + static_cast<int64_t>(slot_of(i)) * kStreamSlotFloats + g * kHeadDim; },
+    merge_parts(half, 2, item.z - cta + 1, lane, [&](int i) { return sp.part_o + static_cast<int64_t>(slot_of(i)) * kStreamSlotFloats + g * kHeadDim; },
                 [&](int i) { return sp.part_ml[slot_of(i) * 8 + g]; }, M, x, l);
-    finish_row(sp.d, item.x, item.y, g, lane, x, l);
+    if (half == 1) {
+        so[g][lane] = make_float4(x[0], x[1], x[2], x[3]);
+        if (lane == 0) sml[g] = make_float2(M, l);
+    }
+    __syncthreads();
+    if (half == 1) return;
+    const float2 other = sml[g];   // at least two parts, so both halves have one
+    const float Ma = fmaxf(M, other.x), sa = ex2(M - Ma), sb = ex2(other.x - Ma);
+    const float4 v = so[g][lane];
+    x[0] = fmaf(sb, v.x, sa * x[0]);
+    x[1] = fmaf(sb, v.y, sa * x[1]);
+    x[2] = fmaf(sb, v.z, sa * x[2]);
+    x[3] = fmaf(sb, v.w, sa * x[3]);
+    finish_row(sp.d, item.x, item.y, g, lane, x, fmaf(sb, other.y, sa * l));
 }
 
 }  // namespace
