@@ -656,12 +656,12 @@ def config_dict(workload: str, layers: int, gpus: int) -> dict:
 
 def traffic_from_profile(workload: str, world: int):
     """DRAM bytes per launch of the dominant kernel from the committed ncu summary of this exact shape
-    (a line `traffic_bytes_per_launch: N` in profiles/decode_partial_turbo3_cfg3.md); None for other shapes."""
+    (a line `traffic_bytes_per_launch: N` in profiles/decode_stream_turbo3_cfg3.md); None for other shapes."""
     if workload != "cfg3" or world != 1:
         return None
     import re
     try:
-        with open(os.path.join(ROOT, "profiles", "decode_partial_turbo3_cfg3.md")) as fh:
+        with open(os.path.join(ROOT, "profiles", "decode_stream_turbo3_cfg3.md")) as fh:
             m = re.search(r"traffic_bytes_per_launch:\s*(\d+)", fh.read())
         return int(m.group(1)) if m else None
     except OSError:
@@ -819,7 +819,7 @@ def main():
                          # committed ncu summary; other shapes were not captured
                          "traffic": traffic_from_profile(args.workload, world),
                          "peak_source": peak_src,
-                         "kernel": "decode_partial_kernel (+ merge) per layer per GPU",
+                         "kernel": "decode_stream_kernel (+ merge) per layer per GPU",
                          "algorithmic_bytes_per_launch": bytes_layer_rank},
             "clocks": clocks,
             "gpu_launches": args.steps * layers * 2,
