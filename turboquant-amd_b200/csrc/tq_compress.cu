@@ -280,13 +280,13 @@ __device__ __forceinline__ ItemId identify_item(const PagedParams& p, int64_t it
     return id;
 }
 
+// slot: the token's entry of slot_mapping (not looked at unless id.live).
 template <int PAGE>
-__device__ __forceinline__ ItemPlace place_item(const PagedParams& p, const ItemId& id, int quarter) {
+__device__ __forceinline__ ItemPlace place_item(const PagedParams& p, const ItemId& id, int64_t slot, int quarter) {
     ItemPlace w;
     w.tok = id.tok; w.head = id.head; w.t = 0; w.page = nullptr;
     w.live = id.live;
     if (w.live) {
-        int64_t slot = p.slot_mapping[w.tok];
         if (slot < 0) slot = 0;   // the reference clamps padding slots to 0
         if (slot >= p.num_slots) {
             if (quarter == 0 && p.status) atomicOr(p.status, TQ_STATUS_BAD_SLOT);
@@ -302,6 +302,11 @@ __device__ __forceinline__ ItemPlace place_item(const PagedParams& p, const Item
         }
     }
     return w;
+}
+
+template <int PAGE>
+__device__ __forceinline__ ItemPlace place_item(const PagedParams& p, const ItemId& id, int quarter) {
+    return place_item<PAGE>(p, id, id.live ? p.slot_mapping[id.tok] : 0, quarter);
 }
 
 template <int PAGE>

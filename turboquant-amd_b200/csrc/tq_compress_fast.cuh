@@ -820,22 +820,53 @@ __global__ void __launch_bounds__(kFastWarps * 32, TQ_CMP_MINBLOCKS) compress_pa
     asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
-// Small launches (the new tokens of one decode step): no tables to build, one group of 32 items per CTA.
+// Small launches (the new tokens of one decode step): no tables to build.  Such a launch is one chain of latencies, so
+// a warp takes the keys or the values of 8 items, not both one after the other, its rows are requested together with
+// their slots, and the boundaries before the previous launch has ended.  Measured, us per launch in a graph of such launches,
+// both in one warp / now, 8 KV heads: turbo3 64 tokens 6.1 / 3.4, 1024 tokens 9.8 / 5.4, 2048 tokens 10.1 / 8.9; turbo4 64
+// tokens 6.2 / 3.5.
 template <int KB, int VB, bool QJL>
 __global__ void __launch_bounds__(kWarpsPerCta * 32) compress_paged_small_kernel(const __grid_constant__ PagedParams p) {
+    constexpr int PAGE = page_bytes(KB, VB, QJL ? 1 : 0);
     __shared__ float csm[1 << KB];
     pdl_release();
-    if (threadIdx.x < (1 << KB)) csm[threadIdx.x] = p.kc[threadIdx.x];
-    __syncthreads();
-    pdl_wait();
-    const int lane = threadIdx.x & 31;
-    const int64_t item = (static_cast<int64_t>(blockIdx.x) * kWarpsPerCta + (threadIdx.x >> 5)) * kItemsPerWarp + (lane >> 2);
-    compress_items_generic<KB, VB, QJL>(p, item, lane, csm);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, quarter = lane & 3;
+    const ItemId id = identify_item(p, (static_cast<int64_t>(blockIdx.x) * (kWarpsPerCta / 2) + (warp >> 1)) * kItemsPerWarp + (lane >> 2));
+    if (QJL && threadIdx.x < (1 << KB)) csm[threadIdx.x] = p.kc[threadIdx.x];
+    if (QJL) __syncthreads();
+    float x[32];
+#pragma unroll
+    for (int i = 0; i < 32; ++i) x[i] = 0.f;   // lanes past the end take part in the shuffles
+    int64_t slot = 0;
+    Quarter q;
+    if ((warp & 1) == 0) {
+        Boundaries<KB> bd;
+        bd.load(p.kb);
+        pdl_wait();
+        if (id.live) {
+            slot = p.slot_mapping[id.tok];
+            load32(p.key, id.tok * p.ks_t + id.head * p.ks_h + 32 * quarter, p.in_dtype, x);
+        }
+        const ItemPlace w = place_item<PAGE>(p, id, slot, quarter);
+        quantize_quarter<KB, QJL>(x, p.rotate != 0, lane, bd, csm, q);
+        if (w.live) store_k_paged<KB, QJL>(w.page, w.t, quarter, q);
+    } else {
+        Boundaries<VB> bd;
+        bd.load(p.vb);
+        pdl_wait();
+        if (id.live) {
+            slot = p.slot_mapping[id.tok];
+            load32(p.value, id.tok * p.vs_t + id.head * p.vs_h + 32 * quarter, p.in_dtype, x);
+        }
+        const ItemPlace w = place_item<PAGE>(p, id, slot, quarter);
+        quantize_quarter<VB, false>(x, p.rotate != 0, lane, bd, nullptr, q);
+        if (w.live) store_v_paged<VB>(w.page + k_part_bytes(KB, QJL ? 1 : 0), w.t, quarter, q);
+    }
 }
 
-// Up to here launches take the generic kernel, whose rotation is the plain butterfly.  The tensor-core kernel is a little faster
-// at these sizes too (turbo3, 8 KV heads, 64 tokens 5.5 us against 6.4, 2048 tokens 8.5 against 11.3), but its rotation
-// rounds differently, and a coordinate in a million would go to the neighbouring centroid.
+// Up to here launches take the small kernel, whose rotation is the plain butterfly.  The tensor-core kernel rounds its
+// rotation differently, and a coordinate in a million would go to the neighbouring centroid; it takes 8.5 us for turbo3, 2048
+// tokens, where the small kernel takes 8.9.
 constexpr int64_t kSmallLaunchItems = 16384;
 
 template <int KB, int VB, bool QJL>
@@ -844,7 +875,8 @@ int launch_paged_tc(const PagedParams& p, cudaStream_t st);   // tq_compress_tc.
 template <int KB, int VB, bool QJL>
 int launch_paged_fast(const PagedParams& p, cudaStream_t st) {
     if (p.n_items <= kSmallLaunchItems) {
-        const unsigned grid = static_cast<unsigned>((p.n_items + kItemsPerCta - 1) / kItemsPerCta);
+        constexpr int64_t kItems = kItemsPerCta / 2;   // every item has a key warp and a value warp
+        const unsigned grid = static_cast<unsigned>((p.n_items + kItems - 1) / kItems);
         return launch_chained(compress_paged_small_kernel<KB, VB, QJL>, dim3(grid), dim3(kWarpsPerCta * 32), 0, st, p) == cudaSuccess ? TQ_OK : TQ_ERR_LAUNCH;
     }
     // on request: fp16 / bf16 rows that still need the rotation go to the tensor-memory kernel (rotation as one
