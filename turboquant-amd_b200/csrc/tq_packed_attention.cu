@@ -442,8 +442,8 @@ constexpr int kMergeWarps = 4;
 __global__ void __launch_bounds__(kMergeWarps * 32) packed_attn_merge(const PAParams p, int n_ctas) {
     __shared__ float4 so[kMergeWarps][32];
     __shared__ float sl[kMergeWarps];
+    __shared__ float sm[kMergeWarps];
     pdl_release();
-    pdl_wait();
     const int bh = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int64_t slot0, parts, step = 1;
     if (p.num_splits > 0) {
@@ -454,7 +454,10 @@ __global__ void __launch_bounds__(kMergeWarps * 32) packed_attn_merge(const PAPa
         const int64_t total = static_cast<int64_t>(p.BH) * steps, first = static_cast<int64_t>(bh) * steps;
         // the CTA whose share holds step u is the largest c with floor(c total / n) <= u
         const int64_t c0 = ((first + 1) * n_ctas - 1) / total, c1 = ((first + steps) * n_ctas - 1) / total;
-        if (c0 == c1) return;                    // written by that CTA
+        if (c0 == c1) {                          // written by that CTA
+            pdl_wait();
+            return;
+        }
         slot0 = 2 * c0;                          // slot 2 c0 + 1, then 2 c for the others
         parts = c1 - c0 + 1;
         step = 2;
@@ -462,36 +465,63 @@ __global__ void __launch_bounds__(kMergeWarps * 32) packed_attn_merge(const PAPa
     auto slot_of = [&](int64_t i) { return slot0 + step * i + (step == 2 && i == 0 ? 1 : 0); };
     const float2* lse = p.ws_lse;
     const float4* part = reinterpret_cast<const float4*>(p.ws_acc);
-    float M = -INFINITY;
-    for (int64_t i = lane; i < parts; i += 32) M = fmaxf(M, lse[slot_of(i)].x);
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
+    pdl_wait();
+    // four parts at a time, fetched independently of the maxima
+    float M = -INFINITY, l = 0.f;
     float4 o4 = make_float4(0.f, 0.f, 0.f, 0.f);
-    float l = 0.f;
-#pragma unroll 4
-    for (int64_t i = warp; i < parts; i += kMergeWarps) {
-        const int64_t s = slot_of(i);
-        const float2 ml = lse[s];
-        const float w = (ml.x == -INFINITY) ? 0.f : pa_ex2(ml.x - M);   // empty parts carry no weight
-        const float4 v = part[s * (kHeadDim / 4) + lane];
-        o4.x = fmaf(w, v.x, o4.x);
-        o4.y = fmaf(w, v.y, o4.y);
-        o4.z = fmaf(w, v.z, o4.z);
-        o4.w = fmaf(w, v.w, o4.w);
-        l = fmaf(w, ml.y, l);
+    constexpr int kAtOnce = 4;
+    for (int64_t i0 = warp; i0 < parts; i0 += kAtOnce * kMergeWarps) {
+        float2 ml[kAtOnce];
+        float4 v[kAtOnce];
+#pragma unroll
+        for (int k = 0; k < kAtOnce; ++k) {
+            const int64_t i = i0 + k * kMergeWarps;
+            ml[k] = make_float2(-INFINITY, 0.f);
+            v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (i < parts) {
+                ml[k] = lse[slot_of(i)];
+                v[k] = part[slot_of(i) * (kHeadDim / 4) + lane];
+            }
+        }
+        float m = M;
+#pragma unroll
+        for (int k = 0; k < kAtOnce; ++k) m = fmaxf(m, ml[k].x);
+        if (m == -INFINITY) continue;            // empty parts carry no weight
+        const float old = pa_ex2(M - m);
+        o4.x *= old; o4.y *= old; o4.z *= old; o4.w *= old;
+        l *= old;
+#pragma unroll
+        for (int k = 0; k < kAtOnce; ++k) {
+            const float w = ml[k].x == -INFINITY ? 0.f : pa_ex2(ml[k].x - m);
+            o4.x = fmaf(w, v[k].x, o4.x);
+            o4.y = fmaf(w, v[k].y, o4.y);
+            o4.z = fmaf(w, v[k].z, o4.z);
+            o4.w = fmaf(w, v[k].w, o4.w);
+            l = fmaf(w, ml[k].y, l);
+        }
+        M = m;
     }
     so[warp][lane] = o4;
-    if (lane == 0) sl[warp] = l;
+    if (lane == 0) {
+        sl[warp] = l;
+        sm[warp] = M;
+    }
     __syncthreads();
     if (warp == 0) {
+        float Ma = sm[0];
 #pragma unroll
-        for (int w = 1; w < kMergeWarps; ++w) {
+        for (int w = 1; w < kMergeWarps; ++w) Ma = fmaxf(Ma, sm[w]);
+        o4 = make_float4(0.f, 0.f, 0.f, 0.f);
+        l = 0.f;
+#pragma unroll
+        for (int w = 0; w < kMergeWarps; ++w) {
             const float4 v = so[w][lane];
-            o4.x += v.x;
-            o4.y += v.y;
-            o4.z += v.z;
-            o4.w += v.w;
-            l += sl[w];
+            const float f = sm[w] == -INFINITY ? 0.f : pa_ex2(sm[w] - Ma);
+            o4.x = fmaf(f, v.x, o4.x);
+            o4.y = fmaf(f, v.y, o4.y);
+            o4.z = fmaf(f, v.z, o4.z);
+            o4.w = fmaf(f, v.w, o4.w);
+            l = fmaf(f, sl[w], l);
         }
         *reinterpret_cast<uint2*>(p.out + static_cast<int64_t>(bh) * kHeadDim + 4 * lane) =
             make_uint2(pack_half2(o4.x / l, o4.y / l), pack_half2(o4.z / l, o4.w / l));
