@@ -284,14 +284,32 @@ __global__ void __launch_bounds__(kThreads, TQ_DEC_MINBLOCKS) decode_partial_ker
     __shared__ float sm_m[kWarps][8];
     __shared__ float sm_l[kWarps][8];
 
+    // A launch of few pages is one chain of latencies, so nothing in it waits that need not: the tables (codebooks only)
+    // are filled before the previous kernel is known to be done, and the length, the block-table entries and the query are
+    // requested together.  Entries past the length are fetched too (the table row is max_pages wide), and not looked at.
     pdl_release();
-    pdl_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int gid = lane >> 2, tig = lane & 3;
     const int chunk = blockIdx.x;
     const int kvh = blockIdx.y / p.ngroups, qg = blockIdx.y % p.ngroups;
     const int seq = blockIdx.z;
+    fill_pair_lut<KB>(tabk, p.kc, warp, lane);
+    if (!p.share_tables) fill_pair_lut<VB>(tabv, p.vc, warp, lane);
+    uint64_t* mybar = bars + warp * 2 * NSTAGE;        // [0..NSTAGE) K (or whole page), [NSTAGE..) V
+    if (lane == 0) {
+#pragma unroll
+        for (int s = 0; s < 2 * NSTAGE; ++s) mbar_init(mybar + s, 1);
+        fence_barrier_init();
+    }
+    pdl_wait();
     const int L = p.seq_lens[seq];
+    const int p0 = chunk * p.chunk_pages;
+    const int32_t* bt = p.block_tables + static_cast<int64_t>(seq) * p.bt_stride;
+    int32_t bt_first = 0;                               // entry of this warp's page `lane`
+    {
+        const int pg = p0 + warp + kWarps * lane;
+        if (pg < min(p0 + p.chunk_pages, p.max_pages)) bt_first = __ldg(bt + (pg >> p.sub_shift));
+    }
     // A length beyond what the block table and the workspace were sized for is cut to that size and flagged:
     // the walk never leaves the table row and a chunk index never leaves the workspace.
     const bool too_long = L > p.max_pages * kPageTokens;
@@ -299,6 +317,8 @@ __global__ void __launch_bounds__(kThreads, TQ_DEC_MINBLOCKS) decode_partial_ker
     const int g_in_group = qg * 8 + gid;                // query index inside the GQA group
     const int nq = min(8, p.G - qg * 8);                // live query heads in this CTA
     const int head0 = kvh * p.G + qg * 8;
+    float xq[32];
+    load_q32(p.q, (static_cast<int64_t>(seq) * p.Hq + head0 + gid) * kHeadDim, tig, p.io_dtype, g_in_group < p.G, xq);
 
     if (L <= 0) {
         if (chunk == 0) {  // zeros for empty sequences
@@ -309,37 +329,30 @@ __global__ void __launch_bounds__(kThreads, TQ_DEC_MINBLOCKS) decode_partial_ker
         }
         return;
     }
-    const int p0 = chunk * p.chunk_pages;
     if (p0 >= npages) return;
     const int p1 = min(p0 + p.chunk_pages, npages);
     const int n_my = (p0 + warp < p1) ? (p1 - p0 - warp + kWarps - 1) / kWarps : 0;
 
-    uint64_t* mybar = bars + warp * 2 * NSTAGE;        // [0..NSTAGE) K (or whole page), [NSTAGE..) V
     uint8_t* myring = ring + warp * NSTAGE * PAGE;
-    if (lane == 0) {
-#pragma unroll
-        for (int s = 0; s < 2 * NSTAGE; ++s) mbar_init(mybar + s, 1);
-        fence_barrier_init();
-    }
     __syncwarp();
 
     // ---- block-table window: lane l holds the entry of this warp's page jbase + l ---
-    const int32_t* bt = p.block_tables + static_cast<int64_t>(seq) * p.bt_stride;
     int jbase = 0;
     int32_t btreg = 0;
     bool bad_block = false;
-    auto load_bt = [&](int jb) {
+    auto take_bt = [&](int jb, int32_t b) {
         jbase = jb;
-        const int j = jb + lane;
-        int32_t b = 0;
-        if (j < n_my) {
-            b = __ldg(bt + ((p0 + warp + kWarps * j) >> p.sub_shift));
-            if (b < 0 || b >= p.num_blocks) {
-                bad_block = true;
-                b = 0;
-            }
+        if (jb + lane >= n_my) {
+            b = 0;
+        } else if (b < 0 || b >= p.num_blocks) {
+            bad_block = true;
+            b = 0;
         }
         btreg = b;
+    };
+    auto load_bt = [&](int jb) {
+        const int j = jb + lane;
+        take_bt(jb, j < n_my ? __ldg(bt + ((p0 + warp + kWarps * j) >> p.sub_shift)) : 0);
     };
     const uint8_t* head_base = p.cache + (static_cast<int64_t>(kvh) << p.sub_shift) * PAGE;
     auto page_src = [&](int j) -> const uint8_t* {
@@ -368,21 +381,18 @@ __global__ void __launch_bounds__(kThreads, TQ_DEC_MINBLOCKS) decode_partial_ker
         }
     };
 
-    // The first pages are requested before anything else is set up: their HBM latency hides behind the
-    // table fill and the query fragments.
-    if (n_my > 0) load_bt(0);
+    // The first pages are requested before the query fragments are made, which hide part of their latency.
+    if (n_my > 0) take_bt(0, bt_first);
 #pragma unroll
     for (int j = 0; j < NSTAGE; ++j)
         if (j < n_my) issue_k(j);
 
-    // ---- query fragments (their loads are in flight together with the first pages and the table fill) -----
+    // ---- query fragments -------------------------------------------------------------------------------
     uint32_t qf[16], qpf[QJL ? 16 : 1];
     float sq_init0 = 0.f, sq_init1 = 0.f;   // minus the query sums of the one-sided sign forms
     {
         const bool valid = g_in_group < p.G;
         const int64_t row = (static_cast<int64_t>(seq) * p.Hq + head0 + gid) * kHeadDim;
-        float xq[32];
-        load_q32(p.q, row, tig, p.io_dtype, valid, xq);
         if (p.rotate_q) rotate_q32(xq, lane, p.io_dtype);
         q_frag_from(xq, qf);
         if constexpr (QJL) {
@@ -396,10 +406,7 @@ __global__ void __launch_bounds__(kThreads, TQ_DEC_MINBLOCKS) decode_partial_ker
         }
     }
 
-    // ---- per-CTA constants: pair tables of the codebooks ----------------------------------------------
-    fill_pair_lut<KB>(tabk, p.kc, warp, lane);
-    if (!p.share_tables) fill_pair_lut<VB>(tabv, p.vc, warp, lane);
-    __syncthreads();
+    __syncthreads();   // the pair tables are there
     const uint32_t klut = smem_u32(tabk) + (KB == 2 ? 8 * (lane & 15) : 4 * lane);
     const uint32_t vlut = smem_u32(tabv) + (VB == 2 ? 8 * (lane & 15) : 4 * lane);
     // this lane's three access patterns inside a ring stage: its two K records, the norm slots, the V words
@@ -555,28 +562,34 @@ __global__ void __launch_bounds__(kThreads, TQ_DEC_MINBLOCKS) decode_partial_ker
 
 // Weighted combination of partial rows by one warp: part(i) is the 128 sums of part i (fp32), ml(i) its (maximum,
 // denominator).  Eight parts are fetched at a time, independently of one another and of the maxima: what a merge costs is the
-// latency of its chain of loads.
+// latency of its chain of loads.  The first eight are fetched up to part `room`, before `parts` has to be known.
 template <typename Part, typename Ml>
-__device__ __forceinline__ void merge_parts(int first, int step, int parts, int lane, Part part, Ml ml, float& M, float (&x)[4], float& l) {
+__device__ __forceinline__ void merge_parts(int first, int step, int parts, int room, int lane, Part part, Ml ml, float& M, float (&x)[4], float& l) {
     M = -INFINITY;
     l = 0.f;
 #pragma unroll
     for (int i = 0; i < 4; ++i) x[i] = 0.f;
     constexpr int kAtOnce = 8;
-    for (int i0 = first; i0 < parts; i0 += kAtOnce * step) {
-        float4 v[kAtOnce];
-        float2 w[kAtOnce];
+    float4 v[kAtOnce];
+    float2 w[kAtOnce];
+    auto fetch = [&](int i0, int end) {
 #pragma unroll
         for (int k = 0; k < kAtOnce; ++k) {
             const int i = i0 + k * step;
-            if (i < parts) {
+            if (i < end) {
                 w[k] = ml(i);
                 v[k] = *reinterpret_cast<const float4*>(part(i) + 4 * lane);
-            } else {
+            }
+        }
+    };
+    fetch(first, room);
+    for (int i0 = first; i0 < parts;) {
+#pragma unroll
+        for (int k = 0; k < kAtOnce; ++k)
+            if (i0 + k * step >= parts) {
                 w[k] = make_float2(-INFINITY, 0.f);
                 v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
             }
-        }
         float m = M;
 #pragma unroll
         for (int k = 0; k < kAtOnce; ++k) m = fmaxf(m, w[k].x);
@@ -594,6 +607,8 @@ __device__ __forceinline__ void merge_parts(int first, int step, int parts, int 
             x[3] = fmaf(sc, v[k].w, x[3]);
         }
         M = m;
+        i0 += kAtOnce * step;
+        if (i0 < parts) fetch(i0, parts);
     }
 }
 
@@ -608,13 +623,13 @@ __global__ void __launch_bounds__(kChunkMergeWarps * 32) decode_merge_kernel(con
     const int L = p.seq_lens[seq];
     const int npages = min((L + kPageTokens - 1) / kPageTokens, p.max_pages);   // same cut as the partial kernel
     const int nchunks = (npages + p.chunk_pages - 1) / p.chunk_pages;
-    if (nchunks <= 1) return;  // written by the partial kernel
     const int kvh = head / p.G, gi = head % p.G;
     const int by = kvh * p.ngroups + gi / 8, g = gi % 8;
     const int64_t base = (static_cast<int64_t>(seq) * p.Hkv * p.ngroups + by) * p.max_chunks;
     float M, l, x[4];
-    merge_parts(warp, kChunkMergeWarps, nchunks, lane, [&](int c) { return p.ws_o + ((base + c) * 8 + g) * kHeadDim; },
+    merge_parts(warp, kChunkMergeWarps, nchunks, p.max_chunks, lane, [&](int c) { return p.ws_o + ((base + c) * 8 + g) * kHeadDim; },
                 [&](int c) { return reinterpret_cast<const float2*>(p.ws_ml)[(base + c) * 8 + g]; }, M, x, l);
+    if (nchunks <= 1) return;  // written by the partial kernel
     so[warp][lane] = make_float4(x[0], x[1], x[2], x[3]);
     if (lane == 0) sml[warp] = make_float2(M, l);
     __syncthreads();

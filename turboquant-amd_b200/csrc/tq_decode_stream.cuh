@@ -810,7 +810,7 @@ __global__ void __launch_bounds__(kStreamMergeWarps * 32) decode_stream_merge_ke
     if (item.z < 0) return;
     auto slot_of = [&](int i) { return sp.n_warps + 2 * (cta + i) + (i == 0 ? 1 : 0); };   // slot 1 of this CTA, slot 0 of the others
     float M, l, x[4];
-    merge_parts(half, 2, item.z - cta + 1, lane, [&](int i) { return sp.part_o + static_cast<int64_t>(slot_of(i)) * kStreamSlotFloats + g * kHeadDim; },
+    merge_parts(half, 2, item.z - cta + 1, item.z - cta + 1, lane, [&](int i) { return sp.part_o + static_cast<int64_t>(slot_of(i)) * kStreamSlotFloats + g * kHeadDim; },
                 [&](int i) { return sp.part_ml[slot_of(i) * 8 + g]; }, M, x, l);
     if (half == 1) {
         so[g][lane] = make_float4(x[0], x[1], x[2], x[3]);
