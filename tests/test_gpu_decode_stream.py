@@ -43,7 +43,7 @@ def _tables(lens, bs, seed):
 
 
 @pytest.mark.parametrize("kb,vb,qjl", [(2, 2, True), (3, 3, True), (4, 4, False), (4, 3, False), (3, 2, True), (2, 4, True), (4, 4, True)])
-@pytest.mark.parametrize("lens,hq,hkv,bs,dtype", [(RAGGED, 16, 2, 16, torch.float16), (SHORT_TOTAL, 24, 2, 32, torch.bfloat16),
+@pytest.mark.parametrize("lens,hq,hkv,bs,dtype", [(RAGGED, 32, 4, 16, torch.float16), (SHORT_TOTAL, 24, 2, 32, torch.bfloat16),
                                                   (MANY_ITEMS, 4, 1, 16, torch.float16)])
 def test_persistent_matches_chunked(kb, vb, qjl, lens, hq, hkv, bs, dtype):
     fmt = CacheFormat(kb, vb, qjl)
@@ -68,7 +68,7 @@ def test_persistent_matches_chunked(kb, vb, qjl, lens, hq, hkv, bs, dtype):
 def test_persistent_matches_oracle_and_flags_bad_tables():
     fmt = CacheFormat.named("turbo3")
     books = Codebooks(fmt, DEV)
-    lens = [8192 + 5, 0, 40, 16, 17, 700, 15, 1]
+    lens = [16384 + 5, 0, 40, 16, 17, 700, 15, 1]
     bt, blocks = _tables(lens, 16, 3)
     f = random_fields(fmt, blocks, 16, 2, 5)
     cache = paged_layout.pack_cache(f, 16, 3, 3, True).to(DEV)
@@ -87,7 +87,7 @@ def test_persistent_matches_oracle_and_flags_bad_tables():
     paged_decode_attention(q.to(DEV), cache, bad.to(DEV), lens_t.to(DEV), books, 16, sm, cs)
     assert _native.read_status(DEV) == _native.STATUS_BAD_BLOCK
     cut = lens_t.clone()
-    cut[0] = 9000                                             # beyond the table: cut to its width and flagged
+    cut[0] = 17000                                            # beyond the table: cut to its width and flagged
     out = paged_decode_attention(q.to(DEV), cache, bt.to(DEV), cut.to(DEV), books, 16, sm, cs)
     assert _native.read_status(DEV) == _native.STATUS_BAD_BLOCK
     assert_attn_close(out[1:].float().cpu().numpy(), ref[1:])

@@ -717,17 +717,18 @@ int dispatch_v(const DecodeParams& p, int vb, const Plan& plan, cudaStream_t str
 }
 
 // Which kernel is the better one, by the pages that the batch can have at most.  The persistent kernel pays about 12 us
-// however few pages there are (all its tables, one more level of merging), the chunked one 8 to 11, but it takes
+// however few pages there are (all its tables, one more level of merging), the chunked one 5 to 9, but it takes
 // 0.45 (4-bit) to 0.55 us (with sign term) per 1000 pages where the chunked one takes 0.7 to 0.8; sequences of few pages
-// cost it more, a warp then changes item every few pages.  Measured us, chunked / persistent, 8 KV heads: turbo4 2 x 4096
-// tokens (4096 pages) 12.2 / 13.9, 4 x 4096 (8192 pages) 19.2 / 16.5, 64 x 256 17.2 / 16.8; turbo3 4 x 4096 16.3 / 17.4,
-// 1 x 16384 19.1 / 18.0, 64 x 512 (16384 pages) 21.5 / 24.5, 32 x 1024 24.3 / 23.3, 256 x 256 (32768 pages) 45.2 / 40.4.
-constexpr int64_t kStreamMinPages = 8192;
+// cost it more, a warp then changes item every few pages.  Measured us, chunked / persistent, 8 KV heads, turbo4 and turbo3:
+// 1 x 16384 tokens (8192 pages) 16.9 / 16.9 and 15.0 / 17.9; 24 x 1024 (12288) 16.8 / 19.6 and 23.1 / 20.6; 64 x 512 (16384)
+// 21.3 / 22.8 and 20.5 / 24.2, 32 x 1024 25.3 / 21.7 and 24.2 / 23.2; 256 x 256 (32768) 44.1 / 39.4 and 44.0 / 42.4;
+// 32 x 3000 (48128) 50.1 / 37.8 and 52.6 / 42.5.
+constexpr int64_t kStreamMinPages = 16384;
 constexpr int64_t kStreamSlots = static_cast<int64_t>(kStreamCtas) * (kStreamWarps + 2);   // partials of warps and of CTAs
 int64_t pages_at_most(int64_t ns, int64_t hq, int64_t hkv, int64_t max_pages) { return ns * max_pages * hkv * ((hq / hkv + 7) / 8); }
-bool stream_is_better(int64_t pages, int64_t cache_pages, int max_pages, bool qjl) {
+bool stream_is_better(int64_t pages, int64_t cache_pages, int max_pages) {
     if (pages < kStreamMinPages || pages > INT32_MAX || cache_pages > UINT32_MAX) return false;
-    return !qjl || max_pages >= 512 || pages >= 32768 || (pages >= 16384 && max_pages >= 64);
+    return pages >= 32768 || max_pages >= 64;
 }
 // Workspace of the persistent kernel, or 0 where no format would take it.
 int64_t stream_bytes(int64_t pages) {
@@ -830,7 +831,7 @@ extern "C" int tq_decode_paged(void* out, const void* q_rot, const void* q_proj,
     // The persistent kernel takes the calls that leave the split to the library and bring the workspace for it.
     const bool tensor_memory = use_tcgen05 && k_bits <= 3 && v_bits <= 3 && !(sparse_thresh > 0.f);
     const int64_t pages = pages_at_most(num_seqs, num_q_heads, num_kv_heads, max_pages_per_seq);
-    const int64_t stream_need = chunk_pages <= 0 && !tensor_memory && stream_is_better(pages, num_blocks * num_kv_heads * (block_size / kPageTokens), max_pages_per_seq, use_qjl != 0) ? stream_bytes(pages) : 0;
+    const int64_t stream_need = chunk_pages <= 0 && !tensor_memory && stream_is_better(pages, num_blocks * num_kv_heads * (block_size / kPageTokens), max_pages_per_seq) ? stream_bytes(pages) : 0;
     const bool persistent = stream_need > 0 && workspace && workspace_bytes >= stream_need && !(reinterpret_cast<uintptr_t>(workspace) & 15);
     if (chunk_pages <= 0) chunk_pages = tq_decode_auto_chunk_pages(num_seqs, num_kv_heads, num_q_heads, max_pages_per_seq);
     const int64_t need = tq_decode_workspace_bytes(num_seqs, num_q_heads, num_kv_heads, max_pages_per_seq, chunk_pages);
