@@ -93,6 +93,27 @@ def test_persistent_matches_oracle_and_flags_bad_tables():
     assert_attn_close(out[1:].float().cpu().numpy(), ref[1:])
 
 
+@pytest.mark.parametrize("kw", [dict(), dict(chunk_pages=64), dict(chunk_pages=2048), dict(tcgen05=True)])
+@pytest.mark.parametrize("length", [2 ** 31 - 1, 2 ** 31 - 16, 2 ** 31 - 17])
+def test_lengths_near_2_31_are_cut_and_flagged(kw, length):
+    """Such an entry is cut to the table's width like any other that is too long, and its neighbours are untouched."""
+    fmt = CacheFormat.named("turbo3")
+    books = Codebooks(fmt, DEV)
+    lens = [40, 16384, 0, 700, 1, 33]
+    bt, blocks = _tables(lens, 16, 3)                         # 1024 pages wide
+    f = random_fields(fmt, blocks, 16, 4, 6)
+    cache = paged_layout.pack_cache(f, 16, 3, 3, True).to(DEV)
+    q = torch.randn(6, 32, 128, generator=torch.Generator().manual_seed(2)).half().to(DEV)
+    bt, good = bt.to(DEV), torch.tensor(lens, dtype=torch.int32, device=DEV)
+    want = paged_decode_attention(q, cache, bt, good, books, 16, **kw)
+    assert _native.read_status(DEV) == 0
+    bad = good.clone()
+    bad[1] = length
+    got = paged_decode_attention(q, cache, bt, bad, books, 16, **kw)
+    assert _native.read_status(DEV) == _native.STATUS_BAD_BLOCK
+    assert torch.equal(got, want)
+
+
 def test_persistent_sparse_v_skips_and_stays_close():
     """A peaked softmax over long sequences: V parts are left in memory, the result is the dense one within the threshold."""
     fmt = CacheFormat.named("turbo3")

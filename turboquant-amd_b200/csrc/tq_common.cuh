@@ -23,6 +23,12 @@ __host__ __device__ constexpr int v_part_bytes(int vb) { return 256 * vb + 32; }
 __host__ __device__ constexpr int page_bytes(int kb, int vb, int qjl) { return k_part_bytes(kb, qjl) + v_part_bytes(vb); }
 __host__ __device__ constexpr int norm_slot(int t) { return (t & 7) * 2 + (t >> 3); }
 
+// Pages that a sequence of len tokens takes: right for every int, so that a length is compared with what the block table holds
+// only after it is known how long it is.
+__host__ __device__ constexpr int pages_of_length(int len) { return len <= 0 ? 0 : (len - 1) / kPageTokens + 1; }
+static_assert(pages_of_length(INT32_MIN) == 0 && pages_of_length(0) == 0 && pages_of_length(1) == 1 && pages_of_length(16) == 1 &&
+              pages_of_length(17) == 2 && pages_of_length(INT32_MAX) == 1 << 27, "a length near 2^31 must not wrap");
+
 // ---- small PTX wrappers ---------------------------------------------------------
 __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
     uint32_t r;

@@ -312,8 +312,8 @@ __global__ void __launch_bounds__(kThreads, TQ_DEC_MINBLOCKS) decode_partial_ker
     }
     // A length beyond what the block table and the workspace were sized for is cut to that size and flagged:
     // the walk never leaves the table row and a chunk index never leaves the workspace.
-    const bool too_long = L > p.max_pages * kPageTokens;
-    const int npages = too_long ? p.max_pages : (L + kPageTokens - 1) / kPageTokens;
+    const bool too_long = pages_of_length(L) > p.max_pages;
+    const int npages = min(pages_of_length(L), p.max_pages);
     const int g_in_group = qg * 8 + gid;                // query index inside the GQA group
     const int nq = min(8, p.G - qg * 8);                // live query heads in this CTA
     const int head0 = kvh * p.G + qg * 8;
@@ -620,8 +620,7 @@ __global__ void __launch_bounds__(kChunkMergeWarps * 32) decode_merge_kernel(con
     pdl_release();
     pdl_wait();
     const int head = blockIdx.x, seq = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int L = p.seq_lens[seq];
-    const int npages = min((L + kPageTokens - 1) / kPageTokens, p.max_pages);   // same cut as the partial kernel
+    const int npages = min(pages_of_length(p.seq_lens[seq]), p.max_pages);   // same cut as the partial kernel
     const int nchunks = (npages + p.chunk_pages - 1) / p.chunk_pages;
     const int kvh = head / p.G, gi = head % p.G;
     const int by = kvh * p.ngroups + gi / 8, g = gi % 8;

@@ -42,7 +42,7 @@ struct Shares {
 };
 
 __device__ __forceinline__ int pages_of(const DecodeParams& p, int len) {
-    return len <= 0 ? 0 : min((len + kPageTokens - 1) / kPageTokens, p.max_pages);
+    return min(pages_of_length(len), p.max_pages);
 }
 
 // Byte k of w as the second byte of a table address: entry stride 256, so the address is one byte permute.
@@ -284,7 +284,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
     if (blockIdx.x == 0) {   // flags and zero outputs are written once
         for (int s = threadIdx.x * per; s < min(sp.ns, (static_cast<int>(threadIdx.x) + 1) * per); ++s) {
             const int len = p.seq_lens[s];
-            if (len > p.max_pages * kPageTokens && p.status) atomicOr(p.status, TQ_STATUS_BAD_BLOCK);
+            if (pages_of_length(len) > p.max_pages && p.status) atomicOr(p.status, TQ_STATUS_BAD_BLOCK);
             if (len <= 0) {
                 uint4* o = reinterpret_cast<uint4*>(static_cast<uint16_t*>(p.out) + static_cast<int64_t>(s) * p.Hq * kHeadDim);
                 for (int i = 0; i < p.Hq * kHeadDim / 8; ++i) o[i] = make_uint4(0, 0, 0, 0);

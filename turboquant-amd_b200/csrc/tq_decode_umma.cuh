@@ -258,8 +258,8 @@ __global__ void __launch_bounds__(kUmThreads, 2) decode_umma_kernel(const Decode
     UM_TRACE(4, 0, 0);
 #endif
     const int L = p.seq_lens[seq];
-    const bool too_long = L > p.max_pages * kPageTokens;
-    const int npages = too_long ? p.max_pages : (L + kPageTokens - 1) / kPageTokens;
+    const bool too_long = pages_of_length(L) > p.max_pages;
+    const int npages = min(pages_of_length(L), p.max_pages);
     const int nq = min(8, p.G - qg * 8);
     const int head0 = kvh * p.G + qg * 8;
     if (L <= 0) {
