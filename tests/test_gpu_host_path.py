@@ -146,3 +146,52 @@ def test_packed_attention_work_sharing(bits, BH, Sk):
         want = packed_attention(*args, num_splits=splits).float()
         # logits reach |q| |k| ~ 11 * 12: their own rounding, 2^-24 * 132 * log2(e), moves a weight by 2^-16 of itself
         assert ((got - want).abs() <= 2.0 ** -10 * want.abs() + (2.0 ** -15 + Sk * 2.0 ** -24) * 12 * c.abs().max()).all()
+
+
+@pytest.mark.parametrize("bits", [2, 3, 4])
+def test_codebook_written_on_the_stream_just_before_the_call(bits):
+    """The kernel before may be the one that makes the codebook: a cast (general path) or a copy into the caller's tensors
+    (native path).  Every entry point gives what it gives for a codebook that was there all along."""
+    good = tuple(t.clone() for t in make_codebook(128, bits, device=DEV))
+    h = make_wht_matrix(128, device=DEV)
+    fmt = CacheFormat(bits, bits, bits < 4)
+    cache, tables, lens, K, V, slots = _filled(fmt, [4000, 17, 900, 33], 2, 16, torch.float16)
+    short, tall = tables[:2, :4].contiguous(), tables.repeat(64, 1)
+    lens_short, lens_tall = torch.tensor([60, 17], dtype=torch.int32, device=DEV), lens.repeat(64)
+    q = torch.randn(256, 16, 128, device=DEV, dtype=torch.float16)
+    X = torch.randn(40000, 128, device=DEV, dtype=torch.float16)
+    k, v = compress_k_permuted(X[:1000], h, None, *good), compress_v(X[:1000], h, *good)
+    packed = [t.view(2, 500, *t.shape[1:]) for t in (*k, *v)]
+
+    def all_calls(fresh, books, c):
+        def call(f):
+            fresh()
+            r = f()
+            return list(r.values()) if isinstance(r, dict) else list(r) if isinstance(r, tuple) else [r]
+        def append(n):
+            out = torch.zeros_like(cache)
+            fresh()
+            compress_and_scatter(K[:n], V[:n], out, slots[:n], books, 16)
+            return out
+        filled = append(K.shape[0])
+        res = [append(64), filled]                                                    # small and persistent kernel
+        res += call(lambda: paged_decode_attention(q[:2], filled, short, lens_short, books, 16))          # chunked
+        res += call(lambda: paged_decode_attention(q, filled, tall, lens_tall, books, 16))                # persistent
+        res += call(lambda: packed_attention(q[0, :2], q[0, :2], *packed, c[0], 0.01))
+        for x in (X[:100], X):
+            res += call(lambda: compress_k(x, h, None, *c)) + call(lambda: compress_v(x, h, *c))
+        return res + call(lambda: polarquant_compress(X[:100], *c, PolarQuantConfig(bits=bits, use_qjl=True), h))
+
+    want = all_calls(lambda: None, Codebooks(fmt, DEV, good, None), good)
+    own = [t.clone() for t in good]
+    books = Codebooks(fmt, DEV, own, None)
+
+    def copied():
+        for t in own:
+            t.zero_()
+        torch.empty(1 << 24, device=DEV).normal_()
+        for t, g in zip(own, good):
+            t.copy_(g)
+
+    for got in (all_calls(copied, books, own), all_calls(lambda: None, books, [t.double() for t in good])):
+        assert len(got) == len(want) and all(torch.equal(a, b) for a, b in zip(got, want))

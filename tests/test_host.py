@@ -187,6 +187,24 @@ def test_head_counts_that_form_no_query_group_are_refused_on_the_host():
                                     null, null, 0, 4, 8, 100, 3, 3, 1, 0, null) == 0      # zero sequences
 
 
+def test_kernels_read_no_global_memory_before_the_previous_kernel_is_complete():
+    """Kernels are launched while their predecessor runs, and the predecessor may have written any of their inputs, the
+    codebook included: no pointer of the parameters is named between the start of a kernel and its griddepcontrol.wait."""
+    csrc = os.path.join(ROOT, "turboquant-amd_b200", "csrc")
+    waiting = 0
+    for name in sorted(os.listdir(csrc)):
+        text = re.sub(r"//[^\n]*", "", open(os.path.join(csrc, name)).read())
+        pointers = set(re.findall(r"^\s+(?:const )?\w+\*\s+(\w+);", text, flags=re.M)) | {"kc", "vc", "kb", "vb", "c", "b"}
+        for kernel in re.split(r"__global__", text)[1:]:
+            if "pdl_wait();" not in kernel:
+                continue
+            waiting += 1
+            before = kernel[kernel.index("{"):kernel.index("pdl_wait();")]
+            named = re.findall(r"\b(?:p|sp|sp\.d)\.(\w+)\b", before) + re.findall(r"\b(__ldg|cp\.async)\b", before)
+            assert not (set(named) & (pointers | {"__ldg", "cp.async"})), (name, kernel[:90], named)
+    assert waiting >= 11
+
+
 def test_no_cpu_fallback():
     x = torch.randn(4, 128)
     c, b = make_codebook(128, 3)

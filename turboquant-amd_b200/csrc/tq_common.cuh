@@ -72,9 +72,9 @@ __device__ __forceinline__ float ex2(float x) {
 // ---- programmatic dependent launch ------------------------------------------------
 // All kernels of the library are launched with the stream-serialization attribute: a kernel's CTAs are scheduled while the
 // previous kernel drains, which hides the launch gap (1.5 to 2 us between short kernels).  Each kernel lets its successor go
-// at once and waits until its predecessor is complete before it reads or writes anything but its own shared memory and the
-// codebooks, which no kernel of the library writes.  Every CTA waits, so a kernel that is complete has all kernels
-// before it complete, too.  Both instructions do nothing in a kernel launched without the attribute.
+// at once and waits until its predecessor is complete before it reads or writes anything but its own shared memory: the
+// predecessor is whatever ran on the stream before, also the kernel that made the codebook.  Every CTA waits, so a
+// kernel that is complete has all kernels before it complete, too.  Both instructions do nothing in a kernel launched without the attribute.
 __device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

@@ -433,9 +433,10 @@ __device__ __forceinline__ void store_contig_tail(const ContigParams& p, int64_t
 }
 
 // One group of 8 rows per warp on the generic quantizer (binary-search bucketize over arbitrary sorted boundaries).
-// Lanes of rows past the end still take part in the shuffles (on zeros) and store nothing.
-template <int BITS, OutMode MODE>
-__device__ __forceinline__ void compress_contig_rows(const ContigParams& p, int64_t row, int lane, const float* csm) {
+// Lanes of rows past the end still take part in the shuffles (on zeros) and store nothing.  ready() is called when the row has
+// been requested: csm has to hold the centroids after it.
+template <int BITS, OutMode MODE, class Ready>
+__device__ __forceinline__ void compress_contig_rows(const ContigParams& p, int64_t row, int lane, const float* csm, Ready ready) {
     constexpr bool QJL = MODE != OutMode::kPackedV;
     const int quarter = lane & 3;
     const bool live = row < p.n;
@@ -448,6 +449,7 @@ __device__ __forceinline__ void compress_contig_rows(const ContigParams& p, int6
 #pragma unroll
         for (int i = 0; i < 32; ++i) x[i] = 0.f;
     }
+    ready();
     quantize_quarter<BITS, QJL>(x, p.rotate != 0, lane, bd, csm, q);
     if (live) store_idx_contig<BITS>(p.idx_out + row * (16 * BITS), quarter, q.idx);
     store_contig_tail<QJL>(p, row, quarter, q.signs, q.norm, q.rnorm, live);
@@ -455,14 +457,16 @@ __device__ __forceinline__ void compress_contig_rows(const ContigParams& p, int6
 
 template <int BITS, OutMode MODE>
 __global__ void __launch_bounds__(kWarpsPerCta * 32) compress_contig_kernel(const __grid_constant__ ContigParams p) {
-    __shared__ float csm[1 << BITS];
+    __shared__ float csm[kWarpsPerCta][1 << BITS];   // a copy per warp: no barrier between the codebook's latency and the row's
     pdl_release();
-    if (threadIdx.x < (1 << BITS)) csm[threadIdx.x] = p.c ? p.c[threadIdx.x] : 0.f;
-    __syncthreads();
     pdl_wait();
-    const int lane = threadIdx.x & 31;
-    compress_contig_rows<BITS, MODE>(
-        p, (static_cast<int64_t>(blockIdx.x) * kWarpsPerCta + (threadIdx.x >> 5)) * kItemsPerWarp + (lane >> 2), lane, csm);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr bool QJL = MODE != OutMode::kPackedV;  // V needs no centroids
+    const float c = QJL ? p.c[lane & ((1 << BITS) - 1)] : 0.f;
+    compress_contig_rows<BITS, MODE>(p, (static_cast<int64_t>(blockIdx.x) * kWarpsPerCta + warp) * kItemsPerWarp + (lane >> 2), lane, csm[warp], [&] {
+        if (QJL && lane < (1 << BITS)) csm[warp][lane] = c;
+        __syncwarp();
+    });
 }
 
 // ---- unpacked outputs (polarquant_compress) -------------------------------------------------------------------
@@ -540,13 +544,13 @@ __device__ __forceinline__ void fwht128_chunks(float (&x)[32], int lane) {
 
 template <int BITS, bool SIGNS, bool WIDE>
 __global__ void __launch_bounds__(kWarpsPerCta * 32) compress_unpacked_kernel(const ContigParams p) {
-    __shared__ float csm[1 << BITS];
+    __shared__ float csm_of[kWarpsPerCta][1 << BITS];   // a copy per warp: no barrier between the codebook's latency and the row's
     pdl_release();
-    if (threadIdx.x < (1 << BITS)) csm[threadIdx.x] = p.c[threadIdx.x];
-    __syncthreads();
     pdl_wait();
-    const int lane = threadIdx.x & 31, j = lane & 3;
-    const int64_t row = (static_cast<int64_t>(blockIdx.x) * kWarpsPerCta + (threadIdx.x >> 5)) * kItemsPerWarp + (lane >> 2);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, j = lane & 3;
+    float* csm = csm_of[warp];
+    const float centroid = p.c[lane & ((1 << BITS) - 1)];
+    const int64_t row = (static_cast<int64_t>(blockIdx.x) * kWarpsPerCta + warp) * kItemsPerWarp + (lane >> 2);
     const bool live = row < p.n;   // lanes of rows past the end take part in the shuffles, on zeros
     const int64_t at = row * kHeadDim + 8 * j;
     Boundaries<BITS> bd;
@@ -560,6 +564,8 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) compress_unpacked_kernel(co
             for (int e = 0; e < 8; ++e) x[8 * i + e] = 0.f;
         }
     }
+    if (lane < (1 << BITS)) csm[lane] = centroid;
+    __syncwarp();
     if (p.rotate) {
         fwht128_chunks(x, lane);
 #pragma unroll
@@ -672,7 +678,7 @@ __global__ void __launch_bounds__(kFastWarps * 32, 1) compress_contig_fast_kerne
     if (bad != 0) {   // two boundaries inside one cell: the generic quantizer
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         for (; unit < n_units; unit += step)
-            compress_contig_rows<BITS, QJL ? OutMode::kPackedK : OutMode::kPackedV>(p, row_of(unit), lane, csm);
+            compress_contig_rows<BITS, QJL ? OutMode::kPackedK : OutMode::kPackedV>(p, row_of(unit), lane, csm, [] {});
         return;
     }
     constexpr uint32_t kBias = kMagicBits * static_cast<uint32_t>(kCellStride);   // modulo 2^32

@@ -821,39 +821,40 @@ __global__ void __launch_bounds__(kFastWarps * 32, TQ_CMP_MINBLOCKS) compress_pa
 }
 
 // Small launches (the new tokens of one decode step): no tables to build.  Such a launch is one chain of latencies, so
-// a warp takes the keys or the values of 8 items, not both one after the other, its rows are requested together with
-// their slots, and the boundaries before the previous launch has ended.  Measured, us per launch in a graph of such launches,
+// a warp takes the keys or the values of 8 items, not both one after the other, and its rows, their slots and the codebook
+// are requested together (a warp of keys holds the centroids in a copy of its own: no barrier of the CTA).  Measured, us per launch in a graph of such launches,
 // both in one warp / now, 8 KV heads: turbo3 64 tokens 6.1 / 3.4, 1024 tokens 9.8 / 5.4, 2048 tokens 10.1 / 8.9; turbo4 64
 // tokens 6.2 / 3.5.
 template <int KB, int VB, bool QJL>
 __global__ void __launch_bounds__(kWarpsPerCta * 32) compress_paged_small_kernel(const __grid_constant__ PagedParams p) {
     constexpr int PAGE = page_bytes(KB, VB, QJL ? 1 : 0);
-    __shared__ float csm[1 << KB];
+    __shared__ float csm_of[kWarpsPerCta / 2][1 << KB];
     pdl_release();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, quarter = lane & 3;
     const ItemId id = identify_item(p, (static_cast<int64_t>(blockIdx.x) * (kWarpsPerCta / 2) + (warp >> 1)) * kItemsPerWarp + (lane >> 2));
-    if (QJL && threadIdx.x < (1 << KB)) csm[threadIdx.x] = p.kc[threadIdx.x];
-    if (QJL) __syncthreads();
+    pdl_wait();
     float x[32];
 #pragma unroll
     for (int i = 0; i < 32; ++i) x[i] = 0.f;   // lanes past the end take part in the shuffles
     int64_t slot = 0;
     Quarter q;
     if ((warp & 1) == 0) {
+        float* csm = csm_of[warp >> 1];
         Boundaries<KB> bd;
         bd.load(p.kb);
-        pdl_wait();
+        const float centroid = QJL ? p.kc[lane & ((1 << KB) - 1)] : 0.f;
         if (id.live) {
             slot = p.slot_mapping[id.tok];
             load32(p.key, id.tok * p.ks_t + id.head * p.ks_h + 32 * quarter, p.in_dtype, x);
         }
+        if (QJL && lane < (1 << KB)) csm[lane] = centroid;
+        __syncwarp();
         const ItemPlace w = place_item<PAGE>(p, id, slot, quarter);
         quantize_quarter<KB, QJL>(x, p.rotate != 0, lane, bd, csm, q);
         if (w.live) store_k_paged<KB, QJL>(w.page, w.t, quarter, q);
     } else {
         Boundaries<VB> bd;
         bd.load(p.vb);
-        pdl_wait();
         if (id.live) {
             slot = p.slot_mapping[id.tok];
             load32(p.value, id.tok * p.vs_t + id.head * p.vs_h + 32 * quarter, p.in_dtype, x);

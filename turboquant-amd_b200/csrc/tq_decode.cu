@@ -89,22 +89,27 @@ __host__ __device__ constexpr int lut_entries() { return BITS == 2 ? 256 : (BITS
 template <int BITS>
 __host__ __device__ constexpr int lut_bytes() { return lut_entries<BITS>() * 128; }
 
-// Every lane fetches one centroid (already rounded to fp16) and the entries are assembled from warp shuffles, so the
-// fill does not wait on a global load per entry.
+// Every lane fetches one centroid (lane_centroid, rounded to fp16 by the fill) and the entries are assembled from warp
+// shuffles, so the fill does not wait on a global load per entry.  Eight lanes write an entry, 16 bytes each: with 4 bytes a
+// lane the fill of a 256-entry table took 1.3 us of a launch.
 template <int BITS>
-__device__ __forceinline__ void fill_pair_lut(uint32_t* tab, const float* __restrict__ c, int warp, int lane) {
-    const float cv = __half2float(__float2half_rn(__ldg(c + (lane & ((1 << BITS) - 1)))));
-    if constexpr (BITS == 2) {
-        for (int b = warp; b < 256; b += kWarps) {
-            const int i0 = (lane & 1) ? (b >> 2) & 3 : b & 3, i1 = (lane & 1) ? (b >> 6) & 3 : (b >> 4) & 3;   // word 0: pair A, word 1: pair B
-            tab[b * 32 + lane] = pack_half2(__shfl_sync(0xffffffffu, cv, i0), __shfl_sync(0xffffffffu, cv, i1));
-        }
-        return;
-    }
-    for (int b = warp; b < lut_entries<BITS>(); b += kWarps) {
-        const int i0 = b & 15, i1 = b >> 4;
-        const float c0 = __shfl_sync(0xffffffffu, cv, i0 & ((1 << BITS) - 1)), c1 = __shfl_sync(0xffffffffu, cv, i1 & ((1 << BITS) - 1));
-        if (i0 < (1 << BITS) && i1 < (1 << BITS)) tab[b * 32 + lane] = pack_half2(c0, c1);
+__device__ __forceinline__ float lane_centroid(const float* __restrict__ c, int lane) { return __ldg(c + (lane & ((1 << BITS) - 1))); }
+// 16 bytes of entry b: the half2 of its two nibbles four times, or, 2-bit, its two half2 (pair A: bits 1:0 with 5:4, pair B:
+// bits 3:2 with 7:6) twice.  Nibbles past the codebook are never looked up.
+template <int BITS>
+__device__ __forceinline__ uint4 pair_entry(float cv, int b) {
+    constexpr int kMask = (1 << BITS) - 1;
+    const uint32_t a = pack_half2(__shfl_sync(0xffffffffu, cv, b & kMask), __shfl_sync(0xffffffffu, cv, (b >> 4) & kMask));
+    if constexpr (BITS > 2) return make_uint4(a, a, a, a);
+    const uint32_t o = pack_half2(__shfl_sync(0xffffffffu, cv, (b >> 2) & kMask), __shfl_sync(0xffffffffu, cv, (b >> 6) & kMask));
+    return make_uint4(a, o, a, o);
+}
+template <int BITS>
+__device__ __forceinline__ void fill_pair_lut(uint32_t* tab, float centroid, int warp, int lane) {
+    const float cv = __half2float(__float2half_rn(centroid));
+    for (int b0 = 4 * warp; b0 < lut_entries<BITS>(); b0 += 4 * kWarps) {
+        const int b = b0 + (lane >> 3);
+        *reinterpret_cast<uint4*>(tab + b * 32 + 4 * (lane & 7)) = pair_entry<BITS>(cv, b);
     }
 }
 
@@ -284,17 +289,15 @@ __global__ void __launch_bounds__(kThreads, TQ_DEC_MINBLOCKS) decode_partial_ker
     __shared__ float sm_m[kWarps][8];
     __shared__ float sm_l[kWarps][8];
 
-    // A launch of few pages is one chain of latencies, so nothing in it waits that need not: the tables (codebooks only)
-    // are filled before the previous kernel is known to be done, and the length, the block-table entries and the query are
-    // requested together.  Entries past the length are fetched too (the table row is max_pages wide), and not looked at.
+    // A launch of few pages is one chain of latencies, so nothing in it waits that need not: the length, the block-table
+    // entries, the query and the codebooks are requested together, and the tables are filled behind the first pages' copies.
+    // Entries past the length are fetched too (the table row is max_pages wide), and not looked at.
     pdl_release();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int gid = lane >> 2, tig = lane & 3;
     const int chunk = blockIdx.x;
     const int kvh = blockIdx.y / p.ngroups, qg = blockIdx.y % p.ngroups;
     const int seq = blockIdx.z;
-    fill_pair_lut<KB>(tabk, p.kc, warp, lane);
-    if (!p.share_tables) fill_pair_lut<VB>(tabv, p.vc, warp, lane);
     uint64_t* mybar = bars + warp * 2 * NSTAGE;        // [0..NSTAGE) K (or whole page), [NSTAGE..) V
     if (lane == 0) {
 #pragma unroll
@@ -317,6 +320,7 @@ __global__ void __launch_bounds__(kThreads, TQ_DEC_MINBLOCKS) decode_partial_ker
     const int g_in_group = qg * 8 + gid;                // query index inside the GQA group
     const int nq = min(8, p.G - qg * 8);                // live query heads in this CTA
     const int head0 = kvh * p.G + qg * 8;
+    const float ck = lane_centroid<KB>(p.kc, lane), cv = lane_centroid<VB>(p.vc, lane);
     float xq[32];
     load_q32(p.q, (static_cast<int64_t>(seq) * p.Hq + head0 + gid) * kHeadDim, tig, p.io_dtype, g_in_group < p.G, xq);
 
@@ -381,11 +385,13 @@ __global__ void __launch_bounds__(kThreads, TQ_DEC_MINBLOCKS) decode_partial_ker
         }
     };
 
-    // The first pages are requested before the query fragments are made, which hide part of their latency.
+    // The first pages are requested before the tables and the query fragments are made, which hide part of their latency.
     if (n_my > 0) take_bt(0, bt_first);
 #pragma unroll
     for (int j = 0; j < NSTAGE; ++j)
         if (j < n_my) issue_k(j);
+    fill_pair_lut<KB>(tabk, ck, warp, lane);
+    if (!p.share_tables) fill_pair_lut<VB>(tabv, cv, warp, lane);
 
     // ---- query fragments -------------------------------------------------------------------------------
     uint32_t qf[16], qpf[QJL ? 16 : 1];

@@ -106,20 +106,16 @@ __device__ __forceinline__ uint32_t paired_dims(uint32_t w, uint32_t two12) {
     return bit_select(bit_select(w, w << 6, 0x33003300u), w >> 6, 0x00cc00ccu);
 }
 
+__device__ __forceinline__ void store_entry(uint32_t addr, uint4 v) {
+    asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
+
 template <int BITS>
-__device__ __forceinline__ void fill_stream_table(uint32_t smem_addr, const float* __restrict__ c, int warp, int lane) {
-    const float cv = __half2float(__float2half_rn(__ldg(c + (lane & ((1 << BITS) - 1)))));
-    for (int b = warp; b < 256; b += kStreamWarps) {
-        int i0, i1;
-        if constexpr (BITS == 2) {
-            i0 = (lane & 1) ? (b >> 2) & 3 : b & 3;
-            i1 = (lane & 1) ? (b >> 6) & 3 : (b >> 4) & 3;
-        } else {
-            i0 = b & ((1 << BITS) - 1);
-            i1 = (b >> 4) & ((1 << BITS) - 1);
-        }
-        const uint32_t v = pack_half2(__shfl_sync(0xffffffffu, cv, i0), __shfl_sync(0xffffffffu, cv, i1));
-        asm volatile("st.shared.u32 [%0], %1;" ::"r"(smem_addr + b * 256 + lane * 4), "r"(v) : "memory");
+__device__ __forceinline__ void fill_stream_table(uint32_t smem_addr, float centroid, int warp, int lane) {
+    const float cv = __half2float(__float2half_rn(centroid));
+    for (int b0 = 4 * warp; b0 < 256; b0 += 4 * kStreamWarps) {   // eight lanes an entry
+        const int b = b0 + (lane >> 3);
+        store_entry(smem_addr + b * 256 + 16 * (lane & 7), pair_entry<BITS>(cv, b));
     }
 }
 
@@ -192,10 +188,10 @@ __device__ __forceinline__ void wht_16x8(float (&x)[16], int lane) {
 // operand of one score product, in its register order (A dims 0 1, B dims 0 1, A dims 2 3, B dims 2 3), 8 copies.  (With the
 // eight signs of a byte of one token per entry, every second register had to be moved before the products.)
 __device__ __forceinline__ void fill_sign_table(uint32_t smem_addr, int warp, int lane) {
-    for (int b = warp; b < 256; b += kStreamWarps) {
-        const int pair = b >> (((lane & 1) << 2) | (lane & 2));
-        const uint32_t v = 0xBC00BC00u ^ ((pair & 1) ? 0x8000u : 0u) ^ ((pair & 2) ? 0x80000000u : 0u);
-        asm volatile("st.shared.u32 [%0], %1;" ::"r"(smem_addr + b * 256 + lane * 4), "r"(v) : "memory");
+    auto signs = [](int pair) { return 0xBC00BC00u ^ ((pair & 1) ? 0x8000u : 0u) ^ ((pair & 2) ? 0x80000000u : 0u); };
+    for (int b0 = 4 * warp; b0 < 256; b0 += 4 * kStreamWarps) {
+        const int b = b0 + (lane >> 3);
+        store_entry(smem_addr + b * 256 + 16 * (lane & 7), make_uint4(signs(b), signs(b >> 4), signs(b >> 2), signs(b >> 6)));
     }
 }
 template <int K>
@@ -250,15 +246,13 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
                                        : tab + kStreamTable + (bars_low ? 0 : kBars) + (warp - n_low) * RING;
     const uint32_t bar = bars + warp * 2 * NSTAGE * 8;     // [0 .. NSTAGE) page (or K part), [NSTAGE ..) late V part
 
-    // Only the codebooks, which no kernel of this library writes, are read before the previous kernel is known to be done.
     pdl_release();
-    fill_stream_table<KB>(tab, p.kc, warp, lane);
-    if constexpr (SIGN_TABLE) fill_sign_table(tab + 128, warp, lane);
-    else fill_stream_table<VB>(tab + 128, p.vc, warp, lane);
+    if constexpr (SIGN_TABLE) fill_sign_table(tab + 128, warp, lane);   // constants
     if (lane < 2) sm_part[2 * warp + lane] = make_int4(-1, 0, 0, 0);
     if (lane < 2 * NSTAGE) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar + lane * 8) : "memory");
     fence_barrier_init();
     pdl_wait();
+    const float ck = lane_centroid<KB>(p.kc, lane), cv = SIGN_TABLE ? 0.f : lane_centroid<VB>(p.vc, lane);
 
     // ---- pages before each thread's run of sequences (every CTA does the same scan over all lengths)
     const int per = (sp.ns + kStreamThreads - 1) / kStreamThreads;
@@ -361,6 +355,10 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
     const int first_lot = min(n, NSTAGE);
     if (lane < first_lot) copy_in(ring + lane * PAGE, page_at(src), PAGE, bar + lane * 8);
     if (n > 32) src_next = next_window();
+    // the codebooks' part of the table is filled behind the first pages' copies
+    fill_stream_table<KB>(tab, ck, warp, lane);
+    if constexpr (!SIGN_TABLE) fill_stream_table<VB>(tab + 128, cv, warp, lane);
+    __syncthreads();
 
     const uint32_t klut = tab + (KB == 2 ? 8 * (lane & 15) : 4 * lane);
     const uint32_t vlut = tab + (SIGN_TABLE ? 0 : 128) + (VB == 2 ? 8 * (lane & 15) : 4 * lane);

@@ -181,10 +181,8 @@ __global__ void __launch_bounds__(kPaThreads, 1) packed_attn_partial(const PAPar
     };
     int64_t at = p.num_splits > 0 ? static_cast<int64_t>(blockIdx.x) : u0;
     const int64_t stop = p.num_splits > 0 ? static_cast<int64_t>(n_items) : u1;
-    if (at >= stop) {
-        pdl_wait();
-        return;
-    }
+    pdl_wait();
+    if (at >= stop) return;
 
     // ---- item state: which segment the CTA works on, and the warp's asynchronous staging of it: per step a warp
     // copies its 16 K rows, 16 V rows and 16 sign rows in 16-byte pieces (every row is a multiple of 16 bytes, so any
@@ -250,18 +248,21 @@ __global__ void __launch_bounds__(kPaThreads, 1) packed_attn_partial(const PAPar
         for (int i = 0; i < kPaStages - 1; ++i) issue();
         load_norms(tok16, nrm);
     };
-    // the pair tables depend on the codebook only.  Every lane holds one centroid; an entry's two come by shuffle.
+    // The pair tables are filled behind the first copies.  Every lane holds one centroid; an entry's two come by shuffle.
     {
         const float cv = __ldg(p.centroids + (lane & ((1 << BITS) - 1)));
-#pragma unroll 4
-        for (int pr = warp; pr < LO::kPairs; pr += kPaWarps) {
-            const float c0 = __shfl_sync(0xffffffffu, cv, pr & ((1 << BITS) - 1)), c1 = __shfl_sync(0xffffffffu, cv, pr >> BITS);
-            *reinterpret_cast<float2*>(pair_tab + (pr * 32 + lane) * 8) = make_float2(c0, c1);
-            *reinterpret_cast<uint32_t*>(half_tab + (pr * 32 + lane) * 4) = pack_half2(c0, c1);
+        begin(at);
+        auto pair = [&](int pr) { return make_float2(__shfl_sync(0xffffffffu, cv, pr & ((1 << BITS) - 1)), __shfl_sync(0xffffffffu, cv, pr >> BITS)); };
+        for (int p0 = 2 * warp; p0 < LO::kPairs; p0 += 2 * kPaWarps) {       // 16 bytes a lane
+            const float2 c = pair(p0 + (lane >> 4));
+            *reinterpret_cast<float4*>(pair_tab + p0 * 256 + lane * 16) = make_float4(c.x, c.y, c.x, c.y);
+        }
+        for (int p0 = 4 * warp; p0 < LO::kPairs; p0 += 4 * kPaWarps) {
+            const float2 c = pair(p0 + (lane >> 3));
+            const uint32_t h = pack_half2(c.x, c.y);
+            *reinterpret_cast<uint4*>(half_tab + p0 * 128 + lane * 16) = make_uint4(h, h, h, h);
         }
     }
-    pdl_wait();
-    begin(at);
     const uint32_t lane8 = lane * 8, lane4 = lane * 4;
     // selector that gathers byte `quarter` of two sign words
     const uint32_t sel_lo = static_cast<uint32_t>(quarter) | (static_cast<uint32_t>(4 + quarter) << 4);
