@@ -70,13 +70,26 @@ __device__ __forceinline__ float ex2(float x) {
 }
 
 // ---- programmatic dependent launch ------------------------------------------------
-// All kernels of the library are launched with the stream-serialization attribute: a kernel's CTAs are scheduled while the
-// previous kernel drains, which hides the launch gap (1.5 to 2 us between short kernels).  Each kernel lets its successor go
-// at once and waits until its predecessor is complete before it reads or writes anything but its own shared memory: the
-// predecessor is whatever ran on the stream before, also the kernel that made the codebook.  Every CTA waits, so a
-// kernel that is complete has all kernels before it complete, too.  Both instructions do nothing in a kernel launched without the attribute.
+// All kernels but compress_paged_tc_kernel are launched with the stream-serialization attribute: a kernel's CTAs are scheduled
+// while the previous kernel runs, which hides the launch gap (1.5 to 2 us between short kernels).  Each waits until its
+// predecessor is complete before it reads or writes anything but its own shared memory: the predecessor is whatever ran on
+// the stream before, also the kernel that made the codebook.  Every CTA waits, so a kernel that is complete has all
+// kernels before it complete, too.
+//
+// When a kernel lets its successor go decides where the successor's CTAs are placed.  Kernels that release before they wait
+// let a whole chain of launches settle on the SMs, each where the ones before it left room, and a kernel then runs on part
+// of the GPU.  So a call's first (or only) kernel releases after its wait: at most the merge kernel behind it and the next
+// call's first kernel are there early.  Merge kernels release at once.  Measured in graphs of such calls, everything released at
+// once / this: decode turbo3, 1 KV head, 24 x 1024 tokens 11.5 / 7.9 us, 64 x 512 12.8 / 9.6, 32 x 1500 12.9 / 9.3; append turbo2, 600
+// tokens 5.7 / 4.3, 1000 tokens 7.5 / 5.0; compress_k + compress_v 3-bit, 8000 rows 10.8 / 6.8.  Two kernels of more CTAs than
+// half of what the SMs hold get in each other's way all the same, so large grids of small CTAs release by ending
+// (compress_k + compress_v 3-bit, 22806 rows: 16.3 us with a release, 11.7 without).
 __device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// For CTAs of 128 threads and at most 96 registers, of which an SM holds at least 5: 4 per SM is the line.
+__device__ __forceinline__ void pdl_release_if_small() {
+    if (static_cast<uint64_t>(gridDim.x) * gridDim.y * gridDim.z <= 4 * 148) pdl_release();
+}
 
 template <typename... Params, typename... Args>
 inline cudaError_t launch_chained(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {

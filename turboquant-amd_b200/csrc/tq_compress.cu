@@ -458,8 +458,8 @@ __device__ __forceinline__ void compress_contig_rows(const ContigParams& p, int6
 template <int BITS, OutMode MODE>
 __global__ void __launch_bounds__(kWarpsPerCta * 32) compress_contig_kernel(const __grid_constant__ ContigParams p) {
     __shared__ float csm[kWarpsPerCta][1 << BITS];   // a copy per warp: no barrier between the codebook's latency and the row's
-    pdl_release();
     pdl_wait();
+    pdl_release_if_small();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     constexpr bool QJL = MODE != OutMode::kPackedV;  // V needs no centroids
     const float c = QJL ? p.c[lane & ((1 << BITS) - 1)] : 0.f;
@@ -545,8 +545,8 @@ __device__ __forceinline__ void fwht128_chunks(float (&x)[32], int lane) {
 template <int BITS, bool SIGNS, bool WIDE>
 __global__ void __launch_bounds__(kWarpsPerCta * 32) compress_unpacked_kernel(const ContigParams p) {
     __shared__ float csm_of[kWarpsPerCta][1 << BITS];   // a copy per warp: no barrier between the codebook's latency and the row's
-    pdl_release();
     pdl_wait();
+    pdl_release_if_small();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, j = lane & 3;
     float* csm = csm_of[warp];
     const float centroid = p.c[lane & ((1 << BITS) - 1)];
@@ -663,8 +663,8 @@ __global__ void __launch_bounds__(kFastWarps * 32, 1) compress_contig_fast_kerne
     int64_t unit = static_cast<int64_t>(warp) * gridDim.x + blockIdx.x;
     const int64_t step = static_cast<int64_t>(gridDim.x) * kFastWarps;
     auto row_of = [&](int64_t u) { return u * kItemsPerWarp + (lane >> 2); };
-    pdl_release();
     pdl_wait();
+    pdl_release();
     if constexpr (mma) {
         stage_row(dst, p.x, row_of(unit) * kHeadDim + 8 * quarter, row_of(unit) < p.n);
         stage_row(dst + kRowBuffer, p.x, row_of(unit + step) * kHeadDim + 8 * quarter, row_of(unit + step) < p.n);

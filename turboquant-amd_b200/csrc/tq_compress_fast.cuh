@@ -746,8 +746,8 @@ __global__ void __launch_bounds__(kFastWarps * 32, TQ_CMP_MINBLOCKS) compress_pa
     const uint32_t vtab = smem_u32(tables + kTableBytes) + (lane & 15) * 8 - kBias;
     constexpr bool mma = ROWS != Rows::kPlain, BF16 = ROWS == Rows::kBF16;
 
-    pdl_release();
     pdl_wait();
+    pdl_release();
     // Tensor-core path.  Rows are staged through shared memory one unit ahead: the key rows of the next unit are requested
     // as soon as this unit's have been consumed by the MMAs, the value rows likewise, so every copy has a whole unit's
     // arithmetic to hide behind.  The first ones are under way while the tables are built.
@@ -829,10 +829,10 @@ template <int KB, int VB, bool QJL>
 __global__ void __launch_bounds__(kWarpsPerCta * 32) compress_paged_small_kernel(const __grid_constant__ PagedParams p) {
     constexpr int PAGE = page_bytes(KB, VB, QJL ? 1 : 0);
     __shared__ float csm_of[kWarpsPerCta / 2][1 << KB];
-    pdl_release();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, quarter = lane & 3;
     const ItemId id = identify_item(p, (static_cast<int64_t>(blockIdx.x) * (kWarpsPerCta / 2) + (warp >> 1)) * kItemsPerWarp + (lane >> 2));
     pdl_wait();
+    pdl_release_if_small();
     float x[32];
 #pragma unroll
     for (int i = 0; i < 32; ++i) x[i] = 0.f;   // lanes past the end take part in the shuffles

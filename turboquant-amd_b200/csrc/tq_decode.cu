@@ -292,7 +292,6 @@ __global__ void __launch_bounds__(kThreads, TQ_DEC_MINBLOCKS) decode_partial_ker
     // A launch of few pages is one chain of latencies, so nothing in it waits that need not: the length, the block-table
     // entries, the query and the codebooks are requested together, and the tables are filled behind the first pages' copies.
     // Entries past the length are fetched too (the table row is max_pages wide), and not looked at.
-    pdl_release();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int gid = lane >> 2, tig = lane & 3;
     const int chunk = blockIdx.x;
@@ -305,6 +304,7 @@ __global__ void __launch_bounds__(kThreads, TQ_DEC_MINBLOCKS) decode_partial_ker
         fence_barrier_init();
     }
     pdl_wait();
+    pdl_release();
     const int L = p.seq_lens[seq];
     const int p0 = chunk * p.chunk_pages;
     const int32_t* bt = p.block_tables + static_cast<int64_t>(seq) * p.bt_stride;

@@ -246,12 +246,12 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
                                        : tab + kStreamTable + (bars_low ? 0 : kBars) + (warp - n_low) * RING;
     const uint32_t bar = bars + warp * 2 * NSTAGE * 8;     // [0 .. NSTAGE) page (or K part), [NSTAGE ..) late V part
 
-    pdl_release();
     if constexpr (SIGN_TABLE) fill_sign_table(tab + 128, warp, lane);   // constants
     if (lane < 2) sm_part[2 * warp + lane] = make_int4(-1, 0, 0, 0);
     if (lane < 2 * NSTAGE) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar + lane * 8) : "memory");
     fence_barrier_init();
     pdl_wait();
+    pdl_release();
     const float ck = lane_centroid<KB>(p.kc, lane), cv = SIGN_TABLE ? 0.f : lane_centroid<VB>(p.vc, lane);
 
     // ---- pages before each thread's run of sequences (every CTA does the same scan over all lengths)

@@ -247,8 +247,8 @@ __global__ void __launch_bounds__(kUmThreads, 2) decode_umma_kernel(const Decode
     const uint32_t sbase = smem_u32(smem);
     float* scal = reinterpret_cast<float*>(smem + UmSmem::kScal);
 
-    pdl_release();
     pdl_wait();
+    pdl_release();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int chunk = blockIdx.x;
     const int kvh = blockIdx.y / p.ngroups, qg = blockIdx.y % p.ngroups;

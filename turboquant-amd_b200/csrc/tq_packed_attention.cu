@@ -151,7 +151,6 @@ __global__ void __launch_bounds__(kPaThreads, 1) packed_attn_partial(const PAPar
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int slot = lane >> 2, quarter = lane & 3;
-    pdl_release();
 
     // ---- the CTA's segments ----
     const int steps = (p.Sk + kStepTokens - 1) / kStepTokens;   // per row
@@ -182,6 +181,7 @@ __global__ void __launch_bounds__(kPaThreads, 1) packed_attn_partial(const PAPar
     int64_t at = p.num_splits > 0 ? static_cast<int64_t>(blockIdx.x) : u0;
     const int64_t stop = p.num_splits > 0 ? static_cast<int64_t>(n_items) : u1;
     pdl_wait();
+    pdl_release();
     if (at >= stop) return;
 
     // ---- item state: which segment the CTA works on, and the warp's asynchronous staging of it: per step a warp
@@ -531,8 +531,8 @@ __global__ void __launch_bounds__(kMergeWarps * 32) packed_attn_merge(const PAPa
 
 // ---- row-wise WHT ----------------------------------------------------------------------
 __global__ void __launch_bounds__(128) wht_rows_kernel(const void* in, void* out, int dtype, int64_t n, float scale) {
-    pdl_release();
     pdl_wait();
+    pdl_release_if_small();
     const int lane = threadIdx.x & 31;
     const int64_t row = static_cast<int64_t>(blockIdx.x) * 4 + (threadIdx.x >> 5);
     if (row >= n) return;
