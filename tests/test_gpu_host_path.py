@@ -195,3 +195,35 @@ def test_codebook_written_on_the_stream_just_before_the_call(bits):
 
     for got in (all_calls(copied, books, own), all_calls(lambda: None, books, [t.double() for t in good])):
         assert len(got) == len(want) and all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+def test_general_path_on_two_streams_at_once(general):
+    """Partials and the records of what is split live in the workspace: calls that overlap must not share one."""
+    fmt = CacheFormat.named("turbo3")
+    books = Codebooks(fmt, DEV)
+    lens = [700, 4000, 33, 2100] * 16
+    cache, tables, lens_t, K, V, slots = _filled(fmt, lens, 2, 16, torch.float16)
+    compress_and_scatter(K, V, cache, slots, books, 16)
+    g = torch.Generator(device=DEV).manual_seed(3)
+    q = torch.randn(64, 16, 128, generator=g, device=DEV).half()
+    h, (c, b) = make_wht_matrix(128, device=DEV), make_codebook(128, 3, device=DEV)
+    X = torch.randn(40 * 3000, 128, generator=g, device=DEV).half()
+    packed = [t.view(40, 3000, *t.shape[1:]) for t in (*compress_k_permuted(X, h, None, c, b), *compress_v(X, h, c, b))]
+    few = [t[:3].contiguous() for t in packed]
+    jobs = [(lambda: paged_decode_attention(q, cache, tables, lens_t, books, 16),
+             lambda: paged_decode_attention(q[:6], cache, tables[:6], lens_t[:6], books, 16)),
+            (lambda: packed_attention(q[0, :1].repeat(40, 1), q[0, :1].repeat(40, 1), *packed, c, 0.01),
+             lambda: packed_attention(q[0, :3], q[0, :3], *few, c, 0.01))]
+    for pair in jobs:
+        want = [general(f) for f in pair]
+        streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+        torch.cuda.synchronize()
+        got = [[], []]
+        for _ in range(20):
+            for i in (0, 1):
+                with torch.cuda.stream(streams[i]):
+                    got[i].append(general(pair[i]))
+        torch.cuda.synchronize()
+        for i in (0, 1):
+            assert all(torch.equal(r, want[i]) for r in got[i])
+    assert _native.read_status(DEV) == 0

@@ -146,9 +146,8 @@ def check_is_wht(matrix: torch.Tensor, d: int) -> None:
                          "fast Walsh-Hadamard transform and cannot apply an arbitrary matrix")
     matrix._tq_is_wht_version = matrix._version
 
-# ---- per-device scratch: status word, split-K workspaces --------------------------------------
+# ---- per-device status word -----------------------------------------------------------------
 _status: dict = {}
-_workspaces: dict = {}
 
 
 def status_word(device: torch.device) -> torch.Tensor:
@@ -172,17 +171,10 @@ def read_status(device, reset: bool = True) -> int:
     return val
 
 
-def workspace(device: torch.device, nbytes: int, tag: str = "decode") -> torch.Tensor:
-    """A cached uint8 workspace of at least nbytes; grows geometrically, never shrinks."""
-    device = torch.device(device)
-    if device.index is None:
-        device = torch.device("cuda", torch.cuda.current_device())
-    key = (device, tag)
-    cur = _workspaces.get(key)
-    if cur is None or cur.numel() < nbytes:
-        cur = torch.empty(max(nbytes, 1 << 20), dtype=torch.uint8, device=device)
-        _workspaces[key] = cur
-    return cur
+def workspace(device: torch.device, nbytes: int) -> torch.Tensor:
+    """A uint8 workspace for one call: a block of the caching allocator, whose reuse is ordered by the current stream, so
+    calls on other streams and threads never share it."""
+    return torch.empty(max(nbytes, 16), dtype=torch.uint8, device=device)
 
 
 # ---- thin checked wrappers -----------------------------------------------------------------

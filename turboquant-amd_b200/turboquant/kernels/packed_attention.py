@@ -65,7 +65,7 @@ def packed_attention(Q, Q_proj, k_idx_packed, k_signs_packed, k_r_norm, k_norm,
     L = _native.lib()
     splits = max(0, min(int(num_splits or 0), Sk))          # 0: the library shares the work out
     need = L.tq_packed_attention_workspace_bytes(BH, splits)
-    ws = _native.workspace(dev, need, tag="packed_attention")
+    ws = _native.workspace(dev, need)
     out = torch.empty(BH, D, dtype=torch.float16, device=dev)
     with torch.cuda.device(dev):
         rc = L.tq_packed_attention(
