@@ -93,6 +93,29 @@ def test_persistent_matches_oracle_and_flags_bad_tables():
     assert_attn_close(out[1:].float().cpu().numpy(), ref[1:])
 
 
+@pytest.mark.parametrize("G", [1, 4, 6, 8, 12])
+@pytest.mark.parametrize("chunk", [0, 256])
+def test_sparse_v_skips_for_every_group_size(G, chunk):
+    """Groups of fewer than eight heads, and the last four of twelve: the zero queries that fill up the tile must not keep
+    pages.  chunk 0 runs the persistent kernel, 256 pages the chunked one."""
+    fmt = CacheFormat.named("turbo3")
+    books = Codebooks(fmt, DEV)
+    lens = [32768, 16384 + 5] * 8
+    bt, blocks = _tables(lens, 16, 9)
+    cache = _random_cache(fmt, blocks, 2, 16, 11)
+    q = torch.randn(16, 2 * G, 128, generator=torch.Generator(device=DEV).manual_seed(3), device=DEV).half() * 12
+    args = (q, cache, bt.to(DEV), torch.tensor(lens, dtype=torch.int32, device=DEV), books, 16)
+    stats = torch.zeros(2, dtype=torch.int32, device=DEV)
+    got = paged_decode_attention(*args, sparse_thresh=1e-6, skip_stats=stats, chunk_pages=chunk).float()
+    want = paged_decode_attention(*args, chunk_pages=chunk).float()
+    assert _native.read_status(DEV) == 0
+    seen, skipped = stats.tolist()
+    assert seen == 2 * -(-G // 8) * 8 * (2048 + 1025) and 0 < skipped < seen
+    # as above: the skipped weights add up to at most 1e-6 of the maximum for each of 32768 tokens, times |v|
+    bound = (2 * 2.0 ** -11 + 32768e-6) * 12 * books.vc.abs().max().item()
+    assert ((got - want).abs() <= bound + 2.0 ** -10 * want.abs()).all()
+
+
 @pytest.mark.parametrize("kw", [dict(), dict(chunk_pages=64), dict(chunk_pages=2048), dict(tcgen05=True)])
 @pytest.mark.parametrize("length", [2 ** 31 - 1, 2 ** 31 - 16, 2 ** 31 - 17])
 def test_lengths_near_2_31_are_cut_and_flagged(kw, length):

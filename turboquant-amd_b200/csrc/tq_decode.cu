@@ -428,6 +428,8 @@ __global__ void __launch_bounds__(kThreads, TQ_DEC_MINBLOCKS) decode_partial_ker
 #pragma unroll
         for (int r = 0; r < 4; ++r) oacc[i][r] = 0.f;
     bool timed_out = false;
+    // Sparse-V: a group of fewer than eight heads leaves columns of zero queries, whose scores are all alike; they decide nothing.
+    const float thresh0 = 2 * tig < nq ? p.log2_thresh : INFINITY, thresh1 = 2 * tig + 1 < nq ? p.log2_thresh : INFINITY;
     uint32_t v_skipped = 0;
     uint32_t v_parity = 0;                  // bit s: phase of the V barrier of stage s (sparse mode)
     int j_stop = n_my;

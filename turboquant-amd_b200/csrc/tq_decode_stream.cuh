@@ -398,6 +398,8 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
                 sq_init1 = -__shfl_sync(0xffffffffu, corr, 8 * tig + 4);
             }
         }
+        // Sparse-V: columns past the group's heads hold zero queries, whose scores are all alike; they decide nothing
+        const float thresh0 = 2 * tig < nq ? sp.weight_thresh : INFINITY, thresh1 = 2 * tig + 1 < nq ? sp.weight_thresh : INFINITY;
         float m0 = -INFINITY, m1 = -INFINITY;   // softmax reference of queries 2 tig, 2 tig + 1 (log2 domain)
         float l0 = 0.f, l1 = 0.f;
         float oacc[8][4];
@@ -533,7 +535,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
             // ---- Sparse-V: the V part is not needed when no weight of the group exceeds the threshold.  The reference is
             // at most one above the running maximum.
             bool do_v = true;
-            if constexpr (SPARSE) do_v = __any_sync(0xffffffffu, fmaxf(fmaxf(p0v, p1v), fmaxf(p2v, p3v)) > sp.weight_thresh);
+            if constexpr (SPARSE) do_v = __any_sync(0xffffffffu, fmaxf(p0v, p2v) > thresh0 || fmaxf(p1v, p3v) > thresh1);
             bool have = true;
             if constexpr (SPARSE && !HAVE_V) {
                 if (do_v) {   // first needed page after a run of skipped ones: fetch its V part now
