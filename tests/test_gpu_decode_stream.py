@@ -93,6 +93,28 @@ def test_persistent_matches_oracle_and_flags_bad_tables():
     assert_attn_close(out[1:].float().cpu().numpy(), ref[1:])
 
 
+@pytest.mark.parametrize("ns,live", [(701, 40), (2500, 33), (150, 0)])
+def test_padded_batches(ns, live):
+    """Batches of mostly empty sequences: zeros wherever nothing is attended to, more sequences than warps among them."""
+    fmt = CacheFormat.named("turbo4")
+    books = Codebooks(fmt, DEV)
+    lens = [1700] * live + [0] * (ns - live)
+    lens = [lens[(7 * i) % ns] for i in range(ns)]                # 7 divides no ns: a permutation
+    bt, blocks = _tables(lens + [2000], 16, 4)                    # the table is wide though every sequence may be empty
+    cache = _random_cache(fmt, blocks, 4, 16, 8)
+    q = torch.randn(ns, 20, 128, generator=torch.Generator(device=DEV).manual_seed(1), device=DEV).half()
+    lens_t = torch.tensor(lens, dtype=torch.int32, device=DEV)
+    args = (q, cache, bt[:ns].contiguous().to(DEV), lens_t, books, 16)
+    got = paged_decode_attention(*args, out=torch.full_like(q, float("nan")))
+    assert _native.read_status(DEV) == 0
+    assert (got[lens_t == 0] == 0).all()
+    if live:
+        some = (lens_t > 0).nonzero()[:, 0]
+        want = paged_decode_attention(q[some], cache, args[2][some].contiguous(), lens_t[some].contiguous(), books, 16, chunk_pages=64)
+        bound = 2 * 2.0 ** -11 * 12 * books.vc.abs().max().item()
+        assert ((got[some].float() - want.float()).abs() <= bound + 2.0 ** -10 * want.float().abs()).all()
+
+
 @pytest.mark.parametrize("G", [1, 4, 6, 8, 12])
 @pytest.mark.parametrize("chunk", [0, 256])
 def test_sparse_v_skips_for_every_group_size(G, chunk):
