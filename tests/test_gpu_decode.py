@@ -304,6 +304,21 @@ def test_packed_attention_vs_oracle(bits, BH, Sk, splits):
     assert len(PA._get_config(BH, Sk)) == 4
 
 
+@pytest.mark.parametrize("splits", [None, 64])
+def test_packed_attention_keeps_a_nan(splits):
+    """A run of NaN norms that fills many whole parts of the row: softmax over a NaN is NaN, it must not be left out."""
+    c, _ = make_codebook(128, 3, device=DEV)
+    g = torch.Generator(device=DEV).manual_seed(4)
+    Sk = 65536
+    r = lambda w: torch.randint(0, 256, (1, Sk, w), generator=g, dtype=torch.uint8, device=DEV)
+    norm = torch.full((1, Sk), 10.0, dtype=torch.float16, device=DEV)
+    q = torch.randn(1, 128, generator=g, device=DEV).half()
+    args = [q, q, r(48), r(16), norm * 0.1, norm.clone(), r(48), norm, c, 0.0098]
+    assert torch.isfinite(PA.packed_attention(*args, num_splits=splits)).all()
+    args[5][:, 8192:49152] = float("nan")
+    assert torch.isnan(PA.packed_attention(*args, num_splits=splits)).all()
+
+
 def test_packed_compress_feeds_packed_attention():
     """compress_k_permuted / compress_v output, reshaped to [BH, Sk, ...], is what packed_attention reads."""
     BH, Sk = 4, 512

@@ -467,28 +467,31 @@ __global__ void __launch_bounds__(kMergeWarps * 32) packed_attn_merge(const PAPa
     const float2* lse = p.ws_lse;
     const float4* part = reinterpret_cast<const float4*>(p.ws_acc);
     pdl_wait();
-    // four parts at a time, fetched independently of the maxima
+    // eight parts at a time, fetched independently of the maxima and a turn ahead: what a merge costs is its chain of loads
     float M = -INFINITY, l = 0.f;
     float4 o4 = make_float4(0.f, 0.f, 0.f, 0.f);
-    constexpr int kAtOnce = 4;
-    for (int64_t i0 = warp; i0 < parts; i0 += kAtOnce * kMergeWarps) {
-        float2 ml[kAtOnce];
-        float4 v[kAtOnce];
+    constexpr int kAtOnce = 8;
+    float2 ml[kAtOnce], ml_next[kAtOnce];
+    float4 v[kAtOnce], v_next[kAtOnce];
+    auto fetch = [&](int64_t i0, float2 (&a)[kAtOnce], float4 (&b)[kAtOnce]) {
 #pragma unroll
         for (int k = 0; k < kAtOnce; ++k) {
             const int64_t i = i0 + k * kMergeWarps;
-            ml[k] = make_float2(-INFINITY, 0.f);
-            v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+            a[k] = make_float2(-INFINITY, 0.f);
+            b[k] = make_float4(0.f, 0.f, 0.f, 0.f);
             if (i < parts) {
-                ml[k] = lse[slot_of(i)];
-                v[k] = part[slot_of(i) * (kHeadDim / 4) + lane];
+                a[k] = lse[slot_of(i)];
+                b[k] = part[slot_of(i) * (kHeadDim / 4) + lane];
             }
         }
+    };
+    fetch(warp, ml, v);
+    for (int64_t i0 = warp; i0 < parts; i0 += kAtOnce * kMergeWarps) {
+        fetch(i0 + kAtOnce * kMergeWarps, ml_next, v_next);
         float m = M;
 #pragma unroll
         for (int k = 0; k < kAtOnce; ++k) m = fmaxf(m, ml[k].x);
-        if (m == -INFINITY) continue;            // empty parts carry no weight
-        const float old = pa_ex2(M - m);
+        const float old = M == -INFINITY ? 0.f : pa_ex2(M - m);   // empty parts carry no weight; a part of NaN sums stays one
         o4.x *= old; o4.y *= old; o4.z *= old; o4.w *= old;
         l *= old;
 #pragma unroll
@@ -499,6 +502,8 @@ __global__ void __launch_bounds__(kMergeWarps * 32) packed_attn_merge(const PAPa
             o4.z = fmaf(w, v[k].z, o4.z);
             o4.w = fmaf(w, v[k].w, o4.w);
             l = fmaf(w, ml[k].y, l);
+            ml[k] = ml_next[k];
+            v[k] = v_next[k];
         }
         M = m;
     }
