@@ -227,3 +227,36 @@ def test_general_path_on_two_streams_at_once(general):
         for i in (0, 1):
             assert all(torch.equal(r, want[i]) for r in got[i])
     assert _native.read_status(DEV) == 0
+
+
+def test_packed_attention_takes_a_query_and_an_output_that_start_anywhere():
+    """A query at an odd offset is copied, packed K/V at one are refused; the C call accepts any output address and any
+    workspace that tq_packed_attention_workspace_bytes names for the split count of tq_packed_attention_auto_splits."""
+    h, (c, b) = make_wht_matrix(128, device=DEV), make_codebook(128, 3, device=DEV)
+    g = torch.Generator(device=DEV).manual_seed(8)
+    BH, Sk = 3, 1500
+    X = torch.randn(BH * Sk, 128, generator=g, device=DEV).half()
+    packed = [t.view(BH, Sk, *t.shape[1:]) for t in (*compress_k_permuted(X, h, None, c, b), *compress_v(X, h, c, b))]
+    q = torch.randn(BH, 128, generator=g, device=DEV).half()
+
+    def moved(t):
+        buf = torch.empty(t.numel() + 1, dtype=t.dtype, device=DEV)
+        buf[1:] = t.reshape(-1)
+        return buf[1:].view(t.shape)
+
+    want = packed_attention(q, q, *packed, c, 0.01)
+    k_idx, k_signs, k_rnorm, k_norm, v_idx, v_norm = packed
+    assert torch.equal(packed_attention(moved(q), moved(q), k_idx, k_signs, moved(k_rnorm), moved(k_norm), v_idx, moved(v_norm), c, 0.01), want)
+    for i in (0, 1, 4):
+        with pytest.raises(RuntimeError, match="bad argument"):
+            packed_attention(q, q, *(moved(t) if i == j else t for j, t in enumerate(packed)), c, 0.01)
+    L = _native.lib()
+    splits = L.tq_packed_attention_auto_splits(BH, Sk)
+    ws = torch.empty(L.tq_packed_attention_workspace_bytes(BH, splits), dtype=torch.uint8, device=DEV)
+    assert ws.numel() < L.tq_packed_attention_workspace_bytes(BH, 0)
+    out = torch.zeros(BH * 128 + 1, dtype=torch.float16, device=DEV)
+    p = _native._ptr
+    rc = L.tq_packed_attention(p(q), p(q), *(p(t) for t in packed), p(c), 0.01, BH, Sk, 3, 0, p(ws), ws.numel(), p(out[1:]),
+                               _native._stream(torch.device(DEV)))
+    assert rc == 0
+    assert torch.equal(out[1:].view(BH, 128), packed_attention(q, q, *packed, c, 0.01, num_splits=splits))

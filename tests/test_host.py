@@ -173,6 +173,22 @@ def test_launchers_validate_arguments_without_touching_a_gpu():
                              null, null, 2, 8, 8, 1, 3, 3, 1, 0, null) == -1
 
 
+def test_launchers_refuse_misaligned_pointers_without_touching_a_gpu():
+    """Whatever a kernel reads or writes several bytes at a time has to start there; addresses are looked at, not followed."""
+    L = _native.lib()
+    at = lambda a: ctypes.c_void_p(0x10000 + a)
+    null, ok = ctypes.c_void_p(0), at(0)
+    pa = lambda q, ki, ks, vi: L.tq_packed_attention(q, at(2), ki, ks, at(2), at(2), vi, at(2), at(4), 1.0, 2, 64, 3, 0, ok, 0, at(2), null)
+    for off in (2, 8):
+        assert pa(at(off), ok, ok, ok) == pa(ok, at(off), ok, ok) == pa(ok, ok, at(off), ok) == pa(ok, ok, ok, at(off)) == -1
+    assert pa(ok, ok, ok, ok) == -4                                                  # alignment accepted, then no workspace
+    for bits, off in ((2, 4), (3, 2), (4, 8)):
+        assert L.tq_compress_k(ok, 0, 4, at(4), at(4), bits, 0, 1, at(off), ok, at(2), at(2), null) == -1
+        assert L.tq_compress_v(ok, 0, 4, at(4), bits, 0, at(off), at(2), null) == -1
+    polar = lambda x, i, m, s: L.tq_polarquant_compress(x, 2, 4, at(4), at(4), 3, 1, 0, i, at(4), m, s, at(4), null)
+    assert polar(at(8), ok, ok, ok) == polar(ok, at(8), ok, ok) == polar(ok, ok, at(8), ok) == polar(ok, ok, ok, at(8)) == -1
+
+
 def test_head_counts_that_form_no_query_group_are_refused_on_the_host():
     """Fewer query heads than KV heads (or a non-multiple) used to make the chunk-size search loop for ever."""
     L = _native.lib()

@@ -772,6 +772,9 @@ int launch_contig(const ContigParams& p, int bits, cudaStream_t st) {
     return e == cudaSuccess ? TQ_OK : TQ_ERR_LAUNCH;
 }
 
+// What the index rows have to start on: a lane stores its quarter of a row as one access, or, 3-bit, as three words.
+uintptr_t index_align_mask(int bits) { return bits == 4 ? 15 : bits == 2 ? 7 : 3; }
+
 bool dtype_ok(int d) { return d == TQ_DTYPE_F16 || d == TQ_DTYPE_BF16 || d == TQ_DTYPE_F32; }
 int elem_bytes(int d) { return d == TQ_DTYPE_F32 ? 4 : 2; }
 
@@ -859,6 +862,7 @@ extern "C" int tq_compress_k(const void* K, int in_dtype, int64_t n, const float
     if (!K || !centroids || !boundaries || !k_idx || !k_signs || !k_rnorm || !k_norm || n < 0) return TQ_ERR_ARG;
     if (!dtype_ok(in_dtype)) return TQ_ERR_UNSUPPORTED;
     if ((reinterpret_cast<uintptr_t>(K) | reinterpret_cast<uintptr_t>(k_signs)) & 15) return TQ_ERR_ARG;
+    if (reinterpret_cast<uintptr_t>(k_idx) & index_align_mask(bits)) return TQ_ERR_ARG;
     ContigParams p = {};
     p.x = K; p.c = centroids; p.b = boundaries; p.idx_out = k_idx; p.sign_out = k_signs;
     p.rnorm_h = static_cast<__half*>(k_rnorm); p.norm_h = static_cast<__half*>(k_norm);
@@ -871,7 +875,7 @@ extern "C" int tq_compress_v(const void* V, int in_dtype, int64_t n, const float
     if (n == 0) return TQ_OK;
     if (!V || !boundaries || !v_idx || !v_norm || n < 0) return TQ_ERR_ARG;
     if (!dtype_ok(in_dtype)) return TQ_ERR_UNSUPPORTED;
-    if (reinterpret_cast<uintptr_t>(V) & 15) return TQ_ERR_ARG;
+    if (reinterpret_cast<uintptr_t>(V) & 15 || reinterpret_cast<uintptr_t>(v_idx) & index_align_mask(bits)) return TQ_ERR_ARG;
     ContigParams p = {};
     p.x = V; p.b = boundaries; p.idx_out = v_idx; p.norm_h = static_cast<__half*>(v_norm);
     p.n = n; p.in_dtype = in_dtype; p.rotate = prerotated ? 0 : 1;
@@ -885,7 +889,8 @@ extern "C" int tq_polarquant_compress(const void* x, int in_dtype, int64_t n, co
     if (!x || !centroids || !boundaries || !indices || !norms || !k_mse_rot || n < 0) return TQ_ERR_ARG;
     if (use_qjl && (!signs || !rnorm)) return TQ_ERR_ARG;
     if (!dtype_ok(in_dtype)) return TQ_ERR_UNSUPPORTED;
-    if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(k_mse_rot) | reinterpret_cast<uintptr_t>(signs)) & 15)
+    if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(indices) | reinterpret_cast<uintptr_t>(k_mse_rot) |
+         reinterpret_cast<uintptr_t>(signs)) & 15)
         return TQ_ERR_ARG;
     ContigParams p = {};
     p.x = x; p.c = centroids; p.b = boundaries; p.indices = indices; p.norms = norms; p.mse = k_mse_rot;

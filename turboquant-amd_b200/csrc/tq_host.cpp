@@ -372,6 +372,7 @@ PyObject* packed_attention(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
                         : bytes ? x.dim() == 3 && x.size(0) == BH && x.size(1) == Sk && x.size(2) == width[i]
                                 : x.dim() == 2 && x.size(0) == BH && x.size(1) == Sk;
         if (!fits) return declined();
+        if (i == 0 && reinterpret_cast<uintptr_t>(x.const_data_ptr()) % 16) return declined();   // read 16 bytes at a time: to be copied
     }
     const at::Device dev = t[0]->device();
     const c10::cuda::CUDAGuard guard(dev);

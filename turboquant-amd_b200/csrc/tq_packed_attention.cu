@@ -529,8 +529,15 @@ __global__ void __launch_bounds__(kMergeWarps * 32) packed_attn_merge(const PAPa
             o4.w = fmaf(f, v.w, o4.w);
             l = fmaf(f, sl[w], l);
         }
-        *reinterpret_cast<uint2*>(p.out + static_cast<int64_t>(bh) * kHeadDim + 4 * lane) =
-            make_uint2(pack_half2(o4.x / l, o4.y / l), pack_half2(o4.z / l, o4.w / l));
+        __half* dst = p.out + static_cast<int64_t>(bh) * kHeadDim + 4 * lane;
+        if ((reinterpret_cast<uintptr_t>(p.out) & 7) == 0) {
+            *reinterpret_cast<uint2*>(dst) = make_uint2(pack_half2(o4.x / l, o4.y / l), pack_half2(o4.z / l, o4.w / l));
+        } else {   // an output that starts anywhere
+            dst[0] = __float2half_rn(o4.x / l);
+            dst[1] = __float2half_rn(o4.y / l);
+            dst[2] = __float2half_rn(o4.z / l);
+            dst[3] = __float2half_rn(o4.w / l);
+        }
     }
 }
 
@@ -622,9 +629,12 @@ extern "C" int tq_packed_attention(const void* Q, const void* Q_proj, const uint
         return TQ_ERR_ARG;
     if (BH < 0 || Sk <= 0) return TQ_ERR_ARG;
     if (bits < 2 || bits > 4) return TQ_ERR_UNSUPPORTED;
-    if ((reinterpret_cast<uintptr_t>(k_idx) | reinterpret_cast<uintptr_t>(k_signs_perm) | reinterpret_cast<uintptr_t>(v_idx)) & 15)
+    if ((reinterpret_cast<uintptr_t>(Q) | reinterpret_cast<uintptr_t>(k_idx) | reinterpret_cast<uintptr_t>(k_signs_perm) |
+         reinterpret_cast<uintptr_t>(v_idx)) & 15)
         return TQ_ERR_ARG;
     if (num_splits < 0) num_splits = 0;
+    // A workspace that holds the parts of tq_packed_attention_auto_splits, but not those of shared steps: equal parts.
+    if (num_splits == 0 && workspace_bytes < tq_packed_attention_workspace_bytes(BH, 0)) num_splits = tq_packed_attention_auto_splits(BH, Sk);
     if (num_splits > Sk) num_splits = Sk;
     if (num_splits > 65535) return TQ_ERR_UNSUPPORTED;
     if (!workspace || workspace_bytes < tq_packed_attention_workspace_bytes(BH, num_splits) ||

@@ -59,6 +59,8 @@ def packed_attention(Q, Q_proj, k_idx_packed, k_signs_packed, k_r_norm, k_norm,
         raise ValueError("k_signs_packed must be [BH, Sk, 16]")
     half = lambda t: t.to(torch.float16).contiguous()
     Qh, Qph = half(Q), half(Q_proj)
+    if Qh.data_ptr() % 16:                                  # read 16 bytes at a time; so is packed K/V, which is not copied
+        Qh = Qh.clone()
     kidx, ksg, vidx = k_idx_packed.contiguous(), k_signs_packed.contiguous(), v_idx_packed.contiguous()
     krn, kn, vn = half(k_r_norm), half(k_norm), half(v_norm)
     cb = _native._f32(centroids, dev)
