@@ -260,3 +260,38 @@ def test_packed_attention_takes_a_query_and_an_output_that_start_anywhere():
                                _native._stream(torch.device(DEV)))
     assert rc == 0
     assert torch.equal(out[1:].view(BH, 128), packed_attention(q, q, *packed, c, 0.01, num_splits=splits))
+
+
+def test_tracing_modes_and_autograd_see_the_operators():
+    fmt = CacheFormat.named("turbo3")
+    books = Codebooks(fmt, DEV)
+    cache, tables, lens, K, V, slots = _filled(fmt, [40, 7], 2, 16, torch.float16)
+    compress_and_scatter(K, V, cache, slots, books, 16)
+    q, other = (torch.randn(2, 8, 128, device=DEV, dtype=torch.float16) for _ in range(2))
+    attend = lambda q: paged_decode_attention(q, cache, tables, lens, books, 16)
+
+    traced = torch.jit.trace(attend, (q,), check_trace=False)
+    assert "tq_b200::decode_paged" in str(traced.graph)
+    assert torch.equal(traced(other), attend(other))                       # not the result of the traced query
+
+    class Names(torch.overrides.TorchFunctionMode):
+        def __init__(self):
+            super().__init__()
+            self.names = []
+
+        def __torch_function__(self, func, types, args=(), kwargs=None):
+            self.names.append(str(func))
+            return func(*args, **(kwargs or {}))
+
+    with Names() as mode:
+        attend(q)
+        compress_and_scatter(K, V, cache, slots, books, 16)
+    assert any("decode_paged" in n for n in mode.names) and any("compress_paged" in n for n in mode.names)
+
+    proj = other.clone().requires_grad_(True)                              # no formula for its gradient: not dropped silently
+    out = paged_decode_attention(q, cache, tables, lens, books, 16, q_proj=proj)
+    assert out.requires_grad
+    with torch.no_grad():
+        assert torch.equal(out, paged_decode_attention(q, cache, tables, lens, books, 16, q_proj=proj))
+    with pytest.raises(RuntimeError):
+        out.float().sum().backward()

@@ -12,6 +12,8 @@
 #include <dlfcn.h>
 
 #include <ATen/ATen.h>
+#include <ATen/PythonTorchFunctionTLS.h>
+#include <ATen/TracerMode.h>
 #include <ATen/core/grad_mode.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/core/impl/LocalDispatchKeySet.h>
@@ -46,9 +48,11 @@ int32_t* g_status[kMaxDevices] = {};   // device status words; the tensors are o
 
 PyObject* declined() { Py_RETURN_NONE; }
 
-// Inside torch.func transforms, __torch_dispatch__ modes and the like an operator call has to be seen by the dispatcher.
+// Inside torch.func transforms, __torch_dispatch__ and __torch_function__ modes and torch.jit.trace an operator call has to be
+// seen by the dispatcher.
 bool plain_eager() {
-    if (c10::impl::TorchDispatchModeTLS::any_modes_set()) return false;
+    if (c10::impl::TorchDispatchModeTLS::any_modes_set() || at::impl::torch_function_mode_enabled() || at::tracer::impl::is_dispatch_enabled())
+        return false;
     return !c10::impl::tls_local_dispatch_key_set().included_.has_any(
         c10::DispatchKeySet({c10::DispatchKey::FuncTorchDynamicLayerFrontMode, c10::DispatchKey::Python}));
 }
@@ -170,7 +174,7 @@ PyObject* decode(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     };
     void* tmp = nullptr;
     if (args[6] != Py_None) {
-        if (!like_q(args[6], tmp)) return declined();
+        if (!like_q(args[6], tmp) || (at::GradMode::is_enabled() && THPVariable_Unpack(args[6]).requires_grad())) return declined();
         proj = tmp;
     }
     if (args[7] != Py_None && !like_q(args[7], out_ptr)) return declined();
@@ -393,6 +397,7 @@ PyObject* packed_attention(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
 
 // set_status(device index, int32 tensor that lives as long as the process)
 PyObject* set_status(PyObject*, PyObject* args) {
+    HANDLE_TH_ERRORS
     int dev;
     PyObject* obj;
     if (!PyArg_ParseTuple(args, "iO", &dev, &obj)) return nullptr;
@@ -403,6 +408,7 @@ PyObject* set_status(PyObject*, PyObject* args) {
     }
     if (dev < kMaxDevices) g_status[dev] = t->data_ptr<int32_t>();
     Py_RETURN_NONE;
+    END_HANDLE_TH_ERRORS
 }
 
 // bind(path): take the launchers from the library at path (already loaded by the caller)
