@@ -18,6 +18,32 @@ constexpr int kStreamTable = 65536;          // 256 entries of 256 bytes: 128 by
 constexpr int kStreamCtas = 148;             // one per SM
 constexpr int kStreamSmem = 227328;          // dynamic part of the 227 KB an SM gives one CTA
 constexpr int kStreamSlotFloats = 8 * kHeadDim;
+constexpr int kStreamBars = kStreamWarps * 2 * kStreamStages * 8;
+
+// Where the table and the barriers lie, and how many rings of `ring` bytes fit below and above the table, when the dynamic shared
+// memory starts at address `base`.
+struct StreamPlaces {
+    uint32_t tab, bars, low, high;   // table, barriers, first ring below the table, first ring above it
+    int n_low, n_high;
+    __host__ __device__ constexpr StreamPlaces(uint32_t base, int ring)
+        : tab((base + kStreamTable - 1) & ~static_cast<uint32_t>(kStreamTable - 1)), bars(base), low(base + kStreamBars), high(tab + kStreamTable), n_low(0), n_high(0) {
+        if (tab - base < kStreamBars) {   // no room for the barriers below the table
+            bars = high;
+            low = base;
+            high += kStreamBars;
+        }
+        n_low = static_cast<int>((tab - low) / ring);
+        n_high = static_cast<int>((base + kStreamSmem - high) / ring);
+    }
+    __host__ __device__ constexpr uint32_t ring_of(int warp, int ring) const { return warp < n_low ? low + warp * ring : high + (warp - n_low) * ring; }
+};
+// It starts behind what the system reserves (1 KB) and the kernel's static arrays (under 5 KB); the launch checks that it does.
+constexpr uint32_t kStreamFirstBase = 1024, kStreamLastBase = 6144;
+__host__ __device__ constexpr bool stream_rings_fit(int ring) {
+    for (uint32_t base = kStreamFirstBase; base <= kStreamLastBase; base += 16)
+        if (StreamPlaces(base, ring).n_low + StreamPlaces(base, ring).n_high < kStreamWarps) return false;
+    return true;
+}
 
 struct StreamParams {
     DecodeParams d;
@@ -220,9 +246,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
     constexpr int PAGE = KPART + 256 * VB + 32;
     constexpr int NSTAGE = kStreamStages;
     constexpr int RING = NSTAGE * PAGE;
-    constexpr int kBars = kStreamWarps * 2 * NSTAGE * 8;
-    // Wherever the dynamic part starts in the first 4 KB, the rings fit around the table.
-    static_assert((kStreamTable - 4096 - kBars) / RING + (kStreamSmem + 1024 - 2 * kStreamTable) / RING >= kStreamWarps, "rings do not fit");
+    static_assert(stream_rings_fit(RING), "the rings of all warps fit around the table, wherever the dynamic part may start");
     const DecodeParams& p = sp.d;
 
     extern __shared__ __align__(128) uint8_t smem[];
@@ -236,15 +260,9 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
 
     // ---- shared memory: the table on a 64 KB boundary (its addresses are built by a byte permute), barriers and the
     // rings of as many warps as fit below it, the other rings above it
-    const uint32_t base = smem_u32(smem);
-    const uint32_t tab = (base + kStreamTable - 1) & ~static_cast<uint32_t>(kStreamTable - 1);
-    const uint32_t room = tab - base;
-    const bool bars_low = room >= kBars;
-    const uint32_t bars = bars_low ? base : tab + kStreamTable;
-    const int n_low = bars_low ? static_cast<int>((room - kBars) / RING) : static_cast<int>(room / RING);
-    const uint32_t ring = warp < n_low ? base + (bars_low ? kBars : 0) + warp * RING
-                                       : tab + kStreamTable + (bars_low ? 0 : kBars) + (warp - n_low) * RING;
-    const uint32_t bar = bars + warp * 2 * NSTAGE * 8;     // [0 .. NSTAGE) page (or K part), [NSTAGE ..) late V part
+    const StreamPlaces places(smem_u32(smem), RING);
+    const uint32_t tab = places.tab, ring = places.ring_of(warp, RING);
+    const uint32_t bar = places.bars + warp * 2 * NSTAGE * 8;     // [0 .. NSTAGE) page (or K part), [NSTAGE ..) late V part
 
     if constexpr (SIGN_TABLE) fill_sign_table(tab + 128, warp, lane);   // constants
     if (lane < 2) sm_part[2 * warp + lane] = make_int4(-1, 0, 0, 0);
@@ -723,9 +741,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
         }
         if ((run & 1) != (warp >> 3)) continue;
         const int g = warp & 7;
-        auto ring_of = [&](int w) {
-            return w < n_low ? base + (bars_low ? kBars : 0) + w * RING : tab + kStreamTable + (bars_low ? 0 : kBars) + (w - n_low) * RING;
-        };
+        auto ring_of = [&](int w) { return StreamPlaces(smem_u32(smem), RING).ring_of(w, RING); };
         // lane e holds (maximum, denominator) of entry e
         float2 ml = make_float2(-INFINITY, 0.f);
         if ((mine >> lane) & 1u) {
@@ -783,6 +799,13 @@ int launch_stream_as(const StreamParams& sp, cudaStream_t stream) {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return TQ_ERR_LAUNCH;
     if (!configured[dev]) {
+        cudaFuncAttributes attr;
+        int reserved = 0;
+        if (cudaFuncGetAttributes(&attr, kern) != cudaSuccess ||
+            cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev) != cudaSuccess)
+            return TQ_ERR_LAUNCH;
+        const uint64_t start = (static_cast<uint64_t>(reserved) + attr.sharedSizeBytes + 127) & ~uint64_t{127};
+        if (start < kStreamFirstBase || start > kStreamLastBase) return TQ_ERR_UNSUPPORTED;
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kStreamSmem) != cudaSuccess) return TQ_ERR_LAUNCH;
         configured[dev] = true;
     }
