@@ -148,6 +148,13 @@ def test_packed_attention_work_sharing(bits, BH, Sk):
         assert ((got - want).abs() <= 2.0 ** -10 * want.abs() + (2.0 ** -15 + Sk * 2.0 ** -24) * 12 * c.abs().max()).all()
 
 
+@pytest.mark.parametrize("bits", [2, 3])
+@pytest.mark.parametrize("BH,Sk", [(149, 128), (150, 600), (296, 129), (297, 128), (593, 17), (700, 500)])
+def test_packed_attention_two_ctas_per_sm(bits, BH, Sk):
+    """More rows than SMs: CTAs of 8 warps, two per SM, around one and two waves of them and the ends of a 128-token step."""
+    test_packed_attention_work_sharing(bits, BH, Sk)
+
+
 @pytest.mark.parametrize("bits", [2, 3, 4])
 def test_codebook_written_on_the_stream_just_before_the_call(bits):
     """The kernel before may be the one that makes the codebook: a cast (general path) or a copy into the caller's tensors

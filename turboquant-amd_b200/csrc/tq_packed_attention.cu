@@ -20,9 +20,10 @@
 namespace tq {
 namespace {
 
-constexpr int kPaWarps = 16;                    // one CTA per SM; up to 128 registers per thread
-constexpr int kPaThreads = kPaWarps * 32;
-constexpr int kStepTokens = kPaWarps * 16;      // tokens of one step of the CTA, 16 per warp
+// Warps of a CTA: 16, one CTA per SM (up to 128 registers per thread), or 8, two CTAs per SM, whose sign tables and merges
+// then overlap with one another's steps (2- and 3-bit; the 4-bit tables leave room for one CTA only).
+constexpr int kPaWarps = 16, kPaHalfWarps = 8;
+__host__ __device__ constexpr int step_tokens(int warps) { return warps * 16; }   // tokens of one step of the CTA, 16 per warp
 constexpr int kSignTabBytes = 8 * 16 * 128;     // [nibble position][nibble value][lane]
 constexpr float kLog2e = 1.4426950408889634f;
 
@@ -106,8 +107,10 @@ __device__ __forceinline__ void lds_words(uint32_t addr, uint32_t (&w)[BITS]) {
 
 constexpr int kPaStages = 2;   // ring of 16-token steps per warp: the one being worked on, the other in flight
 
-template <int BITS>
+template <int BITS, int WARPS>
 struct PALayout {
+    static constexpr int kThreads = WARPS * 32;
+    static constexpr int kStepTokens = step_tokens(WARPS);
     static constexpr int kRow = 16 * BITS;                              // index bytes per token
     static constexpr int kPairs = 1 << (2 * BITS);
     static constexpr int kPairTabBytes = kPairs * 256;                  // (c[i0], c[i1]) as two floats per lane: V
@@ -115,7 +118,7 @@ struct PALayout {
     static constexpr int kSignTabOff = kPairTabBytes + kHalfTabBytes;
     static constexpr int kStageOff = kSignTabOff + kSignTabBytes;
     static constexpr int kStageBytes = 32 * kRow + 256;                 // 16 K rows, 16 V rows, 16 sign rows
-    static constexpr int kSmem = kStageOff + kPaWarps * kPaStages * kStageBytes;
+    static constexpr int kSmem = kStageOff + WARPS * kPaStages * kStageBytes;
 };
 
 // A warp takes 16 tokens per step.  Lane (slot, quarter) = (lane >> 2, lane & 3) owns quarter `quarter` (32 dims) of
@@ -137,17 +140,17 @@ struct Segment {   // part of a row
     int slot;            // of its partial; -1: the whole row
 };
 
-template <int BITS>
-__global__ void __launch_bounds__(kPaThreads, 1) packed_attn_partial(const PAParams p, int n_items) {
-    using LO = PALayout<BITS>;
-    constexpr int ROW = LO::kRow;
+template <int BITS, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, kPaWarps / WARPS) packed_attn_partial(const PAParams p, int n_items) {
+    using LO = PALayout<BITS, WARPS>;
+    constexpr int ROW = LO::kRow, kStepTokens = LO::kStepTokens;
     extern __shared__ __align__(128) unsigned char pa_smem[];
     unsigned char* pair_tab = pa_smem;
     unsigned char* half_tab = pa_smem + LO::kPairTabBytes;
     unsigned char* sign_tab = pa_smem + LO::kSignTabOff;        // [nibble position][value][lane] float
     __shared__ __align__(16) float sqp[kHeadDim];
-    __shared__ __align__(16) float sacc[kPaWarps][kHeadDim];
-    __shared__ float sml[kPaWarps][2];
+    __shared__ __align__(16) float sacc[WARPS][kHeadDim];
+    __shared__ float sml[WARPS][2];
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int slot = lane >> 2, quarter = lane & 3;
@@ -253,11 +256,11 @@ __global__ void __launch_bounds__(kPaThreads, 1) packed_attn_partial(const PAPar
         const float cv = __ldg(p.centroids + (lane & ((1 << BITS) - 1)));
         begin(at);
         auto pair = [&](int pr) { return make_float2(__shfl_sync(0xffffffffu, cv, pr & ((1 << BITS) - 1)), __shfl_sync(0xffffffffu, cv, pr >> BITS)); };
-        for (int p0 = 2 * warp; p0 < LO::kPairs; p0 += 2 * kPaWarps) {       // 16 bytes a lane
+        for (int p0 = 2 * warp; p0 < LO::kPairs; p0 += 2 * WARPS) {       // 16 bytes a lane
             const float2 c = pair(p0 + (lane >> 4));
             *reinterpret_cast<float4*>(pair_tab + p0 * 256 + lane * 16) = make_float4(c.x, c.y, c.x, c.y);
         }
-        for (int p0 = 4 * warp; p0 < LO::kPairs; p0 += 4 * kPaWarps) {
+        for (int p0 = 4 * warp; p0 < LO::kPairs; p0 += 4 * WARPS) {
             const float2 c = pair(p0 + (lane >> 3));
             const uint32_t h = pack_half2(c.x, c.y);
             *reinterpret_cast<uint4*>(half_tab + p0 * 128 + lane * 16) = make_uint4(h, h, h, h);
@@ -285,7 +288,7 @@ __global__ void __launch_bounds__(kPaThreads, 1) packed_attn_partial(const PAPar
         __syncthreads();
         // Sign nibble g = 2 c + h of a lane's sign word (byte c = byte `quarter` of sign word c) holds, in bit kk, the
         // sign of local dim 4 (4 h + kk) + c (stride-4 order: dim 4 i + c is bit i of word c).
-        for (int e = tid; e < 8 * 16 * 32; e += kPaThreads) {
+        for (int e = tid; e < 8 * 16 * 32; e += LO::kThreads) {
             const int ln = e & 31, v = (e >> 5) & 15, g = e >> 9, c = g >> 1, h = g & 1, q = ln & 3;
             float acc = 0.f;
 #pragma unroll
@@ -419,10 +422,10 @@ __global__ void __launch_bounds__(kPaThreads, 1) packed_attn_partial(const PAPar
         if (tid < kHeadDim) {
             float Mc = sml[0][0];
 #pragma unroll
-            for (int w = 1; w < kPaWarps; ++w) Mc = fmaxf(Mc, sml[w][0]);
+            for (int w = 1; w < WARPS; ++w) Mc = fmaxf(Mc, sml[w][0]);
             float o = 0.f, l = 0.f;
 #pragma unroll
-            for (int w = 0; w < kPaWarps; ++w) {
+            for (int w = 0; w < WARPS; ++w) {
                 const float fw = (sml[w][0] == -INFINITY) ? 0.f : pa_ex2(sml[w][0] - Mc);
                 o = fmaf(fw, sacc[w][tid], o);
                 l = fmaf(fw, sml[w][1], l);
@@ -440,7 +443,7 @@ __global__ void __launch_bounds__(kPaThreads, 1) packed_attn_partial(const PAPar
 
 // One block per row: four warps share the parts, a lane holds four dims.
 constexpr int kMergeWarps = 4;
-__global__ void __launch_bounds__(kMergeWarps * 32) packed_attn_merge(const PAParams p, int n_ctas) {
+__global__ void __launch_bounds__(kMergeWarps * 32) packed_attn_merge(const PAParams p, int n_ctas, int steps) {
     __shared__ float4 so[kMergeWarps][32];
     __shared__ float sl[kMergeWarps];
     __shared__ float sm[kMergeWarps];
@@ -451,7 +454,6 @@ __global__ void __launch_bounds__(kMergeWarps * 32) packed_attn_merge(const PAPa
         slot0 = static_cast<int64_t>(bh) * p.num_splits;
         parts = p.num_splits;
     } else {
-        const int steps = (p.Sk + kStepTokens - 1) / kStepTokens;
         const int64_t total = static_cast<int64_t>(p.BH) * steps, first = static_cast<int64_t>(bh) * steps;
         // the CTA whose share holds step u is the largest c with floor(c total / n) <= u
         const int64_t c0 = ((first + 1) * n_ctas - 1) / total, c1 = ((first + steps) * n_ctas - 1) / total;
@@ -578,39 +580,54 @@ __global__ void __launch_bounds__(128) wht_rows_kernel(const void* in, void* out
 
 using namespace tq;
 
-constexpr int64_t kMaxCtas = 256;   // CTAs that share the steps of all rows: at most one per SM
+constexpr int64_t kMaxCtas = 512;   // CTAs that share the steps of all rows: at most two per SM
 
-// How many CTAs share the steps of all rows.  All SMs balance best, but a share that crosses into another row pays for
-// another sign table and merge; with few steps per CTA that is dearer than idle SMs.  A step costs about 1.4 us, a row (or
-// part of one) 3 us.  Candidates: one CTA per SM; every row cut into the same number of parts; whole rows.  (64 x 1000
-// tokens: 148 CTAs 15.3 us, 128 CTAs 9; 64 x 32768: 90.8 against 95.)
-static int64_t share_out(int64_t BH, int64_t Sk, int64_t sms) {
-    const int64_t S = (Sk + kStepTokens - 1) / kStepTokens, total = BH * S;
-    auto cost = [](int64_t steps, int64_t rows) { return 1.4 * static_cast<double>(steps) + 3.0 * static_cast<double>(rows); };
-    int64_t best = total < sms ? total : sms;
-    const int64_t each = (total + best - 1) / best;
-    double least = cost(each, 1 + (each - 1 + S - 1) / S);
-    auto consider = [&](int64_t ctas, double c) {
-        if (c < least) {
-            least = c;
-            best = ctas;
-        }
+// How a call without an explicit split runs: so many CTAs of so many warps share the steps of all rows.
+struct Sharing {
+    int warps;
+    int64_t ctas;
+    double us;    // estimated
+    bool whole;   // rows are dealt out whole (no merge kernel); else the steps of all rows are shared
+};
+
+// All SMs balance best, but a share that crosses into another row pays for another sign table and merge; with few steps per
+// CTA that is dearer than idle SMs.  A step of 256 tokens costs about 1.4 us, a row (or part of one) 3 us; two CTAs of 8 warps
+// take 1.5 us for a step of 128 tokens each and 3.3 us for a row, side by side; a merge kernel adds 1.5.  Candidates: all
+// CTAs; every row cut into the same number of parts; whole rows.  (16 warps, 64 x 1000 tokens: 148 CTAs 15.3 us, 128 CTAs 9;
+// 64 x 32768: 90.8 against 95.)
+static Sharing share_among(int64_t BH, int64_t Sk, int64_t ctas, int warps) {
+    const int64_t S = (Sk + step_tokens(warps) - 1) / step_tokens(warps), total = BH * S;
+    const double step_us = warps == kPaWarps ? 1.4 : 1.5, row_us = warps == kPaWarps ? 3.0 : 3.3;
+    auto cost = [&](int64_t steps, int64_t rows) { return step_us * static_cast<double>(steps) + row_us * static_cast<double>(rows); };
+    constexpr double kMergeUs = 1.5;
+    Sharing best = {warps, total < ctas ? total : ctas, 0.0, false};
+    const int64_t each = (total + best.ctas - 1) / best.ctas;
+    best.us = cost(each, 1 + (each - 1 + S - 1) / S) + kMergeUs;
+    auto consider = [&](const Sharing& other) {
+        if (other.us < best.us) best = other;
     };
-    if (BH <= sms) {
-        const int64_t parts = sms / BH < S ? sms / BH : S;
-        consider(BH * parts, cost((S + parts - 1) / parts, 1));
+    if (BH <= ctas) {
+        const int64_t parts = ctas / BH < S ? ctas / BH : S;
+        consider({warps, BH * parts, cost((S + parts - 1) / parts, 1) + kMergeUs, false});
     }
-    for (int64_t rows = (BH + sms - 1) / sms; rows <= BH && rows <= 4 * ((BH + sms - 1) / sms); ++rows)
-        if (BH % rows == 0) {
-            consider(BH / rows, cost(rows * S, rows));
-            break;
-        }
+    const int64_t rows = (BH + ctas - 1) / ctas;
+    consider({warps, BH < ctas ? BH : ctas, cost(rows * S, rows), true});
     return best;
+}
+
+// Many rows of few steps are mostly sign tables and merges, which overlap where two CTAs share an SM.  Measured in a graph, us, one
+// CTA of 16 warps / two of 8, 3-bit: 150 x 300 tokens 14.2 / 10.3, 256 x 500 16.1 / 13.0, 256 x 2048 32.5 / 29.9, 1000 x 256
+// 40.8 / 33.5, 2000 x 64 62.3 / 40.9.
+static Sharing share_out(int64_t BH, int64_t Sk, int bits, int64_t sms) {
+    const Sharing one = share_among(BH, Sk, sms, kPaWarps);
+    if (bits == 4) return one;
+    const Sharing two = share_among(BH, Sk, 2 * sms, kPaHalfWarps);
+    return two.us < one.us ? two : one;
 }
 
 extern "C" int tq_packed_attention_auto_splits(int BH, int Sk) {
     if (BH <= 0 || Sk <= 0) return TQ_ERR_ARG;
-    const int64_t parts = share_out(BH, Sk, 148) / BH;   // CTAs per row
+    const int64_t parts = share_among(BH, Sk, 148, kPaWarps).ctas / BH;   // CTAs per row on the 148 SMs of a B200
     return static_cast<int>(parts < 1 ? 1 : parts);
 }
 
@@ -667,24 +684,43 @@ extern "C" int tq_packed_attention(const void* Q, const void* Q_proj, const uint
     if (dev < 0 || dev >= 64) return TQ_ERR_UNSUPPORTED;
     if (!configured[dev]) {
         if (cudaDeviceGetAttribute(&sm_count[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return TQ_ERR_LAUNCH;
-        if (cudaFuncSetAttribute(packed_attn_partial<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, PALayout<4>::kSmem) != cudaSuccess ||
-            cudaFuncSetAttribute(packed_attn_partial<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, PALayout<3>::kSmem) != cudaSuccess ||
-            cudaFuncSetAttribute(packed_attn_partial<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, PALayout<2>::kSmem) != cudaSuccess)
+        auto opt_in = [](auto kernel, int bytes) { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess; };
+        if (!opt_in(packed_attn_partial<4, kPaWarps>, PALayout<4, kPaWarps>::kSmem) || !opt_in(packed_attn_partial<3, kPaWarps>, PALayout<3, kPaWarps>::kSmem) ||
+            !opt_in(packed_attn_partial<2, kPaWarps>, PALayout<2, kPaWarps>::kSmem) || !opt_in(packed_attn_partial<3, kPaHalfWarps>, PALayout<3, kPaHalfWarps>::kSmem) ||
+            !opt_in(packed_attn_partial<2, kPaHalfWarps>, PALayout<2, kPaHalfWarps>::kSmem))
             return TQ_ERR_LAUNCH;
         configured[dev] = true;
     }
-    const int64_t most = sm_count[dev] < kMaxCtas ? sm_count[dev] : kMaxCtas;
-    const unsigned grid = static_cast<unsigned>(num_splits > 0 ? (slots < most ? slots : most) : share_out(BH, Sk, most));
-    const int n_items = num_splits > 0 ? static_cast<int>(slots) : 0;
+    const int64_t sms = sm_count[dev] < kMaxCtas / 2 ? sm_count[dev] : kMaxCtas / 2;
+    Sharing run = {};
+    if (num_splits > 0) {   // items of their own: two CTAs per SM where there are enough of them
+        run.warps = bits < 4 && slots > sms ? kPaHalfWarps : kPaWarps;
+        const int64_t most = run.warps == kPaWarps ? sms : 2 * sms;
+        run.ctas = slots < most ? slots : most;
+    } else {
+        run = share_out(BH, Sk, bits, sms);
+        if (run.whole) p.num_splits = num_splits = 1;
+    }
+    const int n_items = num_splits > 0 ? BH * num_splits : 0;
+    auto partial = [&](auto kernel, int threads, int smem) {
+        return launch_chained(kernel, dim3(static_cast<unsigned>(run.ctas)), dim3(threads), smem, st, p, n_items) == cudaSuccess;
+    };
     bool launched = false;
-    switch (bits) {
-        case 2: launched = launch_chained(packed_attn_partial<2>, dim3(grid), dim3(kPaThreads), PALayout<2>::kSmem, st, p, n_items) == cudaSuccess; break;
-        case 3: launched = launch_chained(packed_attn_partial<3>, dim3(grid), dim3(kPaThreads), PALayout<3>::kSmem, st, p, n_items) == cudaSuccess; break;
-        case 4: launched = launch_chained(packed_attn_partial<4>, dim3(grid), dim3(kPaThreads), PALayout<4>::kSmem, st, p, n_items) == cudaSuccess; break;
+    if (run.warps == kPaWarps) {
+        switch (bits) {
+            case 2: launched = partial(packed_attn_partial<2, kPaWarps>, kPaWarps * 32, PALayout<2, kPaWarps>::kSmem); break;
+            case 3: launched = partial(packed_attn_partial<3, kPaWarps>, kPaWarps * 32, PALayout<3, kPaWarps>::kSmem); break;
+            case 4: launched = partial(packed_attn_partial<4, kPaWarps>, kPaWarps * 32, PALayout<4, kPaWarps>::kSmem); break;
+        }
+    } else if (bits == 2) {
+        launched = partial(packed_attn_partial<2, kPaHalfWarps>, kPaHalfWarps * 32, PALayout<2, kPaHalfWarps>::kSmem);
+    } else {
+        launched = partial(packed_attn_partial<3, kPaHalfWarps>, kPaHalfWarps * 32, PALayout<3, kPaHalfWarps>::kSmem);
     }
     if (!launched) return TQ_ERR_LAUNCH;
-    if (num_splits == 1 || (num_splits == 0 && grid == 1)) return TQ_OK;   // every row was written whole
-    return launch_chained(packed_attn_merge, dim3(static_cast<unsigned>(BH)), dim3(kMergeWarps * 32), 0, st, p, static_cast<int>(grid)) == cudaSuccess
+    if (num_splits == 1 || (num_splits == 0 && run.ctas == 1)) return TQ_OK;   // every row was written whole
+    const int steps = (Sk + step_tokens(run.warps) - 1) / step_tokens(run.warps);   // per row
+    return launch_chained(packed_attn_merge, dim3(static_cast<unsigned>(BH)), dim3(kMergeWarps * 32), 0, st, p, static_cast<int>(run.ctas), steps) == cudaSuccess
                ? TQ_OK
                : TQ_ERR_LAUNCH;
 }
