@@ -107,8 +107,9 @@ __device__ __forceinline__ uint4 pair_entry(float cv, int b) {
 template <int BITS>
 __device__ __forceinline__ void fill_pair_lut(uint32_t* tab, float centroid, int warp, int lane) {
     const float cv = __half2float(__float2half_rn(centroid));
-    for (int b0 = 4 * warp; b0 < lut_entries<BITS>(); b0 += 4 * kWarps) {
-        const int b = b0 + (lane >> 3);
+#pragma unroll 8
+    for (int i = 0; i < lut_entries<BITS>() / (4 * kWarps); ++i) {   // unrolled: the shuffles of several entries overlap
+        const int b = 4 * (i * kWarps + warp) + (lane >> 3);
         *reinterpret_cast<uint4*>(tab + b * 32 + 4 * (lane & 7)) = pair_entry<BITS>(cv, b);
     }
 }

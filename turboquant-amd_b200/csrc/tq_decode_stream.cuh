@@ -139,8 +139,9 @@ __device__ __forceinline__ void store_entry(uint32_t addr, uint4 v) {
 template <int BITS>
 __device__ __forceinline__ void fill_stream_table(uint32_t smem_addr, float centroid, int warp, int lane) {
     const float cv = __half2float(__float2half_rn(centroid));
-    for (int b0 = 4 * warp; b0 < 256; b0 += 4 * kStreamWarps) {   // eight lanes an entry
-        const int b = b0 + (lane >> 3);
+#pragma unroll
+    for (int i = 0; i < 256 / (4 * kStreamWarps); ++i) {   // eight lanes an entry
+        const int b = 4 * (i * kStreamWarps + warp) + (lane >> 3);
         store_entry(smem_addr + b * 256 + 16 * (lane & 7), pair_entry<BITS>(cv, b));
     }
 }

@@ -256,11 +256,17 @@ __global__ void __launch_bounds__(WARPS * 32, kPaWarps / WARPS) packed_attn_part
         const float cv = __ldg(p.centroids + (lane & ((1 << BITS) - 1)));
         begin(at);
         auto pair = [&](int pr) { return make_float2(__shfl_sync(0xffffffffu, cv, pr & ((1 << BITS) - 1)), __shfl_sync(0xffffffffu, cv, pr >> BITS)); };
-        for (int p0 = 2 * warp; p0 < LO::kPairs; p0 += 2 * WARPS) {       // 16 bytes a lane
+#pragma unroll
+        for (int i = 0; i < (LO::kPairs + 2 * WARPS - 1) / (2 * WARPS); ++i) {       // 16 bytes a lane
+            const int p0 = 2 * (i * WARPS + warp);
+            if (p0 >= LO::kPairs) break;
             const float2 c = pair(p0 + (lane >> 4));
             *reinterpret_cast<float4*>(pair_tab + p0 * 256 + lane * 16) = make_float4(c.x, c.y, c.x, c.y);
         }
-        for (int p0 = 4 * warp; p0 < LO::kPairs; p0 += 4 * WARPS) {
+#pragma unroll
+        for (int i = 0; i < (LO::kPairs + 4 * WARPS - 1) / (4 * WARPS); ++i) {
+            const int p0 = 4 * (i * WARPS + warp);
+            if (p0 >= LO::kPairs) break;
             const float2 c = pair(p0 + (lane >> 3));
             const uint32_t h = pack_half2(c.x, c.y);
             *reinterpret_cast<uint4*>(half_tab + p0 * 128 + lane * 16) = make_uint4(h, h, h, h);
