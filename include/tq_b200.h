@@ -113,8 +113,8 @@ int64_t tq_decode_workspace_bytes(int num_seqs, int num_q_heads, int num_kv_head
                                   int max_pages_per_seq, int chunk_pages);
 
 /* Bytes of workspace with which tq_decode_paged(chunk_pages = 0) runs the kernel that suits the shape best: at least
- * tq_decode_workspace_bytes(...), with which it runs the chunked kernel; about 20 MB where the persistent kernel is the
- * better one.  Host only. */
+ * tq_decode_workspace_bytes(...), with which it runs the chunked kernel; 11 MB where the persistent kernel is the better
+ * one.  The two kernels add in another order: with a workspace between the two sizes the last bits differ.  Host only. */
 int64_t tq_decode_auto_workspace_bytes(int num_seqs, int num_q_heads, int num_kv_heads, int max_pages_per_seq);
 
 /* Asymmetric packed paged decode attention with GQA and split-K, one query
@@ -136,8 +136,10 @@ int64_t tq_decode_auto_workspace_bytes(int num_seqs, int num_q_heads, int num_kv
  * rule (a 16-token V page is not fetched when every softmax weight in it, for
  * every query head of the group, is <= sparse_thresh relative to the running
  * maximum); <= 0 disables it.  block_tables: int32 [num_seqs, bt_stride];
- * seq_lens: int32 [num_seqs].  workspace: at least
- * tq_decode_workspace_bytes(...) bytes, 16-byte aligned.  skip_stats:
+ * seq_lens: int32 [num_seqs].  workspace: 16-byte
+ * aligned, this call's own until its kernels are done; tq_decode_auto_workspace_bytes(...)
+ * bytes with chunk_pages = 0 (tq_decode_workspace_bytes(...) are enough, for the
+ * chunked kernel), tq_decode_workspace_bytes(...) with a chunk_pages.  skip_stats:
  * optional device uint32[2] = {V pages visited, V pages skipped}, accumulated
  * with atomics when non-NULL.  Sequences of length 0 produce zeros. */
 int tq_decode_paged(void* out, const void* q_rot, const void* q_proj, int io_dtype,
@@ -158,7 +160,8 @@ int tq_decode_paged(void* out, const void* q_rot, const void* q_proj, int io_dty
  * start-up, so any later allocation fails, or a foreign-language binding that
  * only passes on pointers it received.  Same arguments as tq_decode_paged
  * without workspace / workspace_bytes; the split-K partials go to a fixed
- * 16 MiB array that is part of the library image (every GPU that loads the
+ * 16 MiB array that is part of the library image (the chunked kernel runs, also
+ * with chunk_pages = 0; every GPU that loads the
  * library holds those 16 MiB until the process exits).  Problems that need
  * more (tq_decode_workspace_bytes(...) > TQ_DECODE_STATIC_SCRATCH_BYTES)
  * are refused with TQ_ERR_WORKSPACE before anything is launched: pass a
@@ -214,7 +217,8 @@ int tq_polarquant_compress(const void* x, int in_dtype, int64_t n, const float* 
                            int64_t* indices, float* norms, float* k_mse_rot, float* signs, float* rnorm,
                            tq_stream_t stream);
 
-/* Bytes of workspace tq_packed_attention needs for a split count, 0 included.  Host only. */
+/* Bytes of workspace tq_packed_attention needs for a split count, 0 (which shares the steps of all rows) included.  With
+ * num_splits = 0 and less than that, but enough for tq_packed_attention_auto_splits parts a row, it runs those.  Host only. */
 int64_t tq_packed_attention_workspace_bytes(int BH, int num_splits);
 
 /* About how many CTAs share a row when num_splits = 0; replaces the MI355X
@@ -225,7 +229,8 @@ int tq_packed_attention_auto_splits(int BH, int Sk);
  * contiguous [BH, Sk, ...] packed K/V, one query row per BH, split-K partial
  * kernel plus merge.  Q, Q_proj fp16 [BH,128]; k_idx/v_idx uint8
  * [BH,Sk,16*bits]; k_signs_perm uint8 [BH,Sk,16] in stride-4 order; norms fp16
- * [BH,Sk]; centroids fp32 [2^bits]; out fp16 [BH,128] in rotated space. */
+ * [BH,Sk]; centroids fp32 [2^bits]; out fp16 [BH,128] in rotated space.  Q, k_idx,
+ * k_signs_perm, v_idx and workspace start on 16 bytes. */
 int tq_packed_attention(const void* Q, const void* Q_proj, const uint8_t* k_idx, const uint8_t* k_signs_perm,
                         const void* k_rnorm, const void* k_norm, const uint8_t* v_idx, const void* v_norm,
                         const float* centroids, float corr_scale, int BH, int Sk, int bits, int num_splits,

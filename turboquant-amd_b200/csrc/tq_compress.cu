@@ -750,8 +750,8 @@ int launch_paged_v(const PagedParams& p, int vb, bool qjl, cudaStream_t st) {
 template <OutMode MODE>
 int launch_contig(const ContigParams& p, int bits, cudaStream_t st) {
     // Large launches: the persistent table-driven kernel.  fp16 rows with the rotation, us, binary-search kernel / persistent:
-    // K 16384 rows 5.8 / 5.6, 32768 8.5 / 8.0, 65536 15.4 / 12.0; V 4.9 / 4.3, 7.0 / 5.8, 12.0 / 8.4.  The line stays above
-    // the crossing: the two rotations round differently.
+    // K 16384 rows 5.6 / 5.1, 32768 8.4 / 7.2, 65536 15.4 / 11.0; V 4.6 / 3.7, 6.6 / 5.2, 12.0 / 7.7.  The line stays above
+    // the crossing: the two rotations round differently, so a lower one would change the bytes of those sizes.
     if (p.n > 2 * kSmallLaunchItems) {
         constexpr bool QJL = MODE == OutMode::kPackedK;
         switch (bits) {

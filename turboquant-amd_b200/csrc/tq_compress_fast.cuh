@@ -38,8 +38,9 @@
 namespace tq {
 namespace {
 
-// Compile-time tunables.  The tensor-core loop needs ~128 registers to stay clear of spills (a spilled build at 80
-// registers and 24 warps per SM measured 1.3-1.6x slower than this one at 16 warps per SM).  One CTA of 16 warps
+// Compile-time tunables.  The tensor-core loop wants the 128 registers that 16 warps per SM leave it: 2-bit keys and keys
+// without signs fit, 3- and 4-bit keys with signs spill 36-44 bytes (a build at 80 registers and 24 warps per SM spilled far
+// more and measured 1.3-1.6x slower).  One CTA of 16 warps
 // per SM builds the tables once for all of them: 4 % faster than two CTAs of 8 warps.
 #ifndef TQ_CMP_MINBLOCKS
 #define TQ_CMP_MINBLOCKS 1
@@ -823,8 +824,8 @@ __global__ void __launch_bounds__(kFastWarps * 32, TQ_CMP_MINBLOCKS) compress_pa
 // Small launches (the new tokens of one decode step): no tables to build.  Such a launch is one chain of latencies, so
 // a warp takes the keys or the values of 8 items, not both one after the other, and its rows, their slots and the codebook
 // are requested together (a warp of keys holds the centroids in a copy of its own: no barrier of the CTA).  Measured, us per launch in a graph of such launches,
-// both in one warp / now, 8 KV heads: turbo3 64 tokens 6.1 / 3.4, 1024 tokens 9.8 / 5.4, 2048 tokens 10.1 / 8.9; turbo4 64
-// tokens 6.2 / 3.5.
+// both in one warp / now, 8 KV heads: turbo3 64 tokens 6.1 / 3.4, 1024 tokens 9.8 / 5.6, 2048 tokens 10.1 / 8.8; turbo4 64
+// tokens 6.2 / 3.4.
 template <int KB, int VB, bool QJL>
 __global__ void __launch_bounds__(kWarpsPerCta * 32) compress_paged_small_kernel(const __grid_constant__ PagedParams p) {
     constexpr int PAGE = page_bytes(KB, VB, QJL ? 1 : 0);
@@ -866,8 +867,9 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) compress_paged_small_kernel
 }
 
 // Up to here launches take the small kernel, whose rotation is the plain butterfly.  The tensor-core kernel rounds its
-// rotation differently, and a coordinate in a million would go to the neighbouring centroid; it takes 8.5 us for turbo3, 2048
-// tokens, where the small kernel takes 8.9.
+// rotation differently, and a coordinate in a million would go to the neighbouring centroid: the line is kept for the bytes,
+// not for the time.  us, small kernel / that one: turbo3 1024 tokens 5.6 / 6.0, 2048 tokens 8.8 / 7.9; turbo4 7.0 / 5.8 and
+// 10.8 / 7.4; turbo2 4.9 / 4.3 and 7.3 / 6.0.
 constexpr int64_t kSmallLaunchItems = 16384;
 
 template <int KB, int VB, bool QJL>

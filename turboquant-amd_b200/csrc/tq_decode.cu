@@ -724,13 +724,14 @@ int dispatch_v(const DecodeParams& p, int vb, const Plan& plan, cudaStream_t str
     return TQ_ERR_UNSUPPORTED;
 }
 
-// Which kernel is the better one, by the pages that the batch can have at most.  The persistent kernel pays about 12 us
+// Which kernel is the better one, by the pages that the batch can have at most.  The persistent kernel pays about 11 us
 // however few pages there are (all its tables, one more level of merging), the chunked one 5 to 9, but it takes
 // 0.45 (4-bit) to 0.55 us (with sign term) per 1000 pages where the chunked one takes 0.7 to 0.8; sequences of few pages
 // cost it more, a warp then changes item every few pages.  Measured us, chunked / persistent, 8 KV heads, turbo4 and turbo3:
-// 1 x 16384 tokens (8192 pages) 16.9 / 16.9 and 15.0 / 17.9; 24 x 1024 (12288) 16.8 / 19.6 and 23.1 / 20.6; 64 x 512 (16384)
-// 21.3 / 22.8 and 20.5 / 24.2, 32 x 1024 25.3 / 21.7 and 24.2 / 23.2; 256 x 256 (32768) 44.1 / 39.4 and 44.0 / 42.4;
-// 32 x 3000 (48128) 50.1 / 37.8 and 52.6 / 42.5.
+// 1 x 16384 tokens (8192 pages) 14.6 / 16.1 and 14.1 / 16.8; 24 x 1024 (12288) 15.9 / 18.2 and 22.1 / 19.5; 64 x 512 (16384)
+// 19.1 / 20.6 and 19.4 / 22.2, 32 x 1024 22.8 / 19.4 and 22.9 / 20.9; 256 x 256 (32768) 35.3 / 32.9 and 36.4 / 36.2, 128 x 512
+// 30.2 / 30.1 and 31.9 / 33.1; 32 x 3000 (48128) 48.0 / 35.1 and 51.3 / 39.1.  The line does not look at the format: it is
+// off by 4 to 13 % for 24 x 1024 and 128 x 512 with sign term.
 constexpr int64_t kStreamMinPages = 16384;
 constexpr int64_t kStreamSlots = static_cast<int64_t>(kStreamCtas) * (kStreamWarps + 2);   // partials of warps and of CTAs
 int64_t pages_at_most(int64_t ns, int64_t hq, int64_t hkv, int64_t max_pages) { return ns * max_pages * hkv * ((hq / hkv + 7) / 8); }

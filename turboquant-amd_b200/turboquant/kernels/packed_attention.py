@@ -18,10 +18,10 @@ from turboquant.kernels.packed_compress import unpack_1bit, unpack_2bit  # noqa:
 def _get_config(BH: int, Sk: int):
     """(block_sk, num_splits, num_warps, num_stages) the kernel will use for a problem size.
 
-    The reference looks these up in a table tuned on MI355X; here the split
-    count comes from the library's B200 heuristic and the other three are
-    fixed properties of the CUDA kernel (steps of 256 tokens, 16 warps, no
-    software pipelining stages).
+    The reference looks these up in a table tuned on MI355X; here they describe
+    what the library does on a B200 with CTAs of 16 warps: steps of 256 tokens,
+    about so many CTAs per row, no software pipelining stages.  The launch
+    itself may take CTAs of 8 warps, two per SM, and whole rows.
     """
     return 256, _native.lib().tq_packed_attention_auto_splits(BH, Sk), 16, 1
 
