@@ -177,3 +177,54 @@ def test_persistent_sparse_v_skips_and_stays_close():
     # the skipped weights add up to at most 1e-6 of the maximum for each of 32768 tokens, times |v|
     bound = (2 * 2.0 ** -11 + 32768e-6) * 12 * books.vc.abs().max().item()
     assert ((got - want).abs() <= bound + 2.0 ** -10 * want.abs()).all()
+
+
+@pytest.mark.parametrize("kb,vb,qjl", [(3, 3, True), (3, 4, False), (3, 2, True)])
+@pytest.mark.parametrize("separate", [False, True])
+def test_integer_scores_of_uneven_queries(kb, vb, qjl, separate):
+    """3-bit keys are scored in 16-bit integers scaled by the row's largest value: rows with outliers, tiny, constant and zero rows
+    are no further from 64 bits than the chunked kernel's half-precision products of the same call, up to the roundings that both
+    share (weights and output, 2^-11 each, which differ from one another), and a row with NaN or infinity gives NaN alone."""
+    if separate and not qjl:
+        pytest.skip("a query of the sign term's own")
+    fmt = CacheFormat(kb, vb, qjl)
+    books = Codebooks(fmt, DEV)
+    lens, hkv, G = [8192 + 5, 513, 16, 1, 700, 40, 333, 1025], 4, 8
+    bt, blocks = _tables(lens, 16, 6)
+    cache = _random_cache(fmt, blocks, hkv, 16, 5)
+    g = torch.Generator(device=DEV).manual_seed(2)
+    q = torch.randn(len(lens), hkv, G, 128, generator=g, device=DEV)
+    q[:, :, 1, 17] *= 30
+    q[:, :, 2] *= 1e-6                                        # subnormal in fp16
+    q[:, :, 3] = 0
+    q[:, :, 4] = 0.7
+    q[:, :, 5] = 0
+    q[:, :, 5, 90] = -3
+    q[:, :, 6, ::2] *= 8
+    q = q.half().reshape(len(lens), hkv * G, 128)
+    qp = torch.randn(q.shape, generator=g, device=DEV).half() * 2 if separate else None
+    args = (q, cache, bt.to(DEV), torch.tensor(lens, dtype=torch.int32, device=DEV), books, 16)
+    ref = torch.empty(q.shape, dtype=torch.float64, device=DEV)
+    for i, n in enumerate(lens):
+        f = paged_layout.unpack_cache(cache[bt[i, :-(-n // 16)].long().to(DEV)], 16, kb, vb, qjl)
+        rows = lambda name: f[name].flatten(0, 1)[:n]
+        for h in range(hkv):
+            heads = slice(h * G, (h + 1) * G)
+            s = q[i, heads].double() @ (books.kc.double()[rows("k_idx")[:, h].long()] * rows("k_norm")[:, h, None].double()).T
+            if qjl:
+                signs = (2 * rows("k_signs")[:, h].double() - 1) * rows("k_rnorm")[:, h, None].double() * math.sqrt(math.pi / 2) / 128
+                s += (q if qp is None else qp)[i, heads].double() @ signs.T
+            ref[i, heads] = torch.softmax(s / math.sqrt(128), -1) @ (books.vc.double()[rows("v_idx")[:, h].long()] * rows("v_norm")[:, h, None].double())
+    kw = {} if qp is None else dict(q_proj=qp)
+    by_head = lambda x: (x.double() - ref).reshape(len(lens), hkv, G, 128).pow(2).sum(dim=(0, 1, 3)).sqrt()
+    got, half = paged_decode_attention(*args, **kw), paged_decode_attention(*args, chunk_pages=64, **kw)
+    assert _native.read_status(DEV) == 0
+    size = ref.reshape(len(lens), hkv, G, 128).pow(2).sum(dim=(0, 1, 3)).sqrt()
+    assert (by_head(got) <= by_head(half) + 2.0 ** -11 * size).all(), (by_head(got) / size, by_head(half) / size)
+    for bad in (float("nan"), float("inf")):
+        q2 = q.clone()
+        q2[0, 9, 5] = bad
+        out = paged_decode_attention(q2, *args[1:], **kw)
+        assert out[0, 9].isnan().all()
+        out[0, 9] = got[0, 9]
+        assert torch.equal(out, got)

@@ -8,42 +8,29 @@
 // two of its own, the item it started in the middle of and the item it could not finish, for decode_stream_merge_kernel.
 // Against the chunked kernel (4-warp CTAs, one chunk of one item each) this takes away the last wave that is three
 // quarters full, the table fill, pipeline start and merge per chunk, and the empty CTAs of a ragged batch.
+//
+// What bounds it: instruction issue (62 % of the cycles with four warps a scheduler; a tensor instruction costs it about
+// three slots), and, where keys are looked up, the shared-memory data path next to it (turbo3 with looked-up keys: 82 %).
+// Pages are staged with cp.async, 16 bytes a lane, into a private ring: a page then costs four copy instructions and a counted
+// wait, where a bulk copy by one elected lane with its barrier cost about 35 instructions.  Together with a page body that has no
+// partly filled pages to look after, table addresses from the multiply-add pipe and loop state in uniform registers, us
+// before / now, 8 KV heads: turbo3 64 x 8192 tokens 154.2 / 150.1, turbo4 1 x 131072 43.4 / 41.2, turbo3 128 x 512 33.2 / 31.9, turbo3
+// with a query of the sign term's own 32 x 4096 52.6 / 50.0; 4 KV heads, 32 x 4096: 3-bit K and 4-bit V 31.0 / 28.8, turbo4 26.3 / 25.1.
+// Two pages per iteration came out the same (the loop's own instructions are few now), and so did V operands without the pairing
+// of tokens (twice the products with half of the weights zero: 19 instructions fewer, 8 products more; 154).
 namespace tq {
 namespace {
 
 constexpr int kStreamWarps = 16;
 constexpr int kStreamThreads = kStreamWarps * 32;
 constexpr int kStreamStages = 4;
-constexpr int kStreamTable = 65536;          // 256 entries of 256 bytes: 128 bytes for K, 128 bytes for V
+constexpr int kStreamTable = 32768;          // 256 entries of 128 bytes
 constexpr int kStreamCtas = 148;             // one per SM
-constexpr int kStreamSmem = 227328;          // dynamic part of the 227 KB an SM gives one CTA
 constexpr int kStreamSlotFloats = 8 * kHeadDim;
-constexpr int kStreamBars = kStreamWarps * 2 * kStreamStages * 8;
 
-// Where the table and the barriers lie, and how many rings of `ring` bytes fit below and above the table, when the dynamic shared
-// memory starts at address `base`.
-struct StreamPlaces {
-    uint32_t tab, bars, low, high;   // table, barriers, first ring below the table, first ring above it
-    int n_low, n_high;
-    __host__ __device__ constexpr StreamPlaces(uint32_t base, int ring)
-        : tab((base + kStreamTable - 1) & ~static_cast<uint32_t>(kStreamTable - 1)), bars(base), low(base + kStreamBars), high(tab + kStreamTable), n_low(0), n_high(0) {
-        if (tab - base < kStreamBars) {   // no room for the barriers below the table
-            bars = high;
-            low = base;
-            high += kStreamBars;
-        }
-        n_low = static_cast<int>((tab - low) / ring);
-        n_high = static_cast<int>((base + kStreamSmem - high) / ring);
-    }
-    __host__ __device__ constexpr uint32_t ring_of(int warp, int ring) const { return warp < n_low ? low + warp * ring : high + (warp - n_low) * ring; }
-};
-// It starts behind what the system reserves (1 KB) and the kernel's static arrays (under 5 KB); the launch checks that it does.
-constexpr uint32_t kStreamFirstBase = 1024, kStreamLastBase = 6144;
-__host__ __device__ constexpr bool stream_rings_fit(int ring) {
-    for (uint32_t base = kStreamFirstBase; base <= kStreamLastBase; base += 16)
-        if (StreamPlaces(base, ring).n_low + StreamPlaces(base, ring).n_high < kStreamWarps) return false;
-    return true;
-}
+// Dynamic shared memory: tables, then one ring per warp.
+__host__ __device__ constexpr int stream_smem(int tables, int ring) { return tables * kStreamTable + kStreamWarps * ring; }
+constexpr int kStreamStaticMost = 6144;      // the kernel's static arrays are smaller
 
 struct StreamParams {
     DecodeParams d;
@@ -67,21 +54,32 @@ struct Shares {
     }
 };
 
+// A value that all lanes of the warp have, as one that the compiler knows to be: it then keeps it in a uniform register and
+// branches on it without preparing for lanes that part.
+__device__ __forceinline__ int uniform(int x) { return __shfl_sync(0xffffffffu, x, 0); }
+
 __device__ __forceinline__ int pages_of(const DecodeParams& p, int len) {
     return min(pages_of_length(len), p.max_pages);
 }
 
-// Byte k of w as the second byte of a table address: entry stride 256, so the address is one byte permute.
+// Address of the table entry that byte k of w names: a dot product with one weight of 128, the size of an entry.  It runs on the
+// multiply-add pipe; the logic pipe, which a byte permute or a shift and a mask would take, is the busier one.
+template <int K>
+__device__ __forceinline__ uint32_t entry_of(uint32_t w, uint32_t base) {
+    uint32_t a;
+    asm("dp4a.u32.u32 %0, %1, %2, %3;" : "=r"(a) : "r"(w), "r"(0x80u << (8 * K)), "r"(base));
+    return a;
+}
 template <int K>
 __device__ __forceinline__ uint32_t table_pair(uint32_t w, uint32_t base) {
     uint32_t v;
-    asm("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(prmt(w, base, 0x7604u | (K << 4))));
+    asm("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(entry_of<K>(w, base)));
     return v;
 }
 template <int K>
 __device__ __forceinline__ uint2 table_quad(uint32_t w, uint32_t base) {
     uint2 v;
-    asm("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(prmt(w, base, 0x7604u | (K << 4))));
+    asm("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(entry_of<K>(w, base)));
     return v;
 }
 
@@ -142,31 +140,22 @@ __device__ __forceinline__ void fill_stream_table(uint32_t smem_addr, float cent
 #pragma unroll
     for (int i = 0; i < 256 / (4 * kStreamWarps); ++i) {   // eight lanes an entry
         const int b = 4 * (i * kStreamWarps + warp) + (lane >> 3);
-        store_entry(smem_addr + b * 256 + 16 * (lane & 7), pair_entry<BITS>(cv, b));
+        store_entry(smem_addr + b * 128 + 16 * (lane & 7), pair_entry<BITS>(cv, b));
     }
 }
 
-__device__ __forceinline__ bool wait_bounded(uint32_t bar, uint32_t parity) {
-    for (int i = 0; i < (1 << 22); ++i) {
-        uint32_t ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok)
-            : "r"(bar), "r"(parity)
-            : "memory");
-        if (ok) return true;
-    }
-    return false;
+// Bytes [FROM, TO) of a page to shared memory, 16 bytes a lane and instruction; all lanes of the warp call it with the same page.
+template <int FROM, int TO>
+__device__ __forceinline__ void copy_in(uint32_t dst, const uint8_t* page, int lane) {
+    static_assert(FROM % 16 == 0 && TO % 16 == 0);
+#pragma unroll
+    for (int at = FROM; at < TO; at += 512)
+        if (at + 512 <= TO || at + 16 * lane < TO)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + at + 16 * lane), "l"(page + at + 16 * lane) : "memory");
 }
-
-__device__ __forceinline__ void copy_in(uint32_t dst, const uint8_t* src, uint32_t bytes, uint32_t bar) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src),
-                 "r"(bytes), "r"(bar)
-                 : "memory");
-}
+__device__ __forceinline__ void copies_end() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int PENDING>
+__device__ __forceinline__ void wait_copies() { asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory"); }
 
 // 16 consecutive values of a row to fp16 / bf16.
 __device__ __forceinline__ void store_row16(void* out, int64_t off, int io_dtype, const float (&x)[16]) {
@@ -218,14 +207,88 @@ __device__ __forceinline__ void fill_sign_table(uint32_t smem_addr, int warp, in
     auto signs = [](int pair) { return 0xBC00BC00u ^ ((pair & 1) ? 0x8000u : 0u) ^ ((pair & 2) ? 0x80000000u : 0u); };
     for (int b0 = 4 * warp; b0 < 256; b0 += 4 * kStreamWarps) {
         const int b = b0 + (lane >> 3);
-        store_entry(smem_addr + b * 256 + 16 * (lane & 7), make_uint4(signs(b), signs(b >> 4), signs(b >> 2), signs(b >> 6)));
+        store_entry(smem_addr + b * 128 + 16 * (lane & 7), make_uint4(signs(b), signs(b >> 4), signs(b >> 2), signs(b >> 6)));
     }
 }
 template <int K>
 __device__ __forceinline__ uint4 table_signs(uint32_t w, uint32_t base) {
     uint4 v;
-    asm("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(prmt(w, base, 0x7604u | (K << 4))));
+    asm("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(entry_of<K>(w, base)));
     return v;
+}
+// The same as bytes, for integer products: four of token A, four of token B, 16 copies.
+__device__ __forceinline__ void fill_sign_bytes(uint32_t smem_addr, int warp, int lane) {
+    auto signs = [](int nibble) {   // 0xff for a clear bit, 0x01 for a set one
+        return 0xffffffffu ^ ((nibble & 1) * 0xfeu) ^ ((nibble & 2) * 0x7f00u) ^ ((nibble & 4) * 0x3f8000u) ^ ((nibble & 8) * 0x1fc00000u);
+    };
+    for (int b0 = 4 * warp; b0 < 256; b0 += 4 * kStreamWarps) {
+        const int b = b0 + (lane >> 3);
+        store_entry(smem_addr + b * 128 + 16 * (lane & 7), make_uint4(signs(b), signs(b >> 4), signs(b), signs(b >> 4)));
+    }
+}
+
+// ---- scores of 3-bit keys in integers --------------------------------------------------------------------
+// Query and codebook are taken to 16 bits (full scale 32512) and written as two signed digits, v = 256 hi + lo.  Four indices in
+// the nibbles of a half word are then the selector of one byte permute that returns the digits of four dims, four of these are the
+// A operand (16 tokens x 32 dims) of an m16n8k32 product, and the digits of the 8 query heads are its B operand.  hi hi, hi lo
+// and lo hi are summed, exactly; lo lo (2^-16 of full scale) is left out.
+// Against half-precision products of looked-up pairs: 75 instead of 121 shared-memory wavefronts a page and about as many issue
+// slots, so no faster where K, V and signs share tables (turbo3 64 x 8192: 150.1 against 149.4 us), but it needs no K table (other
+// calls gain 5 to 7 %) and is closer to 64 bits: the centroids keep 16 bits instead of fp16's 11 (2-norm, turbo3 64 x 8192:
+// 4.7e-4 -> 2.9e-4).  For 2-bit keys, where one look-up serves four dims, it is slower (mixed batch of 256: 401 against 393 us), and
+// 16 centroids do not fit a byte permute.
+constexpr float kDigitScale = 32512.f;          // 127 * 256: the high digit of +-full scale is +-127
+constexpr float kDigitMagic = 12582912.f + 128.f;   // 1.5 * 2^23: the integer lands in the low bits; + 128: its low digit is signed
+
+__device__ __forceinline__ float max_nan(float a, float b) {   // NaN if either is
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ uint32_t to_digits(float x, float scale) { return __float_as_uint(fmaf(x, scale, kDigitMagic)); }
+// High and low digits of four numbers, one per byte.
+__device__ __forceinline__ void pack_digits(uint32_t a, uint32_t b, uint32_t c, uint32_t d, uint32_t& hi, uint32_t& lo) {
+    const uint32_t ab = prmt(a, b, 0x5140u), cd = prmt(c, d, 0x5140u);
+    hi = prmt(ab, cd, 0x7632u);
+    lo = prmt(ab, cd, 0x5410u) ^ 0x80808080u;
+}
+// Digits of a codebook, of which lane l holds entry l mod 8: entry i is byte i of (x[0], x[1]).
+__device__ __forceinline__ void codebook_digits(float c, float scale, uint32_t (&hi)[2], uint32_t (&lo)[2]) {
+    const uint32_t u = to_digits(c, scale);
+    uint32_t v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = __shfl_sync(0xffffffffu, u, i);
+    pack_digits(v[0], v[1], v[2], v[3], hi[0], lo[0]);
+    pack_digits(v[4], v[5], v[6], v[7], hi[1], lo[1]);
+}
+
+__device__ __forceinline__ void mma_s8_16832(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// Selector words of a token's quarter: half h of word j holds the indices of the four dims of chunk 2 j + h, one per nibble.  A
+// selector's top bit would ask the permute for a sign: it has to be clear.
+template <int NW>
+__device__ __forceinline__ void selector_words(const uint32_t (&w)[NW], uint32_t (&m)[4]) {
+#pragma unroll
+    for (int j = 0; j < 3; ++j) m[j] = w[j] & 0x77777777u;
+    m[3] = ((w[0] >> 3) & 0x11111111u) | ((w[1] >> 2) & 0x22222222u) | ((w[2] >> 1) & 0x44444444u);
+}
+
+// Query row (head gid, quarter tig: 32 dims) as B operands: high digits of chunk c (dims 4 c .. 4 c + 3) in f[c], low ones in f[8 + c].
+__device__ __forceinline__ void query_digits(const float (&x)[32], float scale, uint32_t (&f)[16]) {
+#pragma unroll
+    for (int c = 0; c < 8; ++c)
+        pack_digits(to_digits(x[4 * c], scale), to_digits(x[4 * c + 1], scale), to_digits(x[4 * c + 2], scale), to_digits(x[4 * c + 3], scale), f[c], f[8 + c]);
+}
+// Largest magnitude of a row spread over the four lanes of a group, NaN if there is one.
+__device__ __forceinline__ float row_max(const float (&x)[32]) {
+    float m = 0.f;
+#pragma unroll
+    for (int i = 0; i < 32; i += 2) asm("max.NaN.abs.f32 %0, %0, %1, %2;" : "+f"(m) : "f"(x[i]), "f"(x[i + 1]));
+    m = max_nan(m, __shfl_xor_sync(0xffffffffu, m, 1));
+    return max_nan(m, __shfl_xor_sync(0xffffffffu, m, 2));
 }
 
 // Output row g of an item.
@@ -234,9 +297,9 @@ __device__ __forceinline__ void finish_row(const DecodeParams& p, int seq, int h
     if (g < p.G - qg * 8) write_row(p, static_cast<int64_t>(seq) * p.Hq + kvh * p.G + qg * 8 + g, lane, x, l);
 }
 
-// SIGN_TABLE: K and V share a codebook and S = I, so the V half of the table has room for the signs, and the query
-// operands of the index term serve the sign term as well.
-template <int KB, int VB, bool QJL, bool SPARSE, bool SIGN_TABLE>
+// ONE_QUERY: the query operands of the index term serve the sign term as well (S = I).  With 2- and 4-bit keys K and V share a
+// codebook then, so that there is room for the table of signs; without, their sign operands are made by logic.
+template <int KB, int VB, bool QJL, bool SPARSE, bool ONE_QUERY>
 __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const StreamParams sp) {
     constexpr int NWK = KB + (QJL ? 1 : 0);
     constexpr int RK = 16 * NWK;
@@ -247,7 +310,10 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
     constexpr int PAGE = KPART + 256 * VB + 32;
     constexpr int NSTAGE = kStreamStages;
     constexpr int RING = NSTAGE * PAGE;
-    static_assert(stream_rings_fit(RING), "the rings of all warps fit around the table, wherever the dynamic part may start");
+    constexpr bool INTEGER = KB == 3;                       // scores from integer products, else half-precision products of look-ups
+    constexpr bool SIGNS = QJL && (INTEGER || ONE_QUERY);   // table of signs
+    constexpr int TABLES = INTEGER && !QJL ? 1 : 2;         // INTEGER: V, signs; else K and V in one and signs, or K and V
+    static_assert(stream_smem(TABLES, RING) + kStreamStaticMost + 1024 <= 227 * 1024, "what an SM gives one CTA");
     const DecodeParams& p = sp.d;
 
     extern __shared__ __align__(128) uint8_t smem[];
@@ -256,22 +322,18 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
     __shared__ int sm_wsum[kStreamWarps];
     __shared__ int4 sm_part[2 * kStreamWarps];   // partials: (item or -1, sequence, pages of the item after this share, flags)
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
     const int gid = lane >> 2, tig = lane & 3;
 
-    // ---- shared memory: the table on a 64 KB boundary (its addresses are built by a byte permute), barriers and the
-    // rings of as many warps as fit below it, the other rings above it
-    const StreamPlaces places(smem_u32(smem), RING);
-    const uint32_t tab = places.tab, ring = places.ring_of(warp, RING);
-    const uint32_t bar = places.bars + warp * 2 * NSTAGE * 8;     // [0 .. NSTAGE) page (or K part), [NSTAGE ..) late V part
+    const uint32_t ktab = smem_u32(smem), vtab = ktab + (INTEGER || ONE_QUERY ? 0 : kStreamTable), stab = ktab + kStreamTable;
+    const uint32_t rings = ktab + TABLES * kStreamTable, ring = rings + warp * RING;
 
-    if constexpr (SIGN_TABLE) fill_sign_table(tab + 128, warp, lane);   // constants
+    if constexpr (SIGNS && INTEGER) fill_sign_bytes(stab, warp, lane);   // constants
+    else if constexpr (SIGNS) fill_sign_table(stab, warp, lane);
     if (lane < 2) sm_part[2 * warp + lane] = make_int4(-1, 0, 0, 0);
-    if (lane < 2 * NSTAGE) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar + lane * 8) : "memory");
-    fence_barrier_init();
     pdl_wait();
     pdl_release();
-    const float ck = lane_centroid<KB>(p.kc, lane), cv = SIGN_TABLE ? 0.f : lane_centroid<VB>(p.vc, lane);
+    const float ck = lane_centroid<KB>(p.kc, lane), cv = !INTEGER && ONE_QUERY ? 0.f : lane_centroid<VB>(p.vc, lane);
 
     // ---- pages before each thread's run of sequences (every CTA does the same scan over all lengths)
     const int per = (sp.ns + kStreamThreads - 1) / kStreamThreads;
@@ -302,7 +364,8 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
     {
         const Shares shares(static_cast<uint32_t>(sm_scan[kStreamThreads]) * sp.HG, sp.n_warps);   // at most 2^31 pages
         first = shares.start(gw);
-        n = static_cast<int>(shares.start(gw + 1) - first);
+        first = uniform(first);
+        n = uniform(static_cast<int>(shares.start(gw + 1) - first));
     }
 
     // ---- the item and page this warp starts in
@@ -324,6 +387,11 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
         const int r = static_cast<int>(first - at);
         hg = r / np;
         page = r - hg * np;
+        seq = uniform(seq);
+        len = uniform(len);
+        np = uniform(np);
+        hg = uniform(hg);
+        page = uniform(page);
     }
     auto kv_head = [&](int h) { return p.ngroups == 1 ? h : h / p.ngroups; };
 
@@ -361,8 +429,12 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
     };
     uint32_t src = next_window();
     uint32_t src_next = src;
-    const int first_lot = min(n, NSTAGE);
-    if (lane < first_lot) copy_in(ring + lane * PAGE, page_at(src), PAGE, bar + lane * 8);
+#pragma unroll
+    for (int i = 0; i < NSTAGE; ++i) {
+        const uint32_t at = __shfl_sync(0xffffffffu, src, i);
+        if (i < n) copy_in<0, PAGE>(ring + i * PAGE, page_at(at), lane);
+        copies_end();
+    }
     if (n > 32) src_next = next_window();
     // Flags of lengths that are cut and zeros of empty sequences, behind the first pages' copies: sequence s belongs to warp
     // s / gridDim of CTA s % gridDim (one thread a sequence in CTA 0 took 1.8 ms for 1008 empty sequences of 128 heads).
@@ -375,51 +447,84 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
         }
     }
     // the codebooks' part of the table is filled behind the first pages' copies
-    fill_stream_table<KB>(tab, ck, warp, lane);
-    if constexpr (!SIGN_TABLE) fill_stream_table<VB>(tab + 128, cv, warp, lane);
+    if constexpr (!INTEGER) fill_stream_table<KB>(ktab, ck, warp, lane);
+    if constexpr (INTEGER || !ONE_QUERY) fill_stream_table<VB>(vtab, cv, warp, lane);
     __syncthreads();
 
-    const uint32_t klut = tab + (KB == 2 ? 8 * (lane & 15) : 4 * lane);
-    const uint32_t vlut = tab + (SIGN_TABLE ? 0 : 128) + (VB == 2 ? 8 * (lane & 15) : 4 * lane);
-    const uint32_t slut = tab + 128 + 16 * (lane & 7);
+    const uint32_t klut = ktab + (KB == 2 ? 8 * (lane & 15) : 4 * lane);
+    const uint32_t vlut = vtab + (VB == 2 ? 8 * (lane & 15) : 4 * lane);
+    const uint32_t slut = stab + (INTEGER ? 8 * (lane & 15) : 16 * (lane & 7));
     const uint32_t ring_k = ring + lane * (NWK * 4);
     const uint32_t ring_n = ring + gid * 4;
     const uint32_t ring_v = ring + (tig * 8 + gid) * 4;
 
-    const float qpscale = SIGN_TABLE ? p.qpscale * (1.f / 16.f) : p.qpscale;   // the one-sided forms carry 1/16 in the query
-    bool timed_out = false;
-    uint32_t stage = 0, parity = 0;           // ring stage of the current page and the phase of its barrier
-    uint32_t v_parity = 0;                    // Sparse-V: bit s = phase of the late-V barrier of stage s
+    const float qpscale = ONE_QUERY ? p.qpscale * (1.f / 16.f) : p.qpscale;   // the one-sided forms carry 1/16 in the query
+    uint32_t chi[2], clo[2];                  // digits of the K codebook
+    float cmax = 0.f;
+    if constexpr (INTEGER) {
+        cmax = fabsf(ck);
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) cmax = max_nan(cmax, __shfl_xor_sync(0xffffffffu, cmax, o));
+        if (cmax < 1e-20f) cmax = 1e-20f;
+        codebook_digits(ck, kDigitScale / cmax, chi, clo);
+    }
+    uint32_t stage = 0;                       // ring stage of the current page
     uint32_t k_only = 0;                      // Sparse-V: bit s = the page in stage s came without its V part
     uint32_t v_skipped = 0;
     int idx = 0;                              // pages of the share that are done
 
-    while (idx < n && !timed_out) {
+    while (idx < n) {
         const int seg = min(np - page, n - idx);           // pages of this item in the share
         const int kvh = kv_head(hg), qg = hg - kvh * p.ngroups;
         const int head0 = kvh * p.G + qg * 8, nq = min(8, p.G - qg * 8);
         const int64_t row = (static_cast<int64_t>(seq) * p.Hq + head0 + gid) * kHeadDim;
 
-        uint32_t qf[16], qpf[QJL && !SIGN_TABLE ? 16 : 1];
+        // INTEGER: qf[c], qf[8 + c] are the high and low digits of chunk c, qpf those of the sign term's query if it has one of its
+        // own.  A score in the log2 domain is unit * (k norm * (index sum) + residual norm * sign_unit * (sign sum)).
+        uint32_t qf[16], qpf[QJL && !ONE_QUERY ? 16 : 1];
         float sq_init0 = 0.f, sq_init1 = 0.f;   // minus the query sums of the one-sided sign forms
+        float unit0 = 1.f, unit1 = 1.f, sign_unit0 = 0.f, sign_unit1 = 0.f;   // of queries 2 tig, 2 tig + 1
         {
             float xq[32];
             load_q32(p.q, row, tig, p.io_dtype, gid < nq, xq);
             if (p.rotate_q) rotate_q32(xq, lane, p.io_dtype);
-            q_frag_from(xq, qf);
-            if constexpr (QJL && !SIGN_TABLE) {
-                if (p.qp) load_q32(p.qp, row, tig, p.io_dtype, gid < nq, xq);
-                float corr;
-                qp_frag_signed_from(xq, qpf, corr);
-                corr += __shfl_xor_sync(0xffffffffu, corr, 1);
-                corr += __shfl_xor_sync(0xffffffffu, corr, 2);
-                sq_init0 = -__shfl_sync(0xffffffffu, corr, 8 * tig);
-                sq_init1 = -__shfl_sync(0xffffffffu, corr, 8 * tig + 4);
+            if constexpr (INTEGER) {
+                auto take = [&](uint32_t (&f)[16]) {   // the row's digits; returns what a step of them stands for, NaN for a row with NaN or infinity
+                    float most = row_max(xq);
+                    if (most < 1e-30f) most = 1e-30f;
+                    query_digits(xq, kDigitScale / most, f);
+                    return most < INFINITY ? most * (1.f / kDigitScale) : NAN;
+                };
+                const float step = take(qf);
+                float unit = p.qscale * step * (cmax * (256.f / kDigitScale)), sign_unit = 0.f;
+                if constexpr (QJL) {
+                    sign_unit = step;
+                    if constexpr (!ONE_QUERY) {
+                        if (p.qp) load_q32(p.qp, row, tig, p.io_dtype, gid < nq, xq);
+                        sign_unit = take(qpf);
+                    }
+                    sign_unit *= p.qpscale * (1.f / 16.f);
+                }
+                unit0 = __shfl_sync(0xffffffffu, unit, 8 * tig);
+                unit1 = __shfl_sync(0xffffffffu, unit, 8 * tig + 4);
+                sign_unit0 = __shfl_sync(0xffffffffu, sign_unit, 8 * tig);
+                sign_unit1 = __shfl_sync(0xffffffffu, sign_unit, 8 * tig + 4);
+            } else {
+                q_frag_from(xq, qf);
+                if constexpr (QJL && !ONE_QUERY) {
+                    if (p.qp) load_q32(p.qp, row, tig, p.io_dtype, gid < nq, xq);
+                    float corr;
+                    qp_frag_signed_from(xq, qpf, corr);
+                    corr += __shfl_xor_sync(0xffffffffu, corr, 1);
+                    corr += __shfl_xor_sync(0xffffffffu, corr, 2);
+                    sq_init0 = -__shfl_sync(0xffffffffu, corr, 8 * tig);
+                    sq_init1 = -__shfl_sync(0xffffffffu, corr, 8 * tig + 4);
+                }
             }
         }
         // Sparse-V: columns past the group's heads hold zero queries, whose scores are all alike; they decide nothing
         const float thresh0 = 2 * tig < nq ? sp.weight_thresh : INFINITY, thresh1 = 2 * tig + 1 < nq ? sp.weight_thresh : INFINITY;
-        float m0 = -INFINITY, m1 = -INFINITY;   // softmax reference of queries 2 tig, 2 tig + 1 (log2 domain)
+        float r0 = INFINITY, r1 = INFINITY;     // minus the softmax reference of queries 2 tig, 2 tig + 1 (log2 domain)
         float l0 = 0.f, l1 = 0.f;
         float oacc[8][4];
 #pragma unroll
@@ -427,105 +532,138 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
 #pragma unroll
             for (int r = 0; r < 4; ++r) oacc[i][r] = 0.f;
 
-        auto one_page = [&](auto have_v, int j) {
-            constexpr bool HAVE_V = decltype(have_v)::value;
+        auto one_page = [&](auto have_v, auto partly, int j) {
+            constexpr bool HAVE_V = decltype(have_v)::value, PARTLY = decltype(partly)::value;
             const uint32_t so = stage * PAGE;
-            if (!wait_bounded(bar + stage * 8, parity)) {
-                timed_out = true;
-                return;
-            }
+            wait_copies<NSTAGE - 1>();
+            __syncwarp();
             // ---- scores of 16 tokens x 8 queries
             uint32_t wa[NWK], wb[NWK];
             lds_words<NWK, 0>(ring_k + so, wa);
             lds_words<NWK, 32 * NWK * 4>(ring_k + so, wb);
-            float sm[4] = {0.f, 0.f, 0.f, 0.f};
-            float sq[4] = {sq_init0, sq_init1, sq_init0, sq_init1}, sq2[4] = {0.f, 0.f, 0.f, 0.f};
             uint32_t sgn0 = 0, sgn1 = 0;   // bytes: the nibbles 2 k (sgn0), 2 k + 1 (sgn1) of token A, then of token B
-            if constexpr (QJL && SIGN_TABLE) {
+            if constexpr (SIGNS) {
                 sgn0 = bit_select(wb[KB] << 4, wa[KB], 0x0f0f0f0fu);
                 sgn1 = bit_select(wb[KB], wa[KB] >> 4, 0x0f0f0f0fu);
             }
-            auto sign_term = [&](auto quarter) {   // eight dims of two tokens, two products
-                constexpr int B = decltype(quarter)::value;
-                if constexpr (QJL && SIGN_TABLE) {
-                    const uint4 g0 = table_signs<B>(sgn0, slut), g1 = table_signs<B>(sgn1, slut);
-                    mma_f16_16816(sq, g0.x, g0.y, g0.z, g0.w, qf[4 * B], qf[4 * B + 1]);
-                    mma_f16_16816(sq2, g1.x, g1.y, g1.z, g1.w, qf[4 * B + 2], qf[4 * B + 3]);
-                } else if constexpr (QJL) {
-                    const uint32_t xa = wa[KB] << (4 * B), xb = wb[KB] << (4 * B);
-                    mma_f16_16816(sq, and_or(xa, 0x80008000u, 0x3C003C00u), and_or(xb, 0x80008000u, 0x3C003C00u),
-                                  and_bits(xa, 0x40004000u), and_bits(xb, 0x40004000u), qpf[4 * B], qpf[4 * B + 1]);
-                    mma_f16_16816(sq2, and_bits(xa, 0x20002000u), and_bits(xb, 0x20002000u), and_bits(xa, 0x10001000u),
-                                  and_bits(xb, 0x10001000u), qpf[4 * B + 2], qpf[4 * B + 3]);
-                }
-            };
-            if constexpr (KB == 2) {
-                // An entry holds two half2.  Its byte is made of the pair of indices of token A and that of token B, so that
-                // the two are neighbouring registers of the A operand.
-                auto quads = [&](auto word) {
-                    constexpr int J = decltype(word)::value;
-                    const uint32_t y0 = bit_select(wb[J] << 2, wa[J], 0x33333333u), y1 = bit_select(wb[J], wa[J] >> 2, 0x33333333u);
-                    {
-                        const uint2 a = table_quad<0>(y0, klut), b = table_quad<1>(y0, klut);
-                        mma_f16_16816(sm, a.x, a.y, b.x, b.y, qf[8 * J], qf[8 * J + 1]);
-                    }
-                    {
-                        const uint2 a = table_quad<0>(y1, klut), b = table_quad<1>(y1, klut);
-                        mma_f16_16816(sm, a.x, a.y, b.x, b.y, qf[8 * J + 4], qf[8 * J + 5]);
-                    }
-                    sign_term(std::integral_constant<int, 2 * J>{});
-                    {
-                        const uint2 a = table_quad<2>(y0, klut), b = table_quad<3>(y0, klut);
-                        mma_f16_16816(sm, a.x, a.y, b.x, b.y, qf[8 * J + 2], qf[8 * J + 3]);
-                    }
-                    {
-                        const uint2 a = table_quad<2>(y1, klut), b = table_quad<3>(y1, klut);
-                        mma_f16_16816(sm, a.x, a.y, b.x, b.y, qf[8 * J + 6], qf[8 * J + 7]);
-                    }
-                    sign_term(std::integral_constant<int, 2 * J + 1>{});
-                };
-                quads(std::integral_constant<int, 0>{});
-                quads(std::integral_constant<int, 1>{});
-            } else {
-                uint32_t mwa[4], mwb[4];
-                table_words<KB>(wa, mwa);
-                table_words<KB>(wb, mwb);
+            float2 kn = unpack_half2(lds_u32<KN_OFF>(ring_n + so)), krn = make_float2(0.f, 0.f);
+            if constexpr (QJL) krn = unpack_half2(lds_u32<KRN_OFF>(ring_n + so));
+            float s0, s1, s2, s3;   // tokens gid (s0, s1), gid + 8, queries 2 tig (s0, s2), 2 tig + 1
+            if constexpr (INTEGER) {
+                uint32_t ma[4], mb[4];
+                selector_words(wa, ma);
+                selector_words(wb, mb);
+                int hh[4] = {0, 0, 0, 0}, mid[4] = {0, 0, 0, 0}, nh[4] = {0, 0, 0, 0}, nl[4] = {0, 0, 0, 0};
+                auto look = [&](const uint32_t (&t)[2], uint32_t m) { return prmt(t[0], t[1], m); };
                 auto eight_dims = [&](auto word) {
-                    constexpr int C = decltype(word)::value;
-                    const uint32_t a0 = table_pair<0>(mwa[C], klut), a1 = table_pair<1>(mwa[C], klut);
-                    const uint32_t b0 = table_pair<0>(mwb[C], klut), b1 = table_pair<1>(mwb[C], klut);
-                    mma_f16_16816(sm, a0, b0, a1, b1, qf[4 * C], qf[4 * C + 1]);
-                    const uint32_t a2 = table_pair<2>(mwa[C], klut), a3 = table_pair<3>(mwa[C], klut);
-                    const uint32_t b2 = table_pair<2>(mwb[C], klut), b3 = table_pair<3>(mwb[C], klut);
-                    mma_f16_16816(sm, a2, b2, a3, b3, qf[4 * C + 2], qf[4 * C + 3]);
-                    sign_term(word);
+                    constexpr int J = decltype(word)::value;
+                    const uint32_t ua = ma[J] >> 16, ub = mb[J] >> 16;
+                    const uint32_t h0 = look(chi, ma[J]), h1 = look(chi, mb[J]), h2 = look(chi, ua), h3 = look(chi, ub);
+                    mma_s8_16832(hh, h0, h1, h2, h3, qf[2 * J], qf[2 * J + 1]);
+                    mma_s8_16832(mid, h0, h1, h2, h3, qf[8 + 2 * J], qf[8 + 2 * J + 1]);
+                    mma_s8_16832(mid, look(clo, ma[J]), look(clo, mb[J]), look(clo, ua), look(clo, ub), qf[2 * J], qf[2 * J + 1]);
+                    if constexpr (QJL) {
+                        const uint2 g0 = table_quad<J>(sgn0, slut), g1 = table_quad<J>(sgn1, slut);
+                        const uint32_t* f = qf;
+                        if constexpr (!ONE_QUERY) f = qpf;
+                        mma_s8_16832(nh, g0.x, g0.y, g1.x, g1.y, f[2 * J], f[2 * J + 1]);
+                        mma_s8_16832(nl, g0.x, g0.y, g1.x, g1.y, f[8 + 2 * J], f[8 + 2 * J + 1]);
+                    }
                 };
                 eight_dims(std::integral_constant<int, 0>{});
                 eight_dims(std::integral_constant<int, 1>{});
                 eight_dims(std::integral_constant<int, 2>{});
                 eight_dims(std::integral_constant<int, 3>{});
-            }
-            float2 kn = unpack_half2(lds_u32<KN_OFF>(ring_n + so));
-            kn.x *= p.qscale;
-            kn.y *= p.qscale;
-            float s0 = sm[0] * kn.x, s1 = sm[1] * kn.x, s2 = sm[2] * kn.y, s3 = sm[3] * kn.y;
-            if constexpr (QJL) {
-                float2 krn = unpack_half2(lds_u32<KRN_OFF>(ring_n + so));
-                krn.x *= qpscale;
-                krn.y *= qpscale;
-                s0 = fmaf(sq[0] + sq2[0], krn.x, s0);
-                s1 = fmaf(sq[1] + sq2[1], krn.x, s1);
-                s2 = fmaf(sq[2] + sq2[2], krn.y, s2);
-                s3 = fmaf(sq[3] + sq2[3], krn.y, s3);
+                auto sum = [](int hi, int lo) { return static_cast<float>(hi * 256 + lo); };
+                s0 = unit0 * sum(hh[0], mid[0]) * kn.x;
+                s1 = unit1 * sum(hh[1], mid[1]) * kn.x;
+                s2 = unit0 * sum(hh[2], mid[2]) * kn.y;
+                s3 = unit1 * sum(hh[3], mid[3]) * kn.y;
+                if constexpr (QJL) {
+                    s0 = fmaf(sign_unit0 * sum(nh[0], nl[0]), krn.x, s0);
+                    s1 = fmaf(sign_unit1 * sum(nh[1], nl[1]), krn.x, s1);
+                    s2 = fmaf(sign_unit0 * sum(nh[2], nl[2]), krn.y, s2);
+                    s3 = fmaf(sign_unit1 * sum(nh[3], nl[3]), krn.y, s3);
+                }
+            } else {
+                float sm[4] = {0.f, 0.f, 0.f, 0.f};
+                float sq[4] = {sq_init0, sq_init1, sq_init0, sq_init1}, sq2[4] = {0.f, 0.f, 0.f, 0.f};
+                auto sign_term = [&](auto quarter) {   // eight dims of two tokens, two products
+                    constexpr int C = decltype(quarter)::value;
+                    if constexpr (SIGNS) {
+                        const uint4 g0 = table_signs<C>(sgn0, slut), g1 = table_signs<C>(sgn1, slut);
+                        mma_f16_16816(sq, g0.x, g0.y, g0.z, g0.w, qf[4 * C], qf[4 * C + 1]);
+                        mma_f16_16816(sq2, g1.x, g1.y, g1.z, g1.w, qf[4 * C + 2], qf[4 * C + 3]);
+                    } else if constexpr (QJL) {
+                        const uint32_t xa = wa[KB] << (4 * C), xb = wb[KB] << (4 * C);
+                        mma_f16_16816(sq, and_or(xa, 0x80008000u, 0x3C003C00u), and_or(xb, 0x80008000u, 0x3C003C00u),
+                                      and_bits(xa, 0x40004000u), and_bits(xb, 0x40004000u), qpf[4 * C], qpf[4 * C + 1]);
+                        mma_f16_16816(sq2, and_bits(xa, 0x20002000u), and_bits(xb, 0x20002000u), and_bits(xa, 0x10001000u),
+                                      and_bits(xb, 0x10001000u), qpf[4 * C + 2], qpf[4 * C + 3]);
+                    }
+                };
+                if constexpr (KB == 2) {
+                    // An entry holds two half2.  Its byte is made of the pair of indices of token A and that of token B, so that
+                    // the two are neighbouring registers of the A operand.
+                    auto quads = [&](auto word) {
+                        constexpr int J = decltype(word)::value;
+                        const uint32_t y0 = bit_select(wb[J] << 2, wa[J], 0x33333333u), y1 = bit_select(wb[J], wa[J] >> 2, 0x33333333u);
+                        auto product = [&](auto first, uint32_t y, int c) {
+                            constexpr int B = decltype(first)::value;
+                            const uint2 a = table_quad<B>(y, klut), b = table_quad<B + 1>(y, klut);
+                            mma_f16_16816(sm, a.x, a.y, b.x, b.y, qf[8 * J + c], qf[8 * J + c + 1]);
+                        };
+                        product(std::integral_constant<int, 0>{}, y0, 0);
+                        product(std::integral_constant<int, 0>{}, y1, 4);
+                        sign_term(std::integral_constant<int, 2 * J>{});
+                        product(std::integral_constant<int, 2>{}, y0, 2);
+                        product(std::integral_constant<int, 2>{}, y1, 6);
+                        sign_term(std::integral_constant<int, 2 * J + 1>{});
+                    };
+                    quads(std::integral_constant<int, 0>{});
+                    quads(std::integral_constant<int, 1>{});
+                } else {
+                    uint32_t mwa[4], mwb[4];
+                    table_words<KB>(wa, mwa);
+                    table_words<KB>(wb, mwb);
+                    auto eight_dims = [&](auto word) {
+                        constexpr int C = decltype(word)::value;
+                        const uint32_t a0 = table_pair<0>(mwa[C], klut), a1 = table_pair<1>(mwa[C], klut);
+                        const uint32_t b0 = table_pair<0>(mwb[C], klut), b1 = table_pair<1>(mwb[C], klut);
+                        mma_f16_16816(sm, a0, b0, a1, b1, qf[4 * C], qf[4 * C + 1]);
+                        const uint32_t a2 = table_pair<2>(mwa[C], klut), a3 = table_pair<3>(mwa[C], klut);
+                        const uint32_t b2 = table_pair<2>(mwb[C], klut), b3 = table_pair<3>(mwb[C], klut);
+                        mma_f16_16816(sm, a2, b2, a3, b3, qf[4 * C + 2], qf[4 * C + 3]);
+                        sign_term(word);
+                    };
+                    eight_dims(std::integral_constant<int, 0>{});
+                    eight_dims(std::integral_constant<int, 1>{});
+                    eight_dims(std::integral_constant<int, 2>{});
+                    eight_dims(std::integral_constant<int, 3>{});
+                }
+                kn.x *= p.qscale;
+                kn.y *= p.qscale;
+                s0 = sm[0] * kn.x;
+                s1 = sm[1] * kn.x;
+                s2 = sm[2] * kn.y;
+                s3 = sm[3] * kn.y;
+                if constexpr (QJL) {
+                    krn.x *= qpscale;
+                    krn.y *= qpscale;
+                    s0 = fmaf(sq[0] + sq2[0], krn.x, s0);
+                    s1 = fmaf(sq[1] + sq2[1], krn.x, s1);
+                    s2 = fmaf(sq[2] + sq2[2], krn.y, s2);
+                    s3 = fmaf(sq[3] + sq2[3], krn.y, s3);
+                }
             }
             const int valid_tokens = len - (page + j) * kPageTokens;
-            if (valid_tokens < kPageTokens) {   // only the last page of a sequence is partly filled
+            if constexpr (PARTLY) {
                 if (gid >= valid_tokens) { s0 = -INFINITY; s1 = -INFINITY; }
                 if (gid + 8 >= valid_tokens) { s2 = -INFINITY; s3 = -INFINITY; }
             }
-            // ---- online softmax.  The reference m is raised only when a score exceeds it, and then to one above the
+            // ---- online softmax.  The reference is raised only when a score exceeds it, and then to one above the
             // largest score, so weights stay <= 1 and most pages need no shuffle and no rescaling.
-            const bool over = fmaxf(s0, s2) > m0 || fmaxf(s1, s3) > m1;
+            const bool over = fmaxf(s0, s2) > -r0 || fmaxf(s1, s3) > -r1;
             if (__any_sync(0xffffffffu, over)) {
                 float mx0 = fmaxf(s0, s2), mx1 = fmaxf(s1, s3);
 #pragma unroll
@@ -533,8 +671,8 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
                     mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, o));
                     mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, o));
                 }
-                const float mn0 = mx0 > m0 ? mx0 + 1.f : m0, mn1 = mx1 > m1 ? mx1 + 1.f : m1;
-                const float al0 = ex2(m0 - mn0), al1 = ex2(m1 - mn1);
+                const float rn0 = mx0 > -r0 ? -mx0 - 1.f : r0, rn1 = mx1 > -r1 ? -mx1 - 1.f : r1;
+                const float al0 = ex2(rn0 - r0), al1 = ex2(rn1 - r1);
                 l0 *= al0;
                 l1 *= al1;
 #pragma unroll
@@ -544,10 +682,10 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
                     oacc[i][2] *= al0;
                     oacc[i][3] *= al1;
                 }
-                m0 = mn0;
-                m1 = mn1;
+                r0 = rn0;
+                r1 = rn1;
             }
-            const float p0v = ex2(s0 - m0), p1v = ex2(s1 - m1), p2v = ex2(s2 - m0), p3v = ex2(s3 - m1);
+            const float p0v = ex2(s0 + r0), p1v = ex2(s1 + r1), p2v = ex2(s2 + r0), p3v = ex2(s3 + r1);
             l0 += p0v + p2v;
             l1 += p1v + p3v;
 
@@ -558,10 +696,10 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
             bool have = true;
             if constexpr (SPARSE && !HAVE_V) {
                 if (do_v) {   // first needed page after a run of skipped ones: fetch its V part now
-                    const uint32_t vbar = bar + (NSTAGE + stage) * 8;
-                    if (lane == 0) copy_in(ring + so + KPART, page_at(locate(seq, hg, page + j)) + KPART, PAGE - KPART, vbar);
-                    if (!wait_bounded(vbar, (v_parity >> stage) & 1u)) timed_out = true;
-                    v_parity ^= 1u << stage;
+                    copy_in<KPART, PAGE>(ring + so, page_at(locate(seq, hg, page + j)), lane);
+                    copies_end();
+                    wait_copies<0>();
+                    __syncwarp();
                 } else {
                     ++v_skipped;
                     have = false;
@@ -569,7 +707,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
             }
             if (have) {
                 float2 vn = unpack_half2(lds_u32<VN_OFF>(ring_n + so));
-                if (valid_tokens < kPageTokens) {
+                if constexpr (PARTLY) {
                     if (gid >= valid_tokens) vn.x = 0.f;
                     if (gid + 8 >= valid_tokens) vn.y = 0.f;
                 }
@@ -630,30 +768,29 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
                     src = src_next;
                     if (i + 32 < n) src_next = next_window();
                 }
-                const bool whole = !SPARSE || do_v;
-                if (lane == (i & 31)) copy_in(ring + so, page_at(src), whole ? PAGE : KPART, bar + stage * 8);
+                const uint8_t* next = page_at(__shfl_sync(0xffffffffu, src, i & 31));
                 if constexpr (SPARSE) {
-                    if (whole != HAVE_V) k_only ^= 1u << stage;
+                    copy_in<0, KPART>(ring + so, next, lane);
+                    if (do_v) copy_in<KPART, PAGE>(ring + so, next, lane);
+                    if (do_v != HAVE_V) k_only ^= 1u << stage;
+                } else {
+                    copy_in<0, PAGE>(ring + so, next, lane);
                 }
             }
-            if (++stage == NSTAGE) {
-                stage = 0;
-                parity ^= 1u;
-            }
+            copies_end();
+            if (++stage == NSTAGE) stage = 0;
         };
-        auto next_page = [&](int j) {
+        auto next_page = [&](auto partly, int j) {
             if constexpr (SPARSE) {
-                if (k_only == 0 || !((k_only >> stage) & 1u)) one_page(std::true_type{}, j);
-                else one_page(std::false_type{}, j);
+                if (k_only == 0 || !((k_only >> stage) & 1u)) one_page(std::true_type{}, partly, j);
+                else one_page(std::false_type{}, partly, j);
             } else {
-                one_page(std::true_type{}, j);
+                one_page(std::true_type{}, partly, j);
             }
         };
-        for (int j = 0; j < seg && !timed_out; ++j) next_page(j);
-        if (timed_out) {   // let copies that are under way land before the CTA may end
-            for (int s = 0; s < NSTAGE; ++s) (void)wait_bounded(bar + s * 8, s < static_cast<int>(stage) ? parity ^ 1u : parity);
-            break;
-        }
+        const int full = min(seg, (len >> 4) - page);   // at most the last page of a sequence is partly filled
+        for (int j = 0; j < full; ++j) next_page(std::false_type{}, j);
+        if (full < seg) next_page(std::true_type{}, full);
 
         // ---- the item's result, or this warp's part of it
 #pragma unroll
@@ -684,12 +821,12 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
                     asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(ring + (g * kHeadDim + 16 * gid + 4 * i) * 4), "f"(x[4 * i]),
                                  "f"(x[4 * i + 1]), "f"(x[4 * i + 2]), "f"(x[4 * i + 3])
                                  : "memory");
-                if (gid == 0) asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(ring + (kStreamSlotFloats + 2 * g) * 4), "f"(k ? m1 : m0), "f"(l) : "memory");
+                if (gid == 0) asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(ring + (kStreamSlotFloats + 2 * g) * 4), "f"(k ? -r1 : -r0), "f"(l) : "memory");
             } else {
                 float4* dst = reinterpret_cast<float4*>(sp.part_o + static_cast<int64_t>(gw) * kStreamSlotFloats + g * kHeadDim + 16 * gid);
 #pragma unroll
                 for (int i = 0; i < 4; ++i) dst[i] = make_float4(x[4 * i], x[4 * i + 1], x[4 * i + 2], x[4 * i + 3]);
-                if (gid == 0) sp.part_ml[gw * 8 + g] = make_float2(k ? m1 : m0, l);
+                if (gid == 0) sp.part_ml[gw * 8 + g] = make_float2(k ? -r1 : -r0, l);
             }
         }
         if (!whole_item && lane == 0)
@@ -699,16 +836,14 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
         if (idx < n && ++hg == sp.HG) {
             hg = 0;
             do {
-                len = __ldg(p.seq_lens + ++seq);
+                len = uniform(__ldg(p.seq_lens + ++seq));
                 np = pages_of(p, len);
             } while (np == 0);
         }
     }
     if (p.status) {
-        int bits = 0;
-        if (__any_sync(0xffffffffu, bad_block)) bits |= TQ_STATUS_BAD_BLOCK;
-        if (__any_sync(0xffffffffu, timed_out)) bits |= TQ_STATUS_TIMEOUT;
-        if (bits && lane == 0) atomicOr(p.status, bits);
+        const bool bad = __any_sync(0xffffffffu, bad_block);
+        if (bad && lane == 0) atomicOr(p.status, TQ_STATUS_BAD_BLOCK);
     }
     if constexpr (SPARSE) {
         if (p.skip_stats && lane == 0) {
@@ -742,7 +877,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
         }
         if ((run & 1) != (warp >> 3)) continue;
         const int g = warp & 7;
-        auto ring_of = [&](int w) { return StreamPlaces(smem_u32(smem), RING).ring_of(w, RING); };
+        auto ring_of = [&](int w) { return smem_u32(smem) + TABLES * kStreamTable + w * RING; };
         // lane e holds (maximum, denominator) of entry e
         float2 ml = make_float2(-INFINITY, 0.f);
         if ((mine >> lane) & 1u) {
@@ -793,30 +928,24 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
     if (threadIdx.x == 0 && !split) sp.split[blockIdx.x].z = -1;
 }
 
-template <int KB, int VB, bool QJL, bool SPARSE, bool SIGN_TABLE>
+template <int KB, int VB, bool QJL, bool SPARSE, bool ONE_QUERY>
 int launch_stream_as(const StreamParams& sp, cudaStream_t stream) {
-    auto kern = decode_stream_kernel<KB, VB, QJL, SPARSE, SIGN_TABLE>;
+    auto kern = decode_stream_kernel<KB, VB, QJL, SPARSE, ONE_QUERY>;
     static bool configured[64] = {};
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return TQ_ERR_LAUNCH;
+    constexpr int smem = stream_smem(KB == 3 && !QJL ? 1 : 2, kStreamStages * page_bytes(KB, VB, QJL ? 1 : 0));
     if (!configured[dev]) {
-        cudaFuncAttributes attr;
-        int reserved = 0;
-        if (cudaFuncGetAttributes(&attr, kern) != cudaSuccess ||
-            cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev) != cudaSuccess)
-            return TQ_ERR_LAUNCH;
-        const uint64_t start = (static_cast<uint64_t>(reserved) + attr.sharedSizeBytes + 127) & ~uint64_t{127};
-        if (start < kStreamFirstBase || start > kStreamLastBase) return TQ_ERR_UNSUPPORTED;
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kStreamSmem) != cudaSuccess) return TQ_ERR_LAUNCH;
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return TQ_ERR_LAUNCH;
         configured[dev] = true;
     }
-    return launch_chained(kern, dim3(sp.n_warps / kStreamWarps), dim3(kStreamThreads), kStreamSmem, stream, sp) == cudaSuccess ? TQ_OK : TQ_ERR_LAUNCH;
+    return launch_chained(kern, dim3(sp.n_warps / kStreamWarps), dim3(kStreamThreads), smem, stream, sp) == cudaSuccess ? TQ_OK : TQ_ERR_LAUNCH;
 }
 
 template <int KB, int VB, bool QJL, bool SPARSE>
 int launch_stream(const StreamParams& sp, cudaStream_t stream) {
-    if constexpr (QJL && KB == VB) {
-        if (sp.d.share_tables && !sp.d.qp) return launch_stream_as<KB, VB, QJL, SPARSE, true>(sp, stream);
+    if constexpr (QJL && (KB == 3 || KB == VB)) {
+        if (!sp.d.qp && (KB == 3 || sp.d.share_tables)) return launch_stream_as<KB, VB, QJL, SPARSE, true>(sp, stream);
     }
     return launch_stream_as<KB, VB, QJL, SPARSE, false>(sp, stream);
 }
