@@ -142,6 +142,34 @@ def test_fast_kernel_tight_codebook_falls_back_inside_the_kernel(prerotated, tcg
         assert (gs != (ok["signs"] > 0)).mean() <= 1e-3
 
 
+@pytest.mark.parametrize("c,b", [([-0.14, -0.045, 0.04, 0.13], [-0.09, -0.004, 0.085]),        # nothing symmetric
+                                 ([-0.13, -0.04, 0.04, 0.13], [-0.088, 0.0, 0.0851]),         # boundaries are not
+                                 ([-0.13, -0.04, 0.04, 0.14], [-0.085, 0.0, 0.085]),          # centroids are not
+                                 ([-0.13, -0.04, 0.04, 0.13], [-0.085, 0.0, 0.085])])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_two_bit_codebooks_of_any_shape(c, b, dtype):
+    """2-bit codebooks symmetric about zero are halved twice, any other one takes three comparisons: both against the oracle, with the
+    allowances of the rotation's own rounding, and rows with NaN keep to themselves."""
+    fmt = CacheFormat.named("turbo2")
+    c, b = torch.tensor(c), torch.tensor(b)
+    books = Codebooks(fmt, DEV, k_codebook=(c, b), v_codebook=(c, b))
+    key, val = _kv(T_BIG, HKV, dtype, seed=71)
+    got, status, _ = _run(key, val, fmt, books)
+    assert status == 0
+    ok, ov = _oracle(key, val, fmt, books, O.make_wht_matrix(128))
+    gk, gv = got["k_idx"].numpy().reshape(-1, 128).astype(int), got["v_idx"].numpy().reshape(-1, 128).astype(int)
+    assert (gk != ok["indices"]).mean() <= 1e-4 and np.abs(gk - ok["indices"]).max() <= 1
+    assert (gv != ov["indices"]).mean() <= 1e-4 and np.abs(gv - ov["indices"]).max() <= 1
+    assert (got["k_signs"].numpy().reshape(-1, 128) != (ok["signs"] > 0)).mean() <= 1e-4
+    assert _fp16_ulps(got["k_norm"].reshape(-1), ok["norms"]) <= 1 and _fp16_ulps(got["k_rnorm"].reshape(-1), ok["rot_residual_norm"]) <= 2
+    key[5, 3, 9] = float("nan")
+    dirty, _, _ = _run(key, val, fmt, books)
+    keep = torch.ones(T_BIG, HKV, dtype=torch.bool)
+    keep[5, 3] = False
+    assert not torch.isfinite(dirty["k_norm"][5, 3])
+    assert all(torch.equal(got[n][keep], dirty[n][keep]) for n in got)
+
+
 @pytest.mark.parametrize("dtype,prerotated,tcgen05", [(torch.float16, False, False), (torch.bfloat16, False, False),
                                                       (torch.float32, False, False), (torch.float16, True, False),
                                                       (torch.float16, False, True), (torch.bfloat16, False, True)])

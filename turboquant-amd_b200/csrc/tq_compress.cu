@@ -16,6 +16,8 @@
 // of each quotient (q0 = r * inv; q = q0 + (r - q0 * den) * inv), which returns the IEEE quotient.
 // Outputs go either into the paged cache (layout of turboquant/kernels/paged_layout.py) or into
 // the contiguous arrays of compress_k / compress_v (turboquant/kernels/packed_compress.py:157-240).
+#include <type_traits>
+
 #include "tq_common.cuh"
 
 namespace tq {
@@ -654,6 +656,7 @@ template <int BITS, bool QJL, Rows ROWS>
 __global__ void __launch_bounds__(kFastWarps * 32, 1) compress_contig_fast_kernel(const __grid_constant__ ContigParams p, int64_t n_units) {
     extern __shared__ __align__(128) unsigned char tables[];
     __shared__ float csm[1 << BITS];
+    __shared__ Comparisons2 comparisons[BITS == 2 ? kFastWarps : 1];
     __shared__ int bad;
     const int lane = threadIdx.x & 31, quarter = lane & 3, warp = threadIdx.x >> 5;
     constexpr bool mma = ROWS != Rows::kPlain, BF16 = ROWS == Rows::kBF16;
@@ -687,12 +690,12 @@ __global__ void __launch_bounds__(kFastWarps * 32, 1) compress_contig_fast_kerne
     if constexpr (mma) {
         const WhtFragments hf = make_wht_fragments(lane, BF16);
         Codebook2<BITS> cb;
-        if constexpr (BITS == 2) cb.load(p.b, QJL ? p.c : nullptr);
+        if constexpr (BITS == 2) cb.load(p.b, QJL ? p.c : nullptr, &comparisons[warp], lane);
         uint32_t cur = 0;   // offset of the buffer whose turn it is
         for (; unit < n_units; unit += step, cur ^= kRowBuffer) {
             const int64_t row = row_of(unit), nxt = row_of(unit + 2 * step);
             wait_staged();
-            compress_row_mma<BF16, BITS, QJL, false, true>(src + cur, row < p.n, lane, hf, tab, cb, q, [&] {
+            compress_row_mma<BF16, BITS, QJL, false, true>(src + cur, lane, hf, tab, cb, q, [&] {
                 stage_row(dst + cur, p.x, nxt * kHeadDim + 8 * quarter, nxt < p.n);
             });
             store_contig_fast<BITS, QJL>(p, row, quarter, q);

@@ -248,19 +248,42 @@ __device__ __forceinline__ void quant_pair(f2 y, const VecConsts& vc, f2& rr, ui
 
 // The same for rows rotated here: u is the plain product, residuals are not yet multiplied by the norm.
 template <int BITS>
-struct Codebook2 {};   // 3 and 4 bits: everything is in the table
+struct Codebook2 {   // 3 and 4 bits: everything is in the table
+    static constexpr bool split = true;
+};
+// 2 bits by three comparisons: -b_j * 2^126; -c_0 and the steps from -c_(j-1) to -c_j.
+struct Comparisons2 {
+    float nb[3], nc0, nc[3];
+};
+// 2 bits, halving the codebook twice: t = [u > b_1], then t' = [u > b_0] or [u > b_2], idx = 2 t + t'.  The second boundary is a
+// multiply-add away from the first, and the step to the second centroid of either half is the same, in a codebook symmetric about
+// zero; `split` says that these sums give what the comparisons give.  Any other codebook takes the comparisons as they are, whose
+// constants wait in shared memory.
 template <>
 struct Codebook2<2> {
-    float nb[3];        // -b_j * 2^126
-    float nc[4];        // -c_0 and the steps from -c_(j-1) to -c_j
-    __device__ __forceinline__ void load(const float* __restrict__ b, const float* __restrict__ c) {
+    float nb_1;                          // -b_j * 2^126
+    f2 nb_0, nb_0to2;
+    f2 nc_0, step_01, step_12;           // -c_0, and the steps from -c_j to -c_(j+1)
+    const Comparisons2* comparisons;
+    bool split;
+    __device__ __forceinline__ void load(const float* __restrict__ b, const float* __restrict__ c, Comparisons2* of_warp, int lane) {
+        Comparisons2 k;
 #pragma unroll
-        for (int j = 0; j < 3; ++j) nb[j] = -(__ldg(b + j) * big());
-        if (c) {
-            nc[0] = -__ldg(c);
+        for (int j = 0; j < 3; ++j) k.nb[j] = -(__ldg(b + j) * big());
+        k.nc0 = c ? -__ldg(c) : 0.f;
 #pragma unroll
-            for (int j = 1; j < 4; ++j) nc[j] = centroid_step(__ldg(c + j - 1), __ldg(c + j));
-        }
+        for (int j = 0; j < 3; ++j) k.nc[j] = c ? centroid_step(__ldg(c + j), __ldg(c + j + 1)) : 0.f;
+        if (lane == 0) *of_warp = k;
+        __syncwarp();
+        comparisons = of_warp;
+        const float db = centroid_step(-k.nb[0], -k.nb[2]), n2 = (k.nc0 + k.nc[0]) + k.nc[1];
+        split = __all_sync(0xffffffffu, k.nb[0] >= k.nb[1] && k.nb[1] >= k.nb[2] && k.nb[0] + db == k.nb[2] && n2 + k.nc[0] == n2 + k.nc[2]);
+        nb_1 = k.nb[1];
+        nb_0 = f2dup(k.nb[0]);
+        nb_0to2 = f2dup(db);
+        nc_0 = f2dup(k.nc0);
+        step_01 = f2dup(k.nc[0]);
+        step_12 = f2dup(k.nc[1]);
     }
 };
 
@@ -269,21 +292,29 @@ struct RowConsts {
     uint32_t tab;
 };
 
-template <int BITS, bool QJL>
-__device__ __forceinline__ void quant_pair_rotated(f2 y, const RowConsts& rc, const Codebook2<BITS>& cb, f2& ee, uint32_t& sacc, float& kfa,
-                                                   float& kfb) {
+// kf: the pair's two indices.
+template <int BITS, bool QJL, class Book>
+__device__ __forceinline__ void quant_pair_rotated(f2 y, const RowConsts& rc, const Book& cb, f2& ee, uint32_t& sacc, f2& kf) {
     const float kBig = big();
     const f2 u = f2mul(y, rc.inv);
-    float ua, ub, nca = 0.f, ncb = 0.f;   // minus the centroids
+    float ua, ub;
     f2unpack(u, ua, ub);
+    f2 nc = f2dup(0.f);   // minus the centroids
     if constexpr (BITS == 2) {
-        const float a0 = fma_sat(ua, kBig, cb.nb[0]), a1 = fma_sat(ua, kBig, cb.nb[1]), a2 = fma_sat(ua, kBig, cb.nb[2]);
-        const float b0 = fma_sat(ub, kBig, cb.nb[0]), b1 = fma_sat(ub, kBig, cb.nb[1]), b2 = fma_sat(ub, kBig, cb.nb[2]);
-        kfa = (a0 + a1) + a2;
-        kfb = (b0 + b1) + b2;
-        if constexpr (QJL) {
-            nca = fmaf(a2, cb.nc[3], fmaf(a1, cb.nc[2], fmaf(a0, cb.nc[1], cb.nc[0])));
-            ncb = fmaf(b2, cb.nc[3], fmaf(b1, cb.nc[2], fmaf(b0, cb.nc[1], cb.nc[0])));
+        // only the comparisons saturate and take one value at a time: the rest is two dims to an instruction
+        if constexpr (std::is_same_v<Book, Codebook2<2>>) {
+            const f2 t = f2pack(fma_sat(ua, kBig, cb.nb_1), fma_sat(ub, kBig, cb.nb_1));
+            float na, nb;
+            f2unpack(f2fma(t, cb.nb_0to2, cb.nb_0), na, nb);
+            const f2 t2 = f2pack(fma_sat(ua, kBig, na), fma_sat(ub, kBig, nb));
+            kf = f2fma(t, f2dup(2.f), t2);
+            if constexpr (QJL) nc = f2fma(t2, cb.step_01, f2fma(t, cb.step_12, f2fma(t, cb.step_01, cb.nc_0)));
+        } else {
+            const f2 t0 = f2pack(fma_sat(ua, kBig, cb.nb[0]), fma_sat(ub, kBig, cb.nb[0]));
+            const f2 t1 = f2pack(fma_sat(ua, kBig, cb.nb[1]), fma_sat(ub, kBig, cb.nb[1]));
+            const f2 t2 = f2pack(fma_sat(ua, kBig, cb.nb[2]), fma_sat(ub, kBig, cb.nb[2]));
+            kf = f2add(f2add(t0, t1), t2);
+            if constexpr (QJL) nc = f2fma(t2, f2dup(cb.nc[2]), f2fma(t1, f2dup(cb.nc[1]), f2fma(t0, f2dup(cb.nc[0]), f2dup(cb.nc0))));
         }
     } else {
         const f2 cellf = f2fma(y, rc.inv64, f2dup(kMagic + kCellScale));   // low mantissa bits: round(scale u) + scale
@@ -294,18 +325,15 @@ __device__ __forceinline__ void quant_pair_rotated(f2 y, const RowConsts& rc, co
         if constexpr (QJL) {
             const float4 ea = lds128(addr_a), eb = lds128(addr_b);   // NB, lo, -c[lo], c[lo] - c[lo+1]
             const float ta = fma_sat(ua, kBig, ea.x), tb = fma_sat(ub, kBig, eb.x);
-            nca = fmaf(ta, ea.w, ea.z);
-            ncb = fmaf(tb, eb.w, eb.z);
-            kfa = ea.y + ta;
-            kfb = eb.y + tb;
+            nc = f2pack(fmaf(ta, ea.w, ea.z), fmaf(tb, eb.w, eb.z));
+            kf = f2pack(ea.y + ta, eb.y + tb);
         } else {
             const float2 ea = lds64(addr_a), eb = lds64(addr_b);     // NB, lo
-            kfa = ea.y + fma_sat(ua, kBig, ea.x);
-            kfb = eb.y + fma_sat(ub, kBig, eb.x);
+            kf = f2pack(ea.y + fma_sat(ua, kBig, ea.x), eb.y + fma_sat(ub, kBig, eb.x));
         }
     }
     if constexpr (QJL) {
-        const f2 e = f2add(u, f2pack(nca, ncb));
+        const f2 e = f2add(u, nc);
         ee = f2fma(e, e, ee);
         float e0, e1;
         f2unpack(e, e0, e1);
@@ -499,27 +527,22 @@ __device__ __forceinline__ void mma_k8(float (&d)[4], uint32_t a0, uint32_t a1, 
 }
 
 // row: staged_at(...) of this lane (piece j is at row ^ 16 j).
-__device__ __forceinline__ void read_staged(uint32_t row, bool live, uint32_t (&w)[16]) {
-    if (live) {
+__device__ __forceinline__ void read_staged(uint32_t row, uint32_t (&w)[16]) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-            asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
-                         : "=r"(w[4 * j]), "=r"(w[4 * j + 1]), "=r"(w[4 * j + 2]), "=r"(w[4 * j + 3])
-                         : "r"(row ^ (16 * j)));
-    } else {
-#pragma unroll
-        for (int i = 0; i < 16; ++i) w[i] = 0u;
-    }
+    for (int j = 0; j < 4; ++j)
+        asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
+                     : "=r"(w[4 * j]), "=r"(w[4 * j + 1]), "=r"(w[4 * j + 2]), "=r"(w[4 * j + 3])
+                     : "r"(row ^ (16 * j)));
 }
 
 // after_read() is called once the staged row has been read for the last time (the caller requests the next row
-// into the same buffer there).
+// into the same buffer there).  Lanes past the end of the input quantize whatever their buffer holds; nobody stores it.
 template <bool BF16, int BITS, bool QJL, bool ISV, bool CONTIG = false, class AfterRead>
-__device__ __forceinline__ void compress_row_mma(uint32_t row, bool live, int lane, const WhtFragments& hf,
+__device__ __forceinline__ void compress_row_mma(uint32_t row, int lane, const WhtFragments& hf,
                                                  uint32_t tab, const Codebook2<BITS>& cb, Packed& out, AfterRead after_read) {
     constexpr float kStep = CONTIG ? static_cast<float>(1 << BITS) : 16.f;   // spacing of a chunk's four indices
     uint32_t w[16];
-    read_staged(row, live, w);
+    read_staged(row, w);
     // ||x||^2: even words on the diagonal of rows 0..7 of da, odd words on that of rows 8..15 of db
     float da[4], db[4];
     mma_k8<BF16, true>(da, w[0], w[1], w[0]);
@@ -535,7 +558,14 @@ __device__ __forceinline__ void compress_row_mma(uint32_t row, bool live, int la
     // NaN or overflow somewhere in the vector: quantize a zero vector so that the table lookups stay in range (the
     // stored norm still shows the bad value).
     const bool finite = ss < __uint_as_float(0x7f800000u);
-    if (!finite) live = false;
+    // (as zeros in the buffer, behind a branch: 16 predicated moves of zero a row were 4 % of the instructions)
+    if (!__all_sync(0xffffffffu, finite)) {
+        if (!finite) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) asm volatile("st.shared.v4.u32 [%0], {%1,%1,%1,%1};" ::"r"(row ^ (16 * j)), "r"(0) : "memory");
+        }
+        read_staged(row, w);
+    }
     const float n_out = sqrtf(ss);                                // = ||x H / sqrt(128)||
     const float n = finite ? n_out : 0.f;
     const float den = (n + 1e-8f) * 11.313708498984761f;          // the unnormalised transform is sqrt(128) larger
@@ -547,42 +577,59 @@ __device__ __forceinline__ void compress_row_mma(uint32_t row, bool live, int la
     float cv[8];
     f2 ee = f2dup(0.f);
     uint32_t sg = 0u;   // bit l = 1 when the residual of local dim l is negative
+    auto quantize = [&](const auto& book) {
 #pragma unroll
-    for (int nt = 0; nt < 2; ++nt) {
-        if (nt == 1 || !live) read_staged(row, live, w);
-        if (nt == 1) {
-            __syncwarp();
-            after_read();
-        }
-        f2 y[8];   // pair 2 j + r = dims 8 j + 4 nt + 2 r + {0, 1}
+        for (int nt = 0; nt < 2; ++nt) {
+            if (nt == 1) {
+                read_staged(row, w);
+                __syncwarp();
+                after_read();
+            }
+            f2 y[8];   // pair 2 j + r = dims 8 j + 4 nt + 2 r + {0, 1}
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            float d[4];
-            mma_16816_zero<BF16>(d, w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3], hf.b0[nt], hf.b1[nt]);
-            y[2 * j] = f2pack(d[0], d[1]);
-            y[2 * j + 1] = f2pack(d[2], d[3]);
-        }
+            for (int j = 0; j < 4; ++j) {
+                float d[4];
+                mma_16816_zero<BF16>(d, w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3], hf.b0[nt], hf.b1[nt]);
+                y[2 * j] = f2pack(d[0], d[1]);
+                y[2 * j + 1] = f2pack(d[2], d[3]);
+            }
 #pragma unroll
-        for (int h = 1; h < 8; h <<= 1) {
+            for (int h = 1; h < 8; h <<= 1) {
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                if (!(i & h)) {
-                    const f2 a = y[i], b = y[i + h];
-                    y[i] = f2add(a, b);
-                    y[i + h] = f2sub(a, b);
+                for (int i = 0; i < 8; ++i) {
+                    if (!(i & h)) {
+                        const f2 a = y[i], b = y[i + h];
+                        y[i] = f2add(a, b);
+                        y[i + h] = f2sub(a, b);
+                    }
                 }
             }
-        }
 #pragma unroll
-        for (int j = 3; j >= 0; --j) {
-            const int c = 2 * j + nt;   // chunk of dims 4 c .. 4 c + 3
-            float k0, k1, k2, k3;
-            uint32_t nib = 0u;
-            quant_pair_rotated<BITS, QJL>(y[2 * j + 1], rc, cb, ee, nib, k2, k3);
-            quant_pair_rotated<BITS, QJL>(y[2 * j], rc, cb, ee, nib, k0, k1);
-            cv[c] = fmaf(fmaf(fmaf(k3, kStep, k2), kStep, k1), kStep, k0);
-            if constexpr (QJL) sg |= nib << (4 * c);
+            for (int j = 3; j >= 0; --j) {
+                const int c = 2 * j + nt;   // chunk of dims 4 c .. 4 c + 3
+                f2 k01, k23;
+                uint32_t nib = 0u;
+                quant_pair_rotated<BITS, QJL>(y[2 * j + 1], rc, book, ee, nib, k23);
+                quant_pair_rotated<BITS, QJL>(y[2 * j], rc, book, ee, nib, k01);
+                float a, b;
+                if constexpr (BITS == 4 && QJL && CONTIG) {   // one register short for the form below: 200 us for 1 M rows of K and V instead of 197
+                    float k0, k1;
+                    f2unpack(k01, k0, k1);
+                    f2unpack(k23, a, b);
+                    cv[c] = fmaf(fmaf(fmaf(b, kStep, a), kStep, k1), kStep, k0);
+                } else {
+                    f2unpack(f2fma(k23, f2dup(kStep * kStep), k01), a, b);   // indices 0 and 2, 1 and 3
+                    cv[c] = fmaf(b, kStep, a);
+                }
+                if constexpr (QJL) sg |= nib << (4 * c);
+            }
         }
+    };
+    if constexpr (BITS == 2) {
+        if (cb.split) quantize(cb);
+        else quantize(Comparisons2(*cb.comparisons));
+    } else {
+        quantize(cb);
     }
     if constexpr (CONTIG) assemble_contig<BITS>(cv, out);
     else assemble_indices<BITS, ISV>(cv, out);
@@ -741,6 +788,7 @@ __global__ void __launch_bounds__(kFastWarps * 32, TQ_CMP_MINBLOCKS) compress_pa
     extern __shared__ __align__(128) unsigned char tables[];
     __shared__ float csm[1 << KB];
     __shared__ int bad;
+    __shared__ Comparisons2 comparisons[KB == 2 || VB == 2 ? kFastWarps : 1][2];
     const int lane = threadIdx.x & 31, quarter = lane & 3, warp = threadIdx.x >> 5;
     constexpr uint32_t kBias = kMagicBits * static_cast<uint32_t>(kCellStride);   // modulo 2^32
     const uint32_t ktab = smem_u32(tables) + (QJL ? (lane & 7) * 16 : (lane & 15) * 8) - kBias;
@@ -789,8 +837,8 @@ __global__ void __launch_bounds__(kFastWarps * 32, TQ_CMP_MINBLOCKS) compress_pa
     const WhtFragments hf = make_wht_fragments(lane, BF16);
     Codebook2<KB> kcb;
     Codebook2<VB> vcb;
-    if constexpr (KB == 2) kcb.load(p.kb, QJL ? p.kc : nullptr);
-    if constexpr (VB == 2) vcb.load(p.vb, nullptr);
+    if constexpr (KB == 2) kcb.load(p.kb, QJL ? p.kc : nullptr, &comparisons[warp][0], lane);
+    if constexpr (VB == 2) vcb.load(p.vb, nullptr, &comparisons[warp][1], lane);
     Packed q;
     // Only the identity (token, head) of the next unit's item is carried across the loop body; where the current item
     // goes in the cache is looked up when its turn comes.
@@ -804,12 +852,12 @@ __global__ void __launch_bounds__(kFastWarps * 32, TQ_CMP_MINBLOCKS) compress_pa
         unit += step;
         id = identify_paired(p, unit * kItemsPerWarp + (lane >> 2));
         wait_staged();
-        compress_row_mma<BF16, KB, QJL, false>(krow, w.live, lane, hf, ktab, kcb, q, [&] {
+        compress_row_mma<BF16, KB, QJL, false>(krow, lane, hf, ktab, kcb, q, [&] {
             stage_row(kdst, p.key, id.tok * p.ks_t + id.head * p.ks_h + 8 * quarter, id.live);
         });
         if (w.live) store_k_fast<KB, QJL>(w.page, w.t, quarter, q);
         wait_staged();
-        compress_row_mma<BF16, VB, false, true>(vrow, w.live, lane, hf, vtab, vcb, q, [&] {
+        compress_row_mma<BF16, VB, false, true>(vrow, lane, hf, vtab, vcb, q, [&] {
             stage_row(vdst, p.value, id.tok * p.vs_t + id.head * p.vs_h + 8 * quarter, id.live);
         });
         if (pairs) {
