@@ -840,21 +840,23 @@ __global__ void __launch_bounds__(kFastWarps * 32, TQ_CMP_MINBLOCKS) compress_pa
     if constexpr (KB == 2) kcb.load(p.kb, QJL ? p.kc : nullptr, &comparisons[warp][0], lane);
     if constexpr (VB == 2) vcb.load(p.vb, nullptr, &comparisons[warp][1], lane);
     Packed q;
-    // Only the identity (token, head) of the next unit's item is carried across the loop body; where the current item
-    // goes in the cache is looked up when its turn comes.
+    // Only the identity (token, head) of the next unit's item is carried across the loop body.  The current item's slot is
+    // requested at its turn and waited for when its key is done.
     while (unit < units) {
-        const ItemPlace w = place_item<PAGE>(p, id, quarter);
-        const unsigned long long at = reinterpret_cast<unsigned long long>(w.page);
-        const unsigned long long at_other = __shfl_xor_sync(0xffffffffu, at, 4);
-        const int t_other = __shfl_xor_sync(0xffffffffu, w.t, 4);
-        // both tokens of every pair in one word of one page, or neither of them stored (no page)
-        const bool pairs = __all_sync(0xffffffffu, at_other == at && (at == 0 || t_other == (w.t ^ 1)));
+        const ItemId now = id;
+        const int64_t slot = now.live ? p.slot_mapping[now.tok] : 0;
         unit += step;
         id = identify_paired(p, unit * kItemsPerWarp + (lane >> 2));
         wait_staged();
         compress_row_mma<BF16, KB, QJL, false>(krow, lane, hf, ktab, kcb, q, [&] {
             stage_row(kdst, p.key, id.tok * p.ks_t + id.head * p.ks_h + 8 * quarter, id.live);
         });
+        const ItemPlace w = place_item<PAGE>(p, now, slot, quarter);
+        const unsigned long long at = reinterpret_cast<unsigned long long>(w.page);
+        const unsigned long long at_other = __shfl_xor_sync(0xffffffffu, at, 4);
+        const int t_other = __shfl_xor_sync(0xffffffffu, w.t, 4);
+        // both tokens of every pair in one word of one page, or neither of them stored (no page)
+        const bool pairs = __all_sync(0xffffffffu, at_other == at && (at == 0 || t_other == (w.t ^ 1)));
         if (w.live) store_k_fast<KB, QJL>(w.page, w.t, quarter, q);
         wait_staged();
         compress_row_mma<BF16, VB, false, true>(vrow, lane, hf, vtab, vcb, q, [&] {
