@@ -19,9 +19,9 @@
 //    cell's table entry gives lo = #{boundaries below the cell}, and NB = -b * 2^126 for the boundary b inside
 //    the cell (-inf when there is none), so  t = sat(u * 2^126 + NB)  is exactly [u > b]  (ties stay down,
 //    as searchsorted(right=False)), and idx = lo + t.  The entry also carries the centroids.
-//  * bucketize, 2-bit: the three comparisons directly, t_j = sat(u * 2^126 - b_j * 2^126), idx = t_0 + t_1 + t_2: about
-//    as many instructions as the table look-up, and none of its shared-memory traffic, which at 8 wavefronts (V) and
-//    16 (K) per element and four schedulers was half of what the data path of the SM can do.
+//  * bucketize, 2-bit: comparisons t = sat(u * 2^126 - b * 2^126) without a table, whose shared-memory traffic was half of what
+//    the data path of the SM can do.  A codebook symmetric about zero is halved twice (two comparisons, the second boundary by
+//    a multiply-add), any other one takes all three; sums and centroids are two dims to an instruction.
 //  * where the rotation is done here (fp16 / bf16 rows), u = y * (1 / (n + 1e-8)) is a plain product, the centroid one FMA
 //    (c[lo] + t (c[lo+1] - c[lo])), and ||residual|| = n ||u - c|| is scaled once per vector.
 //  * packing: the four indices of a chunk of adjacent dims are combined by three FMAs into one float (one index
@@ -38,10 +38,11 @@
 namespace tq {
 namespace {
 
-// Compile-time tunables.  The tensor-core loop wants the 128 registers that 16 warps per SM leave it: 2-bit keys and keys
-// without signs fit, 3- and 4-bit keys with signs spill 36-44 bytes (a build at 80 registers and 24 warps per SM spilled far
-// more and measured 1.3-1.6x slower).  One CTA of 16 warps
-// per SM builds the tables once for all of them: 4 % faster than two CTAs of 8 warps.
+// What bounds it: issue (58 to 63 % of the cycles with 16 warps per SM, which is what 128 registers allow; a build at 80
+// registers and 24 warps per SM spilled and measured 1.3-1.6x slower), so what counts is how many instructions an item takes: 108 with
+// 2 bits (133 before indices and centroids went two to an instruction), us for 8 KV heads: 1 M tokens of turbo2 1505 -> 1420, and
+// 1368 with the slots requested a key ahead of their use; 256 K of turbo3 416 -> 381 -> 378, of turbo4 351 -> 340 -> 335.
+// One CTA of 16 warps per SM builds the tables once for all of them: 4 % faster than two CTAs of 8 warps.
 #ifndef TQ_CMP_MINBLOCKS
 #define TQ_CMP_MINBLOCKS 1
 #endif

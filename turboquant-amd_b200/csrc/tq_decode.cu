@@ -738,7 +738,8 @@ int dispatch_v(const DecodeParams& p, int vb, const Plan& plan, cudaStream_t str
 // 1 x 16384 tokens (8192 pages) 14.6 / 16.1 and 14.1 / 16.8; 24 x 1024 (12288) 15.9 / 18.2 and 22.1 / 19.5; 64 x 512 (16384)
 // 19.1 / 20.6 and 19.4 / 22.2, 32 x 1024 22.8 / 19.4 and 22.9 / 20.9; 256 x 256 (32768) 35.3 / 32.9 and 36.4 / 36.2, 128 x 512
 // 30.2 / 30.1 and 31.9 / 33.1; 32 x 3000 (48128) 48.0 / 35.1 and 51.3 / 39.1.  The line does not look at the format: it is
-// off by 4 to 13 % for 24 x 1024 and 128 x 512 with sign term.
+// off by 4 to 13 % for 24 x 1024 and 128 x 512 with sign term.  (Since these were taken the persistent kernel became 3 to 6 % faster:
+// turbo4 128 x 512 28.8, turbo3 31.9, 256 x 256 32.1 and 34.9.)
 constexpr int64_t kStreamMinPages = 16384;
 constexpr int64_t kStreamSlots = static_cast<int64_t>(kStreamCtas) * (kStreamWarps + 2);   // partials of warps and of CTAs
 int64_t pages_at_most(int64_t ns, int64_t hq, int64_t hkv, int64_t max_pages) { return ns * max_pages * hkv * ((hq / hkv + 7) / 8); }

@@ -31,6 +31,9 @@ constexpr int kStreamSlotFloats = 8 * kHeadDim;
 // Dynamic shared memory: tables, then one ring per warp.
 __host__ __device__ constexpr int stream_smem(int tables, int ring) { return tables * kStreamTable + kStreamWarps * ring; }
 constexpr int kStreamStaticMost = 6144;      // the kernel's static arrays are smaller
+// Which keys are scored in integers (the reasons stand at the digits below).  Not with Sparse-V: 64 x 16-32K tokens of turbo3 took 456 us
+// so and 443 with looked-up keys.
+__host__ __device__ constexpr bool stream_integer(int k_bits, bool sparse) { return k_bits == 3 && !sparse; }
 
 struct StreamParams {
     DecodeParams d;
@@ -297,8 +300,8 @@ __device__ __forceinline__ void finish_row(const DecodeParams& p, int seq, int h
     if (g < p.G - qg * 8) write_row(p, static_cast<int64_t>(seq) * p.Hq + kvh * p.G + qg * 8 + g, lane, x, l);
 }
 
-// ONE_QUERY: the query operands of the index term serve the sign term as well (S = I).  With 2- and 4-bit keys K and V share a
-// codebook then, so that there is room for the table of signs; without, their sign operands are made by logic.
+// ONE_QUERY: the query operands of the index term serve the sign term as well (S = I).  Where keys are looked up K and V share a
+// codebook then, so that there is room for the table of signs; without, the sign operands are made by logic.
 template <int KB, int VB, bool QJL, bool SPARSE, bool ONE_QUERY>
 __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const StreamParams sp) {
     constexpr int NWK = KB + (QJL ? 1 : 0);
@@ -310,7 +313,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
     constexpr int PAGE = KPART + 256 * VB + 32;
     constexpr int NSTAGE = kStreamStages;
     constexpr int RING = NSTAGE * PAGE;
-    constexpr bool INTEGER = KB == 3;                       // scores from integer products, else half-precision products of look-ups
+    constexpr bool INTEGER = stream_integer(KB, SPARSE);    // scores from integer products, else half-precision products of look-ups
     constexpr bool SIGNS = QJL && (INTEGER || ONE_QUERY);   // table of signs
     constexpr int TABLES = INTEGER && !QJL ? 1 : 2;         // INTEGER: V, signs; else K and V in one and signs, or K and V
     static_assert(stream_smem(TABLES, RING) + kStreamStaticMost + 1024 <= 227 * 1024, "what an SM gives one CTA");
@@ -934,7 +937,7 @@ int launch_stream_as(const StreamParams& sp, cudaStream_t stream) {
     static bool configured[64] = {};
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return TQ_ERR_LAUNCH;
-    constexpr int smem = stream_smem(KB == 3 && !QJL ? 1 : 2, kStreamStages * page_bytes(KB, VB, QJL ? 1 : 0));
+    constexpr int smem = stream_smem(stream_integer(KB, SPARSE) && !QJL ? 1 : 2, kStreamStages * page_bytes(KB, VB, QJL ? 1 : 0));
     if (!configured[dev]) {
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return TQ_ERR_LAUNCH;
         configured[dev] = true;
@@ -944,8 +947,8 @@ int launch_stream_as(const StreamParams& sp, cudaStream_t stream) {
 
 template <int KB, int VB, bool QJL, bool SPARSE>
 int launch_stream(const StreamParams& sp, cudaStream_t stream) {
-    if constexpr (QJL && (KB == 3 || KB == VB)) {
-        if (!sp.d.qp && (KB == 3 || sp.d.share_tables)) return launch_stream_as<KB, VB, QJL, SPARSE, true>(sp, stream);
+    if constexpr (QJL && (stream_integer(KB, SPARSE) || KB == VB)) {
+        if (!sp.d.qp && (stream_integer(KB, SPARSE) || sp.d.share_tables)) return launch_stream_as<KB, VB, QJL, SPARSE, true>(sp, stream);
     }
     return launch_stream_as<KB, VB, QJL, SPARSE, false>(sp, stream);
 }
