@@ -228,13 +228,6 @@ __device__ __forceinline__ uint32_t lds_u32(uint32_t addr) {
     return v;
 }
 
-template <int OFF>
-__device__ __forceinline__ uint2 lds_u64(uint32_t addr) {
-    uint2 v;
-    asm volatile("ld.shared.v2.u32 {%0,%1}, [%2+%3];" : "=r"(v.x), "=r"(v.y) : "r"(addr), "n"(OFF));
-    return v;
-}
-
 template <int NW, int OFF>
 __device__ __forceinline__ void lds_words(uint32_t addr, uint32_t (&w)[NW]) {
     if constexpr (NW == 4) {

@@ -9,15 +9,20 @@
 // Against the chunked kernel (4-warp CTAs, one chunk of one item each) this takes away the last wave that is three
 // quarters full, the table fill, pipeline start and merge per chunk, and the empty CTAs of a ragged batch.
 //
-// What bounds it: instruction issue (62 % of the cycles with four warps a scheduler; a tensor instruction costs it about
-// three slots), and, where keys are looked up, the shared-memory data path next to it (turbo3 with looked-up keys: 82 %).
+// What bounds it: instruction issue (about 62 % of the cycles with four warps a scheduler; a tensor instruction costs it about
+// three slots), and the shared-memory data path next to it (turbo3: 82 %).
 // Pages are staged with cp.async, 16 bytes a lane, into a private ring: a page then costs four copy instructions and a counted
 // wait, where a bulk copy by one elected lane with its barrier cost about 35 instructions.  Together with a page body that has no
-// partly filled pages to look after, table addresses from the multiply-add pipe and loop state in uniform registers, us
-// before / now, 8 KV heads: turbo3 64 x 8192 tokens 154.2 / 150.1, turbo4 1 x 131072 43.4 / 41.2, turbo3 128 x 512 33.2 / 31.9, turbo3
-// with a query of the sign term's own 32 x 4096 52.6 / 50.0; 4 KV heads, 32 x 4096: 3-bit K and 4-bit V 31.0 / 28.8, turbo4 26.3 / 25.1.
+// partly filled pages to look after, table addresses from the multiply-add pipe and loop state in uniform registers, us per
+// launch in a graph of 8 or more over different caches, before / now, 8 KV heads: turbo3 64 x 8192 tokens 151.8 / 145.4, turbo4
+// 1 x 131072 43.5 / 41.5, turbo3 128 x 512 34.8 / 34.1, turbo3 with a query of the sign term's own 32 x 4096 53.3 / 49.4, turbo2 with
+// four heads a group 64 x 4096 74.5 / 75.3; 4 KV heads, 32 x 4096: 3-bit K and 4-bit V 28.1 / 26.6, turbo4 28.2 / 27.1.
 // Two pages per iteration came out the same (the loop's own instructions are few now), and so did V operands without the pairing
-// of tokens (twice the products with half of the weights zero: 19 instructions fewer, 8 products more; 154).
+// of tokens (twice the products with half of the weights zero: 19 instructions fewer, 8 products more).
+// 3-bit keys as integer products (m16n8k32: 16-bit queries and centroids as two signed digits, made by byte permutes from the
+// packed indices) were slower (147.8) and lost precision where one coordinate of a query is much larger than the others: the digits
+// share one step per row, while a looked-up product keeps the fp16 query as it is.  With one coordinate x 100 the error against 64
+// bits was 4 times that of the chunked kernel, with x 1000 35 times.
 namespace tq {
 namespace {
 
@@ -28,12 +33,9 @@ constexpr int kStreamTable = 32768;          // 256 entries of 128 bytes
 constexpr int kStreamCtas = 148;             // one per SM
 constexpr int kStreamSlotFloats = 8 * kHeadDim;
 
-// Dynamic shared memory: tables, then one ring per warp.
-__host__ __device__ constexpr int stream_smem(int tables, int ring) { return tables * kStreamTable + kStreamWarps * ring; }
+// Dynamic shared memory: two tables, then one ring per warp.
+__host__ __device__ constexpr int stream_smem(int ring) { return 2 * kStreamTable + kStreamWarps * ring; }
 constexpr int kStreamStaticMost = 6144;      // the kernel's static arrays are smaller
-// Which keys are scored in integers (the reasons stand at the digits below).  Not with Sparse-V: 64 x 16-32K tokens of turbo3 took 456 us
-// so and 443 with looked-up keys.
-__host__ __device__ constexpr bool stream_integer(int k_bits, bool sparse) { return k_bits == 3 && !sparse; }
 
 struct StreamParams {
     DecodeParams d;
@@ -219,90 +221,15 @@ __device__ __forceinline__ uint4 table_signs(uint32_t w, uint32_t base) {
     asm("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(entry_of<K>(w, base)));
     return v;
 }
-// The same as bytes, for integer products: four of token A, four of token B, 16 copies.
-__device__ __forceinline__ void fill_sign_bytes(uint32_t smem_addr, int warp, int lane) {
-    auto signs = [](int nibble) {   // 0xff for a clear bit, 0x01 for a set one
-        return 0xffffffffu ^ ((nibble & 1) * 0xfeu) ^ ((nibble & 2) * 0x7f00u) ^ ((nibble & 4) * 0x3f8000u) ^ ((nibble & 8) * 0x1fc00000u);
-    };
-    for (int b0 = 4 * warp; b0 < 256; b0 += 4 * kStreamWarps) {
-        const int b = b0 + (lane >> 3);
-        store_entry(smem_addr + b * 128 + 16 * (lane & 7), make_uint4(signs(b), signs(b >> 4), signs(b), signs(b >> 4)));
-    }
-}
-
-// ---- scores of 3-bit keys in integers --------------------------------------------------------------------
-// Query and codebook are taken to 16 bits (full scale 32512) and written as two signed digits, v = 256 hi + lo.  Four indices in
-// the nibbles of a half word are then the selector of one byte permute that returns the digits of four dims, four of these are the
-// A operand (16 tokens x 32 dims) of an m16n8k32 product, and the digits of the 8 query heads are its B operand.  hi hi, hi lo
-// and lo hi are summed, exactly; lo lo (2^-16 of full scale) is left out.
-// Against half-precision products of looked-up pairs: 75 instead of 121 shared-memory wavefronts a page and about as many issue
-// slots, so no faster where K, V and signs share tables (turbo3 64 x 8192: 150.1 against 149.4 us), but it needs no K table (other
-// calls gain 5 to 7 %) and is closer to 64 bits: the centroids keep 16 bits instead of fp16's 11 (2-norm, turbo3 64 x 8192:
-// 4.7e-4 -> 2.9e-4).  For 2-bit keys, where one look-up serves four dims, it is slower (mixed batch of 256: 401 against 393 us), and
-// 16 centroids do not fit a byte permute.
-constexpr float kDigitScale = 32512.f;          // 127 * 256: the high digit of +-full scale is +-127
-constexpr float kDigitMagic = 12582912.f + 128.f;   // 1.5 * 2^23: the integer lands in the low bits; + 128: its low digit is signed
-
-__device__ __forceinline__ float max_nan(float a, float b) {   // NaN if either is
-    float r;
-    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ uint32_t to_digits(float x, float scale) { return __float_as_uint(fmaf(x, scale, kDigitMagic)); }
-// High and low digits of four numbers, one per byte.
-__device__ __forceinline__ void pack_digits(uint32_t a, uint32_t b, uint32_t c, uint32_t d, uint32_t& hi, uint32_t& lo) {
-    const uint32_t ab = prmt(a, b, 0x5140u), cd = prmt(c, d, 0x5140u);
-    hi = prmt(ab, cd, 0x7632u);
-    lo = prmt(ab, cd, 0x5410u) ^ 0x80808080u;
-}
-// Digits of a codebook, of which lane l holds entry l mod 8: entry i is byte i of (x[0], x[1]).
-__device__ __forceinline__ void codebook_digits(float c, float scale, uint32_t (&hi)[2], uint32_t (&lo)[2]) {
-    const uint32_t u = to_digits(c, scale);
-    uint32_t v[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) v[i] = __shfl_sync(0xffffffffu, u, i);
-    pack_digits(v[0], v[1], v[2], v[3], hi[0], lo[0]);
-    pack_digits(v[4], v[5], v[6], v[7], hi[1], lo[1]);
-}
-
-__device__ __forceinline__ void mma_s8_16832(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-        : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
-// Selector words of a token's quarter: half h of word j holds the indices of the four dims of chunk 2 j + h, one per nibble.  A
-// selector's top bit would ask the permute for a sign: it has to be clear.
-template <int NW>
-__device__ __forceinline__ void selector_words(const uint32_t (&w)[NW], uint32_t (&m)[4]) {
-#pragma unroll
-    for (int j = 0; j < 3; ++j) m[j] = w[j] & 0x77777777u;
-    m[3] = ((w[0] >> 3) & 0x11111111u) | ((w[1] >> 2) & 0x22222222u) | ((w[2] >> 1) & 0x44444444u);
-}
-
-// Query row (head gid, quarter tig: 32 dims) as B operands: high digits of chunk c (dims 4 c .. 4 c + 3) in f[c], low ones in f[8 + c].
-__device__ __forceinline__ void query_digits(const float (&x)[32], float scale, uint32_t (&f)[16]) {
-#pragma unroll
-    for (int c = 0; c < 8; ++c)
-        pack_digits(to_digits(x[4 * c], scale), to_digits(x[4 * c + 1], scale), to_digits(x[4 * c + 2], scale), to_digits(x[4 * c + 3], scale), f[c], f[8 + c]);
-}
-// Largest magnitude of a row spread over the four lanes of a group, NaN if there is one.
-__device__ __forceinline__ float row_max(const float (&x)[32]) {
-    float m = 0.f;
-#pragma unroll
-    for (int i = 0; i < 32; i += 2) asm("max.NaN.abs.f32 %0, %0, %1, %2;" : "+f"(m) : "f"(x[i]), "f"(x[i + 1]));
-    m = max_nan(m, __shfl_xor_sync(0xffffffffu, m, 1));
-    return max_nan(m, __shfl_xor_sync(0xffffffffu, m, 2));
-}
-
 // Output row g of an item.
 __device__ __forceinline__ void finish_row(const DecodeParams& p, int seq, int hg, int g, int lane, float (&x)[4], float l) {
     const int kvh = p.ngroups == 1 ? hg : hg / p.ngroups, qg = hg - kvh * p.ngroups;
     if (g < p.G - qg * 8) write_row(p, static_cast<int64_t>(seq) * p.Hq + kvh * p.G + qg * 8 + g, lane, x, l);
 }
 
-// ONE_QUERY: the query operands of the index term serve the sign term as well (S = I).  Where keys are looked up K and V share a
-// codebook then, so that there is room for the table of signs; without, the sign operands are made by logic.
-template <int KB, int VB, bool QJL, bool SPARSE, bool ONE_QUERY>
+// SIGN_TABLE: K and V share a codebook and S = I, so the second table has room for the signs, and the query operands of the
+// index term serve the sign term as well; without, the sign operands are made by logic.
+template <int KB, int VB, bool QJL, bool SPARSE, bool SIGN_TABLE>
 __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const StreamParams sp) {
     constexpr int NWK = KB + (QJL ? 1 : 0);
     constexpr int RK = 16 * NWK;
@@ -313,10 +240,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
     constexpr int PAGE = KPART + 256 * VB + 32;
     constexpr int NSTAGE = kStreamStages;
     constexpr int RING = NSTAGE * PAGE;
-    constexpr bool INTEGER = stream_integer(KB, SPARSE);    // scores from integer products, else half-precision products of look-ups
-    constexpr bool SIGNS = QJL && (INTEGER || ONE_QUERY);   // table of signs
-    constexpr int TABLES = INTEGER && !QJL ? 1 : 2;         // INTEGER: V, signs; else K and V in one and signs, or K and V
-    static_assert(stream_smem(TABLES, RING) + kStreamStaticMost + 1024 <= 227 * 1024, "what an SM gives one CTA");
+    static_assert(stream_smem(RING) + kStreamStaticMost + 1024 <= 227 * 1024, "what an SM gives one CTA");
     const DecodeParams& p = sp.d;
 
     extern __shared__ __align__(128) uint8_t smem[];
@@ -328,15 +252,14 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
     const int warp = uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
     const int gid = lane >> 2, tig = lane & 3;
 
-    const uint32_t ktab = smem_u32(smem), vtab = ktab + (INTEGER || ONE_QUERY ? 0 : kStreamTable), stab = ktab + kStreamTable;
-    const uint32_t rings = ktab + TABLES * kStreamTable, ring = rings + warp * RING;
+    const uint32_t ktab = smem_u32(smem), vtab = ktab + (SIGN_TABLE ? 0 : kStreamTable), stab = ktab + kStreamTable;
+    const uint32_t rings = ktab + 2 * kStreamTable, ring = rings + warp * RING;
 
-    if constexpr (SIGNS && INTEGER) fill_sign_bytes(stab, warp, lane);   // constants
-    else if constexpr (SIGNS) fill_sign_table(stab, warp, lane);
+    if constexpr (SIGN_TABLE) fill_sign_table(stab, warp, lane);   // constants
     if (lane < 2) sm_part[2 * warp + lane] = make_int4(-1, 0, 0, 0);
     pdl_wait();
     pdl_release();
-    const float ck = lane_centroid<KB>(p.kc, lane), cv = !INTEGER && ONE_QUERY ? 0.f : lane_centroid<VB>(p.vc, lane);
+    const float ck = lane_centroid<KB>(p.kc, lane), cv = SIGN_TABLE ? 0.f : lane_centroid<VB>(p.vc, lane);
 
     // ---- pages before each thread's run of sequences (every CTA does the same scan over all lengths)
     const int per = (sp.ns + kStreamThreads - 1) / kStreamThreads;
@@ -450,27 +373,18 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
         }
     }
     // the codebooks' part of the table is filled behind the first pages' copies
-    if constexpr (!INTEGER) fill_stream_table<KB>(ktab, ck, warp, lane);
-    if constexpr (INTEGER || !ONE_QUERY) fill_stream_table<VB>(vtab, cv, warp, lane);
+    fill_stream_table<KB>(ktab, ck, warp, lane);
+    if constexpr (!SIGN_TABLE) fill_stream_table<VB>(vtab, cv, warp, lane);
     __syncthreads();
 
     const uint32_t klut = ktab + (KB == 2 ? 8 * (lane & 15) : 4 * lane);
     const uint32_t vlut = vtab + (VB == 2 ? 8 * (lane & 15) : 4 * lane);
-    const uint32_t slut = stab + (INTEGER ? 8 * (lane & 15) : 16 * (lane & 7));
+    const uint32_t slut = stab + 16 * (lane & 7);
     const uint32_t ring_k = ring + lane * (NWK * 4);
     const uint32_t ring_n = ring + gid * 4;
     const uint32_t ring_v = ring + (tig * 8 + gid) * 4;
 
-    const float qpscale = ONE_QUERY ? p.qpscale * (1.f / 16.f) : p.qpscale;   // the one-sided forms carry 1/16 in the query
-    uint32_t chi[2], clo[2];                  // digits of the K codebook
-    float cmax = 0.f;
-    if constexpr (INTEGER) {
-        cmax = fabsf(ck);
-#pragma unroll
-        for (int o = 1; o < 8; o <<= 1) cmax = max_nan(cmax, __shfl_xor_sync(0xffffffffu, cmax, o));
-        if (cmax < 1e-20f) cmax = 1e-20f;
-        codebook_digits(ck, kDigitScale / cmax, chi, clo);
-    }
+    const float qpscale = SIGN_TABLE ? p.qpscale * (1.f / 16.f) : p.qpscale;   // the one-sided forms carry 1/16 in the query
     uint32_t stage = 0;                       // ring stage of the current page
     uint32_t k_only = 0;                      // Sparse-V: bit s = the page in stage s came without its V part
     uint32_t v_skipped = 0;
@@ -482,47 +396,21 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
         const int head0 = kvh * p.G + qg * 8, nq = min(8, p.G - qg * 8);
         const int64_t row = (static_cast<int64_t>(seq) * p.Hq + head0 + gid) * kHeadDim;
 
-        // INTEGER: qf[c], qf[8 + c] are the high and low digits of chunk c, qpf those of the sign term's query if it has one of its
-        // own.  A score in the log2 domain is unit * (k norm * (index sum) + residual norm * sign_unit * (sign sum)).
-        uint32_t qf[16], qpf[QJL && !ONE_QUERY ? 16 : 1];
+        uint32_t qf[16], qpf[QJL && !SIGN_TABLE ? 16 : 1];
         float sq_init0 = 0.f, sq_init1 = 0.f;   // minus the query sums of the one-sided sign forms
-        float unit0 = 1.f, unit1 = 1.f, sign_unit0 = 0.f, sign_unit1 = 0.f;   // of queries 2 tig, 2 tig + 1
         {
             float xq[32];
             load_q32(p.q, row, tig, p.io_dtype, gid < nq, xq);
             if (p.rotate_q) rotate_q32(xq, lane, p.io_dtype);
-            if constexpr (INTEGER) {
-                auto take = [&](uint32_t (&f)[16]) {   // the row's digits; returns what a step of them stands for, NaN for a row with NaN or infinity
-                    float most = row_max(xq);
-                    if (most < 1e-30f) most = 1e-30f;
-                    query_digits(xq, kDigitScale / most, f);
-                    return most < INFINITY ? most * (1.f / kDigitScale) : NAN;
-                };
-                const float step = take(qf);
-                float unit = p.qscale * step * (cmax * (256.f / kDigitScale)), sign_unit = 0.f;
-                if constexpr (QJL) {
-                    sign_unit = step;
-                    if constexpr (!ONE_QUERY) {
-                        if (p.qp) load_q32(p.qp, row, tig, p.io_dtype, gid < nq, xq);
-                        sign_unit = take(qpf);
-                    }
-                    sign_unit *= p.qpscale * (1.f / 16.f);
-                }
-                unit0 = __shfl_sync(0xffffffffu, unit, 8 * tig);
-                unit1 = __shfl_sync(0xffffffffu, unit, 8 * tig + 4);
-                sign_unit0 = __shfl_sync(0xffffffffu, sign_unit, 8 * tig);
-                sign_unit1 = __shfl_sync(0xffffffffu, sign_unit, 8 * tig + 4);
-            } else {
-                q_frag_from(xq, qf);
-                if constexpr (QJL && !ONE_QUERY) {
-                    if (p.qp) load_q32(p.qp, row, tig, p.io_dtype, gid < nq, xq);
-                    float corr;
-                    qp_frag_signed_from(xq, qpf, corr);
-                    corr += __shfl_xor_sync(0xffffffffu, corr, 1);
-                    corr += __shfl_xor_sync(0xffffffffu, corr, 2);
-                    sq_init0 = -__shfl_sync(0xffffffffu, corr, 8 * tig);
-                    sq_init1 = -__shfl_sync(0xffffffffu, corr, 8 * tig + 4);
-                }
+            q_frag_from(xq, qf);
+            if constexpr (QJL && !SIGN_TABLE) {
+                if (p.qp) load_q32(p.qp, row, tig, p.io_dtype, gid < nq, xq);
+                float corr;
+                qp_frag_signed_from(xq, qpf, corr);
+                corr += __shfl_xor_sync(0xffffffffu, corr, 1);
+                corr += __shfl_xor_sync(0xffffffffu, corr, 2);
+                sq_init0 = -__shfl_sync(0xffffffffu, corr, 8 * tig);
+                sq_init1 = -__shfl_sync(0xffffffffu, corr, 8 * tig + 4);
             }
         }
         // Sparse-V: columns past the group's heads hold zero queries, whose scores are all alike; they decide nothing
@@ -545,119 +433,78 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
             lds_words<NWK, 0>(ring_k + so, wa);
             lds_words<NWK, 32 * NWK * 4>(ring_k + so, wb);
             uint32_t sgn0 = 0, sgn1 = 0;   // bytes: the nibbles 2 k (sgn0), 2 k + 1 (sgn1) of token A, then of token B
-            if constexpr (SIGNS) {
+            if constexpr (SIGN_TABLE) {
                 sgn0 = bit_select(wb[KB] << 4, wa[KB], 0x0f0f0f0fu);
                 sgn1 = bit_select(wb[KB], wa[KB] >> 4, 0x0f0f0f0fu);
             }
             float2 kn = unpack_half2(lds_u32<KN_OFF>(ring_n + so)), krn = make_float2(0.f, 0.f);
             if constexpr (QJL) krn = unpack_half2(lds_u32<KRN_OFF>(ring_n + so));
-            float s0, s1, s2, s3;   // tokens gid (s0, s1), gid + 8, queries 2 tig (s0, s2), 2 tig + 1
-            if constexpr (INTEGER) {
-                uint32_t ma[4], mb[4];
-                selector_words(wa, ma);
-                selector_words(wb, mb);
-                int hh[4] = {0, 0, 0, 0}, mid[4] = {0, 0, 0, 0}, nh[4] = {0, 0, 0, 0}, nl[4] = {0, 0, 0, 0};
-                auto look = [&](const uint32_t (&t)[2], uint32_t m) { return prmt(t[0], t[1], m); };
-                auto eight_dims = [&](auto word) {
+            float sm[4] = {0.f, 0.f, 0.f, 0.f};
+            float sq[4] = {sq_init0, sq_init1, sq_init0, sq_init1}, sq2[4] = {0.f, 0.f, 0.f, 0.f};
+            auto sign_term = [&](auto quarter) {   // eight dims of two tokens, two products
+                constexpr int C = decltype(quarter)::value;
+                if constexpr (SIGN_TABLE) {
+                    const uint4 g0 = table_signs<C>(sgn0, slut), g1 = table_signs<C>(sgn1, slut);
+                    mma_f16_16816(sq, g0.x, g0.y, g0.z, g0.w, qf[4 * C], qf[4 * C + 1]);
+                    mma_f16_16816(sq2, g1.x, g1.y, g1.z, g1.w, qf[4 * C + 2], qf[4 * C + 3]);
+                } else if constexpr (QJL) {
+                    const uint32_t xa = wa[KB] << (4 * C), xb = wb[KB] << (4 * C);
+                    mma_f16_16816(sq, and_or(xa, 0x80008000u, 0x3C003C00u), and_or(xb, 0x80008000u, 0x3C003C00u),
+                                  and_bits(xa, 0x40004000u), and_bits(xb, 0x40004000u), qpf[4 * C], qpf[4 * C + 1]);
+                    mma_f16_16816(sq2, and_bits(xa, 0x20002000u), and_bits(xb, 0x20002000u), and_bits(xa, 0x10001000u),
+                                  and_bits(xb, 0x10001000u), qpf[4 * C + 2], qpf[4 * C + 3]);
+                }
+            };
+            if constexpr (KB == 2) {
+                // An entry holds two half2.  Its byte is made of the pair of indices of token A and that of token B, so that
+                // the two are neighbouring registers of the A operand.
+                auto quads = [&](auto word) {
                     constexpr int J = decltype(word)::value;
-                    const uint32_t ua = ma[J] >> 16, ub = mb[J] >> 16;
-                    const uint32_t h0 = look(chi, ma[J]), h1 = look(chi, mb[J]), h2 = look(chi, ua), h3 = look(chi, ub);
-                    mma_s8_16832(hh, h0, h1, h2, h3, qf[2 * J], qf[2 * J + 1]);
-                    mma_s8_16832(mid, h0, h1, h2, h3, qf[8 + 2 * J], qf[8 + 2 * J + 1]);
-                    mma_s8_16832(mid, look(clo, ma[J]), look(clo, mb[J]), look(clo, ua), look(clo, ub), qf[2 * J], qf[2 * J + 1]);
-                    if constexpr (QJL) {
-                        const uint2 g0 = table_quad<J>(sgn0, slut), g1 = table_quad<J>(sgn1, slut);
-                        const uint32_t* f = qf;
-                        if constexpr (!ONE_QUERY) f = qpf;
-                        mma_s8_16832(nh, g0.x, g0.y, g1.x, g1.y, f[2 * J], f[2 * J + 1]);
-                        mma_s8_16832(nl, g0.x, g0.y, g1.x, g1.y, f[8 + 2 * J], f[8 + 2 * J + 1]);
-                    }
+                    const uint32_t y0 = bit_select(wb[J] << 2, wa[J], 0x33333333u), y1 = bit_select(wb[J], wa[J] >> 2, 0x33333333u);
+                    auto product = [&](auto first, uint32_t y, int c) {
+                        constexpr int B = decltype(first)::value;
+                        const uint2 a = table_quad<B>(y, klut), b = table_quad<B + 1>(y, klut);
+                        mma_f16_16816(sm, a.x, a.y, b.x, b.y, qf[8 * J + c], qf[8 * J + c + 1]);
+                    };
+                    product(std::integral_constant<int, 0>{}, y0, 0);
+                    product(std::integral_constant<int, 0>{}, y1, 4);
+                    sign_term(std::integral_constant<int, 2 * J>{});
+                    product(std::integral_constant<int, 2>{}, y0, 2);
+                    product(std::integral_constant<int, 2>{}, y1, 6);
+                    sign_term(std::integral_constant<int, 2 * J + 1>{});
+                };
+                quads(std::integral_constant<int, 0>{});
+                quads(std::integral_constant<int, 1>{});
+            } else {
+                uint32_t mwa[4], mwb[4];
+                table_words<KB>(wa, mwa);
+                table_words<KB>(wb, mwb);
+                auto eight_dims = [&](auto word) {
+                    constexpr int C = decltype(word)::value;
+                    const uint32_t a0 = table_pair<0>(mwa[C], klut), a1 = table_pair<1>(mwa[C], klut);
+                    const uint32_t b0 = table_pair<0>(mwb[C], klut), b1 = table_pair<1>(mwb[C], klut);
+                    mma_f16_16816(sm, a0, b0, a1, b1, qf[4 * C], qf[4 * C + 1]);
+                    const uint32_t a2 = table_pair<2>(mwa[C], klut), a3 = table_pair<3>(mwa[C], klut);
+                    const uint32_t b2 = table_pair<2>(mwb[C], klut), b3 = table_pair<3>(mwb[C], klut);
+                    mma_f16_16816(sm, a2, b2, a3, b3, qf[4 * C + 2], qf[4 * C + 3]);
+                    sign_term(word);
                 };
                 eight_dims(std::integral_constant<int, 0>{});
                 eight_dims(std::integral_constant<int, 1>{});
                 eight_dims(std::integral_constant<int, 2>{});
                 eight_dims(std::integral_constant<int, 3>{});
-                auto sum = [](int hi, int lo) { return static_cast<float>(hi * 256 + lo); };
-                s0 = unit0 * sum(hh[0], mid[0]) * kn.x;
-                s1 = unit1 * sum(hh[1], mid[1]) * kn.x;
-                s2 = unit0 * sum(hh[2], mid[2]) * kn.y;
-                s3 = unit1 * sum(hh[3], mid[3]) * kn.y;
-                if constexpr (QJL) {
-                    s0 = fmaf(sign_unit0 * sum(nh[0], nl[0]), krn.x, s0);
-                    s1 = fmaf(sign_unit1 * sum(nh[1], nl[1]), krn.x, s1);
-                    s2 = fmaf(sign_unit0 * sum(nh[2], nl[2]), krn.y, s2);
-                    s3 = fmaf(sign_unit1 * sum(nh[3], nl[3]), krn.y, s3);
-                }
-            } else {
-                float sm[4] = {0.f, 0.f, 0.f, 0.f};
-                float sq[4] = {sq_init0, sq_init1, sq_init0, sq_init1}, sq2[4] = {0.f, 0.f, 0.f, 0.f};
-                auto sign_term = [&](auto quarter) {   // eight dims of two tokens, two products
-                    constexpr int C = decltype(quarter)::value;
-                    if constexpr (SIGNS) {
-                        const uint4 g0 = table_signs<C>(sgn0, slut), g1 = table_signs<C>(sgn1, slut);
-                        mma_f16_16816(sq, g0.x, g0.y, g0.z, g0.w, qf[4 * C], qf[4 * C + 1]);
-                        mma_f16_16816(sq2, g1.x, g1.y, g1.z, g1.w, qf[4 * C + 2], qf[4 * C + 3]);
-                    } else if constexpr (QJL) {
-                        const uint32_t xa = wa[KB] << (4 * C), xb = wb[KB] << (4 * C);
-                        mma_f16_16816(sq, and_or(xa, 0x80008000u, 0x3C003C00u), and_or(xb, 0x80008000u, 0x3C003C00u),
-                                      and_bits(xa, 0x40004000u), and_bits(xb, 0x40004000u), qpf[4 * C], qpf[4 * C + 1]);
-                        mma_f16_16816(sq2, and_bits(xa, 0x20002000u), and_bits(xb, 0x20002000u), and_bits(xa, 0x10001000u),
-                                      and_bits(xb, 0x10001000u), qpf[4 * C + 2], qpf[4 * C + 3]);
-                    }
-                };
-                if constexpr (KB == 2) {
-                    // An entry holds two half2.  Its byte is made of the pair of indices of token A and that of token B, so that
-                    // the two are neighbouring registers of the A operand.
-                    auto quads = [&](auto word) {
-                        constexpr int J = decltype(word)::value;
-                        const uint32_t y0 = bit_select(wb[J] << 2, wa[J], 0x33333333u), y1 = bit_select(wb[J], wa[J] >> 2, 0x33333333u);
-                        auto product = [&](auto first, uint32_t y, int c) {
-                            constexpr int B = decltype(first)::value;
-                            const uint2 a = table_quad<B>(y, klut), b = table_quad<B + 1>(y, klut);
-                            mma_f16_16816(sm, a.x, a.y, b.x, b.y, qf[8 * J + c], qf[8 * J + c + 1]);
-                        };
-                        product(std::integral_constant<int, 0>{}, y0, 0);
-                        product(std::integral_constant<int, 0>{}, y1, 4);
-                        sign_term(std::integral_constant<int, 2 * J>{});
-                        product(std::integral_constant<int, 2>{}, y0, 2);
-                        product(std::integral_constant<int, 2>{}, y1, 6);
-                        sign_term(std::integral_constant<int, 2 * J + 1>{});
-                    };
-                    quads(std::integral_constant<int, 0>{});
-                    quads(std::integral_constant<int, 1>{});
-                } else {
-                    uint32_t mwa[4], mwb[4];
-                    table_words<KB>(wa, mwa);
-                    table_words<KB>(wb, mwb);
-                    auto eight_dims = [&](auto word) {
-                        constexpr int C = decltype(word)::value;
-                        const uint32_t a0 = table_pair<0>(mwa[C], klut), a1 = table_pair<1>(mwa[C], klut);
-                        const uint32_t b0 = table_pair<0>(mwb[C], klut), b1 = table_pair<1>(mwb[C], klut);
-                        mma_f16_16816(sm, a0, b0, a1, b1, qf[4 * C], qf[4 * C + 1]);
-                        const uint32_t a2 = table_pair<2>(mwa[C], klut), a3 = table_pair<3>(mwa[C], klut);
-                        const uint32_t b2 = table_pair<2>(mwb[C], klut), b3 = table_pair<3>(mwb[C], klut);
-                        mma_f16_16816(sm, a2, b2, a3, b3, qf[4 * C + 2], qf[4 * C + 3]);
-                        sign_term(word);
-                    };
-                    eight_dims(std::integral_constant<int, 0>{});
-                    eight_dims(std::integral_constant<int, 1>{});
-                    eight_dims(std::integral_constant<int, 2>{});
-                    eight_dims(std::integral_constant<int, 3>{});
-                }
-                kn.x *= p.qscale;
-                kn.y *= p.qscale;
-                s0 = sm[0] * kn.x;
-                s1 = sm[1] * kn.x;
-                s2 = sm[2] * kn.y;
-                s3 = sm[3] * kn.y;
-                if constexpr (QJL) {
-                    krn.x *= qpscale;
-                    krn.y *= qpscale;
-                    s0 = fmaf(sq[0] + sq2[0], krn.x, s0);
-                    s1 = fmaf(sq[1] + sq2[1], krn.x, s1);
-                    s2 = fmaf(sq[2] + sq2[2], krn.y, s2);
-                    s3 = fmaf(sq[3] + sq2[3], krn.y, s3);
-                }
+            }
+            kn.x *= p.qscale;
+            kn.y *= p.qscale;
+            // tokens gid (s0, s1), gid + 8, queries 2 tig (s0, s2), 2 tig + 1
+            float s0 = sm[0] * kn.x, s1 = sm[1] * kn.x, s2 = sm[2] * kn.y, s3 = sm[3] * kn.y;
+            if constexpr (QJL) {
+                krn.x *= qpscale;
+                krn.y *= qpscale;
+                s0 = fmaf(sq[0] + sq2[0], krn.x, s0);
+                s1 = fmaf(sq[1] + sq2[1], krn.x, s1);
+                s2 = fmaf(sq[2] + sq2[2], krn.y, s2);
+                s3 = fmaf(sq[3] + sq2[3], krn.y, s3);
             }
             const int valid_tokens = len - (page + j) * kPageTokens;
             if constexpr (PARTLY) {
@@ -880,7 +727,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
         }
         if ((run & 1) != (warp >> 3)) continue;
         const int g = warp & 7;
-        auto ring_of = [&](int w) { return smem_u32(smem) + TABLES * kStreamTable + w * RING; };
+        auto ring_of = [&](int w) { return smem_u32(smem) + 2 * kStreamTable + w * RING; };
         // lane e holds (maximum, denominator) of entry e
         float2 ml = make_float2(-INFINITY, 0.f);
         if ((mine >> lane) & 1u) {
@@ -931,13 +778,13 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
     if (threadIdx.x == 0 && !split) sp.split[blockIdx.x].z = -1;
 }
 
-template <int KB, int VB, bool QJL, bool SPARSE, bool ONE_QUERY>
+template <int KB, int VB, bool QJL, bool SPARSE, bool SIGN_TABLE>
 int launch_stream_as(const StreamParams& sp, cudaStream_t stream) {
-    auto kern = decode_stream_kernel<KB, VB, QJL, SPARSE, ONE_QUERY>;
+    auto kern = decode_stream_kernel<KB, VB, QJL, SPARSE, SIGN_TABLE>;
     static bool configured[64] = {};
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return TQ_ERR_LAUNCH;
-    constexpr int smem = stream_smem(stream_integer(KB, SPARSE) && !QJL ? 1 : 2, kStreamStages * page_bytes(KB, VB, QJL ? 1 : 0));
+    constexpr int smem = stream_smem(kStreamStages * page_bytes(KB, VB, QJL ? 1 : 0));
     if (!configured[dev]) {
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return TQ_ERR_LAUNCH;
         configured[dev] = true;
@@ -947,8 +794,8 @@ int launch_stream_as(const StreamParams& sp, cudaStream_t stream) {
 
 template <int KB, int VB, bool QJL, bool SPARSE>
 int launch_stream(const StreamParams& sp, cudaStream_t stream) {
-    if constexpr (QJL && (stream_integer(KB, SPARSE) || KB == VB)) {
-        if (!sp.d.qp && (stream_integer(KB, SPARSE) || sp.d.share_tables)) return launch_stream_as<KB, VB, QJL, SPARSE, true>(sp, stream);
+    if constexpr (QJL && KB == VB) {
+        if (sp.d.share_tables && !sp.d.qp) return launch_stream_as<KB, VB, QJL, SPARSE, true>(sp, stream);
     }
     return launch_stream_as<KB, VB, QJL, SPARSE, false>(sp, stream);
 }
