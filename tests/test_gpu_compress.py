@@ -147,6 +147,31 @@ def test_compress_contiguous_large_tight_codebook_and_nonfinite_rows(rotate):
         assert not torch.isfinite(k_n[17].float()) and not torch.isfinite(k_n[n - 1].float())
 
 
+@pytest.mark.parametrize("c,b", [([-0.14, -0.045, 0.04, 0.13], [-0.09, -0.004, 0.085]),        # nothing symmetric
+                                 ([-0.13, -0.04, 0.04, 0.13], [-0.088, 0.0, 0.0851]),         # boundaries are not
+                                 ([-0.13, -0.04, 0.04, 0.14], [-0.085, 0.0, 0.085]),          # centroids are not
+                                 ([-0.13, -0.04, 0.04, 0.13], [-0.085, 0.0, 0.085]),
+                                 ([-0.13, -0.04, 0.04, 0.13], [-0.1, 0.1, float("inf")])])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_compress_contiguous_large_two_bit_codebooks_of_any_shape(c, b, dtype):
+    """More than 32768 rotated rows: 2-bit codebooks symmetric about zero are halved twice, others take three comparisons."""
+    n = 33189
+    x, c, b, H = _inputs(n, seed=6).to(dtype), torch.tensor(c), torch.tensor(b), O.make_wht_matrix(128)
+    PiT = make_wht_matrix(128).to(DEV)
+    k_idx, k_sg, k_rn, k_n = packed_compress.compress_k(x.to(DEV), PiT, None, c.to(DEV), b.to(DEV))
+    v_idx, v_n = packed_compress.compress_v(x.to(DEV), PiT, c.to(DEV), b.to(DEV))
+    o_idx, o_sg, o_rn, o_n = O.compress_k_packed(x.float().numpy(), c.numpy(), b.numpy(), 2, H, permuted=False)
+    want = O.unpack_indices(o_idx, 2).astype(int)
+    for idx in (k_idx, v_idx):
+        got = packed_compress.unpack_indices(idx.cpu(), 2).numpy().astype(int)
+        assert (got != want).mean() <= 1e-4 and np.abs(got - want).max() <= 1
+    assert (np.unpackbits(k_sg.cpu().numpy(), axis=1) != np.unpackbits(o_sg, axis=1)).mean() <= 1e-4
+    assert _half_ulp_close(k_n, o_n.astype(np.float32)) and _half_ulp_close(v_n, o_n.astype(np.float32))
+    # a coordinate that the rotation's rounding takes over a boundary which is not half way has another residual
+    same = (packed_compress.unpack_indices(k_idx.cpu(), 2).numpy() == want).all(axis=1)
+    assert _half_ulp_close(k_rn.cpu()[torch.from_numpy(same)], o_rn.astype(np.float32)[same], 2)
+
+
 def test_compress_k_v_general_rotation_and_projection_matrices():
     """The reference's own demo (packed_compress.py:247-275) passes a QR-orthogonal Pi and PiST = Pi S^T with a
     Gaussian S.  Such matrices take the composed path (matrix products around the same quantizer kernels): indices

@@ -170,6 +170,28 @@ def test_two_bit_codebooks_of_any_shape(c, b, dtype):
     assert all(torch.equal(got[n][keep], dirty[n][keep]) for n in got)
 
 
+@pytest.mark.parametrize("use_qjl", [False, True])
+@pytest.mark.parametrize("b", [[-0.1, 0.1, float("inf")], [-0.1, 0.1, 5.0], [float("-inf"), -0.1, 0.1], [-5.0, -0.1, 0.1],
+                               [-5.0, 0.0, 5.0], [float("-inf"), 0.0, float("inf")], [0.05, float("inf"), float("inf")]])
+def test_two_bit_codebooks_padded_with_boundaries_out_of_reach(b, use_qjl):
+    """Ascending boundaries of which some lie where no coordinate does, symmetric centroids: the indices follow the others."""
+    fmt = CacheFormat(2, 2, use_qjl)
+    c, b = torch.tensor([-0.13, -0.04, 0.04, 0.13]), torch.tensor(b)
+    books = Codebooks(fmt, DEV, k_codebook=(c, b), v_codebook=(c, b))
+    key, val = _kv(T_BIG, HKV, torch.float16, seed=73)
+    got, status, _ = _run(key, val, fmt, books)
+    assert status == 0
+    ok, ov = _oracle(key, val, fmt, books, O.make_wht_matrix(128))
+    for name, want in (("v_idx", ov), ("k_idx", ok)):
+        idx = got[name].numpy().reshape(-1, 128).astype(int)
+        assert (idx != want["indices"]).mean() <= 1e-4 and np.abs(idx - want["indices"]).max() <= 1
+    if use_qjl:
+        assert (got["k_signs"].numpy().reshape(-1, 128) != (ok["signs"] > 0)).mean() <= 1e-4
+        # a coordinate that the rotation's rounding takes over a boundary which is not half way has another residual
+        same = (idx == ok["indices"]).all(axis=1)
+        assert _fp16_ulps(got["k_rnorm"].reshape(-1)[torch.from_numpy(same)], ok["rot_residual_norm"][same]) <= 2
+
+
 @pytest.mark.parametrize("dtype,prerotated,tcgen05", [(torch.float16, False, False), (torch.bfloat16, False, False),
                                                       (torch.float32, False, False), (torch.float16, True, False),
                                                       (torch.float16, False, True), (torch.bfloat16, False, True)])

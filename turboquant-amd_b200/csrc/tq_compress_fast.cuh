@@ -259,7 +259,8 @@ struct Comparisons2 {
 // 2 bits, halving the codebook twice: t = [u > b_1], then t' = [u > b_0] or [u > b_2], idx = 2 t + t'.  The second boundary is a
 // multiply-add away from the first, and the step to the second centroid of either half is the same, in a codebook symmetric about
 // zero; `split` says that these sums give what the comparisons give.  Any other codebook takes the comparisons as they are, whose
-// constants wait in shared memory.
+// constants wait in shared memory; also one with a boundary at or near infinity (a padded codebook), as 0 times an infinite distance
+// would be NaN.
 template <>
 struct Codebook2<2> {
     float nb_1;                          // -b_j * 2^126
@@ -278,7 +279,8 @@ struct Codebook2<2> {
         __syncwarp();
         comparisons = of_warp;
         const float db = centroid_step(-k.nb[0], -k.nb[2]), n2 = (k.nc0 + k.nc[0]) + k.nc[1];
-        split = __all_sync(0xffffffffu, k.nb[0] >= k.nb[1] && k.nb[1] >= k.nb[2] && k.nb[0] + db == k.nb[2] && n2 + k.nc[0] == n2 + k.nc[2]);
+        split = __all_sync(0xffffffffu, k.nb[0] >= k.nb[1] && k.nb[1] >= k.nb[2] && k.nb[0] + db == k.nb[2] && n2 + k.nc[0] == n2 + k.nc[2] &&
+                                     fabsf(db) < INFINITY && fabsf(n2 + k.nc[0]) < INFINITY);
         nb_1 = k.nb[1];
         nb_0 = f2dup(k.nb[0]);
         nb_0to2 = f2dup(db);
