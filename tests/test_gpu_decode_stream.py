@@ -254,3 +254,36 @@ def test_scores_of_uneven_queries(kb, vb, qjl, form, dtype):
             assert out[0, 9].isnan().all()
             out[0, 9] = got[0, 9]
             assert torch.equal(out, got)
+
+
+@pytest.mark.parametrize("kb,vb", [(2, 2), (3, 3), (4, 4)])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("kw", [dict(), dict(chunk_pages=64), dict(chunk_pages=64, sparse_thresh=1e-6)])
+@pytest.mark.parametrize("separate", [False, True])
+def test_sign_term_of_large_queries(kb, vb, dtype, kw, separate):
+    """Coordinates beyond 255, at each of the four places that the one-sided sign forms treat differently: no overflow to NaN.
+    The scores reach thousands, so one rounding in 32 bits moves a weight by up to 5e-4; next to that weights and output are rounded
+    to 11 bits (bf16: the output to 8)."""
+    fmt = CacheFormat(kb, vb, True)
+    books = Codebooks(fmt, DEV)
+    ns, hkv = len(LONG), 4
+    bt, blocks = _tables(LONG, 16, 6)
+    cache = _random_cache(fmt, blocks, hkv, 16, 5)
+    g = torch.Generator(device=DEV).manual_seed(2)
+
+    def make():
+        q = torch.randn(ns, hkv, 8, 128, generator=g, device=DEV)
+        for head, dim, value in ((1, 16, 254), (2, 16, 256), (3, 17, 300), (4, 31, 1000), (5, 18, 30000), (6, 16, -40000)):
+            q[:, :, head, dim] = value
+        q[:, :, 7] *= 80
+        q[:, :, 7, 100] = 290
+        return q.to(dtype)
+
+    q = make()
+    qp = make() if separate else q
+    out = paged_decode_attention(q.view(ns, -1, 128), cache, bt.to(DEV), torch.tensor(LONG, dtype=torch.int32, device=DEV), books, 16,
+                                 q_proj=qp.view(ns, -1, 128) if separate else None, **kw)
+    assert _native.read_status(DEV) == 0
+    ref = torch.stack([_attend64(q[i], qp[i], cache, bt[i, :-(-n // 16)], books, 16, n, hkv) for i, n in enumerate(LONG)])
+    error = (out.double().view(ref.shape) - ref).pow(2).sum(dim=(0, 1, 3)).sqrt() / ref.pow(2).sum(dim=(0, 1, 3)).sqrt()
+    assert (error <= (2e-3 if dtype == torch.float16 else 4e-3)).all(), error

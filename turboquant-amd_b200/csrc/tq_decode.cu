@@ -160,7 +160,7 @@ __device__ __forceinline__ uint2 lut_quad(uint32_t lane_base, uint32_t w, int k)
 // 2 * [s >= 0] = sigma + 1, the query operand of those slots is pre-scaled (1, 2^8, 2^12) and
 // the constant sum of the query over those dims is subtracted once (accumulator start value).
 // Form 0 yields -sigma, so its query operand is negated.  All query operands carry 1/16 to keep
-// 2^12 * q inside fp16; the factor 16 is folded into the fp32 scale of the residual norm.
+// 2^12 * q inside fp16 (rows with larger values: fit_sign_rows); the factor 16 is folded into the fp32 scale of the residual norm.
 // This lane's 32 query values (dims 32 * tig .. 32 * tig + 31 of query row gid) as fp32; zeros when !valid.
 __device__ __forceinline__ void load_q32(const void* q, int64_t row_off, int tig, int io_dtype, bool valid, float (&x)[32]) {
     if (!valid) {
@@ -217,6 +217,30 @@ __device__ __forceinline__ void qp_frag_signed_from(const float (&x)[32], uint32
             if (form) correction += (x[j] + x[j + 16]) * (1.f / 16.f);
         }
     }
+}
+
+// The coefficients of 16 and 256 (dims 4 i + 1 and 4 i) take values of 255 and more out of fp16's range, and infinity times an absent
+// sign is NaN.  A row that has such a value there goes in divided by 256: with the smallest coefficient this rounds coordinates below
+// 1/4 to multiples of 2^-12, 2^-20 of the largest one or less.  Returns the lanes of divided rows.  (A launch of few pages
+// pays 0.04 us of 7.6 for it; 0.13 with the maximum as a chain instead of a tree, and ahead of the tables' barrier.)
+__device__ __forceinline__ uint32_t fit_sign_rows(float (&x)[32], int lane) {
+    float most[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) most[i] = fmaxf(fabsf(x[4 * i]), fabsf(x[4 * i + 1]));
+#pragma unroll
+    for (int h = 4; h > 0; h >>= 1)
+#pragma unroll
+        for (int i = 0; i < h; ++i) most[i] = fmaxf(most[i], most[i + h]);
+    const uint32_t over = __ballot_sync(0xffffffffu, most[0] >= 255.f);
+    if (!over) return 0;
+    const bool row_over = (over >> (lane & 28)) & 15;
+#pragma unroll
+    for (int i = 0; i < 32; ++i) x[i] *= row_over ? 1.f / 256.f : 1.f;
+    return __ballot_sync(0xffffffffu, row_over);
+}
+// What the sign sums of queries 2 tig, 2 tig + 1 are multiplied by then.
+__device__ __forceinline__ float2 divided_by(uint32_t rows, int tig) {
+    return make_float2((rows >> (8 * tig)) & 1 ? 256.f : 1.f, (rows >> (8 * tig + 4)) & 1 ? 256.f : 1.f);
 }
 
 // Shared-memory loads by 32-bit shared address + compile-time offset (one add per page and access pattern instead
@@ -394,9 +418,11 @@ __global__ void __launch_bounds__(kThreads, TQ_DEC_MINBLOCKS) decode_partial_ker
     fill_pair_lut<KB>(tabk, ck, warp, lane);
     if (!p.share_tables) fill_pair_lut<VB>(tabv, cv, warp, lane);
 
+    __syncthreads();   // the pair tables are there; the query's operands are made while the first pages are under way
     // ---- query fragments -------------------------------------------------------------------------------
     uint32_t qf[16], qpf[QJL ? 16 : 1];
     float sq_init0 = 0.f, sq_init1 = 0.f;   // minus the query sums of the one-sided sign forms
+    float qpscale0 = 0.f, qpscale1 = 0.f;   // of queries 2 tig, 2 tig + 1
     {
         const bool valid = g_in_group < p.G;
         const int64_t row = (static_cast<int64_t>(seq) * p.Hq + head0 + gid) * kHeadDim;
@@ -405,6 +431,9 @@ __global__ void __launch_bounds__(kThreads, TQ_DEC_MINBLOCKS) decode_partial_ker
         if constexpr (QJL) {
             if (p.qp) load_q32(p.qp, row, tig, p.io_dtype, valid, xq);   // S q' given separately
             float corr;
+            const float2 by = divided_by(fit_sign_rows(xq, lane), tig);
+            qpscale0 = by.x * p.qpscale;
+            qpscale1 = by.y * p.qpscale;
             qp_frag_signed_from(xq, qpf, corr);
             corr += __shfl_xor_sync(0xffffffffu, corr, 1);
             corr += __shfl_xor_sync(0xffffffffu, corr, 2);      // total over the 128 dims of query gid
@@ -413,7 +442,6 @@ __global__ void __launch_bounds__(kThreads, TQ_DEC_MINBLOCKS) decode_partial_ker
         }
     }
 
-    __syncthreads();   // the pair tables are there
     const uint32_t klut = smem_u32(tabk) + (KB == 2 ? 8 * (lane & 15) : 4 * lane);
     const uint32_t vlut = smem_u32(tabv) + (VB == 2 ? 8 * (lane & 15) : 4 * lane);
     // this lane's three access patterns inside a ring stage: its two K records, the norm slots, the V words

@@ -398,6 +398,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
 
         uint32_t qf[16], qpf[QJL && !SIGN_TABLE ? 16 : 1];
         float sq_init0 = 0.f, sq_init1 = 0.f;   // minus the query sums of the one-sided sign forms
+        uint32_t divided = 0;                   // queries whose one-sided sign operands are divided by 256
         {
             float xq[32];
             load_q32(p.q, row, tig, p.io_dtype, gid < nq, xq);
@@ -406,6 +407,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
             if constexpr (QJL && !SIGN_TABLE) {
                 if (p.qp) load_q32(p.qp, row, tig, p.io_dtype, gid < nq, xq);
                 float corr;
+                divided = fit_sign_rows(xq, lane);
                 qp_frag_signed_from(xq, qpf, corr);
                 corr += __shfl_xor_sync(0xffffffffu, corr, 1);
                 corr += __shfl_xor_sync(0xffffffffu, corr, 2);
@@ -423,8 +425,8 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
 #pragma unroll
             for (int r = 0; r < 4; ++r) oacc[i][r] = 0.f;
 
-        auto one_page = [&](auto have_v, auto partly, int j) {
-            constexpr bool HAVE_V = decltype(have_v)::value, PARTLY = decltype(partly)::value;
+        auto one_page = [&](auto have_v, auto partly, auto large, int j) {
+            constexpr bool HAVE_V = decltype(have_v)::value, PARTLY = decltype(partly)::value, LARGE = decltype(large)::value;
             const uint32_t so = stage * PAGE;
             wait_copies<NSTAGE - 1>();
             __syncwarp();
@@ -501,10 +503,18 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
             if constexpr (QJL) {
                 krn.x *= qpscale;
                 krn.y *= qpscale;
-                s0 = fmaf(sq[0] + sq2[0], krn.x, s0);
-                s1 = fmaf(sq[1] + sq2[1], krn.x, s1);
-                s2 = fmaf(sq[2] + sq2[2], krn.y, s2);
-                s3 = fmaf(sq[3] + sq2[3], krn.y, s3);
+                float t0 = sq[0] + sq2[0], t1 = sq[1] + sq2[1], t2 = sq[2] + sq2[2], t3 = sq[3] + sq2[3];
+                if constexpr (LARGE) {
+                    const float2 by = divided_by(divided, tig);
+                    t0 *= by.x;
+                    t1 *= by.y;
+                    t2 *= by.x;
+                    t3 *= by.y;
+                }
+                s0 = fmaf(t0, krn.x, s0);
+                s1 = fmaf(t1, krn.x, s1);
+                s2 = fmaf(t2, krn.y, s2);
+                s3 = fmaf(t3, krn.y, s3);
             }
             const int valid_tokens = len - (page + j) * kPageTokens;
             if constexpr (PARTLY) {
@@ -630,17 +640,21 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
             copies_end();
             if (++stage == NSTAGE) stage = 0;
         };
-        auto next_page = [&](auto partly, int j) {
+        auto next_page = [&](auto partly, auto large, int j) {
             if constexpr (SPARSE) {
-                if (k_only == 0 || !((k_only >> stage) & 1u)) one_page(std::true_type{}, partly, j);
-                else one_page(std::false_type{}, partly, j);
+                if (k_only == 0 || !((k_only >> stage) & 1u)) one_page(std::true_type{}, partly, large, j);
+                else one_page(std::false_type{}, partly, large, j);
             } else {
-                one_page(std::true_type{}, partly, j);
+                one_page(std::true_type{}, partly, large, j);
             }
         };
         const int full = min(seg, (len >> 4) - page);   // at most the last page of a sequence is partly filled
-        for (int j = 0; j < full; ++j) next_page(std::false_type{}, j);
-        if (full < seg) next_page(std::true_type{}, full);
+        auto pages = [&](auto large) {
+            for (int j = 0; j < full; ++j) next_page(std::false_type{}, large, j);
+            if (full < seg) next_page(std::true_type{}, large, full);
+        };
+        if (QJL && !SIGN_TABLE && divided) pages(std::bool_constant<QJL && !SIGN_TABLE>{});
+        else pages(std::false_type{});
 
         // ---- the item's result, or this warp's part of it
 #pragma unroll
