@@ -40,8 +40,9 @@ namespace {
 
 // What bounds it: issue (58 to 63 % of the cycles with 16 warps per SM, which is what 128 registers allow; a build at 80
 // registers and 24 warps per SM spilled and measured 1.3-1.6x slower), so what counts is how many instructions an item takes: 108 with
-// 2 bits (133 before indices and centroids went two to an instruction), us for 8 KV heads: 1 M tokens of turbo2 1505 -> 1420, and
-// 1368 with the slots requested a key ahead of their use; 256 K of turbo3 416 -> 381 -> 378, of turbo4 351 -> 340 -> 335.
+// 2 bits (133 before indices and centroids went two to an instruction), us in a graph for 8 KV heads: 1 M tokens of turbo2
+// 1505 -> 1420, and 1368 with the slots requested a key ahead of their use (single calls 1615 -> 1520); 256 K of turbo3 416 -> 381
+// -> 377, of turbo4 351 -> 340 -> 336 to 346.
 // One CTA of 16 warps per SM builds the tables once for all of them: 4 % faster than two CTAs of 8 warps.
 #ifndef TQ_CMP_MINBLOCKS
 #define TQ_CMP_MINBLOCKS 1
@@ -122,7 +123,8 @@ __device__ __forceinline__ int scan_cell(int cell, const float* __restrict__ b, 
     return inside;
 }
 
-// d with -c_lo + d == -c_hi in fp32: the rounded difference, or one of its neighbours.
+// d with -c_lo + d == -c_hi in fp32, to within an ulp: the rounded difference, or its neighbour against the error.  There need be no
+// exact one where c_hi has finer ulps than the sum; the residual then sees a centroid one ulp away.
 __device__ __forceinline__ float centroid_step(float c_lo, float c_hi) {
     float d = c_lo - c_hi;
     const float off = (d - c_lo) + c_hi;
@@ -249,9 +251,7 @@ __device__ __forceinline__ void quant_pair(f2 y, const VecConsts& vc, f2& rr, ui
 
 // The same for rows rotated here: u is the plain product, residuals are not yet multiplied by the norm.
 template <int BITS>
-struct Codebook2 {   // 3 and 4 bits: everything is in the table
-    static constexpr bool split = true;
-};
+struct Codebook2 {};   // 3 and 4 bits: everything is in the table
 // 2 bits by three comparisons: -b_j * 2^126; -c_0 and the steps from -c_(j-1) to -c_j.
 struct Comparisons2 {
     float nb[3], nc0, nc[3];

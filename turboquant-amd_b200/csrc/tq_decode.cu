@@ -755,12 +755,13 @@ int dispatch_v(const DecodeParams& p, int vb, const Plan& plan, cudaStream_t str
 // Which kernel is the better one, by the pages that the batch can have at most.  The persistent kernel pays about 11 us
 // however few pages there are (all its tables, one more level of merging), the chunked one 5 to 9, but it takes
 // 0.45 (4-bit) to 0.55 us (with sign term) per 1000 pages where the chunked one takes 0.7 to 0.8; sequences of few pages
-// cost it more, a warp then changes item every few pages.  Measured us, chunked / persistent, 8 KV heads, turbo4 and turbo3:
-// 1 x 16384 tokens (8192 pages) 14.6 / 16.1 and 14.1 / 16.8; 24 x 1024 (12288) 15.9 / 18.2 and 22.1 / 19.5; 64 x 512 (16384)
-// 19.1 / 20.6 and 19.4 / 22.2, 32 x 1024 22.8 / 19.4 and 22.9 / 20.9; 256 x 256 (32768) 35.3 / 32.9 and 36.4 / 36.2, 128 x 512
-// 30.2 / 30.1 and 31.9 / 33.1; 32 x 3000 (48128) 48.0 / 35.1 and 51.3 / 39.1.  The line does not look at the format: it is
-// off by 4 to 13 % for 24 x 1024 and 128 x 512 with sign term.  (Since these were taken the persistent kernel became 3 to 6 % faster:
-// turbo4 128 x 512 28.8, turbo3 31.9, 256 x 256 32.1 and 34.9.)
+// cost it more, a warp then changes item every few pages.  Measured with both as they are, us per launch in a graph over caches that
+// L2 does not hold, chunked / persistent, 8 KV heads, turbo4 and turbo3: 16 x 512 tokens (4096 pages) 10.6 / 12.5 and
+// 13.6 / 13.0; 1 x 16384 (8192) 14.8 / 16.0 and 13.9 / 16.7, 32 x 512 16.2 / 15.4 and 15.5 / 16.3; 24 x 1024 (12288) 15.8 / 18.8
+// and 21.8 / 20.2; 64 x 512 (16384) 19.2 / 21.3 and 19.3 / 22.9, 32 x 1024 22.8 / 20.2 and 22.9 / 21.8; 256 x 256 (32768)
+// 37.0 / 34.1 and 36.6 / 36.8, 128 x 512 31.9 / 30.9 and 32.0 / 33.8; 32 x 3000 (48128) 47.9 / 34.6 and 50.9 / 39.2.  The line does
+// not look at the format or at how the chunks come out: the other kernel is 4 to 8 % faster for 16 x 512, 24 x 1024 and
+// 128 x 512 of turbo3, and 5 % for 32 x 512 of turbo4.
 constexpr int64_t kStreamMinPages = 16384;
 constexpr int64_t kStreamSlots = static_cast<int64_t>(kStreamCtas) * (kStreamWarps + 2);   // partials of warps and of CTAs
 int64_t pages_at_most(int64_t ns, int64_t hq, int64_t hkv, int64_t max_pages) { return ns * max_pages * hkv * ((hq / hkv + 7) / 8); }

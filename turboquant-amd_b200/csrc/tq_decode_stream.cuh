@@ -9,14 +9,15 @@
 // Against the chunked kernel (4-warp CTAs, one chunk of one item each) this takes away the last wave that is three
 // quarters full, the table fill, pipeline start and merge per chunk, and the empty CTAs of a ragged batch.
 //
-// What bounds it: instruction issue (about 62 % of the cycles with four warps a scheduler; a tensor instruction costs it about
-// three slots), and the shared-memory data path next to it (turbo3: 82 %).
+// What bounds it: the shared-memory data path (turbo3: 82 % of its peak, 125 wavefronts a page) and, next to it, instruction issue
+// (360 instructions a page, 58 % of the cycles with four warps a scheduler; a tensor instruction costs it about three slots).
 // Pages are staged with cp.async, 16 bytes a lane, into a private ring: a page then costs four copy instructions and a counted
 // wait, where a bulk copy by one elected lane with its barrier cost about 35 instructions.  Together with a page body that has no
 // partly filled pages to look after, table addresses from the multiply-add pipe and loop state in uniform registers, us per
-// launch in a graph of 8 or more over different caches, before / now, 8 KV heads: turbo3 64 x 8192 tokens 151.8 / 145.4, turbo4
-// 1 x 131072 43.5 / 41.5, turbo3 128 x 512 34.8 / 34.1, turbo3 with a query of the sign term's own 32 x 4096 53.3 / 49.4, turbo2 with
-// four heads a group 64 x 4096 74.5 / 75.3; 4 KV heads, 32 x 4096: 3-bit K and 4-bit V 28.1 / 26.6, turbo4 28.2 / 27.1.
+// launch in a graph of 8 or more over different caches, before / now, 8 KV heads: turbo3 64 x 8192 tokens 151.8 / 145.6, turbo4
+// 128.5 / 122.3 and 1 x 131072 43.5 / 41.5, turbo3 128 x 512 34.8 / 34.1, turbo3 with a query of the sign term's own 32 x 4096 53.3 / 49.0;
+// 4 KV heads, 32 x 4096: 3-bit K and 4-bit V 28.1 / 26.6, turbo4 28.2 / 27.1.  Only large turbo2 batches lost: 64 x 8192 134.1 / 134.9
+// (4 KV heads, 32 x 4096: 28.5 / 28.1); norms loaded behind the products or one body for all pages did not bring it back.
 // Two pages per iteration came out the same (the loop's own instructions are few now), and so did V operands without the pairing
 // of tokens (twice the products with half of the weights zero: 19 instructions fewer, 8 products more).
 // 3-bit keys as integer products (m16n8k32: 16-bit queries and centroids as two signed digits, made by byte permutes from the
