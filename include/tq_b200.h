@@ -42,7 +42,9 @@ typedef struct CUstream_st* tq_stream_t; /* same type as cudaStream_t */
 #define TQ_IO_DEROTATE_OUT 0x200 /* write out in original space (out H), as the reference's rotate_output does */
 #define TQ_IO_TCGEN05 0x400      /* run the tensor-memory (tcgen05) variant of the decode kernel where it exists: 2- and
                                     3-bit codebooks without Sparse-V; other formats ignore the flag.  Slower than the
-                                    default kernel on this hardware and held to the same output tolerance. */
+                                    default kernel on this hardware.  The query heads of a group share one scale: held to
+                                    3e-3 + 1.5e-2 |ref| for heads of like size; a head whose query is far smaller than
+                                    another one's of its group loses precision. */
 
 /* Bits set by kernels in the optional device-side status word. */
 #define TQ_COMPRESS_TCGEN05 2 /* flag in tq_compress_paged's `prerotated` argument, see there */
