@@ -161,46 +161,92 @@ __device__ __forceinline__ uint2 lut_quad(uint32_t lane_base, uint32_t w, int k)
 // the constant sum of the query over those dims is subtracted once (accumulator start value).
 // Form 0 yields -sigma, so its query operand is negated.  All query operands carry 1/16 to keep
 // 2^12 * q inside fp16 (rows with larger values: fit_sign_rows); the factor 16 is folded into the fp32 scale of the residual norm.
-// This lane's 32 query values (dims 32 * tig .. 32 * tig + 31 of query row gid) as fp32; zeros when !valid.
-__device__ __forceinline__ void load_q32(const void* q, int64_t row_off, int tig, int io_dtype, bool valid, float (&x)[32]) {
-    if (!valid) {
-#pragma unroll
-        for (int i = 0; i < 32; ++i) x[i] = 0.f;
-        return;
-    }
-    const uint16_t* base = static_cast<const uint16_t*>(q) + row_off + tig * 32;
+// This lane's 32 query values (dims 32 * tig .. 32 * tig + 31 of query row gid) as they are stored, two to a word; zeros when !valid.
+__device__ __forceinline__ void load_q_words(const void* q, int64_t row_off, int tig, bool valid, uint32_t (&w)[16]) {
+    const uint4* base = reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(q) + row_off + tig * 32);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        const uint4 v = __ldg(reinterpret_cast<const uint4*>(base) + i);
-        const uint32_t r[4] = {v.x, v.y, v.z, v.w};
+        const uint4 v = valid ? __ldg(base + i) : make_uint4(0u, 0u, 0u, 0u);
+        w[4 * i] = v.x;
+        w[4 * i + 1] = v.y;
+        w[4 * i + 2] = v.z;
+        w[4 * i + 3] = v.w;
+    }
+}
+__device__ __forceinline__ float2 unpack_bf162(uint32_t x) { return make_float2(__uint_as_float(x << 16), __uint_as_float(x & 0xffff0000u)); }
+// The words' values as fp32.
+__device__ __forceinline__ void unpack_q(const uint32_t (&w)[16], int io_dtype, float (&x)[32]) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            if (io_dtype == TQ_DTYPE_F16) {
-                const float2 t = unpack_half2(r[j]);
-                x[8 * i + 2 * j] = t.x;
-                x[8 * i + 2 * j + 1] = t.y;
-            } else {
-                x[8 * i + 2 * j] = __uint_as_float(r[j] << 16);
-                x[8 * i + 2 * j + 1] = __uint_as_float(r[j] & 0xffff0000u);
+    for (int i = 0; i < 16; ++i) {
+        const float2 t = io_dtype == TQ_DTYPE_F16 ? unpack_half2(w[i]) : unpack_bf162(w[i]);
+        x[2 * i] = t.x;
+        x[2 * i + 1] = t.y;
+    }
+}
+
+template <bool BF16>
+__device__ __forceinline__ void mma_hadamard(float (&d)[4], uint32_t a, uint32_t a3, uint32_t b0, uint32_t b1) {
+    if constexpr (BF16)
+        asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%4,%4,%5}, {%6,%7}, {%8,%8,%8,%8};"
+            : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3]) : "r"(a), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
+    else
+        asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%4,%4,%5}, {%6,%7}, {%8,%8,%8,%8};"
+            : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3]) : "r"(a), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
+}
+// (a, b) -> (a + b, a - b) on two pairs of fp32 at a time.
+__device__ __forceinline__ void butterfly2(float& a0, float& a1, float& b0, float& b1) {
+    asm("{\n\t.reg .b64 a, b, n, s;\n\tmov.b64 a, {%0, %1};\n\tmov.b64 b, {%2, %3};\n\tmov.b64 n, {%4, %4};\n\t"
+        "add.rn.f32x2 s, a, b;\n\tfma.rn.f32x2 a, b, n, a;\n\tmov.b64 {%0, %1}, s;\n\tmov.b64 {%2, %3}, a;\n\t}"
+        : "+f"(a0), "+f"(a1), "+f"(b0), "+f"(b1) : "f"(-1.f));
+}
+// q' = q H for the eight query rows of a warp, from and to the words of load_q_words, rounded to the io dtype as a separate
+// rotation pass writing fp16 / bf16 would.  Four of the seven index bits (dims bits 0, 1, 5 and 6) are one product with a 16 x 16
+// matrix of +-1 per four dims a lane: exact products, fp32 sums.  The other three lie in the eight accumulators of a lane.  What
+// comes out has the queries across a row of four lanes, where the score products want them across the eight: movmatrix.
+// About 110 instructions and no shuffle, against some 400 with 64 shuffles for a butterfly over the lanes, which every warp of a launch
+// of few pages ran cold: us per launch in a graph, butterfly / now, 32 query and 8 KV heads: turbo4 1 x 4096 tokens 7.3 / 6.8,
+// 4 x 1000 7.85 / 6.95, 8 x 2000 15.2 / 14.0; turbo3 1 x 4096 8.3 / 7.65, 16 x 2000 22.3 / 21.3.
+template <bool BF16>
+__device__ __forceinline__ void rotate_q_words_as(uint32_t (&w)[16], int lane) {
+    const int gid = lane >> 2, tig = lane & 3;
+    const uint32_t one = BF16 ? 0x3F803F80u : 0x3C003C00u;
+    const uint32_t a = one ^ ((__popc(gid & (2 * tig)) & 1) << 15) ^ (static_cast<uint32_t>(__popc(gid & (2 * tig + 1))) << 31);
+    float d[8][4];
+#pragma unroll
+    for (int s = 0; s < 8; ++s) mma_hadamard<BF16>(d[s], a, a ^ 0x80008000u, w[2 * s], w[2 * s + 1]);
+#pragma unroll
+    for (int h = 1; h < 8; h <<= 1)
+#pragma unroll
+        for (int s = 0; s < 8; ++s)
+            if (!(s & h)) {
+                butterfly2(d[s][0], d[s][1], d[s + h][0], d[s + h][1]);
+                butterfly2(d[s][2], d[s][3], d[s + h][2], d[s + h][3]);
             }
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+        const float x = d[i >> 1][2 * (i & 1)] * kWhtScale, y = d[i >> 1][2 * (i & 1) + 1] * kWhtScale;
+        uint32_t pair;
+        if constexpr (BF16) {
+            const __nv_bfloat162 r = __floats2bfloat162_rn(x, y);
+            pair = *reinterpret_cast<const uint32_t*>(&r);
+        } else {
+            pair = pack_half2(x, y);
         }
+        w[i] = movmatrix_trans(pair);
     }
 }
-
-// q' = q H for the query row spread over the 4 lanes of a tig group, rounded to the io dtype exactly as
-// a separate rotation pass writing fp16 / bf16 would.
-__device__ __forceinline__ void rotate_q32(float (&x)[32], int lane, int io_dtype) {
-    fwht128(x, lane);
-#pragma unroll
-    for (int i = 0; i < 32; ++i) {
-        const float v = x[i] * kWhtScale;
-        x[i] = io_dtype == TQ_DTYPE_F16 ? __half2float(__float2half_rn(v)) : __bfloat162float(__float2bfloat16_rn(v));
-    }
+__device__ __forceinline__ void rotate_q_words(uint32_t (&w)[16], int lane, int io_dtype) {
+    if (io_dtype == TQ_DTYPE_F16) rotate_q_words_as<false>(w, lane);
+    else rotate_q_words_as<true>(w, lane);
 }
-
-__device__ __forceinline__ void q_frag_from(const float (&x)[32], uint32_t (&f)[16]) {
+// The words as fp16, the operands of the score products.
+__device__ __forceinline__ void q_words_to_half(uint32_t (&w)[16], int io_dtype) {
+    if (io_dtype == TQ_DTYPE_F16) return;
 #pragma unroll
-    for (int i = 0; i < 16; ++i) f[i] = pack_half2(x[2 * i], x[2 * i + 1]);
+    for (int i = 0; i < 16; ++i) {
+        const float2 t = unpack_bf162(w[i]);
+        w[i] = pack_half2(t.x, t.y);
+    }
 }
 
 // Query operands of the sign term (see above): per MMA m and slot, half2 of dims (j, j + 16) times the
@@ -346,8 +392,8 @@ __global__ void __launch_bounds__(kThreads, TQ_DEC_MINBLOCKS) decode_partial_ker
     const int nq = min(8, p.G - qg * 8);                // live query heads in this CTA
     const int head0 = kvh * p.G + qg * 8;
     const float ck = lane_centroid<KB>(p.kc, lane), cv = lane_centroid<VB>(p.vc, lane);
-    float xq[32];
-    load_q32(p.q, (static_cast<int64_t>(seq) * p.Hq + head0 + gid) * kHeadDim, tig, p.io_dtype, g_in_group < p.G, xq);
+    uint32_t qf[16];
+    load_q_words(p.q, (static_cast<int64_t>(seq) * p.Hq + head0 + gid) * kHeadDim, tig, g_in_group < p.G, qf);
 
     if (L <= 0) {
         if (chunk == 0) {  // zeros for empty sequences
@@ -420,17 +466,19 @@ __global__ void __launch_bounds__(kThreads, TQ_DEC_MINBLOCKS) decode_partial_ker
 
     __syncthreads();   // the pair tables are there; the query's operands are made while the first pages are under way
     // ---- query fragments -------------------------------------------------------------------------------
-    uint32_t qf[16], qpf[QJL ? 16 : 1];
+    uint32_t qpf[QJL ? 16 : 1];
     float sq_init0 = 0.f, sq_init1 = 0.f;   // minus the query sums of the one-sided sign forms
     float qpscale0 = 0.f, qpscale1 = 0.f;   // of queries 2 tig, 2 tig + 1
     {
-        const bool valid = g_in_group < p.G;
-        const int64_t row = (static_cast<int64_t>(seq) * p.Hq + head0 + gid) * kHeadDim;
-        if (p.rotate_q) rotate_q32(xq, lane, p.io_dtype);
-        q_frag_from(xq, qf);
+        if (p.rotate_q) rotate_q_words(qf, lane, p.io_dtype);
         if constexpr (QJL) {
-            if (p.qp) load_q32(p.qp, row, tig, p.io_dtype, valid, xq);   // S q' given separately
-            float corr;
+            float xq[32], corr;
+            if (p.qp) {   // S q' given separately
+                load_q_words(p.qp, (static_cast<int64_t>(seq) * p.Hq + head0 + gid) * kHeadDim, tig, g_in_group < p.G, qpf);
+                unpack_q(qpf, p.io_dtype, xq);
+            } else {
+                unpack_q(qf, p.io_dtype, xq);
+            }
             const float2 by = divided_by(fit_sign_rows(xq, lane), tig);
             qpscale0 = by.x * p.qpscale;
             qpscale1 = by.y * p.qpscale;
@@ -440,6 +488,7 @@ __global__ void __launch_bounds__(kThreads, TQ_DEC_MINBLOCKS) decode_partial_ker
             sq_init0 = -__shfl_sync(0xffffffffu, corr, 8 * tig);       // query 2 * tig lives on lanes 8 * tig ..
             sq_init1 = -__shfl_sync(0xffffffffu, corr, 8 * tig + 4);   // query 2 * tig + 1
         }
+        q_words_to_half(qf, p.io_dtype);
     }
 
     const uint32_t klut = smem_u32(tabk) + (KB == 2 ? 8 * (lane & 15) : 4 * lane);

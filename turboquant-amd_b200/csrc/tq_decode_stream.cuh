@@ -30,6 +30,7 @@ namespace {
 constexpr int kStreamWarps = 16;
 constexpr int kStreamThreads = kStreamWarps * 32;
 constexpr int kStreamStages = 4;
+constexpr int kStreamFirst = 1;              // pages of a ring that are requested at once
 constexpr int kStreamTable = 32768;          // 256 entries of 128 bytes
 constexpr int kStreamCtas = 148;             // one per SM
 constexpr int kStreamSlotFloats = 8 * kHeadDim;
@@ -354,14 +355,29 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
         wbase += 32;
         return src;
     };
+    // The words of an item's queries, for the operands made of them when the item begins: requested ahead of the first pages, and from
+    // the second item on before the result of the one before is written.
+    uint32_t qf[16];
+    auto request_queries = [&](int s, int h) {
+        const int kvh = kv_head(h), head = kvh * p.G + (h - kvh * p.ngroups) * 8;
+        load_q_words(p.q, (static_cast<int64_t>(s) * p.Hq + head + gid) * kHeadDim, tig, kvh * p.G + p.G - head > gid, qf);
+    };
     uint32_t src = next_window();
     uint32_t src_next = src;
+    if (n > 0) request_queries(seq, hg);
+    // Full rings of all warps are 13 to 20 MB, 2 to 3 us of the memory's time, in which nothing else comes through: the queries and the
+    // first page are requested at once, the rest of the ring when the tables are filled.  us per launch in a graph, rings first and
+    // queries last / this: turbo3 128 x 512 tokens 34.1 / 32.4, 32 x 4096 48.0 / 46.9, Sparse-V 32 x 8192 84.6 / 82.7 (two pages at
+    // once: 32.9, 46.9, 83.4).
+    auto first_copies = [&](int from, int to) {
 #pragma unroll
-    for (int i = 0; i < NSTAGE; ++i) {
-        const uint32_t at = __shfl_sync(0xffffffffu, src, i);
-        if (i < n) copy_in<0, PAGE>(ring + i * PAGE, page_at(at), lane);
-        copies_end();
-    }
+        for (int i = from; i < to; ++i) {
+            const uint32_t at = __shfl_sync(0xffffffffu, src, i);
+            if (i < n) copy_in<0, PAGE>(ring + i * PAGE, page_at(at), lane);
+            copies_end();
+        }
+    };
+    first_copies(0, kStreamFirst);
     if (n > 32) src_next = next_window();
     // Flags of lengths that are cut and zeros of empty sequences, behind the first pages' copies: sequence s belongs to warp
     // s / gridDim of CTA s % gridDim (one thread a sequence in CTA 0 took 1.8 ms for 1008 empty sequences of 128 heads).
@@ -376,6 +392,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
     // the codebooks' part of the table is filled behind the first pages' copies
     fill_stream_table<KB>(ktab, ck, warp, lane);
     if constexpr (!SIGN_TABLE) fill_stream_table<VB>(vtab, cv, warp, lane);
+    first_copies(kStreamFirst, NSTAGE);
     __syncthreads();
 
     const uint32_t klut = ktab + (KB == 2 ? 8 * (lane & 15) : 4 * lane);
@@ -395,19 +412,20 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
         const int seg = min(np - page, n - idx);           // pages of this item in the share
         const int kvh = kv_head(hg), qg = hg - kvh * p.ngroups;
         const int head0 = kvh * p.G + qg * 8, nq = min(8, p.G - qg * 8);
-        const int64_t row = (static_cast<int64_t>(seq) * p.Hq + head0 + gid) * kHeadDim;
 
-        uint32_t qf[16], qpf[QJL && !SIGN_TABLE ? 16 : 1];
+        uint32_t qpf[QJL && !SIGN_TABLE ? 16 : 1];
         float sq_init0 = 0.f, sq_init1 = 0.f;   // minus the query sums of the one-sided sign forms
         uint32_t divided = 0;                   // queries whose one-sided sign operands are divided by 256
         {
-            float xq[32];
-            load_q32(p.q, row, tig, p.io_dtype, gid < nq, xq);
-            if (p.rotate_q) rotate_q32(xq, lane, p.io_dtype);
-            q_frag_from(xq, qf);
+            if (p.rotate_q) rotate_q_words(qf, lane, p.io_dtype);
             if constexpr (QJL && !SIGN_TABLE) {
-                if (p.qp) load_q32(p.qp, row, tig, p.io_dtype, gid < nq, xq);
-                float corr;
+                float xq[32], corr;
+                if (p.qp) {
+                    load_q_words(p.qp, (static_cast<int64_t>(seq) * p.Hq + head0 + gid) * kHeadDim, tig, gid < nq, qpf);
+                    unpack_q(qpf, p.io_dtype, xq);
+                } else {
+                    unpack_q(qf, p.io_dtype, xq);
+                }
                 divided = fit_sign_rows(xq, lane);
                 qp_frag_signed_from(xq, qpf, corr);
                 corr += __shfl_xor_sync(0xffffffffu, corr, 1);
@@ -415,6 +433,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
                 sq_init0 = -__shfl_sync(0xffffffffu, corr, 8 * tig);
                 sq_init1 = -__shfl_sync(0xffffffffu, corr, 8 * tig + 4);
             }
+            q_words_to_half(qf, p.io_dtype);
         }
         // Sparse-V: columns past the group's heads hold zero queries, whose scores are all alike; they decide nothing
         const float thresh0 = 2 * tig < nq ? sp.weight_thresh : INFINITY, thresh1 = 2 * tig + 1 < nq ? sp.weight_thresh : INFINITY;
@@ -657,6 +676,18 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
         if (QJL && !SIGN_TABLE && divided) pages(std::bool_constant<QJL && !SIGN_TABLE>{});
         else pages(std::false_type{});
 
+        // ---- the next item
+        int next_seq = seq, next_hg = hg, next_len = len, next_np = np;
+        if (idx + seg < n) {
+            if (++next_hg == sp.HG) {
+                next_hg = 0;
+                do {
+                    next_len = uniform(__ldg(p.seq_lens + ++next_seq));
+                    next_np = pages_of(p, next_len);
+                } while (next_np == 0);
+            }
+            request_queries(next_seq, next_hg);
+        }
         // ---- the item's result, or this warp's part of it
 #pragma unroll
         for (int o = 4; o < 32; o <<= 1) {
@@ -698,13 +729,10 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
             sm_part[2 * warp + (at_end ? 1 : 0)] = make_int4(hg, seq, np - page - seg, page == 0 ? 1 : 0);
         idx += seg;
         page = 0;
-        if (idx < n && ++hg == sp.HG) {
-            hg = 0;
-            do {
-                len = uniform(__ldg(p.seq_lens + ++seq));
-                np = pages_of(p, len);
-            } while (np == 0);
-        }
+        seq = next_seq;
+        hg = next_hg;
+        len = next_len;
+        np = next_np;
     }
     if (p.status) {
         const bool bad = __any_sync(0xffffffffu, bad_block);

@@ -314,8 +314,10 @@ __global__ void __launch_bounds__(kUmThreads, 2) decode_umma_kernel(const Decode
         const bool valid = qg * 8 + gid < p.G;
         const int64_t row = (static_cast<int64_t>(seq) * p.Hq + head0 + gid) * kHeadDim;
         float xq[32];
-        load_q32(p.q, row, tig, p.io_dtype, valid, xq);
-        if (p.rotate_q) rotate_q32(xq, lane, p.io_dtype);
+        uint32_t qw[16];
+        load_q_words(p.q, row, tig, valid, qw);
+        if (p.rotate_q) rotate_q_words(qw, lane, p.io_dtype);
+        unpack_q(qw, p.io_dtype, xq);
         auto write_operand = [&](const float (&x)[32], uint32_t dst, bool permute_for_signs) -> float {
             float mx = 0.f;
 #pragma unroll
@@ -353,7 +355,10 @@ __global__ void __launch_bounds__(kUmThreads, 2) decode_umma_kernel(const Decode
         const float inv_sq = write_operand(xq, sbase + UmSmem::kQ, false);
         float inv_sqp = inv_sq;
         if constexpr (QJL) {
-            if (p.qp) load_q32(p.qp, row, tig, p.io_dtype, valid, xq);
+            if (p.qp) {
+                load_q_words(p.qp, row, tig, valid, qw);
+                unpack_q(qw, p.io_dtype, xq);
+            }
             inv_sqp = write_operand(xq, sbase + UmSmem::kQP, true);
         }
         if (lane == 0) {
