@@ -58,7 +58,7 @@ struct DecodeParams {
     int64_t bt_stride;
     int64_t num_blocks;
     float qscale;    // sm_scale * log2(e)
-    float qpscale;   // sm_scale * corr_scale * log2(e) * 16
+    float qpscale;   // sm_scale * corr_scale * log2(e) / kSignUnit
     float log2_thresh;
     int Hq, Hkv, G, ngroups;
     int sub_shift;           // log2(block_size / 16)
@@ -152,15 +152,22 @@ __device__ __forceinline__ uint2 lut_quad(uint32_t lane_base, uint32_t w, int k)
 
 // QJL sign term on fp16 tensor cores with one logic op per pair of signs.
 //
-// The sign word holds bit l = 1 when the residual of local dim l is >= 0.  A register of the
-// A fragment is a pair of dims (j, j + 16), i.e. bits j and j + 16.  After x = sw << k the pair
-// whose bits landed on 15/31 is turned into +-1 by one and-or; the pairs on bits 14/30, 13/29
-// and 12/28 are used as they are: a lone exponent bit of an fp16 number is the value 2, 2^-7 or
-// 2^-11.  Those three forms give (value) * [sign >= 0] instead of +-1; since
-// 2 * [s >= 0] = sigma + 1, the query operand of those slots is pre-scaled (1, 2^8, 2^12) and
-// the constant sum of the query over those dims is subtracted once (accumulator start value).
-// Form 0 yields -sigma, so its query operand is negated.  All query operands carry 1/16 to keep
-// 2^12 * q inside fp16 (rows with larger values: fit_sign_rows); the factor 16 is folded into the fp32 scale of the residual norm.
+// The sign word holds bit l = 1 when the residual of local dim l is >= 0.  A register of the A fragment is a pair of dims
+// (j, j + 16), bits j and j + 16, masked where they are: a lone bit 4 .. 11 of an fp16 number is the value 2^-20 .. 2^-13 (the
+// subnormal ones too: tensor cores take them as they are).  The other eight pairs come to these bits when the word is rotated by
+// a byte, each with its dims swapped or not (qp_frag_signed_from).  This gives value * [sign >= 0] instead of +-1; since
+// 2 * [s >= 0] = sigma + 1, a query operand is scaled by 2^7 .. 1, so that every product counts in 2^-13, and the query sum, in
+// halves of that, is subtracted once (accumulator start value).  (Bits 12 .. 15 by shifts of four, with operands scaled by up to
+// 2^12 that overflowed from 255 on, took 40 instructions a page instead of 34.)
+constexpr float kSignUnit = 1.f / 16384.f;   // of sigma * q in the sign sums
+__device__ __forceinline__ uint32_t rotate_signs(uint32_t w) { return prmt(w, w, 0x0321u); }
+// Pair slot I = 0 .. 15: bits 4 + I of the word w, or for I >= 8 bits I - 4 of w rotated.
+template <int I>
+__device__ __forceinline__ uint32_t sign_pair(uint32_t w, uint32_t rotated) {
+    uint32_t r;
+    asm("and.b32 %0, %1, %2;" : "=r"(r) : "r"(I < 8 ? w : rotated), "n"(0x00100010u << (I & 7)));
+    return r;
+}
 // This lane's 32 query values (dims 32 * tig .. 32 * tig + 31 of query row gid) as they are stored, two to a word; zeros when !valid.
 __device__ __forceinline__ void load_q_words(const void* q, int64_t row_off, int tig, bool valid, uint32_t (&w)[16]) {
     const uint4* base = reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(q) + row_off + tig * 32);
@@ -249,35 +256,32 @@ __device__ __forceinline__ void q_words_to_half(uint32_t (&w)[16], int io_dtype)
     }
 }
 
-// Query operands of the sign term (see above): per MMA m and slot, half2 of dims (j, j + 16) times the
-// coefficient of the form; `correction` returns this lane's share of the query sum over the one-sided forms.
+// Query operands of the sign term: half2 of the two dims of slot i times 2^(7 - i % 8); `correction` returns this lane's share of the
+// query sum.
 __device__ __forceinline__ void qp_frag_signed_from(const float (&x)[32], uint32_t (&f)[16], float& correction) {
     correction = 0.f;
-    const float coef[4] = {-1.f / 16.f, 1.f / 16.f, 16.f, 256.f};   // form 0..3, times the common 1/16
 #pragma unroll
-    for (int m = 0; m < 8; ++m) {
-#pragma unroll
-        for (int sl = 0; sl < 2; ++sl) {
-            const int form = 2 * (m & 1) + sl, k = 4 * (m >> 1), j = 15 - form - k;
-            f[2 * m + sl] = pack_half2(coef[form] * x[j], coef[form] * x[j + 16]);
-            if (form) correction += (x[j] + x[j + 16]) * (1.f / 16.f);
-        }
+    for (int i = 0; i < 16; ++i) {
+        const int lo = (i < 8 ? 4 : 12) + (i & 7), hi = (lo + 16) & 31;
+        const float coef = static_cast<float>(1 << (7 - (i & 7)));
+        f[i] = pack_half2(coef * x[lo], coef * x[hi]);
+        correction += (x[lo] + x[hi]) * kSignUnit;
     }
 }
 
-// The coefficients of 16 and 256 (dims 4 i + 1 and 4 i) take values of 255 and more out of fp16's range, and infinity times an absent
-// sign is NaN.  A row that has such a value there goes in divided by 256: with the smallest coefficient this rounds coordinates below
-// 1/4 to multiples of 2^-12, 2^-20 of the largest one or less.  Returns the lanes of divided rows.  (A launch of few pages
-// pays 0.04 us of 7.6 for it; 0.13 with the maximum as a chain instead of a tree, and ahead of the tables' barrier.)
+// The coefficients, up to 128, take values of 512 and more out of fp16's range, and infinity times an absent sign is NaN.  A row that
+// has such a value (511: it may round up) goes in divided by 256: with the smallest coefficient this rounds coordinates below 1/64 to
+// multiples of 2^-16, 2^-25 of the largest one or less.  Returns the lanes of divided rows.  (The maximum as a tree: as a chain it
+// costs a launch of few pages 0.1 us.)
 __device__ __forceinline__ uint32_t fit_sign_rows(float (&x)[32], int lane) {
-    float most[8];
+    float most[16];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) most[i] = fmaxf(fabsf(x[4 * i]), fabsf(x[4 * i + 1]));
+    for (int i = 0; i < 16; ++i) most[i] = fmaxf(fabsf(x[2 * i]), fabsf(x[2 * i + 1]));
 #pragma unroll
-    for (int h = 4; h > 0; h >>= 1)
+    for (int h = 8; h > 0; h >>= 1)
 #pragma unroll
         for (int i = 0; i < h; ++i) most[i] = fmaxf(most[i], most[i + h]);
-    const uint32_t over = __ballot_sync(0xffffffffu, most[0] >= 255.f);
+    const uint32_t over = __ballot_sync(0xffffffffu, most[0] >= 511.f);
     if (!over) return 0;
     const bool row_over = (over >> (lane & 28)) & 15;
 #pragma unroll
@@ -947,7 +951,7 @@ extern "C" int tq_decode_paged(void* out, const void* q_rot, const void* q_proj,
     p.bt_stride = bt_stride;
     p.num_blocks = num_blocks;
     p.qscale = sm_scale * kLog2e;
-    p.qpscale = sm_scale * corr_scale * kLog2e * 16.f;   // the sign-term query operands carry 1/16
+    p.qpscale = sm_scale * corr_scale * kLog2e / kSignUnit;   // what the sign sums count in
     p.log2_thresh = sparse_thresh > 0.f ? log2f(sparse_thresh) : -INFINITY;
     p.Hq = num_q_heads;
     p.Hkv = num_kv_heads;

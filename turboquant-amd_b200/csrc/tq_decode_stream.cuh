@@ -9,8 +9,13 @@
 // Against the chunked kernel (4-warp CTAs, one chunk of one item each) this takes away the last wave that is three
 // quarters full, the table fill, pipeline start and merge per chunk, and the empty CTAs of a ragged batch.
 //
-// What bounds it: the shared-memory data path (turbo3: 82 % of its peak, 125 wavefronts a page) and, next to it, instruction issue
-// (360 instructions a page, 58 % of the cycles with four warps a scheduler; a tensor instruction costs it about three slots).
+// What bounds it: instruction issue with four warps a scheduler (a tensor instruction costs about three slots) next to the
+// shared-memory data path (turbo3: 93 wavefronts a page), and under constant load the GPU's power: at 1000 W the clock falls from 1965
+// to 1765 MHz.  Sign operands by logic, 34 instructions and no shared memory, instead of looked up (20 instructions, 32 wavefronts,
+// 32 KB of table), us per launch in a graph, looked up / by logic: turbo3 64 x 8192 tokens 145.5 / 142.4, turbo2 64 x 4096 75.1 / 69.3,
+// Sparse-V turbo3 32 x 8192 82.8 / 84.2 (84.6 with the queries rotated by butterflies, as it was when this was decided: dense and
+// Sparse-V calls keep the same arithmetic).  20 warps of 96 registers (151.6 for 145.6) or 24 of 80 (157.6) lose: the look-ups in flight
+// need registers.
 // Pages are staged with cp.async, 16 bytes a lane, into a private ring: a page then costs four copy instructions and a counted
 // wait, where a bulk copy by one elected lane with its barrier cost about 35 instructions.  Together with a page body that has no
 // partly filled pages to look after, table addresses from the multiply-add pipe and loop state in uniform registers, us per
@@ -90,24 +95,13 @@ __device__ __forceinline__ uint2 table_quad(uint32_t w, uint32_t base) {
     return v;
 }
 
-// mask ? b : a, bit by bit; and a and-or.  As PTX, so that the shift that makes an operand is not moved behind a mask of
+// mask ? b : a, bit by bit.  As PTX, so that the shift that makes an operand is not moved behind a mask of
 // its own (the compiler then spends two logic instructions on each of these).
 __device__ __forceinline__ uint32_t bit_select(uint32_t a, uint32_t b, uint32_t mask) {
     uint32_t r;
     asm("lop3.b32 %0, %1, %2, %3, 0xd8;" : "=r"(r) : "r"(a), "r"(b), "r"(mask));
     return r;
 }
-__device__ __forceinline__ uint32_t and_or(uint32_t a, uint32_t mask, uint32_t bits) {
-    uint32_t r;
-    asm("lop3.b32 %0, %1, %2, %3, 0xea;" : "=r"(r) : "r"(a), "r"(mask), "r"(bits));
-    return r;
-}
-__device__ __forceinline__ uint32_t and_bits(uint32_t a, uint32_t mask) {
-    uint32_t r;
-    asm("and.b32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(mask));
-    return r;
-}
-
 // Words whose bytes address the table.  The table does not look at the spare top bit of a 3-bit nibble.
 template <int BITS>
 __device__ __forceinline__ void table_words(const uint32_t* w, uint32_t (&mw)[4]) {
@@ -207,31 +201,13 @@ __device__ __forceinline__ void wht_16x8(float (&x)[16], int lane) {
     for (int i = 0; i < 16; ++i) x[i] *= kWhtScale;
 }
 
-// Sign table, indexed by one nibble of signs (four dims) of token A and one of token B: the four half2 of +-1 that are the A
-// operand of one score product, in its register order (A dims 0 1, B dims 0 1, A dims 2 3, B dims 2 3), 8 copies.  (With the
-// eight signs of a byte of one token per entry, every second register had to be moved before the products.)
-__device__ __forceinline__ void fill_sign_table(uint32_t smem_addr, int warp, int lane) {
-    auto signs = [](int pair) { return 0xBC00BC00u ^ ((pair & 1) ? 0x8000u : 0u) ^ ((pair & 2) ? 0x80000000u : 0u); };
-    for (int b0 = 4 * warp; b0 < 256; b0 += 4 * kStreamWarps) {
-        const int b = b0 + (lane >> 3);
-        store_entry(smem_addr + b * 128 + 16 * (lane & 7), make_uint4(signs(b), signs(b >> 4), signs(b >> 2), signs(b >> 6)));
-    }
-}
-template <int K>
-__device__ __forceinline__ uint4 table_signs(uint32_t w, uint32_t base) {
-    uint4 v;
-    asm("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(entry_of<K>(w, base)));
-    return v;
-}
 // Output row g of an item.
 __device__ __forceinline__ void finish_row(const DecodeParams& p, int seq, int hg, int g, int lane, float (&x)[4], float l) {
     const int kvh = p.ngroups == 1 ? hg : hg / p.ngroups, qg = hg - kvh * p.ngroups;
     if (g < p.G - qg * 8) write_row(p, static_cast<int64_t>(seq) * p.Hq + kvh * p.G + qg * 8 + g, lane, x, l);
 }
 
-// SIGN_TABLE: K and V share a codebook and S = I, so the second table has room for the signs, and the query operands of the
-// index term serve the sign term as well; without, the sign operands are made by logic.
-template <int KB, int VB, bool QJL, bool SPARSE, bool SIGN_TABLE>
+template <int KB, int VB, bool QJL, bool SPARSE>
 __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const StreamParams sp) {
     constexpr int NWK = KB + (QJL ? 1 : 0);
     constexpr int RK = 16 * NWK;
@@ -249,19 +225,19 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
     __shared__ int sm_scan[kStreamThreads + 1];
     __shared__ int sm_len[kStreamThreads];       // length of the first sequence of each thread's run
     __shared__ int sm_wsum[kStreamWarps];
+    __shared__ int4 sm_window[kStreamWarps];     // where the next window of a warp starts: (sequence, item of it, page, pages of the sequence)
     __shared__ int4 sm_part[2 * kStreamWarps];   // partials: (item or -1, sequence, pages of the item after this share, flags)
 
     const int warp = uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
     const int gid = lane >> 2, tig = lane & 3;
 
-    const uint32_t ktab = smem_u32(smem), vtab = ktab + (SIGN_TABLE ? 0 : kStreamTable), stab = ktab + kStreamTable;
+    const uint32_t ktab = smem_u32(smem), vtab = ktab + kStreamTable;
     const uint32_t rings = ktab + 2 * kStreamTable, ring = rings + warp * RING;
 
-    if constexpr (SIGN_TABLE) fill_sign_table(stab, warp, lane);   // constants
     if (lane < 2) sm_part[2 * warp + lane] = make_int4(-1, 0, 0, 0);
     pdl_wait();
     pdl_release();
-    const float ck = lane_centroid<KB>(p.kc, lane), cv = SIGN_TABLE ? 0.f : lane_centroid<VB>(p.vc, lane);
+    const float ck = lane_centroid<KB>(p.kc, lane), cv = lane_centroid<VB>(p.vc, lane);
 
     // ---- pages before each thread's run of sequences (every CTA does the same scan over all lengths)
     const int per = (sp.ns + kStreamThreads - 1) / kStreamThreads;
@@ -334,11 +310,13 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
         return (static_cast<uint32_t>(blk * p.Hkv + kv_head(h)) << p.sub_shift) + (pg & ((1 << p.sub_shift) - 1));
     };
     auto page_at = [&](uint32_t at) { return p.cache + static_cast<uint64_t>(at) * PAGE; };
-    int wseq = seq, whg = hg, wpage = page, wnp = np, wbase = 0;     // where window `wbase / 32` starts
-    auto next_window = [&]() -> uint32_t {
+    if (lane == 0) sm_window[warp] = make_int4(seq, hg, page, np);
+    auto next_window = [&](int base) -> uint32_t {   // of pages base .. base + 31 of the share
+        __syncwarp();
+        const int4 from = sm_window[warp];
         uint32_t src = 0;
-        int s = wseq, h = whg, pg = wpage + lane, m = wnp;
-        if (wbase + lane < n) {
+        int s = from.x, h = from.y, pg = from.z + lane, m = from.w;
+        if (base + lane < n) {
             while (pg >= m) {
                 pg -= m;
                 if (++h == sp.HG) {
@@ -348,11 +326,8 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
             }
             src = locate(s, h, pg);
         }
-        wseq = __shfl_sync(0xffffffffu, s, 31);
-        whg = __shfl_sync(0xffffffffu, h, 31);
-        wpage = __shfl_sync(0xffffffffu, pg, 31) + 1;
-        wnp = __shfl_sync(0xffffffffu, m, 31);
-        wbase += 32;
+        __syncwarp();
+        if (lane == 31) sm_window[warp] = make_int4(s, h, pg + 1, m);
         return src;
     };
     // The words of an item's queries, for the operands made of them when the item begins: requested ahead of the first pages, and from
@@ -362,7 +337,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
         const int kvh = kv_head(h), head = kvh * p.G + (h - kvh * p.ngroups) * 8;
         load_q_words(p.q, (static_cast<int64_t>(s) * p.Hq + head + gid) * kHeadDim, tig, kvh * p.G + p.G - head > gid, qf);
     };
-    uint32_t src = next_window();
+    uint32_t src = next_window(0);
     uint32_t src_next = src;
     if (n > 0) request_queries(seq, hg);
     // Full rings of all warps are 13 to 20 MB, 2 to 3 us of the memory's time, in which nothing else comes through: the queries and the
@@ -378,7 +353,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
         }
     };
     first_copies(0, kStreamFirst);
-    if (n > 32) src_next = next_window();
+    if (n > 32) src_next = next_window(32);
     // Flags of lengths that are cut and zeros of empty sequences, behind the first pages' copies: sequence s belongs to warp
     // s / gridDim of CTA s % gridDim (one thread a sequence in CTA 0 took 1.8 ms for 1008 empty sequences of 128 heads).
     for (int s = warp * static_cast<int>(gridDim.x) + static_cast<int>(blockIdx.x); s < sp.ns; s += sp.n_warps) {
@@ -391,18 +366,16 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
     }
     // the codebooks' part of the table is filled behind the first pages' copies
     fill_stream_table<KB>(ktab, ck, warp, lane);
-    if constexpr (!SIGN_TABLE) fill_stream_table<VB>(vtab, cv, warp, lane);
+    fill_stream_table<VB>(vtab, cv, warp, lane);
     first_copies(kStreamFirst, NSTAGE);
     __syncthreads();
 
     const uint32_t klut = ktab + (KB == 2 ? 8 * (lane & 15) : 4 * lane);
     const uint32_t vlut = vtab + (VB == 2 ? 8 * (lane & 15) : 4 * lane);
-    const uint32_t slut = stab + 16 * (lane & 7);
     const uint32_t ring_k = ring + lane * (NWK * 4);
     const uint32_t ring_n = ring + gid * 4;
     const uint32_t ring_v = ring + (tig * 8 + gid) * 4;
 
-    const float qpscale = SIGN_TABLE ? p.qpscale * (1.f / 16.f) : p.qpscale;   // the one-sided forms carry 1/16 in the query
     uint32_t stage = 0;                       // ring stage of the current page
     uint32_t k_only = 0;                      // Sparse-V: bit s = the page in stage s came without its V part
     uint32_t v_skipped = 0;
@@ -413,12 +386,12 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
         const int kvh = kv_head(hg), qg = hg - kvh * p.ngroups;
         const int head0 = kvh * p.G + qg * 8, nq = min(8, p.G - qg * 8);
 
-        uint32_t qpf[QJL && !SIGN_TABLE ? 16 : 1];
+        uint32_t qpf[QJL ? 16 : 1];
         float sq_init0 = 0.f, sq_init1 = 0.f;   // minus the query sums of the one-sided sign forms
         uint32_t divided = 0;                   // queries whose one-sided sign operands are divided by 256
         {
             if (p.rotate_q) rotate_q_words(qf, lane, p.io_dtype);
-            if constexpr (QJL && !SIGN_TABLE) {
+            if constexpr (QJL) {
                 float xq[32], corr;
                 if (p.qp) {
                     load_q_words(p.qp, (static_cast<int64_t>(seq) * p.Hq + head0 + gid) * kHeadDim, tig, gid < nq, qpf);
@@ -454,10 +427,10 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
             uint32_t wa[NWK], wb[NWK];
             lds_words<NWK, 0>(ring_k + so, wa);
             lds_words<NWK, 32 * NWK * 4>(ring_k + so, wb);
-            uint32_t sgn0 = 0, sgn1 = 0;   // bytes: the nibbles 2 k (sgn0), 2 k + 1 (sgn1) of token A, then of token B
-            if constexpr (SIGN_TABLE) {
-                sgn0 = bit_select(wb[KB] << 4, wa[KB], 0x0f0f0f0fu);
-                sgn1 = bit_select(wb[KB], wa[KB] >> 4, 0x0f0f0f0fu);
+            uint32_t ra = 0, rb = 0;   // the sign words, rotated
+            if constexpr (QJL) {
+                ra = rotate_signs(wa[KB]);
+                rb = rotate_signs(wb[KB]);
             }
             float2 kn = unpack_half2(lds_u32<KN_OFF>(ring_n + so)), krn = make_float2(0.f, 0.f);
             if constexpr (QJL) krn = unpack_half2(lds_u32<KRN_OFF>(ring_n + so));
@@ -465,16 +438,12 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
             float sq[4] = {sq_init0, sq_init1, sq_init0, sq_init1}, sq2[4] = {0.f, 0.f, 0.f, 0.f};
             auto sign_term = [&](auto quarter) {   // eight dims of two tokens, two products
                 constexpr int C = decltype(quarter)::value;
-                if constexpr (SIGN_TABLE) {
-                    const uint4 g0 = table_signs<C>(sgn0, slut), g1 = table_signs<C>(sgn1, slut);
-                    mma_f16_16816(sq, g0.x, g0.y, g0.z, g0.w, qf[4 * C], qf[4 * C + 1]);
-                    mma_f16_16816(sq2, g1.x, g1.y, g1.z, g1.w, qf[4 * C + 2], qf[4 * C + 3]);
-                } else if constexpr (QJL) {
-                    const uint32_t xa = wa[KB] << (4 * C), xb = wb[KB] << (4 * C);
-                    mma_f16_16816(sq, and_or(xa, 0x80008000u, 0x3C003C00u), and_or(xb, 0x80008000u, 0x3C003C00u),
-                                  and_bits(xa, 0x40004000u), and_bits(xb, 0x40004000u), qpf[4 * C], qpf[4 * C + 1]);
-                    mma_f16_16816(sq2, and_bits(xa, 0x20002000u), and_bits(xb, 0x20002000u), and_bits(xa, 0x10001000u),
-                                  and_bits(xb, 0x10001000u), qpf[4 * C + 2], qpf[4 * C + 3]);
+                if constexpr (QJL) {
+                    constexpr int I = 4 * C;
+                    const uint32_t xa = wa[KB], xb = wb[KB];
+                    mma_f16_16816(sq, sign_pair<I>(xa, ra), sign_pair<I>(xb, rb), sign_pair<I + 1>(xa, ra), sign_pair<I + 1>(xb, rb), qpf[I], qpf[I + 1]);
+                    mma_f16_16816(sq2, sign_pair<I + 2>(xa, ra), sign_pair<I + 2>(xb, rb), sign_pair<I + 3>(xa, ra), sign_pair<I + 3>(xb, rb),
+                                  qpf[I + 2], qpf[I + 3]);
                 }
             };
             if constexpr (KB == 2) {
@@ -509,11 +478,15 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
                     const uint32_t a2 = table_pair<2>(mwa[C], klut), a3 = table_pair<3>(mwa[C], klut);
                     const uint32_t b2 = table_pair<2>(mwb[C], klut), b3 = table_pair<3>(mwb[C], klut);
                     mma_f16_16816(sm, a2, b2, a3, b3, qf[4 * C + 2], qf[4 * C + 3]);
-                    sign_term(word);
                 };
+                // the signs of a quarter ahead of its look-ups: they need no table and fill the look-ups' latency
+                sign_term(std::integral_constant<int, 0>{});
                 eight_dims(std::integral_constant<int, 0>{});
+                sign_term(std::integral_constant<int, 1>{});
                 eight_dims(std::integral_constant<int, 1>{});
+                sign_term(std::integral_constant<int, 2>{});
                 eight_dims(std::integral_constant<int, 2>{});
+                sign_term(std::integral_constant<int, 3>{});
                 eight_dims(std::integral_constant<int, 3>{});
             }
             kn.x *= p.qscale;
@@ -521,8 +494,8 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
             // tokens gid (s0, s1), gid + 8, queries 2 tig (s0, s2), 2 tig + 1
             float s0 = sm[0] * kn.x, s1 = sm[1] * kn.x, s2 = sm[2] * kn.y, s3 = sm[3] * kn.y;
             if constexpr (QJL) {
-                krn.x *= qpscale;
-                krn.y *= qpscale;
+                krn.x *= p.qpscale;
+                krn.y *= p.qpscale;
                 float t0 = sq[0] + sq2[0], t1 = sq[1] + sq2[1], t2 = sq[2] + sq2[2], t3 = sq[3] + sq2[3];
                 if constexpr (LARGE) {
                     const float2 by = divided_by(divided, tig);
@@ -646,12 +619,12 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
             if (i < n) {
                 if ((i & 31) == 0) {
                     src = src_next;
-                    if (i + 32 < n) src_next = next_window();
+                    if (i + 32 < n) src_next = next_window(i + 32);
                 }
                 const uint8_t* next = page_at(__shfl_sync(0xffffffffu, src, i & 31));
                 if constexpr (SPARSE) {
-                    copy_in<0, KPART>(ring + so, next, lane);
-                    if (do_v) copy_in<KPART, PAGE>(ring + so, next, lane);
+                    if (do_v) copy_in<0, PAGE>(ring + so, next, lane);
+                    else copy_in<0, KPART>(ring + so, next, lane);
                     if (do_v != HAVE_V) k_only ^= 1u << stage;
                 } else {
                     copy_in<0, PAGE>(ring + so, next, lane);
@@ -673,7 +646,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
             for (int j = 0; j < full; ++j) next_page(std::false_type{}, large, j);
             if (full < seg) next_page(std::true_type{}, large, full);
         };
-        if (QJL && !SIGN_TABLE && divided) pages(std::bool_constant<QJL && !SIGN_TABLE>{});
+        if (QJL && divided) pages(std::bool_constant<QJL>{});
         else pages(std::false_type{});
 
         // ---- the next item
@@ -821,9 +794,9 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
     if (threadIdx.x == 0 && !split) sp.split[blockIdx.x].z = -1;
 }
 
-template <int KB, int VB, bool QJL, bool SPARSE, bool SIGN_TABLE>
-int launch_stream_as(const StreamParams& sp, cudaStream_t stream) {
-    auto kern = decode_stream_kernel<KB, VB, QJL, SPARSE, SIGN_TABLE>;
+template <int KB, int VB, bool QJL, bool SPARSE>
+int launch_stream(const StreamParams& sp, cudaStream_t stream) {
+    auto kern = decode_stream_kernel<KB, VB, QJL, SPARSE>;
     static bool configured[64] = {};
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return TQ_ERR_LAUNCH;
@@ -833,14 +806,6 @@ int launch_stream_as(const StreamParams& sp, cudaStream_t stream) {
         configured[dev] = true;
     }
     return launch_chained(kern, dim3(sp.n_warps / kStreamWarps), dim3(kStreamThreads), smem, stream, sp) == cudaSuccess ? TQ_OK : TQ_ERR_LAUNCH;
-}
-
-template <int KB, int VB, bool QJL, bool SPARSE>
-int launch_stream(const StreamParams& sp, cudaStream_t stream) {
-    if constexpr (QJL && KB == VB) {
-        if (sp.d.share_tables && !sp.d.qp) return launch_stream_as<KB, VB, QJL, SPARSE, true>(sp, stream);
-    }
-    return launch_stream_as<KB, VB, QJL, SPARSE, false>(sp, stream);
 }
 
 // One block per CTA of the stream kernel: combines the parts of the item that starts there and ends in a later CTA, two

@@ -363,7 +363,7 @@ __global__ void __launch_bounds__(kUmThreads, 2) decode_umma_kernel(const Decode
         }
         if (lane == 0) {
             scal[3] = inv_sq * p.qscale;                      // times 1 / S_k below
-            scal[1] = inv_sqp * p.qpscale * (1.f / 16.f);     // qpscale carries the mma.sync kernel's factor 16
+            scal[1] = inv_sqp * p.qpscale * kSignUnit;     // qpscale is for sums of the mma.sync kernels
         }
     }
     fence_proxy_async();
