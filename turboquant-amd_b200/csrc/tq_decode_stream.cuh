@@ -55,10 +55,10 @@ struct StreamParams {
     float weight_thresh; // Sparse-V: weights are relative to a reference at most one (log2) above the running maximum
 };
 
-// Shares of U pages for W warps: the first U % W have one page more.
+// Shares of U pages for W warps: the first U % W have one page more.  (W is a constant: a division by a parameter cost a launch 0.2 us.)
 struct Shares {
     uint32_t each, more;
-    __device__ __forceinline__ Shares(uint32_t pages, uint32_t warps) : each(pages / warps), more(pages % warps) {}
+    __device__ __forceinline__ explicit Shares(uint32_t pages) : each(pages / (kStreamCtas * kStreamWarps)), more(pages % (kStreamCtas * kStreamWarps)) {}
     __device__ __forceinline__ uint32_t start(uint32_t w) const { return each * w + min(w, more); }
     __device__ __forceinline__ uint32_t owner(uint32_t page) const {
         const uint32_t longer = more * (each + 1);
@@ -235,6 +235,12 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
     const uint32_t rings = ktab + 2 * kStreamTable, ring = rings + warp * RING;
 
     if (lane < 2) sm_part[2 * warp + lane] = make_int4(-1, 0, 0, 0);
+    // Lengths and codebooks may come from the kernel before this one, but their lines can be on their way into L2.  (With the sums of the
+    // scan by one reduction, shares by a constant and the K table filled while the block table's entries come: turbo4 1 x 131072 tokens
+    // 40.5 / 39.7 us in a graph, a bf16 decode step of 32 sequences with its append 37.9 / 36.8.)
+    if (threadIdx.x * 32 < sp.ns) prefetch_l2(p.seq_lens + threadIdx.x * 32);
+    if (threadIdx.x == kStreamThreads - 1) prefetch_l2(p.kc);
+    if (threadIdx.x == kStreamThreads - 2) prefetch_l2(p.vc);
     pdl_wait();
     pdl_release();
     const float ck = lane_centroid<KB>(p.kc, lane), cv = lane_centroid<VB>(p.vc, lane);
@@ -256,21 +262,21 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
     }
     if (lane == 31) sm_wsum[warp] = incl;
     __syncthreads();
-    int before = incl - own;
-    for (int w = 0; w < warp; ++w) before += sm_wsum[w];
-    sm_scan[threadIdx.x] = before;
-    if (threadIdx.x == kStreamThreads - 1) sm_scan[kStreamThreads] = before + own;
-    __syncthreads();
+    const int wsum = lane < kStreamWarps ? sm_wsum[lane] : 0;
+    const int total = __reduce_add_sync(0xffffffffu, wsum);
+    sm_scan[threadIdx.x] = incl - own + __reduce_add_sync(0xffffffffu, lane < warp ? wsum : 0);
+    if (threadIdx.x == 0) sm_scan[kStreamThreads] = total;
 
     const uint32_t gw = blockIdx.x * kStreamWarps + warp;
     uint32_t first;                                     // this warp's first page
     int n;                                              // and how many it has
     {
-        const Shares shares(static_cast<uint32_t>(sm_scan[kStreamThreads]) * sp.HG, sp.n_warps);   // at most 2^31 pages
+        const Shares shares(static_cast<uint32_t>(total) * sp.HG);   // at most 2^31 pages
         first = shares.start(gw);
         first = uniform(first);
         n = uniform(static_cast<int>(shares.start(gw + 1) - first));
     }
+    __syncthreads();
 
     // ---- the item and page this warp starts in
     int seq = 0, hg = 0, page = 0, np = 0, len = 0;
@@ -301,8 +307,8 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
 
     // ---- copies in: lane l holds the place in the cache (in pages) of page 32 k + l of the warp's share, one window of 32 ahead
     bool bad_block = false;
-    auto locate = [&](int s, int h, int pg) -> uint32_t {
-        int32_t blk = __ldg(p.block_tables + static_cast<int64_t>(s) * p.bt_stride + (pg >> p.sub_shift));
+    auto block_of = [&](int s, int pg) { return __ldg(p.block_tables + static_cast<int64_t>(s) * p.bt_stride + (pg >> p.sub_shift)); };
+    auto place = [&](int32_t blk, int h, int pg) -> uint32_t {
         if (blk < 0 || blk >= p.num_blocks) {
             bad_block = true;
             blk = 0;
@@ -311,12 +317,13 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
     };
     auto page_at = [&](uint32_t at) { return p.cache + static_cast<uint64_t>(at) * PAGE; };
     if (lane == 0) sm_window[warp] = make_int4(seq, hg, page, np);
-    auto next_window = [&](int base) -> uint32_t {   // of pages base .. base + 31 of the share
+    struct Entry { int32_t blk; int h, pg; bool live; };
+    auto window_entry = [&](int base) -> Entry {   // of page base + lane of the share
         __syncwarp();
         const int4 from = sm_window[warp];
-        uint32_t src = 0;
         int s = from.x, h = from.y, pg = from.z + lane, m = from.w;
-        if (base + lane < n) {
+        Entry e = {0, 0, 0, base + lane < n};
+        if (e.live) {
             while (pg >= m) {
                 pg -= m;
                 if (++h == sp.HG) {
@@ -324,11 +331,17 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
                     do m = pages_of(p, __ldg(p.seq_lens + ++s)); while (m == 0);
                 }
             }
-            src = locate(s, h, pg);
+            e.blk = block_of(s, pg);
+            e.h = h;
+            e.pg = pg;
         }
         __syncwarp();
         if (lane == 31) sm_window[warp] = make_int4(s, h, pg + 1, m);
-        return src;
+        return e;
+    };
+    auto next_window = [&](int base) -> uint32_t {
+        const Entry e = window_entry(base);
+        return e.live ? place(e.blk, e.h, e.pg) : 0;
     };
     // The words of an item's queries, for the operands made of them when the item begins: requested ahead of the first pages, and from
     // the second item on before the result of the one before is written.
@@ -337,9 +350,10 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
         const int kvh = kv_head(h), head = kvh * p.G + (h - kvh * p.ngroups) * 8;
         load_q_words(p.q, (static_cast<int64_t>(s) * p.Hq + head + gid) * kHeadDim, tig, kvh * p.G + p.G - head > gid, qf);
     };
-    uint32_t src = next_window(0);
-    uint32_t src_next = src;
+    const Entry entry = window_entry(0);
     if (n > 0) request_queries(seq, hg);
+    fill_stream_table<KB>(ktab, ck, warp, lane);   // while the block table's entries come
+    uint32_t src = entry.live ? place(entry.blk, entry.h, entry.pg) : 0, src_next = src;
     // Full rings of all warps are 13 to 20 MB, 2 to 3 us of the memory's time, in which nothing else comes through: the queries and the
     // first page are requested at once, the rest of the ring when the tables are filled.  us per launch in a graph, rings first and
     // queries last / this: turbo3 128 x 512 tokens 34.1 / 32.4, 32 x 4096 48.0 / 46.9, Sparse-V 32 x 8192 84.6 / 82.7 (two pages at
@@ -364,9 +378,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
             for (int i = lane; i < p.Hq * kHeadDim / 8; i += 32) o[i] = make_uint4(0, 0, 0, 0);
         }
     }
-    // the codebooks' part of the table is filled behind the first pages' copies
-    fill_stream_table<KB>(ktab, ck, warp, lane);
-    fill_stream_table<VB>(vtab, cv, warp, lane);
+    fill_stream_table<VB>(vtab, cv, warp, lane);   // behind the first pages' copies
     first_copies(kStreamFirst, NSTAGE);
     __syncthreads();
 
@@ -549,7 +561,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
             bool have = true;
             if constexpr (SPARSE && !HAVE_V) {
                 if (do_v) {   // first needed page after a run of skipped ones: fetch its V part now
-                    copy_in<KPART, PAGE>(ring + so, page_at(locate(seq, hg, page + j)), lane);
+                    copy_in<KPART, PAGE>(ring + so, page_at(place(block_of(seq, page + j), hg, page + j)), lane);
                     copies_end();
                     wait_copies<0>();
                     __syncwarp();
@@ -720,7 +732,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
     // ---- combine the partials of the CTA's warps: entry 2 w (item that ended inside warp w's share) and 2 w + 1 (the one
     // its share ended in), in page order.  Warp (c, q) takes query row q of every other run of entries of one item.
     __syncthreads();
-    const Shares shares(static_cast<uint32_t>(*static_cast<volatile int*>(sm_scan + kStreamThreads)) * sp.HG, sp.n_warps);
+    const Shares shares(static_cast<uint32_t>(*static_cast<volatile int*>(sm_scan + kStreamThreads)) * sp.HG);
     const int4 part = sm_part[lane];
     const uint32_t live = __ballot_sync(0xffffffffu, part.x >= 0);
     const int prev = 31 - __clz(live & ((1u << lane) - 1u));   // the live entry before this one, or -1
