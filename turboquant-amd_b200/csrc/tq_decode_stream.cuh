@@ -12,10 +12,11 @@
 // What bounds it: instruction issue with four warps a scheduler (a tensor instruction costs about three slots) next to the
 // shared-memory data path (turbo3: 93 wavefronts a page), and under constant load the GPU's power: at 1000 W the clock falls from 1965
 // to 1765 MHz.  Sign operands by logic, 34 instructions and no shared memory, instead of looked up (20 instructions, 32 wavefronts,
-// 32 KB of table), us per launch in a graph, looked up / by logic: turbo3 64 x 8192 tokens 145.5 / 142.4, turbo2 64 x 4096 75.1 / 69.3,
-// Sparse-V turbo3 32 x 8192 82.8 / 84.2 (84.6 with the queries rotated by butterflies, as it was when this was decided: dense and
-// Sparse-V calls keep the same arithmetic).  20 warps of 96 registers (151.6 for 145.6) or 24 of 80 (157.6) lose: the look-ups in flight
-// need registers.
+// 32 KB of table), us per launch in a graph, looked up / by logic: turbo3 64 x 8192 tokens 145.5 / 142.4, turbo2 64 x 4096 75.1 / 69.3.
+// A Sparse-V call does the same arithmetic; its page body has registers to spare for it since the count of skipped V parts lies in
+// shared memory and columns without a query are kept from deciding by their reference instead of by thresholds of their own
+// (32 x 8192: looked up 82.8, by logic 85.3, so 82.7; 64 x 8192 with groups of 4 150.4 / 155.3 / 148.3).
+// 20 warps of 96 registers (151.6 for 145.6) or 24 of 80 (157.6) lose: the look-ups in flight need registers.
 // Pages are staged with cp.async, 16 bytes a lane, into a private ring: a page then costs four copy instructions and a counted
 // wait, where a bulk copy by one elected lane with its barrier cost about 35 instructions.  Together with a page body that has no
 // partly filled pages to look after, table addresses from the multiply-add pipe and loop state in uniform registers, us per
@@ -40,9 +41,15 @@ constexpr int kStreamTable = 32768;          // 256 entries of 128 bytes
 constexpr int kStreamCtas = 148;             // one per SM
 constexpr int kStreamSlotFloats = 8 * kHeadDim;
 
-// Dynamic shared memory: two tables, then one ring per warp.
-__host__ __device__ constexpr int stream_smem(int ring) { return 2 * kStreamTable + kStreamWarps * ring; }
+constexpr int kStreamPartBytes = kStreamSlotFloats * 4 + 64;   // a partial in shared memory: 8 rows, then their (maximum, denominator)
 constexpr int kStreamStaticMost = 6144;      // the kernel's static arrays are smaller
+
+// Dynamic shared memory: two tables, then one ring per warp, then as many partials as there is room for, at most one per warp.
+__host__ __device__ constexpr int stream_pool(int ring) {
+    const int room = (227 * 1024 - 1024 - kStreamStaticMost - 2 * kStreamTable - kStreamWarps * ring) / kStreamPartBytes;
+    return room < kStreamWarps ? room : kStreamWarps;
+}
+__host__ __device__ constexpr int stream_smem(int ring) { return 2 * kStreamTable + kStreamWarps * ring + stream_pool(ring) * kStreamPartBytes; }
 
 struct StreamParams {
     DecodeParams d;
@@ -207,8 +214,112 @@ __device__ __forceinline__ void finish_row(const DecodeParams& p, int seq, int h
     if (g < p.G - qg * 8) write_row(p, static_cast<int64_t>(seq) * p.Hq + kvh * p.G + qg * 8 + g, lane, x, l);
 }
 
+// Combines the partials of the CTA's warps: entry 2 w (item that ended inside warp w's share) and 2 w + 1 (the one its share ended in),
+// in page order.  A run is the entries of one item.  First warp g finds what the entries of all runs weigh in query row g, lane e for
+// entry e, then the rows of all runs are dealt out to the warps.  Entries of even number lie in shared
+// memory too while there is room for them.  (One run after the other, each with its own reductions and the even entries in the
+// workspace, took 4 us of turbo3 64 x 8192, 5.4 of a mixed turbo2 batch of 256 sequences.  us per launch in a graph, before / now: turbo2
+// 64 x 4096 tokens 69.1 / 67.0, turbo3 128 x 512 32.5 / 31.2; the mixed batch 366 / 354.)  sm_scan and sm_len have served their purpose.
+template <int RING>
+__device__ __forceinline__ void combine_partials(const StreamParams& sp, const int4* sm_part, uint32_t rings, int* sm_scan, int* sm_len) {
+    const DecodeParams& p = sp.d;
+    float* weight = reinterpret_cast<float*>(sm_scan);     // [8][32]
+    float2* sum = reinterpret_cast<float2*>(sm_len);       // [8][32], at a run's first entry: (maximum, denominator)
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rows = min(8, p.G);
+    const int4 part = sm_part[lane];
+    const uint32_t live = __ballot_sync(0xffffffffu, part.x >= 0);
+    const int prev = 31 - __clz(live & ((1u << lane) - 1u));   // the live entry before this one, or -1
+    const int prev_x = __shfl_sync(0xffffffffu, part.x, max(prev, 0)), prev_y = __shfl_sync(0xffffffffu, part.y, max(prev, 0));
+    const uint32_t heads = __ballot_sync(0xffffffffu, part.x >= 0 && (prev < 0 || prev_x != part.x || prev_y != part.y));
+    // where entry `lane` lies: an address in shared memory, or 0 for the warp's slot in the workspace
+    const int place = part.w >> 1;
+    const uint32_t at = (lane & 1) ? rings + (lane >> 1) * RING : place ? rings + kStreamWarps * RING + (place - 1) * kStreamPartBytes : 0;
+    if (warp < rows) {
+        const uint32_t upto = 0xffffffffu >> (31 - lane);
+        const int head = max(31 - __clz(heads & upto), 0), last = (heads & ~upto) ? __ffs(heads & ~upto) - 2 : 31;
+        float2 ml = make_float2(-INFINITY, 0.f);
+        if (part.x >= 0) {
+            if (at) asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(ml.x), "=f"(ml.y) : "r"(at + (kStreamSlotFloats + 2 * warp) * 4));
+            else ml = __ldcg(sp.part_ml + (blockIdx.x * kStreamWarps + (lane >> 1)) * 8 + warp);
+        }
+        float M = ml.x;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const float v = __shfl_up_sync(0xffffffffu, M, o);
+            if (lane - o >= head) M = fmaxf(M, v);
+        }
+        M = __shfl_sync(0xffffffffu, M, last);
+        const float w = part.x >= 0 ? ex2(ml.x - M) : 0.f;
+        float l = w * ml.y;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const float v = __shfl_up_sync(0xffffffffu, l, o);
+            if (lane - o >= head) l += v;
+        }
+        l = __shfl_sync(0xffffffffu, l, last);
+        weight[warp * 32 + lane] = w;
+        if (lane == head) sum[warp * 32 + lane] = make_float2(M, l);
+    } else if (warp == kStreamWarps - 1 && lane == 0) {
+        // the item that starts in this CTA and ends in a later one, if there is one, is the last run
+        const int4 first = sm_part[heads ? 31 - __clz(heads) : 0], end = sm_part[live ? 31 - __clz(live) : 0];
+        int last_cta = -1;
+        if (live && (first.w & 1) && end.z > 0) {
+            const Shares shares(static_cast<uint32_t>(sm_scan[kStreamThreads]) * sp.HG);
+            last_cta = static_cast<int>(shares.owner(shares.start((blockIdx.x + 1) * kStreamWarps) + end.z - 1)) / kStreamWarps;
+        }
+        sp.split[blockIdx.x] = make_int4(first.y, first.x, last_cta, 0);
+    }
+    __syncthreads();
+    uint32_t after_heads = heads;
+    for (int run = 0; after_heads; ++run) {
+        const int head = __ffs(after_heads) - 1;
+        after_heads &= after_heads - 1;
+        const int g = (warp - run * rows) & (kStreamWarps - 1);
+        if (g >= rows) continue;
+        uint32_t rest = live & ~((1u << head) - 1u) & (after_heads ? (1u << (__ffs(after_heads) - 1)) - 1u : 0xffffffffu);
+        const int4 item = sm_part[head];
+        const int after = sm_part[31 - __clz(rest)].z;
+        const float2 ml = sum[g * 32 + head];
+        const bool starts = item.w & 1;
+        float x[4] = {0.f, 0.f, 0.f, 0.f};
+        while (rest) {   // four entries at a time
+            float4 v[4];
+            float w[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const int e = rest ? __ffs(rest) - 1 : -1;
+                rest &= rest - 1;
+                const uint32_t from = __shfl_sync(0xffffffffu, at, e & 31);
+                v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+                w[k] = 0.f;
+                if (e >= 0) {
+                    w[k] = weight[g * 32 + e];
+                    if (from)
+                        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[k].x), "=f"(v[k].y), "=f"(v[k].z), "=f"(v[k].w) : "r"(from + (g * kHeadDim + 4 * lane) * 4));
+                    else
+                        v[k] = __ldcg(reinterpret_cast<const float4*>(sp.part_o + static_cast<int64_t>(blockIdx.x * kStreamWarps + (e >> 1)) * kStreamSlotFloats + g * kHeadDim + 4 * lane));
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                x[0] = fmaf(w[k], v[k].x, x[0]);
+                x[1] = fmaf(w[k], v[k].y, x[1]);
+                x[2] = fmaf(w[k], v[k].z, x[2]);
+                x[3] = fmaf(w[k], v[k].w, x[3]);
+            }
+        }
+        if (starts && after == 0) {
+            finish_row(p, item.y, item.x, g, lane, x, ml.y);
+        } else {
+            const int slot = sp.n_warps + 2 * blockIdx.x + (starts ? 1 : 0);
+            *reinterpret_cast<float4*>(sp.part_o + static_cast<int64_t>(slot) * kStreamSlotFloats + g * kHeadDim + 4 * lane) = make_float4(x[0], x[1], x[2], x[3]);
+            if (lane == 0) sp.part_ml[slot * 8 + g] = ml;
+        }
+    }
+}
+
 template <int KB, int VB, bool QJL, bool SPARSE>
-__global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const StreamParams sp) {
+__global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const __grid_constant__ StreamParams sp) {
     constexpr int NWK = KB + (QJL ? 1 : 0);
     constexpr int RK = 16 * NWK;
     constexpr int KN_OFF = 16 * RK;
@@ -223,10 +334,14 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
 
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ int sm_scan[kStreamThreads + 1];
-    __shared__ int sm_len[kStreamThreads];       // length of the first sequence of each thread's run
+    __shared__ __align__(16) int sm_len[kStreamThreads];   // length of the first sequence of each thread's run
     __shared__ int sm_wsum[kStreamWarps];
     __shared__ int4 sm_window[kStreamWarps];     // where the next window of a warp starts: (sequence, item of it, page, pages of the sequence)
-    __shared__ int4 sm_part[2 * kStreamWarps];   // partials: (item or -1, sequence, pages of the item after this share, flags)
+    // partials: (item or -1, sequence, pages of the item after this share, bit 0: starts at the item's first page; above it, where an
+    // entry of even number lies: partial of the pool from 1, or 0 for the warp's slot in the workspace)
+    __shared__ int4 sm_part[2 * kStreamWarps];
+    __shared__ int sm_pool;
+    __shared__ uint32_t sm_skipped[SPARSE ? kStreamWarps : 1];
 
     const int warp = uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
     const int gid = lane >> 2, tig = lane & 3;
@@ -235,6 +350,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
     const uint32_t rings = ktab + 2 * kStreamTable, ring = rings + warp * RING;
 
     if (lane < 2) sm_part[2 * warp + lane] = make_int4(-1, 0, 0, 0);
+    if (threadIdx.x == 0) sm_pool = 0;
     // Lengths and codebooks may come from the kernel before this one, but their lines can be on their way into L2.  (With the sums of the
     // scan by one reduction, shares by a constant and the K table filled while the block table's entries come: turbo4 1 x 131072 tokens
     // 40.5 / 39.7 us in a graph, a bf16 decode step of 32 sequences with its append 37.9 / 36.8.)
@@ -390,7 +506,9 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
 
     uint32_t stage = 0;                       // ring stage of the current page
     uint32_t k_only = 0;                      // Sparse-V: bit s = the page in stage s came without its V part
-    uint32_t v_skipped = 0;
+    if constexpr (SPARSE) {
+        if (lane == 0) sm_skipped[warp] = 0;   // V parts never fetched
+    }
     int idx = 0;                              // pages of the share that are done
 
     while (idx < n) {
@@ -420,9 +538,9 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
             }
             q_words_to_half(qf, p.io_dtype);
         }
-        // Sparse-V: columns past the group's heads hold zero queries, whose scores are all alike; they decide nothing
-        const float thresh0 = 2 * tig < nq ? sp.weight_thresh : INFINITY, thresh1 = 2 * tig + 1 < nq ? sp.weight_thresh : INFINITY;
-        float r0 = INFINITY, r1 = INFINITY;     // minus the softmax reference of queries 2 tig, 2 tig + 1 (log2 domain)
+        // minus the softmax reference of queries 2 tig, 2 tig + 1 (log2 domain).  Sparse-V: columns past the group's heads hold zero
+        // queries, whose scores are all alike; with a reference that no score reaches they weigh nothing and decide nothing.
+        float r0 = SPARSE && 2 * tig >= nq ? -INFINITY : INFINITY, r1 = SPARSE && 2 * tig + 1 >= nq ? -INFINITY : INFINITY;
         float l0 = 0.f, l1 = 0.f;
         float oacc[8][4];
 #pragma unroll
@@ -557,7 +675,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
             // ---- Sparse-V: the V part is not needed when no weight of the group exceeds the threshold.  The reference is
             // at most one above the running maximum.
             bool do_v = true;
-            if constexpr (SPARSE) do_v = __any_sync(0xffffffffu, fmaxf(p0v, p2v) > thresh0 || fmaxf(p1v, p3v) > thresh1);
+            if constexpr (SPARSE) do_v = __any_sync(0xffffffffu, fmaxf(fmaxf(p0v, p2v), fmaxf(p1v, p3v)) > sp.weight_thresh);
             bool have = true;
             if constexpr (SPARSE && !HAVE_V) {
                 if (do_v) {   // first needed page after a run of skipped ones: fetch its V part now
@@ -566,7 +684,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
                     wait_copies<0>();
                     __syncwarp();
                 } else {
-                    ++v_skipped;
+                    if (lane == 0) ++sm_skipped[warp];
                     have = false;
                 }
             }
@@ -648,7 +766,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
         auto next_page = [&](auto partly, auto large, int j) {
             if constexpr (SPARSE) {
                 if (k_only == 0 || !((k_only >> stage) & 1u)) one_page(std::true_type{}, partly, large, j);
-                else one_page(std::false_type{}, partly, large, j);
+                else one_page(std::false_type{}, partly, std::bool_constant<QJL>{}, j);   // (a row that is not divided is multiplied by one)
             } else {
                 one_page(std::true_type{}, partly, large, j);
             }
@@ -681,6 +799,18 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
         }
         // accumulator 2 u + s, register r: dim 16 gid + 4 u + s + 2 (r >> 1) of query 2 tig + (r & 1)
         const bool whole_item = page == 0 && seg == np, at_end = idx + seg == n;
+        uint32_t keep = 0;      // where in shared memory a partial is kept; the ring has served its purpose at the end of the share
+        int place = 0;
+        if (!whole_item) {
+            if (at_end) {
+                keep = ring;
+            } else {
+                if (lane == 0) place = atomicAdd(&sm_pool, 1) + 1;
+                place = __shfl_sync(0xffffffffu, place, 0);
+                if (place > stream_pool(RING)) place = 0;
+                else keep = rings + kStreamWarps * RING + (place - 1) * kStreamPartBytes;
+            }
+        }
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
             const int g = 2 * tig + k;
@@ -696,13 +826,13 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
                 for (int i = 0; i < 16; ++i) x[i] *= inv;
                 if (p.derotate_out) wht_16x8(x, lane);
                 if (g < nq) store_row16(p.out, (static_cast<int64_t>(seq) * p.Hq + head0 + g) * kHeadDim + 16 * gid, p.io_dtype, x);
-            } else if (at_end) {   // the ring has served its purpose
+            } else if (keep) {
 #pragma unroll
                 for (int i = 0; i < 4; ++i)
-                    asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(ring + (g * kHeadDim + 16 * gid + 4 * i) * 4), "f"(x[4 * i]),
+                    asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(keep + (g * kHeadDim + 16 * gid + 4 * i) * 4), "f"(x[4 * i]),
                                  "f"(x[4 * i + 1]), "f"(x[4 * i + 2]), "f"(x[4 * i + 3])
                                  : "memory");
-                if (gid == 0) asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(ring + (kStreamSlotFloats + 2 * g) * 4), "f"(k ? -r1 : -r0), "f"(l) : "memory");
+                if (gid == 0) asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(keep + (kStreamSlotFloats + 2 * g) * 4), "f"(k ? -r1 : -r0), "f"(l) : "memory");
             } else {
                 float4* dst = reinterpret_cast<float4*>(sp.part_o + static_cast<int64_t>(gw) * kStreamSlotFloats + g * kHeadDim + 16 * gid);
 #pragma unroll
@@ -711,7 +841,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
             }
         }
         if (!whole_item && lane == 0)
-            sm_part[2 * warp + (at_end ? 1 : 0)] = make_int4(hg, seq, np - page - seg, page == 0 ? 1 : 0);
+            sm_part[2 * warp + (at_end ? 1 : 0)] = make_int4(hg, seq, np - page - seg, (page == 0 ? 1 : 0) | place << 1);
         idx += seg;
         page = 0;
         seq = next_seq;
@@ -726,84 +856,11 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
     if constexpr (SPARSE) {
         if (p.skip_stats && lane == 0) {
             atomicAdd(p.skip_stats, static_cast<uint32_t>(idx));
-            atomicAdd(p.skip_stats + 1, v_skipped);
+            atomicAdd(p.skip_stats + 1, sm_skipped[warp]);
         }
     }
-    // ---- combine the partials of the CTA's warps: entry 2 w (item that ended inside warp w's share) and 2 w + 1 (the one
-    // its share ended in), in page order.  Warp (c, q) takes query row q of every other run of entries of one item.
     __syncthreads();
-    const Shares shares(static_cast<uint32_t>(*static_cast<volatile int*>(sm_scan + kStreamThreads)) * sp.HG);
-    const int4 part = sm_part[lane];
-    const uint32_t live = __ballot_sync(0xffffffffu, part.x >= 0);
-    const int prev = 31 - __clz(live & ((1u << lane) - 1u));   // the live entry before this one, or -1
-    const int4 before_me = make_int4(__shfl_sync(0xffffffffu, part.x, max(prev, 0)), __shfl_sync(0xffffffffu, part.y, max(prev, 0)), 0, 0);
-    uint32_t heads = __ballot_sync(0xffffffffu, part.x >= 0 && (prev < 0 || before_me.x != part.x || before_me.y != part.y));
-    bool split = false;
-    int run = 0;
-    for (; heads; ++run) {
-        const int head = __ffs(heads) - 1;
-        heads &= heads - 1;
-        const uint32_t mine = live & ~((1u << head) - 1u) & (heads ? (1u << (__ffs(heads) - 1)) - 1u : 0xffffffffu);
-        const int last = 31 - __clz(mine);
-        const int rhg = __shfl_sync(0xffffffffu, part.x, head), rseq = __shfl_sync(0xffffffffu, part.y, head);
-        const bool starts = __shfl_sync(0xffffffffu, part.w, head) != 0;
-        const int after = __shfl_sync(0xffffffffu, part.z, last);
-        if (starts && after > 0 && threadIdx.x == 0) {
-            split = true;
-            const uint32_t end = shares.start((blockIdx.x + 1) * kStreamWarps) + after;   // pages before the item's end
-            sp.split[blockIdx.x] = make_int4(rseq, rhg, static_cast<int>(shares.owner(end - 1)) / kStreamWarps, 0);
-        }
-        if ((run & 1) != (warp >> 3)) continue;
-        const int g = warp & 7;
-        auto ring_of = [&](int w) { return smem_u32(smem) + 2 * kStreamTable + w * RING; };
-        // lane e holds (maximum, denominator) of entry e
-        float2 ml = make_float2(-INFINITY, 0.f);
-        if ((mine >> lane) & 1u) {
-            if (lane & 1) asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(ml.x), "=f"(ml.y) : "r"(ring_of(lane >> 1) + (kStreamSlotFloats + 2 * g) * 4));
-            else ml = __ldcg(sp.part_ml + (blockIdx.x * kStreamWarps + (lane >> 1)) * 8 + g);
-        }
-        float M = ml.x;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
-        const float scale = ex2(ml.x - M);
-        float l = scale * ml.y;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-        float x[4] = {0.f, 0.f, 0.f, 0.f};
-        for (uint32_t rest = mine; rest;) {   // two entries at a time
-            float4 v[2];
-            float sc[2];
-#pragma unroll
-            for (int k = 0; k < 2; ++k) {
-                const int e = rest ? __ffs(rest) - 1 : 32;
-                rest &= rest - 1;
-                sc[k] = __shfl_sync(0xffffffffu, scale, e & 31);
-                if (e == 32) {
-                    sc[k] = 0.f;
-                    v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-                } else if (e & 1) {
-                    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[k].x), "=f"(v[k].y), "=f"(v[k].z), "=f"(v[k].w) : "r"(ring_of(e >> 1) + (g * kHeadDim + 4 * lane) * 4));
-                } else {
-                    v[k] = __ldcg(reinterpret_cast<const float4*>(sp.part_o + static_cast<int64_t>(blockIdx.x * kStreamWarps + (e >> 1)) * kStreamSlotFloats + g * kHeadDim + 4 * lane));
-                }
-            }
-#pragma unroll
-            for (int k = 0; k < 2; ++k) {
-                x[0] = fmaf(sc[k], v[k].x, x[0]);
-                x[1] = fmaf(sc[k], v[k].y, x[1]);
-                x[2] = fmaf(sc[k], v[k].z, x[2]);
-                x[3] = fmaf(sc[k], v[k].w, x[3]);
-            }
-        }
-        if (starts && after == 0) {
-            finish_row(p, rseq, rhg, g, lane, x, l);
-        } else {
-            const int slot = sp.n_warps + 2 * blockIdx.x + (starts ? 1 : 0);
-            *reinterpret_cast<float4*>(sp.part_o + static_cast<int64_t>(slot) * kStreamSlotFloats + g * kHeadDim + 4 * lane) = make_float4(x[0], x[1], x[2], x[3]);
-            if (lane == 0) sp.part_ml[slot * 8 + g] = make_float2(M, l);
-        }
-    }
-    if (threadIdx.x == 0 && !split) sp.split[blockIdx.x].z = -1;
+    combine_partials<RING>(sp, sm_part, rings, sm_scan, sm_len);
 }
 
 template <int KB, int VB, bool QJL, bool SPARSE>
