@@ -287,3 +287,43 @@ def test_sign_term_of_large_queries(kb, vb, dtype, kw, separate):
     ref = torch.stack([_attend64(q[i], qp[i], cache, bt[i, :-(-n // 16)], books, 16, n, hkv) for i, n in enumerate(LONG)])
     error = (out.double().view(ref.shape) - ref).pow(2).sum(dim=(0, 1, 3)).sqrt() / ref.pow(2).sum(dim=(0, 1, 3)).sqrt()
     assert (error <= (2e-3 if dtype == torch.float16 else 4e-3)).all(), error
+
+
+@pytest.mark.parametrize("fmt,hq", [((2, 2, True), 16), ((3, 3, True), 64), ((4, 4, False), 32), ((4, 4, True), 8)])
+@pytest.mark.parametrize("kw", [dict(), dict(rotate_q=True, derotate_out=True), dict(sparse_thresh=1e-9)])
+def test_more_partials_than_shared_memory_keeps(fmt, hq, kw):
+    """Sequences of one and a half shares: in every CTA about ten items end inside a share they did not start, more than shared memory has
+    room for in the wider formats.  Both kernels round the weights (2-norm 1e-4) and the output (2.8e-4) to fp16 on their own."""
+    fmt = CacheFormat(*fmt)
+    books = Codebooks(fmt, DEV)
+    lens = [370 + 7 * (i % 5) for i in range(197)]
+    bt, blocks = _tables(lens, 16, 9)
+    cache = _random_cache(fmt, blocks, 8, 16, 10)
+    q = torch.randn(len(lens), hq, 128, generator=torch.Generator(device=DEV).manual_seed(11), device=DEV).half()
+    call = lambda **more: paged_decode_attention(q, cache, bt.to(DEV), torch.tensor(lens, dtype=torch.int32, device=DEV), books, 16, **kw, **more)
+    got, chunked = call().float(), call(chunk_pages=64).float()
+    assert _native.read_status(DEV) == 0
+    assert not torch.equal(got, chunked)
+    rows = (got - chunked).pow(2).sum(-1).sqrt() / chunked.pow(2).sum(-1).sqrt()
+    assert rows.max() < 2e-3 and rows.pow(2).mean().sqrt() < 8e-4, (rows.max(), rows.pow(2).mean().sqrt())
+
+
+@pytest.mark.parametrize("value", [500.0, 511.0, 512.0, 65000.0])
+@pytest.mark.parametrize("kw", [dict(), dict(chunk_pages=64)])
+def test_sign_operands_at_the_edge_of_fp16(value, kw):
+    """The sign term scales the query by 2^7 at dims 4, 12, 20 and 28 of a quarter and by less up to 1 at the next seven: rows are divided from
+    511 on, and no place overflows.  Weights and output are rounded to 11 bits, scores of thousands to 2^-12 in 32 bits."""
+    fmt, hkv, n = CacheFormat(3, 3, True), 4, 24576 + 5
+    books = Codebooks(fmt, DEV)
+    lens = [n, 3000, 8000, 5000]
+    bt, blocks = _tables(lens, 16, 6)
+    cache = _random_cache(fmt, blocks, hkv, 16, 5)
+    q = torch.randn(len(lens), hkv, 8, 128, generator=torch.Generator(device=DEV).manual_seed(3), device=DEV)
+    for head, dim in enumerate((4, 12, 20, 28, 11, 32 + 19, 64 + 27, 96 + 3)):
+        q[:, :, head, dim] = value if head & 1 else -value
+    q = q.half()
+    out = paged_decode_attention(q.view(len(lens), -1, 128), cache, bt.to(DEV), torch.tensor(lens, dtype=torch.int32, device=DEV), books, 16, **kw)
+    assert _native.read_status(DEV) == 0
+    ref = torch.stack([_attend64(q[i], q[i], cache, bt[i, :-(-m // 16)], books, 16, m, hkv) for i, m in enumerate(lens)])
+    error = (out.double().view(ref.shape) - ref).pow(2).sum(dim=(0, 1, 3)).sqrt() / ref.pow(2).sum(dim=(0, 1, 3)).sqrt()
+    assert (error <= 2e-3).all(), error
