@@ -805,22 +805,25 @@ int dispatch_v(const DecodeParams& p, int vb, const Plan& plan, cudaStream_t str
     return TQ_ERR_UNSUPPORTED;
 }
 
-// Which kernel is the better one, by the pages that the batch can have at most.  The persistent kernel pays about 11 us
+// Which kernel is the better one, by the pages that the batch can have at most.  The persistent kernel pays about 9 us
 // however few pages there are (all its tables, one more level of merging), the chunked one 5 to 9, but it takes
-// 0.45 (4-bit) to 0.55 us (with sign term) per 1000 pages where the chunked one takes 0.7 to 0.8; sequences of few pages
+// 0.4 (4-bit) to 0.5 us (with sign term) per 1000 pages where the chunked one takes 0.7 to 0.8; sequences of few pages
 // cost it more, a warp then changes item every few pages.  Measured with both as they are, us per launch in a graph over caches that
-// L2 does not hold, chunked / persistent, 8 KV heads, turbo4 and turbo3: 16 x 512 tokens (4096 pages) 10.6 / 12.5 and
-// 13.6 / 13.0; 1 x 16384 (8192) 14.8 / 16.0 and 13.9 / 16.7, 32 x 512 16.2 / 15.4 and 15.5 / 16.3; 24 x 1024 (12288) 15.8 / 18.8
-// and 21.8 / 20.2; 64 x 512 (16384) 19.2 / 21.3 and 19.3 / 22.9, 32 x 1024 22.8 / 20.2 and 22.9 / 21.8; 256 x 256 (32768)
-// 37.0 / 34.1 and 36.6 / 36.8, 128 x 512 31.9 / 30.9 and 32.0 / 33.8; 32 x 3000 (48128) 47.9 / 34.6 and 50.9 / 39.2.  The line does
-// not look at the format or at how the chunks come out: the other kernel is 4 to 8 % faster for 16 x 512, 24 x 1024 and
-// 128 x 512 of turbo3, and 5 % for 32 x 512 of turbo4.
-constexpr int64_t kStreamMinPages = 16384;
+// L2 does not hold, rotated queries, chunked / persistent, 8 KV heads, turbo4 and turbo3: 16 x 512 tokens (4096 pages) 8.8 / 13.2 and
+// 9.7 / 13.8; 1 x 16384 (8192) 14.4 / 15.5 and 13.6 / 16.4, 32 x 512 14.4 / 14.7 and 13.8 / 16.0; 24 x 1024 (12288) 14.8 / 17.7 and
+// 20.4 / 19.6; 64 x 512 (16384) 18.7 / 18.9 and 18.4 / 21.0, 128 x 256 20.4 / 18.5 and 19.3 / 20.0.
+// Below 16384 pages sequences of 64 pages or more go by waves: 4-bit chunks run 3 to an SM, and with more than 444 of them the
+// chunked kernel takes 5 us more at once: 27 x 1024 tokens (432 chunks) 14.8 / 17.7 and 20.4 / 19.5, 28 x 1024 (448) 20.3 / 18.3 and
+// 20.6 / 20.4, 13 x 2000 (416) 15.1 / 17.4 and 20.7 / 19.2, 14 x 2000 (448) 19.9 / 17.7 and 20.9 / 19.4, 7 x 4096 (448) 19.7 / 18.1 and
+// 20.8 / 20.1, 1 x 28000 (440) 14.9 / 18.2 and 20.3 / 19.6, 31 x 1024 (496) 20.8 / 18.8 and 20.6 / 20.9.  The lines do not look at the format: the
+// other kernel is up to 8 % faster for 12288 to 13824 pages of turbo3 and 10 % for 128 x 256 of turbo4.
+constexpr int64_t kStreamMinPages = 12288;
+constexpr int64_t kChunkedWave = 3 * 148;
 constexpr int64_t kStreamSlots = static_cast<int64_t>(kStreamCtas) * (kStreamWarps + 2);   // partials of warps and of CTAs
 int64_t pages_at_most(int64_t ns, int64_t hq, int64_t hkv, int64_t max_pages) { return ns * max_pages * hkv * ((hq / hkv + 7) / 8); }
-bool stream_is_better(int64_t pages, int64_t cache_pages, int max_pages) {
+bool stream_is_better(int64_t pages, int64_t cache_pages, int max_pages, int64_t chunks) {
     if (pages < kStreamMinPages || pages > INT32_MAX || cache_pages > UINT32_MAX) return false;
-    return pages >= 32768 || max_pages >= 64;
+    return pages >= 32768 || (max_pages >= 64 && (pages >= 16384 || chunks > kChunkedWave));
 }
 // Workspace of the persistent kernel, or 0 where no format would take it.
 int64_t stream_bytes(int64_t pages) {
@@ -923,11 +926,13 @@ extern "C" int tq_decode_paged(void* out, const void* q_rot, const void* q_proj,
     // The persistent kernel takes the calls that leave the split to the library and bring the workspace for it.
     const bool tensor_memory = use_tcgen05 && k_bits <= 3 && v_bits <= 3 && !(sparse_thresh > 0.f);
     const int64_t pages = pages_at_most(num_seqs, num_q_heads, num_kv_heads, max_pages_per_seq);
-    const int64_t stream_need = chunk_pages <= 0 && !tensor_memory && stream_is_better(pages, num_blocks * num_kv_heads * (block_size / kPageTokens), max_pages_per_seq) ? stream_bytes(pages) : 0;
-    const bool persistent = stream_need > 0 && workspace && workspace_bytes >= stream_need && !(reinterpret_cast<uintptr_t>(workspace) & 15);
-    if (chunk_pages <= 0) chunk_pages = tq_decode_auto_chunk_pages(num_seqs, num_kv_heads, num_q_heads, max_pages_per_seq);
+    const bool split_is_ours = chunk_pages <= 0;
+    if (split_is_ours) chunk_pages = tq_decode_auto_chunk_pages(num_seqs, num_kv_heads, num_q_heads, max_pages_per_seq);
     const int64_t need = tq_decode_workspace_bytes(num_seqs, num_q_heads, num_kv_heads, max_pages_per_seq, chunk_pages);
     const int max_chunks = (max_pages_per_seq + chunk_pages - 1) / chunk_pages;
+    const int64_t chunks = pages / max_pages_per_seq * max_chunks;   // of all sequences, KV heads and query groups
+    const int64_t stream_need = split_is_ours && !tensor_memory && stream_is_better(pages, num_blocks * num_kv_heads * (block_size / kPageTokens), max_pages_per_seq, chunks) ? stream_bytes(pages) : 0;
+    const bool persistent = stream_need > 0 && workspace && workspace_bytes >= stream_need && !(reinterpret_cast<uintptr_t>(workspace) & 15);
     if (!persistent && max_chunks > 1 && (!workspace || workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 15)))
         return TQ_ERR_WORKSPACE;
     if (num_seqs > 65535 || max_chunks > 65535) return TQ_ERR_UNSUPPORTED;
