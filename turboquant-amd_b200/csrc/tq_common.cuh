@@ -106,8 +106,6 @@ inline cudaError_t launch_chained(void (*kernel)(Params...), dim3 grid, dim3 blo
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
 }
 
-__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
-
 // ---- mbarrier + bulk async copy (global -> this CTA's shared memory) ------------
 __device__ __forceinline__ void mbar_init(uint64_t* bar, int count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));

@@ -351,17 +351,13 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
 
     if (lane < 2) sm_part[2 * warp + lane] = make_int4(-1, 0, 0, 0);
     if (threadIdx.x == 0) sm_pool = 0;
-    // Lengths and codebooks may come from the kernel before this one, but their lines can be on their way into L2.  (With the sums of the
-    // scan by one reduction, shares by a constant and the K table filled while the block table's entries come: turbo4 1 x 131072 tokens
-    // 40.5 / 39.7 us in a graph, a bf16 decode step of 32 sequences with its append 37.9 / 36.8.)
-    if (threadIdx.x * 32 < sp.ns) prefetch_l2(p.seq_lens + threadIdx.x * 32);
-    if (threadIdx.x == kStreamThreads - 1) prefetch_l2(p.kc);
-    if (threadIdx.x == kStreamThreads - 2) prefetch_l2(p.vc);
     pdl_wait();
     pdl_release();
     const float ck = lane_centroid<KB>(p.kc, lane), cv = lane_centroid<VB>(p.vc, lane);
 
     // ---- pages before each thread's run of sequences (every CTA does the same scan over all lengths)
+    // (With its sums by one reduction, shares by a constant and the K table filled while the block table's entries come: turbo4 1 x 131072
+    // tokens 40.5 / 39.7 us in a graph, a bf16 decode step of 32 sequences with its append 37.9 / 36.8.)
     const int per = (sp.ns + kStreamThreads - 1) / kStreamThreads;
     int own = 0, len0 = 0;
     for (int s = threadIdx.x * per; s < min(sp.ns, (static_cast<int>(threadIdx.x) + 1) * per); ++s) {
