@@ -415,19 +415,24 @@ __global__ void __launch_bounds__(WARPS * 32, kPaWarps / WARPS) packed_attn_part
         float L = l_run * f;
 #pragma unroll
         for (int o = 4; o < 32; o <<= 1) L += __shfl_xor_sync(0xffffffffu, L, o);
+        // The eight slots' sums: at each of three steps a lane gives away the half of its values that the other lane keeps, so it
+        // ends with four dims: 28 shuffles, where summing every value over all slots took 96 and 1 us a row (us per launch in a
+        // graph, so / now: 4-bit 32 rows x 1000 tokens 7.85 / 6.9, 3-bit 1000 x 256 27.6 / 23.4, 64 x 32768 89.0 / 87.0).
+        float t[32];
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-            float x, y;
-            pa_unpack(acc[j], x, y);
-            x *= f;
-            y *= f;
+        for (int j = 0; j < 16; ++j) pa_unpack(pa_mul(acc[j], pa_pack(f, f)), t[2 * j], t[2 * j + 1]);
+        int dim = 0;
 #pragma unroll
-            for (int o = 4; o < 32; o <<= 1) {
-                x += __shfl_xor_sync(0xffffffffu, x, o);
-                y += __shfl_xor_sync(0xffffffffu, y, o);
+        for (int o = 16, n = 16; o >= 4; o >>= 1, n >>= 1) {
+            const bool upper = lane & o;
+            dim += upper ? n : 0;
+#pragma unroll
+            for (int i = 0; i < n; ++i) {
+                const float keep = upper ? t[n + i] : t[i], give = upper ? t[i] : t[n + i];
+                t[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
             }
-            if (slot == 0) *reinterpret_cast<float2*>(&sacc[warp][32 * quarter + 2 * j]) = make_float2(x, y);
         }
+        *reinterpret_cast<float4*>(&sacc[warp][32 * quarter + dim]) = make_float4(t[0], t[1], t[2], t[3]);
         if (lane == 0) {
             sml[warp][0] = M;
             sml[warp][1] = L;
@@ -605,13 +610,13 @@ struct Sharing {
 };
 
 // All SMs balance best, but a share that crosses into another row pays for another sign table and merge; with few steps per
-// CTA that is dearer than idle SMs.  A step of 256 tokens costs about 1.4 us, a row (or part of one) 3 us; two CTAs of 8 warps
-// take 1.5 us for a step of 128 tokens each and 3.3 us for a row, side by side; a merge kernel adds 1.5.  Candidates: all
+// CTA that is dearer than idle SMs.  A step of 256 tokens costs about 1.4 us, a row (or part of one) 2.2 us; two CTAs of 8 warps
+// take 1.5 us for a step of 128 tokens each and 2.5 us for a row, side by side; a merge kernel adds 1.5.  Candidates: all
 // CTAs; every row cut into the same number of parts; whole rows.  (16 warps, 64 x 1000 tokens: 148 CTAs 15.3 us, 128 CTAs 9;
 // 64 x 32768: 90.8 against 95.)
 static Sharing share_among(int64_t BH, int64_t Sk, int64_t ctas, int warps) {
     const int64_t S = (Sk + step_tokens(warps) - 1) / step_tokens(warps), total = BH * S;
-    const double step_us = warps == kPaWarps ? 1.4 : 1.5, row_us = warps == kPaWarps ? 3.0 : 3.3;
+    const double step_us = warps == kPaWarps ? 1.4 : 1.5, row_us = warps == kPaWarps ? 2.2 : 2.5;
     auto cost = [&](int64_t steps, int64_t rows) { return step_us * static_cast<double>(steps) + row_us * static_cast<double>(rows); };
     constexpr double kMergeUs = 1.5;
     Sharing best = {warps, total < ctas ? total : ctas, 0.0, false};
