@@ -611,7 +611,8 @@ struct Sharing {
 
 // All SMs balance best, but a share that crosses into another row pays for another sign table and merge; with few steps per
 // CTA that is dearer than idle SMs.  A step of 256 tokens costs about 1.4 us, a row (or part of one) 2.2 us; two CTAs of 8 warps
-// take 1.5 us for a step of 128 tokens each and 2.5 us for a row, side by side; a merge kernel adds 1.5.  Candidates: all
+// take 1.5 us for a step of 128 tokens each and 2.5 us for a row, side by side; a merge kernel adds 1.5.  (Rows
+// alone have come down to 1.3 and 1.6; with that 3-bit 256 x 2048 takes 30.9 us instead of 27.1, 128 x 4000 28.4 for 27.0.)  Candidates: all
 // CTAs; every row cut into the same number of parts; whole rows.  (16 warps, 64 x 1000 tokens: 148 CTAs 15.3 us, 128 CTAs 9;
 // 64 x 32768: 90.8 against 95.)
 static Sharing share_among(int64_t BH, int64_t Sk, int64_t ctas, int warps) {
