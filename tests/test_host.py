@@ -221,6 +221,18 @@ def test_kernels_read_no_global_memory_before_the_previous_kernel_is_complete():
     assert waiting >= 11
 
 
+def test_barriers_are_initialised_once():
+    """mbarrier.init on a barrier that is one already is undefined: a kernel's set-up names each barrier a single time."""
+    csrc = os.path.join(ROOT, "turboquant-amd_b200", "csrc")
+    kernels = 0
+    for name in sorted(os.listdir(csrc)):
+        for kernel in re.split(r"__global__", re.sub(r"//[^\n]*", "", open(os.path.join(csrc, name)).read()))[1:]:
+            barriers = re.findall(r"\b(?:tc_)?mbar_init\(([^,]+),", kernel)
+            kernels += bool(barriers)
+            assert len(barriers) == len(set(barriers)), (name, barriers)
+    assert kernels >= 3
+
+
 def test_no_cpu_fallback():
     x = torch.randn(4, 128)
     c, b = make_codebook(128, 3)

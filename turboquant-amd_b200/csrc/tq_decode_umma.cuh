@@ -291,8 +291,6 @@ __global__ void __launch_bounds__(kUmThreads, 2) decode_umma_kernel(const Decode
         }
         mbar_init(bars + kSDone, 1);                  // tcgen05.commit
         mbar_init(bars + kSFree, 4);                  // key warps have read the score accumulators
-        mbar_init(bars + kSDone, 1);                  // tcgen05.commit
-        mbar_init(bars + kSFree, 4);                  // key warps have read the score accumulators
         fence_barrier_init();
     }
     if (warp == 9) {
