@@ -825,11 +825,13 @@ bool stream_is_better(int64_t pages, int64_t cache_pages, int max_pages, int64_t
     if (pages < kStreamMinPages || pages > INT32_MAX || cache_pages > UINT32_MAX) return false;
     return pages >= 32768 || (max_pages >= 64 && (pages >= 16384 || chunks > kChunkedWave));
 }
-// Workspace of the persistent kernel, or 0 where no format would take it.
-int64_t stream_bytes(int64_t pages) {
-    if (pages < kStreamMinPages || pages > INT32_MAX) return 0;
+// Workspace of the persistent kernel, or 0 where no call takes it.
+int64_t stream_bytes(int64_t pages, int64_t cache_pages, int max_pages, int64_t chunks) {
+    if (!stream_is_better(pages, cache_pages, max_pages, chunks)) return 0;
     return kStreamSlots * (kStreamSlotFloats + 16) * static_cast<int64_t>(sizeof(float)) + kStreamCtas * static_cast<int64_t>(sizeof(int4));
 }
+// Chunks of all sequences, KV heads and query groups.
+int64_t chunks_at_most(int64_t pages, int max_pages, int chunk_pages) { return pages / max_pages * ((max_pages + chunk_pages - 1) / chunk_pages); }
 
 }  // namespace
 }  // namespace tq
@@ -898,7 +900,10 @@ extern "C" int64_t tq_decode_workspace_bytes(int num_seqs, int num_q_heads, int 
 extern "C" int64_t tq_decode_auto_workspace_bytes(int num_seqs, int num_q_heads, int num_kv_heads, int max_pages_per_seq) {
     const int64_t chunked = tq_decode_workspace_bytes(num_seqs, num_q_heads, num_kv_heads, max_pages_per_seq, 0);
     if (chunked < 0) return chunked;
-    const int64_t stream = stream_bytes(pages_at_most(num_seqs, num_q_heads, num_kv_heads, max_pages_per_seq));
+    const int64_t pages = pages_at_most(num_seqs, num_q_heads, num_kv_heads, max_pages_per_seq);
+    const int chunk_pages = tq_decode_auto_chunk_pages(num_seqs, num_kv_heads, num_q_heads, max_pages_per_seq);
+    // (a cache of too many pages for the persistent kernel is not known here: such a call has the larger workspace and does without)
+    const int64_t stream = stream_bytes(pages, 0, max_pages_per_seq, chunks_at_most(pages, max_pages_per_seq, chunk_pages));
     return stream > chunked ? stream : chunked;
 }
 
@@ -930,8 +935,8 @@ extern "C" int tq_decode_paged(void* out, const void* q_rot, const void* q_proj,
     if (split_is_ours) chunk_pages = tq_decode_auto_chunk_pages(num_seqs, num_kv_heads, num_q_heads, max_pages_per_seq);
     const int64_t need = tq_decode_workspace_bytes(num_seqs, num_q_heads, num_kv_heads, max_pages_per_seq, chunk_pages);
     const int max_chunks = (max_pages_per_seq + chunk_pages - 1) / chunk_pages;
-    const int64_t chunks = pages / max_pages_per_seq * max_chunks;   // of all sequences, KV heads and query groups
-    const int64_t stream_need = split_is_ours && !tensor_memory && stream_is_better(pages, num_blocks * num_kv_heads * (block_size / kPageTokens), max_pages_per_seq, chunks) ? stream_bytes(pages) : 0;
+    const int64_t cache_pages = num_blocks * num_kv_heads * (block_size / kPageTokens);
+    const int64_t stream_need = split_is_ours && !tensor_memory ? stream_bytes(pages, cache_pages, max_pages_per_seq, chunks_at_most(pages, max_pages_per_seq, chunk_pages)) : 0;
     const bool persistent = stream_need > 0 && workspace && workspace_bytes >= stream_need && !(reinterpret_cast<uintptr_t>(workspace) & 15);
     if (!persistent && max_chunks > 1 && (!workspace || workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 15)))
         return TQ_ERR_WORKSPACE;
