@@ -327,3 +327,22 @@ def test_sign_operands_at_the_edge_of_fp16(value, kw):
     ref = torch.stack([_attend64(q[i], q[i], cache, bt[i, :-(-m // 16)], books, 16, m, hkv) for i, m in enumerate(lens)])
     error = (out.double().view(ref.shape) - ref).pow(2).sum(dim=(0, 1, 3)).sqrt() / ref.pow(2).sum(dim=(0, 1, 3)).sqrt()
     assert (error <= 2e-3).all(), error
+
+
+@pytest.mark.parametrize("fmt", [(4, 4, False), (3, 3, True), (2, 2, True), (4, 3, False)])
+@pytest.mark.parametrize("ns,persistent", [(31, False), (32, True)])
+def test_which_kernel_takes_a_batch(fmt, ns, persistent):
+    """1024 tokens and 8 KV heads: below 16384 pages the chunked kernel runs as if its split had been asked for, from there the persistent
+    one, with the workspace that the host path names.  Both round the weights (2-norm 1e-4) and the output (2.8e-4) to fp16 on their own."""
+    fmt = CacheFormat(*fmt)
+    books = Codebooks(fmt, DEV)
+    lens = [1024 - 37 * (i % 4) for i in range(ns)]
+    bt, blocks = _tables(lens, 16, 9)
+    cache = _random_cache(fmt, blocks, 8, 16, 10)
+    q = torch.randn(ns, 32, 128, generator=torch.Generator(device=DEV).manual_seed(11), device=DEV).half()
+    call = lambda **kw: paged_decode_attention(q, cache, bt.to(DEV), torch.tensor(lens, dtype=torch.int32, device=DEV), books, 16, **kw)
+    got, chunked = call(), call(chunk_pages=_native.lib().tq_decode_auto_chunk_pages(ns, 8, 32, 64))
+    assert _native.read_status(DEV) == 0
+    assert torch.equal(got, chunked) != persistent
+    rows = (got.float() - chunked.float()).pow(2).sum(-1).sqrt() / chunked.float().pow(2).sum(-1).sqrt()
+    assert rows.max() < 2e-3 and rows.pow(2).mean().sqrt() < 8e-4, (rows.max(), rows.pow(2).mean().sqrt())

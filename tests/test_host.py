@@ -161,11 +161,11 @@ def test_host_only_entry_points():
     assert L.tq_packed_attention_workspace_bytes(8, 16) == 8 * 16 * 130 * 4
 
 
-@pytest.mark.parametrize("seqs,pages,persistent", [(24, 64, False), (27, 64, False), (28, 64, True), (1, 1750, False), (1, 2048, True),
+@pytest.mark.parametrize("seqs,pages,persistent", [(24, 64, False), (28, 64, False), (31, 64, False), (1, 2047, False), (1, 2048, True), (32, 64, True),
                                                    (64, 32, False), (128, 16, False), (127, 32, False), (128, 32, True), (32, 63, False), (33, 64, True)])
 def test_decode_workspace_is_that_of_the_kernel_that_runs(seqs, pages, persistent):
-    """The persistent kernel's 11 MB are named only for shapes that it takes; 8 KV heads, 32 query heads.  From 12288 pages on it takes
-    sequences of 64 pages or more in more than 444 chunks, from 16384 all of those, from 32768 everything."""
+    """The persistent kernel's 11 MB are named only for shapes that it takes; 8 KV heads, 32 query heads.  From 16384 pages on it takes
+    sequences of 64 pages or more, from 32768 everything."""
     L = _native.lib()
     chunked = L.tq_decode_workspace_bytes(seqs, 32, 8, pages, 0)
     named = L.tq_decode_auto_workspace_bytes(seqs, 32, 8, pages)

@@ -805,33 +805,35 @@ int dispatch_v(const DecodeParams& p, int vb, const Plan& plan, cudaStream_t str
     return TQ_ERR_UNSUPPORTED;
 }
 
-// Which kernel is the better one, by the pages that the batch can have at most.  The persistent kernel pays about 9 us
-// however few pages there are (all its tables, one more level of merging), the chunked one 5 to 9, but it takes
-// 0.4 (4-bit) to 0.5 us (with sign term) per 1000 pages where the chunked one takes 0.7 to 0.8; sequences of few pages
-// cost it more, a warp then changes item every few pages.  Measured with both as they are, us per launch in a graph over caches that
-// L2 does not hold, rotated queries, chunked / persistent, 8 KV heads, turbo4 and turbo3: 16 x 512 tokens (4096 pages) 8.8 / 13.2 and
-// 9.7 / 13.8; 1 x 16384 (8192) 14.4 / 15.5 and 13.6 / 16.4, 32 x 512 14.4 / 14.7 and 13.8 / 16.0; 24 x 1024 (12288) 14.8 / 17.7 and
-// 20.4 / 19.6; 64 x 512 (16384) 18.7 / 18.9 and 18.4 / 21.0, 128 x 256 20.4 / 18.5 and 19.3 / 20.0.
-// Below 16384 pages sequences of 64 pages or more go by waves: 4-bit chunks run 3 to an SM, and with more than 444 of them the
-// chunked kernel takes 5 us more at once: 27 x 1024 tokens (432 chunks) 14.8 / 17.7 and 20.4 / 19.5, 28 x 1024 (448) 20.3 / 18.3 and
-// 20.6 / 20.4, 13 x 2000 (416) 15.1 / 17.4 and 20.7 / 19.2, 14 x 2000 (448) 19.9 / 17.7 and 20.9 / 19.4, 7 x 4096 (448) 19.7 / 18.1 and
-// 20.8 / 20.1, 1 x 28000 (440) 14.9 / 18.2 and 20.3 / 19.6, 31 x 1024 (496) 20.8 / 18.8 and 20.6 / 20.9.  The lines do not look at the format: the
-// other kernel is up to 8 % faster for 12288 to 13824 pages of turbo3 and 10 % for 128 x 256 of turbo4.
-constexpr int64_t kStreamMinPages = 12288;
-constexpr int64_t kChunkedWave = 3 * 148;
+// Which kernel is the better one, by the pages that the batch can have at most: the table's width (or the longest length, where the
+// caller names it), for the lengths are on the device.  The persistent kernel pays 8 to 9 us however few pages there are (all its tables,
+// one more level of merging), the chunked one 5 to 7, but it takes 0.4 (4-bit) to 0.5 us (with sign term) per 1000 pages where the chunked
+// one takes 0.7 to 0.8; sequences of few pages cost it more, a warp then changes item every few pages.  us per launch in a graph over
+// caches that L2 does not hold, rotated queries, 32 query and 8 KV heads, tables as wide as the sequences are long, chunked / persistent,
+// turbo4 and turbo3: 1 x 16384 tokens (8192 pages) 14.5 / 15.6 and 13.7 / 16.5, 32 x 512 14.5 / 14.6 and 13.8 / 15.6; 64 x 512 (16384)
+// 18.8 / 18.8 and 18.4 / 20.6, 32 x 1024 20.9 / 19.0 and 20.6 / 20.7; 64 x 640 (20480) 21.9 / 21.1 and 21.9 / 23.0.
+// The lines do not look at the format, nor at how long the sequences in the table are.  What that costs, for 28 x 1024 tokens (14336 pages) and
+// for 28 sequences of 512 and of 100 tokens in tables for 1024:
+//   turbo4            20.4 / 18.6   14.6 / 14.6   7.8 / 11.0
+//   turbo4 Sparse-V   21.6 / 18.4   15.2 / 14.5   8.1 / 11.0
+//   turbo3            20.6 / 20.4   20.1 / 15.5   9.0 / 11.6
+//   turbo2            19.6 / 19.2   18.3 / 15.2   9.3 / 11.6
+//   K 4, V 3 bits     21.8 / 18.2   13.2 / 14.3   7.7 / 10.9
+// (turbo4 27 x 1024, whose 432 chunks run three to an SM in one wave: 14.8 / 17.8.)  A rule that sent more than 444 chunks of 12288 pages or
+// more to the persistent kernel took 2 to 4 us from nearly empty tables, such as a captured step of few requests has, and was taken back; from
+// 16384 pages on they lose as much (1 sequence of 100 tokens in a table for 32768: 5.8 / 10.1 and 6.1 / 10.6).
+constexpr int64_t kStreamMinPages = 16384;
 constexpr int64_t kStreamSlots = static_cast<int64_t>(kStreamCtas) * (kStreamWarps + 2);   // partials of warps and of CTAs
 int64_t pages_at_most(int64_t ns, int64_t hq, int64_t hkv, int64_t max_pages) { return ns * max_pages * hkv * ((hq / hkv + 7) / 8); }
-bool stream_is_better(int64_t pages, int64_t cache_pages, int max_pages, int64_t chunks) {
+bool stream_is_better(int64_t pages, int64_t cache_pages, int max_pages) {
     if (pages < kStreamMinPages || pages > INT32_MAX || cache_pages > UINT32_MAX) return false;
-    return pages >= 32768 || (max_pages >= 64 && (pages >= 16384 || chunks > kChunkedWave));
+    return pages >= 32768 || max_pages >= 64;
 }
 // Workspace of the persistent kernel, or 0 where no call takes it.
-int64_t stream_bytes(int64_t pages, int64_t cache_pages, int max_pages, int64_t chunks) {
-    if (!stream_is_better(pages, cache_pages, max_pages, chunks)) return 0;
+int64_t stream_bytes(int64_t pages, int64_t cache_pages, int max_pages) {
+    if (!stream_is_better(pages, cache_pages, max_pages)) return 0;
     return kStreamSlots * (kStreamSlotFloats + 16) * static_cast<int64_t>(sizeof(float)) + kStreamCtas * static_cast<int64_t>(sizeof(int4));
 }
-// Chunks of all sequences, KV heads and query groups.
-int64_t chunks_at_most(int64_t pages, int max_pages, int chunk_pages) { return pages / max_pages * ((max_pages + chunk_pages - 1) / chunk_pages); }
 
 }  // namespace
 }  // namespace tq
@@ -901,9 +903,8 @@ extern "C" int64_t tq_decode_auto_workspace_bytes(int num_seqs, int num_q_heads,
     const int64_t chunked = tq_decode_workspace_bytes(num_seqs, num_q_heads, num_kv_heads, max_pages_per_seq, 0);
     if (chunked < 0) return chunked;
     const int64_t pages = pages_at_most(num_seqs, num_q_heads, num_kv_heads, max_pages_per_seq);
-    const int chunk_pages = tq_decode_auto_chunk_pages(num_seqs, num_kv_heads, num_q_heads, max_pages_per_seq);
     // (a cache of too many pages for the persistent kernel is not known here: such a call has the larger workspace and does without)
-    const int64_t stream = stream_bytes(pages, 0, max_pages_per_seq, chunks_at_most(pages, max_pages_per_seq, chunk_pages));
+    const int64_t stream = stream_bytes(pages, 0, max_pages_per_seq);
     return stream > chunked ? stream : chunked;
 }
 
@@ -931,13 +932,12 @@ extern "C" int tq_decode_paged(void* out, const void* q_rot, const void* q_proj,
     // The persistent kernel takes the calls that leave the split to the library and bring the workspace for it.
     const bool tensor_memory = use_tcgen05 && k_bits <= 3 && v_bits <= 3 && !(sparse_thresh > 0.f);
     const int64_t pages = pages_at_most(num_seqs, num_q_heads, num_kv_heads, max_pages_per_seq);
-    const bool split_is_ours = chunk_pages <= 0;
-    if (split_is_ours) chunk_pages = tq_decode_auto_chunk_pages(num_seqs, num_kv_heads, num_q_heads, max_pages_per_seq);
+    const int64_t cache_pages = num_blocks * num_kv_heads * (block_size / kPageTokens);
+    const int64_t stream_need = chunk_pages <= 0 && !tensor_memory ? stream_bytes(pages, cache_pages, max_pages_per_seq) : 0;
+    const bool persistent = stream_need > 0 && workspace && workspace_bytes >= stream_need && !(reinterpret_cast<uintptr_t>(workspace) & 15);
+    if (chunk_pages <= 0) chunk_pages = tq_decode_auto_chunk_pages(num_seqs, num_kv_heads, num_q_heads, max_pages_per_seq);
     const int64_t need = tq_decode_workspace_bytes(num_seqs, num_q_heads, num_kv_heads, max_pages_per_seq, chunk_pages);
     const int max_chunks = (max_pages_per_seq + chunk_pages - 1) / chunk_pages;
-    const int64_t cache_pages = num_blocks * num_kv_heads * (block_size / kPageTokens);
-    const int64_t stream_need = split_is_ours && !tensor_memory ? stream_bytes(pages, cache_pages, max_pages_per_seq, chunks_at_most(pages, max_pages_per_seq, chunk_pages)) : 0;
-    const bool persistent = stream_need > 0 && workspace && workspace_bytes >= stream_need && !(reinterpret_cast<uintptr_t>(workspace) & 15);
     if (!persistent && max_chunks > 1 && (!workspace || workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 15)))
         return TQ_ERR_WORKSPACE;
     if (num_seqs > 65535 || max_chunks > 65535) return TQ_ERR_UNSUPPORTED;
