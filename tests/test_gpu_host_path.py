@@ -149,6 +149,27 @@ def test_packed_attention_work_sharing(bits, BH, Sk):
 
 
 @pytest.mark.parametrize("bits", [2, 3])
+@pytest.mark.parametrize("BH,Sk", [(1, 129), (1, 1000), (2, 257), (16, 500), (30, 255), (74, 250), (148, 130), (148, 700), (50, 9000)])
+def test_packed_attention_few_steps(bits, BH, Sk):
+    """Calls of few steps: CTAs of 8 warps, one to an SM or two, whole rows or steps shared evenly."""
+    test_packed_attention_work_sharing(bits, BH, Sk)
+
+
+@pytest.mark.parametrize("bits", [2, 3])
+@pytest.mark.parametrize("BH,Sk", [(150, 700), (180, 700), (290, 1500), (600, 200)])
+def test_packed_attention_deals_whole_rows_where_they_cost_least(bits, BH, Sk):
+    """Rows of some steps, about as many as CTAs run at a time: dealt out whole to CTAs of 8 warps, the arrangement of num_splits = 1."""
+    c, b = make_codebook(128, bits, device=DEV)
+    g = torch.Generator(device=DEV).manual_seed(BH + Sk)
+    r = lambda w: torch.randint(0, 256, (BH, Sk, w), generator=g, dtype=torch.uint8, device=DEV)
+    norm = lambda: torch.rand(BH, Sk, generator=g, device=DEV).half()
+    q = torch.randn(BH, 128, generator=g, device=DEV).half()
+    args = (q, q, r(16 * bits), r(16), norm(), norm(), r(16 * bits), norm(), c, 0.0098)
+    # another arrangement adds the same fp32 weights in another order: some fp16 output of thousands differs
+    assert torch.equal(packed_attention(*args), packed_attention(*args, num_splits=1))
+
+
+@pytest.mark.parametrize("bits", [2, 3])
 @pytest.mark.parametrize("BH,Sk", [(149, 128), (150, 600), (296, 129), (297, 128), (593, 17), (700, 500)])
 def test_packed_attention_two_ctas_per_sm(bits, BH, Sk):
     """More rows than SMs: CTAs of 8 warps, two per SM, around one and two waves of them and the ends of a 128-token step."""

@@ -20,7 +20,7 @@
 namespace tq {
 namespace {
 
-// Warps of a CTA: 16, one CTA per SM (up to 128 registers per thread), or 8, two CTAs per SM, whose sign tables and merges
+// Warps of a CTA: 16, one CTA per SM (up to 128 registers per thread), or 8, up to two CTAs per SM, whose sign tables and merges
 // then overlap with one another's steps (2- and 3-bit; the 4-bit tables leave room for one CTA only).
 constexpr int kPaWarps = 16, kPaHalfWarps = 8;
 __host__ __device__ constexpr int step_tokens(int warps) { return warps * 16; }   // tokens of one step of the CTA, 16 per warp
@@ -609,39 +609,60 @@ struct Sharing {
     bool whole;   // rows are dealt out whole (no merge kernel); else the steps of all rows are shared
 };
 
+// What a call is estimated to take, in us: a launch costs `start`, a step of the CTA `step`, a row (or part of one) of its share `row`
+// for the sign table and the merge, the merge kernel kMergeUs and for every further 32 parts of a row kMorePartsUs.  CTAs of 8 warps
+// depend on whether another one runs on the SM.  Times of every arrangement of 1339 calls, 1 to 2000 rows of 64 to 65536 tokens, at most 2.7 M
+// in all, 2, 3 and 4 bits, in a graph: least squares give 1.0 / 1.5 / 1.6, 2.1 / 1.4 / 1.5 and 2.1 / 0.8 / 0.4, merge 1.25; the
+// values below choose best among them (0.2 % over the fastest arrangement in the mean, 13 % at most; steps of 1.4 or 1.5 and rows of 2.2 or
+// 2.5 whatever else runs on the SM: 4 % and 35 %).  On 520 other calls 0.2 % and 15 %; against those values 3.6 % faster in the mean, 7 %
+// slower at most (35 x 434), 2 % next to that.
+struct ShareCosts { double start, step, row; };
+constexpr ShareCosts kCostsOneCta = {1.1, 1.5, 1.7}, kCostsTwoCtas = {1.75, 1.45, 1.35}, kCostsHalfCta = {1.75, 0.85, 0.45};
+constexpr double kMergeUs = 2.1, kMorePartsUs = 0.65;
+
 // All SMs balance best, but a share that crosses into another row pays for another sign table and merge; with few steps per
-// CTA that is dearer than idle SMs.  A step of 256 tokens costs about 1.4 us, a row (or part of one) 2.2 us; two CTAs of 8 warps
-// take 1.5 us for a step of 128 tokens each and 2.5 us for a row, side by side; a merge kernel adds 1.5.  (Rows
-// alone have come down to 1.3 and 1.6; with that 3-bit 256 x 2048 takes 30.9 us instead of 27.1, 128 x 4000 28.4 for 27.0.)  Candidates: all
-// CTAs; every row cut into the same number of parts; whole rows.  (16 warps, 64 x 1000 tokens: 148 CTAs 15.3 us, 128 CTAs 9;
-// 64 x 32768: 90.8 against 95.)
-static Sharing share_among(int64_t BH, int64_t Sk, int64_t ctas, int warps) {
+// CTA that is dearer than idle SMs.  Candidates: all CTAs; every row cut into the same number of parts; whole rows.
+static Sharing share_among(int64_t BH, int64_t Sk, int64_t sms, int warps) {
+    const int64_t ctas = warps == kPaWarps ? sms : 2 * sms;
     const int64_t S = (Sk + step_tokens(warps) - 1) / step_tokens(warps), total = BH * S;
-    const double step_us = warps == kPaWarps ? 1.4 : 1.5, row_us = warps == kPaWarps ? 2.2 : 2.5;
-    auto cost = [&](int64_t steps, int64_t rows) { return step_us * static_cast<double>(steps) + row_us * static_cast<double>(rows); };
-    constexpr double kMergeUs = 1.5;
+    auto costs = [&](int64_t running) { return warps == kPaWarps ? kCostsOneCta : running > sms ? kCostsTwoCtas : kCostsHalfCta; };
+    auto share = [&](int64_t running, int64_t steps, int64_t rows) {
+        const ShareCosts c = costs(running);
+        return c.start + c.step * static_cast<double>(steps) + c.row * static_cast<double>(rows);
+    };
+    auto merge = [&](int64_t parts) { return kMergeUs + kMorePartsUs * static_cast<double>((parts - 1) / 32); };
     Sharing best = {warps, total < ctas ? total : ctas, 0.0, false};
     const int64_t each = (total + best.ctas - 1) / best.ctas;
-    best.us = cost(each, 1 + (each - 1 + S - 1) / S) + kMergeUs;
+    best.us = share(best.ctas, each, 1 + (each - 1 + S - 1) / S) + merge((best.ctas + BH - 1) / BH);
     auto consider = [&](const Sharing& other) {
         if (other.us < best.us) best = other;
     };
     if (BH <= ctas) {
         const int64_t parts = ctas / BH < S ? ctas / BH : S;
-        consider({warps, BH * parts, cost((S + parts - 1) / parts, 1) + kMergeUs, false});
+        consider({warps, BH * parts, share(BH * parts, (S + parts - 1) / parts, 1) + merge(parts), false});
+        consider({warps, BH, share(BH, S, 1), true});
+    } else {   // the rows of the last round have an SM to themselves the more the fewer they are
+        const int64_t rounds = BH / ctas, left = BH % ctas;
+        double us = share(ctas, rounds * S, rounds);
+        if (left) {
+            const ShareCosts busy = costs(ctas), lone = costs(left);
+            const double crowd = left < sms ? static_cast<double>(left) / static_cast<double>(sms) : 1.0;
+            const double alone = lone.step * static_cast<double>(S) + lone.row, among = busy.step * static_cast<double>(S) + busy.row;
+            us += alone + crowd * (among - alone);
+        }
+        consider({warps, ctas, us, true});
     }
-    const int64_t rows = (BH + ctas - 1) / ctas;
-    consider({warps, BH < ctas ? BH : ctas, cost(rows * S, rows), true});
     return best;
 }
 
-// Many rows of few steps are mostly sign tables and merges, which overlap where two CTAs share an SM.  Measured in a graph, us, one
-// CTA of 16 warps / two of 8, 3-bit: 150 x 300 tokens 14.2 / 10.3, 256 x 500 16.1 / 13.0, 256 x 2048 32.5 / 29.9, 1000 x 256
-// 40.8 / 33.5, 2000 x 64 62.3 / 40.9.
+// Many rows of few steps are mostly sign tables and merges, which overlap where two CTAs share an SM.  Measured in a graph, us, the best
+// arrangement with CTAs of 16 warps / of 8, 3-bit: 150 x 700 tokens 13.5 / 12.2, 256 x 500 12.6 / 10.4, 256 x 2048 30.6 / 28.0, 1000 x 256
+// 26.7 / 22.5, 2000 x 64 37.3 / 22.0, 64 x 32768 87.4 / 85.7.  Few steps start sooner with 8: 1 x 1000 6.4 / 4.9, 16 x 500 6.5 / 5.2.  A row of many
+// steps takes fewer parts with 16: 1 x 32768 9.1 / 12.7, 2 x 16000 7.5 / 9.4.
 static Sharing share_out(int64_t BH, int64_t Sk, int bits, int64_t sms) {
     const Sharing one = share_among(BH, Sk, sms, kPaWarps);
     if (bits == 4) return one;
-    const Sharing two = share_among(BH, Sk, 2 * sms, kPaHalfWarps);
+    const Sharing two = share_among(BH, Sk, sms, kPaHalfWarps);
     return two.us < one.us ? two : one;
 }
 
