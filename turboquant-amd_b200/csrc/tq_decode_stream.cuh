@@ -225,6 +225,7 @@ __device__ __forceinline__ void combine_partials(const StreamParams& sp, const i
     const DecodeParams& p = sp.d;
     float* weight = reinterpret_cast<float*>(sm_scan);     // [8][32]
     float2* sum = reinterpret_cast<float2*>(sm_len);       // [8][32], at a run's first entry: (maximum, denominator)
+    static_assert(2 * kStreamWarps == 32 && kStreamThreads * sizeof(int) >= 8 * 32 * sizeof(float2), "one lane an entry; the scan's arrays hold weights and sums");
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rows = min(8, p.G);
     const int4 part = sm_part[lane];
     const uint32_t live = __ballot_sync(0xffffffffu, part.x >= 0);
@@ -342,6 +343,9 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
     __shared__ int4 sm_part[2 * kStreamWarps];
     __shared__ int sm_pool;
     __shared__ uint32_t sm_skipped[SPARSE ? kStreamWarps : 1];
+    static_assert(RING >= kStreamPartBytes, "a warp's last partial lies in its ring");
+    static_assert(sizeof(sm_scan) + sizeof(sm_len) + sizeof(sm_wsum) + sizeof(sm_window) + sizeof(sm_part) + sizeof(sm_pool) + sizeof(sm_skipped) + 7 * 16 <= kStreamStaticMost,
+                  "what stream_pool leaves for static arrays");
 
     const int warp = uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
     const int gid = lane >> 2, tig = lane & 3;
