@@ -9,6 +9,7 @@ import pytest
 import torch
 
 from tests.test_gpu_decode import DEV, assert_attn_close, oracle_decode, random_fields
+from turboquant.core.codebook import make_codebook
 from turboquant.kernels import _native, paged_layout
 from turboquant.kernels.paged import CacheFormat, Codebooks, paged_decode_attention
 
@@ -258,33 +259,44 @@ def test_scores_of_uneven_queries(kb, vb, qjl, form, dtype):
 
 @pytest.mark.parametrize("kb,vb", [(2, 2), (3, 3), (4, 4)])
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
-@pytest.mark.parametrize("kw", [dict(), dict(chunk_pages=64), dict(chunk_pages=64, sparse_thresh=1e-6)])
+@pytest.mark.parametrize("kw", [dict(), dict(chunk_pages=64), dict(chunk_pages=64, sparse_thresh=1e-6), dict(sparse_thresh=1e-9)])
 @pytest.mark.parametrize("separate", [False, True])
 def test_sign_term_of_large_queries(kb, vb, dtype, kw, separate):
-    """Coordinates beyond 255, at each of the four places that the one-sided sign forms treat differently: no overflow to NaN.
+    """Coordinates on both sides of 511, where rows begin to be divided, at each of the four dims of a quarter that the sign term scales by
+    2^7; far larger ones at others; a row of many: no overflow to NaN, no place treated wrongly.
     The scores reach thousands, so one rounding in 32 bits moves a weight by up to 5e-4; next to that weights and output are rounded
-    to 11 bits (bf16: the output to 8)."""
+    to 11 bits (bf16: the output to 8).  Without a split Sparse-V runs the persistent kernel on sequences four times as long, 20 pages a warp,
+    of which all but the first four can come without their V part (4000 of 47624 pages and more do); what is left out adds up to 1e-9 for each
+    of 98324 tokens at most."""
     fmt = CacheFormat(kb, vb, True)
-    books = Codebooks(fmt, DEV)
-    ns, hkv = len(LONG), 4
-    bt, blocks = _tables(LONG, 16, 6)
+    c, b = make_codebook(128, kb)
+    books = Codebooks(fmt, DEV, k_codebook=(c.half().float(), b))   # fp16 operands: rounding a centroid moves a score of thousands by more
+    skips = "sparse_thresh" in kw and "chunk_pages" not in kw
+    lens = [4 * n for n in LONG] if skips else LONG
+    ns, hkv = len(lens), 4
+    bt, blocks = _tables(lens, 16, 6)
     cache = _random_cache(fmt, blocks, hkv, 16, 5)
     g = torch.Generator(device=DEV).manual_seed(2)
 
     def make():
         q = torch.randn(ns, hkv, 8, 128, generator=g, device=DEV)
-        for head, dim, value in ((1, 16, 254), (2, 16, 256), (3, 17, 300), (4, 31, 1000), (5, 18, 30000), (6, 16, -40000)):
+        if skips:
+            q *= 100                                          # a softmax so peaked that many pages weigh nothing in any row
+        for head, dim, value in ((1, 4, 508), (2, 32 + 12, 511.5), (3, 64 + 20, -512), (4, 96 + 28, 1000), (5, 18, 30000), (6, 16, -40000)):
             q[:, :, head, dim] = value
-        q[:, :, 7] *= 80
-        q[:, :, 7, 100] = 290
+        q[:, :, 7] *= 4 if skips else 400
         return q.to(dtype)
 
     q = make()
     qp = make() if separate else q
-    out = paged_decode_attention(q.view(ns, -1, 128), cache, bt.to(DEV), torch.tensor(LONG, dtype=torch.int32, device=DEV), books, 16,
-                                 q_proj=qp.view(ns, -1, 128) if separate else None, **kw)
+    stats = torch.zeros(2, dtype=torch.int32, device=DEV)
+    out = paged_decode_attention(q.view(ns, -1, 128), cache, bt.to(DEV), torch.tensor(lens, dtype=torch.int32, device=DEV), books, 16,
+                                 q_proj=qp.view(ns, -1, 128) if separate else None, skip_stats=stats, **kw)
     assert _native.read_status(DEV) == 0
-    ref = torch.stack([_attend64(q[i], qp[i], cache, bt[i, :-(-n // 16)], books, 16, n, hkv) for i, n in enumerate(LONG)])
+    if skips:
+        seen, skipped = stats.tolist()
+        assert seen == hkv * sum(-(-n // 16) for n in lens) and skipped > seen // 25, (seen, skipped)
+    ref = torch.stack([_attend64(q[i], qp[i], cache, bt[i, :-(-n // 16)], books, 16, n, hkv) for i, n in enumerate(lens)])
     error = (out.double().view(ref.shape) - ref).pow(2).sum(dim=(0, 1, 3)).sqrt() / ref.pow(2).sum(dim=(0, 1, 3)).sqrt()
     assert (error <= (2e-3 if dtype == torch.float16 else 4e-3)).all(), error
 
