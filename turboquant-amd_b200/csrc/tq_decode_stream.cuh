@@ -12,10 +12,14 @@
 // What bounds it: instruction issue with four warps a scheduler (a tensor instruction costs about three slots) next to the
 // shared-memory data path (turbo3: 93 wavefronts a page), and under constant load the GPU's power: at 1000 W the clock falls from 1965
 // to 1765 MHz.  Sign operands by logic, 34 instructions and no shared memory, instead of looked up (20 instructions, 32 wavefronts,
-// 32 KB of table), us per launch in a graph, looked up / by logic: turbo3 64 x 8192 tokens 145.5 / 142.4, turbo2 64 x 4096 75.1 / 69.3.
-// A Sparse-V call does the same arithmetic; its page body has registers to spare for it since the count of skipped V parts lies in
-// shared memory and columns without a query are kept from deciding by their reference instead of by thresholds of their own
-// (32 x 8192: looked up 82.8, by logic 85.3, so 82.7; 64 x 8192 with groups of 4 150.4 / 155.3 / 148.3).
+// 32 KB of table), us per launch in a graph, looked up / by logic: turbo3 64 x 8192 tokens 145.5 / 142.4, turbo2 64 x 4096 75.1 / 70.5.
+// A Sparse-V call does the same arithmetic on the pages that come with their V part: one that skips nothing gives the dense result bit for bit.
+// A page without V part is the other way round: there is little else to do, so the instructions count.  Signs looked up there (3 and 4
+// bits, K and V of one codebook: the second table is free), rows not divided, and the count of skipped V parts where it needs no
+// register, us per launch in a graph, everything by logic / this, V parts skipped in brackets: turbo3 64 x 8192 150.5 / 143.5 (0 %),
+// 149 / 142 (45 %), with groups of 4 136 / 130.5 (68 %), 64 x 32768 467 / 446 (82 %), 16 x 32768 with one head a group 121 / 117.5 (88 %); looked up on
+// all pages, with 16 registers less of query operands, 427 and 113 of the last two, 153, 147 and 133 of the others.  2 bits: looked up 427, by
+// logic 415 (64 x 32768, 82 %).
 // 20 warps of 96 registers (151.6 for 145.6) or 24 of 80 (157.6) lose: the look-ups in flight need registers.
 // Pages are staged with cp.async, 16 bytes a lane, into a private ring: a page then costs four copy instructions and a counted
 // wait, where a bulk copy by one elected lane with its barrier cost about 35 instructions.  Together with a page body that has no
@@ -208,6 +212,22 @@ __device__ __forceinline__ void wht_16x8(float (&x)[16], int lane) {
     for (int i = 0; i < 16; ++i) x[i] *= kWhtScale;
 }
 
+// Sign table, indexed by one nibble of signs (four dims) of token A and one of token B: the four half2 of +-kSignUnit that are the A
+// operand of one score product, in its register order (A dims 0 1, B dims 0 1, A dims 2 3, B dims 2 3), 8 copies.  The sums then count
+// in what the one-sided operands count in.
+__device__ __forceinline__ void fill_sign_table(uint32_t smem_addr, int warp, int lane) {
+    auto signs = [](int pair) { return 0x84008400u ^ ((pair & 1) ? 0x8000u : 0u) ^ ((pair & 2) ? 0x80000000u : 0u); };
+    for (int b0 = 4 * warp; b0 < 256; b0 += 4 * kStreamWarps) {
+        const int b = b0 + (lane >> 3);
+        store_entry(smem_addr + b * 128 + 16 * (lane & 7), make_uint4(signs(b), signs(b >> 4), signs(b >> 2), signs(b >> 6)));
+    }
+}
+template <int K>
+__device__ __forceinline__ uint4 table_signs(uint32_t w, uint32_t base) {
+    uint4 v;
+    asm("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(entry_of<K>(w, base)));
+    return v;
+}
 // Output row g of an item.
 __device__ __forceinline__ void finish_row(const DecodeParams& p, int seq, int hg, int g, int lane, float (&x)[4], float l) {
     const int kvh = p.ngroups == 1 ? hg : hg / p.ngroups, qg = hg - kvh * p.ngroups;
@@ -319,7 +339,9 @@ __device__ __forceinline__ void combine_partials(const StreamParams& sp, const i
     }
 }
 
-template <int KB, int VB, bool QJL, bool SPARSE>
+// SIGN_TABLE: Sparse-V with K and V of one codebook and S = I looks up the signs of pages that come without their V part, in the second
+// table; the query operands of the index term serve them as well.
+template <int KB, int VB, bool QJL, bool SPARSE, bool SIGN_TABLE>
 __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const __grid_constant__ StreamParams sp) {
     constexpr int NWK = KB + (QJL ? 1 : 0);
     constexpr int RK = 16 * NWK;
@@ -342,7 +364,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
     // entry of even number lies: partial of the pool from 1, or 0 for the warp's slot in the workspace)
     __shared__ int4 sm_part[2 * kStreamWarps];
     __shared__ int sm_pool;
-    __shared__ uint32_t sm_skipped[SPARSE ? kStreamWarps : 1];
+    __shared__ uint32_t sm_skipped[SIGN_TABLE ? kStreamWarps : 1];
     static_assert(RING >= kStreamPartBytes, "a warp's last partial lies in its ring");
     static_assert(sizeof(sm_scan) + sizeof(sm_len) + sizeof(sm_wsum) + sizeof(sm_window) + sizeof(sm_part) + sizeof(sm_pool) + sizeof(sm_skipped) + 7 * 16 <= kStreamStaticMost,
                   "what stream_pool leaves for static arrays");
@@ -350,14 +372,15 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
     const int warp = uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
     const int gid = lane >> 2, tig = lane & 3;
 
-    const uint32_t ktab = smem_u32(smem), vtab = ktab + kStreamTable;
+    const uint32_t ktab = smem_u32(smem), vtab = ktab + (SIGN_TABLE ? 0 : kStreamTable), stab = ktab + kStreamTable;
     const uint32_t rings = ktab + 2 * kStreamTable, ring = rings + warp * RING;
 
+    if constexpr (SIGN_TABLE) fill_sign_table(stab, warp, lane);   // constants
     if (lane < 2) sm_part[2 * warp + lane] = make_int4(-1, 0, 0, 0);
     if (threadIdx.x == 0) sm_pool = 0;
     pdl_wait();
     pdl_release();
-    const float ck = lane_centroid<KB>(p.kc, lane), cv = lane_centroid<VB>(p.vc, lane);
+    const float ck = lane_centroid<KB>(p.kc, lane), cv = SIGN_TABLE ? 0.f : lane_centroid<VB>(p.vc, lane);
 
     // ---- pages before each thread's run of sequences (every CTA does the same scan over all lengths)
     // (With its sums by one reduction, shares by a constant and the K table filled while the block table's entries come: turbo4 1 x 131072
@@ -494,20 +517,23 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
             for (int i = lane; i < p.Hq * kHeadDim / 8; i += 32) o[i] = make_uint4(0, 0, 0, 0);
         }
     }
-    fill_stream_table<VB>(vtab, cv, warp, lane);   // behind the first pages' copies
+    if constexpr (!SIGN_TABLE) fill_stream_table<VB>(vtab, cv, warp, lane);   // behind the first pages' copies
     first_copies(kStreamFirst, NSTAGE);
     __syncthreads();
 
     const uint32_t klut = ktab + (KB == 2 ? 8 * (lane & 15) : 4 * lane);
     const uint32_t vlut = vtab + (VB == 2 ? 8 * (lane & 15) : 4 * lane);
+    const uint32_t slut = stab + 16 * (lane & 7);
     const uint32_t ring_k = ring + lane * (NWK * 4);
     const uint32_t ring_n = ring + gid * 4;
     const uint32_t ring_v = ring + (tig * 8 + gid) * 4;
 
     uint32_t stage = 0;                       // ring stage of the current page
-    uint32_t k_only = 0;                      // Sparse-V: bit s = the page in stage s came without its V part
-    if constexpr (SPARSE) {
-        if (lane == 0) sm_skipped[warp] = 0;   // V parts never fetched
+    // Sparse-V: bit s = the page in stage s came without its V part; above the stages' bits how many V parts were never fetched, or in
+    // shared memory (us per launch in a graph, here / in shared memory, turbo3 64 x 8192: with the sign table 146.3 / 143.7, without 150.7 / 156)
+    uint32_t k_only = 0;
+    if constexpr (SIGN_TABLE) {
+        if (lane == 0) sm_skipped[warp] = 0;
     }
     int idx = 0;                              // pages of the share that are done
 
@@ -550,6 +576,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
 
         auto one_page = [&](auto have_v, auto partly, auto large, int j) {
             constexpr bool HAVE_V = decltype(have_v)::value, PARTLY = decltype(partly)::value, LARGE = decltype(large)::value;
+            constexpr bool LOOK_UP = SIGN_TABLE && !HAVE_V;
             const uint32_t so = stage * PAGE;
             wait_copies<NSTAGE - 1>();
             __syncwarp();
@@ -557,8 +584,11 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
             uint32_t wa[NWK], wb[NWK];
             lds_words<NWK, 0>(ring_k + so, wa);
             lds_words<NWK, 32 * NWK * 4>(ring_k + so, wb);
-            uint32_t ra = 0, rb = 0;   // the sign words, rotated
-            if constexpr (QJL) {
+            uint32_t ra = 0, rb = 0;   // the sign words, rotated; to look up: the nibbles 2 k (ra), 2 k + 1 (rb) of token A, then of token B
+            if constexpr (LOOK_UP) {
+                ra = bit_select(wb[KB] << 4, wa[KB], 0x0f0f0f0fu);
+                rb = bit_select(wb[KB], wa[KB] >> 4, 0x0f0f0f0fu);
+            } else if constexpr (QJL) {
                 ra = rotate_signs(wa[KB]);
                 rb = rotate_signs(wb[KB]);
             }
@@ -566,9 +596,14 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
             if constexpr (QJL) krn = unpack_half2(lds_u32<KRN_OFF>(ring_n + so));
             float sm[4] = {0.f, 0.f, 0.f, 0.f};
             float sq[4] = {sq_init0, sq_init1, sq_init0, sq_init1}, sq2[4] = {0.f, 0.f, 0.f, 0.f};
+            if constexpr (LOOK_UP) sq[0] = sq[1] = sq[2] = sq[3] = 0.f;
             auto sign_term = [&](auto quarter) {   // eight dims of two tokens, two products
                 constexpr int C = decltype(quarter)::value;
-                if constexpr (QJL) {
+                if constexpr (LOOK_UP) {
+                    const uint4 g0 = table_signs<C>(ra, slut), g1 = table_signs<C>(rb, slut);
+                    mma_f16_16816(sq, g0.x, g0.y, g0.z, g0.w, qf[4 * C], qf[4 * C + 1]);
+                    mma_f16_16816(sq2, g1.x, g1.y, g1.z, g1.w, qf[4 * C + 2], qf[4 * C + 3]);
+                } else if constexpr (QJL) {
                     constexpr int I = 4 * C;
                     const uint32_t xa = wa[KB], xb = wb[KB];
                     mma_f16_16816(sq, sign_pair<I>(xa, ra), sign_pair<I>(xb, rb), sign_pair<I + 1>(xa, ra), sign_pair<I + 1>(xb, rb), qpf[I], qpf[I + 1]);
@@ -627,7 +662,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
                 krn.x *= p.qpscale;
                 krn.y *= p.qpscale;
                 float t0 = sq[0] + sq2[0], t1 = sq[1] + sq2[1], t2 = sq[2] + sq2[2], t3 = sq[3] + sq2[3];
-                if constexpr (LARGE) {
+                if constexpr (LARGE && !LOOK_UP) {
                     const float2 by = divided_by(divided, tig);
                     t0 *= by.x;
                     t1 *= by.y;
@@ -684,7 +719,8 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
                     wait_copies<0>();
                     __syncwarp();
                 } else {
-                    if (lane == 0) ++sm_skipped[warp];
+                    if constexpr (!SIGN_TABLE) k_only += 1u << NSTAGE;
+                    else if (lane == 0) ++sm_skipped[warp];
                     have = false;
                 }
             }
@@ -765,7 +801,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
         };
         auto next_page = [&](auto partly, auto large, int j) {
             if constexpr (SPARSE) {
-                if (k_only == 0 || !((k_only >> stage) & 1u)) one_page(std::true_type{}, partly, large, j);
+                if ((SIGN_TABLE && k_only == 0) || !((k_only >> stage) & 1u)) one_page(std::true_type{}, partly, large, j);
                 else one_page(std::false_type{}, partly, std::bool_constant<QJL>{}, j);   // (a row that is not divided is multiplied by one)
             } else {
                 one_page(std::true_type{}, partly, large, j);
@@ -856,16 +892,16 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
     if constexpr (SPARSE) {
         if (p.skip_stats && lane == 0) {
             atomicAdd(p.skip_stats, static_cast<uint32_t>(idx));
-            atomicAdd(p.skip_stats + 1, sm_skipped[warp]);
+            atomicAdd(p.skip_stats + 1, SIGN_TABLE ? sm_skipped[SIGN_TABLE ? warp : 0] : k_only >> NSTAGE);
         }
     }
     __syncthreads();
     combine_partials<RING>(sp, sm_part, rings, sm_scan, sm_len);
 }
 
-template <int KB, int VB, bool QJL, bool SPARSE>
-int launch_stream(const StreamParams& sp, cudaStream_t stream) {
-    auto kern = decode_stream_kernel<KB, VB, QJL, SPARSE>;
+template <int KB, int VB, bool QJL, bool SPARSE, bool SIGN_TABLE>
+int launch_stream_as(const StreamParams& sp, cudaStream_t stream) {
+    auto kern = decode_stream_kernel<KB, VB, QJL, SPARSE, SIGN_TABLE>;
     static bool configured[64] = {};
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return TQ_ERR_LAUNCH;
@@ -875,6 +911,14 @@ int launch_stream(const StreamParams& sp, cudaStream_t stream) {
         configured[dev] = true;
     }
     return launch_chained(kern, dim3(sp.n_warps / kStreamWarps), dim3(kStreamThreads), smem, stream, sp) == cudaSuccess ? TQ_OK : TQ_ERR_LAUNCH;
+}
+
+template <int KB, int VB, bool QJL, bool SPARSE>
+int launch_stream(const StreamParams& sp, cudaStream_t stream) {
+    if constexpr (QJL && SPARSE && KB == VB && KB >= 3) {
+        if (sp.d.share_tables && !sp.d.qp) return launch_stream_as<KB, VB, QJL, SPARSE, true>(sp, stream);
+    }
+    return launch_stream_as<KB, VB, QJL, SPARSE, false>(sp, stream);
 }
 
 // One block per CTA of the stream kernel: combines the parts of the item that starts there and ends in a later CTA, two
