@@ -383,8 +383,9 @@ __global__ void __launch_bounds__(kStreamThreads, 1) decode_stream_kernel(const 
     const float ck = lane_centroid<KB>(p.kc, lane), cv = SIGN_TABLE ? 0.f : lane_centroid<VB>(p.vc, lane);
 
     // ---- pages before each thread's run of sequences (every CTA does the same scan over all lengths)
-    // (With its sums by one reduction, shares by a constant and the K table filled while the block table's entries come: turbo4 1 x 131072
-    // tokens 40.5 / 39.7 us in a graph, a bf16 decode step of 32 sequences with its append 37.9 / 36.8.)
+    // (With its sums by one reduction, shares by a constant and the K table filled while the block table's entries come, all at once and with a
+    // prefetch of the lengths that alone gave nothing and is gone: turbo4 1 x 131072 tokens 40.5 / 39.7 us in a graph, a bf16 decode step of
+    // 32 sequences with its append 37.9 / 36.8.)
     const int per = (sp.ns + kStreamThreads - 1) / kStreamThreads;
     int own = 0, len0 = 0;
     for (int s = threadIdx.x * per; s < min(sp.ns, (static_cast<int>(threadIdx.x) + 1) * per); ++s) {
